@@ -216,7 +216,7 @@ int b200conv_padded_channels(int C, int dtype);
 int b200conv_malloc(b200conv_ctx* ctx, size_t bytes, void** dptr);   /* pooled, stream ordered */
 int b200conv_free(b200conv_ctx* ctx, void* dptr);
 int b200conv_host_alloc(b200conv_ctx* ctx, size_t bytes, void** hptr); /* pinned host memory */
-int b200conv_host_free(b200conv_ctx* ctx, void* hptr);
+int b200conv_host_free(b200conv_ctx* ctx, void* hptr);   /* ctx may be NULL: the memory may outlive its context */
 int b200conv_memcpy_h2d(b200conv_ctx* ctx, void* dst, const void* src, size_t bytes);  /* async */
 int b200conv_memcpy_d2h(b200conv_ctx* ctx, void* dst, const void* src, size_t bytes);  /* async */
 /* Background copies for callers that overlap transfers with compute (PCIe moves both ways at once):

@@ -1,0 +1,84 @@
+"""Host-pointer calls: batches that travel in chunks of images, pageable and page-locked results, and the
+pool of result memory."""
+import gc
+
+import numpy as np
+import pytest
+
+from oracle import corr_oracle as O
+from theano_b200 import shim
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 2, 7, 13, 24], ids=lambda n: "n%d" % n)     # one chunk, equal chunks, a smaller last one
+@pytest.mark.parametrize("pageable_out", [False, True])
+def test_chunked_batches_against_oracle(n, pageable_out):
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(n)
+    x = rs.standard_normal((n, 64, 61, 64)).astype(np.float32)              # 1 MB per image and side
+    w = (rs.standard_normal((64, 64, 1, 1)) / 8).astype(np.float32)
+    b, r = rs.standard_normal(64).astype(np.float32), rs.standard_normal(x.shape).astype(np.float32)
+    kw = dict(border_mode="valid", subsample=(1, 1))
+    out = np.full(x.shape, 7, np.float32) if pageable_out else None
+    y = shim.conv2d_forward(x, w, bias=b, residual=r, out=out, ctx=ctx, **kw)
+    assert (y is out) == pageable_out
+    # TF32 rounds each factor by at most 2^-10 relative: 5e-3 of the largest result is the repository's bound
+    assert O.rel_err(y, O.conv2d(x, w, **kw) + b[None, :, None, None] + r) < 5e-3
+    out = np.full(x.shape, 7, np.float32) if pageable_out else None
+    dx = shim.conv2d_grad_inputs(w, r, x.shape[2:], out=out, ctx=ctx, **kw)
+    assert O.rel_err(dx, O.conv2d_grad_inputs(w, r, x.shape[2:], **kw)) < 5e-3
+    # results of one call are inputs of the next: page-locked inputs take no staging copy
+    dw = shim.conv2d_grad_weights(y, dx, (1, 1), ctx=ctx, **kw)
+    assert O.rel_err(dw, O.conv2d_grad_weights(np.array(y), np.array(dx), (1, 1), **kw)) < 5e-3
+
+
+@pytest.mark.gpu
+def test_results_keep_their_values_while_others_are_made():
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(0)
+    xs = [rs.standard_normal((8, 8, 40, 40)).astype(np.float32) for _ in range(6)]
+    ys = [shim.maxpool2x2(x, ctx=ctx) for x in xs]
+    for x, y in zip(xs, ys):
+        assert np.array_equal(y, x.reshape(8, 8, 20, 2, 20, 2).max(axis=(3, 5)))
+
+
+class _FakeLibrary(object):
+    """Stands in for the library's page-locked allocator."""
+
+    def __init__(self):
+        self.made, self.buffers = 0, {}
+
+    def b200conv_host_alloc(self, h, size, p):
+        buf = np.empty(size, np.uint8)
+        self.buffers[buf.ctypes.data] = buf
+        p._obj.value = buf.ctypes.data
+        self.made += 1
+        return 0
+
+    def b200conv_host_free(self, h, p):
+        del self.buffers[p.value]
+        return 0
+
+
+def test_result_pool_reuses_and_gives_back(monkeypatch):
+    class Ctx(object):
+        lib, h = _FakeLibrary(), None
+    monkeypatch.setattr(shim, "load_library", lambda: Ctx.lib)
+    pool = shim._ResultPool()
+    pool.LIMIT, pool.KEEP = 4 << 20, 1 << 20
+    f32 = np.dtype(np.float32)
+    assert pool.empty(Ctx, (10,), f32).base is None                     # small: an ordinary array
+    a = pool.empty(Ctx, (100, 1000), f32)
+    ptr = a.ctypes.data
+    view = a[3:5]
+    del a
+    gc.collect()
+    assert pool.kept == 0                                               # the view keeps the memory
+    del view
+    b = pool.empty(Ctx, (99, 1001), f32)
+    assert b.ctypes.data == ptr and b.shape == (99, 1001) and b.dtype == f32 and b.flags.writeable
+    many = [pool.empty(Ctx, (1 << 18,), f32) for _ in range(8)]         # 1 MB each: over the limit
+    assert sum(m.base is not None for m in many) == 3 and pool.total <= pool.LIMIT
+    del many, b
+    gc.collect()
+    assert pool.kept <= pool.KEEP and pool.total == pool.kept and len(Ctx.lib.buffers) <= 2

@@ -4,8 +4,6 @@
 
 #include <algorithm>
 #include <chrono>
-#include <condition_variable>
-#include <functional>
 #include <thread>
 #include <cstdarg>
 #include <cstdio>
@@ -17,6 +15,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "staging.h"
 
 using namespace b200;
 
@@ -44,66 +43,11 @@ struct b200conv_graph {
   long long launches = 0;   // kernels in the graph
 };
 
-// Host staging for the host-pointer calls.  A pageable array travels over PCIe at the speed of
-// the driver's own staging copy (a single thread); here the array is cut into chunks that a few
-// threads copy into (out of) pinned buffers while the DMA engine moves the previous chunk, so the
-// link sees pinned transfers and the host side is copied in parallel.
-class CopyPool {
- public:
-  explicit CopyPool(int nthreads) {
-    for (int i = 0; i < nthreads; ++i) workers_.emplace_back([this, i, nthreads] { loop(i, nthreads); });
-  }
-  ~CopyPool() {
-    {
-      std::lock_guard<std::mutex> g(mu_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (auto& t : workers_) t.join();
-  }
-  // memcpy(dst, src, bytes), cut into one slice per worker; returns when all of it is copied
-  void copy(void* dst, const void* src, size_t bytes) {
-    std::unique_lock<std::mutex> g(mu_);
-    dst_ = static_cast<char*>(dst); src_ = static_cast<const char*>(src); bytes_ = bytes;
-    pending_ = static_cast<int>(workers_.size());
-    ++generation_;
-    cv_.notify_all();
-    done_.wait(g, [this] { return pending_ == 0; });
-  }
-
- private:
-  void loop(int index, int nthreads) {
-    unsigned long long seen = 0;
-    for (;;) {
-      char* d; const char* s_; size_t n;
-      {
-        std::unique_lock<std::mutex> g(mu_);
-        cv_.wait(g, [&] { return stop_ || generation_ != seen; });
-        if (stop_) return;
-        seen = generation_;
-        d = dst_; s_ = src_; n = bytes_;
-      }
-      const size_t per = (n / nthreads + 63) & ~static_cast<size_t>(63);
-      const size_t a = std::min(n, per * index), b = index == nthreads - 1 ? n : std::min(n, per * (index + 1));
-      if (b > a) memcpy(d + a, s_ + a, b - a);
-      {
-        std::lock_guard<std::mutex> g(mu_);
-        if (--pending_ == 0) done_.notify_all();
-      }
-    }
-  }
-  std::vector<std::thread> workers_;
-  std::mutex mu_;
-  std::condition_variable cv_, done_;
-  char* dst_ = nullptr; const char* src_ = nullptr; size_t bytes_ = 0;
-  int pending_ = 0;
-  unsigned long long generation_ = 0;
-  bool stop_ = false;
-};
-
-constexpr size_t kStageChunk = 16u << 20;      // bytes per pinned staging buffer
-constexpr size_t kStageMinBytes = 4u << 20;    // smaller arrays go the driver's way
-constexpr int kStageBuffers = 2;
+// Ring of pinned buffers that host arrays travel through (staging.h): chunks of at most a slot, so
+// that the copy of one chunk runs beside the transfer of the one before.
+constexpr size_t kRingSlotBytes = 2u << 20;    // 2 MB: 27 us to copy with 8 threads, 41 us on the link
+constexpr int kRingSlots = 16;
+constexpr size_t kSmallInput = 64u << 10;      // inputs up to this size share one slot and one transfer
 
 struct b200conv_ctx {
   int device = 0;
@@ -112,8 +56,9 @@ struct b200conv_ctx {
   cudaStream_t stream = nullptr;
   std::mutex mu;
   std::string err;
-  int* d_status = nullptr;
-  int* h_status = nullptr;  // pinned
+  int* d_status = nullptr;  // status word of the kernels: h_status as the device sees it
+  volatile int* h_status = nullptr;  // pinned and mapped: written by kernels only when they give up, so that
+                                     // a synchronising call reads it without a transfer
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t ev_tune0 = nullptr, ev_tune1 = nullptr;   // kernel selection timing
   long long launches = 0;
@@ -156,11 +101,13 @@ struct b200conv_ctx {
   long long graph_launch_count = 0;
   long long wait_clocks = 4000000000LL;     // bound of device-side waits (about two seconds)
   int comm_timeout_ms = 60000;              // host watchdog of streams that carry collectives
-  // pinned staging of the host-pointer calls (made on first use)
-  void* stage_buf[kStageBuffers] = {nullptr, nullptr};
-  cudaEvent_t stage_ev[kStageBuffers] = {nullptr, nullptr};
-  bool stage_busy[kStageBuffers] = {false, false};
+  // pinned ring of the host-pointer calls (made on first use); every such call ends with all slots free
+  char* ring = nullptr;
+  cudaEvent_t ring_ev[kRingSlots] = {};
+  bool ring_busy[kRingSlots] = {};
+  int ring_next = 0;
   CopyPool* copy_pool = nullptr;
+  std::vector<cudaEvent_t> chunk_ev;        // order a batch's chunks across the upload, compute and download streams
   // packed filters made ahead of time (b200conv_prepack): key -> device buffer and validity
   struct Packed { void* ptr; size_t bytes; bool valid; const void* src; };
   std::map<std::string, Packed> packed;
@@ -300,7 +247,6 @@ int check_status(b200conv_ctx* c) {
   const int st = *c->h_status;
   if (st != kStatusOk) {
     *c->h_status = 0;
-    cudaMemsetAsync(c->d_status, 0, sizeof(int), c->stream);
     if (st == kStatusBadIndex)
       return fail(c, B200CONV_E_CUDA, "a kernel of the range-checked build computed an index outside its buffer "
                   "(the access was skipped); results are invalid");
@@ -363,7 +309,6 @@ int sync_and_check(b200conv_ctx* c) {
   if (c->capturing) return fail(c, B200CONV_E_INVALID, "not allowed while a graph is being captured");
   int rcj = join_comm(c);
   if (rcj) return rcj;
-  CU_OK(c, cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   if ((rcj = wait_stream(c))) return rcj;
   if (c->down_pending) {            // background downloads end after the work they waited for
     CU_OK(c, cudaStreamSynchronize(c->down_stream));
@@ -1875,11 +1820,13 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
 }
 
 // ---- host-pointer wrappers: copy in, run, copy out, synchronise ---------------------------
-int stage_setup(b200conv_ctx* c) {
+int ring_setup(b200conv_ctx* c) {
   if (c->copy_pool) return 0;
-  for (int i = 0; i < kStageBuffers; ++i) {
-    cudaError_t e = cudaHostAlloc(&c->stage_buf[i], kStageChunk, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->stage_ev[i], cudaEventDisableTiming);
+  if (!c->ring) {
+    void* p = nullptr;
+    cudaError_t e = cudaHostAlloc(&p, kRingSlotBytes * kRingSlots, cudaHostAllocDefault);
+    c->ring = static_cast<char*>(p);
+    for (int i = 0; i < kRingSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&c->ring_ev[i], cudaEventDisableTiming);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(c, B200CONV_E_NOMEM, "pinned staging buffers: %s", cudaGetErrorString(e));
@@ -1887,73 +1834,225 @@ int stage_setup(b200conv_ctx* c) {
   }
   const char* env = getenv("B200CONV_COPY_THREADS");
   const int cores = (int)std::thread::hardware_concurrency();
-  int n = env ? atoi(env) : std::min(8, std::max(2, cores / 2));   // 1.51 s -> 1.36 s per ResNet-50 step from 4 to 8 threads
-  n = std::max(1, std::min(n, 16));
-  c->copy_pool = new CopyPool(n);
+  // 16 MB into pinned memory: 1069 / 615 / 331 / 218 / 237 us with 1 / 2 / 4 / 8 / 12 threads (link: 310 us)
+  int n = env ? atoi(env) : std::min(8, std::max(2, cores / 2));
+  c->copy_pool = new CopyPool(std::max(1, std::min(n, 16)));
   return 0;
 }
 
-// Host array -> device memory through the pinned buffers: while the DMA engine moves chunk i, the
-// copy threads fill the other buffer with chunk i + 1.
-int stage_upload(b200conv_ctx* c, void* d, const void* h, size_t bytes) {
-  int rc = stage_setup(c);
+// A free slot of the ring (waits for the transfer that used it last).
+int ring_slot(b200conv_ctx* c, int* k) {
+  *k = c->ring_next;
+  c->ring_next = (c->ring_next + 1) % kRingSlots;
+  if (c->ring_busy[*k]) CU_OK(c, cudaEventSynchronize(c->ring_ev[*k]));
+  c->ring_busy[*k] = false;
+  return 0;
+}
+int ring_used(b200conv_ctx* c, int k, cudaStream_t s) {
+  CU_OK(c, cudaEventRecord(c->ring_ev[k], s));
+  c->ring_busy[k] = true;
+  return 0;
+}
+
+// The next chunk of an array of which `off` of `bytes` have gone: small ones first, so that the link
+// starts early, doubling up to a slot (the calls per chunk cost about 4 us).
+size_t chunk_bytes(size_t off, size_t bytes) {
+  return std::min(bytes - off, std::min(kRingSlotBytes, std::max<size_t>(256u << 10, off)));
+}
+
+bool is_pinned(const void* h, size_t bytes) {
+  cudaPointerAttributes a, b;
+  if (cudaPointerGetAttributes(&a, h) != cudaSuccess ||
+      cudaPointerGetAttributes(&b, static_cast<const char*>(h) + bytes - 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeHost && b.type == cudaMemoryTypeHost;
+}
+
+// Host array -> device memory on stream s.  The array may be reused when this returns unless it is pinned.
+int upload(b200conv_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s, bool pinned) {
+  if (pinned) {
+    CU_OK(c, cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
+    return 0;
+  }
+  int rc = ring_setup(c);
   if (rc) return rc;
-  int k = 0;
-  for (size_t off = 0; off < bytes; off += kStageChunk, k ^= 1) {
-    const size_t n = std::min(kStageChunk, bytes - off);
-    if (c->stage_busy[k]) CU_OK(c, cudaEventSynchronize(c->stage_ev[k]));      // its previous transfer has left
-    c->copy_pool->copy(c->stage_buf[k], static_cast<const char*>(h) + off, n);
-    CU_OK(c, cudaMemcpyAsync(static_cast<char*>(d) + off, c->stage_buf[k], n, cudaMemcpyHostToDevice, c->stream));
-    CU_OK(c, cudaEventRecord(c->stage_ev[k], c->stream));
-    c->stage_busy[k] = true;
+  for (size_t off = 0, n; off < bytes; off += n) {
+    n = chunk_bytes(off, bytes);
+    int k;
+    if ((rc = ring_slot(c, &k))) return rc;
+    char* slot = c->ring + kRingSlotBytes * k;
+    c->copy_pool->copy(slot, static_cast<const char*>(h) + off, n, true);
+    CU_OK(c, cudaMemcpyAsync(static_cast<char*>(d) + off, slot, n, cudaMemcpyHostToDevice, s));
+    if ((rc = ring_used(c, k, s))) return rc;
   }
   return 0;
 }
 
-// Device memory -> host array: chunk i + 1 travels into one buffer while the copy threads empty the
-// other into the array.  Returns with everything in place (it waits for the stream).
-int stage_download(b200conv_ctx* c, void* h, const void* d, size_t bytes) {
-  int rc = stage_setup(c);
+// Device memory -> host array on stream s.  A pinned array is complete when the stream is; a pageable
+// one when this returns: chunks travel into ring slots, up to half a ring ahead of the copy threads
+// that empty them.
+int download(b200conv_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s, bool pinned) {
+  if (pinned) {
+    CU_OK(c, cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
+    return 0;
+  }
+  int rc = ring_setup(c);
   if (rc) return rc;
-  for (int k = 0; k < kStageBuffers; ++k)
-    if (c->stage_busy[k]) { CU_OK(c, cudaEventSynchronize(c->stage_ev[k])); c->stage_busy[k] = false; }
-  size_t prev_off = 0, prev_n = 0;
-  int k = 0;
-  for (size_t off = 0; off < bytes; off += kStageChunk, k ^= 1) {
-    const size_t n = std::min(kStageChunk, bytes - off);
-    CU_OK(c, cudaMemcpyAsync(c->stage_buf[k], static_cast<const char*>(d) + off, n, cudaMemcpyDeviceToHost, c->stream));
-    CU_OK(c, cudaEventRecord(c->stage_ev[k], c->stream));
-    if (prev_n) {
-      CU_OK(c, cudaEventSynchronize(c->stage_ev[k ^ 1]));
-      c->copy_pool->copy(static_cast<char*>(h) + prev_off, c->stage_buf[k ^ 1], prev_n);
+  constexpr int kAhead = kRingSlots / 2;
+  struct { int slot; size_t off, n; } flying[kAhead];
+  size_t off = 0;
+  int issued = 0;
+  for (int taken = 0; off < bytes || taken < issued; ++taken) {
+    for (; off < bytes && issued - taken < kAhead; ++issued) {
+      auto& f = flying[issued % kAhead];
+      f.off = off;
+      f.n = chunk_bytes(off, bytes);
+      if ((rc = ring_slot(c, &f.slot))) return rc;
+      CU_OK(c, cudaMemcpyAsync(c->ring + kRingSlotBytes * f.slot, static_cast<const char*>(d) + off, f.n, cudaMemcpyDeviceToHost, s));
+      if ((rc = ring_used(c, f.slot, s))) return rc;
+      off += f.n;
     }
-    prev_off = off; prev_n = n;
-  }
-  if (prev_n) {
-    CU_OK(c, cudaEventSynchronize(c->stage_ev[k ^ 1]));
-    c->copy_pool->copy(static_cast<char*>(h) + prev_off, c->stage_buf[k ^ 1], prev_n);
+    const auto& f = flying[taken % kAhead];
+    CU_OK(c, cudaEventSynchronize(c->ring_ev[f.slot]));
+    c->ring_busy[f.slot] = false;
+    c->copy_pool->copy(static_cast<char*>(h) + f.off, c->ring + kRingSlotBytes * f.slot, f.n, false);
   }
   return 0;
 }
 
+int copy_streams(b200conv_ctx* c) {
+  if (!c->up_stream) {
+    CU_OK(c, cudaStreamCreateWithFlags(&c->up_stream, cudaStreamNonBlocking));
+    CU_OK(c, cudaStreamCreateWithFlags(&c->down_stream, cudaStreamNonBlocking));
+    CU_OK(c, cudaEventCreateWithFlags(&c->ev_up, cudaEventDisableTiming));
+    CU_OK(c, cudaEventCreateWithFlags(&c->ev_down, cudaEventDisableTiming));
+  }
+  return 0;
+}
+
+int chunk_event(b200conv_ctx* c, size_t i, cudaEvent_t* e) {
+  while (c->chunk_ev.size() <= i) {
+    cudaEvent_t n;
+    CU_OK(c, cudaEventCreateWithFlags(&n, cudaEventDisableTiming));
+    c->chunk_ev.push_back(n);
+  }
+  *e = c->chunk_ev[i];
+  return 0;
+}
+
+// The tensors of one host-pointer call.
 struct HostIO {
   b200conv_ctx* c;
   Scratch tmp;
+  char *group_dev = nullptr, *group_host = nullptr;   // small inputs side by side: one transfer for all
+  size_t group_used = 0;
+  int group_slot = -1;
   explicit HostIO(b200conv_ctx* ctx) : c(ctx), tmp(ctx) {}
-  int in(const void* h, size_t bytes, void** d) {
-    int rc = tmp.get(bytes, d);
-    if (rc) return rc;
-    if (bytes >= kStageMinBytes) return stage_upload(c, *d, h, bytes);
-    if (bytes) CU_OK(c, cudaMemcpyAsync(*d, h, bytes, cudaMemcpyHostToDevice, c->stream));
-    return 0;
-  }
   int out(size_t bytes, void** d) { return tmp.get(bytes, d); }
+  // A small input joins the group (start() sends it), a larger one is on its way when this returns.
+  int in(const void* h, size_t bytes, void** d) {
+    int rc;
+    if (bytes <= kSmallInput) {
+      if ((rc = small_space(bytes, d))) return rc;
+      memcpy(group_host + (static_cast<char*>(*d) - group_dev), h, bytes);
+      return 0;
+    }
+    if ((rc = tmp.get(bytes, d))) return rc;
+    return upload(c, *d, h, bytes, c->stream, is_pinned(h, bytes));
+  }
+  int start() {
+    if (!group_used) return 0;
+    CU_OK(c, cudaMemcpyAsync(group_dev, group_host, group_used, cudaMemcpyHostToDevice, c->stream));
+    return ring_used(c, group_slot, c->stream);
+  }
   int back(void* h, const void* d, size_t bytes) {
-    if (bytes >= kStageMinBytes) return stage_download(c, h, d, bytes);
-    if (bytes) CU_OK(c, cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, c->stream));
+    return bytes ? download(c, h, d, bytes, c->stream, is_pinned(h, bytes)) : 0;
+  }
+
+ private:
+  int small_space(size_t bytes, void** d) {
+    int rc;
+    if (!group_dev) {
+      if ((rc = ring_setup(c)) || (rc = ring_slot(c, &group_slot))) return rc;
+      void* p;
+      if ((rc = tmp.get(4 * (kSmallInput + 256), &p))) return rc;      // at most four inputs per call
+      group_dev = static_cast<char*>(p);
+      group_host = c->ring + kRingSlotBytes * group_slot;
+    }
+    *d = group_dev + group_used;
+    group_used += (bytes + 255) & ~static_cast<size_t>(255);
     return 0;
   }
 };
+
+// Forward and gradInputs compute every image by itself, so a large batch goes through in chunks of
+// images: the upload of one chunk, the kernels of the one before and the download of the one before
+// that run side by side (the link carries both directions at once).
+struct BatchPlan {
+  int chunks, images;      // chunks of `images` images, the last one possibly smaller
+};
+BatchPlan plan_batch(int N, size_t in_bytes, size_t out_bytes) {
+  // chunks of about 4 MB of the larger side (75 us on the link, against 20 to 40 us of launches and
+  // transfers' latencies per chunk), at most 8; equal ones where a count near that divides the batch
+  // (another batch size is another geometry to choose kernels for)
+  const size_t big = std::max(in_bytes, out_bytes);
+  const int n = (int)std::min<size_t>(std::min<size_t>(8, N), big / (4u << 20));
+  if (n <= 1 || std::min(in_bytes, out_bytes) < (1u << 20)) return {1, N};
+  for (int m = n; m > n / 2 && m > 1; --m)
+    if (N % m == 0) return {m, N / m};
+  const int per = (int)cdiv(N, n);
+  return {(int)cdiv(N, per), per};
+}
+
+// Runs `compute(images, device input, device output)` over the batch.
+template <class Compute>
+int run_batch(b200conv_ctx* c, HostIO& io, int N, const void* hin, size_t in_bytes, void* hout, size_t out_bytes,
+              Compute compute) {
+  int rc;
+  void *din, *dout;
+  const BatchPlan bp = plan_batch(N, in_bytes, out_bytes);
+  if (bp.chunks == 1) {
+    if ((rc = io.in(hin, in_bytes, &din)) || (rc = io.out(out_bytes, &dout)) || (rc = io.start())) return rc;
+    if ((rc = compute(N, din, dout))) return rc;
+    return io.back(hout, dout, out_bytes);
+  }
+  if ((rc = io.start()) || (rc = copy_streams(c)) || (rc = io.out(in_bytes, &din)) || (rc = io.out(out_bytes, &dout))) return rc;
+  const bool pin_in = is_pinned(hin, in_bytes), pin_out = is_pinned(hout, out_bytes);
+  const size_t in1 = in_bytes / N, out1 = out_bytes / N;
+  // the buffers come from the pool of the main stream: what still uses them there goes first
+  CU_OK(c, cudaEventRecord(c->ev_up, c->stream));
+  CU_OK(c, cudaStreamWaitEvent(c->up_stream, c->ev_up, 0));
+  // An error leaves the loop with transfers in flight: they are waited for before the buffers go back.
+  auto step = [&](int i) -> int {
+    const int a = i * bp.images, b = std::min(N, a + bp.images);
+    cudaEvent_t up, done;
+    int r;
+    if ((r = chunk_event(c, 2 * i, &up)) || (r = chunk_event(c, 2 * i + 1, &done))) return r;
+    if ((r = upload(c, static_cast<char*>(din) + in1 * a, static_cast<const char*>(hin) + in1 * a, in1 * (b - a), c->up_stream, pin_in))) return r;
+    CU_OK(c, cudaEventRecord(up, c->up_stream));
+    CU_OK(c, cudaStreamWaitEvent(c->stream, up, 0));
+    if ((r = compute(b - a, static_cast<char*>(din) + in1 * a, static_cast<char*>(dout) + out1 * a))) return r;
+    CU_OK(c, cudaEventRecord(done, c->stream));
+    CU_OK(c, cudaStreamWaitEvent(c->down_stream, done, 0));
+    return 0;
+  };
+  auto fetch = [&](int i) -> int {
+    const int a = i * bp.images, b = std::min(N, a + bp.images);
+    return download(c, static_cast<char*>(hout) + out1 * a, static_cast<const char*>(dout) + out1 * a, out1 * (b - a), c->down_stream, pin_out);
+  };
+  // a pageable result is copied out by the host, one chunk behind, so that it does not hold up the uploads
+  for (int i = 0; i < bp.chunks && !rc; ++i) {
+    rc = step(i);
+    if (!rc && pin_out) rc = fetch(i);
+    if (!rc && !pin_out && i > 0) rc = fetch(i - 1);
+  }
+  if (!rc && !pin_out) rc = fetch(bp.chunks - 1);
+  cudaStreamSynchronize(c->up_stream);
+  cudaStreamSynchronize(c->down_stream);
+  return rc;
+}
 
 }  // namespace
 
@@ -1998,12 +2097,13 @@ int b200conv_create(int device, b200conv_ctx** out) {
   b200conv_ctx* c = new b200conv_ctx();
   c->device = device;
   c->num_sms = c->device_sms = prop.multiProcessorCount;
+  void* hs = nullptr;
   bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
-            cudaMalloc(&c->d_status, sizeof(int)) == cudaSuccess &&
-            cudaMemset(c->d_status, 0, sizeof(int)) == cudaSuccess &&
-            cudaHostAlloc(&c->h_status, sizeof(int), cudaHostAllocDefault) == cudaSuccess &&
+            cudaHostAlloc(&hs, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
+            cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->d_status), hs, 0) == cudaSuccess &&
             cudaEventCreate(&c->ev0) == cudaSuccess && cudaEventCreate(&c->ev1) == cudaSuccess;
   if (ok) {
+    c->h_status = static_cast<volatile int*>(hs);
     *c->h_status = 0;
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult qr;
@@ -2041,12 +2141,11 @@ void b200conv_destroy(b200conv_ctx* c) {
     cudaEventDestroy(c->ev_comm_done);
   }
   delete c->copy_pool;
-  for (int i = 0; i < kStageBuffers; ++i) {
-    if (c->stage_buf[i]) cudaFreeHost(c->stage_buf[i]);
-    if (c->stage_ev[i]) cudaEventDestroy(c->stage_ev[i]);
-  }
-  cudaFree(c->d_status);
-  cudaFreeHost(c->h_status);
+  if (c->ring) cudaFreeHost(c->ring);
+  for (cudaEvent_t e : c->ring_ev)
+    if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : c->chunk_ev) cudaEventDestroy(e);
+  cudaFreeHost(const_cast<int*>(c->h_status));
   for (auto& r : c->prof_recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   for (auto& e : c->prof_pool) cudaEventDestroy(e);
   cudaEventDestroy(c->ev0);
@@ -2096,16 +2195,20 @@ static int fwd_call(b200conv_ctx* c, const b200conv_desc* d, const void* x, cons
   const size_t nx = es * (size_t)d->N * d->C * d->H * d->W, nw = es * (size_t)d->K * (d->C / d->groups) * d->kH * d->kW,
                ny = es * (size_t)d->N * d->K * d->Ho * d->Wo;
   HostIO io(c);
-  void *dx_, *dw_, *db_ = nullptr, *dr_ = nullptr, *dy_;
-  if ((rc = io.in(x, nx, &dx_)) || (rc = io.in(w, nw, &dw_)) || (rc = io.out(ny, &dy_))) return rc;
+  void *dw_, *db_ = nullptr, *dr_ = nullptr;
+  if ((rc = io.in(w, nw, &dw_))) return rc;
   if (bias && (rc = io.in(bias, es * d->K, &db_))) return rc;
   if (residual && (rc = io.in(residual, ny, &dr_))) return rc;
-  epi.residual = dr_;
-  {
+  const char* res = static_cast<const char*>(dr_);
+  rc = run_batch(c, io, d->N, x, nx, y, ny, [&](int images, const void* xin, void* yout) {
+    b200conv_desc part = *d;
+    part.N = images;
+    epi.residual = res;
+    if (res) res += ny / d->N * images;
     EpilogueScope scope(c, epi);
-    if ((rc = fwd_device(c, *d, dx_, dw_, db_, dy_, flags & ~B200CONV_HOST_PTRS))) return rc;
-  }
-  if ((rc = io.back(y, dy_, ny))) return rc;
+    return fwd_device(c, part, xin, dw_, db_, yout, flags & ~B200CONV_HOST_PTRS);
+  });
+  if (rc) return rc;
   return sync_and_check(c);
 }
 
@@ -2140,10 +2243,14 @@ int b200conv_dgrad(b200conv_ctx* c, const b200conv_desc* d, const void* w, const
   const size_t nx = es * (size_t)d->N * d->C * d->H * d->W, nw = es * (size_t)d->K * (d->C / d->groups) * d->kH * d->kW,
                ny = es * (size_t)d->N * d->K * d->Ho * d->Wo;
   HostIO io(c);
-  void *dw_, *dy_, *dx_;
-  if ((rc = io.in(w, nw, &dw_)) || (rc = io.in(dy, ny, &dy_)) || (rc = io.out(nx, &dx_))) return rc;
-  if ((rc = dgrad_device(c, *d, dw_, dy_, dx_, flags & ~B200CONV_HOST_PTRS))) return rc;
-  if ((rc = io.back(dx, dx_, nx))) return rc;
+  void* dw_;
+  if ((rc = io.in(w, nw, &dw_))) return rc;
+  rc = run_batch(c, io, d->N, dy, ny, dx, nx, [&](int images, const void* dyin, void* dxout) {
+    b200conv_desc part = *d;
+    part.N = images;
+    return dgrad_device(c, part, dw_, dyin, dxout, flags & ~B200CONV_HOST_PTRS);
+  });
+  if (rc) return rc;
   return sync_and_check(c);
 }
 
@@ -2164,7 +2271,7 @@ int b200conv_wgrad(b200conv_ctx* c, const b200conv_desc* d, const void* x, const
   HostIO io(c);
   void *dx_, *dy_, *dw_;
   const size_t nw_out = (flags & B200CONV_DW_F32) ? nw / es * sizeof(float) : nw;
-  if ((rc = io.in(x, nx, &dx_)) || (rc = io.in(dy, ny, &dy_)) || (rc = io.out(nw_out, &dw_))) return rc;
+  if ((rc = io.in(x, nx, &dx_)) || (rc = io.in(dy, ny, &dy_)) || (rc = io.out(nw_out, &dw_)) || (rc = io.start())) return rc;
   if ((rc = wgrad_device(c, *d, dx_, dy_, dw_, flags & ~B200CONV_HOST_PTRS))) return rc;
   if ((rc = io.back(dw, dw_, nw_out))) return rc;
   return sync_and_check(c);
@@ -2187,7 +2294,7 @@ int b200conv_maxpool2x2(b200conv_ctx* c, const void* x, void* y, int N, int C, i
   void *dx_, *dy_;
   int rc;
   const size_t nx = es * (size_t)N * C * H * W, ny = es * (size_t)N * C * (H / 2) * (W / 2);
-  if ((rc = io.in(x, nx, &dx_)) || (rc = io.out(ny, &dy_))) return rc;
+  if ((rc = io.in(x, nx, &dx_)) || (rc = io.out(ny, &dy_)) || (rc = io.start())) return rc;
   KLAUNCH(c, kKPool, launch_maxpool2x2(dx_, dy_, N, C, H, W, 0, Cp, dtype, c->stream));
   if ((rc = io.back(y, dy_, ny))) return rc;
   return sync_and_check(c);
@@ -2211,7 +2318,7 @@ int b200conv_maxpool2x2_grad(b200conv_ctx* c, const void* x, const void* y, cons
   int rc;
   const size_t nx = es * (size_t)N * C * H * W, ny = es * (size_t)N * C * (H / 2) * (W / 2);
   if ((rc = io.in(x, nx, &dx_)) || (rc = io.in(y, ny, &dy_)) || (rc = io.in(gy, ny, &dgy_)) ||
-      (rc = io.out(nx, &dgx_)))
+      (rc = io.out(nx, &dgx_)) || (rc = io.start()))
     return rc;
   KLAUNCH(c, kKPool, launch_maxpool2x2_grad(dx_, dy_, dgy_, dgx_, N, C, H, W, 0, Cp, dtype, c->stream));
   if ((rc = io.back(gx, dgx_, nx))) return rc;
@@ -2285,7 +2392,7 @@ int b200conv_host_alloc(b200conv_ctx* c, size_t bytes, void** hptr) {
   return 0;
 }
 int b200conv_host_free(b200conv_ctx* c, void* hptr) {
-  if (!c) return B200CONV_E_INVALID;
+  if (!c) return cudaFreeHost(hptr) == cudaSuccess ? 0 : B200CONV_E_CUDA;
   std::lock_guard<std::mutex> g(c->mu);
   DeviceGuard dg(c->device);
   CU_OK(c, cudaFreeHost(hptr));
@@ -2312,16 +2419,6 @@ int b200conv_memset(b200conv_ctx* c, void* dst, int value, size_t bytes) {
   if (bytes) CU_OK(c, cudaMemsetAsync(dst, value, bytes, c->stream));
   return 0;
 }
-static int copy_streams(b200conv_ctx* c) {
-  if (!c->up_stream) {
-    CU_OK(c, cudaStreamCreateWithFlags(&c->up_stream, cudaStreamNonBlocking));
-    CU_OK(c, cudaStreamCreateWithFlags(&c->down_stream, cudaStreamNonBlocking));
-    CU_OK(c, cudaEventCreateWithFlags(&c->ev_up, cudaEventDisableTiming));
-    CU_OK(c, cudaEventCreateWithFlags(&c->ev_down, cudaEventDisableTiming));
-  }
-  return 0;
-}
-
 int b200conv_memcpy_h2d_bg(b200conv_ctx* c, void* dst, const void* src, size_t bytes) {
   if (!c) return B200CONV_E_INVALID;
   std::lock_guard<std::mutex> g(c->mu);

@@ -124,7 +124,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == kFilterProducer) {
     // Filter producer: the same walk over tiles, channel blocks and taps, filter tiles only.
     const bool leader = elect_one();
@@ -149,7 +149,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == 1 || warp == kSecondIssuer) {
     // this issuer's accumulators of every tile: [a_begin, a_end)
     const int a_split = issuers == 2 ? (p.n_acc + 1) / 2 : p.n_acc;
@@ -217,7 +217,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         if (ok && leader) umma_commit(&bars->acc_full[buf]);
         if (trace && it == 0) trace[3] = clock64();
       }
-      if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+      if (!ok && leader) report_status(p.status, kStatusTimeout);
       if (trace) {
         trace[9] = tw_acc; trace[10] = tw_slab; trace[11] = tw_b;
         trace[12] = clock64() - t_loop0; trace[13] = it;
@@ -479,7 +479,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       for (int q = 0; q < 4; ++q) trace[16 + q] = tp[q];
     }
     if (p.tma_out && lane == 0) bulk_wait<0>();  // this thread's stores (if it issued any) have left shared memory
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
 
   tc_fence_before();

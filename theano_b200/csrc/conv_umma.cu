@@ -145,7 +145,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == 1) {
     const bool leader = elect_one();
     int stage = 0;
@@ -178,7 +178,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       }
       if (ok && leader) umma_commit(&bars->acc_full[buf]);
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else {
     // Epilogue, 16 warps: warp w reads TMEM lanes [32*(w%4), +32) (the hardware's rule) and, of
     // those rows, every fourth 32-column chunk.  One warp keeps only a few stores in flight, so
@@ -259,7 +259,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       tc_fence_before();
       mbar_arrive(&bars->acc_empty[buf]);
     }
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
 
   tc_fence_before();

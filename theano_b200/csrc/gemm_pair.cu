@@ -97,7 +97,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == 1) {
     if (rank == 0) {
       const bool leader = elect_one();
@@ -128,7 +128,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
         }
         if (ok && leader) umma_commit_pair(&bars->acc_full[buf]);
       }
-      if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+      if (!ok && leader) report_status(p.status, kStatusTimeout);
     }
   } else if (warp < 2 + kEpilogueWarps) {
     // Epilogue: warp w reads TMEM lanes [32 * (w % 4), +32) of this CTA's 128 accumulator rows; the four
@@ -199,7 +199,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
       named_barrier(5, 32 * kEpilogueWarps);
       if (warp == 2 && lane == 0) mbar_arrive_leader(&bars->acc_empty[buf]);
     }
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
     if (lane == 0) bulk_wait<0>();           // this thread's stores (if it issued any) have left shared memory
   }
 

@@ -15,7 +15,7 @@ namespace b200 {
 // fails the call).  The stand-in for a memory checker on machines where none may run.  In the
 // normal build the macro is the constant true and costs nothing.
 #ifdef B200CONV_DEBUG
-#define B200_IN_RANGE(cond, status) ((cond) ? true : (atomicExch((status), 2 /* kStatusBadIndex */), false))
+#define B200_IN_RANGE(cond, status) ((cond) ? true : (b200::report_status((status), 2 /* kStatusBadIndex */), false))
 #else
 #define B200_IN_RANGE(cond, status) (true)
 #endif
@@ -44,6 +44,12 @@ __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
+}
+
+// The status word lives in mapped host memory: a plain system-scope store that the host reads after
+// it has waited for the stream.
+__device__ __forceinline__ void report_status(int* status, int code) {
+  asm volatile("st.relaxed.sys.global.s32 [%0], %1;" ::"l"(status), "r"(code) : "memory");
 }
 
 // ---- mbarrier -----------------------------------------------------------------------

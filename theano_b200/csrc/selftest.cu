@@ -24,10 +24,10 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int* status, long 
   bool ok;
   if (warp == 0) {
     ok = uniform_wait(&bars.never, 0, &bars, limit);                               // the issuers' wait
-    if (!ok && elect_one()) atomicExch(status, kStatusTimeout);
+    if (!ok && elect_one()) report_status(status, kStatusTimeout);
   } else {
     ok = warp_wait_or_abort(&bars.never, 0, &bars, threadIdx.x & 31, limit);       // the epilogue warps' wait
-    if (!ok && (threadIdx.x & 31) == 0) atomicExch(status, kStatusTimeout);
+    if (!ok && (threadIdx.x & 31) == 0) report_status(status, kStatusTimeout);
   }
   __syncthreads();
   if (bars.abort) abort_grace(limit);

@@ -1,0 +1,172 @@
+// Host side of the host-pointer calls: copies between pageable arrays and pinned buffers.
+//
+// What bounds a host-pointer call is the PCIe link (54 GB/s measured each way) and what feeds it.
+// Two measured facts decide the shape of this code (B200 box, 16 cores):
+//  * A DMA transfer that finds its lines in the caches of several cores crawls: 4 MB that eight
+//    threads had just memcpy'd into the pinned buffer went to the device in 450-700 us instead of
+//    82, and 4 MB coming back into lines that eight threads had read the last time took 320-450.
+//    So the copy INTO a pinned buffer uses streaming stores (the lines end up in memory, the
+//    transfer runs at 83 us per 4 MB), and the copy OUT of one evicts the lines it has read.
+//  * Waking a sleeping thread costs tens of microseconds, as much as copying a megabyte.  The
+//    calling thread starts on the first piece at once, the workers spin for a moment after a job
+//    before they sleep, and pieces are handed out one by one so that nobody waits for a late one.
+#pragma once
+#include <immintrin.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace b200 {
+
+// memcpy with streaming stores; dst 32-byte aligned.
+__attribute__((target("avx2"))) inline void copy_streaming_avx2(char* d, const char* s, size_t n) {
+  size_t i = 0;
+  for (; i + 128 <= n; i += 128) {
+    const __m256i a = _mm256_loadu_si256(reinterpret_cast<const __m256i*>(s + i));
+    const __m256i b = _mm256_loadu_si256(reinterpret_cast<const __m256i*>(s + i + 32));
+    const __m256i c = _mm256_loadu_si256(reinterpret_cast<const __m256i*>(s + i + 64));
+    const __m256i e = _mm256_loadu_si256(reinterpret_cast<const __m256i*>(s + i + 96));
+    _mm256_stream_si256(reinterpret_cast<__m256i*>(d + i), a);
+    _mm256_stream_si256(reinterpret_cast<__m256i*>(d + i + 32), b);
+    _mm256_stream_si256(reinterpret_cast<__m256i*>(d + i + 64), c);
+    _mm256_stream_si256(reinterpret_cast<__m256i*>(d + i + 96), e);
+  }
+  if (i < n) memcpy(d + i, s + i, n - i);
+  _mm_sfence();
+}
+
+// memcpy that leaves the source's lines in no cache; in blocks, so that the eviction finds them
+// in the first level.
+__attribute__((target("clflushopt"))) inline void copy_and_evict_clflushopt(char* d, const char* s, size_t n) {
+  constexpr size_t kBlock = 16384;
+  for (size_t off = 0; off < n; off += kBlock) {
+    const size_t m = n - off < kBlock ? n - off : kBlock;
+    memcpy(d + off, s + off, m);
+    for (size_t i = 0; i < m; i += 64) _mm_clflushopt(const_cast<char*>(s + off + i));
+  }
+  _mm_sfence();
+}
+
+inline bool cpu_has_clflushopt() {
+  unsigned a = 7, b = 0, c = 0, d = 0;
+  __asm__ volatile("cpuid" : "+a"(a), "=b"(b), "+c"(c), "=d"(d));
+  return (b >> 23) & 1;
+}
+
+inline void copy_to_pinned(char* d, const char* s, size_t n) {
+  static const bool avx2 = __builtin_cpu_supports("avx2");
+  if (avx2) copy_streaming_avx2(d, s, n);
+  else memcpy(d, s, n);
+}
+inline void copy_from_pinned(char* d, const char* s, size_t n) {
+  static const bool flush = cpu_has_clflushopt();
+  if (flush) copy_and_evict_clflushopt(d, s, n);
+  else memcpy(d, s, n);
+}
+
+// A few threads that copy one array together with the caller.  One producer at a time (the
+// context's lock).
+class CopyPool {
+ public:
+  explicit CopyPool(int nthreads) {
+    for (int i = 1; i < nthreads; ++i) workers_.emplace_back([this] { loop(); });
+  }
+  ~CopyPool() {
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      stop_.store(true);
+    }
+    cv_.notify_all();
+    for (auto& t : workers_) t.join();
+  }
+  // Copies `bytes` (to_pinned: into a pinned buffer, else out of one) and returns when done.
+  void copy(void* dst, const void* src, size_t bytes, bool to_pinned) {
+    // 128 KB pieces: four pages' worth of work per hand-out and 16 pieces in a 2 MB chunk
+    constexpr size_t kPiece = 128 << 10;
+    const uint32_t pieces = static_cast<uint32_t>((bytes + kPiece - 1) / kPiece);
+    const uint64_t gen = (ticket_.load(std::memory_order_relaxed) >> 32) + 1;
+    // nobody takes a piece while the job is being described: a worker takes one by exchanging the
+    // ticket it has read, so what it read in between belongs to that ticket's job
+    ticket_.store(gen << 32 | 0xffffffffu, std::memory_order_seq_cst);
+    dst_.store(static_cast<char*>(dst), std::memory_order_relaxed);
+    src_.store(static_cast<const char*>(src), std::memory_order_relaxed);
+    bytes_.store(bytes, std::memory_order_relaxed);
+    pieces_.store(pieces, std::memory_order_relaxed);
+    to_pinned_.store(to_pinned, std::memory_order_relaxed);
+    done_.store(0, std::memory_order_relaxed);
+    ticket_.store(gen << 32, std::memory_order_seq_cst);
+    if (pieces > 1 && sleeping_.load(std::memory_order_seq_cst) > 0) {
+      { std::lock_guard<std::mutex> g(mu_); }
+      cv_.notify_all();
+    }
+    work(gen);
+    while (done_.load(std::memory_order_acquire) != pieces) _mm_pause();
+  }
+
+ private:
+  void work(uint64_t gen) {
+    constexpr size_t kPiece = 128 << 10;
+    for (;;) {
+      uint64_t t = ticket_.load(std::memory_order_acquire);
+      char* d = dst_.load(std::memory_order_relaxed);
+      const char* s = src_.load(std::memory_order_relaxed);
+      const size_t n = bytes_.load(std::memory_order_relaxed);
+      const uint32_t pieces = pieces_.load(std::memory_order_relaxed);
+      const bool in = to_pinned_.load(std::memory_order_relaxed);
+      const uint32_t i = static_cast<uint32_t>(t);
+      if (t >> 32 != gen || i >= pieces) return;
+      if (!ticket_.compare_exchange_strong(t, t + 1, std::memory_order_acq_rel)) continue;
+      const size_t off = static_cast<size_t>(i) * kPiece, m = n - off < kPiece ? n - off : kPiece;
+      if (in) copy_to_pinned(d + off, s + off, m);
+      else copy_from_pinned(d + off, s + off, m);
+      done_.fetch_add(1, std::memory_order_release);
+    }
+  }
+  void loop() {
+    uint64_t seen = 0;
+    for (;;) {
+      // spin for about 50 us (the gap between the chunks of one call), then sleep
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(50);
+      bool fresh = false;
+      do {
+        for (int k = 0; k < 32 && !fresh; ++k) {
+          fresh = posted() != seen;
+          if (!fresh) _mm_pause();
+        }
+      } while (!fresh && !stop_.load(std::memory_order_relaxed) && std::chrono::steady_clock::now() < until);
+      if (!fresh) {
+        std::unique_lock<std::mutex> g(mu_);
+        sleeping_.fetch_add(1, std::memory_order_seq_cst);
+        cv_.wait(g, [&] { return stop_.load() || posted() != seen; });
+        sleeping_.fetch_sub(1, std::memory_order_seq_cst);
+      }
+      if (stop_.load()) return;
+      seen = posted();
+      work(seen);
+    }
+  }
+  // generation of the last job that is open for work
+  uint64_t posted() const {
+    const uint64_t t = ticket_.load(std::memory_order_seq_cst);
+    return static_cast<uint32_t>(t) == 0xffffffffu ? (t >> 32) - 1 : t >> 32;
+  }
+  std::vector<std::thread> workers_;
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::atomic<bool> stop_{false};
+  std::atomic<int> sleeping_{0};
+  std::atomic<uint64_t> ticket_{0};      // generation << 32 | next piece
+  std::atomic<char*> dst_{nullptr};
+  std::atomic<const char*> src_{nullptr};
+  std::atomic<size_t> bytes_{0};
+  std::atomic<uint32_t> pieces_{0}, done_{0};
+  std::atomic<bool> to_pinned_{true};
+};
+
+}  // namespace b200

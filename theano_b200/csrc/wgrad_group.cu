@@ -278,7 +278,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
     if (trace && leader && pw == 0) { trace[2] = t_wait; trace[3] = clock64() - t_begin; }
   } else if (warp == 1) {
     // all lanes follow the loop and wait; one elected lane issues the MMAs and their commits
@@ -319,7 +319,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
       }
       if (ok && leader) umma_commit(&bars->acc_full);
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
     if (trace && leader) { trace[0] = t_wait; trace[1] = clock64() - t_begin; }
   } else {
     const int quad = warp & 3;
@@ -370,7 +370,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
       tc_fence_before();
       mbar_arrive(&bars->acc_empty);
     }
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
 
   tc_fence_before();

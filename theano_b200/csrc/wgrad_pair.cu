@@ -143,7 +143,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == 1) {
     if (rank == 0) {
       const bool leader = elect_one();
@@ -176,7 +176,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
         }
         if (ok && leader) umma_commit_pair(&bars->acc_full[buf]);
       }
-      if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+      if (!ok && leader) report_status(p.status, kStatusTimeout);
     }
   } else {
     // Epilogue, 16 warps: warp w reads TMEM lanes [32 * (w % 4), +32) = 32 of this CTA's 128 filter rows and,
@@ -229,7 +229,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
       named_barrier(5, 32 * kEpilogueWarps);
       if (warp == 2 && lane == 0) mbar_arrive_leader(&bars->acc_empty[buf]);
     }
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
 
   tc_fence_before();

@@ -239,7 +239,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
     if (trace && leader && pw == 0) { trace[2] = t_wait; trace[3] = clock64() - t_begin; }
   } else if (warp == 1) {
     // all lanes follow the loop and wait; one elected lane issues the MMAs and their commits
@@ -268,7 +268,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
       else ok = mma_tiles<KIND, BN, 0, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
       if (ok && leader) umma_commit(&bars->acc_full[buf]);
     }
-    if (!ok && leader) atomicExch(p.status, kStatusTimeout);
+    if (!ok && leader) report_status(p.status, kStatusTimeout);
     if (trace && leader) { trace[0] = t_wait; trace[1] = clock64() - t_begin; }
   } else {
     // warp w reads TMEM lanes [32*(w%4), +32) and every fourth 32-column chunk of them
@@ -320,7 +320,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
       tc_fence_before();
       mbar_arrive(&bars->acc_empty[buf]);
     }
-    if (!ok && lane == 0) atomicExch(p.status, kStatusTimeout);
+    if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
 
   tc_fence_before();
