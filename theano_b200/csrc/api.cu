@@ -487,7 +487,7 @@ long long out_extent(const FwdLikeArgs& a, int Wt, int Ht, long long sn, long lo
 // error code.
 int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps, int rh,
                   int rw, int Wt, int Ht, void* out, long long sn, long long sc, long long sh,
-                  long long sw, long long off, const float* bias, int relu) {
+                  long long sw, long long off, const void* bias, int relu) {
   if (taps.empty() || (int)taps.size() > kMaxTaps) return 2;
   int dh_min = taps[0].dh, dh_max = taps[0].dh, dw_min = taps[0].dw, dw_max = taps[0].dw;
   for (const ConvTap& t : taps) {
@@ -745,7 +745,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
 int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps_in,
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
-                      const float* bias, int relu, bool allow_slab) {
+                      const void* bias, int relu, bool allow_slab) {
   if (allow_slab && view_parity.size() == 1) {
     const int rh = view_parity[0].first, rw = view_parity[0].second;
     if (rh < a.Hs && rw < a.Ws) {
@@ -806,7 +806,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
 int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps_in,
                   const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                   long long sn, long long sc, long long sh, long long sw, long long off,
-                  const float* bias, int relu, bool allow_slab = true) {
+                  const void* bias, int relu, bool allow_slab = true) {
   if (c->epi.pool) {                  // only the slab kernel's staged epilogue pools
     if (!allow_slab || view_parity.size() != 1) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
     const int rh = view_parity[0].first, rw = view_parity[0].second;
@@ -969,12 +969,17 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   if (!(flags & B200CONV_FORCE_DIRECT) && !c->epi.pool && flatten_1x1(d, in_nhwc && out_nhwc, &flat))
     return fwd_device(c, flat, x, w, bias, y, flags);
   Scratch tmp(c);
-  float* bias_f = nullptr;
-  if (bias) {
-    int rc = tmp.get(sizeof(float) * d.K, reinterpret_cast<void**>(&bias_f));
-    if (rc) return rc;
-    KLAUNCH(c, kKPack, launch_convert_bias(bias, bias_f, d.K, d.dtype, c->stream));
-  }
+  // the direct kernels take the bias as float32; the tensor-core kernels read it in the data type
+  const float* bias_f = d.dtype == B200CONV_F32 ? static_cast<const float*>(bias) : nullptr;
+  auto convert_bias = [&]() -> int {
+    if (!bias || bias_f) return 0;
+    float* f;
+    int r = tmp.get(sizeof(float) * d.K, reinterpret_cast<void**>(&f));
+    if (r) return r;
+    KLAUNCH(c, kKPack, launch_convert_bias(bias, f, d.K, d.dtype, c->stream));
+    bias_f = f;
+    return 0;
+  };
   const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor(d);
   if (mg > 1) {
     b200conv_desc dm = d;
@@ -991,6 +996,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   if (!use_umma) {
     if (flags & B200CONV_FORCE_UMMA) return fail(c, B200CONV_E_UNSUPPORTED, "geometry not covered by the tensor-core kernel");
     if (in_nhwc || out_nhwc) return fail(c, B200CONV_E_UNSUPPORTED, "direct kernels take NCHW tensors only");
+    if (int r = convert_bias()) return r;
     KLAUNCH(c, kKDirect, launch_direct_fwd(d, x, w, bias_f, y, (flags & B200CONV_RELU) ? 1 : 0, c->epi, c->stream));
     c->last_algo = "direct";
     return 0;
@@ -1031,7 +1037,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     } else {
       sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
     }
-    rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias_f,
+    rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias,
                        (flags & B200CONV_RELU) ? 1 : 0, !(flags & B200CONV_NO_SLAB));
     if (rc == 1) return fail(c, B200CONV_E_CUDA, "internal: empty space-to-depth view");
     c->last_algo = "umma";
@@ -1074,7 +1080,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     } else {
       sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
     }
-    rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias_f,
+    rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias,
                        (flags & B200CONV_RELU) ? 1 : 0, !(flags & B200CONV_NO_SLAB));
     if (rc == 1) return fail(c, B200CONV_E_CUDA, "internal: empty folded view");
     c->last_algo = "umma";
@@ -1128,12 +1134,13 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   } else {
     sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
   }
-  rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias_f,
+  rc = run_conv_umma(c, a, taps, parity, d.Wo, d.Ho, y, sn, sc, sh, sw, 0, bias,
                      (flags & B200CONV_RELU) ? 1 : 0, !(flags & B200CONV_NO_SLAB));
   if (rc == 1) {  // every tap fell outside the image: conv == 0, only the epilogue remains
     b200conv_desc z = d;
     z.C = 0;
     if (out_nhwc) return fail(c, B200CONV_E_UNSUPPORTED, "degenerate geometry with channels-last output");
+    if (int r = convert_bias()) return r;
     KLAUNCH(c, kKDirect, launch_direct_fwd(z, x, w, bias_f, y, (flags & B200CONV_RELU) ? 1 : 0, c->epi, c->stream));
     rc = 0;
   }

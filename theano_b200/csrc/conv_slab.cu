@@ -279,7 +279,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           uint8_t* stg = smem + p.stage_off + (grp * bufs + (bufs == 2 ? (nstore & 1) : 0)) * p.stage_bytes;
           uint8_t* srow = stg + drow * 128;
           const int co0 = co_base + ch * kCh;
-          const float* bias = p.bias ? p.bias + g * p.n_out + co0 : nullptr;
+          const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
           long long tq = trace ? clock64() : 0;
           if (nstore >= bufs) {                // the buffer's previous box must have been read
             if (issuer) {
@@ -296,7 +296,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             tmem_ld_wait();
             if (trace) { const long long t = clock64(); tp[1] += t - tq; tq = t; }
             if (!inbox) continue;
-            const float* bp = bias ? bias + part * 32 : nullptr;
+            const OutT* bp = bias ? bias + part * 32 : nullptr;
             if (plain) {
               // no scale, bias or activation (gradInputs, bare forward): convert and stage only.
               // The epilogue warps are bound by their instruction issue, not by TMEM or shared memory.
@@ -323,7 +323,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                   f[q] = p.epi.alpha * __uint_as_float(r[4 * j + q]);
-                  if (bp) f[q] += bp[4 * j + q];
+                  if (bp) f[q] += static_cast<float>(bp[4 * j + q]);
                   if (p.relu) f[q] = p.epi.lin * f[q] + p.epi.abs * fabsf(f[q]);
                 }
                 *reinterpret_cast<float4*>(srow + ((j ^ (drow & 7)) << 4)) = make_float4(f[0], f[1], f[2], f[3]);
@@ -336,7 +336,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
                 for (int q = 0; q < 4; ++q) {
                   float f0 = p.epi.alpha * __uint_as_float(r[8 * j + 2 * q]);
                   float f1 = p.epi.alpha * __uint_as_float(r[8 * j + 2 * q + 1]);
-                  if (bp) { f0 += bp[8 * j + 2 * q]; f1 += bp[8 * j + 2 * q + 1]; }
+                  if (bp) { f0 += static_cast<float>(bp[8 * j + 2 * q]); f1 += static_cast<float>(bp[8 * j + 2 * q + 1]); }
                   if (p.relu) {
                     f0 = p.epi.lin * f0 + p.epi.abs * fabsf(f0);
                     f1 = p.epi.lin * f1 + p.epi.abs * fabsf(f1);
@@ -426,7 +426,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           tmem_ld_wait();
           if (!valid) continue;
           const int co0 = co_base + ch * 32;
-          const float* bias = p.bias ? p.bias + g * p.n_out + co0 : nullptr;
+          const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
           if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
 #pragma unroll
             for (int j = 0; j < 32; j += 16 / sizeof(OutT)) {
@@ -435,7 +435,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
 #pragma unroll
               for (int q = 0; q < 16 / (int)sizeof(OutT); ++q) {
                 f[q] = p.epi.alpha * __uint_as_float(r[j + q]);
-                if (bias) f[q] += bias[j + q];
+                if (bias) f[q] += static_cast<float>(bias[j + q]);
                 if (res) f[q] += p.epi.beta * static_cast<float>(res[co0 + j + q]);
                 if (p.relu) f[q] = p.epi.lin * f[q] + p.epi.abs * fabsf(f[q]);
               }
@@ -459,7 +459,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             for (int j = 0; j < 32; ++j) {
               if (co0 + j < p.n_out) {
                 float v = p.epi.alpha * __uint_as_float(r[j]);
-                if (bias) v += bias[j];
+                if (bias) v += static_cast<float>(bias[j]);
                 if (res) v += p.epi.beta * static_cast<float>(res[(co0 + j) * p.out_sc]);
                 if (p.relu) v = p.epi.lin * v + p.epi.abs * fabsf(v);
                 if (B200_IN_RANGE((pix - out) + (co0 + j) * p.out_sc >= 0 && (pix - out) + (co0 + j) * p.out_sc < p.out_elems, p.status))

@@ -214,7 +214,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
         tmem_ld_wait();
         if (!valid) continue;
-        const float* bias = p.bias ? p.bias + g * p.n_out + co0 : nullptr;
+        const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
         if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
 #pragma unroll
           for (int j = 0; j < 32; j += 16 / sizeof(OutT)) {
@@ -223,7 +223,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
 #pragma unroll
             for (int q = 0; q < 16 / (int)sizeof(OutT); ++q) {
               f[q] = p.epi.alpha * __uint_as_float(r[j + q]);
-              if (bias) f[q] += bias[j + q];
+              if (bias) f[q] += static_cast<float>(bias[j + q]);
               if (res) f[q] += p.epi.beta * static_cast<float>(res[co0 + j + q]);
               if (p.relu) f[q] = p.epi.lin * f[q] + p.epi.abs * fabsf(f[q]);
             }
@@ -247,7 +247,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
           for (int j = 0; j < 32; ++j) {
             if (co0 + j < p.n_out) {
               float v = p.epi.alpha * __uint_as_float(r[j]);
-              if (bias) v += bias[j];
+              if (bias) v += static_cast<float>(bias[j]);
               if (res) v += p.epi.beta * static_cast<float>(res[(co0 + j) * p.out_sc]);
               if (p.relu) v = p.epi.lin * v + p.epi.abs * fabsf(v);
               if (B200_IN_RANGE((pix - out) + (co0 + j) * p.out_sc >= 0 && (pix - out) + (co0 + j) * p.out_sc < p.out_elems, p.status))

@@ -154,7 +154,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
       const uint32_t lane_base = tmem + buf * kBN + (static_cast<uint32_t>(quad * 32) << 16);
       if (grp < nstaged) {
         const int co0 = co_base + grp * 64;
-        const float* bias = p.bias ? p.bias + co0 : nullptr;
+        const __half* bias = p.bias ? static_cast<const __half*>(p.bias) + co0 : nullptr;
         if (nstore > 0) {                                            // the buffer's previous box must have been read
           if (issuer) bulk_wait_read<0>();
           named_barrier(1 + grp, 128);
@@ -164,7 +164,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
           uint32_t r[32];
           tmem_ld32(lane_base + grp * 64 + part * 32, r);
           tmem_ld_wait();
-          const float* bp = bias ? bias + part * 32 : nullptr;
+          const __half* bp = bias ? bias + part * 32 : nullptr;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             uint32_t h[4];
@@ -173,7 +173,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
               float f0 = __uint_as_float(r[8 * j + 2 * q]), f1 = __uint_as_float(r[8 * j + 2 * q + 1]);
               if (!plain) {
                 f0 *= p.epi.alpha; f1 *= p.epi.alpha;
-                if (bp) { f0 += bp[8 * j + 2 * q]; f1 += bp[8 * j + 2 * q + 1]; }
+                if (bp) { f0 += static_cast<float>(bp[8 * j + 2 * q]); f1 += static_cast<float>(bp[8 * j + 2 * q + 1]); }
                 if (p.relu) {
                   f0 = p.epi.lin * f0 + p.epi.abs * fabsf(f0);
                   f1 = p.epi.lin * f1 + p.epi.abs * fabsf(f1);

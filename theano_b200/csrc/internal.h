@@ -73,7 +73,7 @@ struct alignas(64) UmmaConvParams {
   int tiles_w, tiles_h, tiles_n, tiles_co;
   int n_out;                     // output channels per group
   void* out;
-  const float* bias;             // per output channel (groups*n_out) or null
+  const void* bias;              // per output channel (groups*n_out), in the data type, or null
   long long out_sn, out_sc, out_sh, out_sw, out_off;  // element strides / offset of `out`
   long long out_elems;           // elements of `out` this launch may touch (checked in the range-checked build)
   int relu;
@@ -109,7 +109,7 @@ struct alignas(64) SlabConvParams {
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
   int n_out;
   void* out;
-  const float* bias;
+  const void* bias;
   long long out_sn, out_sc, out_sh, out_sw, out_off;
   long long out_elems;           // elements of `out` this launch may touch (checked in the range-checked build)
   int relu;
@@ -142,7 +142,7 @@ struct alignas(64) PairGemmParams {
   int tiles_pix, tiles_co;       // 256-pixel tiles, 256-filter tiles
   int pixels, n_out;
   int stages;                    // ring depth (2 .. 5)
-  const float* bias;
+  const void* bias;
   int relu;
   ConvEpilogue epi;
   int* status;
@@ -291,7 +291,6 @@ cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits,
 cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int Kg, int m, int taps,
                                 int extract, int dtype, cudaStream_t s);
 cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, cudaStream_t s);
-cudaError_t launch_convert_to_half(const float* src, void* dst, int n, cudaStream_t s);
 cudaError_t launch_maxpool2x2(const void* x, void* y, int N, int C, int H, int W, int nhwc,
                               int Cp, int dtype, cudaStream_t s);
 cudaError_t launch_maxpool2x2_grad(const void* x, const void* y, const void* gy, void* gx, int N, int C,
