@@ -30,83 +30,52 @@ __global__ void transpose_kernel(const T* __restrict__ in, T* __restrict__ out, 
 //   mode 0 (forward):        rows = filters of the group, cols = channels,
 //                            tap t = i*kW + j multiplies the pixel at offset (i, j);
 //   mode 1 (input gradient): rows = channels, cols = filters of the group.
-// With flip the correlation tap (i, j) reads w[..][kH-1-i][kW-1-j].
-// One block moves a small patch of (filters x channels) for a chunk of taps through shared
-// memory: the read runs along (channel, tap), which is contiguous in OIHW, the write along the
-// destination's column index.  The patch is 8 filters x 32 channels for mode 0 and 32 filters x
-// 8 channels for mode 1, so that 32 consecutive destination columns are written together and
-// there are enough blocks to fill the GPU.
-constexpr int kPackTaps = 9;
-// MODE and the tap count (TAPS = kH * kW for the usual 1 and 9, 0 = any, read at run time) are
-// template parameters: the element loop divides by patch width x taps, and with run-time divisors
-// those divisions, not the memory traffic, set the pace (47 MB of ResNet-50 filters took 0.4 ms).
-template <typename T, int MODE, int TAPS>
-__device__ __forceinline__ void pack_filters_block_t(const T* __restrict__ w, T* __restrict__ dst, int K, int Cg,
-                                                     int kH, int kW, int groups, int flip, int ldc,
-                                                     int bx, int by, int bz, T* tile) {
-  constexpr int PK = MODE == 0 ? 8 : 32, PC = MODE == 0 ? 32 : 8;
-  constexpr int pitch = PC * kPackTaps + 1;
-  const int Kg = K / groups, T_ = TAPS > 0 ? TAPS : kH * kW;
-  const int g = bz;
-  const int k0 = by * PK, c0 = bx * PC;
-  const int rows = MODE == 0 ? Kg : Cg;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  for (int t0 = 0; t0 < T_; t0 += kPackTaps) {
-    const int nt = min(kPackTaps, T_ - t0);
-    // load: for one filter, PC channels x all taps are contiguous in memory
-    for (int i = tid; i < PK * PC * T_; i += 256) {
-      const int kk = i / (PC * T_), rem = i % (PC * T_);
-      const int cc = rem / T_, tt = rem % T_;
-      if (tt < t0 || tt >= t0 + nt) continue;
-      const int kq = k0 + kk;
-      T v = T(0);
-      if (kq < Kg && c0 + cc < Cg) v = w[(1LL * (g * Kg + kq) * Cg + c0 + cc) * T_ + tt];
-      tile[kk * pitch + cc * kPackTaps + (tt - t0)] = v;
-    }
-    __syncthreads();
-    for (int tt = 0; tt < nt; ++tt) {
-      const int src_tap = t0 + tt;                       // position in the filter as stored
-      const int i = src_tap / kW, j = src_tap % kW;
-      const int tap = flip ? (kH - 1 - i) * kW + (kW - 1 - j) : src_tap;   // correlation tap it serves
-      T* d = dst + 1LL * (tap * groups + g) * rows * ldc;
-      const int rr = threadIdx.y, xx = threadIdx.x;
-      if (MODE == 0) {       // row = filter (8 per block), col = channel (32 per block)
-        const int kq = k0 + rr, c = c0 + xx;
-        if (kq < Kg && c < ldc) d[1LL * kq * ldc + c] = c < Cg ? tile[rr * pitch + xx * kPackTaps + tt] : T(0);
-      } else {               // row = channel (8 per block), col = filter (32 per block)
-        const int c = c0 + rr, kq = k0 + xx;
-        if (c < Cg && kq < ldc) d[1LL * c * ldc + kq] = kq < Kg ? tile[xx * pitch + rr * kPackTaps + tt] : T(0);
-      }
-    }
-    __syncthreads();
-  }
+// With flip the correlation tap t reads position taps - 1 - t of the filter.
+// A block moves a patch of filters x channels with all its taps through shared memory: the taps of
+// a filter's consecutive channels are one contiguous run of OIHW, the write runs along 32 columns
+// of the destination.  What bounds a small bank is the chain of loads in a block and the number of
+// blocks, so the patch is cut to about kPackPatch elements whatever the tap count (a warp loads a
+// filter's run without any division, all loads of a thread in flight), and rows of the patch go
+// to warps tap by tap.  Measured: 50 x 20 x 5x5 float32 25 -> 3 us, 64 x 64 x 3x3 float16 4.5 -> 3 us.
+constexpr int kPackPatch = 2560;
+constexpr int kPackSmem = kPackPatch + 64;
+// filters (mode 0) or channels (mode 1) of a patch beside the 32 along the destination's columns
+__host__ __device__ inline int pack_rows(int taps) {
+  const int r = kPackPatch / (32 * taps);
+  return r < 1 ? 1 : r > 8 ? 8 : r;
 }
-
 template <typename T>
 __device__ __forceinline__ void pack_filters_block(const T* __restrict__ w, T* __restrict__ dst, int K, int Cg,
-                                                   int kH, int kW, int groups, int flip, int mode, int ldc,
-                                                   int bx, int by, int bz) {
-  __shared__ T tile[256 * kPackTaps + 40];
-  const int taps = kH * kW;
-  if (mode == 0) {
-    if (taps == 9) pack_filters_block_t<T, 0, 9>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
-    else if (taps == 1) pack_filters_block_t<T, 0, 1>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
-    else pack_filters_block_t<T, 0, 0>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
-  } else {
-    if (taps == 9) pack_filters_block_t<T, 1, 9>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
-    else if (taps == 1) pack_filters_block_t<T, 1, 1>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
-    else pack_filters_block_t<T, 1, 0>(w, dst, K, Cg, kH, kW, groups, flip, ldc, bx, by, bz, tile);
+                                                   int taps, int groups, int flip, int mode, int ldc,
+                                                   int bx, int by, int g) {
+  __shared__ T tile[kPackSmem];
+  const int pr = pack_rows(taps);
+  const int PK = mode == 0 ? pr : 32, PC = mode == 0 ? 32 : pr;
+  const int Kg = K / groups, k0 = by * PK, c0 = bx * PC;
+  const int lane = threadIdx.x, wp = threadIdx.y;
+  const int nk = min(PK, Kg - k0), nc = min(PC, Cg - c0);      // <= 0 in patches that only pad
+  const int run = nc * taps, pitch = (PC * taps) | 1;
+  for (int kk = wp; kk < nk; kk += 8) {
+    const T* src = w + (1LL * (g * Kg + k0 + kk) * Cg + c0) * taps;
+#pragma unroll 8
+    for (int i = lane; i < run; i += 32) tile[kk * pitch + i] = src[i];
+  }
+  __syncthreads();
+  const int rows = mode == 0 ? Kg : Cg, nrow = mode == 0 ? nk : nc;
+  const int col = (mode == 0 ? c0 : k0) + lane, row0 = mode == 0 ? k0 : c0;
+  const bool real = lane < (mode == 0 ? nc : nk);
+  if (col >= ldc) return;
+  for (int rr = wp % pr, t = wp / pr; t < taps;) {             // warp unit u = t * pr + rr, u += 8
+    if (rr < nrow) {
+      const int tap = flip ? taps - 1 - t : t;
+      const T v = real ? (mode == 0 ? tile[rr * pitch + lane * taps + t] : tile[lane * pitch + rr * taps + t]) : T(0);
+      dst[(1LL * (tap * groups + g) * rows + row0 + rr) * ldc + col] = v;
+    }
+    rr += 8;
+    while (rr >= pr) { rr -= pr; ++t; }
   }
 }
 
-template <typename T>
-__global__ void pack_filters_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int Cg,
-                                    int kH, int kW, int groups, int flip, int mode, int ldc) {
-  pack_filters_block<T>(w, dst, K, Cg, kH, kW, groups, flip, mode, ldc, blockIdx.x, blockIdx.y, blockIdx.z);
-}
-
-// Many filter banks in one launch: block b belongs to the job j with first_block[j] <= b <
-// first_block[j + 1] and does there what block (bx, by, bz) of pack_filters_kernel would do.
 // 1x1 banks for gradInputs are plain transposes [K][C] -> [C][ldc]: 64 x 64 tiles through shared memory, read
 // along c and written along k in 128-byte runs (the general patch kernel moves 16-byte runs here).
 template <typename T>
@@ -131,20 +100,25 @@ __device__ __forceinline__ void transpose_1x1_block(const T* __restrict__ w, T* 
 }
 
 template <typename T>
-__global__ void pack_filters_batch_kernel(const __grid_constant__ PackBatch b) {
+__device__ __forceinline__ void pack_job_block(const PackJob& q, int local) {
+  const int bx = local % q.gx, by = local / q.gx % q.gy, bz = local / q.gx / q.gy;
+  const T* src = static_cast<const T*>(q.src);
+  T* dst = static_cast<T*>(q.dst);
+  if (q.kH * q.kW == 1 && q.mode == 1) transpose_1x1_block<T>(src, dst, q.K, q.Cg, q.groups, q.ldc, bx, by, bz);
+  else pack_filters_block<T>(src, dst, q.K, q.Cg, q.kH * q.kW, q.groups, q.flip, q.mode, q.ldc, bx, by, bz);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ PackJob q) {
+  pack_job_block<T>(q, blockIdx.x);
+}
+
+// Many filter banks in one launch: block b belongs to the job j with first_block[j] <= b < first_block[j + 1].
+template <typename T>
+__global__ void __launch_bounds__(256) pack_filters_batch_kernel(const __grid_constant__ PackBatch b) {
   int j = 0;
   while (j + 1 < b.njobs && static_cast<int>(blockIdx.x) >= b.jobs[j + 1].first_block) ++j;
-  const PackJob& q = b.jobs[j];
-  int local = blockIdx.x - q.first_block;
-  const int bx = local % q.gx;
-  local /= q.gx;
-  const int by = local % q.gy, bz = local / q.gy;
-  if (q.kH * q.kW == 1 && q.mode == 1) {
-    transpose_1x1_block<T>(static_cast<const T*>(q.src), static_cast<T*>(q.dst), q.K, q.Cg, q.groups, q.ldc, bx, by, bz);
-    return;
-  }
-  pack_filters_block<T>(static_cast<const T*>(q.src), static_cast<T*>(q.dst), q.K, q.Cg, q.kH, q.kW, q.groups, q.flip,
-                        q.mode, q.ldc, bx, by, bz);
+  pack_job_block<T>(b.jobs[j], blockIdx.x - b.jobs[j].first_block);
 }
 
 // Few-channel layers ("row folding"): the image is copied channels-last with explicit zero
@@ -518,7 +492,7 @@ void pack_filters_grid(int Kg, int Cg, int groups, int mode, int ldc, int taps, 
   }
   // the patch grid covers the padded column range [0, ldc) of the destination as well
   const int cols_c = mode == 0 ? ldc : Cg, cols_k = mode == 0 ? Kg : ldc;
-  const int PK = mode == 0 ? 8 : 32, PC = mode == 0 ? 32 : 8;
+  const int PK = mode == 0 ? pack_rows(taps) : 32, PC = mode == 0 ? 32 : pack_rows(taps);
   *gx = (cols_c + PC - 1) / PC;
   *gy = (cols_k + PK - 1) / PK;
   *gz = groups;
@@ -534,20 +508,15 @@ cudaError_t launch_pack_filters_batch(const PackBatch& b, int total_blocks, int 
 cudaError_t launch_pack_filters(const void* w, void* dst, int K, int Cg, int kH, int kW,
                                 int groups, int flip, int mode, int ldc, int dtype,
                                 cudaStream_t s) {
-  const int Kg = K / groups;
   if (1LL * kH * kW * K * Cg == 0) return cudaSuccess;
-  // the patch grid covers the padded column range [0, ldc) of the destination as well
-  const int cols_c = mode == 0 ? ldc : Cg, cols_k = mode == 0 ? Kg : ldc;
-  const int PK = mode == 0 ? 8 : 32, PC = mode == 0 ? 32 : 8;
-  dim3 grid((cols_c + PC - 1) / PC, (cols_k + PK - 1) / PK, groups), block(32, 8);
-  if (dtype == B200CONV_F16)
-    pack_filters_kernel<__half><<<grid, block, 0, s>>>(static_cast<const __half*>(w),
-                                                       static_cast<__half*>(dst), K, Cg, kH, kW,
-                                                       groups, flip, mode, ldc);
-  else
-    pack_filters_kernel<float><<<grid, block, 0, s>>>(static_cast<const float*>(w),
-                                                      static_cast<float*>(dst), K, Cg, kH, kW, groups,
-                                                      flip, mode, ldc);
+  PackJob q;
+  int gz;
+  q.src = w; q.dst = dst;
+  q.K = K; q.Cg = Cg; q.kH = kH; q.kW = kW; q.groups = groups; q.flip = flip; q.mode = mode; q.ldc = ldc;
+  pack_filters_grid(K / groups, Cg, groups, mode, ldc, kH * kW, &q.gx, &q.gy, &gz);
+  q.first_block = 0;
+  if (dtype == B200CONV_F16) pack_filters_kernel<__half><<<q.gx * q.gy * gz, dim3(32, 8), 0, s>>>(q);
+  else pack_filters_kernel<float><<<q.gx * q.gy * gz, dim3(32, 8), 0, s>>>(q);
   return cudaGetLastError();
 }
 

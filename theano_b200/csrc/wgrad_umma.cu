@@ -336,40 +336,41 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
   }
 }
 
-// out[k][c][tap] = sum_s partial[s][tap][k][c].  A block takes kReduceElems consecutive (k, c)
-// elements and all taps.  Its 256 threads are 32 groups of four elements x 8 lanes over the
-// slabs: lane q adds the slabs q, q + 8, ... in that order and the eight partial sums are then
-// added in lane order, so the result does not depend on scheduling (it is the same on every run)
-// and no thread walks more than an eighth of the slabs (a layer with few filters and channels has
-// up to one slab per SM, and one thread adding 148 of them one after the other took longer than
-// the gradient kernel's tail).  The sums go to shared memory in output order [element][tap] and
-// leave as one contiguous run of kReduceElems * taps values.
-constexpr int kReduceElems = 128;      // (k, c) elements per block tile of the reduction kernel
-constexpr int kReduceLanes = 8;
+// out[k][c][tap] = sum_s partial[s][tap][k][c].  A block takes `elems` consecutive (k, c) elements and
+// all taps: (elems / 4) * taps groups of four, each added by `lanes` threads: lane q takes the slabs
+// q, q + lanes, ... in that order and the partial sums are then added in lane order, so the result
+// does not depend on scheduling (it is the same on every run).  The sums go to shared memory in
+// output order [element][tap] and leave as one contiguous run of elems * taps values.
+// The slabs are read once, from L2 or HBM; what bounds the kernel below a few megabytes is the length
+// of the chain of loads in a thread, so small gradients get small blocks (16 elements: two rounds of
+// 256 threads for a 3x3 filter; 64 x 64 x 3x3 float16: 7.5 -> 3 us) and only long sums are split over lanes.
 template <typename T>
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ dw,
-                                                            int splits, int taps, long long kc) {
+                                                            int splits, int taps, long long kc, int log_elems, int log_lanes) {
   extern __shared__ float tile[];
-  __shared__ float4 part[kReduceLanes][kReduceElems / 4];
-  const long long tiles = (kc + kReduceElems - 1) / kReduceElems;
+  __shared__ float4 part[256];
+  const int elems = 1 << log_elems, lanes = 1 << log_lanes, slots = 256 >> log_lanes;
+  const int lane = threadIdx.x >> (8 - log_lanes), slot = threadIdx.x & (slots - 1);
+  const long long tiles = (kc + elems - 1) >> log_elems, slab = taps * kc;
   const bool vec = (kc & 3) == 0;
-  const int q = threadIdx.x >> 5, gi = threadIdx.x & 31, e = gi * 4;
+  const int units = (elems >> 2) * taps;
   for (long long tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
-    const long long e0 = tl * kReduceElems;
-    const int ne = static_cast<int>(kc - e0 < kReduceElems ? kc - e0 : kReduceElems);
-    for (int t = 0; t < taps; ++t) {
+    const long long e0 = tl << log_elems;
+    const int ne = static_cast<int>(kc - e0 < elems ? kc - e0 : elems);
+    for (int base = 0; base < units; base += slots) {
+      const int u = base + slot, t = u >> (log_elems - 2), e = (u & ((elems >> 2) - 1)) << 2;
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < ne) {
+      if (u < units && e < ne) {
         const float* src = partial + 1LL * t * kc + e0 + e;
-        const long long slab = 1LL * taps * kc;
         if (vec) {
-#pragma unroll 4
-          for (int s = q; s < splits; s += kReduceLanes) {
+#pragma unroll 8
+          for (int s = lane; s < splits; s += lanes) {
             const float4 v = *reinterpret_cast<const float4*>(src + s * slab);
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
           }
         } else {
-          for (int s = q; s < splits; s += kReduceLanes) {
+#pragma unroll 4
+          for (int s = lane; s < splits; s += lanes) {
             const float* ps = src + s * slab;
             acc.x += ps[0];
             if (e + 1 < ne) acc.y += ps[1];
@@ -378,24 +379,26 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restri
           }
         }
       }
-      part[q][gi] = acc;
-      __syncthreads();
-      if (q == 0 && e < ne) {
-        float4 sum = part[0][gi];
-#pragma unroll
-        for (int l = 1; l < kReduceLanes; ++l) {
-          const float4 v = part[l][gi];
-          sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-        }
-        tile[(e + 0) * taps + t] = sum.x;
-        tile[(e + 1) * taps + t] = sum.y;
-        tile[(e + 2) * taps + t] = sum.z;
-        tile[(e + 3) * taps + t] = sum.w;
+      if (lanes > 1) {
+        part[threadIdx.x] = acc;
+        __syncthreads();
+        if (lane == 0)
+          for (int l = 1; l < lanes; ++l) {
+            const float4 v = part[l * slots + slot];
+            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+          }
       }
-      __syncthreads();
+      if (lane == 0 && u < units && e < ne) {
+        tile[(e + 0) * taps + t] = acc.x;
+        tile[(e + 1) * taps + t] = acc.y;
+        tile[(e + 2) * taps + t] = acc.z;
+        tile[(e + 3) * taps + t] = acc.w;
+      }
+      if (lanes > 1) __syncthreads();
     }
+    __syncthreads();
     T* dst = dw + e0 * taps;
-    for (int i = threadIdx.x; i < ne * taps; i += blockDim.x) dst[i] = static_cast<T>(tile[i]);
+    for (int i = threadIdx.x; i < ne * taps; i += 256) dst[i] = static_cast<T>(tile[i]);
     __syncthreads();
   }
 }
@@ -436,15 +439,20 @@ cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int 
                                 int Cg, int dtype, cudaStream_t s) {
   const long long kc = 1LL * K * Cg;
   if (kc == 0 || taps == 0) return cudaSuccess;
-  long long g = (kc + kReduceElems - 1) / kReduceElems;
+  // 128 elements per block, fewer while that leaves SMs without two blocks; 2^log_lanes threads per
+  // sum: about four slabs each, at most 8 threads
+  int log_elems = 7, log_lanes = 0;
+  while (log_elems > 4 && (kc >> log_elems) < 2 * 148) --log_elems;
+  while (log_lanes < 3 && splits > (4 << log_lanes)) ++log_lanes;
+  long long g = (kc + (1 << log_elems) - 1) >> log_elems;
   if (g > 148 * 16) g = 148 * 16;
-  const size_t smem = sizeof(float) * kReduceElems * taps;
+  const size_t smem = sizeof(float) * taps << log_elems;
   if (dtype == B200CONV_F16)
     wgrad_reduce_kernel<__half><<<static_cast<int>(g), 256, smem, s>>>(
-        partial, static_cast<__half*>(dw), splits, taps, kc);
+        partial, static_cast<__half*>(dw), splits, taps, kc, log_elems, log_lanes);
   else
     wgrad_reduce_kernel<float><<<static_cast<int>(g), 256, smem, s>>>(
-        partial, static_cast<float*>(dw), splits, taps, kc);
+        partial, static_cast<float*>(dw), splits, taps, kc, log_elems, log_lanes);
   return cudaGetLastError();
 }
 
