@@ -2364,15 +2364,10 @@ int b200conv_channel_sum(b200conv_ctx* c, const void* x, void* out, long long pi
     return fail(c, B200CONV_E_INVALID, "bad channel sum");
   const int Cp = pad_channels(C, dtype);
   Scratch tmp(c);
-  float *partial = nullptr, *sums = nullptr;
+  float* partial = nullptr;
   int rc = tmp.get(sizeof(float) * Cp * channel_sum_blocks(pixels), reinterpret_cast<void**>(&partial));
-  if (rc || (rc = tmp.get(sizeof(float) * Cp, reinterpret_cast<void**>(&sums)))) return rc;
-  KLAUNCH(c, kKTranspose, launch_channel_sum(x, partial, sums, pixels, C, Cp, dtype, c->stream));
-  if (dtype == B200CONV_F32) {
-    CU_OK(c, cudaMemcpyAsync(out, sums, sizeof(float) * C, cudaMemcpyDeviceToDevice, c->stream));
-  } else {                                  // float32 sums -> float16 values
-    KLAUNCH(c, kKPack, launch_convert_to_half(sums, out, C, c->stream));
-  }
+  if (rc) return rc;
+  KLAUNCH(c, kKTranspose, launch_channel_sum(x, partial, out, pixels, C, Cp, dtype, c->stream));
   return 0;
 }
 

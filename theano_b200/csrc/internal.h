@@ -304,7 +304,7 @@ enum : int { kEwAdd = 0, kEwMul, kEwSub, kEwRSub, kEwDiv, kEwRDiv, kEwMax, kEwAb
 cudaError_t launch_elementwise(const void* a, const void* b, const float* chan, void* out, long long elems, int C,
                                int Cp, int op, int b_kind, float s, int dtype, cudaStream_t st);
 int channel_sum_blocks(long long pixels);          // rows of Cp floats the partial buffer needs
-cudaError_t launch_channel_sum(const void* x, float* partial, float* out, long long pixels, int C, int Cp, int dtype,
+cudaError_t launch_channel_sum(const void* x, float* partial, void* out, long long pixels, int C, int Cp, int dtype,
                                cudaStream_t st);
 
 // ---- bounded-wait self-test (selftest.cu): one CTA waits, with `limit`, on a barrier nobody arrives on

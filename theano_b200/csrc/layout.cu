@@ -331,67 +331,122 @@ __global__ void convert_bias_kernel(const T* __restrict__ b, float* __restrict__
 // NCHW: one thread per output element.  NHWC: one thread per (pixel, channel) with the
 // channel fastest, so neighbouring threads read neighbouring addresses.
 template <typename T>
-__global__ void maxpool2x2_kernel(const T* __restrict__ x, T* __restrict__ y, int N, int C, int H,
-                                  int W, int nhwc, int Cp) {
+__global__ void maxpool2x2_nchw_kernel(const T* __restrict__ x, T* __restrict__ y, long long NC, int H, int W) {
   const int Ho = H / 2, Wo = W / 2;
-  const int Cx = nhwc ? Cp : C;
-  const long long total = 1LL * N * Cx * Ho * Wo;
+  const long long total = NC * Ho * Wo;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
-    if (nhwc) {
-      const int c = idx % Cp;
-      const int ow = (idx / Cp) % Wo;
-      const int oh = (idx / (1LL * Cp * Wo)) % Ho;
-      const int n = idx / (1LL * Cp * Wo * Ho);
-      const T* p = x + ((1LL * n * H + 2 * oh) * W + 2 * ow) * Cp + c;
-      float m = static_cast<float>(p[0]);
-      m = fmaxf(m, static_cast<float>(p[Cp]));
-      m = fmaxf(m, static_cast<float>(p[1LL * W * Cp]));
-      m = fmaxf(m, static_cast<float>(p[1LL * W * Cp + Cp]));
-      y[idx] = static_cast<T>(m);
-    } else {
-      const int ow = idx % Wo;
-      const int oh = (idx / Wo) % Ho;
-      const long long nc = idx / (1LL * Wo * Ho);
-      const T* p = x + (nc * H + 2 * oh) * W + 2 * ow;
-      float m = static_cast<float>(p[0]);
-      m = fmaxf(m, static_cast<float>(p[1]));
-      m = fmaxf(m, static_cast<float>(p[W]));
-      m = fmaxf(m, static_cast<float>(p[W + 1]));
-      y[idx] = static_cast<T>(m);
-    }
+    const int ow = idx % Wo;
+    const int oh = (idx / Wo) % Ho;
+    const long long nc = idx / (1LL * Wo * Ho);
+    const T* p = x + (nc * H + 2 * oh) * W + 2 * ow;
+    float m = static_cast<float>(p[0]);
+    m = fmaxf(m, static_cast<float>(p[1]));
+    m = fmaxf(m, static_cast<float>(p[W]));
+    m = fmaxf(m, static_cast<float>(p[W + 1]));
+    y[idx] = static_cast<T>(m);
   }
 }
 
-// Gradient of the 2x2 / stride 2 max pooling: one thread per input element (so every element of
-// gx is written): gx = gy of its window if x equals the window maximum, else 0.
+// Gradient of the 2x2 / stride 2 max pooling: gx = gy of its window if x equals the window maximum y, else 0;
+// every element of gx is written.  One thread per input element.
 template <typename T>
-__global__ void maxpool2x2_grad_kernel(const T* __restrict__ x, const T* __restrict__ y,
-                                       const T* __restrict__ gy, T* __restrict__ gx, int N, int C, int H,
-                                       int W, int nhwc, int Cp) {
+__global__ void maxpool2x2_grad_nchw_kernel(const T* __restrict__ x, const T* __restrict__ y,
+                                            const T* __restrict__ gy, T* __restrict__ gx, long long NC, int H, int W) {
   const int Ho = H / 2, Wo = W / 2;
-  const int Cx = nhwc ? Cp : C;
-  const long long total = 1LL * N * Cx * H * W;
+  const long long total = NC * H * W;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
-    int h, w;
-    long long o;            // index of the window in y / gy
-    if (nhwc) {
-      const int c = idx % Cp;
-      w = (idx / Cp) % W;
-      h = (idx / (1LL * Cp * W)) % H;
-      const long long n = idx / (1LL * Cp * W * H);
-      o = ((n * Ho + h / 2) * Wo + w / 2) * Cp + c;
-    } else {
-      w = idx % W;
-      h = (idx / W) % H;
-      const long long nc = idx / (1LL * W * H);
-      o = (nc * Ho + h / 2) * Wo + w / 2;
-    }
+    const int w = idx % W, h = (idx / W) % H;
+    const long long nc = idx / (1LL * W * H), o = (nc * Ho + h / 2) * Wo + w / 2;
     T g = static_cast<T>(0.f);
     if (h < 2 * Ho && w < 2 * Wo && static_cast<float>(x[idx]) == static_cast<float>(y[o])) g = gy[o];
     gx[idx] = g;
   }
+}
+
+// Channels-last forms: one thread per window and 16-byte piece of the channel vector, so that every access
+// is 16 bytes wide, the four pixels' loads are in flight together and the index arithmetic is paid once per
+// 16 to 32 elements (HBM bound: 64 x 128 x 112 x 112 float32 gradient 846 -> 176 us at 1.03 GB).
+template <typename T> struct Piece;               // 16 bytes of T
+template <> struct Piece<float> {
+  float4 v;
+  __device__ __forceinline__ void max(const Piece& o) {
+    v.x = fmaxf(v.x, o.v.x); v.y = fmaxf(v.y, o.v.y); v.z = fmaxf(v.z, o.v.z); v.w = fmaxf(v.w, o.v.w);
+  }
+  __device__ __forceinline__ static Piece route(const Piece& x, const Piece& y, const Piece& g) {
+    return {make_float4(x.v.x == y.v.x ? g.v.x : 0.f, x.v.y == y.v.y ? g.v.y : 0.f, x.v.z == y.v.z ? g.v.z : 0.f,
+                        x.v.w == y.v.w ? g.v.w : 0.f)};
+  }
+};
+template <> struct Piece<__half> {
+  __align__(16) __half2 v[4];
+  __device__ __forceinline__ void max(const Piece& o) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __hmax2(v[i], o.v[i]);
+  }
+  __device__ __forceinline__ static Piece route(const Piece& x, const Piece& y, const Piece& g) {
+    Piece r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __half z = __float2half(0.f);
+      r.v[i] = __halves2half2(__heq(__low2half(x.v[i]), __low2half(y.v[i])) ? __low2half(g.v[i]) : z,
+                              __heq(__high2half(x.v[i]), __high2half(y.v[i])) ? __high2half(g.v[i]) : z);
+    }
+    return r;
+  }
+};
+template <typename T> __device__ __forceinline__ Piece<T> load_piece(const T* p) { return *reinterpret_cast<const Piece<T>*>(p); }
+
+template <typename T, typename Index>
+__global__ void __launch_bounds__(256) maxpool2x2_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y, Index total,
+                                                              int H, int W, int pieces) {
+  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
+  if (idx >= total) return;
+  const Index Ho = H / 2, Wo = W / 2, Cv = pieces;
+  const Index pix = idx / Cv, row = pix / Wo;
+  const long long Cp = static_cast<long long>(pieces) * V;
+  const int c = static_cast<int>(idx - pix * Cv) * V, ow = static_cast<int>(pix - row * Wo), oh = static_cast<int>(row % Ho);
+  const long long n = row / Ho;
+  const T* p = x + ((n * H + 2 * oh) * W + 2 * ow) * Cp + c;
+  Piece<T> m = load_piece(p);
+  const Piece<T> a = load_piece(p + Cp), b = load_piece(p + W * Cp), d = load_piece(p + W * Cp + Cp);
+  m.max(a); m.max(b); m.max(d);
+  *reinterpret_cast<Piece<T>*>(y + static_cast<long long>(idx) * V) = m;
+}
+
+// The grid covers (H + 1) / 2 x (W + 1) / 2 windows: in an odd-sized image the last row / column belongs to no
+// window and gets zeros.
+template <typename T, typename Index>
+__global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __restrict__ x, const T* __restrict__ y,
+                                                                   const T* __restrict__ gy, T* __restrict__ gx,
+                                                                   Index total, int H, int W, int pieces) {
+  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
+  if (idx >= total) return;
+  const int Ho = H / 2, Wo = W / 2;
+  const Index Hc = (H + 1) / 2, Wc = (W + 1) / 2, Cv = pieces;
+  const Index pix = idx / Cv, row = pix / Wc;
+  const long long Cp = static_cast<long long>(pieces) * V;
+  const int c = static_cast<int>(idx - pix * Cv) * V, ow = static_cast<int>(pix - row * Wc), oh = static_cast<int>(row % Hc);
+  const long long n = row / Hc;
+  const long long base = ((n * H + 2 * oh) * W + 2 * ow) * Cp + c;
+  Piece<T> r[4];
+  memset(r, 0, sizeof r);
+  if (oh < Ho && ow < Wo) {
+    const long long o = ((n * Ho + oh) * Wo + ow) * Cp + c;
+    const Piece<T> m = load_piece(y + o), g = load_piece(gy + o);
+    Piece<T> v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = load_piece(x + base + (k & 1) * Cp + (k >> 1) * W * Cp);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r[k] = Piece<T>::route(v[k], m, g);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (2 * oh + (k >> 1) < H && 2 * ow + (k & 1) < W)
+      *reinterpret_cast<Piece<T>*>(gx + base + (k & 1) * Cp + (k >> 1) * W * Cp) = r[k];
 }
 
 template <typename T>
@@ -633,42 +688,63 @@ cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, 
   return cudaGetLastError();
 }
 
-__global__ void convert_to_half_kernel(const float* __restrict__ src, __half* __restrict__ dst, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dst[i] = __float2half_rn(src[i]);
-}
-cudaError_t launch_convert_to_half(const float* src, void* dst, int n, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  convert_to_half_kernel<<<(n + 255) / 256, 256, 0, s>>>(src, static_cast<__half*>(dst), n);
+namespace {
+// Launches a channels-last pooling kernel with 32-bit indices where they suffice (64-bit divisions cost more
+// than the memory accesses).
+template <typename T, class Launch>
+cudaError_t for_index(long long total, Launch launch) {
+  const long long grid = (total + 255) / 256;
+  if (grid >= (1LL << 31)) return cudaErrorInvalidValue;
+  launch(static_cast<int>(grid), total < (1LL << 31));
   return cudaGetLastError();
 }
+template <typename T>
+cudaError_t maxpool_typed(const T* x, T* y, int N, int C, int H, int W, int nhwc, int Cp, cudaStream_t s) {
+  if (!nhwc) {
+    maxpool2x2_nchw_kernel<T><<<grid_for(1LL * N * C * (H / 2) * (W / 2), 256), 256, 0, s>>>(x, y, 1LL * N * C, H, W);
+    return cudaGetLastError();
+  }
+  const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
+  const long long total = 1LL * N * (H / 2) * (W / 2) * pieces;
+  return for_index<T>(total, [&](int grid, bool small) {
+    if (small) maxpool2x2_nhwc_kernel<T, unsigned><<<grid, 256, 0, s>>>(x, y, static_cast<unsigned>(total), H, W, pieces);
+    else maxpool2x2_nhwc_kernel<T, long long><<<grid, 256, 0, s>>>(x, y, total, H, W, pieces);
+  });
+}
+template <typename T>
+cudaError_t maxpool_grad_typed(const T* x, const T* y, const T* gy, T* gx, int N, int C, int H, int W, int nhwc, int Cp,
+                               cudaStream_t s) {
+  if (!nhwc) {
+    maxpool2x2_grad_nchw_kernel<T><<<grid_for(1LL * N * C * H * W, 256), 256, 0, s>>>(x, y, gy, gx, 1LL * N * C, H, W);
+    return cudaGetLastError();
+  }
+  const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
+  const long long total = 1LL * N * ((H + 1) / 2) * ((W + 1) / 2) * pieces;
+  return for_index<T>(total, [&](int grid, bool small) {
+    if (small)
+      maxpool2x2_grad_nhwc_kernel<T, unsigned><<<grid, 256, 0, s>>>(x, y, gy, gx, static_cast<unsigned>(total), H, W, pieces);
+    else
+      maxpool2x2_grad_nhwc_kernel<T, long long><<<grid, 256, 0, s>>>(x, y, gy, gx, total, H, W, pieces);
+  });
+}
+}  // namespace
 
 cudaError_t launch_maxpool2x2(const void* x, void* y, int N, int C, int H, int W, int nhwc,
                               int Cp, int dtype, cudaStream_t s) {
-  const long long total = 1LL * N * (nhwc ? Cp : C) * (H / 2) * (W / 2);
-  if (total == 0) return cudaSuccess;
+  if (1LL * N * C * (H / 2) * (W / 2) == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    maxpool2x2_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
-        static_cast<const __half*>(x), static_cast<__half*>(y), N, C, H, W, nhwc, Cp);
-  else
-    maxpool2x2_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
-        static_cast<const float*>(x), static_cast<float*>(y), N, C, H, W, nhwc, Cp);
-  return cudaGetLastError();
+    return maxpool_typed(static_cast<const __half*>(x), static_cast<__half*>(y), N, C, H, W, nhwc, Cp, s);
+  return maxpool_typed(static_cast<const float*>(x), static_cast<float*>(y), N, C, H, W, nhwc, Cp, s);
 }
 
 cudaError_t launch_maxpool2x2_grad(const void* x, const void* y, const void* gy, void* gx, int N, int C,
                                    int H, int W, int nhwc, int Cp, int dtype, cudaStream_t s) {
-  const long long total = 1LL * N * (nhwc ? Cp : C) * H * W;
-  if (total == 0) return cudaSuccess;
+  if (1LL * N * C * H * W == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    maxpool2x2_grad_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
-        static_cast<const __half*>(x), static_cast<const __half*>(y), static_cast<const __half*>(gy),
-        static_cast<__half*>(gx), N, C, H, W, nhwc, Cp);
-  else
-    maxpool2x2_grad_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
-        static_cast<const float*>(x), static_cast<const float*>(y), static_cast<const float*>(gy),
-        static_cast<float*>(gx), N, C, H, W, nhwc, Cp);
-  return cudaGetLastError();
+    return maxpool_grad_typed(static_cast<const __half*>(x), static_cast<const __half*>(y), static_cast<const __half*>(gy),
+                              static_cast<__half*>(gx), N, C, H, W, nhwc, Cp, s);
+  return maxpool_grad_typed(static_cast<const float*>(x), static_cast<const float*>(y), static_cast<const float*>(gy),
+                            static_cast<float*>(gx), N, C, H, W, nhwc, Cp, s);
 }
 
 cudaError_t launch_pack_filters_merged(const void* w, void* dst, int K, int C, int kH, int kW, int flip,
