@@ -10,8 +10,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <initializer_list>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "internal.h"
@@ -48,6 +50,47 @@ struct b200conv_graph {
 constexpr size_t kRingSlotBytes = 2u << 20;    // 2 MB: 27 us to copy with 8 threads, 41 us on the link
 constexpr int kRingSlots = 16;
 constexpr size_t kSmallInput = 64u << 10;      // inputs up to this size share one slot and one transfer
+
+// Key of what the context remembers per geometry: a kind and up to 23 integers.  Looked up on every call,
+// so it is compared and hashed as integers (text keys cost 1.5 us of the host's 10 us per call).
+struct GeoKey {
+  int n = 0;
+  int v[24];
+  GeoKey(std::initializer_list<int> l) {
+    for (int x : l) v[n++] = x;
+  }
+  void add(long long x) { v[n++] = static_cast<int>(x); }
+  bool operator==(const GeoKey& o) const { return n == o.n && !memcmp(v, o.v, sizeof(int) * n); }
+  std::string text() const {
+    std::string t;
+    for (int i = 0; i < n; ++i) t += (i ? "." : "") + std::to_string(v[i]);
+    return t;
+  }
+  static bool parse(const char* t, GeoKey* k) {
+    k->n = 0;
+    while (*t && k->n < 24) {
+      char* end;
+      k->v[k->n++] = static_cast<int>(strtol(t, &end, 10));
+      if (end == t) return false;
+      t = *end == '.' ? end + 1 : end;
+    }
+    return !*t && k->n > 0;
+  }
+};
+struct GeoHash {
+  size_t operator()(const GeoKey& k) const {
+    uint64_t h = 1469598103934665603ull;
+    for (int i = 0; i < k.n; ++i) h = (h ^ static_cast<uint32_t>(k.v[i])) * 1099511628211ull;
+    return h ^ (h >> 29);
+  }
+};
+enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance };      // kinds (first integer of a key)
+
+// Tile of the slab kernel for one geometry (the result of the search in try_conv_slab).
+struct SlabTile {
+  int wt = 0, th = 0, nb = 0, n_acc = 0, slab_bytes = 0;
+  bool found = false;
+};
 
 struct b200conv_ctx {
   int device = 0;
@@ -89,9 +132,12 @@ struct b200conv_ctx {
   long long* trace = nullptr;               // debug: phase stamps of the slab kernel
   ConvEpilogue epi = default_epilogue();    // epilogue of the forward call in progress
   // forward / gradInputs kernel choice per geometry (true = slab kernel), filled by timing
-  std::map<std::string, bool> algo_cache;
+  std::unordered_map<GeoKey, int, GeoHash> algo_cache;
   // gradWeights split-K slice count per geometry and kernel, chosen by timing
-  std::map<std::string, int> split_cache;
+  std::unordered_map<GeoKey, int, GeoHash> split_cache;
+  // tiles found by search: the same on every call of a geometry, and the search costs 2 to 30 us
+  std::unordered_map<GeoKey, SlabTile, GeoHash> slab_tiles;
+  std::unordered_map<GeoKey, SlabTile, GeoHash> pixel_tiles;
   int force_splits = 0;                     // > 0: use this slice count (tests, tuning by hand)
   bool use_pair = true;                     // 1x1 layers with deep reductions on CTA pairs (gemm_pair.cu)
   bool stack_taps = true;                   // grouped gradWeights of narrow layers: taps as column groups of one MMA
@@ -355,7 +401,12 @@ int validate(b200conv_ctx* c, const b200conv_desc* d) {
 
 // Pixel tile for a grid of Wt x Ht x N positions holding at most `cap` rows: fewest tiles,
 // each tile weighted by the MMA steps it costs (`kk` rows per step); widest box on ties.
-void choose_tile(int Wt, int Ht, int N, int cap, int kk, int* bw, int* bh, int* bn) {
+void choose_tile(b200conv_ctx* c, int Wt, int Ht, int N, int cap, int kk, int* bw, int* bh, int* bn) {
+  SlabTile& memo = c->pixel_tiles[GeoKey{kGeoTile, Wt, Ht, N, cap, kk}];
+  if (memo.found) {
+    *bw = memo.wt; *bh = memo.th; *bn = memo.nb;
+    return;
+  }
   long long best = -1;
   *bw = *bh = *bn = 1;
   for (int w = 1; w <= std::min(Wt, cap); ++w) {
@@ -369,6 +420,8 @@ void choose_tile(int Wt, int Ht, int N, int cap, int kk, int* bw, int* bh, int* 
       }
     }
   }
+  memo.wt = *bw; memo.th = *bh; memo.nb = *bn;
+  memo.found = true;
 }
 
 // 5-D channels-last view (c_in_group, group, w, h, n) of a [N][Hs][Ws][Cp] tensor that keeps
@@ -437,7 +490,10 @@ struct FwdLikeArgs {
   int Hs, Ws, Cin_g, Cp_in;
   const void* wpacked;   // [(tap*groups+g)][n_out][ld_w]
   int ld_w, nmats;
-  int n_out, groups, N;
+  int n_out, groups, N;  // n_out: output channels per group as stored: a channels-last output of one group
+                         // includes its pad channels, so that whole 16-byte pieces leave and no separate
+                         // launch has to zero them
+  int w_rows;            // rows of a packed filter matrix (the rows up to n_out read as zero)
   int dtype;
   int view_sH, view_sW;  // parity pitch of the activation views
   // Row folding (few input channels): `act` is [N][Hs][fold_Wp][Cp_in] with explicit zero columns;
@@ -524,7 +580,15 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   const bool tma_layout_ok = sc == 1 && a.n_out % (int)(128 / es_out) == 0 && !c->epi.residual &&
                              (sw * es_out) % 16 == 0 && (sh * es_out) % 16 == 0 && (sn * es_out) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es_out) % 16 == 0;
-  for (int parts = 1; parts <= 16; ++parts) {
+  GeoKey tile_key{kGeoSlab, a.dtype, a.n_out, a.Cin_g, a.groups, a.N, Wt, Ht, ntap_all, Eh, Ew, tma_layout_ok ? 1 : 0,
+                  c->epi.pool, c->num_sms};
+  auto known = c->slab_tiles.find(tile_key);
+  if (known != c->slab_tiles.end() && known->second.found) {
+    const SlabTile& k = known->second;
+    b_wt = k.wt; b_th = k.th; b_nb = k.nb; b_acc = k.n_acc; b_slab = k.slab_bytes;
+    best_cost = 0;
+  }
+  for (int parts = 1; parts <= 16 && known == c->slab_tiles.end(); ++parts) {
     const int wt = (int)cdiv(Wt, parts);
     if (parts > 1 && wt < 8) break;
     const int Ws = wt + Ew;
@@ -576,6 +640,11 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       }
     }
   }
+  if (known == c->slab_tiles.end()) {
+    SlabTile& k = c->slab_tiles[tile_key];
+    k.wt = b_wt; k.th = b_th; k.nb = b_nb; k.n_acc = b_acc; k.slab_bytes = b_slab;
+    k.found = best_cost >= 0;
+  }
 #ifndef B200_PAIR_MIN_KBLOCKS
 #define B200_PAIR_MIN_KBLOCKS 4
 #endif
@@ -589,7 +658,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     memset(&q, 0, sizeof q);
     int rc = make_act_view(c, &q.view, a, rh, rw, 64, 128, 1, 1);
     if (rc) return rc;
-    if ((rc = make_wmap(c, &q.wmap, a.wpacked, a.dtype, a.Cin_g, a.n_out, a.nmats, a.ld_w, 64, 128))) return rc;
+    if ((rc = make_wmap(c, &q.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, 64, 128))) return rc;
     cuuint64_t dims[4] = {(cuuint64_t)a.n_out, (cuuint64_t)Wt, 1, 1};
     cuuint64_t strides[3] = {(cuuint64_t)(sw * es_out), (cuuint64_t)(sh * es_out), (cuuint64_t)(sn * es_out)};
     cuuint32_t box[4] = {64, 128, 1, 1};
@@ -711,7 +780,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   int rc = make_act_view(c, &p.view, a, rh, rw, kBK, p.Ws, p.Hs, p.nb);
   if (rc) return rc;
-  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.n_out, a.nmats, a.ld_w, kBK, BN);
+  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN);
   if (rc) return rc;
   for (const ConvTap& t : taps) {
     p.tap_shift[p.ntaps] = (int16_t)((t.dh - dh_min) * p.Ws + (t.dw - dw_min));
@@ -756,7 +825,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   UmmaConvParams p;
   memset(&p, 0, sizeof p);
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
-  choose_tile(Wt, Ht, a.N, 128, 0, &p.bw, &p.bh, &p.bn);
+  choose_tile(c, Wt, Ht, a.N, 128, 0, &p.bw, &p.bh, &p.bn);
   // views that exist (non-empty); taps pointing at empty views contribute nothing
   std::vector<int> remap(view_parity.size(), -1);
   int nviews = 0;
@@ -776,7 +845,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   if (p.ntaps == 0) return 1;  // caller zero-fills
   for (int v = nviews; v < kMaxViews; ++v) p.views[v] = p.views[0];
   const int BN = conv_umma_bn(a.n_out);
-  int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.n_out, a.nmats, a.ld_w, kBK, BN);
+  int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN);
   if (rc) return rc;
   p.kblocks = static_cast<int>(cdiv(a.Cin_g, kBK));
   p.groups = a.groups;
@@ -815,11 +884,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   if (!allow_slab || view_parity.size() != 1 || !c->autotune)
     return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, allow_slab);
-  char key[256];
   int tsum = 0;
   for (const ConvTap& t : taps_in) tsum = tsum * 31 + t.dh * 7 + t.dw;
-  snprintf(key, sizeof key, "%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%zu.%d.%lld.%lld", a.dtype, a.N, a.Hs, a.Ws,
-           a.Cin_g, a.n_out, a.groups, Wt, Ht, a.view_sH, a.view_sW, taps_in.size(), tsum, sc, sw);
+  GeoKey key{kGeoConv, a.dtype, a.N, a.Hs, a.Ws, a.Cin_g, a.n_out, a.groups, Wt, Ht, a.view_sH, a.view_sW, (int)taps_in.size(), tsum};
+  key.add(sc);
+  key.add(sw);
   auto it = c->algo_cache.find(key);
   if (it != c->algo_cache.end())
     return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, it->second);
@@ -980,6 +1049,13 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     bias_f = f;
     return 0;
   };
+  if (bias && out_nhwc && Kp != d.K) {           // the epilogue reads one value per stored channel
+    void* padded;
+    int rc = tmp.get(es * Kp, &padded);
+    if (rc) return rc;
+    KLAUNCH(c, kKPack, launch_pad_bias(bias, padded, d.K, Kp, d.dtype, c->stream));
+    bias = padded;
+  }
   const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor(d);
   if (mg > 1) {
     b200conv_desc dm = d;
@@ -1026,14 +1102,13 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     FwdLikeArgs a;
     a.act = xs; a.Hs = H2; a.Ws = d.Wo; a.Cin_g = win; a.Cp_in = kS2dChannels;
     a.wpacked = wf; a.ld_w = win; a.nmats = s2_nt;
-    a.n_out = d.K; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
+    a.n_out = out_nhwc ? Kp : d.K; a.w_rows = d.K; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
     a.view_sH = 1; a.view_sW = 1;
     a.fold = true; a.fold_Wp = Wq; a.fold_sW = 1;
     long long sn, sc, sh, sw;
     if (out_nhwc) {
       const int pl = c->epi.pool ? 2 : 1;
       sn = 1LL * (d.Ho / pl) * (d.Wo / pl) * Kp; sc = 1; sh = 1LL * (d.Wo / pl) * Kp; sw = Kp;
-      if (Kp != d.K) CU_OK(c, cudaMemsetAsync(y, 0, es * (size_t)d.N * (d.Ho / pl) * (d.Wo / pl) * Kp, c->stream));
     } else {
       sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
     }
@@ -1069,14 +1144,13 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     FwdLikeArgs a;
     a.act = xp; a.Hs = d.H; a.Ws = d.Wo; a.Cin_g = kBK; a.Cp_in = Cp;
     a.wpacked = wf; a.ld_w = kBK; a.nmats = d.kH;
-    a.n_out = d.K; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
+    a.n_out = out_nhwc ? Kp : d.K; a.w_rows = d.K; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
     a.view_sH = d.sH; a.view_sW = 1;
     a.fold = true; a.fold_Wp = Wp; a.fold_sW = d.sW;
     long long sn, sc, sh, sw;
     if (out_nhwc) {
       const int pl = c->epi.pool ? 2 : 1;
       sn = 1LL * (d.Ho / pl) * (d.Wo / pl) * Kp; sc = 1; sh = 1LL * (d.Wo / pl) * Kp; sw = Kp;
-      if (Kp != d.K) CU_OK(c, cudaMemsetAsync(y, 0, es * (size_t)d.N * (d.Ho / pl) * (d.Wo / pl) * Kp, c->stream));
     } else {
       sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
     }
@@ -1124,13 +1198,12 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   FwdLikeArgs a;
   a.act = xin; a.Hs = d.H; a.Ws = d.W; a.Cin_g = Cg; a.Cp_in = Cp;
   a.wpacked = wp; a.ld_w = ldw; a.nmats = d.kH * d.kW * d.groups;
-  a.n_out = Kg; a.groups = d.groups; a.N = d.N; a.dtype = d.dtype;
+  a.n_out = out_nhwc && d.groups == 1 ? Kp : Kg; a.w_rows = Kg; a.groups = d.groups; a.N = d.N; a.dtype = d.dtype;
   a.view_sH = d.sH; a.view_sW = d.sW;
   long long sn, sc, sh, sw;
   if (out_nhwc) {
     const int pl = c->epi.pool ? 2 : 1;
     sn = 1LL * (d.Ho / pl) * (d.Wo / pl) * Kp; sc = 1; sh = 1LL * (d.Wo / pl) * Kp; sw = Kp;
-    if (Kp != d.K) CU_OK(c, cudaMemsetAsync(y, 0, es * (size_t)d.N * (d.Ho / pl) * (d.Wo / pl) * Kp, c->stream));
   } else {
     sn = 1LL * d.K * d.Ho * d.Wo; sc = 1LL * d.Ho * d.Wo; sh = d.Wo; sw = 1;
   }
@@ -1193,7 +1266,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
   // the taps with (h0 + padH_l - i*dilH) divisible by sH (same for columns).
   struct Cls { int h0, w0, Ht, Wt; std::vector<ConvTap> taps; };
   std::vector<Cls> classes;
-  bool need_zero = out_nhwc && Cp != d.C;
+  bool need_zero = out_nhwc && Cp != d.C && d.groups > 1;
   for (int h0 = 0; h0 < d.sH; ++h0)
     for (int w0 = 0; w0 < d.sW; ++w0) {
       Cls k;
@@ -1252,7 +1325,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       FwdLikeArgs a;
       a.act = gin; a.Hs = d.Ho; a.Ws = d.Wo; a.Cin_g = Kg; a.Cp_in = Kp;
       a.wpacked = wp; a.ld_w = ldw; a.nmats = nu;
-      a.n_out = n_out; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
+      a.n_out = a.w_rows = n_out; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
       a.view_sH = 1; a.view_sW = 1;
       std::vector<std::pair<int, int>> parity(1, {0, 0});
       rc = run_conv_umma(c, a, utaps, parity, Wq, Hq, merged, 1LL * Hq * Wq * Ct, 1, 1LL * Wq * Ct, Ct, 0,
@@ -1273,7 +1346,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
   FwdLikeArgs a;
   a.act = gin; a.Hs = d.Ho; a.Ws = d.Wo; a.Cin_g = Kg; a.Cp_in = Kp;
   a.wpacked = wp; a.ld_w = ldw; a.nmats = d.kH * d.kW * d.groups;
-  a.n_out = Cg; a.groups = d.groups; a.N = d.N; a.dtype = d.dtype;
+  a.n_out = out_nhwc && d.groups == 1 ? Cp : Cg; a.w_rows = Cg; a.groups = d.groups; a.N = d.N; a.dtype = d.dtype;
   a.view_sH = 1; a.view_sW = 1;
   std::vector<std::pair<int, int>> parity(1, {0, 0});
   for (const Cls& k : classes) {
@@ -1314,6 +1387,16 @@ static long long balanced_splits(long long pix_tiles, long long base_items, int 
   return best;
 }
 
+// The same, remembered (the loop above runs up to 444 times).
+long long balanced_splits(b200conv_ctx* c, long long pix_tiles, long long base_items, int sms, long long cap, long long fixed) {
+  SlabTile& memo = c->pixel_tiles[GeoKey{kGeoBalance, (int)pix_tiles, (int)base_items, sms, (int)cap, (int)fixed}];
+  if (!memo.found) {
+    memo.wt = (int)balanced_splits(pix_tiles, base_items, sms, cap, fixed);
+    memo.found = true;
+  }
+  return memo.wt;
+}
+
 int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const void* dy, void* dw,
                  int flags);
 
@@ -1331,13 +1414,16 @@ int valid_splits(long long pix_tiles, long long s) {
 // GPU back end gives its meta-optimizer (theano/gpuarray/opt.py:2144-2222).  `run(splits, scratch)`
 // enqueues the launch.  Returns the count, or a negative error code.
 template <class Run>
-int pick_splits(b200conv_ctx* c, const std::string& key, long long pix_tiles, long long cap, int s0, Run run) {
+int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long long cap, long long base_items, int sms,
+                long long fixed, Run run) {
   cap = std::max(1LL, std::min(cap, pix_tiles));
   if (c->force_splits > 0) return valid_splits(pix_tiles, std::min<long long>(c->force_splits, cap));
-  if (!c->autotune) return s0;
-  auto it = c->split_cache.find(key);
-  if (it != c->split_cache.end()) return it->second;
-  if (c->capturing) return s0;
+  if (c->autotune) {
+    auto it = c->split_cache.find(key);
+    if (it != c->split_cache.end()) return it->second;
+  }
+  const int s0 = (int)balanced_splits(c, pix_tiles, base_items, sms, cap, fixed);
+  if (!c->autotune || c->capturing) return s0;
   int cand[3] = {s0, valid_splits(pix_tiles, std::min<long long>(cap, std::max(1, s0 / 2))),
                  valid_splits(pix_tiles, std::min<long long>(cap, 2LL * s0))};
   if (!c->ev_tune0) {
@@ -1362,6 +1448,11 @@ int pick_splits(b200conv_ctx* c, const std::string& key, long long pix_tiles, lo
   }
   c->split_cache[key] = best;
   return best;
+}
+
+GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
+  return GeoKey{kind, d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.Ho, d.Wo,
+                d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : 0))};
 }
 
 // gradWeights with tap groups (wgrad_group.cu).  Returns 0 when launched, 2 when the geometry is
@@ -1473,8 +1564,6 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
   p.taps_total = d.kH * d.kW;
   const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
   const long long base_items = 1LL * p.ktiles * p.ctiles * d.groups * p.ngroups;
-  // accumulators are not double buffered: aim at one item per SM
-  const int s0 = (int)balanced_splits(pix_tiles, base_items, c->num_sms, pix_tiles, 6);
   p.atomic = (flags & B200CONV_ATOMIC_SPLITK) ? 1 : 0;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
@@ -1495,10 +1584,10 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
                                                   (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, c->stream));
     return 0;
   };
-  char skey[220];
-  snprintf(skey, sizeof skey, "sg.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d", d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH,
-           d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.groups, flags & (B200CONV_ATOMIC_SPLITK | B200CONV_DW_F32));
-  const int splits = pick_splits(c, skey, pix_tiles, pix_tiles, s0, run);
+  GeoKey skey = wgrad_key(kGeoSplits, d, flags);
+  skey.add(0);
+  // accumulators are not double buffered: aim at one item per SM
+  const int splits = pick_splits(c, skey, pix_tiles, pix_tiles, base_items, c->num_sms, 6, run);
   if (splits < 0) return splits;
   if ((rc = run(splits, tmp))) return rc;
   c->last_algo = "umma";
@@ -1567,7 +1656,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     UmmaWgradParams p;
     memset(&p, 0, sizeof p);
     const int atom = kBK;
-    choose_tile(d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
+    choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
     const bool swz32 = d.dtype == B200CONV_F32;
     if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
                         p.bn, swz32)))
@@ -1598,7 +1687,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     p.taps_total = s2_nt;
     const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const long long base_items = 1LL * p.ktiles * p.ntaps;
-    p.splits = (int)balanced_splits(pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
+    p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
     const size_t slab_elems = (size_t)s2_nt * d.K * win;
     float* partial;
     if ((rc = tmp.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
@@ -1631,7 +1720,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     UmmaWgradParams p;
     memset(&p, 0, sizeof p);
     const int atom = kBK;
-    choose_tile(d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
+    choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
     const bool swz32 = d.dtype == B200CONV_F32;
     if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
                         p.bn, swz32)))
@@ -1674,7 +1763,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     p.taps_total = d.kH;
     const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
     const long long base_items = 1LL * p.ktiles * std::max(1, p.ntaps);
-    p.splits = (int)balanced_splits(pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
+    p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
     const size_t slab_elems = (size_t)d.kH * d.K * kBK;
     float* partial;
     if ((rc = tmp.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
@@ -1698,9 +1787,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   // Two tensor-core kernels: tap groups sharing operands, or one tap per work item.  As for the
   // forward kernels the first call of a geometry times both and the context remembers the winner.
   bool try_group = !(flags & B200CONV_NO_GROUP);
-  char key[200];
-  snprintf(key, sizeof key, "w.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d", d.dtype, d.N, d.C, d.H, d.W,
-           d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.groups, flags & B200CONV_ATOMIC_SPLITK);
+  const GeoKey key = wgrad_key(kGeoWgrad, d, flags);
   // without timings: the one-tap kernel where it runs 256-column MMAs (their issue and TMA
   // budgets are comfortable), tap groups for narrower layers (they read the operands 3x less)
   if (try_group && !c->autotune && d.C / d.groups >= 256) try_group = false;
@@ -1747,7 +1834,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   const int atom = d.dtype == B200CONV_F16 ? 64 : 32;
   const int kk = d.dtype == B200CONV_F16 ? 16 : 8;
   const int BN = Cg <= 64 ? 64 : Cg <= 128 ? 128 : 256;
-  choose_tile(d.Wo, d.Ho, d.N, wgrad_pix(d.dtype, BN), kk, &p.bw, &p.bh, &p.bn);
+  choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype, BN), kk, &p.bw, &p.bh, &p.bn);
   const bool swz32 = d.dtype == B200CONV_F32;  // MN-major tf32 operands need 32-byte swizzle atoms
   rc = make_view(c, &p.dy_map, gin, d.dtype, Kg, d.groups, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom,
                  p.bw, p.bh, p.bn, swz32);
@@ -1793,7 +1880,6 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   p.taps_total = d.kH * d.kW;
   const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
   const long long base_items = 1LL * p.ktiles * p.ctiles * d.groups * std::max(1, p.ntaps);
-  const int s0 = (int)balanced_splits(pix_tiles, base_items, pair ? c->num_sms / 2 : c->num_sms, pix_tiles / 4, 2);
   p.atomic = (flags & B200CONV_ATOMIC_SPLITK) ? 1 : 0;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
@@ -1816,10 +1902,9 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, odt, c->stream));
     return 0;
   };
-  char skey[220];
-  snprintf(skey, sizeof skey, pair ? "sp.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d" : "su.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d.%d", d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH,
-           d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.groups, flags & (B200CONV_ATOMIC_SPLITK | B200CONV_DW_F32));
-  const int splits = pick_splits(c, skey, pix_tiles, std::max(1LL, pix_tiles / 4), s0, run);
+  GeoKey skey = wgrad_key(kGeoSplits, d, flags);
+  skey.add(pair ? 2 : 1);
+  const int splits = pick_splits(c, skey, pix_tiles, std::max(1LL, pix_tiles / 4), base_items, pair ? c->num_sms / 2 : c->num_sms, 2, run);
   if (splits < 0) return splits;
   if ((rc = run(splits, tmp))) return rc;
   c->last_algo = "umma";
@@ -2696,8 +2781,8 @@ int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
   FILE* f = fopen(path, "w");
   if (!f) return fail(c, B200CONV_E_INVALID, "cannot write %s", path);
   fprintf(f, "%s\n", tuning_header(c).c_str());
-  for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.c_str(), kv.second ? 1 : 0);
-  for (auto& kv : c->split_cache) fprintf(f, "s %s %d\n", kv.first.c_str(), kv.second);
+  for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.text().c_str(), kv.second ? 1 : 0);
+  for (auto& kv : c->split_cache) fprintf(f, "s %s %d\n", kv.first.text().c_str(), kv.second);
   fclose(f);
   return 0;
 }
@@ -2722,9 +2807,10 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
     return fail(c, B200CONV_E_INVALID, "%s was not written for this device and SM count", path);
   }
   while (fgets(line, sizeof line, f)) {
-    char kind = 0, key[400];
+    char kind = 0, text[400];
     int val = 0;
-    if (sscanf(line, "%c %399s %d", &kind, key, &val) != 3) continue;
+    GeoKey key{};
+    if (sscanf(line, "%c %399s %d", &kind, text, &val) != 3 || !GeoKey::parse(text, &key)) continue;
     if (kind == 'a') { c->algo_cache[key] = val != 0; ++n; }
     else if (kind == 's' && val >= 1) { c->split_cache[key] = val; ++n; }
   }
@@ -3003,7 +3089,7 @@ extern "C" int b200conv_wgrad_static(b200conv_ctx* c, const b200conv_desc* dp, c
   const int kk = d.dtype == B200CONV_F16 ? 16 : 8;
   const bool swz32 = d.dtype == B200CONV_F32;
   const int BN = Cg <= 64 ? 64 : Cg <= 128 ? 128 : 256;
-  choose_tile(d.Wo, d.Ho, d.N, wgrad_pix(d.dtype, BN), kk, &p.bw, &p.bh, &p.bn);
+  choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype, BN), kk, &p.bw, &p.bh, &p.bn);
   if ((rc = make_view(c, &p.dy_map, dy, d.dtype, Kg, d.groups, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom,
                       p.bw, p.bh, p.bn, swz32)))
     return rc;
@@ -3045,7 +3131,7 @@ extern "C" int b200conv_wgrad_static(b200conv_ctx* c, const b200conv_desc* dp, c
   p.taps_total = d.kH * d.kW;
   const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
   const long long base_items = 1LL * p.ktiles * p.ctiles * d.groups * std::max(1, p.ntaps);
-  p.splits = (int)balanced_splits(pix_tiles, base_items, c->num_sms,
+  p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms,
                                   std::min<long long>(pix_tiles / 4, (long long)(kStaticScratchBytes / slab_bytes)), 2);
   p.atomic = (flags & B200CONV_ATOMIC_SPLITK) ? 1 : 0;
   const int slabs = p.atomic ? 1 : p.splits;

@@ -290,6 +290,8 @@ cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits,
 // Block-diagonal filters for merged groups (extract = 0) and the inverse for the gradient (1).
 cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int Kg, int m, int taps,
                                 int extract, int dtype, cudaStream_t s);
+// n values followed by zeros up to np values.
+cudaError_t launch_pad_bias(const void* bias, void* dst, int n, int np, int dtype, cudaStream_t s);
 cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, cudaStream_t s);
 cudaError_t launch_maxpool2x2(const void* x, void* y, int N, int C, int H, int W, int nhwc,
                               int Cp, int dtype, cudaStream_t s);

@@ -679,6 +679,21 @@ cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int K
   return cudaGetLastError();
 }
 
+namespace {
+template <typename T>
+__global__ void pad_bias_kernel(const T* __restrict__ b, T* __restrict__ dst, int n, int np) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < np) dst[i] = i < n ? b[i] : T(0);
+}
+}  // namespace
+cudaError_t launch_pad_bias(const void* bias, void* dst, int n, int np, int dtype, cudaStream_t s) {
+  if (dtype == B200CONV_F16)
+    pad_bias_kernel<<<(np + 255) / 256, 256, 0, s>>>(static_cast<const __half*>(bias), static_cast<__half*>(dst), n, np);
+  else
+    pad_bias_kernel<<<(np + 255) / 256, 256, 0, s>>>(static_cast<const float*>(bias), static_cast<float*>(dst), n, np);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)

@@ -10,6 +10,7 @@ plus the ``filter_flip`` of the abstract ops they are lowered from
 (theano/tensor/nnet/abstract_conv.py:2454,2737,3041).
 """
 import ctypes
+import math
 import os
 import threading
 
@@ -22,6 +23,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("B200CONV_LIB") or os.path.join(_HERE, "libb200conv.so")
 
 F32, F16 = 0, 1
+_F32T, _F16T = np.dtype(np.float32), np.dtype(np.float16)
 HOST_PTRS, RELU, IN_NHWC, OUT_NHWC, IN2_NHWC = 1, 2, 4, 8, 16
 FORCE_DIRECT, FORCE_UMMA, ATOMIC_SPLITK, NO_SLAB, NO_GROUP, NO_MERGE_PARITY, NO_S2D = 32, 64, 128, 256, 512, 1024, 2048
 DW_F32 = 4096
@@ -122,15 +124,20 @@ def load_library():
     return _lib
 
 
+def _ref(desc):
+    """A descriptor as a C pointer argument; ready references pass through."""
+    return ctypes.byref(desc) if isinstance(desc, Desc) else desc
+
+
 class B200Error(RuntimeError):
     pass
 
 
 def _dtype_code(dt):
     dt = np.dtype(dt)
-    if dt == np.float32:
+    if dt is _F32T or dt == _F32T:
         return F32
-    if dt == np.float16:
+    if dt is _F16T or dt == _F16T:
         return F16
     raise TypeError("b200conv handles float32 and float16, not %s" % dt)
 
@@ -299,17 +306,22 @@ class Context(object):
         """y = act(alpha * conv + bias + beta * residual); the plain entry point when the
         epilogue is the default one."""
         if residual is None and alpha == 1.0 and slope == 0.0:
-            self.check(self.lib.b200conv_fwd(self.h, ctypes.byref(desc), _P(x), _P(w), _P(bias), _P(y), flags))
+            rc = self.lib.b200conv_fwd(self.h, _ref(desc), x, w, bias, y, flags)
         else:
-            self.check(self.lib.b200conv_fwd_epilogue(self.h, ctypes.byref(desc), _P(x), _P(w), _P(bias),
-                                                      _P(residual), _P(y), float(alpha), float(beta),
-                                                      float(slope), flags))
+            rc = self.lib.b200conv_fwd_epilogue(self.h, _ref(desc), x, w, bias, residual, y, float(alpha), float(beta),
+                                                float(slope), flags)
+        if rc:
+            self.check(rc)
 
     def dgrad(self, desc, w, dy, dx, flags):
-        self.check(self.lib.b200conv_dgrad(self.h, ctypes.byref(desc), _P(w), _P(dy), _P(dx), flags))
+        rc = self.lib.b200conv_dgrad(self.h, _ref(desc), w, dy, dx, flags)
+        if rc:
+            self.check(rc)
 
     def wgrad(self, desc, x, dy, dw, flags):
-        self.check(self.lib.b200conv_wgrad(self.h, ctypes.byref(desc), _P(x), _P(dy), _P(dw), flags))
+        rc = self.lib.b200conv_wgrad(self.h, _ref(desc), x, dy, dw, flags)
+        if rc:
+            self.check(rc)
 
     def wgrad_static(self, desc, x_nhwc, dy_nhwc, dw, flags=0):
         """gradWeights that allocates nothing (fixed scratch inside the library); device pointers,
@@ -535,8 +547,73 @@ def make_desc(xshape, wshape, yshape, pads, subsample, dilation, groups, flip, d
     return d
 
 
+class _Plans(dict):
+    """Results of the pure shape logic per call signature: (result shape, pads or kernel shape, descriptor
+    reference).  A training loop repeats a few signatures for ever, and working them out again cost as
+    much host time as the launches.  Bounded: emptied when it holds LIMIT signatures."""
+    LIMIT = 4096
+
+    def find(self, make, *sig):
+        try:
+            return self[sig]
+        except KeyError:
+            pass
+        except TypeError:                # a list among the arguments: not remembered
+            return make(*sig[1:])
+        plan = make(*sig[1:])
+        if len(self) >= self.LIMIT:
+            self.clear()
+        self[sig] = plan
+        return plan
+
+
+_plans = _Plans()
+
+
+def _plan_forward(xs, ws, border_mode, subsample, dilation, groups, flip, dtype):
+    yshape, pads = hostlogic.forward_shape(xs, ws, border_mode, subsample, dilation, groups)
+    return yshape, ctypes.byref(make_desc(xs, ws, yshape, pads, subsample, dilation, groups, flip, dtype))
+
+
+def _plan_grad_weights(xs, dys, kshape, border_mode, subsample, dilation, groups, flip, dtype):
+    if len(xs) != 4:
+        raise TypeError("img must be 4D tensor")
+    if len(dys) != 4:
+        raise TypeError("topgrad must be 4D tensor")
+    ksz = hostlogic.gradweights_kshape(xs, dys, border_mode, subsample, dilation, kshape)
+    if xs[1] % groups:
+        raise ValueError("CorrMM images and kernel must have the same stack size")
+    wshape = (dys[1], xs[1] // groups) + ksz
+    pads = hostlogic.resolve_pads(border_mode, ksz, dilation)
+    hostlogic.check_consistent(xs, wshape, dys, pads, subsample, dilation, groups)
+    return wshape, ctypes.byref(make_desc(xs, wshape, dys, pads, subsample, dilation, groups, flip, dtype))
+
+
+def _plan_grad_inputs(ws, dys, imshape, border_mode, subsample, dilation, groups, flip, dtype):
+    if len(ws) != 4:
+        raise TypeError("kern must be 4D tensor")
+    if len(dys) != 4:
+        raise TypeError("topgrad must be 4D tensor")
+    hw, pads = hostlogic.gradinputs_imshape(ws, dys, border_mode, subsample, dilation, imshape)
+    xshape = (dys[0], ws[1] * groups) + hw
+    hostlogic.check_consistent(xshape, ws, dys, pads, subsample, dilation, groups)
+    return xshape, ctypes.byref(make_desc(xshape, ws, dys, pads, subsample, dilation, groups, flip, dtype))
+
+
+def _key(pair):
+    """A size pair as part of a plan's signature (lists and arrays become tuples)."""
+    return pair if pair is None or type(pair) is tuple else tuple(pair)
+
+
+def _address(a):
+    return a.__array_interface__["data"][0]
+
+
 def _common(a, b):
     """Upcast like BaseCorrMM.as_common_dtype (corr.py:156-162); float64 is not handled here."""
+    if a.dtype is b.dtype and a.flags.c_contiguous and b.flags.c_contiguous:
+        _dtype_code(a.dtype)
+        return a, b
     dt = np.promote_types(a.dtype, b.dtype)
     _dtype_code(dt)
     return np.ascontiguousarray(a, dtype=dt), np.ascontiguousarray(b, dtype=dt)
@@ -553,13 +630,13 @@ def conv2d_forward(x, w, border_mode="valid", subsample=(1, 1), filter_dilation=
     `relu` (slope 0: ReLU), else the identity.  x: [N,C,H,W], w: [K,C/g,kH,kW]; returns
     [N,K,Ho,Wo]."""
     x, w = _common(np.asarray(x), np.asarray(w))
-    yshape, pads = hostlogic.forward_shape(x.shape, w.shape, border_mode, subsample, filter_dilation, num_groups)
+    yshape, d = _plans.find(_plan_forward, "fwd", x.shape, w.shape, border_mode, subsample, filter_dilation,
+                            num_groups, filter_flip, x.dtype)
     ctx = ctx or get_context()
     if out is None or out.shape != yshape or out.dtype != x.dtype or not out.flags.c_contiguous:
         out = _results.empty(ctx, yshape, x.dtype)
     if out.size == 0:
         return out
-    d = make_desc(x.shape, w.shape, yshape, pads, subsample, filter_dilation, num_groups, filter_flip, x.dtype)
     b = None
     if bias is not None:
         b = np.ascontiguousarray(bias, dtype=x.dtype)
@@ -570,9 +647,9 @@ def conv2d_forward(x, w, border_mode="valid", subsample=(1, 1), filter_dilation=
         r = np.ascontiguousarray(residual, dtype=x.dtype)
         if r.shape != yshape:
             raise ValueError("residual must have the shape of the output %s, not %s" % (yshape, r.shape))
-    ctx.fwd(d, x.ctypes.data, w.ctypes.data, b.ctypes.data if b is not None else None,
-            out.ctypes.data, flags | HOST_PTRS | (RELU if relu else 0),
-            residual=r.ctypes.data if r is not None else None, alpha=alpha, beta=beta, slope=slope)
+    ctx.fwd(d, _address(x), _address(w), _address(b) if b is not None else None,
+            _address(out), flags | HOST_PTRS | (RELU if relu else 0),
+            residual=_address(r) if r is not None else None, alpha=alpha, beta=beta, slope=slope)
     return out
 
 
@@ -581,23 +658,14 @@ def conv2d_grad_weights(x, dy, kshape=None, border_mode="valid", subsample=(1, 1
                         flags=0):
     """AbstractConv2d_gradWeights: x [N,C,H,W], dy [N,K,Ho,Wo] -> dw [K,C/g,kH,kW]."""
     x, dy = _common(np.asarray(x), np.asarray(dy))
-    if x.ndim != 4:
-        raise TypeError("img must be 4D tensor")
-    if dy.ndim != 4:
-        raise TypeError("topgrad must be 4D tensor")
-    ksz = hostlogic.gradweights_kshape(x.shape, dy.shape, border_mode, subsample, filter_dilation, kshape)
-    if x.shape[1] % num_groups:
-        raise ValueError("CorrMM images and kernel must have the same stack size")
-    wshape = (dy.shape[1], x.shape[1] // num_groups) + ksz
-    pads = hostlogic.resolve_pads(border_mode, ksz, filter_dilation)
-    hostlogic.check_consistent(x.shape, wshape, dy.shape, pads, subsample, filter_dilation, num_groups)
+    wshape, d = _plans.find(_plan_grad_weights, "gw", x.shape, dy.shape, _key(kshape), border_mode, subsample,
+                            filter_dilation, num_groups, filter_flip, x.dtype)
     ctx = ctx or get_context()
     if out is None or out.shape != wshape or out.dtype != x.dtype or not out.flags.c_contiguous:
         out = _results.empty(ctx, wshape, x.dtype)
     if out.size == 0:
         return out
-    d = make_desc(x.shape, wshape, dy.shape, pads, subsample, filter_dilation, num_groups, filter_flip, x.dtype)
-    ctx.wgrad(d, x.ctypes.data, dy.ctypes.data, out.ctypes.data, flags | HOST_PTRS)
+    ctx.wgrad(d, _address(x), _address(dy), _address(out), flags | HOST_PTRS)
     return out
 
 
@@ -606,20 +674,14 @@ def conv2d_grad_inputs(w, dy, imshape=None, border_mode="valid", subsample=(1, 1
                        flags=0):
     """AbstractConv2d_gradInputs: w [K,C/g,kH,kW], dy [N,K,Ho,Wo] -> dx [N,C,H,W]."""
     w, dy = _common(np.asarray(w), np.asarray(dy))
-    if w.ndim != 4:
-        raise TypeError("kern must be 4D tensor")
-    if dy.ndim != 4:
-        raise TypeError("topgrad must be 4D tensor")
-    hw, pads = hostlogic.gradinputs_imshape(w.shape, dy.shape, border_mode, subsample, filter_dilation, imshape)
-    xshape = (dy.shape[0], w.shape[1] * num_groups) + hw
-    hostlogic.check_consistent(xshape, w.shape, dy.shape, pads, subsample, filter_dilation, num_groups)
+    xshape, d = _plans.find(_plan_grad_inputs, "gi", w.shape, dy.shape, _key(imshape), border_mode, subsample,
+                            filter_dilation, num_groups, filter_flip, w.dtype)
     ctx = ctx or get_context()
     if out is None or out.shape != xshape or out.dtype != w.dtype or not out.flags.c_contiguous:
         out = _results.empty(ctx, xshape, w.dtype)
     if out.size == 0:
         return out
-    d = make_desc(xshape, w.shape, dy.shape, pads, subsample, filter_dilation, num_groups, filter_flip, w.dtype)
-    ctx.dgrad(d, w.ctypes.data, dy.ctypes.data, out.ctypes.data, flags | HOST_PTRS)
+    ctx.dgrad(d, _address(w), _address(dy), _address(out), flags | HOST_PTRS)
     return out
 
 
@@ -741,7 +803,8 @@ def device_conv2d(x, w, border_mode="valid", subsample=(1, 1), filter_dilation=(
     the result then has half the rows and columns.  Geometries whose epilogue cannot pool raise B200Error
     (E_UNSUPPORTED): run `device_maxpool2x2` on the unpooled result instead."""
     ctx = x.ctx
-    yshape, pads = hostlogic.forward_shape(x.shape, w.shape, border_mode, subsample, filter_dilation, num_groups)
+    yshape, d = _plans.find(_plan_forward, "fwd", x.shape, w.shape, border_mode, subsample, filter_dilation,
+                            num_groups, filter_flip, x.dtype)
     out_layout = out_layout or x.layout
     oshape = (yshape[0], yshape[1], yshape[2] // 2, yshape[3] // 2) if pool else yshape
     if pool:
@@ -752,11 +815,10 @@ def device_conv2d(x, w, border_mode="valid", subsample=(1, 1), filter_dilation=(
         out = DeviceTensor(ctx, oshape, x.dtype, out_layout)
     elif tuple(out.shape) != tuple(oshape):
         raise ValueError("output tensor has shape %s, expected %s" % (out.shape, oshape))
-    d = make_desc(x.shape, w.shape, yshape, pads, subsample, filter_dilation, num_groups, filter_flip, x.dtype)
     f = flags | (IN_NHWC if x.layout == "nhwc" else 0) | (OUT_NHWC if out.layout == "nhwc" else 0) | (RELU if relu else 0)
     if residual is not None and (residual.shape != tuple(yshape) or residual.layout != out.layout):
         raise ValueError("residual must have the shape and layout of the output")
-    if bias is not None and int(np.prod(bias.shape)) != int(w.shape[0]):
+    if bias is not None and math.prod(bias.shape) != w.shape[0]:
         raise ValueError("bias must have one value per filter (%d), not %d" % (w.shape[0], int(np.prod(bias.shape))))
     ctx.fwd(d, x.ptr, w.ptr, bias.ptr if bias is not None else None, out.ptr, f,
             residual=residual.ptr if residual is not None else None, alpha=alpha, beta=beta, slope=slope)
@@ -766,13 +828,11 @@ def device_conv2d(x, w, border_mode="valid", subsample=(1, 1), filter_dilation=(
 def device_grad_inputs(w, dy, imshape, border_mode="valid", subsample=(1, 1), filter_dilation=(1, 1),
                        num_groups=1, filter_flip=True, out_layout=None, out=None, flags=0):
     ctx = dy.ctx
-    hw, pads = hostlogic.gradinputs_imshape(w.shape, dy.shape, border_mode, subsample, filter_dilation, imshape)
-    xshape = (dy.shape[0], w.shape[1] * num_groups) + hw
-    hostlogic.check_consistent(xshape, w.shape, dy.shape, pads, subsample, filter_dilation, num_groups)
+    xshape, d = _plans.find(_plan_grad_inputs, "gi", w.shape, dy.shape, _key(imshape), border_mode, subsample,
+                            filter_dilation, num_groups, filter_flip, dy.dtype)
     out_layout = out_layout or dy.layout
     if out is None:
         out = DeviceTensor(ctx, xshape, dy.dtype, out_layout)
-    d = make_desc(xshape, w.shape, dy.shape, pads, subsample, filter_dilation, num_groups, filter_flip, dy.dtype)
     f = flags | (IN_NHWC if dy.layout == "nhwc" else 0) | (OUT_NHWC if out.layout == "nhwc" else 0)
     ctx.dgrad(d, w.ptr, dy.ptr, out.ptr, f)
     return out
@@ -781,13 +841,10 @@ def device_grad_inputs(w, dy, imshape, border_mode="valid", subsample=(1, 1), fi
 def device_grad_weights(x, dy, kshape, border_mode="valid", subsample=(1, 1), filter_dilation=(1, 1),
                         num_groups=1, filter_flip=True, out=None, flags=0):
     ctx = x.ctx
-    ksz = hostlogic.gradweights_kshape(x.shape, dy.shape, border_mode, subsample, filter_dilation, kshape)
-    wshape = (dy.shape[1], x.shape[1] // num_groups) + ksz
-    pads = hostlogic.resolve_pads(border_mode, ksz, filter_dilation)
-    hostlogic.check_consistent(x.shape, wshape, dy.shape, pads, subsample, filter_dilation, num_groups)
+    wshape, d = _plans.find(_plan_grad_weights, "gw", x.shape, dy.shape, _key(kshape), border_mode, subsample,
+                            filter_dilation, num_groups, filter_flip, x.dtype)
     if out is None:
         out = DeviceTensor(ctx, wshape, x.dtype, "nchw")
-    d = make_desc(x.shape, wshape, dy.shape, pads, subsample, filter_dilation, num_groups, filter_flip, x.dtype)
     f = flags | (IN_NHWC if x.layout == "nhwc" else 0) | (IN2_NHWC if dy.layout == "nhwc" else 0)
     if out.dtype == np.float32 and x.dtype == np.float16:
         f |= DW_F32              # float16 tensors, gradient kept in float32 (e.g. an all-reduce bucket)
