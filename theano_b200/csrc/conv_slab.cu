@@ -96,6 +96,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
   if (trace && threadIdx.x == 0) trace[1] = clock64();
 
   if (warp == 0) {
@@ -504,7 +505,7 @@ cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cu
   });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  conv_slab_kernel<KIND, BN><<<grid, kThreads, smem, s>>>(p);
+  launch_chained(conv_slab_kernel<KIND, BN>, grid, kThreads, smem, s, p);
   return cudaGetLastError();
 }
 

@@ -103,6 +103,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
   if (warp == 0 || warp >= kFirstExtraProducer) {
     // every lane follows the loop (warp-uniform control flow and addresses), one elected lane issues
@@ -278,7 +279,7 @@ cudaError_t launch_one(const UmmaConvParams& p, long long total, int num_sms, cu
   cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(conv_umma_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  conv_umma_kernel<KIND, BN><<<grid, kThreads, smem, s>>>(p);
+  launch_chained(conv_umma_kernel<KIND, BN>, grid, kThreads, smem, s, p);
   return cudaGetLastError();
 }
 

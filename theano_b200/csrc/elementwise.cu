@@ -68,6 +68,7 @@ template <typename T, bool PLAIN>
 __global__ void __launch_bounds__(256) elementwise_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                           const float* __restrict__ chan, T* __restrict__ out,
                                                           long long nvec, int C, int Cp, int op, int b_kind, float s) {
+  pdl_enter();
   constexpr int V = Vec<T>::n;
   const long long base = blockIdx.x * (256LL * kEwVecs) + threadIdx.x;
   float fa[kEwVecs][V], fb[kEwVecs][V];
@@ -101,6 +102,7 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const T* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) channel_sum_partial_kernel(const T* __restrict__ x, float* __restrict__ partial,
                                                                   long long pixels, int Cp, int log_lanes) {
+  pdl_enter();
   constexpr int V = Vec<T>::n;
   __shared__ float part[256][V + 1];
   const int cols = 256 >> log_lanes, lane = threadIdx.x >> (8 - log_lanes), col = threadIdx.x & (cols - 1);
@@ -140,6 +142,7 @@ __global__ void __launch_bounds__(256) channel_sum_partial_kernel(const T* __res
 template <typename T>
 __global__ void __launch_bounds__(512) channel_sum_final_kernel(const float* __restrict__ partial, T* __restrict__ out,
                                                                 int blocks, int C, int Cp) {
+  pdl_enter();
   __shared__ float part[16][32];
   const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * 32 + lane;
   float acc = 0.f;
@@ -165,7 +168,7 @@ cudaError_t launch_elementwise(const void* a, const void* b, const float* chan, 
   if (grid >= (1LL << 31)) return cudaErrorInvalidValue;
   const bool plain = C == Cp && b_kind != 2;
 #define B200_EW(T, PLAIN)                                                                                      \
-  elementwise_kernel<T, PLAIN><<<static_cast<int>(grid), 256, 0, st>>>(                                        \
+  launch_streaming(elementwise_kernel<T, PLAIN>, static_cast<int>(grid), 256, 0, st,                                         \
       static_cast<const T*>(a), static_cast<const T*>(b), chan, static_cast<T*>(out), nvec, C, Cp, op, b_kind, s)
   if (dtype == B200CONV_F16) {
     if (plain) B200_EW(__half, true);
@@ -191,15 +194,15 @@ cudaError_t launch_channel_sum(const void* x, float* partial, void* out, long lo
   int log_lanes = 0;                             // as many rows of threads over the pixels as the channel vector leaves
   while (log_lanes < 8 && (vecs << (log_lanes + 1)) <= 256) ++log_lanes;
   if (dtype == B200CONV_F16)
-    channel_sum_partial_kernel<__half><<<blocks, 256, 0, st>>>(static_cast<const __half*>(x), partial, pixels, Cp, log_lanes);
+    launch_streaming(channel_sum_partial_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(x), partial, pixels, Cp, log_lanes);
   else
-    channel_sum_partial_kernel<float><<<blocks, 256, 0, st>>>(static_cast<const float*>(x), partial, pixels, Cp, log_lanes);
+    launch_streaming(channel_sum_partial_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(x), partial, pixels, Cp, log_lanes);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (dtype == B200CONV_F16)
-    channel_sum_final_kernel<__half><<<(C + 31) / 32, 512, 0, st>>>(partial, static_cast<__half*>(out), blocks, C, Cp);
+    launch_chained(channel_sum_final_kernel<__half>, (C + 31) / 32, 512, 0, st, partial, static_cast<__half*>(out), blocks, C, Cp);
   else
-    channel_sum_final_kernel<float><<<(C + 31) / 32, 512, 0, st>>>(partial, static_cast<float*>(out), blocks, C, Cp);
+    launch_chained(channel_sum_final_kernel<float>, (C + 31) / 32, 512, 0, st, partial, static_cast<float*>(out), blocks, C, Cp);
   return cudaGetLastError();
 }
 

@@ -73,6 +73,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
   cluster_sync_all();                                            // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
   if (warp == 0) {
     const bool leader = elect_one();
@@ -228,7 +229,7 @@ cudaError_t launch_gemm_pair(const PairGemmParams& p, int num_sms, cudaStream_t 
   });
   if (e != cudaSuccess) return e;
   long long pairs = std::min<long long>(total, num_sms / 2);
-  gemm_pair_kernel<<<static_cast<int>(2 * pairs), kThreads, smem, s>>>(p);
+  launch_chained(gemm_pair_kernel, static_cast<int>(2 * pairs), kThreads, smem, s, p);
   return cudaGetLastError();
 }
 

@@ -10,6 +10,7 @@ namespace {
 template <typename T>
 __global__ void transpose_kernel(const T* __restrict__ in, T* __restrict__ out, int R, int S,
                                  int ld_in, int ld_out) {
+  pdl_enter();
   __shared__ T tile[32][33];
   const long long b = blockIdx.z;
   const T* src = in + b * R * ld_in;
@@ -110,12 +111,14 @@ __device__ __forceinline__ void pack_job_block(const PackJob& q, int local) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ PackJob q) {
+  pdl_enter();
   pack_job_block<T>(q, blockIdx.x);
 }
 
 // Many filter banks in one launch: block b belongs to the job j with first_block[j] <= b < first_block[j + 1].
 template <typename T>
 __global__ void __launch_bounds__(256) pack_filters_batch_kernel(const __grid_constant__ PackBatch b) {
+  pdl_enter();
   int j = 0;
   while (j + 1 < b.njobs && static_cast<int>(blockIdx.x) >= b.jobs[j + 1].first_block) ++j;
   pack_job_block<T>(b.jobs[j], blockIdx.x - b.jobs[j].first_block);
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(256) pack_filters_batch_kernel(const __grid_co
 template <typename T>
 __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int C, int H,
                                 int W, int Cp, int Wp, int pad_l, int nhwc_in) {
+  pdl_enter();
   const long long total = 1LL * N * H * Wp;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -165,6 +169,7 @@ __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, 
 template <typename T>
 __global__ void pack_filters_fold_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C,
                                          int kH, int kW, int Cp, int ld, int flip) {
+  pdl_enter();
   const long long total = 1LL * kH * K * ld;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -190,6 +195,7 @@ __global__ void pack_filters_fold_kernel(const T* __restrict__ w, T* __restrict_
 template <typename T, int C>
 __global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H,
                                int W, int Cp_in, int H2, int Wq, int q0, int nhwc_in) {
+  pdl_enter();
   const long long total = 1LL * N * H2 * Wq;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -231,6 +237,7 @@ template <typename T>
 __global__ void pack_filters_s2d_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C,
                                         int kH, int kW, int ntaps, int t0, int q0, int padH, int padW,
                                         int ld, int flip) {
+  pdl_enter();
   const long long total = 1LL * ntaps * K * ld;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -257,6 +264,7 @@ template <typename T>
 __global__ void wgrad_reduce_s2d_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits,
                                         int K, int C, int kH, int kW, int ntaps, int t0, int q0, int padH,
                                         int padW, int ld, int flip) {
+  pdl_enter();
   const long long total = 1LL * K * C * kH * kW;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -281,6 +289,7 @@ template <typename T>
 __global__ void wgrad_reduce_fold_kernel(const float* __restrict__ partial, T* __restrict__ dw,
                                          int splits, int K, int C, int kH, int kW, int Cp, int ld,
                                          int flip) {
+  pdl_enter();
   const long long total = 1LL * K * C * kH * kW;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -303,6 +312,7 @@ __global__ void wgrad_reduce_fold_kernel(const float* __restrict__ partial, T* _
 template <typename T>
 __global__ void merge_groups_kernel(const T* __restrict__ src, T* __restrict__ dst, int K, int Cg,
                                     int Kg, int m, int taps, int extract) {
+  pdl_enter();
   const int CgE = Cg * m;
   const long long total = 1LL * K * (extract ? Cg : CgE) * taps;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
@@ -324,6 +334,7 @@ __global__ void merge_groups_kernel(const T* __restrict__ src, T* __restrict__ d
 
 template <typename T>
 __global__ void convert_bias_kernel(const T* __restrict__ b, float* __restrict__ dst, int n) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dst[i] = static_cast<float>(b[i]);
 }
@@ -332,6 +343,7 @@ __global__ void convert_bias_kernel(const T* __restrict__ b, float* __restrict__
 // channel fastest, so neighbouring threads read neighbouring addresses.
 template <typename T>
 __global__ void maxpool2x2_nchw_kernel(const T* __restrict__ x, T* __restrict__ y, long long NC, int H, int W) {
+  pdl_enter();
   const int Ho = H / 2, Wo = W / 2;
   const long long total = NC * Ho * Wo;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
@@ -353,6 +365,7 @@ __global__ void maxpool2x2_nchw_kernel(const T* __restrict__ x, T* __restrict__ 
 template <typename T>
 __global__ void maxpool2x2_grad_nchw_kernel(const T* __restrict__ x, const T* __restrict__ y,
                                             const T* __restrict__ gy, T* __restrict__ gx, long long NC, int H, int W) {
+  pdl_enter();
   const int Ho = H / 2, Wo = W / 2;
   const long long total = NC * H * W;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
@@ -401,6 +414,7 @@ template <typename T> __device__ __forceinline__ Piece<T> load_piece(const T* p)
 template <typename T, typename Index>
 __global__ void __launch_bounds__(256) maxpool2x2_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y, Index total,
                                                               int H, int W, int pieces) {
+  pdl_enter();
   constexpr int V = 16 / static_cast<int>(sizeof(T));
   const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
   if (idx >= total) return;
@@ -422,6 +436,7 @@ template <typename T, typename Index>
 __global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __restrict__ x, const T* __restrict__ y,
                                                                    const T* __restrict__ gy, T* __restrict__ gx,
                                                                    Index total, int H, int W, int pieces) {
+  pdl_enter();
   constexpr int V = 16 / static_cast<int>(sizeof(T));
   const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
   if (idx >= total) return;
@@ -452,6 +467,7 @@ __global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __re
 template <typename T>
 __global__ void pack_filters_merged_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C, int kH,
                                            int kW, int flip, MergedTapTable tb, int nu, int ncls, int rows, int ldw) {
+  pdl_enter();
   const long long total = 1LL * nu * rows * ldw;
   for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
        idx += 1LL * gridDim.x * blockDim.x) {
@@ -475,6 +491,7 @@ __global__ void pack_filters_merged_kernel(const T* __restrict__ w, T* __restric
 template <typename T>
 __global__ void depth_to_space_kernel(const T* __restrict__ tmp, T* __restrict__ dx, int N, int C, int H, int W,
                                       int sH, int sW, int Ct, int Cp, int nhwc) {
+  pdl_enter();
   const int Hq = (H + sH - 1) / sH, Wq = (W + sW - 1) / sW;
   if (nhwc) {
     constexpr int kVec = 16 / static_cast<int>(sizeof(T));      // Cp is a multiple of kVec
@@ -527,11 +544,11 @@ cudaError_t launch_transpose(const void* in, void* out, int B, int R, int S, int
     const int nb = (B - b0) < 65535 ? (B - b0) : 65535;
     dim3 grid((S + 31) / 32, (rows + 31) / 32, nb), block(32, 8);
     if (dtype == B200CONV_F16)
-      transpose_kernel<__half><<<grid, block, 0, s>>>(
+      launch_streaming(transpose_kernel<__half>, grid, block, 0, s,
           static_cast<const __half*>(in) + 1LL * b0 * R * ld_in,
           static_cast<__half*>(out) + 1LL * b0 * S * ld_out, R, S, ld_in, ld_out);
     else
-      transpose_kernel<float><<<grid, block, 0, s>>>(
+      launch_streaming(transpose_kernel<float>, grid, block, 0, s,
           static_cast<const float*>(in) + 1LL * b0 * R * ld_in,
           static_cast<float*>(out) + 1LL * b0 * S * ld_out, R, S, ld_in, ld_out);
   }
@@ -555,8 +572,8 @@ void pack_filters_grid(int Kg, int Cg, int groups, int mode, int ldc, int taps, 
 
 cudaError_t launch_pack_filters_batch(const PackBatch& b, int total_blocks, int dtype, cudaStream_t s) {
   if (b.njobs == 0 || total_blocks == 0) return cudaSuccess;
-  if (dtype == B200CONV_F16) pack_filters_batch_kernel<__half><<<total_blocks, dim3(32, 8), 0, s>>>(b);
-  else pack_filters_batch_kernel<float><<<total_blocks, dim3(32, 8), 0, s>>>(b);
+  if (dtype == B200CONV_F16) launch_chained(pack_filters_batch_kernel<__half>, total_blocks, dim3(32, 8), 0, s, b);
+  else launch_chained(pack_filters_batch_kernel<float>, total_blocks, dim3(32, 8), 0, s, b);
   return cudaGetLastError();
 }
 
@@ -570,8 +587,8 @@ cudaError_t launch_pack_filters(const void* w, void* dst, int K, int Cg, int kH,
   q.K = K; q.Cg = Cg; q.kH = kH; q.kW = kW; q.groups = groups; q.flip = flip; q.mode = mode; q.ldc = ldc;
   pack_filters_grid(K / groups, Cg, groups, mode, ldc, kH * kW, &q.gx, &q.gy, &gz);
   q.first_block = 0;
-  if (dtype == B200CONV_F16) pack_filters_kernel<__half><<<q.gx * q.gy * gz, dim3(32, 8), 0, s>>>(q);
-  else pack_filters_kernel<float><<<q.gx * q.gy * gz, dim3(32, 8), 0, s>>>(q);
+  if (dtype == B200CONV_F16) launch_chained(pack_filters_kernel<__half>, q.gx * q.gy * gz, dim3(32, 8), 0, s, q);
+  else launch_chained(pack_filters_kernel<float>, q.gx * q.gy * gz, dim3(32, 8), 0, s, q);
   return cudaGetLastError();
 }
 
@@ -580,10 +597,10 @@ cudaError_t launch_pad_fold(const void* src, void* dst, int N, int C, int H, int
   const long long total = 1LL * N * H * Wp;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    pad_fold_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(pad_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(src), static_cast<__half*>(dst), N, C, H, W, Cp, Wp, pad_l, nhwc_in);
   else
-    pad_fold_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(pad_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(src), static_cast<float*>(dst), N, C, H, W, Cp, Wp, pad_l, nhwc_in);
   return cudaGetLastError();
 }
@@ -593,10 +610,10 @@ cudaError_t launch_pack_filters_fold(const void* w, void* dst, int K, int C, int
   const long long total = 1LL * kH * K * ld;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    pack_filters_fold_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, Cp, ld, flip);
   else
-    pack_filters_fold_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, Cp, ld, flip);
   return cudaGetLastError();
 }
@@ -607,10 +624,10 @@ cudaError_t launch_wgrad_reduce_s2d(const float* partial, void* dw, int splits, 
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    wgrad_reduce_s2d_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(wgrad_reduce_s2d_kernel<__half>, grid_for(total, 256), 256, 0, s,
         partial, static_cast<__half*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   else
-    wgrad_reduce_s2d_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(wgrad_reduce_s2d_kernel<float>, grid_for(total, 256), 256, 0, s,
         partial, static_cast<float*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   return cudaGetLastError();
 }
@@ -623,10 +640,10 @@ cudaError_t pad_s2d_typed(const void* src, void* dst, int N, int C, int H, int W
   T* out = static_cast<T*>(dst);
   const int grid = grid_for(total, 256);
   switch (C) {   // the channel count as a constant keeps the assembled pixel in registers
-    case 1: pad_s2d_kernel<T, 1><<<grid, 256, 0, s>>>(in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 2: pad_s2d_kernel<T, 2><<<grid, 256, 0, s>>>(in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 3: pad_s2d_kernel<T, 3><<<grid, 256, 0, s>>>(in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 4: pad_s2d_kernel<T, 4><<<grid, 256, 0, s>>>(in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
+    case 1: launch_streaming(pad_s2d_kernel<T, 1>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
+    case 2: launch_streaming(pad_s2d_kernel<T, 2>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
+    case 3: launch_streaming(pad_s2d_kernel<T, 3>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
+    case 4: launch_streaming(pad_s2d_kernel<T, 4>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -645,10 +662,10 @@ cudaError_t launch_pack_filters_s2d(const void* w, void* dst, int K, int C, int 
   const long long total = 1LL * ntaps * K * ld;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    pack_filters_s2d_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_s2d_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   else
-    pack_filters_s2d_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_s2d_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   return cudaGetLastError();
 }
@@ -658,10 +675,10 @@ cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits,
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    wgrad_reduce_fold_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(wgrad_reduce_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
         partial, static_cast<__half*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
   else
-    wgrad_reduce_fold_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(wgrad_reduce_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
         partial, static_cast<float*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
   return cudaGetLastError();
 }
@@ -671,10 +688,10 @@ cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int K
   const long long total = 1LL * K * (extract ? Cg : Cg * m) * taps;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    merge_groups_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(merge_groups_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(src), static_cast<__half*>(dst), K, Cg, Kg, m, taps, extract);
   else
-    merge_groups_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(merge_groups_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(src), static_cast<float*>(dst), K, Cg, Kg, m, taps, extract);
   return cudaGetLastError();
 }
@@ -682,24 +699,25 @@ cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int K
 namespace {
 template <typename T>
 __global__ void pad_bias_kernel(const T* __restrict__ b, T* __restrict__ dst, int n, int np) {
+  pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < np) dst[i] = i < n ? b[i] : T(0);
 }
 }  // namespace
 cudaError_t launch_pad_bias(const void* bias, void* dst, int n, int np, int dtype, cudaStream_t s) {
   if (dtype == B200CONV_F16)
-    pad_bias_kernel<<<(np + 255) / 256, 256, 0, s>>>(static_cast<const __half*>(bias), static_cast<__half*>(dst), n, np);
+    launch_chained(pad_bias_kernel<__half>, (np + 255) / 256, 256, 0, s, static_cast<const __half*>(bias), static_cast<__half*>(dst), n, np);
   else
-    pad_bias_kernel<<<(np + 255) / 256, 256, 0, s>>>(static_cast<const float*>(bias), static_cast<float*>(dst), n, np);
+    launch_chained(pad_bias_kernel<float>, (np + 255) / 256, 256, 0, s, static_cast<const float*>(bias), static_cast<float*>(dst), n, np);
   return cudaGetLastError();
 }
 
 cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, cudaStream_t s) {
   if (n == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    convert_bias_kernel<__half><<<(n + 255) / 256, 256, 0, s>>>(static_cast<const __half*>(bias), dst, n);
+    launch_chained(convert_bias_kernel<__half>, (n + 255) / 256, 256, 0, s, static_cast<const __half*>(bias), dst, n);
   else
-    convert_bias_kernel<float><<<(n + 255) / 256, 256, 0, s>>>(static_cast<const float*>(bias), dst, n);
+    launch_chained(convert_bias_kernel<float>, (n + 255) / 256, 256, 0, s, static_cast<const float*>(bias), dst, n);
   return cudaGetLastError();
 }
 
@@ -716,30 +734,30 @@ cudaError_t for_index(long long total, Launch launch) {
 template <typename T>
 cudaError_t maxpool_typed(const T* x, T* y, int N, int C, int H, int W, int nhwc, int Cp, cudaStream_t s) {
   if (!nhwc) {
-    maxpool2x2_nchw_kernel<T><<<grid_for(1LL * N * C * (H / 2) * (W / 2), 256), 256, 0, s>>>(x, y, 1LL * N * C, H, W);
+    launch_streaming(maxpool2x2_nchw_kernel<T>, grid_for(1LL * N * C * (H / 2) * (W / 2), 256), 256, 0, s, x, y, 1LL * N * C, H, W);
     return cudaGetLastError();
   }
   const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
   const long long total = 1LL * N * (H / 2) * (W / 2) * pieces;
   return for_index<T>(total, [&](int grid, bool small) {
-    if (small) maxpool2x2_nhwc_kernel<T, unsigned><<<grid, 256, 0, s>>>(x, y, static_cast<unsigned>(total), H, W, pieces);
-    else maxpool2x2_nhwc_kernel<T, long long><<<grid, 256, 0, s>>>(x, y, total, H, W, pieces);
+    if (small) launch_streaming(maxpool2x2_nhwc_kernel<T, unsigned>, grid, 256, 0, s, x, y, static_cast<unsigned>(total), H, W, pieces);
+    else launch_streaming(maxpool2x2_nhwc_kernel<T, long long>, grid, 256, 0, s, x, y, total, H, W, pieces);
   });
 }
 template <typename T>
 cudaError_t maxpool_grad_typed(const T* x, const T* y, const T* gy, T* gx, int N, int C, int H, int W, int nhwc, int Cp,
                                cudaStream_t s) {
   if (!nhwc) {
-    maxpool2x2_grad_nchw_kernel<T><<<grid_for(1LL * N * C * H * W, 256), 256, 0, s>>>(x, y, gy, gx, 1LL * N * C, H, W);
+    launch_streaming(maxpool2x2_grad_nchw_kernel<T>, grid_for(1LL * N * C * H * W, 256), 256, 0, s, x, y, gy, gx, 1LL * N * C, H, W);
     return cudaGetLastError();
   }
   const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
   const long long total = 1LL * N * ((H + 1) / 2) * ((W + 1) / 2) * pieces;
   return for_index<T>(total, [&](int grid, bool small) {
     if (small)
-      maxpool2x2_grad_nhwc_kernel<T, unsigned><<<grid, 256, 0, s>>>(x, y, gy, gx, static_cast<unsigned>(total), H, W, pieces);
+      launch_streaming(maxpool2x2_grad_nhwc_kernel<T, unsigned>, grid, 256, 0, s, x, y, gy, gx, static_cast<unsigned>(total), H, W, pieces);
     else
-      maxpool2x2_grad_nhwc_kernel<T, long long><<<grid, 256, 0, s>>>(x, y, gy, gx, total, H, W, pieces);
+      launch_streaming(maxpool2x2_grad_nhwc_kernel<T, long long>, grid, 256, 0, s, x, y, gy, gx, total, H, W, pieces);
   });
 }
 }  // namespace
@@ -768,10 +786,10 @@ cudaError_t launch_pack_filters_merged(const void* w, void* dst, int K, int C, i
   const long long total = 1LL * nu * rows * ldw;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    pack_filters_merged_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_merged_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
   else
-    pack_filters_merged_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_chained(pack_filters_merged_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
   return cudaGetLastError();
 }
@@ -781,10 +799,10 @@ cudaError_t launch_depth_to_space(const void* tmp, void* dx, int N, int C, int H
   const long long total = 1LL * N * (nhwc ? 1 : C) * H * W;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    depth_to_space_kernel<__half><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(depth_to_space_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(tmp), static_cast<__half*>(dx), N, C, H, W, sH, sW, Ct, Cp, nhwc);
   else
-    depth_to_space_kernel<float><<<grid_for(total, 256), 256, 0, s>>>(
+    launch_streaming(depth_to_space_kernel<float>, grid_for(total, 256), 256, 0, s,
         static_cast<const float*>(tmp), static_cast<float*>(dx), N, C, H, W, sH, sW, Ct, Cp, nhwc);
   return cudaGetLastError();
 }

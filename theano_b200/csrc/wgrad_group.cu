@@ -228,6 +228,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
   if (warp == 0 || warp >= kFirstExtraProducer) {
     const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
@@ -393,7 +394,7 @@ cudaError_t launch_one(const GroupWgradParams& p, long long total, int num_sms, 
   cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_group_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  wgrad_group_kernel<KIND><<<grid, kThreads, smem, s>>>(p);
+  launch_chained(wgrad_group_kernel<KIND>, grid, kThreads, smem, s, p);
   return cudaGetLastError();
 }
 

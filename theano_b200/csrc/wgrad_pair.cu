@@ -107,6 +107,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
   cluster_sync_all();                                              // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
   if (warp == 0) {
     const bool leader = elect_one();
@@ -256,7 +257,7 @@ cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int num_sms, cudaStream_
   });
   if (e != cudaSuccess) return e;
   const long long pairs = std::min<long long>(total, num_sms / 2);
-  wgrad_pair_kernel<<<static_cast<int>(2 * pairs), kThreads, smem, s>>>(p);
+  launch_chained(wgrad_pair_kernel, static_cast<int>(2 * pairs), kThreads, smem, s, p);
   return cudaGetLastError();
 }
 

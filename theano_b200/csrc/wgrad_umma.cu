@@ -187,6 +187,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
+  pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
   if (warp == 0 || warp >= kFirstExtraProducer) {
     const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
@@ -347,6 +348,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
 template <typename T>
 __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ dw,
                                                             int splits, int taps, long long kc, int log_elems, int log_lanes) {
+  pdl_enter();
   extern __shared__ float tile[];
   __shared__ float4 part[256];
   const int elems = 1 << log_elems, lanes = 1 << log_lanes, slots = 256 >> log_lanes;
@@ -410,7 +412,7 @@ cudaError_t launch_one(const UmmaWgradParams& p, long long total, int num_sms, c
   cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_umma_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  wgrad_umma_kernel<KIND, BN><<<grid, kThreads, smem, s>>>(p);
+  launch_chained(wgrad_umma_kernel<KIND, BN>, grid, kThreads, smem, s, p);
   return cudaGetLastError();
 }
 
@@ -448,10 +450,10 @@ cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int 
   if (g > 148 * 16) g = 148 * 16;
   const size_t smem = sizeof(float) * taps << log_elems;
   if (dtype == B200CONV_F16)
-    wgrad_reduce_kernel<__half><<<static_cast<int>(g), 256, smem, s>>>(
+    launch_streaming(wgrad_reduce_kernel<__half>, static_cast<int>(g), 256, smem, s,
         partial, static_cast<__half*>(dw), splits, taps, kc, log_elems, log_lanes);
   else
-    wgrad_reduce_kernel<float><<<static_cast<int>(g), 256, smem, s>>>(
+    launch_streaming(wgrad_reduce_kernel<float>, static_cast<int>(g), 256, smem, s,
         partial, static_cast<float*>(dw), splits, taps, kc, log_elems, log_lanes);
   return cudaGetLastError();
 }
