@@ -258,7 +258,8 @@ long long b200conv_launch_count(b200conv_ctx* ctx);
 /* Per-kernel timing.  While enabled, every launch of the library's own kernels is bracketed by
  * CUDA events on the context's stream; b200conv_kernel_time() then returns the summed duration
  * and the launch count of one kernel family since timing was enabled: "conv_umma" (forward and
- * gradInputs main kernel), "wgrad_umma", "wgrad_reduce", "transpose", "pack", "direct", "pool". */
+ * gradInputs main kernel), "conv_reduce" (its second half when the reduction is split over CTAs), "wgrad_umma",
+ * "wgrad_reduce", "transpose", "pack", "direct", "pool". */
 int b200conv_kernel_timing(b200conv_ctx* ctx, int enable);
 int b200conv_kernel_time(b200conv_ctx* ctx, const char* family, float* total_ms, int* launches);
 /* Forward and gradInputs have two tensor-core kernels (activations fetched once per channel

@@ -86,9 +86,11 @@ struct GeoHash {
 };
 enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance };      // kinds (first integer of a key)
 
-// Tile of the slab kernel for one geometry (the result of the search in try_conv_slab).
+// Tile of a convolution kernel for one geometry (the result of a search).
 struct SlabTile {
   int wt = 0, th = 0, nb = 0, n_acc = 0, slab_bytes = 0;
+  int bn = 0, splits = 1;        // accumulator columns, slices of the reduction
+  bool row = false;              // slab kernel: whole 128-pixel pieces of one long row (flattened 1x1 layers)
   bool found = false;
 };
 
@@ -180,9 +182,9 @@ int fail(b200conv_ctx* c, int code, const char* fmt, ...) {
   } while (0)
 
 // Kernel families, for the launch counter and the optional per-kernel timing.
-enum { kKConvUmma = 0, kKWgradUmma, kKWgradReduce, kKTranspose, kKPack, kKDirect, kKPool, kKCount };
+enum { kKConvUmma = 0, kKWgradUmma, kKWgradReduce, kKTranspose, kKPack, kKDirect, kKPool, kKConvReduce, kKCount };
 const char* const kKernelNames[kKCount] = {"conv_umma", "wgrad_umma", "wgrad_reduce", "transpose",
-                                           "pack", "direct", "pool"};
+                                           "pack", "direct", "pool", "conv_reduce"};
 
 cudaEvent_t prof_event(b200conv_ctx* c) {
   cudaEvent_t e = nullptr;
@@ -538,13 +540,185 @@ long long out_extent(const FwdLikeArgs& a, int Wt, int Ht, long long sn, long lo
   return off + (a.N - 1) * sn + (Ht - 1) * sh + (Wt - 1) * sw + (1LL * a.n_out * a.groups - 1) * sc + 1;
 }
 
+// Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
+// the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
+// and / or a reduction cut into slices where that occupies more SMs.  The numbers appear in tuning files.
+enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvVariants = 4 };
+
+// Clocks of four MMAs over 128 rows x bn columns x 32 bytes of the reduction, one after the other: half the
+// columns up to 128 (N = 64 and 32 are bound by their operands' shared-memory reads).
+int mma_clocks(int bn) { return bn >= 256 ? 128 : bn == 128 ? 64 : bn == 64 ? 48 : 40; }
+
+// Clocks that splitting the reduction of `items` = tiles x slices work items of rows x bn accumulators adds:
+// raw accumulators leave at 32 B/clk per SM, and the reduction kernel costs about 4500 clocks of launch and
+// latency plus its reads (48 B/clk per SM from L2).
+long long split_clocks(long long items, int rows, int bn, int sms) {
+  return 1LL * rows * bn * 4 / 32 + 4500 + items * rows * bn * 4 / (48LL * sms);
+}
+
+// Filter taps per stage of the slab kernel's filter ring.  Narrow tiles (few filters) have small filter tiles and
+// short MMAs: several taps then share one stage, so that a barrier round trip is paid per 16 to 32 KB of
+// filters, not per 4 or 8 KB (the issuing warp spends about 150 clocks per stage on the hand-over, as much as
+// the stage's MMAs take when a tap is four 128 x 64 MMAs).  Measured: 64 -> 64 3x3 layers 8 to 16 % faster with a
+// filter row per stage, the 7x7 stem 8 to 16 % with four taps; 128-filter tiles are better off with one tap per stage.
+int slab_tps(int bn, int ntaps) { return bn > 64 ? 1 : ntaps % 3 == 0 ? 3 : std::min(4, ntaps); }
+
+// Tile of the slab kernel.  spread = false: widest tile that holds the outputs, unsplit; true: the best over the
+// tile widths and slice counts as well.  `found` is false when nothing fits.
+SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, int Eh, int Ew, bool tma_layout_ok, bool spread) {
+  SlabTile& memo = c->slab_tiles[GeoKey{kGeoSlab, a.dtype, a.n_out, a.Cin_g, a.groups, a.N, Wt, Ht, ntaps, Eh, Ew, tma_layout_ok ? 1 : 0,
+                                        c->epi.pool, c->num_sms, spread ? 1 : 0}];
+  if (memo.bn) return memo;
+  const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
+  const int bn_max = conv_umma_bn(a.n_out);
+  const long long kblocks_n = cdiv(a.Cin_g, kBK);
+  const long long es_out = (long long)elem_size(a.dtype);
+  long long best_cost = -1, best_work = 0, best_tiles = 0;
+  SlabTile best;
+  best.bn = bn_max;
+  for (int BN = bn_max; BN >= (spread ? 32 : bn_max); BN /= 2) {
+    const int tiles_co = (int)cdiv(a.n_out, BN);
+    const int acc_cap = std::min(512 / BN, 4);
+    const int tps = slab_tps(BN, ntaps);
+    const int b_bytes = tps * BN * 128;
+    const int mma_clk = mma_clocks(BN);
+    const long long stages = kblocks_n * cdiv(ntaps, tps);
+    // one tile candidate: search the one with the least serial work per SM
+    auto consider = [&](int wt, int th, int nb, int n_acc, long long slab_bytes, bool row) {
+      const long long tiles = cdiv(Wt, wt) * cdiv(Ht, th) * cdiv(a.N, nb);
+      const long long total = tiles * tiles_co * a.groups;
+      // Clocks of the busiest SM: per tile and (tap, channel block) 4 MMAs per accumulator plus
+      // about 120 clocks of stage hand-over in the issuing thread; then the accumulators are read
+      // out, beside the next tile's MMAs when two accumulator sets fit the 512 TMEM columns.
+      // Epilogue: through staged TMA stores when the output is channels-last and the staging
+      // buffers fit beside two slabs and two filter stages (about 2500 clocks of latency per tile
+      // plus the tile's bytes at the SM's store rate of 32 B/clk), else lane-per-row stores from
+      // registers (1200 to 2500 clocks per 128 x 32 block: 16-byte pieces scattered over the pixel rows)
+      const long long dense_rows = 1LL * wt * th * nb;
+      const int ngr = n_acc == 3 ? 0 : 4 / n_acc;
+      const long long stg = (dense_rows * 128 + 1023) / 1024 * 1024;
+      const long long min_b = std::min<long long>(3, stages + 1);   // filter stages the staged epilogue insists on
+      if (c->epi.pool && ((wt | th) & 1)) return;          // pooling windows must not straddle tiles
+      const bool tma_fit = tma_layout_ok && ngr > 0 && BN * es_out >= 128 && ngr * stg <= kSlabStageBytes &&
+                           (total <= c->num_sms ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
+                                                : 2 * slab_bytes + min_b * b_bytes + kSlabStageBytes <= kSlabSmemBudget);
+      // plus about 1500 clocks per tile for the pipeline to fill again
+      auto mma_part = [&](long long st) { return st * (1LL * std::min(tps, ntaps) * 4 * n_acc * mma_clk + 120) + 1500; };
+      const long long whole = 1LL * kblocks_n * (ntaps * 4LL * n_acc * mma_clk + cdiv(ntaps, tps) * 120) + 1500;
+      const long long epi_part = tma_fit ? 2500 + dense_rows * BN * es_out / 32 : 2400LL * n_acc * (BN / 32);
+      const long long per_tile = 2 * n_acc * BN <= 512 ? std::max(whole, epi_part) : whole + epi_part;
+      long long cost = cdiv(total, c->num_sms) * per_tile;
+      if (spread) cost += std::min(whole, epi_part);      // the last tile's read-out runs beside nothing (a few tiles per SM only)
+      int splits = 1;
+      const bool unsplit_ok = !c->epi.pool || tma_fit;     // unsplit, pooling happens in the staged epilogue only
+      if (spread && 2 * total <= c->num_sms)
+        for (int s = 2; s <= std::min(stages, c->num_sms / total); ++s) {
+          const long long cs = mma_part(cdiv(stages, s)) + split_clocks(total * s, 128 * n_acc, BN, c->num_sms);
+          if (cs < cost || (s == 2 && !unsplit_ok)) { cost = cs; splits = s; }
+        }
+      if (splits == 1 && !unsplit_ok) return;
+      const long long work = total * n_acc;
+      if (best_cost < 0 || cost < best_cost || (cost == best_cost && work < best_work) ||
+          (cost == best_cost && work == best_work && tiles < best_tiles)) {
+        best_cost = cost; best_work = work; best_tiles = tiles;
+        best.wt = wt; best.th = th; best.nb = nb; best.n_acc = n_acc; best.slab_bytes = (int)slab_bytes;
+        best.bn = BN; best.splits = splits; best.row = row;
+        best.found = true;
+      }
+    };
+    for (int parts = 1; parts <= 16; ++parts) {
+      const int wt = (int)cdiv(Wt, parts);
+      if (parts > 1 && wt < 8) break;
+      const int Ws = wt + Ew;
+      if (Ws > 256) continue;
+      const int shift_max = Eh * Ws + Ew;
+      for (int th = 1; th <= Ht; ++th) {
+        const int Hs = th + Eh;
+        if (Hs > 256) break;
+        const int per_img = Hs * Ws;
+        if ((th - 1) * Ws + wt - 1 >= 128 * acc_cap) break;
+        for (int nb = 1; nb <= std::min(a.N, 256); ++nb) {
+          const long long last = 1LL * (nb - 1) * per_img + (th - 1) * Ws + (wt - 1);
+          if (last >= 128LL * acc_cap) break;
+          const int n_acc = (int)(last / 128) + 1;
+          const long long rows = std::max<long long>(1LL * nb * per_img, 128LL * n_acc + shift_max);
+          const long long slab_bytes = (rows * 128 + 1023) / 1024 * 1024;
+          if (2 * slab_bytes + 2 * b_bytes > kSlabSmemBudget) break;
+          consider(wt, th, nb, n_acc, slab_bytes, false);
+        }
+      }
+    }
+    if (Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && !c->epi.pool) {
+      // one long row of pixels without halo (a flattened 1x1 layer): whole 128-pixel accumulators,
+      // as many as still leave room for a second accumulator set
+      if (spread) {
+        for (int n_acc = 1; n_acc <= (BN >= 256 ? 1 : 2); ++n_acc) consider(128 * n_acc, 1, 1, n_acc, 128 * 128 * n_acc, true);
+      } else if (!best.found) {
+        best.n_acc = BN >= 256 ? 1 : 2;
+        best.wt = 128 * best.n_acc; best.th = best.nb = 1;
+        best.slab_bytes = best.wt * 128;
+        best.row = best.found = true;
+      }
+    }
+  }
+  memo = best;
+  return best;
+}
+
+// Tile of the per-tap kernel: the pixel box with the fewest tiles; spread: also a narrower accumulator and
+// slices of the reduction where that occupies more SMs.
+SlabTile tap_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, bool spread) {
+  SlabTile best;
+  choose_tile(c, Wt, Ht, a.N, 128, 0, &best.wt, &best.th, &best.nb);
+  best.bn = conv_umma_bn(a.n_out);
+  best.found = true;
+  if (!spread) return best;
+  const long long tiles = cdiv(Wt, best.wt) * cdiv(Ht, best.th) * cdiv(a.N, best.nb) * a.groups;
+  const long long steps = ntaps * cdiv(a.Cin_g, a.dtype == B200CONV_F16 ? 64 : 32);
+  const int bn_max = best.bn;
+  long long best_cost = -1;
+  for (int bn = bn_max; bn >= 32; bn /= 2) {
+    const long long total = tiles * cdiv(a.n_out, bn);
+    // a stage of the per-tap kernel is never shorter than its two TMA boxes take to issue (about 300 clocks)
+    const long long step = std::max(300, 4 * mma_clocks(bn) + 60);
+    const long long epi = 2400LL * bn / 32;
+    const int most = 2 * total <= c->num_sms ? (int)std::min<long long>(steps, c->num_sms / total) : 1;
+    for (int s = 1; s <= most; ++s) {
+      const long long cost = s == 1 ? cdiv(total, c->num_sms) * std::max(steps * step, epi) + std::min(steps * step, epi)
+                                    : cdiv(steps, s) * step + split_clocks(total * s, 128, bn, c->num_sms);
+      if (best_cost < 0 || cost < best_cost) { best_cost = cost; best.bn = bn; best.splits = s; }
+    }
+  }
+  return best;
+}
+
+// Slabs of a split launch and the parameters of its reduction that both kernels share.
+template <class P>
+int split_output(b200conv_ctx* c, Scratch& tmp, const P& p, int bn, int rows, ConvReduceParams* q) {
+  memset(q, 0, sizeof *q);
+  const long long tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  float* partial;
+  int rc = tmp.get(sizeof(float) * tiles * p.splits * rows * bn, reinterpret_cast<void**>(&partial));
+  if (rc) return rc;
+  q->partial = partial;
+  q->splits = p.splits; q->rows = rows; q->bn_cols = bn;
+  q->tiles_w = p.tiles_w; q->tiles_h = p.tiles_h; q->tiles_n = p.tiles_n; q->tiles_co = p.tiles_co; q->groups = p.groups;
+  q->Wt = p.Wt; q->Ht = p.Ht; q->Nimg = p.Nimg; q->n_out = p.n_out;
+  q->out = p.out; q->bias = p.bias;
+  q->out_sn = p.out_sn; q->out_sc = p.out_sc; q->out_sh = p.out_sh; q->out_sw = p.out_sw; q->out_off = p.out_off;
+  q->relu = p.relu;
+  q->epi = p.epi;
+  return 0;
+}
+
 // Slab variant (conv_slab.cu) for launches whose taps all read one view.  Returns 0 when it was
 // launched, 2 when the geometry does not fit (the caller then uses the per-tap kernel), or an
 // error code.
 int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps, int rh,
                   int rw, int Wt, int Ht, void* out, long long sn, long long sc, long long sh,
-                  long long sw, long long off, const void* bias, int relu) {
+                  long long sw, long long off, const void* bias, int relu, bool spread) {
   if (taps.empty() || (int)taps.size() > kMaxTaps) return 2;
+  const int ntap_all = (int)taps.size();
   int dh_min = taps[0].dh, dh_max = taps[0].dh, dw_min = taps[0].dw, dw_max = taps[0].dw;
   for (const ConvTap& t : taps) {
     dh_min = std::min<int>(dh_min, t.dh); dh_max = std::max<int>(dh_max, t.dh);
@@ -552,106 +726,23 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   const int Eh = dh_max - dh_min, Ew = dw_max - dw_min;
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
-  int BN = conv_umma_bn(a.n_out);
-#ifdef B200CONV_TUNE                       // development build: tile parameters from the environment
-  if (getenv("B200_BN") && atoi(getenv("B200_BN")) <= BN) BN = atoi(getenv("B200_BN"));
-#endif
-  const int tiles_co = (int)cdiv(a.n_out, BN);
-  const int acc_cap = std::min(512 / BN, 4);
-  // Narrow tiles (few filters) have small filter tiles and short MMAs: several taps then share one
-  // stage of the filter ring, so that a barrier round trip is paid per 16 to 32 KB of filters, not
-  // per 4 or 8 KB (the issuing warp spends about 150 clocks per stage on the hand-over, as much as
-  // the stage's MMAs take when a tap is four 128 x 64 MMAs)
-  // (measured: 64 -> 64 3x3 layers 8 to 16 % faster with a filter row per stage, the 7x7 stem 8 to 16 % with four
-  // taps; 128-filter tiles are better off with one tap per stage)
-  const int ntap_all = (int)taps.size();
-  int tps = BN <= 64 ? (ntap_all % 3 == 0 ? 3 : std::min(4, ntap_all)) : 1;
-#ifdef B200CONV_TUNE
-  if (getenv("B200_TPS")) tps = std::max(1, std::min({8, atoi(getenv("B200_TPS")), (int)taps.size()}));
-#endif
-  const int b_bytes = tps * BN * 128;
-  // search the tile (wt x th x nb) with the least serial work per SM
-  const int mma_clk = BN >= 256 ? 128 : BN == 128 ? 64 : BN == 64 ? 48 : 40;   // 128 x BN x 32-byte MMA
   const long long kblocks_n = cdiv(a.Cin_g, kBK);
-  long long best_cost = -1, best_work = 0, best_tiles = 0;
-  int b_wt = 0, b_th = 0, b_nb = 0, b_acc = 0, b_slab = 0;
   const long long es_out = (long long)elem_size(a.dtype);
   // can the output leave through tiled TMA stores at all (channels-last, whole 128-byte channel rows, aligned)?
   const bool tma_layout_ok = sc == 1 && a.n_out % (int)(128 / es_out) == 0 && !c->epi.residual &&
                              (sw * es_out) % 16 == 0 && (sh * es_out) % 16 == 0 && (sn * es_out) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es_out) % 16 == 0;
-  GeoKey tile_key{kGeoSlab, a.dtype, a.n_out, a.Cin_g, a.groups, a.N, Wt, Ht, ntap_all, Eh, Ew, tma_layout_ok ? 1 : 0,
-                  c->epi.pool, c->num_sms};
-  auto known = c->slab_tiles.find(tile_key);
-  if (known != c->slab_tiles.end() && known->second.found) {
-    const SlabTile& k = known->second;
-    b_wt = k.wt; b_th = k.th; b_nb = k.nb; b_acc = k.n_acc; b_slab = k.slab_bytes;
-    best_cost = 0;
-  }
-  for (int parts = 1; parts <= 16 && known == c->slab_tiles.end(); ++parts) {
-    const int wt = (int)cdiv(Wt, parts);
-    if (parts > 1 && wt < 8) break;
-    const int Ws = wt + Ew;
-    if (Ws > 256) continue;
-    const int shift_max = Eh * Ws + Ew;
-    for (int th = 1; th <= Ht; ++th) {
-      const int Hs = th + Eh;
-      if (Hs > 256) break;
-      const int per_img = Hs * Ws;
-      if ((th - 1) * Ws + wt - 1 >= 128 * acc_cap) break;
-      for (int nb = 1; nb <= std::min(a.N, 256); ++nb) {
-        const long long last = 1LL * (nb - 1) * per_img + (th - 1) * Ws + (wt - 1);
-        if (last >= 128LL * acc_cap) break;
-        const int n_acc = (int)(last / 128) + 1;
-        const long long rows = std::max<long long>(1LL * nb * per_img, 128LL * n_acc + shift_max);
-        const long long slab_bytes = (rows * 128 + 1023) / 1024 * 1024;
-        if (2 * slab_bytes + 2 * b_bytes > kSlabSmemBudget) break;
-        const long long tiles = cdiv(Wt, wt) * cdiv(Ht, th) * cdiv(a.N, nb);
-        const long long total = tiles * tiles_co * a.groups;
-        // clocks of the busiest SM: per tile and (tap, channel block) 4 MMAs per accumulator plus
-        // about 400 clocks of stage hand-over in the issuing thread
-        // about 400 clocks of stage hand-over in the issuing thread; then the accumulators are read
-        // out (about 1000 clocks per 128 x 32 block), beside the next tile's MMAs when two
-        // accumulator sets fit the 512 TMEM columns
-        // Epilogue: through staged TMA stores when the output is channels-last and the staging
-        // buffers fit beside two slabs and two filter stages (about 2500 clocks of latency per tile
-        // plus the tile's bytes at the SM's store rate of 32 B/clk), else lane-per-row stores from
-        // registers (1200 to 2500 clocks per 128 x 32 block: 16-byte pieces scattered over the pixel rows)
-        const long long dense_rows = 1LL * wt * th * nb;
-        const int ngr = n_acc == 3 ? 0 : 4 / n_acc;
-        const long long stg = (dense_rows * 128 + 1023) / 1024 * 1024;
-        const long long min_b = std::min<long long>(3, kblocks_n * cdiv((long long)taps.size(), tps) + 1);   // filter stages the staged epilogue insists on
-        if (c->epi.pool && ((wt | th) & 1)) continue;        // pooling windows must not straddle tiles
-        const bool tma_fit = tma_layout_ok && ngr > 0 && ngr * stg <= kSlabStageBytes &&
-                             (total <= c->num_sms ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
-                                                  : 2 * slab_bytes + min_b * b_bytes + kSlabStageBytes <= kSlabSmemBudget);
-        // plus about 1500 clocks per tile for the pipeline to fill again
-        const long long mma_part = 1LL * kblocks_n * ((long long)taps.size() * 4LL * n_acc * mma_clk + cdiv((long long)taps.size(), tps) * 120) + 1500;
-        if (c->epi.pool && !tma_fit) continue;               // pooling happens in the staged epilogue only
-        const long long epi_part = tma_fit ? 2500 + dense_rows * BN * (long long)es_out / 32 : 2400LL * n_acc * (BN / 32);
-        const long long per_tile = 2 * n_acc * BN <= 512 ? std::max(mma_part, epi_part) : mma_part + epi_part;
-        const long long cost = cdiv(total, c->num_sms) * per_tile;
-        const long long work = total * n_acc;
-        if (best_cost < 0 || cost < best_cost || (cost == best_cost && work < best_work) ||
-            (cost == best_cost && work == best_work && tiles < best_tiles)) {
-          best_cost = cost; best_work = work; best_tiles = tiles;
-          b_wt = wt; b_th = th; b_nb = nb; b_acc = n_acc; b_slab = (int)slab_bytes;
-        }
-      }
-    }
-  }
-  if (known == c->slab_tiles.end()) {
-    SlabTile& k = c->slab_tiles[tile_key];
-    k.wt = b_wt; k.th = b_th; k.nb = b_nb; k.n_acc = b_acc; k.slab_bytes = b_slab;
-    k.found = best_cost >= 0;
-  }
+  const SlabTile tile = find_slab_tile(c, a, ntap_all, Wt, Ht, Eh, Ew, tma_layout_ok, spread);
+  if (!tile.found) return 2;
+  const int BN = tile.bn, tiles_co = (int)cdiv(a.n_out, BN);
+  const int tps = slab_tps(BN, ntap_all), b_bytes = tps * BN * 128;
 #ifndef B200_PAIR_MIN_KBLOCKS
 #define B200_PAIR_MIN_KBLOCKS 4
 #endif
   constexpr long long kPairMinKblocks = B200_PAIR_MIN_KBLOCKS;
   // Flattened 1x1 layers with a deep reduction and 256-filter tiles: pairs of CTAs share the filter tile
   // (each loads half of it), which brings the operand traffic from L2 under what an SM can take.
-  if (best_cost < 0 && Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && c->use_pair &&
+  if (!spread && tile.row && c->use_pair &&
       a.dtype == B200CONV_F16 && BN == 256 && a.n_out % 64 == 0 && a.groups == 1 && !a.fold && taps.size() == 1 &&
       kblocks_n >= kPairMinKblocks && tma_layout_ok && c->num_sms >= 2 && c->epi.beta == 0.f && !c->epi.pool) {
     PairGemmParams q;
@@ -680,29 +771,19 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       return 0;
     }
   }
-  if (best_cost < 0 && Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && !c->epi.pool) {
-    // one long row of pixels without halo (a flattened 1x1 layer): whole 128-pixel accumulators,
-    // as many as still leave room for a second accumulator set
-    b_acc = BN >= 256 ? 1 : 2;
-#ifdef B200CONV_TUNE
-    if (getenv("B200_NACC")) b_acc = std::max(1, std::min(2, atoi(getenv("B200_NACC"))));
-#endif
-    b_wt = 128 * b_acc; b_th = 1; b_nb = 1;
-    b_slab = b_wt * 128;
-    best_cost = 0;
-  }
-  if (best_cost < 0) return 2;
   SlabConvParams p;
   memset(&p, 0, sizeof p);
-  p.wt = b_wt; p.th = b_th; p.nb = b_nb; p.n_acc = b_acc;
-  p.Ws = b_wt + Ew; p.Hs = b_th + Eh;
+  const int b_slab = tile.slab_bytes;
+  p.wt = tile.wt; p.th = tile.th; p.nb = tile.nb; p.n_acc = tile.n_acc;
+  p.Ws = tile.wt + Ew; p.Hs = tile.th + Eh;
   p.dw_min = dw_min; p.dh_min = dh_min;
   p.slab_bytes = b_slab;
+  p.splits = tile.splits;
   p.tps = tps;
   // Ring depths for `avail` bytes.  Activations come from HBM (the longer latency, and the stream
   // that bounds most layers): the slab ring gets up to 6 buffers once the filter ring holds what
   // one tile consumes (2 to 4 stages); the filter ring then takes what is left, up to 8 stages.
-  const int per_tile = (int)std::min<long long>(8, kblocks_n * cdiv((long long)taps.size(), tps));
+  const int per_tile = (int)std::min<long long>(8, cdiv(kblocks_n * cdiv((long long)taps.size(), tps), tile.splits));
   auto plan_rings = [&](long long avail, int* ss, int* bs) {
     if (2LL * b_slab + 2LL * b_bytes > avail) return false;
     const int fit = (int)std::min<long long>(8, (avail - 2LL * b_slab) / b_bytes);
@@ -722,7 +803,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     return true;
   };
   if (!plan_rings(kSlabSmemBudget, &p.s_stages, &p.b_stages)) return 2;
-  {
+  if (tile.splits == 1) {
     // TMA-store epilogue: channels-last output whose 128-byte channel chunks never straddle a
     // group, 1/2/4 accumulators (so that the 16 epilogue warps split into equal groups)
     const long long tiles = cdiv(Wt, p.wt) * cdiv(Ht, p.th) * cdiv(a.N, p.nb);
@@ -733,7 +814,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     const int ngroups = p.n_acc == 3 ? 0 : 4 / p.n_acc;
     const char* obase = static_cast<const char*>(out) + off * (long long)es;
     const int row_ch = (int)(128 / es);     // channels of one staged 128-byte row
-    bool ok = sc == 1 && a.n_out % row_ch == 0 && ngroups > 0 && !c->epi.residual &&
+    bool ok = sc == 1 && a.n_out % row_ch == 0 && BN >= row_ch && ngroups > 0 && !c->epi.residual &&
               ngroups * stage_bytes <= kSlabStageBytes && p.wt <= 256 && p.th <= 256 && p.nb <= 256 &&
               (sw * es) % 16 == 0 && (sh * es) % 16 == 0 && (sn * es) % 16 == 0 &&
               reinterpret_cast<uintptr_t>(obase) % 16 == 0;
@@ -803,29 +884,43 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.trace = c->trace;
 #ifdef B200CONV_TUNE
   if (getenv("B200_VERBOSE"))
-    fprintf(stderr, "slab: Wt %d Ht %d N %d Cin %d n_out %d taps %d | BN %d wt %d th %d nb %d n_acc %d slab %d s %d b %d tma %d nbuf %d cost %lld\n",
-            Wt, Ht, a.N, a.Cin_g, a.n_out, (int)taps.size(), BN, p.wt, p.th, p.nb, p.n_acc, p.slab_bytes, p.s_stages, p.b_stages,
-            p.tma_out, p.stage_nbuf, best_cost);
+    fprintf(stderr, "slab: Wt %d Ht %d N %d Cin %d n_out %d taps %d | BN %d splits %d wt %d th %d nb %d n_acc %d slab %d s %d b %d tma %d nbuf %d\n",
+            Wt, Ht, a.N, a.Cin_g, a.n_out, (int)taps.size(), BN, p.splits, p.wt, p.th, p.nb, p.n_acc, p.slab_bytes, p.s_stages, p.b_stages,
+            p.tma_out, p.stage_nbuf);
 #endif
+  if (p.splits == 1) {
+    KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
+    return 0;
+  }
+  Scratch tmp(c);
+  ConvReduceParams q;
+  if ((rc = split_output(c, tmp, p, BN, p.n_acc * 128, &q))) return rc;
+  q.Ws = p.Ws; q.Hs = p.Hs; q.wt = p.wt; q.th = p.th; q.nb = p.nb;
+  p.partial = const_cast<float*>(q.partial);
   KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
+  KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
   return 0;
 }
 
 int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps_in,
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
-                      const void* bias, int relu, bool allow_slab) {
-  if (allow_slab && view_parity.size() == 1) {
+                      const void* bias, int relu, int variant) {
+  if (variant == kConvSlab || variant == kConvSlabSpread) {
     const int rh = view_parity[0].first, rw = view_parity[0].second;
     if (rh < a.Hs && rw < a.Ws) {
-      const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu);
+      const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant == kConvSlabSpread);
       if (rc != 2) return rc;
     }
+    variant = variant == kConvSlab ? kConvTap : kConvTapSpread;
   }
   UmmaConvParams p;
   memset(&p, 0, sizeof p);
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
-  choose_tile(c, Wt, Ht, a.N, 128, 0, &p.bw, &p.bh, &p.bn);
+  const SlabTile tile = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, variant == kConvTapSpread);
+  p.bw = tile.wt; p.bh = tile.th; p.bn = tile.nb;
+  p.splits = tile.splits;
+  p.bn_cols = tile.bn;
   // views that exist (non-empty); taps pointing at empty views contribute nothing
   std::vector<int> remap(view_parity.size(), -1);
   int nviews = 0;
@@ -844,10 +939,11 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   }
   if (p.ntaps == 0) return 1;  // caller zero-fills
   for (int v = nviews; v < kMaxViews; ++v) p.views[v] = p.views[0];
-  const int BN = conv_umma_bn(a.n_out);
+  const int BN = tile.bn;
   int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN);
   if (rc) return rc;
   p.kblocks = static_cast<int>(cdiv(a.Cin_g, kBK));
+  p.splits = std::min(p.splits, p.ntaps * p.kblocks);
   p.groups = a.groups;
   p.Wt = Wt; p.Ht = Ht; p.Nimg = a.N;
   p.tiles_w = static_cast<int>(cdiv(Wt, p.bw));
@@ -862,58 +958,101 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.epi = c->epi;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
+  if (p.splits == 1) {
+    KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
+    return 0;
+  }
+  Scratch tmp(c);
+  ConvReduceParams q;
+  if ((rc = split_output(c, tmp, p, BN, 128, &q))) return rc;
+  q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
+  p.partial = const_cast<float*>(q.partial);
   KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
+  KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
   return 0;
 }
 
-// Picks between the slab kernel and the per-tap kernel.  Both compute the same thing; which one
-// is faster depends on the layer (halo rows wasted by the slab grid against activations fetched
-// once per tap), so the first call of a geometry times both with CUDA events and the context
-// remembers the winner (the reference's GPU path selects its convolution algorithm the same way,
-// theano/gpuarray/opt.py:2144-2222).  While a graph is being captured the remembered choice, or
-// the slab kernel, is used.
+// Picks the kernel variant.  All compute the same thing; which one is fastest depends on the layer (halo
+// rows wasted by the slab grid against activations fetched once per tap; few tiles per SM against a second
+// kernel that adds slices), so the first call of a geometry times the variants that apply with CUDA events
+// and the context remembers the winner (the reference's GPU path selects its convolution algorithm the same
+// way, theano/gpuarray/opt.py:2144-2222).  While a graph is being captured, or with timing off, the remembered
+// choice or the model's is used.
 int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps_in,
                   const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                   long long sn, long long sc, long long sh, long long sw, long long off,
                   const void* bias, int relu, bool allow_slab = true) {
-  if (c->epi.pool) {                  // only the slab kernel's staged epilogue pools
-    if (!allow_slab || view_parity.size() != 1) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
-    const int rh = view_parity[0].first, rw = view_parity[0].second;
-    const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu);
-    return rc == 2 ? fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool") : rc;
-  }
-  if (!allow_slab || view_parity.size() != 1 || !c->autotune)
-    return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, allow_slab);
+  if (view_parity.size() != 1) allow_slab = false;
+  auto run = [&](int variant) -> int {
+    if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
+      const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
+                                   relu, variant == kConvSlabSpread);
+      return rc == 2 ? fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool") : rc;
+    }
+    return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant);
+  };
   int tsum = 0;
   for (const ConvTap& t : taps_in) tsum = tsum * 31 + t.dh * 7 + t.dw;
   GeoKey key{kGeoConv, a.dtype, a.N, a.Hs, a.Ws, a.Cin_g, a.n_out, a.groups, Wt, Ht, a.view_sH, a.view_sW, (int)taps_in.size(), tsum};
   key.add(sc);
   key.add(sw);
-  auto it = c->algo_cache.find(key);
-  if (it != c->algo_cache.end())
-    return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, it->second);
-  if (c->capturing)
-    return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true);
-  float ms[2] = {0.f, 0.f};
+  key.add(c->epi.pool * 2 + (allow_slab ? 1 : 0));
+  if (c->autotune) {
+    auto it = c->algo_cache.find(key);
+    if (it != c->algo_cache.end()) return run(it->second);
+  }
+  // the variants that apply, the static preference last
+  int cand[kConvVariants], ncand = 0;
+  const SlabTile narrow = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, true);
+  const bool tap_spread = narrow.splits > 1 || narrow.bn != conv_umma_bn(a.n_out);
+  if (!c->epi.pool) {
+    cand[ncand++] = kConvTap;
+    if (tap_spread) cand[ncand++] = kConvTapSpread;
+  }
+  if (c->epi.pool && !allow_slab) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+  if (allow_slab) {
+    int eh[2] = {0, 0}, ew[2] = {0, 0};
+    for (size_t i = 0; i < taps_in.size(); ++i) {
+      const ConvTap& t = taps_in[i];
+      if (i == 0) { eh[0] = eh[1] = t.dh; ew[0] = ew[1] = t.dw; }
+      eh[0] = std::min<int>(eh[0], t.dh); eh[1] = std::max<int>(eh[1], t.dh);
+      ew[0] = std::min<int>(ew[0], t.dw); ew[1] = std::max<int>(ew[1], t.dw);
+    }
+    const size_t es = elem_size(a.dtype);
+    const bool tma = sc == 1 && a.n_out % (int)(128 / es) == 0 && !c->epi.residual && (sw * es) % 16 == 0 && (sh * es) % 16 == 0 &&
+                     (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
+    const SlabTile w = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, false);
+    const SlabTile n = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, true);
+    if (w.found) cand[ncand++] = kConvSlab;
+    if (n.found && (!w.found || n.splits > 1 || n.bn != w.bn || n.wt != w.wt || n.th != w.th || n.nb != w.nb)) cand[ncand++] = kConvSlabSpread;
+  }
+  if (ncand == 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+  if (!c->autotune || c->capturing || ncand == 1) return run(cand[ncand - 1]);
   if (!c->ev_tune0) {
     CU_OK(c, cudaEventCreate(&c->ev_tune0));
     CU_OK(c, cudaEventCreate(&c->ev_tune1));
   }
-  for (int variant = 0; variant < 2; ++variant) {        // 0: per tap, 1: slab; two runs each, keep the second
-    for (int rep = 0; rep < 2; ++rep) {
+  int best = -1;
+  float best_ms = 0.f;
+  for (int i = 0; i < ncand; ++i) {                       // a warm-up run and two timed ones each
+    float ms = 0.f;
+    for (int rep = 0; rep < 3; ++rep) {
+      float m;
       CU_OK(c, cudaEventRecord(c->ev_tune0, c->stream));
-      int rc = run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant == 1);
+      const int rc = run(cand[i]);
+      if (rc == B200CONV_E_UNSUPPORTED && c->epi.pool && ncand > 1) { ms = -1.f; break; }
       if (rc) return rc;
       CU_OK(c, cudaEventRecord(c->ev_tune1, c->stream));
       CU_OK(c, cudaStreamSynchronize(c->stream));
-      CU_OK(c, cudaEventElapsedTime(&ms[variant], c->ev_tune0, c->ev_tune1));
+      CU_OK(c, cudaEventElapsedTime(&m, c->ev_tune0, c->ev_tune1));
+      if (rep == 1 || (rep == 2 && m < ms)) ms = m;
     }
+    if (ms >= 0.f && (best < 0 || ms < best_ms)) { best = cand[i]; best_ms = ms; }
   }
-  const bool slab = ms[1] <= ms[0];
-  c->algo_cache[key] = slab;
-  if (!slab)   // the last run was the slab kernel: leave the output of the chosen kernel (identical up to rounding order)
-    return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, false);
-  return 0;
+  if (best < 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+  c->algo_cache[key] = best;
+  // the last run may have been another variant: leave the output of the chosen one (identical up to rounding order)
+  return best == cand[ncand - 1] ? 0 : run(best);
 }
 
 int to_nhwc(b200conv_ctx* c, Scratch& tmp, const void* src, int N, int C, int H, int W, int dtype,
@@ -2781,7 +2920,7 @@ int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
   FILE* f = fopen(path, "w");
   if (!f) return fail(c, B200CONV_E_INVALID, "cannot write %s", path);
   fprintf(f, "%s\n", tuning_header(c).c_str());
-  for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.text().c_str(), kv.second ? 1 : 0);
+  for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.text().c_str(), kv.second);
   for (auto& kv : c->split_cache) fprintf(f, "s %s %d\n", kv.first.text().c_str(), kv.second);
   fclose(f);
   return 0;
@@ -2811,7 +2950,7 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
     int val = 0;
     GeoKey key{};
     if (sscanf(line, "%c %399s %d", &kind, text, &val) != 3 || !GeoKey::parse(text, &key)) continue;
-    if (kind == 'a') { c->algo_cache[key] = val != 0; ++n; }
+    if (kind == 'a' && val >= 0 && val < kConvVariants) { c->algo_cache[key] = val; ++n; }
     else if (kind == 's' && val >= 1) { c->split_cache[key] = val; ++n; }
   }
   fclose(f);

@@ -66,7 +66,17 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   const uint32_t slab_tx = static_cast<uint32_t>(p.nb * p.Hs * p.Ws) * 128u;
   // tile counts fit 32 bits (the launcher checks): 64-bit divisions per tile would cost each
   // role about a thousand clocks, a fifth of a small tile
-  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
+  // Work item = (tile, slice of the reduction), the slices of a tile side by side.  A slice is a range of
+  // filter stages (channel block x group of tps taps), in the order the unsplit loop walks them.
+  const uint32_t splits = p.splits;
+  const uint32_t stages_kb = (p.ntaps + p.tps - 1) / p.tps, stages_all = stages_kb * p.kblocks;
+  struct Range { int kb0, kb1, tg0, tg1; };        // channel blocks kb0..kb1, tap groups from tg0 in the first, up to tg1 in the last (inclusive)
+  auto slice_range = [&](uint32_t slice) {
+    if (splits == 1) return Range{0, p.kblocks - 1, 0, static_cast<int>(stages_kb) - 1};
+    const uint32_t a = stages_all * slice / splits, b = stages_all * (slice + 1) / splits - 1;
+    return Range{static_cast<int>(a / stages_kb), static_cast<int>(b / stages_kb), static_cast<int>(a % stages_kb), static_cast<int>(b % stages_kb)};
+  };
   const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
   const bool dbl = 2 * p.n_acc * BN <= 512;
   const int issuers = p.n_acc >= 2 ? 2 : 1;
@@ -109,13 +119,15 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     int sb = 0;
     uint32_t sphase = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
+      const uint32_t t = item / splits;
+      const Range r = slice_range(item - t * splits);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
       const uint32_t pt = t / co_groups;
       const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
       const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.th;
       const int n0 = (pt / tiles_wh) * p.nb;
-      for (int kb = 0; kb < p.kblocks; ++kb) {
+      for (int kb = r.kb0; kb <= r.kb1; ++kb) {
         if (!uniform_wait(&bars->slab_empty[sb], sphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (leader) {
           mbar_expect_tx(&bars->slab_full[sb], slab_tx);
@@ -133,11 +145,14 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     int bs = 0;
     uint32_t bphase = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
+      const uint32_t t = item / splits;
+      const Range r = slice_range(item - t * splits);
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      for (int kb = 0; kb < p.kblocks && ok; ++kb) {
-        for (int tap = 0; tap < p.ntaps; tap += p.tps) {
+      for (int kb = r.kb0; kb <= r.kb1 && ok; ++kb) {
+        const int tap_end = kb == r.kb1 ? min(p.ntaps, (r.tg1 + 1) * p.tps) : p.ntaps;
+        for (int tap = kb == r.kb0 ? r.tg0 * p.tps : 0; tap < tap_end; tap += p.tps) {
           if (!uniform_wait(&bars->b_empty[bs], bphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
           const int nt = min(p.tps, p.ntaps - tap);         // taps of this stage
           if (leader) {
@@ -172,7 +187,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const uint64_t desc_bits = smem_desc(0, 16, 1024);
       const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
       const uint32_t desc_lo = static_cast<uint32_t>(desc_bits);
-      for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
+      for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+        const Range r = slice_range(item % splits);
         // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
         // runs beside the MMAs of the next one
         const int buf = dbl ? (it & 1) : 0;
@@ -182,13 +198,15 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (trace) tw_acc += clock64() - tq;
         tc_fence_after();
-        for (int kb = 0; kb < p.kblocks && ok; ++kb) {
+        for (int kb = r.kb0; kb <= r.kb1 && ok; ++kb) {
           tq = trace ? clock64() : 0;
           if (!uniform_wait(&bars->slab_full[sb], sphase, bars, p.wait_clocks)) { ok = false; break; }
           if (trace) tw_slab += clock64() - tq;
-          if (trace && it == 0 && kb == 0) trace[2] = clock64();
+          if (trace && it == 0 && kb == r.kb0) trace[2] = clock64();
           const uint32_t sbase = smem_u32(smem + sb * p.slab_bytes);
-          for (int tap0 = 0; tap0 < p.ntaps; tap0 += p.tps) {
+          const int tap_begin = kb == r.kb0 ? r.tg0 * p.tps : 0;
+          const int tap_end = kb == r.kb1 ? min(p.ntaps, (r.tg1 + 1) * p.tps) : p.ntaps;
+          for (int tap0 = tap_begin; tap0 < tap_end; tap0 += p.tps) {
             tq = trace ? clock64() : 0;
             if (!uniform_wait(&bars->b_full[bs], bphase, bars, p.wait_clocks)) { ok = false; break; }
             if (trace) tw_b += clock64() - tq;
@@ -199,7 +217,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
                 const int tap = tap0 + q;
                 // only the address field of the two descriptors changes from MMA to MMA
                 const uint32_t b_lo = desc_lo + (smem_u32(bring + bs * stage_b + q * kBBytes) >> 4);
-                const uint32_t first = (kb | tap) != 0;
+                const uint32_t first = kb != r.kb0 || tap != tap_begin;      // 0 for the slice's first products
                 uint32_t a_lo = desc_lo + ((sbase + static_cast<uint32_t>(p.tap_shift[tap] + 128 * a_begin) * 128u) >> 4);
                 for (int a = a_begin; a < a_end; ++a) {
 #pragma unroll
@@ -239,7 +257,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     long long te_wait = 0, te_busy = 0;          // clocks of thread 64 (only with trace)
     long long tp[5] = {0, 0, 0, 0, 0};           // its epilogue phases: buffer wait, TMEM read, convert + stage, fence + barrier, store issue
     int nstore = 0;                              // chunks this warp's group has staged so far
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+      const uint32_t t = item / splits;
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
       const uint32_t pt = t / co_groups;
@@ -257,7 +276,26 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const int nchunks = min(BN / 32, (p.n_out - co_base + 31) / 32);
       const uint32_t lane_base = tmem + buf * (p.n_acc * BN) + (static_cast<uint32_t>(quad * 32) << 16);
 
-      if (p.tma_out) {
+      if (splits > 1) {
+        // raw accumulators; conv_reduce.cu adds the slices and applies the epilogue
+        const int rows = p.n_acc * 128;
+        for (int a = 0; a < p.n_acc; ++a) {
+          const int pos = a * 128 + quad * 32 + lane, rem = pos % per_img;
+          const bool inbox = pos / per_img < p.nb && rem / p.Ws < p.th && rem % p.Ws < p.wt;
+          float4* dst = reinterpret_cast<float4*>(p.partial) + static_cast<long long>(item) * rows * (BN / 4) + pos;
+#pragma unroll 1
+          for (int ch = sub; ch < nchunks; ch += kEpilogueWarps / 4) {
+            uint32_t r[32];
+            tmem_ld32(lane_base + a * BN + ch * 32, r);
+            tmem_ld_wait();
+            if (!inbox) continue;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              dst[(ch * 8 + j) * rows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                     __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+          }
+        }
+      } else if (p.tma_out) {
         // Groups of 4 * n_acc warps take whole 128-byte channel chunks of the tile: lane -> its pixel's
         // dense row of a staging buffer (16-byte pieces swizzled like the store map expects),
         // then one thread stores the box.  Bias and ReLU are applied on the way.  A group owns
@@ -512,7 +550,7 @@ cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cu
 }  // namespace
 
 cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num_sms, cudaStream_t s) {
-  const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
   if (total == 0 || p.ntaps == 0) return cudaSuccess;
   if (total >= (1LL << 31)) return cudaErrorInvalidValue;
   const bool f16 = dtype == B200CONV_F16;

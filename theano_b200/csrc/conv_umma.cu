@@ -74,10 +74,11 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int rows_used = p.bw * p.bh * p.bn;
   const uint32_t tx_bytes = rows_used * kRowBytes + BN * kRowBytes;
-  const int kiters = p.ntaps * p.kblocks;
+  const uint32_t kiters = p.ntaps * p.kblocks;
   // tile counts fit 32 bits (the launcher checks): 64-bit divisions per tile would cost each
   // role about a thousand clocks, a fifth of a small tile
-  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
+  const uint32_t splits = p.splits;            // work item = (tile, slice of the reduction), slices of a tile side by side
   const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
 
   if (threadIdx.x == 0) {
@@ -118,16 +119,19 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     int stage = 0;
     uint32_t phase = 0, idx = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
+      const uint32_t t = item / splits, slice = item - t * splits;
+      const uint32_t k0 = kiters * slice / splits, k1 = kiters * (slice + 1) / splits;
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
       const uint32_t pt = t / co_groups;
       const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.bw;
       const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.bh;
       const int n0 = (pt / tiles_wh) * p.bn;
-      for (int tap = 0; tap < p.ntaps && ok; ++tap) {
+      uint32_t k = k0;
+      for (int tap = k0 / p.kblocks, kb = k0 % p.kblocks; k < k1 && ok; ++tap, kb = 0) {
         const ConvTap tp = p.taps[tap];
-        for (int kb = 0; kb < p.kblocks; ++kb, ++idx) {
+        for (; kb < p.kblocks && k < k1; ++kb, ++idx, ++k) {
           if ((idx & 1) == my_parity) {
             if (!uniform_wait(&bars->empty[stage], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
             uint8_t* sa = smem + stage * stage_bytes<BN>();
@@ -156,13 +160,14 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const uint64_t desc_bits = smem_desc(0, 16, 1024);
     const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
     const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+      const uint32_t slice = item % splits, k0 = kiters * slice / splits, k1 = kiters * (slice + 1) / splits;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem + buf * BN;
-      for (int k = 0; k < kiters; ++k) {
+      for (uint32_t k = k0; k < k1; ++k) {
         if (!uniform_wait(&bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
         // 8 tf32 / 16 f16 channels = 32 bytes along the swizzled row per MMA: only the address
@@ -172,7 +177,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         if (leader) {
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_words<KIND>(d_tmem, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, (k | kk) != 0);
+            umma_words<KIND>(d_tmem, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, k != k0 || kk != 0);
           umma_commit(&bars->empty[stage]);
         }
         if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -192,7 +197,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT)) & 15) == 0;
     bool ok = true;
     int it = 0;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++it) {
+    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+      const uint32_t t = item / splits;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
@@ -207,6 +213,20 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       OutT* pix = out + (p.out_off + n * p.out_sn + h * p.out_sh + w * p.out_sw) + 1LL * g * p.n_out * p.out_sc;
       const OutT* res = p.epi.residual ? static_cast<const OutT*>(p.epi.residual) + (pix - out) : nullptr;
       const int co_base = co_t * BN;
+      if (splits > 1) {       // raw accumulators; conv_reduce.cu adds the slices and applies the epilogue
+        float4* dst = reinterpret_cast<float4*>(p.partial) + static_cast<long long>(item) * (kRows * BN / 4) + row;
+#pragma unroll 1
+        for (int ch = sub; ch < BN / 32 && co_base + ch * 32 < p.n_out; ch += kEpilogueWarps / 4) {
+          uint32_t r[32];
+          tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
+          tmem_ld_wait();
+          if (!valid) continue;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            dst[(ch * 8 + j) * kRows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                    __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        }
+      } else
 #pragma unroll 1
       for (int ch = sub; ch < BN / 32; ch += kEpilogueWarps / 4) {
         const int co0 = co_base + ch * 32;          // first channel (within the group) of the chunk
@@ -289,16 +309,15 @@ cudaError_t launch_one(const UmmaConvParams& p, long long total, int num_sms, cu
 int conv_umma_bn(int n_out) { return n_out <= 32 ? 32 : n_out <= 64 ? 64 : n_out <= 128 ? 128 : 256; }
 
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s) {
-  const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
   if (total == 0 || p.ntaps == 0) return cudaSuccess;
   if (total >= (1LL << 31)) return cudaErrorInvalidValue;
-  const int bn = conv_umma_bn(p.n_out);
   const bool f16 = dtype == B200CONV_F16;
 #define B200_CASE(BNV)                                                                  \
   case BNV:                                                                             \
     return f16 ? launch_one<MmaKind::F16, BNV>(p, total, num_sms, s)                    \
                : launch_one<MmaKind::TF32, BNV>(p, total, num_sms, s);
-  switch (bn) {
+  switch (p.bn_cols) {
     B200_CASE(32)
     B200_CASE(64)
     B200_CASE(128)

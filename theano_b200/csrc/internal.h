@@ -107,6 +107,9 @@ struct alignas(64) UmmaConvParams {
   ConvTap taps[kMaxTaps];
   int ntaps;
   int kblocks;                   // ceil(reduction channels per group / channels per stage)
+  int bn_cols;                   // accumulator columns of a tile (32, 64, 128 or 256)
+  int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
+  float* partial;
   int groups;
   int Wt, Ht, Nimg;              // extent of the output pixel grid this launch covers
   int bw, bh, bn;                // pixel tile (bw*bh*bn <= 128 rows of the accumulator)
@@ -122,8 +125,7 @@ struct alignas(64) UmmaConvParams {
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
 };
 
-// Launches the kernel for `total tiles`; kind: 0 = tf32 (float32 data), 1 = f16.
-int conv_umma_bn(int n_out);      // accumulator columns used for n_out outputs per group
+int conv_umma_bn(int n_out);      // accumulator columns that hold n_out outputs per group, at most 256
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s);
 
 // ---- implicit GEMM with one activation slab per channel block (conv_slab.cu) ---------------
@@ -146,6 +148,8 @@ struct alignas(64) SlabConvParams {
   int slab_bytes;                // bytes of one slab buffer (1024-byte multiple)
   int b_stages;                  // filter-tile ring depth
   int s_stages;                  // slab ring depth (2 .. 6)
+  int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
+  float* partial;
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
   int n_out;
   void* out;
@@ -172,6 +176,23 @@ constexpr int kSlabStageBytes = 64 * 1024;    // staging buffers of the TMA-stor
 constexpr int kSlabSmemBudget = 220 * 1024;   // slab buffers + filter ring; the rest of the 227 KB
                                               // holds barriers and the epilogue's transpose tiles
 cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num_sms, cudaStream_t s);
+
+// ---- reductions split over CTAs (conv_reduce.cu) --------------------------------------------
+// The tile geometry is that of the slab kernel (rows of a tile on a grid of Ws x Hs positions per image, of
+// which wt x th are the tile's); for the per-tap kernel Ws = wt and Hs = th.
+struct ConvReduceParams {
+  const float* partial;          // [tile][slice][bn_cols / 4][rows][4]
+  int splits, rows, bn_cols;
+  int Ws, Hs, wt, th, nb;
+  int tiles_w, tiles_h, tiles_n, tiles_co, groups;
+  int Wt, Ht, Nimg, n_out;
+  void* out;                     // strides of the pooled tensor when epi.pool
+  const void* bias;
+  long long out_sn, out_sc, out_sh, out_sw, out_off;
+  int relu;
+  ConvEpilogue epi;
+};
+cudaError_t launch_conv_reduce(const ConvReduceParams& p, int dtype, cudaStream_t s);
 
 // ---- 1x1 layers on CTA pairs (gemm_pair.cu): float16, tiles of 256 pixels x 256 filters ------------
 struct alignas(64) PairGemmParams {
