@@ -452,13 +452,13 @@ int make_view(b200conv_ctx* c, CUtensorMap* m, const void* base, int dtype, int 
   return 0;
 }
 
-// 3-D map over packed filters [mats][rows][ldc]: (cols, rows, mats), box (box_c, box_r, 1).
+// 3-D map over packed filters [mats][rows][ldc]: (cols, rows, mats), box (box_c, box_r, box_m).
 int make_wmap(b200conv_ctx* c, CUtensorMap* m, const void* base, int dtype, int cols, int rows,
-              int mats, int ldc, int box_c, int box_r) {
+              int mats, int ldc, int box_c, int box_r, int box_m = 1) {
   const size_t es = elem_size(dtype);
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)mats};
   cuuint64_t strides[2] = {(cuuint64_t)ldc * es, (cuuint64_t)rows * ldc * es};
-  cuuint32_t box[3] = {(cuuint32_t)box_c, (cuuint32_t)box_r, 1};
+  cuuint32_t box[3] = {(cuuint32_t)box_c, (cuuint32_t)box_r, (cuuint32_t)box_m};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = c->encode(m, dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
                          3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -861,7 +861,9 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   int rc = make_act_view(c, &p.view, a, rh, rw, kBK, p.Ws, p.Hs, p.nb);
   if (rc) return rc;
-  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN);
+  p.tap_boxes = a.groups != 1;
+  for (size_t i = 1; i < taps.size(); ++i) p.tap_boxes |= taps[i].wmat != taps[i - 1].wmat + 1;
+  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN, p.tap_boxes ? 1 : tps);
   if (rc) return rc;
   for (const ConvTap& t : taps) {
     p.tap_shift[p.ntaps] = (int16_t)((t.dh - dh_min) * p.Ws + (t.dw - dw_min));
@@ -972,6 +974,32 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   return 0;
 }
 
+// Time of one variant in milliseconds (run() enqueues it and returns 0 or an error code).  Short launches are
+// timed in bursts of up to 8 back to back, the way a program issues them: alone, between two events, a kernel
+// of 5 us costs 5 us more and the chained launch hides nothing, and the choice then is noise.
+template <class Run>
+int time_variant(b200conv_ctx* c, Run run, float* ms) {
+  if (!c->ev_tune0) {
+    CU_OK(c, cudaEventCreate(&c->ev_tune0));
+    CU_OK(c, cudaEventCreate(&c->ev_tune1));
+  }
+  *ms = -1.f;
+  int reps = 1;
+  for (int round = 0; round < 4; ++round) {               // warm-up, a first estimate, two measurements
+    CU_OK(c, cudaEventRecord(c->ev_tune0, c->stream));
+    for (int i = 0; i < reps; ++i)
+      if (int rc = run()) return rc;
+    CU_OK(c, cudaEventRecord(c->ev_tune1, c->stream));
+    CU_OK(c, cudaStreamSynchronize(c->stream));
+    float m;
+    CU_OK(c, cudaEventElapsedTime(&m, c->ev_tune0, c->ev_tune1));
+    if (round == 1) reps = std::max(1, std::min(8, (int)(0.16f / std::max(m, 0.001f))));
+    if (round >= 2 && (*ms < 0.f || m / reps < *ms)) *ms = m / reps;
+    if (round == 1 && m > 0.5f) { *ms = m; break; }       // long enough for one measurement
+  }
+  return 0;
+}
+
 // Picks the kernel variant.  All compute the same thing; which one is fastest depends on the layer (halo
 // rows wasted by the slab grid against activations fetched once per tap; few tiles per SM against a second
 // kernel that adds slices), so the first call of a geometry times the variants that apply with CUDA events
@@ -1028,25 +1056,13 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   if (ncand == 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
   if (!c->autotune || c->capturing || ncand == 1) return run(cand[ncand - 1]);
-  if (!c->ev_tune0) {
-    CU_OK(c, cudaEventCreate(&c->ev_tune0));
-    CU_OK(c, cudaEventCreate(&c->ev_tune1));
-  }
   int best = -1;
   float best_ms = 0.f;
-  for (int i = 0; i < ncand; ++i) {                       // a warm-up run and two timed ones each
-    float ms = 0.f;
-    for (int rep = 0; rep < 3; ++rep) {
-      float m;
-      CU_OK(c, cudaEventRecord(c->ev_tune0, c->stream));
-      const int rc = run(cand[i]);
-      if (rc == B200CONV_E_UNSUPPORTED && c->epi.pool && ncand > 1) { ms = -1.f; break; }
-      if (rc) return rc;
-      CU_OK(c, cudaEventRecord(c->ev_tune1, c->stream));
-      CU_OK(c, cudaStreamSynchronize(c->stream));
-      CU_OK(c, cudaEventElapsedTime(&m, c->ev_tune0, c->ev_tune1));
-      if (rep == 1 || (rep == 2 && m < ms)) ms = m;
-    }
+  for (int i = 0; i < ncand; ++i) {
+    float ms;
+    const int rc = time_variant(c, [&] { return run(cand[i]); }, &ms);
+    if (rc == B200CONV_E_UNSUPPORTED && c->epi.pool && ncand > 1) continue;
+    if (rc) return rc;
     if (ms >= 0.f && (best < 0 || ms < best_ms)) { best = cand[i]; best_ms = ms; }
   }
   if (best < 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
@@ -1074,6 +1090,19 @@ int merge_factor(const b200conv_desc& d) {
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;
   int best = 1;
   for (int m = 2; m <= d.groups && Cg * m <= kBK && Kg * m <= 256; ++m)
+    if (d.groups % m == 0) best = m;
+  return best;
+}
+
+// The same for gradWeights, whose MMAs are 128 filters x channels: merging until both fill 128 leaves fewer,
+// fuller MMAs and reads each operand row once instead of in 32-channel pieces (the off-diagonal blocks cost
+// nothing extra: they fill rows and columns that would be empty).  32 groups of 8 -> 8 channels, 256 images of
+// 28 x 28, float32: 590 us at one reduction block per group, 190 us at 128 channels.
+int merge_factor_wgrad(const b200conv_desc& d) {
+  if (d.groups <= 1 || d.C == 0 || d.K == 0) return 1;
+  const int Cg = d.C / d.groups, Kg = d.K / d.groups;
+  int best = 1;
+  for (int m = 2; m <= d.groups && Cg * m <= 128 && Kg * m <= 128; ++m)
     if (d.groups % m == 0) best = m;
   return best;
 }
@@ -1565,24 +1594,13 @@ int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long lo
   if (!c->autotune || c->capturing) return s0;
   int cand[3] = {s0, valid_splits(pix_tiles, std::min<long long>(cap, std::max(1, s0 / 2))),
                  valid_splits(pix_tiles, std::min<long long>(cap, 2LL * s0))};
-  if (!c->ev_tune0) {
-    if (cudaEventCreate(&c->ev_tune0) != cudaSuccess || cudaEventCreate(&c->ev_tune1) != cudaSuccess)
-      return fail(c, B200CONV_E_CUDA, "event creation failed");
-  }
   int best = s0;
   float best_ms = -1.f;
   for (int i = 0; i < 3; ++i) {
     if (i > 0 && (cand[i] == cand[0] || (i == 2 && cand[2] == cand[1]))) continue;
-    float ms = 0.f;
-    for (int rep = 0; rep < 2; ++rep) {
-      Scratch trial(c);
-      cudaEventRecord(c->ev_tune0, c->stream);
-      int rc = run(cand[i], trial);
-      if (rc) return rc < 0 ? rc : -rc;
-      cudaEventRecord(c->ev_tune1, c->stream);
-      if (cudaStreamSynchronize(c->stream) != cudaSuccess) return fail(c, B200CONV_E_CUDA, "synchronisation failed while tuning");
-      cudaEventElapsedTime(&ms, c->ev_tune0, c->ev_tune1);
-    }
+    float ms;
+    const int rc = time_variant(c, [&] { Scratch trial(c); return run(cand[i], trial); }, &ms);
+    if (rc) return rc < 0 ? rc : -rc;
     if (best_ms < 0.f || ms < best_ms) { best_ms = ms; best = cand[i]; }
   }
   c->split_cache[key] = best;
@@ -1750,7 +1768,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   b200conv_desc flat;
   if (!(flags & B200CONV_FORCE_DIRECT) && flatten_1x1(d, x_nhwc && dy_nhwc, &flat))
     return wgrad_device(c, flat, x, dy, dw, flags);
-  const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor(d);
+  const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor_wgrad(d);
   if (mg > 1) {
     b200conv_desc dm = d;
     dm.groups = d.groups / mg;
@@ -1935,30 +1953,14 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if (itc != c->algo_cache.end()) {
       try_group = itc->second;
     } else if (!c->capturing) {
-      if (!c->ev_tune0) {
-        CU_OK(c, cudaEventCreate(&c->ev_tune0));
-        CU_OK(c, cudaEventCreate(&c->ev_tune1));
-      }
       float ms[2] = {0.f, 0.f};
-      bool covered = true;
-      for (int variant = 0; variant < 2 && covered; ++variant) {   // 0: one tap per item, 1: tap groups
-        for (int rep = 0; rep < 2; ++rep) {
-          CU_OK(c, cudaEventRecord(c->ev_tune0, c->stream));
-          if (variant) {
-            // own scratch, returned to the pool after each run: the second run then reuses the
-            // first one's buffers and its timing holds no allocation
-            Scratch trial(c);
-            rc = wgrad_grouped(c, d, xin, gin, dw, flags, trial);
-          } else {
-            rc = wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC);
-          }
-          if (rc == 2) { covered = false; break; }
-          if (rc) return rc;
-          CU_OK(c, cudaEventRecord(c->ev_tune1, c->stream));
-          CU_OK(c, cudaStreamSynchronize(c->stream));
-          CU_OK(c, cudaEventElapsedTime(&ms[variant], c->ev_tune0, c->ev_tune1));
-        }
-      }
+      // own scratch, returned to the pool after each run: the next run then reuses the buffers and its timing
+      // holds no allocation
+      rc = time_variant(c, [&] { Scratch trial(c); return wgrad_grouped(c, d, xin, gin, dw, flags, trial); }, &ms[1]);
+      const bool covered = rc != 2;
+      if (covered && rc) return rc;
+      if (covered && (rc = time_variant(c, [&] { return wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC); }, &ms[0])))
+        return rc;
       try_group = covered && ms[1] <= ms[0];
       c->algo_cache[key] = try_group;
     }

@@ -156,10 +156,18 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           if (!uniform_wait(&bars->b_empty[bs], bphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
           const int nt = min(p.tps, p.ntaps - tap);         // taps of this stage
           if (leader) {
-            mbar_expect_tx(&bars->b_full[bs], nt * kBBytes);
-            for (int q = 0; q < nt; ++q)
-              tma_load_3d(bring + bs * stage_b + q * kBBytes, &p.wmap, &bars->b_full[bs], kb * kBK, co_t * BN,
-                          p.tap_wmat[tap + q] * p.groups + g);
+            // A box takes the issuing thread about 400 clocks whatever its size, as long as the MMAs of two
+            // 128 x 64 taps: neighbouring taps come as one box.  (The box of a last, shorter group reads on into
+            // the next matrix or zeros; its bytes count too.)
+            if (!p.tap_boxes) {
+              mbar_expect_tx(&bars->b_full[bs], p.tps * kBBytes);
+              tma_load_3d(bring + bs * stage_b, &p.wmap, &bars->b_full[bs], kb * kBK, co_t * BN, p.tap_wmat[tap]);
+            } else {
+              mbar_expect_tx(&bars->b_full[bs], nt * kBBytes);
+              for (int q = 0; q < nt; ++q)
+                tma_load_3d(bring + bs * stage_b + q * kBBytes, &p.wmap, &bars->b_full[bs], kb * kBK, co_t * BN,
+                            p.tap_wmat[tap + q] * p.groups + g);
+            }
           }
           if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
         }

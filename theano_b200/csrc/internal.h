@@ -150,6 +150,8 @@ struct alignas(64) SlabConvParams {
   int s_stages;                  // slab ring depth (2 .. 6)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
   float* partial;
+  int tap_boxes;                 // 1: one TMA box per tap; 0: the taps of a stage are neighbours in the packed filters
+                                 // and arrive as one box (the map's box then is tps matrices deep)
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
   int n_out;
   void* out;
