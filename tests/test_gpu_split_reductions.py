@@ -1,0 +1,148 @@
+"""Forward and gradInputs of few output tiles (narrow tiles, reductions split over CTAs), the pad channels of
+channels-last outputs, and tensors that start off the 16-byte boundaries."""
+import numpy as np
+import pytest
+
+from oracle import corr_oracle as O
+from theano_b200 import shim
+
+pytestmark = pytest.mark.gpu
+T = shim.DeviceTensor
+DTYPES = pytest.mark.parametrize("dtype", [np.float32, np.float16], ids=["f32", "f16"])
+TOL = {np.float32: 5e-3, np.float16: 2e-2}      # the repository's bounds: TF32 factors, float16 tensors
+
+
+@pytest.fixture
+def ctx():
+    """A context that takes the model's choice of kernel, which is the spread variant wherever there is one."""
+    c = shim.Context(0)
+    c.set_autotune(False)
+    yield c
+    c.close()
+
+
+def stored(t):
+    """A channels-last tensor as it lies in memory, pad channels included."""
+    n, _, h, w = t.shape
+    a = np.empty((n, h, w, t.stored_channels), t.dtype)
+    t.ctx.d2h(a, t.ptr)
+    t.ctx.sync()
+    return a
+
+
+# one or a few images, reductions from one step to 144; filters below, at and above a tile's columns
+SPLIT = [((1, 512, 14, 14), 512, 3, 1), ((1, 512, 7, 7), 75, 3, 1), ((2, 33, 9, 5), 20, 5, 1), ((1, 64, 8, 8), 32, 1, 1),
+         ((1, 1000, 6, 7), 257, 1, 1), ((3, 130, 13, 11), 129, 3, 2), ((1, 8, 3, 3), 5, 3, 1), ((1, 2048, 1, 1), 64, 1, 1)]
+
+
+@DTYPES
+@pytest.mark.parametrize("flags", [0, shim.NO_SLAB], ids=["slab", "tap"])
+@pytest.mark.parametrize("xs,k,ks,s", SPLIT, ids=lambda v: str(v).replace(" ", ""))
+def test_split_reductions_against_oracle(ctx, dtype, flags, xs, k, ks, s):
+    rs = np.random.RandomState(k)
+    x = rs.standard_normal(xs).astype(dtype)
+    w = (rs.standard_normal((k, xs[1], ks, ks)) / np.sqrt(xs[1] * ks * ks)).astype(dtype)
+    b = rs.standard_normal(k).astype(dtype)
+    kw = dict(border_mode="half", subsample=(s, s))
+    f = np.float32
+    X, W, B = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), T.from_host(ctx, b.reshape(1, k, 1, 1))
+    conv = O.conv2d(x.astype(f), w.astype(f), **kw)
+    dy = rs.standard_normal(conv.shape).astype(dtype)
+    R = DY = T.from_host(ctx, dy, "nhwc")
+    y = shim.device_conv2d(X, W, bias=B, residual=R, relu=True, slope=0.1, alpha=0.5, beta=2., flags=flags, **kw)
+    v = 0.5 * conv + b.astype(f)[None, :, None, None] + 2 * dy.astype(f)
+    assert O.rel_err(y.to_host().astype(f), np.where(v > 0, v, 0.1 * v)) < TOL[dtype]
+    assert not stored(y)[..., k:].any()
+    dx = shim.device_grad_inputs(W, DY, xs[2:], flags=flags, **kw)
+    assert O.rel_err(dx.to_host().astype(f), O.conv2d_grad_inputs(w.astype(f), dy.astype(f), xs[2:], **kw)) < TOL[dtype]
+    assert not stored(dx)[..., xs[1]:].any()
+    y = shim.device_conv2d(X, W, out_layout="nchw", flags=flags, **kw)
+    assert O.rel_err(y.to_host().astype(f), conv) < TOL[dtype]
+
+
+@DTYPES
+@pytest.mark.parametrize("flags", [0, shim.NO_SLAB], ids=["slab", "tap"])
+@pytest.mark.parametrize("xs,k,ks", [((1, 512, 8, 8), 75, 3),       # split reduction
+                                     ((40, 16, 28, 28), 62, 3),     # whole 128-byte channel chunks in float32
+                                     ((40, 16, 28, 28), 21, 3),     # direct stores
+                                     ((16, 256, 40, 40), 255, 1)],  # pairs of CTAs in float16
+                         ids=["split", "staged", "direct", "pair"])
+def test_infinities_leave_pad_channels_zero(ctx, dtype, flags, xs, k, ks):
+    """Pad channels are the product of zero filters and the input; an infinity there would make them NaN."""
+    rs = np.random.RandomState(5)
+    x = rs.standard_normal(xs).astype(dtype)
+    x[0, 1, 3, 2] = np.inf
+    w = (rs.standard_normal((k, xs[1], ks, ks)) / np.sqrt(xs[1] * ks * ks)).astype(dtype)
+    y = shim.device_conv2d(T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), border_mode="half", flags=flags)
+    a = stored(y)
+    assert a.shape[-1] > k and not a[..., k:].any()
+    assert np.isinf(a[0, 3, 2, :k]).all() and np.isfinite(a[1:]).all()
+    # gradInputs of the mirrored layer: its input has the k (padded) channels
+    dx = shim.device_grad_inputs(T.from_host(ctx, np.ascontiguousarray(w.transpose(1, 0, 2, 3))), T.from_host(ctx, x, "nhwc"),
+                                 xs[2:], border_mode="half", flags=flags)
+    a = stored(dx)
+    assert not a[..., k:].any() and np.isinf(a[0, 3, 2, :k]).all() and np.isfinite(a[1:]).all()
+
+
+def shifted(t, fill=None):
+    """The same tensor in memory one element off the 16-byte boundaries (and the memory's owner)."""
+    es = t.dtype.itemsize
+    owner = T(t.ctx, (1, 1, 1, t.nbytes // es + 16), t.dtype)
+    view = T(t.ctx, t.shape, t.dtype, t.layout, _ptr=owner.ptr + es)
+    a = stored(t) if fill is None else np.full((t.nbytes // es,), fill, t.dtype)
+    t.ctx.h2d(view.ptr, a)
+    t.ctx.sync()
+    return view, owner
+
+
+@DTYPES
+@pytest.mark.parametrize("shape", [(2, 33, 9, 6), (1, 8, 5, 5)], ids=["33ch", "8ch"])
+def test_pooling_and_channel_sum_off_the_boundary(ctx, dtype, shape):
+    rs = np.random.RandomState(3)
+    n, c, h, w = shape
+    x = rs.standard_normal(shape).astype(dtype)
+    X = T.from_host(ctx, x, "nhwc")
+    Y = shim.device_maxpool2x2(X)
+    G = T.from_host(ctx, rs.standard_normal(Y.shape).astype(dtype), "nhwc")
+    GX = shim.device_maxpool2x2_grad(X, Y, G)
+    (Xs, o1), (Ys, o2), (Gs, o3), (GXs, o4) = shifted(X), shifted(Y, 7), shifted(G), shifted(GX, 7)
+    assert np.array_equal(stored(shim.device_maxpool2x2(Xs, out=Ys)), stored(Y))
+    assert np.array_equal(stored(shim.device_maxpool2x2_grad(Xs, Ys, Gs, out=GXs)), stored(GX))
+    # float32 sums of at most 108 values of order 1 in another order; float16 results round to 2^-11 on top
+    want = x.astype(np.float64).sum((0, 2, 3))
+    tol = 1e-4 if dtype == np.float32 else 2e-2
+    assert np.abs(shim.device_channel_sum(Xs) - want).max() < tol and np.abs(shim.device_channel_sum(X) - want).max() < tol
+
+
+@DTYPES
+@pytest.mark.parametrize("flags", [0, shim.NO_SLAB], ids=["slab", "tap"])
+@pytest.mark.parametrize("xs,k", [((1, 512, 8, 8), 75), ((40, 16, 28, 28), 21), ((40, 16, 28, 28), 64)], ids=["split", "direct", "whole"])
+def test_outputs_off_the_boundary(ctx, dtype, flags, xs, k):
+    rs = np.random.RandomState(4)
+    X = T.from_host(ctx, rs.standard_normal(xs).astype(dtype), "nhwc")
+    W = T.from_host(ctx, (rs.standard_normal((k, xs[1], 3, 3)) / np.sqrt(xs[1] * 9)).astype(dtype))
+    y = shim.device_conv2d(X, W, border_mode="half", flags=flags)
+    ys, owner = shifted(y, 7)
+    shim.device_conv2d(X, W, border_mode="half", out=ys, flags=flags)
+    a, b = stored(y).astype(np.float32), stored(ys).astype(np.float32)
+    assert O.rel_err(b, a) < TOL[dtype] / 4          # another tile may split the sums elsewhere
+
+
+@DTYPES
+def test_pooling_epilogue_still_asks_for_whole_channel_chunks(ctx, dtype):
+    """A split reduction could pool any channel count, but what the epilogue refuses does not depend on the batch."""
+    X = T.from_host(ctx, np.ones((1, 512, 8, 8), dtype), "nhwc")
+    W = T.from_host(ctx, np.ones((75, 512, 3, 3), dtype))
+    with pytest.raises(shim.B200Error, match="cannot pool"):
+        shim.device_conv2d(X, W, border_mode="half", pool=True)
+
+
+@DTYPES
+@pytest.mark.parametrize("c,k,g", [(256, 256, 32), (96, 48, 12), (64, 128, 8), (48, 48, 3), (512, 256, 2)], ids=lambda v: str(v))
+def test_grad_weights_of_merged_groups(ctx, dtype, c, k, g):
+    rs = np.random.RandomState(g)
+    x, dy = (rs.standard_normal((3, n, 11, 9)).astype(dtype) for n in (c, k))
+    kw = dict(border_mode="half", num_groups=g)
+    dw = shim.device_grad_weights(T.from_host(ctx, x, "nhwc"), T.from_host(ctx, dy, "nhwc"), (3, 3), **kw).to_host()
+    f = np.float32
+    assert O.rel_err(dw.astype(f), O.conv2d_grad_weights(x.astype(f), dy.astype(f), (3, 3), **kw)) < TOL[dtype]

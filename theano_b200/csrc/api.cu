@@ -703,7 +703,7 @@ int split_output(b200conv_ctx* c, Scratch& tmp, const P& p, int bn, int rows, Co
   q->partial = partial;
   q->splits = p.splits; q->rows = rows; q->bn_cols = bn;
   q->tiles_w = p.tiles_w; q->tiles_h = p.tiles_h; q->tiles_n = p.tiles_n; q->tiles_co = p.tiles_co; q->groups = p.groups;
-  q->Wt = p.Wt; q->Ht = p.Ht; q->Nimg = p.Nimg; q->n_out = p.n_out;
+  q->Wt = p.Wt; q->Ht = p.Ht; q->Nimg = p.Nimg; q->n_out = p.n_out; q->n_real = p.n_real;
   q->out = p.out; q->bias = p.bias;
   q->out_sn = p.out_sn; q->out_sc = p.out_sc; q->out_sh = p.out_sh; q->out_sw = p.out_sw; q->out_off = p.out_off;
   q->relu = p.relu;
@@ -762,7 +762,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       q.kblocks = (int)kblocks_n;
       q.tiles_pix = (int)cdiv(Wt, 256);
       q.tiles_co = (int)cdiv(a.n_out, 256);
-      q.pixels = Wt; q.n_out = a.n_out;
+      q.pixels = Wt; q.n_out = a.n_out; q.n_real = a.w_rows;
       q.stages = 5;
       q.bias = bias; q.relu = relu; q.epi = c->epi;
       q.status = c->d_status;
@@ -876,6 +876,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.tiles_w = (int)cdiv(Wt, p.wt); p.tiles_h = (int)cdiv(Ht, p.th); p.tiles_n = (int)cdiv(a.N, p.nb);
   p.tiles_co = tiles_co;
   p.n_out = a.n_out;
+  p.n_real = a.w_rows;
   p.out = out; p.bias = bias;
   p.out_sn = sn; p.out_sc = sc; p.out_sh = sh; p.out_sw = sw; p.out_off = off;
   p.out_elems = out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
@@ -953,6 +954,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.tiles_n = static_cast<int>(cdiv(a.N, p.bn));
   p.tiles_co = static_cast<int>(cdiv(a.n_out, BN));
   p.n_out = a.n_out;
+  p.n_real = a.w_rows;
   p.out = out; p.bias = bias;
   p.out_sn = sn; p.out_sc = sc; p.out_sh = sh; p.out_sw = sw; p.out_off = off;
   p.out_elems = out_extent(a, Wt, Ht, sn, sc, sh, sw, off);

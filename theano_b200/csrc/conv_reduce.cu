@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const __grid_constant_
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       if (c0 + e >= p.n_out) continue;
-      float f = p.epi.alpha * v[e];
+      float f = p.epi.alpha * (c0 + e < p.n_real ? v[e] : 0.f);       // pad channels: 0 x infinity is NaN
       if (p.bias) f += to_f(static_cast<const T*>(p.bias)[g * p.n_out + c0 + e]);
       if (p.epi.residual) f += p.epi.beta * to_f(static_cast<const T*>(p.epi.residual)[(out - static_cast<T*>(p.out)) + e * p.out_sc]);
       if (p.relu) f = p.epi.lin * f + p.epi.abs * fabsf(f);
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const __grid_constant_
       best[e] = k == 0 ? f : fmaxf(best[e], f);
     }
   }
-  if (p.out_sc == 1 && ((p.n_out * sizeof(T)) & 15) == 0) { // four columns are all in
+  if (p.out_sc == 1 && ((p.n_out * sizeof(T) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0) { // four columns are all in
     if (sizeof(T) == 4) {
       *reinterpret_cast<float4*>(out) = make_float4(best[0], best[1], best[2], best[3]);
     } else {

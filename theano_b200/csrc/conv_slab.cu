@@ -259,7 +259,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     OutT* out = static_cast<OutT*>(p.out);
     const int per_img = p.Hs * p.Ws;
     // channels-last output whose 32-channel groups are 16-byte aligned: 16-byte stores
-    const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT)) & 15) == 0;
+    const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
     bool ok = true;
     int it = 0;
     long long te_wait = 0, te_busy = 0;          // clocks of thread 64 (only with trace)
@@ -343,6 +343,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             tmem_ld_wait();
             if (trace) { const long long t = clock64(); tp[1] += t - tq; tq = t; }
             if (!inbox) continue;
+            zero_pad_columns(r, co0 + part * 32, p.n_real);
             const OutT* bp = bias ? bias + part * 32 : nullptr;
             if (plain) {
               // no scale, bias or activation (gradInputs, bare forward): convert and stage only.
@@ -473,6 +474,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           tmem_ld_wait();
           if (!valid) continue;
           const int co0 = co_base + ch * 32;
+          zero_pad_columns(r, co0, p.n_real);
           const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
           if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
 #pragma unroll

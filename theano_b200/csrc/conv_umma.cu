@@ -194,7 +194,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const int row = quad * 32 + lane;
     const int rw = row % p.bw, rh = (row / p.bw) % p.bh, rn = row / (p.bw * p.bh);
     OutT* out = static_cast<OutT*>(p.out);
-    const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT)) & 15) == 0;
+    const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
     bool ok = true;
     int it = 0;
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
@@ -235,6 +235,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
         tmem_ld_wait();
         if (!valid) continue;
+        zero_pad_columns(r, co0, p.n_real);
         const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
         if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
 #pragma unroll

@@ -98,12 +98,11 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const T* __restrict__ 
 // Per-channel sum, stage 1: a block's 256 threads are `lanes` rows of threads over the pixels x `vecs`
 // 16-byte pieces of the channel vector (256 / lanes of them at a time); block b takes the pixels
 // (b * lanes + lane) + k * gridDim.x * lanes in that order, eight loads in flight, then adds its rows in
-// lane order into partial[b][Cp].
-template <typename T>
+// lane order into partial[b][Cp].  V is a piece's element count: 1 for a tensor off the 16-byte boundaries.
+template <typename T, int V>
 __global__ void __launch_bounds__(256) channel_sum_partial_kernel(const T* __restrict__ x, float* __restrict__ partial,
                                                                   long long pixels, int Cp, int log_lanes) {
   pdl_enter();
-  constexpr int V = Vec<T>::n;
   __shared__ float part[256][V + 1];
   const int cols = 256 >> log_lanes, lane = threadIdx.x >> (8 - log_lanes), col = threadIdx.x & (cols - 1);
   const int vecs = Cp / V;
@@ -118,7 +117,8 @@ __global__ void __launch_bounds__(256) channel_sum_partial_kernel(const T* __res
 #pragma unroll 8
       for (long long p = first; p < pixels; p += step) {
         float f[V];
-        load16<T>(src + p * Cp, f);
+        if constexpr (V == 1) f[0] = static_cast<float>(src[p * Cp]);
+        else load16<T>(src + p * Cp, f);
 #pragma unroll
         for (int q = 0; q < V; ++q) acc[q] += f[q];
       }
@@ -190,13 +190,20 @@ int channel_sum_blocks(long long pixels) {
 cudaError_t launch_channel_sum(const void* x, float* partial, void* out, long long pixels, int C, int Cp, int dtype,
                                cudaStream_t st) {
   const int blocks = channel_sum_blocks(pixels);
-  const int vecs = Cp / (dtype == B200CONV_F16 ? 8 : 4);
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int vecs = wide ? Cp / (dtype == B200CONV_F16 ? 8 : 4) : Cp;
   int log_lanes = 0;                             // as many rows of threads over the pixels as the channel vector leaves
   while (log_lanes < 8 && (vecs << (log_lanes + 1)) <= 256) ++log_lanes;
-  if (dtype == B200CONV_F16)
-    launch_streaming(channel_sum_partial_kernel<__half>, blocks, 256, 0, st, static_cast<const __half*>(x), partial, pixels, Cp, log_lanes);
-  else
-    launch_streaming(channel_sum_partial_kernel<float>, blocks, 256, 0, st, static_cast<const float*>(x), partial, pixels, Cp, log_lanes);
+#define B200_SUM(T, V) \
+  launch_streaming(channel_sum_partial_kernel<T, V>, blocks, 256, 0, st, static_cast<const T*>(x), partial, pixels, Cp, log_lanes)
+  if (dtype == B200CONV_F16) {
+    if (wide) B200_SUM(__half, 8);
+    else B200_SUM(__half, 1);
+  } else {
+    if (wide) B200_SUM(float, 4);
+    else B200_SUM(float, 1);
+  }
+#undef B200_SUM
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (dtype == B200CONV_F16)

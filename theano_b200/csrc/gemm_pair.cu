@@ -165,6 +165,7 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
           uint32_t r[32];
           tmem_ld32(lane_base + grp * 64 + part * 32, r);
           tmem_ld_wait();
+          zero_pad_columns(r, co0 + part * 32, p.n_real);
           const __half* bp = bias ? bias + part * 32 : nullptr;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {

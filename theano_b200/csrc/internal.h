@@ -114,7 +114,8 @@ struct alignas(64) UmmaConvParams {
   int Wt, Ht, Nimg;              // extent of the output pixel grid this launch covers
   int bw, bh, bn;                // pixel tile (bw*bh*bn <= 128 rows of the accumulator)
   int tiles_w, tiles_h, tiles_n, tiles_co;
-  int n_out;                     // output channels per group
+  int n_out;                     // output channels per group as stored
+  int n_real;                    // of these, the ones with filters: the pad channels behind them are stored as 0
   void* out;
   const void* bias;              // per output channel (groups*n_out), in the data type, or null
   long long out_sn, out_sc, out_sh, out_sw, out_off;  // element strides / offset of `out`
@@ -153,7 +154,7 @@ struct alignas(64) SlabConvParams {
   int tap_boxes;                 // 1: one TMA box per tap; 0: the taps of a stage are neighbours in the packed filters
                                  // and arrive as one box (the map's box then is tps matrices deep)
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
-  int n_out;
+  int n_out, n_real;             // output channels per group as stored / with filters
   void* out;
   const void* bias;
   long long out_sn, out_sc, out_sh, out_sw, out_off;
@@ -187,7 +188,7 @@ struct ConvReduceParams {
   int splits, rows, bn_cols;
   int Ws, Hs, wt, th, nb;
   int tiles_w, tiles_h, tiles_n, tiles_co, groups;
-  int Wt, Ht, Nimg, n_out;
+  int Wt, Ht, Nimg, n_out, n_real;
   void* out;                     // strides of the pooled tensor when epi.pool
   const void* bias;
   long long out_sn, out_sc, out_sh, out_sw, out_off;
@@ -203,7 +204,7 @@ struct alignas(64) PairGemmParams {
   CUtensorMap out_map;           // 4-D (channel, pixel, 1, 1) over the output, box (64, 128, 1, 1)
   int kblocks;                   // ceil(channels / 64)
   int tiles_pix, tiles_co;       // 256-pixel tiles, 256-filter tiles
-  int pixels, n_out;
+  int pixels, n_out, n_real;
   int stages;                    // ring depth (2 .. 5)
   const void* bias;
   int relu;

@@ -381,8 +381,20 @@ __global__ void maxpool2x2_grad_nchw_kernel(const T* __restrict__ x, const T* __
 // Channels-last forms: one thread per window and 16-byte piece of the channel vector, so that every access
 // is 16 bytes wide, the four pixels' loads are in flight together and the index arithmetic is paid once per
 // 16 to 32 elements (HBM bound: 64 x 128 x 112 x 112 float32 gradient 846 -> 176 us at 1.03 GB).
+// A tensor that does not start on a 16-byte boundary is taken element by element (One).
+template <typename T> struct One {
+  static constexpr int n = 1;
+  using type = T;
+  T v;
+  __device__ __forceinline__ void max(const One& o) { v = static_cast<T>(fmaxf(static_cast<float>(v), static_cast<float>(o.v))); }
+  __device__ __forceinline__ static One route(const One& x, const One& y, const One& g) {
+    return {static_cast<float>(x.v) == static_cast<float>(y.v) ? g.v : static_cast<T>(0.f)};
+  }
+};
 template <typename T> struct Piece;               // 16 bytes of T
 template <> struct Piece<float> {
+  static constexpr int n = 4;
+  using type = float;
   float4 v;
   __device__ __forceinline__ void max(const Piece& o) {
     v.x = fmaxf(v.x, o.v.x); v.y = fmaxf(v.y, o.v.y); v.z = fmaxf(v.z, o.v.z); v.w = fmaxf(v.w, o.v.w);
@@ -393,6 +405,8 @@ template <> struct Piece<float> {
   }
 };
 template <> struct Piece<__half> {
+  static constexpr int n = 8;
+  using type = __half;
   __align__(16) __half2 v[4];
   __device__ __forceinline__ void max(const Piece& o) {
 #pragma unroll
@@ -409,13 +423,13 @@ template <> struct Piece<__half> {
     return r;
   }
 };
-template <typename T> __device__ __forceinline__ Piece<T> load_piece(const T* p) { return *reinterpret_cast<const Piece<T>*>(p); }
+template <typename P, typename T> __device__ __forceinline__ P load_piece(const T* p) { return *reinterpret_cast<const P*>(p); }
 
-template <typename T, typename Index>
+template <typename P, typename Index, typename T = typename P::type>
 __global__ void __launch_bounds__(256) maxpool2x2_nhwc_kernel(const T* __restrict__ x, T* __restrict__ y, Index total,
                                                               int H, int W, int pieces) {
   pdl_enter();
-  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  constexpr int V = P::n;
   const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
   if (idx >= total) return;
   const Index Ho = H / 2, Wo = W / 2, Cv = pieces;
@@ -424,20 +438,20 @@ __global__ void __launch_bounds__(256) maxpool2x2_nhwc_kernel(const T* __restric
   const int c = static_cast<int>(idx - pix * Cv) * V, ow = static_cast<int>(pix - row * Wo), oh = static_cast<int>(row % Ho);
   const long long n = row / Ho;
   const T* p = x + ((n * H + 2 * oh) * W + 2 * ow) * Cp + c;
-  Piece<T> m = load_piece(p);
-  const Piece<T> a = load_piece(p + Cp), b = load_piece(p + W * Cp), d = load_piece(p + W * Cp + Cp);
+  P m = load_piece<P>(p);
+  const P a = load_piece<P>(p + Cp), b = load_piece<P>(p + W * Cp), d = load_piece<P>(p + W * Cp + Cp);
   m.max(a); m.max(b); m.max(d);
-  *reinterpret_cast<Piece<T>*>(y + static_cast<long long>(idx) * V) = m;
+  *reinterpret_cast<P*>(y + static_cast<long long>(idx) * V) = m;
 }
 
 // The grid covers (H + 1) / 2 x (W + 1) / 2 windows: in an odd-sized image the last row / column belongs to no
 // window and gets zeros.
-template <typename T, typename Index>
+template <typename P, typename Index, typename T = typename P::type>
 __global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __restrict__ x, const T* __restrict__ y,
                                                                    const T* __restrict__ gy, T* __restrict__ gx,
                                                                    Index total, int H, int W, int pieces) {
   pdl_enter();
-  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  constexpr int V = P::n;
   const Index idx = blockIdx.x * static_cast<Index>(256) + threadIdx.x;
   if (idx >= total) return;
   const int Ho = H / 2, Wo = W / 2;
@@ -447,21 +461,21 @@ __global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __re
   const int c = static_cast<int>(idx - pix * Cv) * V, ow = static_cast<int>(pix - row * Wc), oh = static_cast<int>(row % Hc);
   const long long n = row / Hc;
   const long long base = ((n * H + 2 * oh) * W + 2 * ow) * Cp + c;
-  Piece<T> r[4];
+  P r[4];
   memset(r, 0, sizeof r);
   if (oh < Ho && ow < Wo) {
     const long long o = ((n * Ho + oh) * Wo + ow) * Cp + c;
-    const Piece<T> m = load_piece(y + o), g = load_piece(gy + o);
-    Piece<T> v[4];
+    const P m = load_piece<P>(y + o), g = load_piece<P>(gy + o);
+    P v[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = load_piece(x + base + (k & 1) * Cp + (k >> 1) * W * Cp);
+    for (int k = 0; k < 4; ++k) v[k] = load_piece<P>(x + base + (k & 1) * Cp + (k >> 1) * W * Cp);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) r[k] = Piece<T>::route(v[k], m, g);
+    for (int k = 0; k < 4; ++k) r[k] = P::route(v[k], m, g);
   }
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (2 * oh + (k >> 1) < H && 2 * ow + (k & 1) < W)
-      *reinterpret_cast<Piece<T>*>(gx + base + (k & 1) * Cp + (k >> 1) * W * Cp) = r[k];
+      *reinterpret_cast<P*>(gx + base + (k & 1) * Cp + (k >> 1) * W * Cp) = r[k];
 }
 
 template <typename T>
@@ -724,12 +738,37 @@ cudaError_t launch_convert_bias(const void* bias, float* dst, int n, int dtype, 
 namespace {
 // Launches a channels-last pooling kernel with 32-bit indices where they suffice (64-bit divisions cost more
 // than the memory accesses).
-template <typename T, class Launch>
+template <class Launch>
 cudaError_t for_index(long long total, Launch launch) {
   const long long grid = (total + 255) / 256;
   if (grid >= (1LL << 31)) return cudaErrorInvalidValue;
   launch(static_cast<int>(grid), total < (1LL << 31));
   return cudaGetLastError();
+}
+bool aligned16(std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
+}
+template <typename P, typename T = typename P::type>
+cudaError_t maxpool_nhwc(const T* x, T* y, int N, int H, int W, int Cp, cudaStream_t s) {
+  const int pieces = Cp / P::n;
+  const long long total = 1LL * N * (H / 2) * (W / 2) * pieces;
+  return for_index(total, [&](int grid, bool small) {
+    if (small) launch_streaming(maxpool2x2_nhwc_kernel<P, unsigned>, grid, 256, 0, s, x, y, static_cast<unsigned>(total), H, W, pieces);
+    else launch_streaming(maxpool2x2_nhwc_kernel<P, long long>, grid, 256, 0, s, x, y, total, H, W, pieces);
+  });
+}
+template <typename P, typename T = typename P::type>
+cudaError_t maxpool_grad_nhwc(const T* x, const T* y, const T* gy, T* gx, int N, int H, int W, int Cp, cudaStream_t s) {
+  const int pieces = Cp / P::n;
+  const long long total = 1LL * N * ((H + 1) / 2) * ((W + 1) / 2) * pieces;
+  return for_index(total, [&](int grid, bool small) {
+    if (small)
+      launch_streaming(maxpool2x2_grad_nhwc_kernel<P, unsigned>, grid, 256, 0, s, x, y, gy, gx, static_cast<unsigned>(total), H, W, pieces);
+    else
+      launch_streaming(maxpool2x2_grad_nhwc_kernel<P, long long>, grid, 256, 0, s, x, y, gy, gx, total, H, W, pieces);
+  });
 }
 template <typename T>
 cudaError_t maxpool_typed(const T* x, T* y, int N, int C, int H, int W, int nhwc, int Cp, cudaStream_t s) {
@@ -737,12 +776,7 @@ cudaError_t maxpool_typed(const T* x, T* y, int N, int C, int H, int W, int nhwc
     launch_streaming(maxpool2x2_nchw_kernel<T>, grid_for(1LL * N * C * (H / 2) * (W / 2), 256), 256, 0, s, x, y, 1LL * N * C, H, W);
     return cudaGetLastError();
   }
-  const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
-  const long long total = 1LL * N * (H / 2) * (W / 2) * pieces;
-  return for_index<T>(total, [&](int grid, bool small) {
-    if (small) launch_streaming(maxpool2x2_nhwc_kernel<T, unsigned>, grid, 256, 0, s, x, y, static_cast<unsigned>(total), H, W, pieces);
-    else launch_streaming(maxpool2x2_nhwc_kernel<T, long long>, grid, 256, 0, s, x, y, total, H, W, pieces);
-  });
+  return aligned16({x, y}) ? maxpool_nhwc<Piece<T>>(x, y, N, H, W, Cp, s) : maxpool_nhwc<One<T>>(x, y, N, H, W, Cp, s);
 }
 template <typename T>
 cudaError_t maxpool_grad_typed(const T* x, const T* y, const T* gy, T* gx, int N, int C, int H, int W, int nhwc, int Cp,
@@ -751,14 +785,8 @@ cudaError_t maxpool_grad_typed(const T* x, const T* y, const T* gy, T* gx, int N
     launch_streaming(maxpool2x2_grad_nchw_kernel<T>, grid_for(1LL * N * C * H * W, 256), 256, 0, s, x, y, gy, gx, 1LL * N * C, H, W);
     return cudaGetLastError();
   }
-  const int pieces = Cp * static_cast<int>(sizeof(T)) / 16;
-  const long long total = 1LL * N * ((H + 1) / 2) * ((W + 1) / 2) * pieces;
-  return for_index<T>(total, [&](int grid, bool small) {
-    if (small)
-      launch_streaming(maxpool2x2_grad_nhwc_kernel<T, unsigned>, grid, 256, 0, s, x, y, gy, gx, static_cast<unsigned>(total), H, W, pieces);
-    else
-      launch_streaming(maxpool2x2_grad_nhwc_kernel<T, long long>, grid, 256, 0, s, x, y, gy, gx, total, H, W, pieces);
-  });
+  return aligned16({x, y, gy, gx}) ? maxpool_grad_nhwc<Piece<T>>(x, y, gy, gx, N, H, W, Cp, s)
+                                   : maxpool_grad_nhwc<One<T>>(x, y, gy, gx, N, H, W, Cp, s);
 }
 }  // namespace
 

@@ -396,6 +396,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// Columns first .. first + 31 of an accumulator row: those from n_real on belong to pad channels and become 0.
+// Their filters are zero, but a product of zero and an infinity in the input is NaN.
+__device__ __forceinline__ void zero_pad_columns(uint32_t (&r)[32], int first, int n_real) {
+  if (first + 32 <= n_real) return;
+#pragma unroll
+  for (int j = 0; j < 32; ++j)
+    if (first + j >= n_real) r[j] = 0;
+}
 
 // ---- descriptors --------------------------------------------------------------------
 // Shared-memory matrix descriptor (64 bit): start address >> 4 in bits [0,14), leading
