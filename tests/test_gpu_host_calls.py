@@ -33,6 +33,24 @@ def test_chunked_batches_against_oracle(n, pageable_out):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("extra", [1, 30], ids=["filters", "residual"])
+def test_small_inputs_wait_for_large_ones_in_their_own_slot(extra):
+    """Small inputs share a slot of the staging ring; an image of more than the whole ring must not take it."""
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(1)
+    n, c, h, w = 1, 8 if extra == 1 else 1, 1200, 1300                      # 50 MB in, or 6 MB in and a residual
+    k = 1 if extra == 1 else 8
+    # small whole numbers: products and sums are exact in TF32
+    x = rs.randint(-8, 9, (n, c, h, w)).astype(np.float32)
+    f = rs.randint(-8, 9, (k, c, 1, 1)).astype(np.float32)
+    b = rs.randint(-8, 9, k).astype(np.float32)
+    r = None if extra == 1 else rs.randint(-8, 9, (n, k, h, w)).astype(np.float32)
+    y = shim.conv2d_forward(x, f, bias=b, residual=r, ctx=ctx)
+    want = np.einsum("kc,nchw->nkhw", f[:, :, 0, 0], x) + b[None, :, None, None] + (0 if r is None else r)
+    assert np.array_equal(y, want)
+
+
+@pytest.mark.gpu
 def test_results_keep_their_values_while_others_are_made():
     ctx = shim.get_context(0)
     rs = np.random.RandomState(0)
@@ -82,3 +100,11 @@ def test_result_pool_reuses_and_gives_back(monkeypatch):
     del many, b
     gc.collect()
     assert pool.kept <= pool.KEEP and pool.total == pool.kept and len(Ctx.lib.buffers) <= 2
+    pool.trim()                                                         # nothing is out: all of it goes back
+    assert pool.total == pool.kept == 0 and not Ctx.lib.buffers
+
+
+def test_operands_in_the_other_byte_order_are_converted():
+    a, b = np.arange(6, dtype=">f4"), np.arange(4, dtype=">f4")
+    for v, w in zip(shim._common(a, b), (a, b)):
+        assert v.dtype.isnative and v.dtype == np.float32 and np.array_equal(v, w)

@@ -1053,6 +1053,7 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                      (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
     const SlabTile w = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, false);
     const SlabTile n = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, true);
+    if (c->epi.pool && !(tma && w.found)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
     if (w.found) cand[ncand++] = kConvSlab;
     if (n.found && (!w.found || n.splits > 1 || n.bn != w.bn || n.wt != w.wt || n.th != w.th || n.nb != w.nb)) cand[ncand++] = kConvSlabSpread;
   }
@@ -2194,13 +2195,19 @@ struct HostIO {
       memcpy(group_host + (static_cast<char*>(*d) - group_dev), h, bytes);
       return 0;
     }
-    if ((rc = tmp.get(bytes, d))) return rc;
+    // the ring turns under a large input, so the slot of a waiting group has to be on its way first
+    if ((rc = start()) || (rc = tmp.get(bytes, d))) return rc;
     return upload(c, *d, h, bytes, c->stream, is_pinned(h, bytes));
   }
   int start() {
-    if (!group_used) return 0;
-    CU_OK(c, cudaMemcpyAsync(group_dev, group_host, group_used, cudaMemcpyHostToDevice, c->stream));
-    return ring_used(c, group_slot, c->stream);
+    if (!group_dev) return 0;
+    if (group_used) {
+      CU_OK(c, cudaMemcpyAsync(group_dev, group_host, group_used, cudaMemcpyHostToDevice, c->stream));
+      if (int rc = ring_used(c, group_slot, c->stream)) return rc;
+    }
+    group_dev = group_host = nullptr;
+    group_used = 0;
+    return 0;
   }
   int back(void* h, const void* d, size_t bytes) {
     return bytes ? download(c, h, d, bytes, c->stream, is_pinned(h, bytes)) : 0;
@@ -2439,7 +2446,7 @@ static int fwd_call(b200conv_ctx* c, const b200conv_desc* d, const void* x, cons
     b200conv_desc part = *d;
     part.N = images;
     epi.residual = res;
-    if (res) res += ny / d->N * images;
+    if (res && images) res += ny / d->N * images;
     EpilogueScope scope(c, epi);
     return fwd_device(c, part, xin, dw_, db_, yout, flags & ~B200CONV_HOST_PTRS);
   });
@@ -2908,13 +2915,14 @@ int b200conv_set_splits(b200conv_ctx* c, int splits) {
 
 // The tuning file: a header line naming the device the choices were timed on, then one line per
 // choice.  Choices made on another device model or SM count are not loaded.
-static std::string tuning_header(b200conv_ctx* c) {
+// Version 2: keys are lists of integers.  Files of version 1 (other keys) are read without effect.
+static std::string tuning_header(b200conv_ctx* c, int version) {
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, c->device);
   std::string name = prop.name;
   for (char& ch : name)
     if (ch == ' ') ch = '_';
-  return "b200conv-tuning 1 " + name + " " + std::to_string(c->num_sms);
+  return "b200conv-tuning " + std::to_string(version) + " " + name + " " + std::to_string(c->num_sms);
 }
 
 int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
@@ -2923,7 +2931,7 @@ int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
   DeviceGuard dg(c->device);
   FILE* f = fopen(path, "w");
   if (!f) return fail(c, B200CONV_E_INVALID, "cannot write %s", path);
-  fprintf(f, "%s\n", tuning_header(c).c_str());
+  fprintf(f, "%s\n", tuning_header(c, 2).c_str());
   for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.text().c_str(), kv.second);
   for (auto& kv : c->split_cache) fprintf(f, "s %s %d\n", kv.first.text().c_str(), kv.second);
   fclose(f);
@@ -2943,7 +2951,11 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
   if (ok) {
     std::string head = line;
     while (!head.empty() && (head.back() == '\n' || head.back() == '\r')) head.pop_back();
-    ok = head == tuning_header(c);
+    ok = head == tuning_header(c, 2);
+    if (!ok && head == tuning_header(c, 1)) {
+      fclose(f);
+      return 0;
+    }
   }
   if (!ok) {
     fclose(f);

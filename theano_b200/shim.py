@@ -160,6 +160,7 @@ class Context(object):
         if getattr(self, "h", None):
             self.lib.b200conv_destroy(self.h)
             self.h = None
+            _results.trim()
 
     def __del__(self):
         try:
@@ -513,11 +514,21 @@ class _ResultPool(object):
             keep = self.kept + size <= self.KEEP
             if keep:
                 self.kept += size
-                self.free[size].append(ptr)
+                self.free.setdefault(size, []).append(ptr)
             else:
                 self.total -= size
         if not keep:
             load_library().b200conv_host_free(None, _P(ptr))
+
+    def trim(self):
+        """Gives the kept memory back (a context that closes does this)."""
+        with self.lock:
+            blocks, self.free = self.free, {}
+            self.total -= self.kept
+            self.kept = 0
+        for size in blocks:
+            for ptr in blocks[size]:
+                load_library().b200conv_host_free(None, _P(ptr))
 
 
 _results = _ResultPool()
@@ -611,8 +622,8 @@ def _address(a):
 
 def _common(a, b):
     """Upcast like BaseCorrMM.as_common_dtype (corr.py:156-162); float64 is not handled here."""
-    if a.dtype is b.dtype and a.flags.c_contiguous and b.flags.c_contiguous:
-        _dtype_code(a.dtype)
+    if (a.dtype is b.dtype and (a.dtype is _F32T or a.dtype is _F16T)      # in native byte order
+            and a.flags.c_contiguous and b.flags.c_contiguous):
         return a, b
     dt = np.promote_types(a.dtype, b.dtype)
     _dtype_code(dt)
