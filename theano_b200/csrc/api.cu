@@ -452,16 +452,18 @@ int make_view(b200conv_ctx* c, CUtensorMap* m, const void* base, int dtype, int 
   return 0;
 }
 
-// 3-D map over packed filters [mats][rows][ldc]: (cols, rows, mats), box (box_c, box_r, box_m).
+// Map over packed filters [mats][rows][ldc]: (cols, rows, mats), box (box_c, box_r, 1); with `groups`, mats = taps x
+// groups as four dimensions (cols, rows, groups, taps), box (box_c, box_r, 1, box_t), so that a box holds box_t taps of a group.
 int make_wmap(b200conv_ctx* c, CUtensorMap* m, const void* base, int dtype, int cols, int rows,
-              int mats, int ldc, int box_c, int box_r, int box_m = 1) {
+              int mats, int ldc, int box_c, int box_r, int groups = 0, int box_t = 1) {
   const size_t es = elem_size(dtype);
-  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)mats};
-  cuuint64_t strides[2] = {(cuuint64_t)ldc * es, (cuuint64_t)rows * ldc * es};
-  cuuint32_t box[3] = {(cuuint32_t)box_c, (cuuint32_t)box_r, (cuuint32_t)box_m};
-  cuuint32_t estr[3] = {1, 1, 1};
+  const int g = std::max(1, groups);
+  cuuint64_t dims[4] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)(groups ? g : mats), (cuuint64_t)(mats / g)};
+  cuuint64_t strides[3] = {(cuuint64_t)ldc * es, (cuuint64_t)rows * ldc * es, (cuuint64_t)g * rows * ldc * es};
+  cuuint32_t box[4] = {(cuuint32_t)box_c, (cuuint32_t)box_r, 1, (cuuint32_t)box_t};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = c->encode(m, dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                         3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         groups ? 4 : 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(filters) failed: %d", (int)r);
@@ -542,8 +544,12 @@ long long out_extent(const FwdLikeArgs& a, int Wt, int Ht, long long sn, long lo
 
 // Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
 // the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
-// and / or a reduction cut into slices where that occupies more SMs.  The numbers appear in tuning files.
-enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvVariants = 4 };
+// and / or a reduction cut into slices where that occupies more SMs; the slab kernel also on pairs of CTAs.  The
+// numbers appear in tuning files.
+enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvVariants = 5 };
+enum SlabMode { kSlabWide = 0, kSlabSpread, kSlabPair };      // of the slab kernel's tile search
+
+SlabMode slab_mode(int variant) { return variant == kConvSlabSpread ? kSlabSpread : variant == kConvSlabPair ? kSlabPair : kSlabWide; }
 
 // Clocks of four MMAs over 128 rows x bn columns x 32 bytes of the reduction, one after the other: half the
 // columns up to 128 (N = 64 and 32 are bound by their operands' shared-memory reads).
@@ -556,18 +562,27 @@ long long split_clocks(long long items, int rows, int bn, int sms) {
   return 1LL * rows * bn * 4 / 32 + 4500 + items * rows * bn * 4 / (48LL * sms);
 }
 
-// Filter taps per stage of the slab kernel's filter ring.  Narrow tiles (few filters) have small filter tiles and
-// short MMAs: several taps then share one stage, so that a barrier round trip is paid per 16 to 32 KB of
-// filters, not per 4 or 8 KB (the issuing warp spends about 150 clocks per stage on the hand-over, as much as
-// the stage's MMAs take when a tap is four 128 x 64 MMAs).  Measured: 64 -> 64 3x3 layers 8 to 16 % faster with a
-// filter row per stage, the 7x7 stem 8 to 16 % with four taps; 128-filter tiles are better off with one tap per stage.
-int slab_tps(int bn, int ntaps) { return bn > 64 ? 1 : ntaps % 3 == 0 ? 3 : std::min(4, ntaps); }
+// Filter taps per stage of the slab kernel's filter ring.  A stage's hand-over in the issuing warp (about 190 clocks,
+// during which the tensor pipe runs dry) is paid once per stage, so a stage holds as many taps as leaves the ring two
+// or three stages: with one CTA 12 to 36 KB for narrow tiles and one tap for 128 and 256 filters, whose stages are 16
+// and 32 KB already; a pair's CTAs hold half of the filters, so they take three taps of 128 and two of 256.
+// Measured (one tap -> several, 64 images, float32 3x3): pairs 256 -> 256 at 56x56 401 -> 340 us, 128 -> 128 at
+// 112x112 with pooling 406 -> 341, 64 -> 128 at 112x112 240 -> 201; float16 512 -> 512 at 7x7, 256 images 110 -> 89.
+// 32-filter tiles, a filter row -> five taps: 32 groups of 8 channels at 28x28 184 -> 172 us.
+int slab_tps(int bn, int ntaps, bool pair) {
+  if (bn >= 128) return pair ? std::min(bn >= 256 ? 2 : 3, ntaps) : 1;
+  if (bn == 32 && ntaps <= 9) return ntaps;
+  return ntaps % 3 == 0 ? 3 : std::min(4, ntaps);
+}
+// Filter stages that a tile with the staged epilogue has to keep.
+int slab_min_stages(bool pair, int tps) { return tps >= 9 || (pair && tps >= 3) ? 2 : 3; }
 
-// Tile of the slab kernel.  spread = false: widest tile that holds the outputs, unsplit; true: the best over the
-// tile widths and slice counts as well.  `found` is false when nothing fits.
-SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, int Eh, int Ew, bool tma_layout_ok, bool spread) {
+// Tile of the slab kernel.  kSlabWide: widest tile that holds the outputs, unsplit; kSlabSpread: the best over the
+// tile widths and slice counts as well; kSlabPair: the tile of each CTA of a pair.  `found` is false when nothing fits.
+SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, int Eh, int Ew, bool tma_layout_ok, SlabMode mode) {
+  const bool spread = mode == kSlabSpread, pair = mode == kSlabPair;
   SlabTile& memo = c->slab_tiles[GeoKey{kGeoSlab, a.dtype, a.n_out, a.Cin_g, a.groups, a.N, Wt, Ht, ntaps, Eh, Ew, tma_layout_ok ? 1 : 0,
-                                        c->epi.pool, c->num_sms, spread ? 1 : 0}];
+                                        c->epi.pool, c->num_sms, mode}];
   if (memo.bn) return memo;
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
   const int bn_max = conv_umma_bn(a.n_out);
@@ -576,17 +591,18 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
   long long best_cost = -1, best_work = 0, best_tiles = 0;
   SlabTile best;
   best.bn = bn_max;
-  for (int BN = bn_max; BN >= (spread ? 32 : bn_max); BN /= 2) {
+  if (pair && (bn_max < 64 || c->num_sms < 2)) { memo = best; return best; }
+  const int units = pair ? c->num_sms / 2 : c->num_sms;
+  for (int BN = bn_max; BN >= (spread ? 32 : pair ? std::max(64, bn_max / 2) : bn_max); BN /= 2) {
     const int tiles_co = (int)cdiv(a.n_out, BN);
     const int acc_cap = std::min(512 / BN, 4);
-    const int tps = slab_tps(BN, ntaps);
-    const int b_bytes = tps * BN * 128;
-    const int mma_clk = mma_clocks(BN);
+    const int tps = slab_tps(BN, ntaps, pair);
+    const int b_bytes = tps * (pair ? BN / 2 : BN) * 128;
     const long long stages = kblocks_n * cdiv(ntaps, tps);
     // one tile candidate: search the one with the least serial work per SM
     auto consider = [&](int wt, int th, int nb, int n_acc, long long slab_bytes, bool row) {
       const long long tiles = cdiv(Wt, wt) * cdiv(Ht, th) * cdiv(a.N, nb);
-      const long long total = tiles * tiles_co * a.groups;
+      const long long total = (pair ? cdiv(tiles, 2) : tiles) * tiles_co * a.groups;
       // Clocks of the busiest SM: per tile and (tap, channel block) 4 MMAs per accumulator plus
       // about 120 clocks of stage hand-over in the issuing thread; then the accumulators are read
       // out, beside the next tile's MMAs when two accumulator sets fit the 512 TMEM columns.
@@ -597,17 +613,18 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
       const long long dense_rows = 1LL * wt * th * nb;
       const int ngr = n_acc == 3 ? 0 : 4 / n_acc;
       const long long stg = (dense_rows * 128 + 1023) / 1024 * 1024;
-      const long long min_b = std::min<long long>(3, stages + 1);   // filter stages the staged epilogue insists on
+      const long long min_b = std::min<long long>(slab_min_stages(pair, tps), stages + 1);   // filter stages the staged epilogue insists on
       if (c->epi.pool && ((wt | th) & 1)) return;          // pooling windows must not straddle tiles
       const bool tma_fit = tma_layout_ok && ngr > 0 && BN * es_out >= 128 && ngr * stg <= kSlabStageBytes &&
-                           (total <= c->num_sms ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
+                           (total <= units ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
                                                 : 2 * slab_bytes + min_b * b_bytes + kSlabStageBytes <= kSlabSmemBudget);
       // plus about 1500 clocks per tile for the pipeline to fill again
+      const int mma_clk = pair && n_acc == 1 && BN <= 128 ? 96 : mma_clocks(BN);
       auto mma_part = [&](long long st) { return st * (1LL * std::min(tps, ntaps) * 4 * n_acc * mma_clk + 120) + 1500; };
       const long long whole = 1LL * kblocks_n * (ntaps * 4LL * n_acc * mma_clk + cdiv(ntaps, tps) * 120) + 1500;
       const long long epi_part = tma_fit ? 2500 + dense_rows * BN * es_out / 32 : 2400LL * n_acc * (BN / 32);
       const long long per_tile = 2 * n_acc * BN <= 512 ? std::max(whole, epi_part) : whole + epi_part;
-      long long cost = cdiv(total, c->num_sms) * per_tile;
+      long long cost = cdiv(total, units) * per_tile;
       if (spread) cost += std::min(whole, epi_part);      // the last tile's read-out runs beside nothing (a few tiles per SM only)
       int splits = 1;
       const bool unsplit_ok = !c->epi.pool || tma_fit;     // unsplit, pooling happens in the staged epilogue only
@@ -651,7 +668,7 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
     if (Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && !c->epi.pool) {
       // one long row of pixels without halo (a flattened 1x1 layer): whole 128-pixel accumulators,
       // as many as still leave room for a second accumulator set
-      if (spread) {
+      if (spread || pair) {
         for (int n_acc = 1; n_acc <= (BN >= 256 ? 1 : 2); ++n_acc) consider(128 * n_acc, 1, 1, n_acc, 128 * 128 * n_acc, true);
       } else if (!best.found) {
         best.n_acc = BN >= 256 ? 1 : 2;
@@ -716,7 +733,7 @@ int split_output(b200conv_ctx* c, Scratch& tmp, const P& p, int bn, int rows, Co
 // error code.
 int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps, int rh,
                   int rw, int Wt, int Ht, void* out, long long sn, long long sc, long long sh,
-                  long long sw, long long off, const void* bias, int relu, bool spread) {
+                  long long sw, long long off, const void* bias, int relu, SlabMode mode) {
   if (taps.empty() || (int)taps.size() > kMaxTaps) return 2;
   const int ntap_all = (int)taps.size();
   int dh_min = taps[0].dh, dh_max = taps[0].dh, dw_min = taps[0].dw, dw_max = taps[0].dw;
@@ -732,17 +749,19 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   const bool tma_layout_ok = sc == 1 && a.n_out % (int)(128 / es_out) == 0 && !c->epi.residual &&
                              (sw * es_out) % 16 == 0 && (sh * es_out) % 16 == 0 && (sn * es_out) % 16 == 0 &&
                              reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es_out) % 16 == 0;
-  const SlabTile tile = find_slab_tile(c, a, ntap_all, Wt, Ht, Eh, Ew, tma_layout_ok, spread);
+  const SlabTile tile = find_slab_tile(c, a, ntap_all, Wt, Ht, Eh, Ew, tma_layout_ok, mode);
   if (!tile.found) return 2;
+  const bool pair = mode == kSlabPair;
   const int BN = tile.bn, tiles_co = (int)cdiv(a.n_out, BN);
-  const int tps = slab_tps(BN, ntap_all), b_bytes = tps * BN * 128;
+  const int b_rows = pair ? BN / 2 : BN;          // filters a CTA loads
+  const int tps = slab_tps(BN, ntap_all, pair), b_bytes = tps * b_rows * 128;
 #ifndef B200_PAIR_MIN_KBLOCKS
 #define B200_PAIR_MIN_KBLOCKS 4
 #endif
   constexpr long long kPairMinKblocks = B200_PAIR_MIN_KBLOCKS;
   // Flattened 1x1 layers with a deep reduction and 256-filter tiles: pairs of CTAs share the filter tile
   // (each loads half of it), which brings the operand traffic from L2 under what an SM can take.
-  if (!spread && tile.row && c->use_pair &&
+  if (mode == kSlabWide && tile.row && c->use_pair &&
       a.dtype == B200CONV_F16 && BN == 256 && a.n_out % 64 == 0 && a.groups == 1 && !a.fold && taps.size() == 1 &&
       kblocks_n >= kPairMinKblocks && tma_layout_ok && c->num_sms >= 2 && c->epi.beta == 0.f && !c->epi.pool) {
     PairGemmParams q;
@@ -779,6 +798,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.dw_min = dw_min; p.dh_min = dh_min;
   p.slab_bytes = b_slab;
   p.splits = tile.splits;
+  p.pair = pair;
   p.tps = tps;
   // Ring depths for `avail` bytes.  Activations come from HBM (the longer latency, and the stream
   // that bounds most layers): the slab ring gets up to 6 buffers once the filter ring holds what
@@ -791,7 +811,9 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     // this tile's MMAs are done: shallow reductions get one stage more than a tile consumes
     // (128 -> 512 1x1 forward: 100 -> 70 us with 3 instead of 2 stages)
     int b = std::min(fit, per_tile <= 2 ? per_tile + 1 : std::min(4, per_tile));
-    const int s_ = (int)std::max<long long>(2, std::min<long long>(6, (avail - 1LL * b * b_bytes) / b_slab));
+    int s_ = (int)std::max<long long>(2, std::min<long long>(6, (avail - 1LL * b * b_bytes) / b_slab));
+    // a slab lasts as many stages as a channel block has: beyond two, as many slabs as four stages consume
+    s_ = std::min(s_, 2 + (int)cdiv(4, cdiv((long long)taps.size(), tps)));
     b = (int)std::min<long long>(8, (avail - 1LL * s_ * b_slab) / b_bytes);
     *ss = s_; *bs = b;
 #ifdef B200CONV_TUNE
@@ -807,7 +829,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     // TMA-store epilogue: channels-last output whose 128-byte channel chunks never straddle a
     // group, 1/2/4 accumulators (so that the 16 epilogue warps split into equal groups)
     const long long tiles = cdiv(Wt, p.wt) * cdiv(Ht, p.th) * cdiv(a.N, p.nb);
-    const long long total = tiles * tiles_co * a.groups;
+    const long long total = (pair ? cdiv(tiles, 2) : tiles) * tiles_co * a.groups;
     const size_t es = elem_size(a.dtype);
     const long long dense_rows = 1LL * p.wt * p.th * p.nb;
     const int stage_bytes = (int)((dense_rows * 128 + 1023) / 1024 * 1024);
@@ -819,13 +841,13 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
               (sw * es) % 16 == 0 && (sh * es) % 16 == 0 && (sn * es) % 16 == 0 &&
               reinterpret_cast<uintptr_t>(obase) % 16 == 0;
     if (ok) {
-      if (total <= c->num_sms) {
+      if (total <= (pair ? c->num_sms / 2 : c->num_sms)) {
         p.stage_off = 0;                       // one tile per CTA: operands are dead by then
         p.stage_nbuf = std::min(8, (p.s_stages * b_slab + p.b_stages * b_bytes) / stage_bytes) / std::max(1, ngroups) * ngroups;
         ok = p.stage_nbuf >= ngroups;
       } else {
         int ss = 0, bs = 0;
-        if (plan_rings(kSlabSmemBudget - kSlabStageBytes, &ss, &bs) && bs >= std::min(3, per_tile + 1)) {
+        if (plan_rings(kSlabSmemBudget - kSlabStageBytes, &ss, &bs) && bs >= std::min(slab_min_stages(pair, tps), per_tile + 1)) {
           p.s_stages = ss;
           p.b_stages = bs;
           p.stage_off = ss * b_slab + bs * b_bytes;
@@ -861,9 +883,9 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   int rc = make_act_view(c, &p.view, a, rh, rw, kBK, p.Ws, p.Hs, p.nb);
   if (rc) return rc;
-  p.tap_boxes = a.groups != 1;
+  p.tap_boxes = 0;
   for (size_t i = 1; i < taps.size(); ++i) p.tap_boxes |= taps[i].wmat != taps[i - 1].wmat + 1;
-  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN, p.tap_boxes ? 1 : tps);
+  rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, b_rows, a.groups, p.tap_boxes ? 1 : tps);
   if (rc) return rc;
   for (const ConvTap& t : taps) {
     p.tap_shift[p.ntaps] = (int16_t)((t.dh - dh_min) * p.Ws + (t.dw - dw_min));
@@ -909,13 +931,13 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
                       const void* bias, int relu, int variant) {
-  if (variant == kConvSlab || variant == kConvSlabSpread) {
+  if (variant == kConvSlab || variant == kConvSlabSpread || variant == kConvSlabPair) {
     const int rh = view_parity[0].first, rw = view_parity[0].second;
     if (rh < a.Hs && rw < a.Ws) {
-      const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant == kConvSlabSpread);
+      const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, slab_mode(variant));
       if (rc != 2) return rc;
     }
-    variant = variant == kConvSlab ? kConvTap : kConvTapSpread;
+    variant = variant == kConvSlabSpread ? kConvTapSpread : kConvTap;
   }
   UmmaConvParams p;
   memset(&p, 0, sizeof p);
@@ -1016,7 +1038,7 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   auto run = [&](int variant) -> int {
     if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
       const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
-                                   relu, variant == kConvSlabSpread);
+                                   relu, slab_mode(variant));
       return rc == 2 ? fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool") : rc;
     }
     return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant);
@@ -1051,11 +1073,15 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     const size_t es = elem_size(a.dtype);
     const bool tma = sc == 1 && a.n_out % (int)(128 / es) == 0 && !c->epi.residual && (sw * es) % 16 == 0 && (sh * es) % 16 == 0 &&
                      (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
-    const SlabTile w = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, false);
-    const SlabTile n = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, true);
+    const SlabTile w = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabWide);
+    const SlabTile n = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabSpread);
     if (c->epi.pool && !(tma && w.found)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+    // pairs of CTAs where at least half of the SMs get work (below, the variants that spread a tile are ahead)
+    const SlabTile m = c->use_pair ? find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabPair) : SlabTile();
+    const bool pair = m.found && cdiv(cdiv(Wt, m.wt) * cdiv(Ht, m.th) * cdiv(a.N, m.nb), 2) * cdiv(a.n_out, m.bn) * a.groups >= c->num_sms / 4;
     if (w.found) cand[ncand++] = kConvSlab;
     if (n.found && (!w.found || n.splits > 1 || n.bn != w.bn || n.wt != w.wt || n.th != w.th || n.nb != w.nb)) cand[ncand++] = kConvSlabSpread;
+    if (pair) cand[ncand++] = kConvSlabPair;
   }
   if (ncand == 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
   if (!c->autotune || c->capturing || ncand == 1) return run(cand[ncand - 1]);
@@ -2915,14 +2941,13 @@ int b200conv_set_splits(b200conv_ctx* c, int splits) {
 
 // The tuning file: a header line naming the device the choices were timed on, then one line per
 // choice.  Choices made on another device model or SM count are not loaded.
-// Version 2: keys are lists of integers.  Files of version 1 (other keys) are read without effect.
-static std::string tuning_header(b200conv_ctx* c, int version) {
+static std::string tuning_header(b200conv_ctx* c) {
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, c->device);
   std::string name = prop.name;
   for (char& ch : name)
     if (ch == ' ') ch = '_';
-  return "b200conv-tuning " + std::to_string(version) + " " + name + " " + std::to_string(c->num_sms);
+  return "b200conv-tuning 1 " + name + " " + std::to_string(c->num_sms);
 }
 
 int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
@@ -2931,7 +2956,7 @@ int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
   DeviceGuard dg(c->device);
   FILE* f = fopen(path, "w");
   if (!f) return fail(c, B200CONV_E_INVALID, "cannot write %s", path);
-  fprintf(f, "%s\n", tuning_header(c, 2).c_str());
+  fprintf(f, "%s\n", tuning_header(c).c_str());
   for (auto& kv : c->algo_cache) fprintf(f, "a %s %d\n", kv.first.text().c_str(), kv.second);
   for (auto& kv : c->split_cache) fprintf(f, "s %s %d\n", kv.first.text().c_str(), kv.second);
   fclose(f);
@@ -2951,11 +2976,7 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
   if (ok) {
     std::string head = line;
     while (!head.empty() && (head.back() == '\n' || head.back() == '\r')) head.pop_back();
-    ok = head == tuning_header(c, 2);
-    if (!ok && head == tuning_header(c, 1)) {
-      fclose(f);
-      return 0;
-    }
+    ok = head == tuning_header(c);
   }
   if (!ok) {
     fclose(f);
@@ -2966,6 +2987,10 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
     int val = 0;
     GeoKey key{};
     if (sscanf(line, "%c %399s %d", &kind, text, &val) != 3 || !GeoKey::parse(text, &key)) continue;
+    // keys of another form (older files) are passed over
+    const bool known = kind == 'a' ? (key.v[0] == kGeoConv && key.n == 17) || (key.v[0] == kGeoWgrad && key.n == 19)
+                                   : key.v[0] == kGeoSplits && key.n == 20;
+    if (!known) continue;
     if (kind == 'a' && val >= 0 && val < kConvVariants) { c->algo_cache[key] = val; ++n; }
     else if (kind == 's' && val >= 1) { c->split_cache[key] = val; ++n; }
   }

@@ -14,6 +14,11 @@
 // warps; warp 18 is a second MMA issuer: with two or more accumulators per tile each issuer takes half
 // of them (different TMEM columns, the same operands, the same order of accumulation).  Producer and
 // issuer loops are followed by all 32 lanes of their warp; one elected lane issues.
+//
+// PAIR: two CTAs of a cluster work on two neighbouring pixel tiles and the same filters as one MMA unit (cta_group::2, M = 256).
+// What bounds the one-CTA form is shared memory, 128 B/clk: four 128 x 256 x 8 tf32 MMAs (512 clocks) read 48 KB and
+// the next filter tile's 32 KB are written beside them, 640 clocks; with 128 filters the operands alone take as long as the
+// MMA.  In a pair each CTA loads, and its MMAs read, half of the filter tile: 32 + 16 KB, 384 clocks.
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -42,13 +47,13 @@ template <typename T> __device__ __forceinline__ void store_out(T* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<__half>(__half* p, float v) { *p = __float2half_rn(v); }
 
-template <MmaKind KIND, int BN>
+template <MmaKind KIND, int BN, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   using OutT = typename std::conditional<KIND == MmaKind::TF32, float, __half>::type;
   constexpr int kBK = KIND == MmaKind::TF32 ? 32 : 64;
-  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, false, false, 128, BN);
-  constexpr int kBBytes = BN * 128;
+  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, false, false, PAIR ? 256 : 128, BN);
+  constexpr int kBBytes = (PAIR ? BN / 2 : BN) * 128;   // filters this CTA loads per tap and channel block
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -66,7 +71,12 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   const uint32_t slab_tx = static_cast<uint32_t>(p.nb * p.Hs * p.Ws) * 128u;
   // tile counts fit 32 bits (the launcher checks): 64-bit divisions per tile would cost each
   // role about a thousand clocks, a fifth of a small tile
-  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
+  const uint32_t pix_tiles = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n;
+  const uint32_t total = (PAIR ? (pix_tiles + 1) / 2 : pix_tiles) * p.groups * p.tiles_co * p.splits;
+  // a pair's CTAs take the pixel tiles 2 i and 2 i + 1 (the second of an odd count's last pair lies behind the last
+  // image: its loads read zeros and its stores are left out); splits is 1
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0;
+  const uint32_t first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;
   // Work item = (tile, slice of the reduction), the slices of a tile side by side.  A slice is a range of
   // filter stages (channel block x group of tps taps), in the order the unsplit loop walks them.
   const uint32_t splits = p.splits;
@@ -93,17 +103,23 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars->acc_full[b], issuers);
-      mbar_init(&bars->acc_empty[b], 32 * kEpilogueWarps);
+      mbar_init(&bars->acc_empty[b], PAIR ? 2 : 32 * kEpilogueWarps);     // a pair: one arrival per CTA, on the even one
     }
     bars->abort = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem_base, 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(&bars->tmem_base, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&bars->tmem_base, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();      // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
@@ -119,20 +135,20 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     int sb = 0;
     uint32_t sphase = 0;
     bool ok = true;
-    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
+    for (uint32_t item = first; item < total && ok; item += stride) {
       const uint32_t t = item / splits;
       const Range r = slice_range(item - t * splits);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = t / co_groups;
+      const uint32_t pt = PAIR ? t / co_groups * 2 + rank : t / co_groups;
       const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
       const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.th;
       const int n0 = (pt / tiles_wh) * p.nb;
       for (int kb = r.kb0; kb <= r.kb1; ++kb) {
         if (!uniform_wait(&bars->slab_empty[sb], sphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (leader) {
-          mbar_expect_tx(&bars->slab_full[sb], slab_tx);
-          tma_load_5d(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, g, w0 + p.dw_min,
-                      h0 + p.dh_min, n0);
+          if (rank == 0) mbar_expect_tx(&bars->slab_full[sb], PAIR ? 2 * slab_tx : slab_tx);      // both CTAs' bytes
+          if (PAIR) tma_load_5d_pair(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, g, w0 + p.dw_min, h0 + p.dh_min, n0);
+          else tma_load_5d(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, g, w0 + p.dw_min, h0 + p.dh_min, n0);
         }
         if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
       }
@@ -145,11 +161,16 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     int bs = 0;
     uint32_t bphase = 0;
     bool ok = true;
-    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
+    for (uint32_t item = first; item < total && ok; item += stride) {
       const uint32_t t = item / splits;
       const Range r = slice_range(item - t * splits);
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
+      const int row0 = co_t * BN + static_cast<int>(rank) * (BN / 2);     // a pair's CTAs load one half each
+      auto load = [&](uint8_t* dst, int kb, int mat) {
+        if (PAIR) tma_load_4d_pair(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);
+        else tma_load_4d(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);
+      };
       for (int kb = r.kb0; kb <= r.kb1 && ok; ++kb) {
         const int tap_end = kb == r.kb1 ? min(p.ntaps, (r.tg1 + 1) * p.tps) : p.ntaps;
         for (int tap = kb == r.kb0 ? r.tg0 * p.tps : 0; tap < tap_end; tap += p.tps) {
@@ -160,13 +181,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             // 128 x 64 taps: neighbouring taps come as one box.  (The box of a last, shorter group reads on into
             // the next matrix or zeros; its bytes count too.)
             if (!p.tap_boxes) {
-              mbar_expect_tx(&bars->b_full[bs], p.tps * kBBytes);
-              tma_load_3d(bring + bs * stage_b, &p.wmap, &bars->b_full[bs], kb * kBK, co_t * BN, p.tap_wmat[tap]);
+              if (rank == 0) mbar_expect_tx(&bars->b_full[bs], (PAIR ? 2 : 1) * p.tps * kBBytes);
+              load(bring + bs * stage_b, kb, p.tap_wmat[tap]);
             } else {
-              mbar_expect_tx(&bars->b_full[bs], nt * kBBytes);
-              for (int q = 0; q < nt; ++q)
-                tma_load_3d(bring + bs * stage_b + q * kBBytes, &p.wmap, &bars->b_full[bs], kb * kBK, co_t * BN,
-                            p.tap_wmat[tap + q] * p.groups + g);
+              if (rank == 0) mbar_expect_tx(&bars->b_full[bs], (PAIR ? 2 : 1) * nt * kBBytes);
+              for (int q = 0; q < nt; ++q) load(bring + bs * stage_b + q * kBBytes, kb, p.tap_wmat[tap + q]);
             }
           }
           if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
@@ -179,7 +198,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     const int a_split = issuers == 2 ? (p.n_acc + 1) / 2 : p.n_acc;
     const int a_begin = warp == 1 ? 0 : a_split, a_end = warp == 1 ? a_split : p.n_acc;
     if (warp != 1) trace = nullptr;            // the stamps are the first issuer's
-    if (a_begin < a_end) {
+    if (rank == 0 && a_begin < a_end) {        // a pair: the even CTA issues for both
       // All 32 lanes follow the loop and wait on the barriers; one elected lane issues the MMAs
       // and their commits.  A lone lane (code under `if (lane == 0)`) computes every descriptor
       // on the per-thread datapath and moves it to uniform registers per MMA, which costs more
@@ -195,7 +214,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const uint64_t desc_bits = smem_desc(0, 16, 1024);
       const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
       const uint32_t desc_lo = static_cast<uint32_t>(desc_bits);
-      for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+      auto commit = [&](uint64_t* bar) {
+        if (PAIR) umma_commit_pair(bar);
+        else umma_commit(bar);
+      };
+      for (uint32_t item = first; item < total && ok; item += stride, ++it) {
         const Range r = slice_range(item % splits);
         // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
         // runs beside the MMAs of the next one
@@ -230,18 +253,18 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
                 for (int a = a_begin; a < a_end; ++a) {
 #pragma unroll
                   for (int kk = 0; kk < 4; ++kk)
-                    umma_words<KIND>(acc_base + a * BN, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, first | (kk != 0));
+                    umma_words<KIND, PAIR>(acc_base + a * BN, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, first | (kk != 0));
                   a_lo += (128 * 128) >> 4;      // next accumulator: 128 slab rows further
                 }
               }
-              umma_commit(&bars->b_empty[bs]);
+              commit(&bars->b_empty[bs]);
             }
             if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
           }
-          if (ok && leader) umma_commit(&bars->slab_empty[sb]);
+          if (ok && leader) commit(&bars->slab_empty[sb]);
           if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
         }
-        if (ok && leader) umma_commit(&bars->acc_full[buf]);
+        if (ok && leader) commit(&bars->acc_full[buf]);
         if (trace && it == 0) trace[3] = clock64();
       }
       if (!ok && leader) report_status(p.status, kStatusTimeout);
@@ -265,11 +288,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     long long te_wait = 0, te_busy = 0;          // clocks of thread 64 (only with trace)
     long long tp[5] = {0, 0, 0, 0, 0};           // its epilogue phases: buffer wait, TMEM read, convert + stage, fence + barrier, store issue
     int nstore = 0;                              // chunks this warp's group has staged so far
-    for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
+    for (uint32_t item = first; item < total && ok; item += stride, ++it) {
       const uint32_t t = item / splits;
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = t / co_groups;
+      const uint32_t pt = PAIR ? t / co_groups * 2 + rank : t / co_groups;
       const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
       const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.th;
       const int n0 = (pt / tiles_wh) * p.nb;
@@ -450,7 +473,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           if (trace) { const long long t = clock64(); tp[3] += t - tq; tq = t; }
           // a tiled store must not start at a negative coordinate, and its staging rows must lie
           // inside the reserved shared memory
-          if (issuer && B200_IN_RANGE(g * p.n_out + co0 >= 0 && w0 >= 0 && h0 >= 0 && n0 >= 0 && w0 < p.Wt && h0 < p.Ht &&
+          if (issuer && (!PAIR || n0 < p.Nimg) && B200_IN_RANGE(g * p.n_out + co0 >= 0 && w0 >= 0 && h0 >= 0 && n0 >= 0 && w0 < p.Wt && h0 < p.Ht &&
                                       n0 < p.Nimg && ch * kCh + kCh <= BN, p.status)) {
             if (p.epi.pool) tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0 >> 1, h0 >> 1, n0);
             else tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0, h0, n0);
@@ -519,7 +542,12 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         }
       }
       tc_fence_before();
-      mbar_arrive(&bars->acc_empty[buf]);
+      if (PAIR) {
+        named_barrier(5, 32 * kEpilogueWarps);
+        if (warp == 2 && lane == 0) mbar_arrive_leader(&bars->acc_empty[buf]);
+      } else {
+        mbar_arrive(&bars->acc_empty[buf]);
+      }
       if (trace && it == 0 && threadIdx.x == 64) trace[5] = clock64();
       if (trace) { te_wait += te1 - te0; te_busy += clock64() - te1; }
     }
@@ -534,9 +562,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   tc_fence_before();
   __syncthreads();
   if (bars->abort) abort_grace(p.wait_clocks);
+  if (PAIR) cluster_sync_all();              // no CTA of the pair leaves (or frees TMEM) while the other may still signal it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    if (PAIR) tmem_dealloc_pair(tmem, 512);
+    else tmem_dealloc(tmem, 512);
   }
   if (trace && threadIdx.x == 0) {
     trace[6] = clock64();
@@ -544,38 +574,51 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   }
 }
 
-template <MmaKind KIND, int BN>
+template <MmaKind KIND, int BN, bool PAIR>
 cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cudaStream_t s) {
-  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.tps * BN * 128 + p.stage_reserved + sizeof(Bars) + 1024;
+  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.tps * (PAIR ? BN / 2 : BN) * 128 + p.stage_reserved + sizeof(Bars) + 1024;
   static PerDeviceOnce configured;
   cudaError_t e = configured.ensure([] {
-    return cudaFuncSetAttribute(conv_slab_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    return cudaFuncSetAttribute(conv_slab_kernel<KIND, BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   });
   if (e != cudaSuccess) return e;
-  const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  launch_chained(conv_slab_kernel<KIND, BN>, grid, kThreads, smem, s, p);
+  const int units = PAIR ? num_sms / 2 : num_sms;
+  const int grid = static_cast<int>(total < units ? total : units) * (PAIR ? 2 : 1);
+  launch_linked(true, conv_slab_kernel<KIND, BN, PAIR>, grid, kThreads, smem, s, PAIR ? 2 : 1, p);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num_sms, cudaStream_t s) {
-  const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
+  const long long pix = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
+  const long long total = (p.pair ? (pix + 1) / 2 : pix) * p.groups * p.tiles_co * p.splits;
   if (total == 0 || p.ntaps == 0) return cudaSuccess;
-  if (total >= (1LL << 31)) return cudaErrorInvalidValue;
+  if (total >= (1LL << 31) || (p.pair && (p.splits != 1 || num_sms < 2))) return cudaErrorInvalidValue;
   const bool f16 = dtype == B200CONV_F16;
 #define B200_CASE(BNV)                                                                  \
   case BNV:                                                                             \
-    return f16 ? launch_one<MmaKind::F16, BNV>(p, total, num_sms, s)                    \
-               : launch_one<MmaKind::TF32, BNV>(p, total, num_sms, s);
+    return f16 ? launch_one<MmaKind::F16, BNV, false>(p, total, num_sms, s)             \
+               : launch_one<MmaKind::TF32, BNV, false>(p, total, num_sms, s);
+#define B200_PAIR(BNV)                                                                  \
+  case BNV:                                                                             \
+    return f16 ? launch_one<MmaKind::F16, BNV, true>(p, total, num_sms, s)              \
+               : launch_one<MmaKind::TF32, BNV, true>(p, total, num_sms, s);
+  if (p.pair) switch (bn) {
+    B200_PAIR(64)
+    B200_PAIR(128)
+    B200_PAIR(256)
+    default: return cudaErrorInvalidValue;
+  }
   switch (bn) {
     B200_CASE(32)
     B200_CASE(64)
     B200_CASE(128)
+    default:
     B200_CASE(256)
   }
 #undef B200_CASE
-  return cudaErrorInvalidValue;
+#undef B200_PAIR
 }
 
 }  // namespace b200

@@ -48,24 +48,26 @@ __device__ __forceinline__ void pdl_enter() {
 }
 #endif
 template <class... Exp, class... Act>
-cudaError_t launch_linked(bool chained, void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = chained ? 1 : 0;
+cudaError_t launch_linked(bool chained, void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster, Act&&... args) {
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = chained ? 1 : 0;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cfg.attrs = &at; cfg.numAttrs = 1;
+  cfg.attrs = at; cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Exp>(args)...);
 }
 
 template <class... Exp, class... Act>
 cudaError_t launch_chained(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
-  return launch_linked(true, kernel, grid, block, smem, s, args...);
+  return launch_linked(true, kernel, grid, block, smem, s, 1, args...);
 }
 constexpr unsigned kChainedBlocks = 148 * 8;      // of 256 threads
 template <class... Exp, class... Act>
 cudaError_t launch_streaming(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
-  return launch_linked(grid.x * grid.y * grid.z <= kChainedBlocks, kernel, grid, block, smem, s, args...);
+  return launch_linked(grid.x * grid.y * grid.z <= kChainedBlocks, kernel, grid, block, smem, s, 1, args...);
 }
 
 // Codes a kernel writes to the device status word when it gives up.
@@ -134,7 +136,7 @@ cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cu
 // once per channel block and every tap is a row offset into it.
 struct alignas(64) SlabConvParams {
   CUtensorMap view;              // 5-D (c_in_group, group, w, h, n), box (kBK, 1, Ws, Hs, nb)
-  CUtensorMap wmap;              // 3-D packed filters, box (kBK, BN, 1)
+  CUtensorMap wmap;              // 4-D packed filters (k_red, n_out, group, tap), box (kBK, BN or half of it, 1, 1 or tps)
   int16_t tap_shift[kMaxTaps];   // row offset of the tap inside the slab
   int16_t tap_wmat[kMaxTaps];
   int ntaps;
@@ -151,6 +153,7 @@ struct alignas(64) SlabConvParams {
   int s_stages;                  // slab ring depth (2 .. 6)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
   float* partial;
+  int pair;                      // 1: CTA pairs (two pixel tiles side by side, M = 256); splits is 1
   int tap_boxes;                 // 1: one TMA box per tap; 0: the taps of a stage are neighbours in the packed filters
                                  // and arrive as one box (the map's box then is tps matrices deep)
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
