@@ -1706,9 +1706,9 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
     p.tap_wmat[i] = (int16_t)taps[i].wmat;
   }
   for (int v = 0; v < nviews; ++v) p.view_dwmin[v] = (int16_t)dwmin[v];
-  // float16 layers with at most 64 channels: a tap group becomes one MMA whose column groups are the taps, if the
-  // taps of every group are evenly spaced (stride and dilation decide the spacing; 1 for a plain 3x3 filter)
-  if (d.dtype == B200CONV_F16 && Cg <= 64 && c->stack_taps) {
+  // Layers with at most 64 channels: a tap group becomes one MMA (tf32: one per 32 channels) whose column groups are
+  // the taps, if the taps of every group are evenly spaced (stride and dilation decide the spacing; 1 for a plain 3x3 filter)
+  if (Cg <= 64 && c->stack_taps) {
     int step = 0;
     bool even = true;
     for (int gi = 0; gi < p.ngroups && even; ++gi)

@@ -274,7 +274,7 @@ struct alignas(64) GroupWgradParams {
   int16_t tap_off[kMaxTaps];       // dw - dw_min of the tap's view: row offset into the x tile
   int16_t tap_wmat[kMaxTaps];      // filter tap index in OIHW order (after flip)
   int stack_step;                  // > 0: at most 64 channels and the taps of every group this many rows apart:
-                                   // a group's taps are column groups of one MMA (0: one MMA per tap)
+                                   // a group's taps are column groups of one MMA, tf32: of one per 32 channels (0: one MMA per tap)
   int ngroups;
   int groups;                      // convolution groups
   int Kg, Cg;
@@ -282,6 +282,7 @@ struct alignas(64) GroupWgradParams {
   int Wa, Wb, th, nb;              // dy / x box widths, rows and images per stage
   int wt;                          // output columns owned by a tile (== Wo in full-width mode)
   int rows_a, rows_b;              // box rows Wa*th*nb, Wb*th*nb
+  int box_bytes, a_boxes, b_boxes, stages, ring_bytes;      // shared-memory ring (set by launch_wgrad_group)
   int tiles_w, tiles_h, tiles_n;
   int ktiles, ctiles;
   int splits;

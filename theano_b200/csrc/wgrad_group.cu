@@ -17,6 +17,8 @@
 // swizzle period are fine because the hardware swizzles on absolute shared-memory address bits.
 // Warp roles: warp 0 and the last three warps TMA producers, warp 1 MMA issuer and TMEM owner,
 // 16 epilogue warps.
+#include <algorithm>
+
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -31,17 +33,20 @@ constexpr int kProducers = 4;
 constexpr int kFirstExtraProducer = 2 + kEpilogueWarps;
 constexpr int kThreads = 32 * (kFirstExtraProducer + kProducers - 1);
 constexpr int kBN = 128;                       // channels per accumulator
-// box rows = the stage's pixel rows + room for the largest column offset (16); bytes are a multiple
-// of the 1024-byte swizzle period
-template <MmaKind KIND> constexpr int box_rows() { return (KIND == MmaKind::TF32 ? kWgradPixF32 : kWgradPixF16) + 16; }
-template <MmaKind KIND> constexpr int box_bytes() { return box_rows<KIND>() * 128; }
-constexpr int kSmemBudget = 208 * 1024;
+// A box holds the stage's pixel rows and room for the largest column offset (p.box_bytes, a multiple of the 1024-byte
+// swizzle period); a stage holds the boxes that the layer's filters and channels fill (p.a_boxes + p.b_boxes of at most
+// 128 / atom each).  What bounds a stage of a narrow layer is the latency of its boxes, so the ring is as deep as
+// the shared memory allows: with room for 128 x 128 in every stage there were two stages for every layer.
+// An MMA reads 128 rows and its columns whatever the layer has: behind a stage's boxes that is other operand data
+// (allocated memory, rows and columns of the accumulator that nobody reads).
+constexpr int kSmemBudget = 222 * 1024;
 constexpr int kMaxStages = 6;
 
 template <MmaKind KIND> constexpr int atom() { return KIND == MmaKind::TF32 ? 32 : 64; }
-template <MmaKind KIND> constexpr int stage_bytes() { return (128 / atom<KIND>() + kBN / atom<KIND>()) * box_bytes<KIND>(); }
-template <MmaKind KIND> constexpr int num_stages() {
-  return (kSmemBudget / stage_bytes<KIND>()) > kMaxStages ? kMaxStages : (kSmemBudget / stage_bytes<KIND>());
+// Operand memory of a ring, the reach of the last stage's MMAs included.
+int ring_bytes(int stages, int atom, int a_boxes, int b_boxes, int box_bytes) {
+  const int full = 128 / atom;
+  return ((stages - 1) * (a_boxes + b_boxes) + a_boxes + full) * box_bytes;
 }
 
 struct alignas(16) Bars {
@@ -82,7 +87,7 @@ __device__ __forceinline__ Item decode(uint32_t it, const GroupWgradParams& p, u
 // takes (64 for 128 x 128 x 8 tf32).
 template <MmaKind KIND, int NT, int KS>
 __device__ __forceinline__ void issue_stage(uint32_t tmem, uint32_t a_lo, uint32_t b_lo, const uint32_t (&toff)[4],
-                                            uint32_t desc_hi, int ksteps, uint32_t acc, uint32_t stack_delta) {
+                                            uint32_t desc_hi, int ksteps, uint32_t acc, uint32_t stack_delta, uint32_t box2) {
   constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;
   constexpr uint32_t kStep = (kK * 128) >> 4;
   constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, kBN);
@@ -90,12 +95,19 @@ __device__ __forceinline__ void issue_stage(uint32_t tmem, uint32_t a_lo, uint32
 #pragma unroll
   for (int q = 0; q < NT; ++q) bq[q] = b_lo + toff[q];
   if (stack_delta) {
-    // Layers with at most 64 channels: the NT taps become NT groups of 64 columns of ONE MMA.  The x operand's
-    // leading-dimension offset (the distance between 64-column groups) is set to the taps' row spacing, so that
-    // column group q reads the x tile q taps further: 128 x (64 NT) instead of NT half-empty 128 x 128 MMAs.
-    constexpr uint32_t kIdescStack = instr_desc(KIND == MmaKind::TF32, true, true, 128, 64 * NT);
+    // Layers with at most 64 channels: the NT taps become NT groups of columns of ONE MMA per swizzle atom of channels
+    // (64 in float16, 32 in tf32).  The x operand's leading-dimension offset (the distance between column groups)
+    // is set to the taps' row spacing, so that column group q reads the x tile q taps further: 128 x (64 NT)
+    // (tf32: at most two of 128 x (32 NT)) instead of NT half-empty 128 x 128 MMAs.
+    constexpr int kAtom = atom<KIND>();
+    constexpr bool kPlain = NT == 1;                 // a single tap: its atoms are the column groups, as ever
+    constexpr uint32_t kIdescStack = instr_desc(KIND == MmaKind::TF32, true, true, 128, kPlain ? 64 : kAtom * NT);
+    const uint32_t b0 = bq[0] + (kPlain ? 0u : stack_delta);
+    const bool second = KIND == MmaKind::TF32 && !kPlain && box2;   // box2: distance of the second atom of channels, or 0
     for (int ks = 0; ks < ksteps; ++ks) {
-      umma_words<KIND>(tmem, a_lo + ks * kStep, bq[0] + stack_delta + ks * kStep, desc_hi, kIdescStack, acc);
+      umma_words<KIND>(tmem, a_lo + ks * kStep, b0 + ks * kStep, desc_hi, kIdescStack, acc);
+      if (second)
+        umma_words<KIND>(tmem + kAtom * NT, a_lo + ks * kStep, b0 + box2 + ks * kStep, desc_hi, kIdescStack, acc);
       acc = 1u;
     }
     return;
@@ -134,11 +146,9 @@ template <MmaKind KIND, int NT, int KS>
 __device__ __forceinline__ bool mma_item(Bars* bars, uint32_t tmem, uint32_t lo_base, uint32_t desc_hi,
                                          const uint32_t (&toff)[4], int ksteps, int ntiles, int& stage,
                                          uint32_t& phase, long long& t_wait, bool timed, bool leader,
-                                         long long limit, uint32_t stack_delta) {
-  constexpr int kAtom = atom<KIND>();
-  constexpr int kABoxes = 128 / kAtom;
-  constexpr int kStages = num_stages<KIND>();
-  constexpr int kBoxBytes = box_bytes<KIND>();
+                                         long long limit, uint32_t stack_delta, uint32_t box2,
+                                         const GroupWgradParams& p) {
+  const uint32_t a_units = (p.a_boxes * p.box_bytes) >> 4, stage_units = ((p.a_boxes + p.b_boxes) * p.box_bytes) >> 4;
   uint32_t acc = 0u;
   for (int t = 0; t < ntiles; ++t) {
     if (timed) {
@@ -149,15 +159,15 @@ __device__ __forceinline__ bool mma_item(Bars* bars, uint32_t tmem, uint32_t lo_
       return false;
     }
     tc_fence_after();
-    const uint32_t a_lo = lo_base + stage * (stage_bytes<KIND>() >> 4);
-    const uint32_t b_lo = a_lo + ((kABoxes * kBoxBytes) >> 4);
+    const uint32_t a_lo = lo_base + stage * stage_units;
+    const uint32_t b_lo = a_lo + a_units;
     if (leader) {
-      issue_stage<KIND, NT, KS>(tmem, a_lo, b_lo, toff, desc_hi, ksteps, acc, stack_delta);
+      issue_stage<KIND, NT, KS>(tmem, a_lo, b_lo, toff, desc_hi, ksteps, acc, stack_delta, box2);
       umma_commit(&bars->empty[stage]);
     }
     acc = 1u;
     const int next = stage + 1;
-    const bool wrap = next == kStages;
+    const bool wrap = next == p.stages;
     stage = wrap ? 0 : next;
     phase ^= wrap ? 1u : 0u;
   }
@@ -169,8 +179,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   constexpr int kAtom = atom<KIND>();
   constexpr int kABoxes = 128 / kAtom, kBBoxes = kBN / kAtom;
-  constexpr int kStages = num_stages<KIND>();
-  constexpr int kBoxBytes = box_bytes<KIND>(), kBoxRows = box_rows<KIND>();
+  const int box_bytes = p.box_bytes, stage_bytes = (p.a_boxes + p.b_boxes) * box_bytes;
   constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;
   constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, kBN);
   constexpr uint32_t kSbo = KIND == MmaKind::TF32 ? 512 : 1024;
@@ -179,7 +188,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  Bars* bars = reinterpret_cast<Bars*>(smem + kStages * stage_bytes<KIND>());
+  Bars* bars = reinterpret_cast<Bars*>(smem + p.ring_bytes);
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   // phase timing (optional): [0] MMA thread waiting for operands, [1] its whole loop,
@@ -194,7 +203,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   const uint32_t total = static_cast<uint32_t>(p.ktiles) * p.ctiles * p.groups * p.ngroups * p.splits;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(&bars->full[s], 1);
       mbar_init(&bars->empty[s], 1);
     }
@@ -211,16 +220,16 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   // for the x operand, up to the largest column offset further: clear those rows once.  (dy rows
   // there must be zero; the x rows only need to be finite.)
   {
-    const int boxes = kStages * (kABoxes + kBBoxes);
+    const int boxes = p.stages * (p.a_boxes + p.b_boxes);
     const int first = min(p.rows_a, p.rows_b);
-    const int nrows = kBoxRows - first;
+    const int nrows = box_bytes / 128 - first;
     for (int i = threadIdx.x; i < boxes * nrows * 8; i += kThreads) {
       const int box = i / (nrows * 8), rem = i % (nrows * 8);
-      const int stage_box = box % (kABoxes + kBBoxes);
+      const int stage_box = box % (p.a_boxes + p.b_boxes);
       const int row = first + rem / 8;
-      const int written = stage_box < kABoxes ? p.rows_a : p.rows_b;
+      const int written = stage_box < p.a_boxes ? p.rows_a : p.rows_b;
       if (row >= written)
-        *(reinterpret_cast<uint4*>(smem + box * kBoxBytes + row * 128) + rem % 8) = make_uint4(0, 0, 0, 0);
+        *(reinterpret_cast<uint4*>(smem + box * box_bytes + row * 128) + rem % 8) = make_uint4(0, 0, 0, 0);
     }
     fence_async_smem();
   }
@@ -263,20 +272,20 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
         const long long tw0 = trace ? clock64() : 0;
         if (!uniform_wait(&bars->empty[stage], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (trace) t_wait += clock64() - tw0;
-        uint8_t* sa = smem + stage * stage_bytes<KIND>();
-        uint8_t* sb = sa + kABoxes * kBoxBytes;
+        uint8_t* sa = smem + stage * stage_bytes;
+        uint8_t* sb = sa + p.a_boxes * box_bytes;
         if (leader) {
           if (pw == 0) mbar_expect_tx(&bars->full[stage], tx);
           for (int j = pw; j < a_boxes + b_boxes; j += kProducers) {
             if (j < a_boxes)
-              tma_load_5d(sa + j * kBoxBytes, &p.dy_map, &bars->full[stage], w.kt * 128 + j * kAtom, w.g,
+              tma_load_5d(sa + j * box_bytes, &p.dy_map, &bars->full[stage], w.kt * 128 + j * kAtom, w.g,
                           w0, h0, n0);
             else
-              tma_load_5d(sb + (j - a_boxes) * kBoxBytes, &p.x_views[view], &bars->full[stage],
+              tma_load_5d(sb + (j - a_boxes) * box_bytes, &p.x_views[view], &bars->full[stage],
                           w.ct * kBN + (j - a_boxes) * kAtom, w.g, w0 + dwmin, h0 + dh, n0);
           }
         }
-        if (++stage == kStages) { stage = 0; phase ^= 1; }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
     }
     if (!ok && leader) report_status(p.status, kStatusTimeout);
@@ -289,14 +298,15 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
     bool ok = true;
     int n = 0;
     long long t_wait = 0;
-    const uint64_t desc_bits = smem_desc(0, kBoxBytes, kSbo, kLayout);
+    const uint64_t desc_bits = smem_desc(0, box_bytes, kSbo, kLayout);
     const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
     const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
     const bool timed = trace != nullptr;
     const long long lim = p.wait_clocks;
     // stacked taps: the low descriptor word carries the leading-dimension offset in bits [16, 30)
     const uint32_t stack_delta = p.stack_step > 0
-        ? ((static_cast<uint32_t>(p.stack_step * 128) >> 4) - (static_cast<uint32_t>(kBoxBytes) >> 4)) << 16 : 0u;
+        ? ((static_cast<uint32_t>(p.stack_step * 128) >> 4) - (static_cast<uint32_t>(box_bytes) >> 4)) << 16 : 0u;
+    const uint32_t box2 = p.Cg > kAtom ? static_cast<uint32_t>(box_bytes) >> 4 : 0u;      // used with stacked taps
     for (uint32_t it = blockIdx.x; it < total && ok; it += gridDim.x, ++n) {
       const Item w = decode(it, p, per_split, pix_tiles);
       const int first_tap = p.grp_first[w.grp], ntap = p.grp_n[w.grp];
@@ -309,14 +319,14 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
       tc_fence_after();
       const int ntiles = static_cast<int>(w.t_end - w.t_begin);
       switch (ntap) {
-        case 1: ok = (ksteps == 8 && !timed ? mma_item<KIND, 1, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta)
-                                             : mma_item<KIND, 1, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta)); break;
-        case 2: ok = (ksteps == 8 && !timed ? mma_item<KIND, 2, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta)
-                                             : mma_item<KIND, 2, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta)); break;
-        case 3: ok = (ksteps == 8 && !timed ? mma_item<KIND, 3, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta)
-                                             : mma_item<KIND, 3, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta)); break;
-        default: ok = (ksteps == 8 && !timed ? mma_item<KIND, 4, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta)
-                                             : mma_item<KIND, 4, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta)); break;
+        case 1: ok = (ksteps == 8 && !timed ? mma_item<KIND, 1, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
+                                             : mma_item<KIND, 1, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
+        case 2: ok = (ksteps == 8 && !timed ? mma_item<KIND, 2, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
+                                             : mma_item<KIND, 2, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
+        case 3: ok = (ksteps == 8 && !timed ? mma_item<KIND, 3, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
+                                             : mma_item<KIND, 3, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
+        default: ok = (ksteps == 8 && !timed ? mma_item<KIND, 4, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
+                                             : mma_item<KIND, 4, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
       }
       if (ok && leader) umma_commit(&bars->acc_full);
     }
@@ -345,7 +355,9 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
         const int c0 = w.ct * kBN + ch * 32;
         if (c0 >= p.Cg) continue;
         uint32_t r[32];
-        tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + q * (p.stack_step > 0 ? 64 : kBN) + ch * 32, r);
+        // columns of tap q, channels 32 ch: side by side per tap, or per atom of channels and then per tap
+        const int col = p.stack_step > 0 ? (ch * 32 / kAtom) * (kAtom * ntap) + q * kAtom + ch * 32 % kAtom : q * kBN + ch * 32;
+        tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + col, r);
         tmem_ld_wait();
         if (!valid) continue;
         float* dst = p.partial +
@@ -389,9 +401,9 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
 
 template <MmaKind KIND>
 cudaError_t launch_one(const GroupWgradParams& p, long long total, int num_sms, cudaStream_t s) {
-  constexpr int smem = num_stages<KIND>() * stage_bytes<KIND>() + sizeof(Bars) + 1024;
+  const int smem = p.ring_bytes + static_cast<int>(sizeof(Bars)) + 1024;
   static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_group_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_group_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
   launch_chained(wgrad_group_kernel<KIND>, grid, kThreads, smem, s, p);
@@ -400,10 +412,23 @@ cudaError_t launch_one(const GroupWgradParams& p, long long total, int num_sms, 
 
 }  // namespace
 
-cudaError_t launch_wgrad_group(const GroupWgradParams& p, int dtype, int num_sms, cudaStream_t s) {
+cudaError_t launch_wgrad_group(const GroupWgradParams& params, int dtype, int num_sms, cudaStream_t s) {
+  GroupWgradParams p = params;
   const long long total = 1LL * p.ktiles * p.ctiles * p.groups * p.ngroups * p.splits;
   if (total == 0) return cudaSuccess;
   if (total >= (1LL << 31) || 1LL * p.tiles_w * p.tiles_h * p.tiles_n >= (1LL << 31)) return cudaErrorInvalidValue;
+  const int at = dtype == B200CONV_F16 ? 64 : 32, kk = dtype == B200CONV_F16 ? 16 : 8;
+  int reach = 0, ntaps = 0;                     // rows of an x tile that the MMAs read
+  for (int g = 0; g < p.ngroups; ++g) ntaps += p.grp_n[g];
+  for (int t = 0; t < ntaps; ++t) reach = std::max<int>(reach, p.tap_off[t]);
+  reach += (p.rows_a + kk - 1) / kk * kk;
+  p.box_bytes = round_up(std::max(reach, std::max(p.rows_a, p.rows_b)), 8) * 128;
+  p.a_boxes = std::min(128 / at, (p.Kg + at - 1) / at);
+  p.b_boxes = std::min(128 / at, (p.Cg + at - 1) / at);
+  p.stages = kMaxStages;
+  while (p.stages > 2 && ring_bytes(p.stages, at, p.a_boxes, p.b_boxes, p.box_bytes) > kSmemBudget) --p.stages;
+  p.ring_bytes = ring_bytes(p.stages, at, p.a_boxes, p.b_boxes, p.box_bytes);
+  if (p.ring_bytes > kSmemBudget) return cudaErrorInvalidValue;
   return dtype == B200CONV_F16 ? launch_one<MmaKind::F16>(p, total, num_sms, s)
                                : launch_one<MmaKind::TF32>(p, total, num_sms, s);
 }
