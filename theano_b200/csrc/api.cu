@@ -84,7 +84,7 @@ struct GeoHash {
     return h ^ (h >> 29);
   }
 };
-enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance };      // kinds (first integer of a key)
+enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance, kGeoClasses };      // kinds (first integer of a key)
 
 // Tile of a convolution kernel for one geometry (the result of a search).
 struct SlabTile {
@@ -503,6 +503,10 @@ struct FwdLikeArgs {
   // Row folding (few input channels): `act` is [N][Hs][fold_Wp][Cp_in] with explicit zero columns;
   // the view's column index is the output column, its innermost extent runs over kW pixels x Cp_in
   // channels (Cin_g is that folded length) and only the filter rows remain as taps.
+  // Output classes of the slab kernel (strided gradInputs): class, extent and element offset of each
+  struct Class { int W, H; long long off; };
+  std::vector<Class> classes;
+  std::vector<uint8_t> tap_cls;
   bool fold = false;
   int fold_Wp = 0, fold_sW = 1;
 };
@@ -582,10 +586,11 @@ int slab_min_stages(bool pair, int tps) { return tps >= 9 || (pair && tps >= 3) 
 SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, int Eh, int Ew, bool tma_layout_ok, SlabMode mode) {
   const bool spread = mode == kSlabSpread, pair = mode == kSlabPair;
   SlabTile& memo = c->slab_tiles[GeoKey{kGeoSlab, a.dtype, a.n_out, a.Cin_g, a.groups, a.N, Wt, Ht, ntaps, Eh, Ew, tma_layout_ok ? 1 : 0,
-                                        c->epi.pool, c->num_sms, mode}];
+                                        c->epi.pool, c->num_sms, mode, (int)a.classes.size()}];
   if (memo.bn) return memo;
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
-  const int bn_max = conv_umma_bn(a.n_out);
+  const int ncls = std::max<int>(1, a.classes.size());
+  const int bn_max = std::min(conv_umma_bn(a.n_out), 512 / (ncls == 3 ? 4 : ncls));
   const long long kblocks_n = cdiv(a.Cin_g, kBK);
   const long long es_out = (long long)elem_size(a.dtype);
   long long best_cost = -1, best_work = 0, best_tiles = 0;
@@ -595,7 +600,7 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
   const int units = pair ? c->num_sms / 2 : c->num_sms;
   for (int BN = bn_max; BN >= (spread ? 32 : pair ? std::max(64, bn_max / 2) : bn_max); BN /= 2) {
     const int tiles_co = (int)cdiv(a.n_out, BN);
-    const int acc_cap = std::min(512 / BN, 4);
+    const int acc_cap = std::min(512 / (BN * ncls), 4);
     const int tps = slab_tps(BN, ntaps, pair);
     const int b_bytes = tps * (pair ? BN / 2 : BN) * 128;
     const long long stages = kblocks_n * cdiv(ntaps, tps);
@@ -614,20 +619,21 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
       const int ngr = n_acc == 3 ? 0 : 4 / n_acc;
       const long long stg = (dense_rows * 128 + 1023) / 1024 * 1024;
       const long long min_b = std::min<long long>(slab_min_stages(pair, tps), stages + 1);   // filter stages the staged epilogue insists on
+      if (ncls > 1 && (n_acc > acc_cap || n_acc == 3)) return;
       if (c->epi.pool && ((wt | th) & 1)) return;          // pooling windows must not straddle tiles
       const bool tma_fit = tma_layout_ok && ngr > 0 && BN * es_out >= 128 && ngr * stg <= kSlabStageBytes &&
                            (total <= units ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
                                                 : 2 * slab_bytes + min_b * b_bytes + kSlabStageBytes <= kSlabSmemBudget);
       // plus about 1500 clocks per tile for the pipeline to fill again
-      const int mma_clk = pair && n_acc == 1 && BN <= 128 ? 96 : mma_clocks(BN);
+      const int mma_clk = pair && n_acc * ncls == 1 && BN <= 128 ? 96 : mma_clocks(BN);
       auto mma_part = [&](long long st) { return st * (1LL * std::min(tps, ntaps) * 4 * n_acc * mma_clk + 120) + 1500; };
       const long long whole = 1LL * kblocks_n * (ntaps * 4LL * n_acc * mma_clk + cdiv(ntaps, tps) * 120) + 1500;
-      const long long epi_part = tma_fit ? 2500 + dense_rows * BN * es_out / 32 : 2400LL * n_acc * (BN / 32);
-      const long long per_tile = 2 * n_acc * BN <= 512 ? std::max(whole, epi_part) : whole + epi_part;
+      const long long epi_part = tma_fit ? 2500 + ncls * dense_rows * BN * es_out / 32 : 2400LL * n_acc * (BN / 32);
+      const long long per_tile = 2 * n_acc * ncls * BN <= 512 ? std::max(whole, epi_part) : whole + epi_part;
       long long cost = cdiv(total, units) * per_tile;
       if (spread) cost += std::min(whole, epi_part);      // the last tile's read-out runs beside nothing (a few tiles per SM only)
       int splits = 1;
-      const bool unsplit_ok = !c->epi.pool || tma_fit;     // unsplit, pooling happens in the staged epilogue only
+      const bool unsplit_ok = (!c->epi.pool && ncls == 1) || tma_fit;     // unsplit, pooling happens in the staged epilogue only
       if (spread && 2 * total <= c->num_sms)
         for (int s = 2; s <= std::min(stages, c->num_sms / total); ++s) {
           const long long cs = mma_part(cdiv(stages, s)) + split_clocks(total * s, 128 * n_acc, BN, c->num_sms);
@@ -665,7 +671,7 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
         }
       }
     }
-    if (Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && !c->epi.pool) {
+    if (Eh == 0 && Ew == 0 && Ht == 1 && a.N == 1 && Wt > 256 && !c->epi.pool && ncls == 1) {
       // one long row of pixels without halo (a flattened 1x1 layer): whole 128-pixel accumulators,
       // as many as still leave room for a second accumulator set
       if (spread || pair) {
@@ -798,6 +804,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.dw_min = dw_min; p.dh_min = dh_min;
   p.slab_bytes = b_slab;
   p.splits = tile.splits;
+  p.ncls = std::max<int>(1, a.classes.size());
   p.pair = pair;
   p.tps = tps;
   // Ring depths for `avail` bytes.  Activations come from HBM (the longer latency, and the stream
@@ -859,21 +866,27 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       }
     }
     if (c->epi.pool && !ok) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+    if (p.ncls > 1 && !ok) return 2;
     if (ok) {
       const int pl = c->epi.pool ? 2 : 1;       // pooled output: half the rows and columns (strides are the pooled tensor's)
-      cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)(Wt / pl), (cuuint64_t)(Ht / pl), (cuuint64_t)a.N};
       cuuint64_t strides[3] = {(cuuint64_t)(sw * es), (cuuint64_t)(sh * es), (cuuint64_t)(sn * es)};
       cuuint32_t box[4] = {(cuuint32_t)row_ch, (cuuint32_t)(p.wt / pl), (cuuint32_t)(p.th / pl), (cuuint32_t)p.nb};
       cuuint32_t estr[4] = {1, 1, 1, 1};
-      CUresult r = c->encode(&p.out_map, a.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                             4, const_cast<char*>(obase), dims, strides,
-                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      CUresult r = CUDA_SUCCESS;
+      for (int q = 0; q < p.ncls && r == CUDA_SUCCESS; ++q) {
+        const FwdLikeArgs::Class k = a.classes.empty() ? FwdLikeArgs::Class{Wt, Ht, 0} : a.classes[q];
+        cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)(k.W / pl), (cuuint64_t)(k.H / pl), (cuuint64_t)a.N};
+        p.cls_W[q] = k.W; p.cls_H[q] = k.H;
+        r = c->encode(&p.out_map[q], a.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                      4, const_cast<char*>(obase) + k.off * (long long)es, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      }
       if (r == CUDA_SUCCESS) {
         p.tma_out = 1;
         p.stage_bytes = stage_bytes;
       } else {
         if (c->epi.pool) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+        if (p.ncls > 1) return 2;
         plan_rings(kSlabSmemBudget, &p.s_stages, &p.b_stages);
         p.stage_off = p.stage_reserved = 0;
       }
@@ -890,6 +903,10 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   for (const ConvTap& t : taps) {
     p.tap_shift[p.ntaps] = (int16_t)((t.dh - dh_min) * p.Ws + (t.dw - dw_min));
     p.tap_wmat[p.ntaps] = t.wmat;
+    if (p.ncls > 1) {
+      p.tap_cls[p.ntaps] = a.tap_cls[p.ntaps];
+      p.tap_first[p.ntaps] = std::find(a.tap_cls.begin(), a.tap_cls.begin() + p.ntaps, a.tap_cls[p.ntaps]) == a.tap_cls.begin() + p.ntaps;
+    }
     ++p.ntaps;
   }
   p.kblocks = (int)cdiv(a.Cin_g, kBK);
@@ -1546,19 +1563,76 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
   a.n_out = out_nhwc && d.groups == 1 ? Cp : Cg; a.w_rows = Cg; a.groups = d.groups; a.N = d.N; a.dtype = d.dtype;
   a.view_sH = 1; a.view_sW = 1;
   std::vector<std::pair<int, int>> parity(1, {0, 0});
-  for (const Cls& k : classes) {
-    if (k.taps.empty()) continue;
-    long long sn, sc, sh, sw, off;
-    if (out_nhwc) {
-      sn = 1LL * d.H * d.W * Cp; sc = 1; sh = 1LL * d.sH * d.W * Cp; sw = 1LL * d.sW * Cp;
-      off = (1LL * k.h0 * d.W + k.w0) * Cp;
-    } else {
-      sn = 1LL * d.C * d.H * d.W; sc = 1LL * d.H * d.W; sh = 1LL * d.sH * d.W; sw = d.sW;
-      off = 1LL * k.h0 * d.W + k.w0;
+  const bool slab_ok = !(flags & B200CONV_NO_SLAB);
+  auto each_class = [&]() -> int {
+    for (const Cls& k : classes) {
+      if (k.taps.empty()) continue;
+      long long sn, sc, sh, sw, off;
+      if (out_nhwc) {
+        sn = 1LL * d.H * d.W * Cp; sc = 1; sh = 1LL * d.sH * d.W * Cp; sw = 1LL * d.sW * Cp;
+        off = (1LL * k.h0 * d.W + k.w0) * Cp;
+      } else {
+        sn = 1LL * d.C * d.H * d.W; sc = 1LL * d.H * d.W; sh = 1LL * d.sH * d.W; sw = d.sW;
+        off = 1LL * k.h0 * d.W + k.w0;
+      }
+      const int r = run_conv_umma(c, a, k.taps, parity, k.Wt, k.Ht, dx, sn, sc, sh, sw, off, nullptr, 0, slab_ok);
+      if (r) return r == 1 ? fail(c, B200CONV_E_CUDA, "internal: empty gradient view") : r;
     }
-    rc = run_conv_umma(c, a, k.taps, parity, k.Wt, k.Ht, dx, sn, sc, sh, sw, off, nullptr, 0,
-                       !(flags & B200CONV_NO_SLAB));
-    if (rc) return rc == 1 ? fail(c, B200CONV_E_CUDA, "internal: empty gradient view") : rc;
+    return 0;
+  };
+  // All classes from one slab of dy: one launch that reads dy once, its taps grouped by class into accumulators of their
+  // own.  Class by class, dy is read ncls times and a class with one tap is a launch that only moves memory
+  // (256 images at 56x56 with the packing: 64 <- 128 channels float32 186 -> 134 us, 64 <- 64 float16 96 -> 57; from 128 channels
+  // on in float16 both forms are bound by their MMAs and equal).
+  const bool full = std::all_of(classes.begin(), classes.end(), [](const Cls& k) { return !k.taps.empty(); });
+  if (ncls > 1 && ncls <= kMaxSlabClasses && (int)classes.size() == ncls && full && out_nhwc && slab_ok &&
+      !(flags & B200CONV_NO_MERGE_PARITY) && d.kH * d.kW <= kMaxTaps) {
+    FwdLikeArgs m = a;
+    std::vector<std::pair<ConvTap, int>> all;
+    int Wt = 0, Ht = 0;
+    for (const Cls& k : classes) {
+      for (const ConvTap& t : k.taps) all.push_back({t, (int)m.classes.size()});
+      m.classes.push_back({k.Wt, k.Ht, (1LL * k.h0 * d.W + k.w0) * Cp});
+      Wt = std::max(Wt, k.Wt); Ht = std::max(Ht, k.Ht);
+    }
+    // in the order of the packed filters, so that a stage's taps arrive as one box
+    std::sort(all.begin(), all.end(), [](const auto& x, const auto& y) { return x.first.wmat < y.first.wmat; });
+    std::vector<ConvTap> taps;
+    for (auto& t : all) { taps.push_back(t.first); m.tap_cls.push_back((uint8_t)t.second); }
+    auto together = [&](SlabMode mode) {
+      return try_conv_slab(c, m, taps, 0, 0, Wt, Ht, dx, 1LL * d.H * d.W * Cp, 1, 1LL * d.sH * d.W * Cp, 1LL * d.sW * Cp, 0, nullptr, 0, mode);
+    };
+    // 0: class by class, 1 / 2: together, on single CTAs / on pairs; timed like the other variants
+    auto run = [&](int v) { return v == 0 ? each_class() : together(v == 1 ? kSlabWide : kSlabPair); };
+    GeoKey key{kGeoClasses, d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.Ho, d.Wo, d.groups,
+               c->use_pair ? 1 : 0};
+    auto it = c->autotune ? c->algo_cache.find(key) : c->algo_cache.end();
+    int choice = it != c->algo_cache.end() ? it->second : -1;
+    if (choice < 0 && (!c->autotune || c->capturing)) {
+      if ((rc = together(c->use_pair ? kSlabPair : kSlabWide)) == 2 && c->use_pair) rc = together(kSlabWide);
+      if (rc != 2) {
+        if (rc) return rc;
+        c->last_algo = "umma";
+        return 0;
+      }
+      choice = 0;
+    }
+    if (choice < 0) {
+      float best = 0.f;
+      for (int v = 0; v <= (c->use_pair ? 2 : 1); ++v) {
+        float ms;
+        rc = time_variant(c, [&] { return run(v); }, &ms);
+        if (rc == 2) continue;
+        if (rc) return rc;
+        if (choice < 0 || ms < best) { choice = v; best = ms; }
+      }
+      c->algo_cache[key] = choice;
+    }
+    rc = run(choice);
+    if (rc == 2) rc = each_class();          // a choice remembered for another alignment
+    if (rc) return rc;
+  } else if ((rc = each_class())) {
+    return rc;
   }
   c->last_algo = "umma";
   return 0;
@@ -2988,7 +3062,7 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
     GeoKey key{};
     if (sscanf(line, "%c %399s %d", &kind, text, &val) != 3 || !GeoKey::parse(text, &key)) continue;
     // keys of another form (older files) are passed over
-    const bool known = kind == 'a' ? (key.v[0] == kGeoConv && key.n == 17) || (key.v[0] == kGeoWgrad && key.n == 19)
+    const bool known = kind == 'a' ? (key.v[0] == kGeoConv && key.n == 17) || ((key.v[0] == kGeoWgrad || key.v[0] == kGeoClasses) && key.n == 19)
                                    : key.v[0] == kGeoSplits && key.n == 20;
     if (!known) continue;
     if (kind == 'a' && val >= 0 && val < kConvVariants) { c->algo_cache[key] = val; ++n; }

@@ -88,7 +88,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     return Range{static_cast<int>(a / stages_kb), static_cast<int>(b / stages_kb), static_cast<int>(a % stages_kb), static_cast<int>(b % stages_kb)};
   };
   const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
-  const bool dbl = 2 * p.n_acc * BN <= 512;
+  const int ncls = p.ncls;                              // accumulator (a, class q): columns (a * ncls + q) * BN
+  const bool dbl = 2 * p.n_acc * ncls * BN <= 512;
   const int issuers = p.n_acc >= 2 ? 2 : 1;
 
   if (threadIdx.x == 0) {
@@ -224,7 +225,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         // runs beside the MMAs of the next one
         const int buf = dbl ? (it & 1) : 0;
         const uint32_t aphase = dbl ? ((it >> 1) & 1) : (it & 1);
-        const uint32_t acc_base = tmem + buf * (p.n_acc * BN);
+        const uint32_t acc_base = tmem + buf * (p.n_acc * ncls * BN);
         long long tq = trace ? clock64() : 0;
         if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (trace) tw_acc += clock64() - tq;
@@ -248,12 +249,14 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
                 const int tap = tap0 + q;
                 // only the address field of the two descriptors changes from MMA to MMA
                 const uint32_t b_lo = desc_lo + (smem_u32(bring + bs * stage_b + q * kBBytes) >> 4);
-                const uint32_t first = kb != r.kb0 || tap != tap_begin;      // 0 for the slice's first products
+                // 0 for the first products of the slice, or of the tap's class
+                const uint32_t first = kb != r.kb0 || (ncls > 1 ? p.tap_first[tap] == 0 : tap != tap_begin);
+                const uint32_t acc_cls = acc_base + (ncls > 1 ? p.tap_cls[tap] * BN : 0);
                 uint32_t a_lo = desc_lo + ((sbase + static_cast<uint32_t>(p.tap_shift[tap] + 128 * a_begin) * 128u) >> 4);
                 for (int a = a_begin; a < a_end; ++a) {
 #pragma unroll
                   for (int kk = 0; kk < 4; ++kk)
-                    umma_words<KIND, PAIR>(acc_base + a * BN, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, first | (kk != 0));
+                    umma_words<KIND, PAIR>(acc_cls + a * (ncls * BN), a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, first | (kk != 0));
                   a_lo += (128 * 128) >> 4;      // next accumulator: 128 slab rows further
                 }
               }
@@ -305,7 +308,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       if (trace && it == 0 && threadIdx.x == 64) trace[4] = clock64();
       const int co_base = co_t * BN;
       const int nchunks = min(BN / 32, (p.n_out - co_base + 31) / 32);
-      const uint32_t lane_base = tmem + buf * (p.n_acc * BN) + (static_cast<uint32_t>(quad * 32) << 16);
+      const uint32_t lane_base = tmem + buf * (p.n_acc * ncls * BN) + (static_cast<uint32_t>(quad * 32) << 16);
 
       if (splits > 1) {
         // raw accumulators; conv_reduce.cu adds the slices and applies the epilogue
@@ -345,7 +348,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         const int bufs = p.stage_nbuf / ngrp >= 2 ? 2 : 1;
         constexpr int kCh = 128 / static_cast<int>(sizeof(OutT));   // channels of one 128-byte staged row
         const int nstaged = min(BN / kCh, (p.n_out - co_base + kCh - 1) / kCh);
-        for (int ch = grp; ch < nstaged; ch += ngrp, ++nstore) {
+        for (int cc = grp; cc < nstaged * ncls; cc += ngrp, ++nstore) {
+          const int cls = ncls > 1 ? cc / nstaged : 0, ch = cc - cls * nstaged;
           uint8_t* stg = smem + p.stage_off + (grp * bufs + (bufs == 2 ? (nstore & 1) : 0)) * p.stage_bytes;
           uint8_t* srow = stg + drow * 128;
           const int co0 = co_base + ch * kCh;
@@ -362,7 +366,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
 #pragma unroll
           for (int part = 0; part < kCh / 32; ++part) {
             uint32_t r[32];
-            tmem_ld32(lane_base + a * BN + ch * kCh + part * 32, r);
+            tmem_ld32(lane_base + (a * ncls + cls) * BN + ch * kCh + part * 32, r);
             tmem_ld_wait();
             if (trace) { const long long t = clock64(); tp[1] += t - tq; tq = t; }
             if (!inbox) continue;
@@ -473,10 +477,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           if (trace) { const long long t = clock64(); tp[3] += t - tq; tq = t; }
           // a tiled store must not start at a negative coordinate, and its staging rows must lie
           // inside the reserved shared memory
-          if (issuer && (!PAIR || n0 < p.Nimg) && B200_IN_RANGE(g * p.n_out + co0 >= 0 && w0 >= 0 && h0 >= 0 && n0 >= 0 && w0 < p.Wt && h0 < p.Ht &&
+          if (issuer && (!PAIR || n0 < p.Nimg) && (ncls == 1 || (w0 < p.cls_W[cls] && h0 < p.cls_H[cls])) &&
+              B200_IN_RANGE(g * p.n_out + co0 >= 0 && w0 >= 0 && h0 >= 0 && n0 >= 0 && w0 < p.Wt && h0 < p.Ht &&
                                       n0 < p.Nimg && ch * kCh + kCh <= BN, p.status)) {
-            if (p.epi.pool) tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0 >> 1, h0 >> 1, n0);
-            else tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0, h0, n0);
+            if (p.epi.pool) tma_store_4d(&p.out_map[0], stg, g * p.n_out + co0, w0 >> 1, h0 >> 1, n0);
+            else tma_store_4d(&p.out_map[cls], stg, g * p.n_out + co0, w0, h0, n0);
             bulk_commit();
           }
         }
@@ -594,6 +599,7 @@ cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num
   const long long pix = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
   const long long total = (p.pair ? (pix + 1) / 2 : pix) * p.groups * p.tiles_co * p.splits;
   if (total == 0 || p.ntaps == 0) return cudaSuccess;
+  if (p.ncls < 1 || p.ncls > kMaxSlabClasses || (p.ncls > 1 && (p.splits != 1 || !p.tma_out || p.epi.pool))) return cudaErrorInvalidValue;
   if (total >= (1LL << 31) || (p.pair && (p.splits != 1 || num_sms < 2))) return cudaErrorInvalidValue;
   const bool f16 = dtype == B200CONV_F16;
 #define B200_CASE(BNV)                                                                  \

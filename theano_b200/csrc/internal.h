@@ -134,11 +134,18 @@ cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cu
 // ---- implicit GEMM with one activation slab per channel block (conv_slab.cu) ---------------
 // For launches whose taps all read the same view: the slab (output tile plus halo) is loaded
 // once per channel block and every tap is a row offset into it.
+constexpr int kMaxSlabClasses = 4;
 struct alignas(64) SlabConvParams {
   CUtensorMap view;              // 5-D (c_in_group, group, w, h, n), box (kBK, 1, Ws, Hs, nb)
   CUtensorMap wmap;              // 4-D packed filters (k_red, n_out, group, tap), box (kBK, BN or half of it, 1, 1 or tps)
   int16_t tap_shift[kMaxTaps];   // row offset of the tap inside the slab
   int16_t tap_wmat[kMaxTaps];
+  // Output classes: the taps of class q add up in accumulators of their own, and the class has its own output tensor
+  // (strided gradInputs: the stride's parity classes of dx, all from one slab of dy).  1: one output, no classes.
+  int ncls;
+  uint8_t tap_cls[kMaxTaps];     // class of the tap
+  uint8_t tap_first[kMaxTaps];   // 1: first tap of its class
+  int cls_W[kMaxSlabClasses], cls_H[kMaxSlabClasses];    // output grid of the class (at most Wt x Ht)
   int ntaps;
   int kblocks;
   int groups;
@@ -170,7 +177,7 @@ struct alignas(64) SlabConvParams {
   // Channels-last outputs are written by TMA: the epilogue warps put 128-byte channel chunks (32
   // float32 / 64 float16) of the tile into shared memory (rows = the tile's pixels, dense) and one
   // thread per chunk stores the box (chunk, wt, th, nb) through out_map.
-  CUtensorMap out_map;           // 4-D (channel, w, h, n) over the output view
+  CUtensorMap out_map[kMaxSlabClasses];      // 4-D (channel, w, h, n) over the output view of each class
   int tma_out;                   // 1: epilogue through out_map, 0: direct stores
   int stage_off;                 // byte offset of the staging buffers in dynamic shared memory
   int stage_reserved;            // bytes set aside for them behind the filter ring (0: they reuse the
