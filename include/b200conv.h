@@ -267,11 +267,12 @@ int b200conv_kernel_time(b200conv_ctx* ctx, const char* family, float* total_ms,
  * context remembers the faster one; with enable = 0 the first is always used where it applies
  * (B200CONV_NO_SLAB still forces the second). */
 int b200conv_set_autotune(b200conv_ctx* ctx, int enable);
-/* 1x1 layers (float16, channels-last, at least 256 channels, filters in whole 64-blocks) run on pairs of
- * CTAs that share the filter tile (tcgen05 cta_group::2); enable = 0 keeps them on the one-CTA kernel
- * (the cross-check of the parity tests). */
+/* 1x1 layers (float16, channels-last, at least 256 channels, filters in whole 64-blocks), and forward and gradInputs
+ * of other layers with more than 32 filters where pairs occupy half of the SMs and timing (or, without it, the static
+ * choice) prefers them, run on pairs of CTAs that share the filter tile (tcgen05 cta_group::2); enable = 0 keeps them
+ * on the one-CTA kernels (the cross-check of the parity tests). */
 int b200conv_set_pair_kernels(b200conv_ctx* ctx, int enable);
-/* gradWeights of float16 layers with at most 64 channels per group computes the taps of a filter row as column
+/* gradWeights of layers with at most 64 channels per group computes the taps of a filter row as column
  * groups of one MMA (the operand descriptor's leading-dimension offset is the taps' spacing) instead of one
  * half-empty MMA per tap; enable = 0 keeps one MMA per tap (the cross-check of the parity tests). */
 int b200conv_set_stacked_taps(b200conv_ctx* ctx, int enable);

@@ -247,11 +247,11 @@ class Context(object):
         self.check(self.lib.b200conv_set_autotune(self.h, int(bool(enable))))
 
     def set_pair_kernels(self, enable):
-        """1x1 layers with deep reductions on CTA pairs (default on); off: the one-CTA kernel."""
+        """Layers with wide filter tiles on CTA pairs (default on); off: the one-CTA kernels."""
         self.check(self.lib.b200conv_set_pair_kernels(self.h, int(bool(enable))))
 
     def set_stacked_taps(self, enable):
-        """gradWeights of narrow float16 layers: taps of a filter row as column groups of one MMA (default on)."""
+        """gradWeights of narrow layers: taps of a filter row as column groups of one MMA (default on)."""
         self.check(self.lib.b200conv_set_stacked_taps(self.h, int(bool(enable))))
 
     def set_splits(self, n):
