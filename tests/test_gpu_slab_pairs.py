@@ -66,3 +66,19 @@ def test_pairs_pool_in_the_epilogue(dtype, n):
     want = O.maxpool2x2(np.maximum(O.conv2d(x.astype(f), w.astype(f), border_mode="half", subsample=(1, 1)), 0))
     assert O.rel_err(got[0], want) < TOL[dtype] and O.rel_err(got[0], got[1]) < TOL[dtype] / 4
     ctx.close()
+
+
+def test_switching_pairs_off_holds_for_geometries_timed_before(tmp_path):
+    ctx = shim.Context(0)
+    X = T.from_host(ctx, np.ones((40, 512, 14, 14), np.float32), "nhwc")
+    W = T.from_host(ctx, np.ones((512, 512, 3, 3), np.float32))
+
+    def choices():
+        shim.device_conv2d(X, W, border_mode="half")
+        ctx.tuning_save(str(tmp_path / "t"))
+        return [l.split() for l in open(str(tmp_path / "t")) if l.startswith("a ")]
+    on = choices()
+    ctx.set_pair_kernels(False)
+    off = [c for c in choices() if c not in on]
+    assert len(on) == 1 and len(off) == 1 and off[0][2] != "4"           # a choice of its own, and not the pairs
+    ctx.close()

@@ -1065,7 +1065,7 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   GeoKey key{kGeoConv, a.dtype, a.N, a.Hs, a.Ws, a.Cin_g, a.n_out, a.groups, Wt, Ht, a.view_sH, a.view_sW, (int)taps_in.size(), tsum};
   key.add(sc);
   key.add(sw);
-  key.add(c->epi.pool * 2 + (allow_slab ? 1 : 0));
+  key.add(c->epi.pool * 4 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
   if (c->autotune) {
     auto it = c->algo_cache.find(key);
     if (it != c->algo_cache.end()) return run(it->second);
