@@ -470,24 +470,6 @@ int make_wmap(b200conv_ctx* c, CUtensorMap* m, const void* base, int dtype, int 
   return 0;
 }
 
-bool fits16(int v) { return v >= -32768 && v <= 32767; }
-
-// Can the tensor-core kernels take this geometry?  (Otherwise the direct kernels do.)
-bool umma_ok(const b200conv_desc& d) {
-  const int Cg = d.C / d.groups, Kg = d.K / d.groups;
-  const size_t es = elem_size(d.dtype);
-  if (d.N == 0 || d.C == 0 || d.K == 0) return false;
-  if (d.kH * d.kW > kMaxTaps) return false;
-  if (d.sH * d.sW > kMaxViews) return false;
-  if (d.groups > 1 && ((Cg * es) % 16 || (Kg * es) % 16)) return false;
-  if (Cg * es < 16 && d.groups > 1) return false;
-  // tap offsets travel as 16-bit numbers; pixel coordinates as 32-bit ones
-  const int reach_h = (d.kH - 1) * d.dilH + d.padH_l, reach_w = (d.kW - 1) * d.dilW + d.padW_l;
-  if (!fits16(reach_h) || !fits16(reach_w)) return false;
-  if (1LL * d.H + reach_h > (1 << 30) || 1LL * d.W + reach_w > (1 << 30)) return false;
-  return true;
-}
-
 // ---- forward-type launch shared by fwd and dgrad ------------------------------------------
 struct FwdLikeArgs {
   const void* act;       // channels-last activations [N][Hs][Ws][Cp_in]
@@ -1128,31 +1110,6 @@ int to_nhwc(b200conv_ctx* c, Scratch& tmp, const void* src, int N, int C, int H,
   return 0;
 }
 
-// Grouped layers with fewer channels per group than one reduction block: how many neighbouring
-// groups to merge into one (block-diagonal filters); 1 = leave as is.
-int merge_factor(const b200conv_desc& d) {
-  if (d.groups <= 1 || d.C == 0 || d.K == 0) return 1;
-  const int kBK = d.dtype == B200CONV_F16 ? 64 : 32;
-  const int Cg = d.C / d.groups, Kg = d.K / d.groups;
-  int best = 1;
-  for (int m = 2; m <= d.groups && Cg * m <= kBK && Kg * m <= 256; ++m)
-    if (d.groups % m == 0) best = m;
-  return best;
-}
-
-// The same for gradWeights, whose MMAs are 128 filters x channels: merging until both fill 128 leaves fewer,
-// fuller MMAs and reads each operand row once instead of in 32-channel pieces (the off-diagonal blocks cost
-// nothing extra: they fill rows and columns that would be empty).  32 groups of 8 -> 8 channels, 256 images of
-// 28 x 28, float32: 590 us at one reduction block per group, 190 us at 128 channels.
-int merge_factor_wgrad(const b200conv_desc& d) {
-  if (d.groups <= 1 || d.C == 0 || d.K == 0) return 1;
-  const int Cg = d.C / d.groups, Kg = d.K / d.groups;
-  int best = 1;
-  for (int m = 2; m <= d.groups && Cg * m <= 128 && Kg * m <= 128; ++m)
-    if (d.groups % m == 0) best = m;
-  return best;
-}
-
 // Row folding applies to ungrouped layers whose whole filter row (kW pixels x padded channels)
 // fits one reduction block of the MMA: the 3-channel stems of VGG and ResNet.
 bool fold_ok(const b200conv_desc& d) {
@@ -1216,7 +1173,6 @@ void* packed_lookup(b200conv_ctx* c, const void* w, int K, int Cg, int kH, int k
 // (mode 1) path of a geometry performs; false when that path packs nothing or is not taken.
 bool fold_ok(const b200conv_desc& d);
 bool s2d_ok(const b200conv_desc& d, int* t0, int* ntaps, int* q0);
-int merge_factor(const b200conv_desc& d);
 bool plain_pack(const b200conv_desc& d, int mode, int* ldc) {
   if (!umma_ok(d) || merge_factor(d) > 1) return false;
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;

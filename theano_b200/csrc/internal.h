@@ -8,6 +8,7 @@
 #include <atomic>
 
 #include "../../include/b200conv.h"
+#include "geometry.h"
 
 namespace b200 {
 
@@ -73,13 +74,6 @@ cudaError_t launch_streaming(void (*kernel)(Exp...), dim3 grid, dim3 block, size
 // Codes a kernel writes to the device status word when it gives up.
 enum : int { kStatusOk = 0, kStatusTimeout = 1, kStatusBadIndex = 2 };
 
-inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
-inline long long cdiv(long long a, long long b) { return (a + b - 1) / b; }
-inline size_t elem_size(int dtype) { return dtype == B200CONV_F16 ? 2 : 4; }
-// Channels-last tensors pad the channel count so that one pixel is a multiple of 16 bytes
-// (tensor-map strides must be).
-inline int pad_channels(int c, int dtype) { return round_up(c < 1 ? 1 : c, dtype == B200CONV_F16 ? 8 : 4); }
-
 // ---- implicit-GEMM convolution (conv_umma.cu) -----------------------------------------
 // One "tap" of the reduction: a spatial offset into one activation view and the filter
 // slice that multiplies it.
@@ -88,8 +82,6 @@ struct ConvTap {
   int16_t view;     // which activation tensor map
   int16_t wmat;     // which packed filter matrix
 };
-constexpr int kMaxTaps = 64;
-constexpr int kMaxViews = 9;
 
 // Forward epilogue: y = act(alpha * conv + bias + beta * residual); with `relu` set
 // act(v) = lin * v + abs * |v|  (ReLU: 0.5, 0.5; leaky ReLU of slope s: 0.5 * (1 + s), 0.5 * (1 - s),
