@@ -114,7 +114,8 @@ int b200conv_fwd(b200conv_ctx* ctx, const b200conv_desc* d, const void* x, const
  * act = identity without B200CONV_RELU, else leaky ReLU of that slope in the reference's form
  * 0.5 * ((1 + slope) * v + (1 - slope) * |v|) (theano/tensor/nnet/nnet.py:2242-2250); slope 0 = ReLU.
  * bias and residual may be NULL; residual has the shape and layout of y (host NCHW with HOST_PTRS,
- * channels-last with OUT_NHWC).  b200conv_fwd == this call with alpha 1, no residual, slope 0. */
+ * channels-last with OUT_NHWC) and may be y itself, which is then accumulated in place.
+ * b200conv_fwd == this call with alpha 1, no residual, slope 0. */
 int b200conv_fwd_epilogue(b200conv_ctx* ctx, const b200conv_desc* d, const void* x, const void* w,
                           const void* bias, const void* residual, void* y, float alpha, float beta,
                           float slope, int flags);

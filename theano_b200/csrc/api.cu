@@ -528,6 +528,11 @@ long long out_extent(const FwdLikeArgs& a, int Wt, int Ht, long long sn, long lo
   return off + (a.N - 1) * sn + (Ht - 1) * sh + (Wt - 1) * sw + (1LL * a.n_out * a.groups - 1) * sc + 1;
 }
 
+bool overlap(const void* a, size_t na, const void* b, size_t nb) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return x < y + nb && y < x + na;
+}
+
 // Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
 // the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
 // and / or a reduction cut into slices where that occupies more SMs; the slab kernel also on pairs of CTAs.  The
@@ -1083,7 +1088,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     if (pair) cand[ncand++] = kConvSlabPair;
   }
   if (ncand == 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
-  if (!c->autotune || c->capturing || ncand == 1) return run(cand[ncand - 1]);
+  // A launch that adds to its own output (residual == y) must run once: it is not timed, and the choice is left to a
+  // later call that may repeat it.
+  const size_t out_bytes = elem_size(a.dtype) * out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
+  const bool in_place = c->epi.residual && overlap(c->epi.residual, out_bytes, out, out_bytes);
+  if (!c->autotune || c->capturing || ncand == 1 || in_place) return run(cand[ncand - 1]);
   int best = -1;
   float best_ms = 0.f;
   for (int i = 0; i < ncand; ++i) {
