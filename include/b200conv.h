@@ -167,8 +167,8 @@ int b200conv_wgrad_static(b200conv_ctx* ctx, const b200conv_desc* d, const void*
  * kernel.  A training loop calls it once per step after the optimizer has updated the filters (the
  * call can be part of a captured graph: a replay packs whatever the filter buffers then hold).
  * b200conv_filters_changed(w) marks the packed forms of one bank (NULL: of all) stale: calls pack
- * per call again until the next prepack.  Writing to a filter buffer without either call makes
- * later calls use stale filters.  Banks whose geometry has no packed form of this kind (1x1
+ * per call again until the next prepack, and b200conv_free does the same for the banks in its block.
+ * Writing to a filter buffer without one of these calls makes later calls use stale filters.  Banks whose geometry has no packed form of this kind (1x1
  * forward banks are read in place; few-channel stems and merged small groups pack differently)
  * are skipped.  No counterpart in the reference (BLAS reads OIHW as it is).
  */

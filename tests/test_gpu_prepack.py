@@ -67,3 +67,34 @@ def test_prepacked_filters_give_the_same_results_with_fewer_launches(ctx, dtype)
     got = shim.device_conv2d(X, W, **kw).to_host()
     assert O.rel_err(got.astype(np.float32), want) < tol
     ctx.filters_changed()
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32], ids=["float16", "float32"])
+def test_packed_forms_end_with_the_filters_memory(dtype):
+    """A bank that was packed ahead of time is freed; the library gives its block to the next filters of that size,
+    those of a host-pointer call (its own scratch) or of another device tensor."""
+    tol = 2e-2 if dtype == np.float16 else 5e-3
+    rs = np.random.RandomState(6)
+    T = shim.DeviceTensor
+    f = np.float32
+    xs, ws, kw = (2, 64, 9, 9), (128, 64, 3, 3), dict(border_mode="half", subsample=(1, 1))
+    x = rs.standard_normal(xs).astype(dtype)
+    w = [(rs.standard_normal(ws) / 24).astype(dtype) for _ in range(3)]
+    want = [O.conv2d(x.astype(f), v.astype(f), **kw) for v in w]
+    dy = rs.standard_normal(want[0].shape).astype(dtype)
+    own = shim.Context(0)
+    X, W = T.from_host(own, x, "nhwc"), T.from_host(own, w[0])
+    desc, block = shim.layer_desc(xs, ws, dtype=dtype, **kw), W.ptr
+    own.prepack([desc], [block])
+    assert O.rel_err(shim.device_conv2d(X, W, **kw).to_host().astype(f), want[0]) < tol
+    W.free()
+    y = shim.conv2d_forward(x, w[1], ctx=own, **kw)
+    assert O.rel_err(y.astype(f), want[1]) < tol
+    dx = shim.conv2d_grad_inputs(w[1], dy, xs[2:], ctx=own, **kw)
+    assert O.rel_err(dx.astype(f), O.conv2d_grad_inputs(w[1].astype(f), dy.astype(f), xs[2:], **kw)) < tol
+    V = T.from_host(own, w[2])
+    assert V.ptr == block                     # the case this test is about
+    assert O.rel_err(shim.device_conv2d(X, V, **kw).to_host().astype(f), want[2]) < tol
+    own.prepack([desc], [block])              # and the new bank can be packed in its turn
+    assert O.rel_err(shim.device_conv2d(X, V, **kw).to_host().astype(f), want[2]) < tol
+    own.close()

@@ -1172,6 +1172,9 @@ std::string pack_key(const void* w, int K, int Cg, int kH, int kW, int groups, i
 }
 // The packed form of `w` if b200conv_prepack made one and the filters have not been reported
 // changed since; nullptr otherwise (the caller then packs into scratch memory as usual).
+// kScratchFilters among the flags of a direction: `w` is scratch of this call (filters uploaded from the host, merged
+// groups), whose address may be that of a bank that was packed ahead of time and has gone since.
+constexpr int kScratchFilters = 1 << 30;
 void* packed_lookup(b200conv_ctx* c, const void* w, int K, int Cg, int kH, int kW, int groups, int flip, int mode,
                     int ldc, int dtype) {
   if (c->packed.empty()) return nullptr;
@@ -1244,7 +1247,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
       int rc = tmp.get(es * (size_t)d.K * Cg * mg * d.kH * d.kW, &wm);
       if (rc) return rc;
       KLAUNCH(c, kKPack, launch_merge_groups(w, wm, d.K, Cg, Kg, mg, d.kH * d.kW, 0, d.dtype, c->stream));
-      return fwd_device(c, dm, x, wm, bias, y, flags);
+      return fwd_device(c, dm, x, wm, bias, y, flags | kScratchFilters);
     }
   }
   const bool use_umma = !(flags & B200CONV_FORCE_DIRECT) && umma_ok(d);
@@ -1351,7 +1354,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     // a 1x1 filter bank [K][C] already is its packed form (rows = filters, channels contiguous)
     wp = const_cast<void*>(w);
   } else {
-    wp = packed_lookup(c, w, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 0, ldw, d.dtype);
+    wp = flags & kScratchFilters ? nullptr : packed_lookup(c, w, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 0, ldw, d.dtype);
     if (!wp) {
       rc = tmp.get(es * (size_t)d.kH * d.kW * d.K * ldw, &wp);
       if (rc) return rc;
@@ -1421,7 +1424,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       int rc = tm.get(es * (size_t)d.K * Cg * mg * d.kH * d.kW, &wm);
       if (rc) return rc;
       KLAUNCH(c, kKPack, launch_merge_groups(w, wm, d.K, Cg, Kg, mg, d.kH * d.kW, 0, d.dtype, c->stream));
-      return dgrad_device(c, dm, wm, dy, dx, flags);
+      return dgrad_device(c, dm, wm, dy, dx, flags | kScratchFilters);
     }
   }
   const bool use_umma = !(flags & B200CONV_FORCE_DIRECT) && umma_ok(d);
@@ -1516,7 +1519,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       return 0;
     }
   }
-  void* wp = packed_lookup(c, w, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 1, ldw, d.dtype);
+  void* wp = flags & kScratchFilters ? nullptr : packed_lookup(c, w, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 1, ldw, d.dtype);
   if (!wp) {
     if ((rc = tmp.get(es * (size_t)d.kH * d.kW * d.C * ldw, &wp))) return rc;
     KLAUNCH(c, kKPack, launch_pack_filters(w, wp, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 1, ldw, d.dtype, c->stream));
@@ -2513,7 +2516,7 @@ static int fwd_call(b200conv_ctx* c, const b200conv_desc* d, const void* x, cons
     epi.residual = res;
     if (res && images) res += ny / d->N * images;
     EpilogueScope scope(c, epi);
-    return fwd_device(c, part, xin, dw_, db_, yout, flags & ~B200CONV_HOST_PTRS);
+    return fwd_device(c, part, xin, dw_, db_, yout, (flags & ~B200CONV_HOST_PTRS) | kScratchFilters);
   });
   if (rc) return rc;
   return sync_and_check(c);
@@ -2555,7 +2558,7 @@ int b200conv_dgrad(b200conv_ctx* c, const b200conv_desc* d, const void* w, const
   rc = run_batch(c, io, d->N, dy, ny, dx, nx, [&](int images, const void* dyin, void* dxout) {
     b200conv_desc part = *d;
     part.N = images;
-    return dgrad_device(c, part, dw_, dyin, dxout, flags & ~B200CONV_HOST_PTRS);
+    return dgrad_device(c, part, dw_, dyin, dxout, (flags & ~B200CONV_HOST_PTRS) | kScratchFilters);
   });
   if (rc) return rc;
   return sync_and_check(c);
@@ -2680,6 +2683,13 @@ int b200conv_malloc(b200conv_ctx* c, size_t bytes, void** dptr) {
 int b200conv_free(b200conv_ctx* c, void* dptr) {
   if (!c) return B200CONV_E_INVALID;
   std::lock_guard<std::mutex> g(c->mu);
+  // the block's next user is not the filter bank that was packed from it
+  auto it = c->live.find(dptr);
+  if (it != c->live.end()) {
+    const char *lo = static_cast<const char*>(dptr), *hi = lo + it->second;
+    for (auto& kv : c->packed)
+      if (kv.second.src >= lo && kv.second.src < hi) kv.second.valid = false;
+  }
   return pool_free(c, dptr);
 }
 int b200conv_host_alloc(b200conv_ctx* c, size_t bytes, void** hptr) {
