@@ -146,3 +146,47 @@ def test_grad_weights_of_merged_groups(ctx, dtype, c, k, g):
     dw = shim.device_grad_weights(T.from_host(ctx, x, "nhwc"), T.from_host(ctx, dy, "nhwc"), (3, 3), **kw).to_host()
     f = np.float32
     assert O.rel_err(dw.astype(f), O.conv2d_grad_weights(x.astype(f), dy.astype(f), (3, 3), **kw)) < TOL[dtype]
+
+
+@DTYPES
+@pytest.mark.parametrize("shape", [(2, 33, 9, 6), (3, 8, 41, 31), (1, 5, 1, 1)], ids=["33ch", "8ch", "one"])
+def test_elementwise_off_the_boundary(ctx, dtype, shape):
+    """Any of the three tensors may start off the 16-byte boundaries; the results are those of aligned tensors."""
+    rs = np.random.RandomState(7)
+    A, B = (T.from_host(ctx, rs.standard_normal(shape).astype(dtype), "nhwc") for _ in range(2))
+    (As, o1), (Bs, o2) = shifted(A), shifted(B)
+    v = rs.standard_normal(shape[1]).astype(dtype)
+    for op, aligned, off in (("add", B, Bs), ("mul", 0.5, 0.5), ("sub", v, v), ("sgn", None, None)):
+        want = stored(shim.device_elementwise(op, A, aligned))
+        for a in (A, As):
+            for b in {id(aligned): aligned, id(off): off}.values():
+                for make in (lambda: (T(ctx, shape, dtype, "nhwc"), None), lambda: shifted(A, 7)):
+                    out, owner = make()
+                    assert np.array_equal(stored(shim.device_elementwise(op, a, b, out=out)), want), (op, a is As, owner)
+    out, owner = shifted(A)
+    assert np.array_equal(stored(shim.device_elementwise("add", out, Bs, out=out)), stored(shim.device_elementwise("add", A, B)))
+
+
+# few-channel layers, whose images are rearranged first: folded rows and 2x2 pixel blocks; strided gradInputs whose
+# parity classes are channels of one launch
+STEMS = [((2, 3, 20, 17), 24, 3, 1), ((3, 1, 15, 18), 8, 5, 1), ((2, 3, 21, 22), 64, 7, 2), ((2, 4, 16, 16), 16, 3, 2)]
+
+
+@DTYPES
+@pytest.mark.parametrize("xs,k,ks,s", STEMS, ids=lambda v: str(v).replace(" ", ""))
+def test_stems_off_the_boundary(ctx, dtype, xs, k, ks, s):
+    rs = np.random.RandomState(8)
+    X = T.from_host(ctx, rs.standard_normal(xs).astype(dtype), "nhwc")
+    W = T.from_host(ctx, (rs.standard_normal((k, xs[1], ks, ks)) / ks).astype(dtype))
+    Xs, owner = shifted(X)
+    kw = dict(border_mode="half", subsample=(s, s))
+    Y = shim.device_conv2d(X, W, **kw)
+    assert np.array_equal(stored(shim.device_conv2d(Xs, W, **kw)), stored(Y))
+    DY = T.from_host(ctx, rs.standard_normal(Y.shape).astype(dtype), "nhwc")
+    assert np.array_equal(shim.device_grad_weights(Xs, DY, (ks, ks), **kw).to_host(),
+                          shim.device_grad_weights(X, DY, (ks, ks), **kw).to_host())
+    if s > 1:
+        DX = shim.device_grad_inputs(W, DY, xs[2:], **kw)
+        DXs, owner2 = shifted(X, 7)
+        assert np.array_equal(stored(shim.device_grad_inputs(W, DY, xs[2:], out=DXs, **kw)), stored(DX))
+        assert not stored(DXs)[..., xs[1]:].any()

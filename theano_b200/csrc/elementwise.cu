@@ -41,6 +41,16 @@ template <> __device__ __forceinline__ void store16<__half>(__half* p, const flo
   *reinterpret_cast<uint4*>(p) = v;
 }
 
+// 16 bytes, or one element
+template <typename T, int V> __device__ __forceinline__ void load(const T* p, float (&f)[V]) {
+  if constexpr (V == 1) f[0] = static_cast<float>(*p);
+  else load16<T>(p, f);
+}
+template <typename T, int V> __device__ __forceinline__ void store(T* p, const float (&f)[V]) {
+  if constexpr (V == 1) *p = static_cast<T>(f[0]);
+  else store16<T>(p, f);
+}
+
 __device__ __forceinline__ float apply(int op, float a, float b) {
   switch (op) {
     case kEwAdd: return a + b;
@@ -62,23 +72,23 @@ __device__ __forceinline__ float apply(int op, float a, float b) {
 // channels are written as 0 so that the tensor stays a valid channels-last operand.
 // HBM bound; what keeps it off that bound is bytes in flight per thread, so a thread takes four vectors
 // whose loads are issued together, and a tensor without pad channels whose operand needs no channel index
-// (PLAIN) computes none.  Unary op, 411 MB float32 in and out: 158 -> 133 us.
+// (PLAIN) computes none.  Unary op, 411 MB float32 in and out: 158 -> 133 us.  V is a vector's element count: 1 where
+// a tensor does not start on a 16-byte boundary.
 constexpr int kEwVecs = 4;
-template <typename T, bool PLAIN>
+template <typename T, int V, bool PLAIN>
 __global__ void __launch_bounds__(256) elementwise_kernel(const T* __restrict__ a, const T* __restrict__ b,
                                                           const float* __restrict__ chan, T* __restrict__ out,
                                                           long long nvec, int C, int Cp, int op, int b_kind, float s) {
   pdl_enter();
-  constexpr int V = Vec<T>::n;
   const long long base = blockIdx.x * (256LL * kEwVecs) + threadIdx.x;
   float fa[kEwVecs][V], fb[kEwVecs][V];
 #pragma unroll
   for (int k = 0; k < kEwVecs; ++k)
-    if (base + k * 256 < nvec) load16<T>(a + (base + k * 256) * V, fa[k]);
+    if (base + k * 256 < nvec) load<T>(a + (base + k * 256) * V, fa[k]);
   if (b_kind == 0)
 #pragma unroll
     for (int k = 0; k < kEwVecs; ++k)
-      if (base + k * 256 < nvec) load16<T>(b + (base + k * 256) * V, fb[k]);
+      if (base + k * 256 < nvec) load<T>(b + (base + k * 256) * V, fb[k]);
 #pragma unroll
   for (int k = 0; k < kEwVecs; ++k) {
     const long long i = base + k * 256;
@@ -91,7 +101,7 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const T* __restrict__ 
       const float bv = b_kind == 0 ? fb[k][q] : b_kind == 1 ? s : !PLAIN && b_kind == 2 ? chan[c0 + q] : 0.f;
       fo[q] = PLAIN || c0 + q < C ? apply(op, fa[k][q], bv) : 0.f;
     }
-    store16<T>(out + i * V, fo);
+    store<T>(out + i * V, fo);
   }
 }
 
@@ -117,8 +127,7 @@ __global__ void __launch_bounds__(256) channel_sum_partial_kernel(const T* __res
 #pragma unroll 8
       for (long long p = first; p < pixels; p += step) {
         float f[V];
-        if constexpr (V == 1) f[0] = static_cast<float>(src[p * Cp]);
-        else load16<T>(src + p * Cp, f);
+        load<T>(src + p * Cp, f);
 #pragma unroll
         for (int q = 0; q < V; ++q) acc[q] += f[q];
       }
@@ -162,20 +171,23 @@ __global__ void __launch_bounds__(512) channel_sum_final_kernel(const float* __r
 cudaError_t launch_elementwise(const void* a, const void* b, const float* chan, void* out, long long elems, int C,
                                int Cp, int op, int b_kind, float s, int dtype, cudaStream_t st) {
   if (elems == 0) return cudaSuccess;
-  const int V = dtype == B200CONV_F16 ? 8 : 4;
+  const bool wide = aligned16({a, b, out});
+  const int V = !wide ? 1 : dtype == B200CONV_F16 ? 8 : 4;
   const long long nvec = elems / V;              // Cp is a multiple of V, so elems is
   const long long grid = (nvec + 256 * kEwVecs - 1) / (256 * kEwVecs);
   if (grid >= (1LL << 31)) return cudaErrorInvalidValue;
   const bool plain = C == Cp && b_kind != 2;
-#define B200_EW(T, PLAIN)                                                                                      \
-  launch_streaming(elementwise_kernel<T, PLAIN>, static_cast<int>(grid), 256, 0, st,                                         \
+#define B200_EW(T, V, PLAIN)                                                                                   \
+  launch_streaming(elementwise_kernel<T, V, PLAIN>, static_cast<int>(grid), 256, 0, st,                        \
       static_cast<const T*>(a), static_cast<const T*>(b), chan, static_cast<T*>(out), nvec, C, Cp, op, b_kind, s)
   if (dtype == B200CONV_F16) {
-    if (plain) B200_EW(__half, true);
-    else B200_EW(__half, false);
+    if (!wide) B200_EW(__half, 1, false);
+    else if (plain) B200_EW(__half, 8, true);
+    else B200_EW(__half, 8, false);
   } else {
-    if (plain) B200_EW(float, true);
-    else B200_EW(float, false);
+    if (!wide) B200_EW(float, 1, false);
+    else if (plain) B200_EW(float, 4, true);
+    else B200_EW(float, 4, false);
   }
 #undef B200_EW
   return cudaGetLastError();
@@ -190,7 +202,7 @@ int channel_sum_blocks(long long pixels) {
 cudaError_t launch_channel_sum(const void* x, float* partial, void* out, long long pixels, int C, int Cp, int dtype,
                                cudaStream_t st) {
   const int blocks = channel_sum_blocks(pixels);
-  const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const bool wide = aligned16({x});
   const int vecs = wide ? Cp / (dtype == B200CONV_F16 ? 8 : 4) : Cp;
   int log_lanes = 0;                             // as many rows of threads over the pixels as the channel vector leaves
   while (log_lanes < 8 && (vecs << (log_lanes + 1)) <= 256) ++log_lanes;

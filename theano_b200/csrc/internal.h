@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 
 #include "../../include/b200conv.h"
 #include "geometry.h"
@@ -69,6 +70,13 @@ constexpr unsigned kChainedBlocks = 148 * 8;      // of 256 threads
 template <class... Exp, class... Act>
 cudaError_t launch_streaming(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
   return launch_linked(grid.x * grid.y * grid.z <= kChainedBlocks, kernel, grid, block, smem, s, 1, args...);
+}
+
+// Kernels with 16-byte accesses take an element-wise form where a caller's tensor starts off the 16-byte boundaries.
+inline bool aligned16(std::initializer_list<const void*> ptrs) {
+  for (const void* p : ptrs)
+    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
+  return true;
 }
 
 // Codes a kernel writes to the device status word when it gives up.

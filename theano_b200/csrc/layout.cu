@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) pack_filters_batch_kernel(const __grid_co
 // Few-channel layers ("row folding"): the image is copied channels-last with explicit zero
 // columns left and right, [N][H][Wp][Cp], so that the kW * Cp values under one filter row are
 // contiguous and can serve as one reduction block of the implicit GEMM.  One thread per output
-// pixel; src is NCHW (nhwc_in = 0) or channels-last [N][H][W][Cp].
+// pixel; src is NCHW (nhwc_in = 0), channels-last [N][H][W][Cp] (1) or that off the 16-byte boundaries (2).
 template <typename T>
 __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int C, int H,
                                 int W, int Cp, int Wp, int pad_l, int nhwc_in) {
@@ -144,11 +144,12 @@ __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, 
       // one pixel is 16 bytes: assemble it in registers, store it once
       uint4 px = make_uint4(0, 0, 0, 0);
       if (inside) {
-        if (nhwc_in) {
+        if (nhwc_in == 1) {
           px = *reinterpret_cast<const uint4*>(src + ((1LL * n * H + h) * W + w) * Cp);
         } else {
           T* v = reinterpret_cast<T*>(&px);
-          for (int c = 0; c < C; ++c) v[c] = src[((1LL * n * C + c) * H + h) * W + w];
+          for (int c = 0; c < C; ++c)
+            v[c] = nhwc_in ? src[((1LL * n * H + h) * W + w) * Cp + c] : src[((1LL * n * C + c) * H + h) * W + w];
         }
       }
       *reinterpret_cast<uint4*>(dst + idx * Cp) = px;
@@ -191,7 +192,8 @@ __global__ void pack_filters_fold_kernel(const T* __restrict__ w, T* __restrict_
 //   dst[n][h2][q][(dy*2 + dx)*C + c] = src[n][c][2*h2 + dy][2*(q + q0) + dx]
 // with zeros outside the image and in the unused channels.  The layer then is a stride-1 layer over
 // dst whose filter rows span a few consecutive pixels: one contiguous reduction block per row.
-// One thread per dst pixel; src is NCHW (nhwc_in = 0) or channels-last [N][H][W][Cp_in].
+// One thread per dst pixel; src is NCHW (nhwc_in = 0), channels-last [N][H][W][Cp_in] (1) or that off the 16-byte
+// boundaries (2).
 template <typename T, int C>
 __global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H,
                                int W, int Cp_in, int H2, int Wq, int q0, int nhwc_in) {
@@ -209,7 +211,7 @@ __global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, i
     for (int par = 0; par < 4; ++par) {
       const int h = 2 * h2 + (par >> 1), w = 2 * (q + q0) + (par & 1);
       if (h < H && w >= 0 && w < W) {
-        if (nhwc_in && Cp_in * sizeof(T) == 16) {     // one source pixel is one 16-byte load
+        if (nhwc_in == 1 && Cp_in * sizeof(T) == 16) {     // one source pixel is one 16-byte load
           const uint4 px = *reinterpret_cast<const uint4*>(src + ((1LL * n * H + h) * W + w) * Cp_in);
           const T* e = reinterpret_cast<const T*>(&px);
 #pragma unroll
@@ -501,7 +503,8 @@ __global__ void pack_filters_merged_kernel(const T* __restrict__ w, T* __restric
 }
 
 // NCHW output: one thread per element.  Channels-last output: one thread per pixel, which reads
-// its C values (contiguous in tmp) and writes the whole padded channel vector in 16-byte pieces.
+// its C values (contiguous in tmp) and writes the whole padded channel vector in 16-byte pieces (nhwc = 1) or, into a
+// tensor off the 16-byte boundaries (2), value by value.
 template <typename T>
 __global__ void depth_to_space_kernel(const T* __restrict__ tmp, T* __restrict__ dx, int N, int C, int H, int W,
                                       int sH, int sW, int Ct, int Cp, int nhwc) {
@@ -518,10 +521,15 @@ __global__ void depth_to_space_kernel(const T* __restrict__ tmp, T* __restrict__
       const T* src = tmp + ((n * Hq + h / sH) * Wq + w / sW) * Ct + cls * C;
       T* dst = dx + idx * Cp;
       for (int c0 = 0; c0 < Cp; c0 += kVec) {
-        T v[kVec];
+        __align__(16) T v[kVec];
 #pragma unroll
         for (int q = 0; q < kVec; ++q) v[q] = c0 + q < C ? src[c0 + q] : T(0);
-        *reinterpret_cast<uint4*>(dst + c0) = *reinterpret_cast<const uint4*>(v);
+        if (nhwc == 1) {
+          *reinterpret_cast<uint4*>(dst + c0) = *reinterpret_cast<const uint4*>(v);
+        } else {
+#pragma unroll
+          for (int q = 0; q < kVec; ++q) dst[c0 + q] = v[q];
+        }
       }
     }
     return;
@@ -606,10 +614,14 @@ cudaError_t launch_pack_filters(const void* w, void* dst, int K, int Cg, int kH,
   return cudaGetLastError();
 }
 
+// 0: NCHW, 1: channels-last, 2: channels-last off the 16-byte boundaries (no wide access)
+static int channels_last_form(int nhwc, const void* p) { return nhwc && !aligned16({p}) ? 2 : nhwc; }
+
 cudaError_t launch_pad_fold(const void* src, void* dst, int N, int C, int H, int W, int Cp, int Wp,
                             int pad_l, int nhwc_in, int dtype, cudaStream_t s) {
   const long long total = 1LL * N * H * Wp;
   if (total == 0) return cudaSuccess;
+  nhwc_in = channels_last_form(nhwc_in, src);
   if (dtype == B200CONV_F16)
     launch_streaming(pad_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(src), static_cast<__half*>(dst), N, C, H, W, Cp, Wp, pad_l, nhwc_in);
@@ -652,6 +664,7 @@ cudaError_t pad_s2d_typed(const void* src, void* dst, int N, int C, int H, int W
   const long long total = 1LL * N * H2 * Wq;
   const T* in = static_cast<const T*>(src);
   T* out = static_cast<T*>(dst);
+  nhwc_in = channels_last_form(nhwc_in, src);
   const int grid = grid_for(total, 256);
   switch (C) {   // the channel count as a constant keeps the assembled pixel in registers
     case 1: launch_streaming(pad_s2d_kernel<T, 1>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
@@ -745,11 +758,6 @@ cudaError_t for_index(long long total, Launch launch) {
   launch(static_cast<int>(grid), total < (1LL << 31));
   return cudaGetLastError();
 }
-bool aligned16(std::initializer_list<const void*> ptrs) {
-  for (const void* p : ptrs)
-    if (reinterpret_cast<uintptr_t>(p) & 15) return false;
-  return true;
-}
 template <typename P, typename T = typename P::type>
 cudaError_t maxpool_nhwc(const T* x, T* y, int N, int H, int W, int Cp, cudaStream_t s) {
   const int pieces = Cp / P::n;
@@ -826,6 +834,7 @@ cudaError_t launch_depth_to_space(const void* tmp, void* dx, int N, int C, int H
                                   int Ct, int Cp, int nhwc, int dtype, cudaStream_t s) {
   const long long total = 1LL * N * (nhwc ? 1 : C) * H * W;
   if (total == 0) return cudaSuccess;
+  nhwc = channels_last_form(nhwc, dx);
   if (dtype == B200CONV_F16)
     launch_streaming(depth_to_space_kernel<__half>, grid_for(total, 256), 256, 0, s,
         static_cast<const __half*>(tmp), static_cast<__half*>(dx), N, C, H, W, sH, sW, Ct, Cp, nhwc);
