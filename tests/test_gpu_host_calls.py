@@ -51,6 +51,30 @@ def test_small_inputs_wait_for_large_ones_in_their_own_slot(extra):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("page_locked", [False, True])
+@pytest.mark.parametrize("start,c", [(0, 64), (0.25, 64), (1, 64), (0, 128)], ids=["front", "inside", "back", "same"])
+def test_a_result_may_lie_over_the_input(start, c, page_locked):
+    """The memory of out= holds the input: a batch in chunks would overwrite images that have not gone up yet."""
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(5)
+    n, k, h = 16, 128, 64                                                    # 2 MB per image of the result, as much or half of the input
+    w = (rs.standard_normal((k, c, 1, 1)) / 8).astype(np.float32)
+    v = np.ascontiguousarray(w.transpose(1, 0, 2, 3))
+    kw = dict(border_mode="valid", subsample=(1, 1))
+    x = rs.standard_normal((n, c, h, h)).astype(np.float32)
+    for call, want in ((lambda a, o: shim.conv2d_forward(a, w, out=o, ctx=ctx, **kw), O.conv2d(x, w, **kw)),
+                       (lambda a, o: shim.conv2d_grad_inputs(v, a, out=o, ctx=ctx, **kw), O.conv2d_grad_inputs(v, x, (h, h), **kw))):
+        # page-locked: a result of the library is such an array
+        out = shim.maxpool2x2(np.zeros((n, k, 2 * h, 2 * h), np.float32), ctx=ctx) if page_locked else np.empty((n, k, h, h), np.float32)
+        first = int(start * (out.size - x.size))
+        a = out.reshape(-1)[first:first + x.size].reshape(x.shape)
+        a[...] = x
+        assert np.shares_memory(a, out)
+        got = call(a, out)
+        assert got is out and O.rel_err(got, want) < 5e-3      # TF32 rounds each factor by at most 2^-10 relative
+
+
+@pytest.mark.gpu
 def test_results_keep_their_values_while_others_are_made():
     ctx = shim.get_context(0)
     rs = np.random.RandomState(0)

@@ -2322,7 +2322,10 @@ int run_batch(b200conv_ctx* c, HostIO& io, int N, const void* hin, size_t in_byt
               Compute compute) {
   int rc;
   void *din, *dout;
-  const BatchPlan bp = plan_batch(N, in_bytes, out_bytes);
+  // a result that lies over the input (and not each image over its own): all of the input goes up before any of the
+  // result comes down
+  const bool over = overlap(hin, in_bytes, hout, out_bytes) && !(hin == hout && in_bytes == out_bytes);
+  const BatchPlan bp = over ? BatchPlan{1, N} : plan_batch(N, in_bytes, out_bytes);
   if (bp.chunks == 1) {
     if ((rc = io.in(hin, in_bytes, &din)) || (rc = io.out(out_bytes, &dout)) || (rc = io.start())) return rc;
     if ((rc = compute(N, din, dout))) return rc;
