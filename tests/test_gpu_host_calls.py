@@ -75,6 +75,21 @@ def test_a_result_may_lie_over_the_input(start, c, page_locked):
 
 
 @pytest.mark.gpu
+def test_a_capture_refuses_host_calls_and_leaves_the_staging_ring_alone():
+    """An event of the ring recorded in a capture could not be waited for by the calls that come after it."""
+    ctx = shim.Context(0)
+    x = np.arange(2 * 3 * 8 * 8, dtype=np.float32).reshape(2, 3, 8, 8)
+    w, want = np.ones((5, 3, 1, 1), np.float32), x.reshape(2, 3, 4, 2, 4, 2).max(axis=(3, 5))
+    y = shim.maxpool2x2(x, ctx=ctx)
+    for call in (lambda: shim.maxpool2x2(x, ctx=ctx), lambda: shim.maxpool2x2_grad(x, y, y, ctx=ctx), lambda: shim.conv2d_forward(x, w, ctx=ctx)):
+        with pytest.raises(ValueError, match="cannot be captured"):
+            ctx.capture(call)
+    for _ in range(40):                          # more calls than the ring has slots
+        assert np.array_equal(shim.maxpool2x2(x, ctx=ctx), want)
+    ctx.close()
+
+
+@pytest.mark.gpu
 def test_results_keep_their_values_while_others_are_made():
     ctx = shim.get_context(0)
     rs = np.random.RandomState(0)

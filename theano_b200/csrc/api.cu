@@ -2603,6 +2603,7 @@ int b200conv_maxpool2x2(b200conv_ctx* c, const void* x, void* y, int N, int C, i
     return 0;
   }
   if (nhwc) return fail(c, B200CONV_E_INVALID, "host tensors are NCHW");
+  if (c->capturing) return fail(c, B200CONV_E_INVALID, "host-pointer calls cannot be captured in a graph");
   HostIO io(c);
   void *dx_, *dy_;
   int rc;
@@ -2626,6 +2627,7 @@ int b200conv_maxpool2x2_grad(b200conv_ctx* c, const void* x, const void* y, cons
     return 0;
   }
   if (nhwc) return fail(c, B200CONV_E_INVALID, "host tensors are NCHW");
+  if (c->capturing) return fail(c, B200CONV_E_INVALID, "host-pointer calls cannot be captured in a graph");
   HostIO io(c);
   void *dx_, *dy_, *dgy_, *dgx_;
   int rc;
