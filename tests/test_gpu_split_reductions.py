@@ -138,6 +138,22 @@ def test_pooling_epilogue_still_asks_for_whole_channel_chunks(ctx, dtype):
 
 
 @DTYPES
+def test_what_the_epilogue_refuses_does_not_depend_on_earlier_calls(dtype):
+    """An output off the 16-byte boundaries is refused also when an aligned one has chosen a split reduction before."""
+    own = shim.Context(0)                        # with timing
+    X = T.from_host(own, np.ones((1, 512, 8, 8), dtype), "nhwc")
+    W = T.from_host(own, np.ones((64, 512, 3, 3), dtype))
+    y = shim.device_conv2d(X, W, border_mode="half", pool=True)
+    ys, owner = shifted(y, 7)
+    for _ in range(2):
+        with pytest.raises(shim.B200Error, match="cannot pool"):
+            shim.device_conv2d(X, W, border_mode="half", pool=True, out=ys)
+        assert (stored(ys) == 7).all()
+        shim.device_conv2d(X, W, border_mode="half", pool=True, out=y)
+    own.close()
+
+
+@DTYPES
 @pytest.mark.parametrize("c,k,g", [(256, 256, 32), (96, 48, 12), (64, 128, 8), (48, 48, 3), (512, 256, 2)], ids=lambda v: str(v))
 def test_grad_weights_of_merged_groups(ctx, dtype, c, k, g):
     rs = np.random.RandomState(g)

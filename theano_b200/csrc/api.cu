@@ -1053,6 +1053,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   key.add(sc);
   key.add(sw);
   key.add(c->epi.pool * 4 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
+  const size_t es = elem_size(a.dtype);
+  const bool tma = sc == 1 && a.n_out % (int)(128 / es) == 0 && !c->epi.residual && (sw * es) % 16 == 0 && (sh * es) % 16 == 0 &&
+                   (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
+  // what cannot pool does not depend on the choice that an earlier call left (a split reduction pools any output)
+  if (c->epi.pool && !(allow_slab && tma)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
   if (c->autotune) {
     auto it = c->algo_cache.find(key);
     if (it != c->algo_cache.end()) return run(it->second);
@@ -1065,7 +1070,6 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     cand[ncand++] = kConvTap;
     if (tap_spread) cand[ncand++] = kConvTapSpread;
   }
-  if (c->epi.pool && !allow_slab) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
   if (allow_slab) {
     int eh[2] = {0, 0}, ew[2] = {0, 0};
     for (size_t i = 0; i < taps_in.size(); ++i) {
@@ -1074,12 +1078,9 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       eh[0] = std::min<int>(eh[0], t.dh); eh[1] = std::max<int>(eh[1], t.dh);
       ew[0] = std::min<int>(ew[0], t.dw); ew[1] = std::max<int>(ew[1], t.dw);
     }
-    const size_t es = elem_size(a.dtype);
-    const bool tma = sc == 1 && a.n_out % (int)(128 / es) == 0 && !c->epi.residual && (sw * es) % 16 == 0 && (sh * es) % 16 == 0 &&
-                     (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
     const SlabTile w = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabWide);
     const SlabTile n = find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabSpread);
-    if (c->epi.pool && !(tma && w.found)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+    if (c->epi.pool && !w.found) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
     // pairs of CTAs where at least half of the SMs get work (below, the variants that spread a tile are ahead)
     const SlabTile m = c->use_pair ? find_slab_tile(c, a, (int)taps_in.size(), Wt, Ht, eh[1] - eh[0], ew[1] - ew[0], tma, kSlabPair) : SlabTile();
     const bool pair = m.found && cdiv(cdiv(Wt, m.wt) * cdiv(Ht, m.th) * cdiv(a.N, m.nb), 2) * cdiv(a.n_out, m.bn) * a.groups >= c->num_sms / 4;
