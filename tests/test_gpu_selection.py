@@ -185,3 +185,28 @@ def test_stacked_tap_gradweights_equals_one_mma_per_tap_and_the_oracle(geo):
     assert np.array_equal(got[True], got[False])
     assert O.rel_err(got[True].astype(np.float32), want) < 2e-2
     ctx.close()
+
+
+@pytest.mark.parametrize("value", range(5))
+def test_any_choice_in_a_tuning_file_gives_the_right_result(tmp_path, value):
+    """The slab kernel reads one view of the image, a strided layer has several: a file that names it for such a layer
+    (written by hand, or for another version) gets the kernel that takes them."""
+    rs = np.random.RandomState(34)
+    x = rs.standard_normal((2, 64, 14, 14)).astype(np.float32)
+    w = (rs.standard_normal((48, 64, 3, 3)) / 24).astype(np.float32)
+    kw = dict(border_mode="half", subsample=(2, 2))
+    want = O.conv2d(x, w, **kw)
+    path = str(tmp_path / "tuning")
+    for loaded in (False, True):
+        ctx = shim.Context(0)
+        if loaded:
+            assert ctx.tuning_load(path) == 1
+        X, W = shim.DeviceTensor.from_host(ctx, x, "nhwc"), shim.DeviceTensor.from_host(ctx, w)
+        assert O.rel_err(shim.device_conv2d(X, W, **kw).to_host(), want) < 5e-3
+        if not loaded:
+            ctx.tuning_save(path)
+            lines = open(path).read().splitlines()
+            choices = [l.split() for l in lines if l.startswith("a ")]
+            assert len(choices) == 1
+            open(path, "w").write("\n".join([lines[0], " ".join(choices[0][:2] + [str(value)])]) + "\n")
+        ctx.close()

@@ -936,8 +936,10 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
                       long long sn, long long sc, long long sh, long long sw, long long off,
                       const void* bias, int relu, int variant) {
   if (variant == kConvSlab || variant == kConvSlabSpread || variant == kConvSlabPair) {
+    // the slab kernel reads one view (a tuning file may name it for a geometry with several)
+    const bool one_view = view_parity.size() == 1;
     const int rh = view_parity[0].first, rw = view_parity[0].second;
-    if (rh < a.Hs && rw < a.Ws) {
+    if (one_view && rh < a.Hs && rw < a.Ws) {
       const int rc = try_conv_slab(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, slab_mode(variant));
       if (rc != 2) return rc;
     }
