@@ -33,6 +33,21 @@ def test_chunked_batches_against_oracle(n, pageable_out):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 13], ids=lambda n: "n%d" % n)
+def test_chunked_batches_in_page_locked_memory(n):
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(n)
+    x, y, dx = (ctx.pinned_empty((n, 64, 61, 64), np.float32) for _ in range(3))
+    x[...] = rs.standard_normal(x.shape)
+    w = (rs.standard_normal((64, 64, 1, 1)) / 8).astype(np.float32)
+    kw = dict(border_mode="valid", subsample=(1, 1))
+    assert shim.conv2d_forward(x, w, out=y, ctx=ctx, **kw) is y
+    assert O.rel_err(np.array(y), O.conv2d(np.array(x), w, **kw)) < 5e-3      # TF32 rounds each factor by at most 2^-10
+    assert shim.conv2d_grad_inputs(w, x, out=dx, ctx=ctx, **kw) is dx
+    assert O.rel_err(np.array(dx), O.conv2d_grad_inputs(w, np.array(x), x.shape[2:], **kw)) < 5e-3
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("extra", [1, 30], ids=["filters", "residual"])
 def test_small_inputs_wait_for_large_ones_in_their_own_slot(extra):
     """Small inputs share a slot of the staging ring; an image of more than the whole ring must not take it."""
@@ -64,8 +79,7 @@ def test_a_result_may_lie_over_the_input(start, c, page_locked):
     x = rs.standard_normal((n, c, h, h)).astype(np.float32)
     for call, want in ((lambda a, o: shim.conv2d_forward(a, w, out=o, ctx=ctx, **kw), O.conv2d(x, w, **kw)),
                        (lambda a, o: shim.conv2d_grad_inputs(v, a, out=o, ctx=ctx, **kw), O.conv2d_grad_inputs(v, x, (h, h), **kw))):
-        # page-locked: a result of the library is such an array
-        out = shim.maxpool2x2(np.zeros((n, k, 2 * h, 2 * h), np.float32), ctx=ctx) if page_locked else np.empty((n, k, h, h), np.float32)
+        out = ctx.pinned_empty((n, k, h, h), np.float32) if page_locked else np.empty((n, k, h, h), np.float32)
         first = int(start * (out.size - x.size))
         a = out.reshape(-1)[first:first + x.size].reshape(x.shape)
         a[...] = x
@@ -141,6 +155,58 @@ def test_result_pool_reuses_and_gives_back(monkeypatch):
     assert pool.kept <= pool.KEEP and pool.total == pool.kept and len(Ctx.lib.buffers) <= 2
     pool.trim()                                                         # nothing is out: all of it goes back
     assert pool.total == pool.kept == 0 and not Ctx.lib.buffers
+
+
+def _pool(monkeypatch, limit=None):
+    class Ctx(object):
+        lib, h = _FakeLibrary(), None
+    monkeypatch.setattr(shim, "load_library", lambda: Ctx.lib)
+    pool = shim._ResultPool()
+    if limit is not None:
+        pool.LIMIT = pool.KEEP = limit
+    return pool, Ctx
+
+
+def _passes(pool, ctx, sizes, count):
+    """Page-locked allocations of each of `count` passes that hold results of `sizes` bytes and then drop them."""
+    made = []
+    for _ in range(count):
+        before = ctx.lib.made
+        held = [pool.empty(ctx, (n,), np.dtype(np.uint8)) for n in sizes]
+        assert pool.total <= pool.LIMIT
+        made.append(ctx.lib.made - before)
+        del held
+        gc.collect()
+    return made
+
+
+@pytest.mark.parametrize("sizes", [[300 << 20], [90 << 20, 100 << 20, 110 << 20], [6 << 20] * 60, [26 << 20, 26 << 20, 1 << 20]],
+                         ids=["one", "three", "sixty", "training"])
+def test_result_pool_does_not_lock_memory_again_and_again(monkeypatch, sizes):
+    """Page-locking costs more than an ordinary array: once per block, and never on every pass."""
+    pool, ctx = _pool(monkeypatch)
+    made = _passes(pool, ctx, sizes, 12)
+    assert not any(made[8:]), made
+    if sum(sizes) < pool.LIMIT:                                          # all of them end up in locked memory
+        assert all(pool.empty(ctx, (n,), np.dtype(np.uint8)).base is not None for n in sizes)
+    # what is locked was earned: twice its bytes went out as ordinary arrays, beyond the credit at the start
+    assert pool.total <= pool.CREDIT + 12 * sum(sizes) // 2
+    assert _passes(pool, ctx, [1 << 29], 2) == [0, 0]                    # beyond the limit: ordinary
+
+
+def test_result_pool_gives_unused_sizes_back(monkeypatch):
+    pool, ctx = _pool(monkeypatch)
+    _passes(pool, ctx, [150 << 20], 6)
+    assert pool.kept >= 150 << 20
+    made = _passes(pool, ctx, [6 << 20] * 20, 20)
+    assert not any(made[14:]) and pool.total <= 256 << 20 and sum(made) == 20
+    assert len(ctx.lib.buffers) == 20 and pool.total == pool.kept
+
+
+def test_result_pool_can_be_turned_off(monkeypatch):
+    pool, ctx = _pool(monkeypatch, 0)
+    a = pool.empty(ctx, (1 << 20,), np.dtype(np.float32))
+    assert a.flags.owndata and ctx.lib.made == 0
 
 
 def test_operands_in_the_other_byte_order_are_converted():

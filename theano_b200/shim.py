@@ -462,24 +462,53 @@ class _ResultPool(object):
     transfer straight into the result: a fresh pageable array costs its page faults (0.8 ms per
     4 MB) and a copy out of a staging buffer on top of the transfer (0.08 ms per 4 MB).
 
-    Page-locking itself is slow (1 ms per MB), so the memory of arrays that died is kept for the
-    next result of that size class: at most ``KEEP`` bytes; beyond that it is given back.  At most
-    ``LIMIT`` bytes are out or kept at once; further results are ordinary numpy arrays, as are those
-    below ``SMALLEST`` bytes.  Safe with several threads (the lock is re-entrant because an array may
-    die in a garbage collection inside one of these methods); the host-pointer calls are synchronous,
-    so nothing on the device writes to a block whose array has died."""
-    SMALLEST, LIMIT, KEEP = 16 << 10, 1 << 30, 256 << 20
+    Page-locking itself is slow (0.4 to 1 ms per MB), so it pays only for memory that is used again:
+    the memory of arrays that died is kept for the next result of that size class, and new memory is
+    page-locked against a credit that starts at ``CREDIT`` bytes and grows by half of what was handed
+    out as ordinary arrays.  At most ``LIMIT`` bytes are out or kept at once and at most ``KEEP`` kept;
+    sizes that have not been asked for during the last ``STALE`` results give way to others.  Whatever
+    does not fit is an ordinary numpy array, as are results below ``SMALLEST`` bytes.
+    ``B200CONV_PINNED_RESULTS_MB`` in the environment sets both bounds; 0 turns the pool off.
+
+    Measured per pass (results dropped after it): 300 MB in one result 20 ms as an ordinary array, but
+    126 to 270 ms when a block beyond KEEP was locked and given back every time; 20 results of 6.4 MB
+    37 ms as ordinary arrays, 90 to 146 ms with locked memory that blocks of another size kept full.
+
+    Safe with several threads (the lock is re-entrant because an array may die in a garbage collection
+    inside one of these methods); the host-pointer calls are synchronous, so nothing on the device writes
+    to a block whose array has died."""
+    SMALLEST, CREDIT, STALE = 16 << 10, 16 << 20, 64
+    LIMIT = KEEP = int(os.environ.get("B200CONV_PINNED_RESULTS_MB", "256")) << 20
 
     def __init__(self):
         self.free = {}                   # size class -> addresses
+        self.asked = {}                  # size class -> number of the last result of that class
         self.lock = threading.RLock()
         self.total = self.kept = 0       # bytes out or kept / kept
+        self.results = 0
+        self.credit = self.CREDIT
 
     @staticmethod
     def size_class(n):
         """n rounded up to 1/4 of its power of two (at least one 16 KB step)."""
         step = max(16 << 10, 1 << max(0, n.bit_length() - 3))
         return -(-n // step) * step
+
+    def _make_room(self, size):
+        """Blocks of stale classes to give back so that `size` fits, or None if it does not."""
+        need, gone = self.total + size - self.LIMIT, []
+        stale = sorted((t, s) for s, t in self.asked.items() if t <= self.results - self.STALE)
+        for _, s in stale:
+            blocks = self.free.get(s, [])
+            count = min(len(blocks), -(-need // s)) if need > 0 else 0
+            gone += [(s, i) for i in range(count)]
+            need -= count * s
+        if need > 0:
+            return None
+        for s, _ in gone:
+            self.total -= s
+            self.kept -= s
+        return [self.free[s].pop() for s, _ in gone]
 
     def empty(self, ctx, shape, dtype, smallest=SMALLEST):
         n = dtype.itemsize
@@ -488,16 +517,23 @@ class _ResultPool(object):
         if n < smallest or n > self.LIMIT:
             return np.empty(shape, dtype)
         size = self.size_class(n)
+        ptr, gone = None, []
         with self.lock:
+            self.results += 1
+            self.asked[size] = self.results
             blocks = self.free.setdefault(size, [])
             if blocks:
                 ptr = blocks.pop()
                 self.kept -= size
-            elif self.total + size > self.LIMIT:
-                return np.empty(shape, dtype)
             else:
-                ptr = None
+                gone = self._make_room(size) if size <= self.credit else None
+                if gone is None:
+                    self.credit = min(self.credit + size // 2, self.LIMIT)
+                    return np.empty(shape, dtype)
+                self.credit -= size
                 self.total += size
+        for old in gone:
+            load_library().b200conv_host_free(None, _P(old))
         if ptr is None:
             p = _P()
             if ctx.lib.b200conv_host_alloc(ctx.h, size, ctypes.byref(p)) != 0:
