@@ -1,0 +1,52 @@
+"""The copy threads of the host-pointer calls (csrc/staging.h), compiled by itself and run on the CPU."""
+import subprocess
+
+from theano_b200 import build
+
+PROGRAM = r"""
+#include <stdio.h>
+#include <stdlib.h>
+#include <algorithm>
+#include <vector>
+%s
+#include "staging.h"
+using namespace b200;
+static int check(int threads) {
+  CopyPool pool(threads);
+  const size_t sizes[] = {1, 63, 64, 4095, 4096, 131071, 131072, 131073, 1 << 20, (2 << 20) - 1, (2 << 20) + 1, (16 << 20) + 12345};
+  std::vector<char> src(17 << 20), raw(17 << 20), back(17 << 20);
+  for (size_t i = 0; i < src.size(); ++i) src[i] = static_cast<char>(i * 2654435761u >> 13);
+  char* pinned = raw.data() + (64 - reinterpret_cast<uintptr_t>(raw.data()) %% 64) %% 64;      // as a ring slot: aligned
+  for (size_t n : sizes)
+    for (size_t off : {0, 1, 5000}) {
+      std::fill(back.begin(), back.end(), 'x');
+      std::fill(raw.begin(), raw.end(), 'y');
+      pool.copy(pinned, src.data() + off, n, true);
+      if (memcmp(pinned, src.data() + off, n) || pinned[n] != 'y') return 1;
+      pool.touch(back.data() + off, n);
+      for (char c : back)
+        if (c != 'x') return 2;
+      pool.copy(back.data() + off, pinned, n, false);
+      if (memcmp(back.data() + off, pinned, n) || back[off + n] != 'x' || (off && back[off - 1] != 'x')) return 3;
+      pool.touch(back.data() + off, n);
+      if (memcmp(back.data() + off, pinned, n)) return 4;
+    }
+  return 0;
+}
+int main() {
+  for (int threads : {1, 2, 8})
+    if (int rc = check(threads)) { printf("%%d threads: %%d\n", threads, rc); return 1; }
+  puts("ok");
+}
+"""
+
+
+def run(tmp_path, before=""):
+    src, exe = tmp_path / "staging.cpp", tmp_path / "staging"
+    src.write_text(PROGRAM % before)
+    subprocess.check_call(["g++", "-O2", "-std=c++17", "-pthread", "-I", build.CSRC, str(src), "-o", str(exe)])
+    return subprocess.run([str(exe)], stdout=subprocess.PIPE, timeout=120).stdout.decode().strip()
+
+
+def test_copies_and_touches_over_sizes_and_offsets(tmp_path):
+    assert run(tmp_path) == "ok"

@@ -2207,6 +2207,9 @@ int download(b200conv_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t
   }
   int rc = ring_setup(c);
   if (rc) return rc;
+  // Large arrays are likely to be fresh memory: while the transfers of a window fly, the threads make its pages present.
+  constexpr size_t kTouchFrom = 4u << 20, kTouchWindow = 16u << 20, kLargeArray = 64u << 20;
+  size_t touched = bytes >= kTouchFrom ? 0 : bytes;
   constexpr int kAhead = kRingSlots / 2;
   struct { int slot; size_t off, n; } flying[kAhead];
   size_t off = 0;
@@ -2222,9 +2225,14 @@ int download(b200conv_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t
       off += f.n;
     }
     const auto& f = flying[taken % kAhead];
+    while (touched < f.off + f.n) {
+      const size_t n = std::min(kTouchWindow, bytes - touched);
+      c->copy_pool->touch(static_cast<char*>(h) + touched, n);
+      touched += n;
+    }
     CU_OK(c, cudaEventSynchronize(c->ring_ev[f.slot]));
     c->ring_busy[f.slot] = false;
-    c->copy_pool->copy(static_cast<char*>(h) + f.off, c->ring + kRingSlotBytes * f.slot, f.n, false);
+    c->copy_pool->copy(static_cast<char*>(h) + f.off, c->ring + kRingSlotBytes * f.slot, f.n, false, bytes >= kLargeArray);
   }
   return 0;
 }
