@@ -464,8 +464,8 @@ class _ResultPool(object):
 
     Page-locking itself is slow (0.4 to 1 ms per MB), so it pays only for memory that is used again:
     the memory of arrays that died is kept for the next result of that size class, and new memory is
-    page-locked against a credit that starts at ``CREDIT`` bytes and grows by half of what was handed
-    out as ordinary arrays.  At most ``LIMIT`` bytes are out or kept at once and at most ``KEEP`` kept;
+    page-locked against a credit that starts at ``CREDIT`` bytes and grows with the ordinary arrays that
+    were handed out where a kept block would have served (a size asked for again).  At most ``LIMIT`` bytes are out or kept at once and at most ``KEEP`` kept;
     sizes that have not been asked for during the last ``STALE`` results give way to others.  Whatever
     does not fit is an ordinary numpy array, as are results below ``SMALLEST`` bytes.
     ``B200CONV_PINNED_RESULTS_MB`` in the environment sets both bounds; 0 turns the pool off.
@@ -477,7 +477,7 @@ class _ResultPool(object):
     Safe with several threads (the lock is re-entrant because an array may die in a garbage collection
     inside one of these methods); the host-pointer calls are synchronous, so nothing on the device writes
     to a block whose array has died."""
-    SMALLEST, CREDIT, STALE = 16 << 10, 16 << 20, 64
+    SMALLEST, CREDIT, STALE = 16 << 10, 64 << 20, 64
     LIMIT = KEEP = int(os.environ.get("B200CONV_PINNED_RESULTS_MB", "256")) << 20
 
     def __init__(self):
@@ -520,6 +520,7 @@ class _ResultPool(object):
         ptr, gone = None, []
         with self.lock:
             self.results += 1
+            again = self.asked.get(size, -self.STALE) > self.results - self.STALE
             self.asked[size] = self.results
             blocks = self.free.setdefault(size, [])
             if blocks:
@@ -528,7 +529,8 @@ class _ResultPool(object):
             else:
                 gone = self._make_room(size) if size <= self.credit else None
                 if gone is None:
-                    self.credit = min(self.credit + size // 2, self.LIMIT)
+                    if again:
+                        self.credit = min(self.credit + size, self.LIMIT)
                     return np.empty(shape, dtype)
                 self.credit -= size
                 self.total += size
