@@ -464,8 +464,8 @@ class _ResultPool(object):
 
     Page-locking itself is slow (0.4 to 1 ms per MB), so it pays only for memory that is used again:
     the memory of arrays that died is kept for the next result of that size class, and new memory is
-    page-locked against a credit that starts at ``CREDIT`` bytes and grows with the ordinary arrays that
-    were handed out where a kept block would have served (a size asked for again).  At most ``LIMIT`` bytes are out or kept at once and at most ``KEEP`` kept;
+    page-locked for a size that is asked for the third time (up to 1 MB at once), against a credit that
+    starts at ``CREDIT`` bytes and grows with the ordinary arrays of sizes asked for again.  At most ``LIMIT`` bytes are out or kept at once and at most ``KEEP`` kept;
     sizes that have not been asked for during the last ``STALE`` results give way to others.  Whatever
     does not fit is an ordinary numpy array, as are results below ``SMALLEST`` bytes.
     ``B200CONV_PINNED_RESULTS_MB`` in the environment sets both bounds; 0 turns the pool off.
@@ -483,6 +483,7 @@ class _ResultPool(object):
     def __init__(self):
         self.free = {}                   # size class -> addresses
         self.asked = {}                  # size class -> number of the last result of that class
+        self.count = {}                  # size class -> results of it before that, each within STALE of the next
         self.lock = threading.RLock()
         self.total = self.kept = 0       # bytes out or kept / kept
         self.results = 0
@@ -520,16 +521,17 @@ class _ResultPool(object):
         ptr, gone = None, []
         with self.lock:
             self.results += 1
-            again = self.asked.get(size, -self.STALE) > self.results - self.STALE
-            self.asked[size] = self.results
+            before = self.count.get(size, 0) if self.asked.get(size, -self.STALE) > self.results - self.STALE else 0
+            self.asked[size], self.count[size] = self.results, before + 1
             blocks = self.free.setdefault(size, [])
             if blocks:
                 ptr = blocks.pop()
                 self.kept -= size
             else:
-                gone = self._make_room(size) if size <= self.credit else None
+                lock = size <= self.credit and (before >= 2 or size <= 1 << 20)
+                gone = self._make_room(size) if lock else None
                 if gone is None:
-                    if again:
+                    if before:
                         self.credit = min(self.credit + size, self.LIMIT)
                     return np.empty(shape, dtype)
                 self.credit -= size
