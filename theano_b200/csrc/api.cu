@@ -141,6 +141,7 @@ struct b200conv_ctx {
   std::unordered_map<GeoKey, SlabTile, GeoHash> slab_tiles;
   std::unordered_map<GeoKey, SlabTile, GeoHash> pixel_tiles;
   int force_splits = 0;                     // > 0: use this slice count (tests, tuning by hand)
+  bool model_only = false;                  // choices that are not remembered yet are the models', not timed (rough comparison)
   bool use_pair = true;                     // 1x1 layers with deep reductions on CTA pairs (gemm_pair.cu)
   bool stack_taps = true;                   // grouped gradWeights of narrow layers: taps as column groups of one MMA
   bool autotune = true;
@@ -1004,31 +1005,68 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   return 0;
 }
 
-// Time of one variant in milliseconds (run() enqueues it and returns 0 or an error code).  Short launches are
-// timed in bursts of up to 8 back to back, the way a program issues them: alone, between two events, a kernel
-// of 5 us costs 5 us more and the chained launch hides nothing, and the choice then is noise.
+// Times of `n` variants in milliseconds: run(i) enqueues variant i and returns 0 or a code, which goes to codes[i] and
+// leaves ms[i] at -1.  Returns an error of the timing itself.
+// Every variant runs twice, the second time between two events (the first loads its code and makes the choices inside
+// it); with one exception this decides: variants within a fifth (and the 4 us by which short launches differ between
+// events) of the best are timed again in bursts of up to 8 back to back, the way a program issues them, once, and
+// once more if they are still within 5 %.  Alone, a kernel of 5 us costs 5 us more and the chained launch hides nothing.
+// All variants in two bursts each made the first passes of 32 cases take 200 ms together, this and rough_times() 127.
 template <class Run>
-int time_variant(b200conv_ctx* c, Run run, float* ms) {
+int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool rough = false) {
   if (!c->ev_tune0) {
     CU_OK(c, cudaEventCreate(&c->ev_tune0));
     CU_OK(c, cudaEventCreate(&c->ev_tune1));
   }
-  *ms = -1.f;
-  int reps = 1;
-  for (int round = 0; round < 4; ++round) {               // warm-up, a first estimate, two measurements
+  auto timed = [&](int i, int reps, float* m) -> int {
     CU_OK(c, cudaEventRecord(c->ev_tune0, c->stream));
-    for (int i = 0; i < reps; ++i)
-      if (int rc = run()) return rc;
+    for (int r = 0; r < reps && !codes[i]; ++r) codes[i] = run(i);
     CU_OK(c, cudaEventRecord(c->ev_tune1, c->stream));
     CU_OK(c, cudaStreamSynchronize(c->stream));
-    float m;
-    CU_OK(c, cudaEventElapsedTime(&m, c->ev_tune0, c->ev_tune1));
-    if (round == 1) reps = std::max(1, std::min(8, (int)(0.16f / std::max(m, 0.001f))));
-    if (round >= 2 && (*ms < 0.f || m / reps < *ms)) *ms = m / reps;
-    if (round == 1 && m > 0.5f) { *ms = m; break; }       // long enough for one measurement
+    CU_OK(c, cudaEventElapsedTime(m, c->ev_tune0, c->ev_tune1));
+    *m = codes[i] ? -1.f : *m / reps;
+    return 0;
+  };
+  auto best = [&] {
+    float b = -1.f;
+    for (int i = 0; i < n; ++i)
+      if (ms[i] >= 0.f && (b < 0.f || ms[i] < b)) b = ms[i];
+    return b;
+  };
+  for (int i = 0; i < n; ++i) {
+    ms[i] = -1.f;
+    if ((codes[i] = run(i))) continue;
+    if (int rc = timed(i, 1, &ms[i])) return rc;
+  }
+  const float first = best();
+  if (first < 0.f || first > 0.5f || rough) return 0;     // long enough for one measurement
+  const int reps = std::max(1, std::min(8, (int)(0.16f / std::max(first, 0.001f))));
+  float limit = 1.2f * first + 0.004f;
+  for (int round = 0; round < 2; ++round) {
+    int close = 0;
+    for (int i = 0; i < n; ++i) close += ms[i] >= 0.f && ms[i] <= limit;
+    if (close < 2) return 0;
+    for (int i = 0; i < n; ++i) {
+      if (ms[i] < 0.f || ms[i] > limit) { ms[i] = -1.f; continue; }     // out of the running
+      float m;
+      if (int rc = timed(i, reps, &m)) return rc;
+      ms[i] = round && m >= 0.f ? std::min(ms[i], m) : m;
+    }
+    limit = 1.05f * best();
   }
   return 0;
 }
+
+// Rough times of `n` variants that make choices of their own: those are the models' where none is remembered, each
+// variant runs twice and the second run counts.  A variant far behind in this comparison is not worth its own timings.
+template <class Run>
+int rough_times(b200conv_ctx* c, int n, Run run, float* ms, int* codes) {
+  c->model_only = true;
+  const int rc = time_variants(c, n, run, ms, codes, true);
+  c->model_only = false;
+  return rc;
+}
+constexpr float kFarBehind = 1.4f;
 
 // Picks the kernel variant.  All compute the same thing; which one is fastest depends on the layer (halo
 // rows wasted by the slab grid against activations fetched once per tap; few tiles per SM against a second
@@ -1095,20 +1133,17 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   // later call that may repeat it.
   const size_t out_bytes = elem_size(a.dtype) * out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
   const bool in_place = c->epi.residual && overlap(c->epi.residual, out_bytes, out, out_bytes);
-  if (!c->autotune || c->capturing || ncand == 1 || in_place) return run(cand[ncand - 1]);
-  int best = -1;
-  float best_ms = 0.f;
+  if (!c->autotune || c->capturing || c->model_only || ncand == 1 || in_place) return run(cand[ncand - 1]);
+  int best = -1, codes[kConvVariants];
+  float ms[kConvVariants], best_ms = 0.f;
+  if (const int rc = time_variants(c, ncand, [&](int i) { return run(cand[i]); }, ms, codes)) return rc;
   for (int i = 0; i < ncand; ++i) {
-    float ms;
-    const int rc = time_variant(c, [&] { return run(cand[i]); }, &ms);
-    if (rc == B200CONV_E_UNSUPPORTED && c->epi.pool && ncand > 1) continue;
-    if (rc) return rc;
-    if (ms >= 0.f && (best < 0 || ms < best_ms)) { best = cand[i]; best_ms = ms; }
+    if (codes[i] && !(codes[i] == B200CONV_E_UNSUPPORTED && c->epi.pool)) return codes[i];
+    if (ms[i] >= 0.f && (best < 0 || ms[i] < best_ms)) { best = cand[i]; best_ms = ms[i]; }
   }
   if (best < 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
   c->algo_cache[key] = best;
-  // the last run may have been another variant: leave the output of the chosen one (identical up to rounding order)
-  return best == cand[ncand - 1] ? 0 : run(best);
+  return run(best);     // the last run may have been another variant: leave the output of the chosen one
 }
 
 int to_nhwc(b200conv_ctx* c, Scratch& tmp, const void* src, int N, int C, int H, int W, int dtype,
@@ -1589,14 +1624,19 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       choice = 0;
     }
     if (choice < 0) {
-      float best = 0.f;
-      for (int v = 0; v <= (c->use_pair ? 2 : 1); ++v) {
-        float ms;
-        rc = time_variant(c, [&] { return run(v); }, &ms);
-        if (rc == 2) continue;
-        if (rc) return rc;
-        if (choice < 0 || ms < best) { choice = v; best = ms; }
+      // class by class makes a choice for each class: those are timed only if it is not far behind with the models'
+      float ms[3];
+      int codes[3];
+      const int n = c->use_pair ? 3 : 2;
+      if ((rc = rough_times(c, n, run, ms, codes))) return rc;
+      const float together_ms = n > 2 && ms[2] >= 0.f && (ms[1] < 0.f || ms[2] < ms[1]) ? ms[2] : ms[1];
+      const int lowest = together_ms >= 0.f && ms[0] > kFarBehind * together_ms ? 1 : 0;
+      if ((rc = time_variants(c, n, [&](int v) { return v < lowest ? 2 : run(v); }, ms, codes))) return rc;
+      for (int v = 0; v < n; ++v) {
+        if (codes[v] && codes[v] != 2) return codes[v];
+        if (ms[v] >= 0.f && (choice < 0 || ms[v] < ms[choice])) choice = v;
       }
+      if (choice < 0) choice = 0;
       c->algo_cache[key] = choice;
     }
     rc = run(choice);
@@ -1652,7 +1692,7 @@ int valid_splits(long long pix_tiles, long long s) {
 // The slice count of a gradWeights launch.  The model's choice `s0` is right about the busiest SM's
 // work but knows nothing of the reduction kernel's cost or of L2 effects, so with timing-based
 // selection on, the first call of a geometry also times half and twice that count (main kernel plus
-// reduction, second of two runs each) and the context remembers the fastest; the role the reference's
+// reduction) and the context remembers the fastest; the role the reference's
 // GPU back end gives its meta-optimizer (theano/gpuarray/opt.py:2144-2222).  `run(splits, scratch)`
 // enqueues the launch.  Returns the count, or a negative error code.
 template <class Run>
@@ -1665,20 +1705,21 @@ int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long lo
     if (it != c->split_cache.end()) return it->second;
   }
   const int s0 = (int)balanced_splits(c, pix_tiles, base_items, sms, cap, fixed);
-  if (!c->autotune || c->capturing) return s0;
+  if (!c->autotune || c->capturing || c->model_only) return s0;
   int cand[3] = {s0, valid_splits(pix_tiles, std::min<long long>(cap, std::max(1, s0 / 2))),
                  valid_splits(pix_tiles, std::min<long long>(cap, 2LL * s0))};
-  int best = s0;
-  float best_ms = -1.f;
-  for (int i = 0; i < 3; ++i) {
-    if (i > 0 && (cand[i] == cand[0] || (i == 2 && cand[2] == cand[1]))) continue;
-    float ms;
-    const int rc = time_variant(c, [&] { Scratch trial(c); return run(cand[i], trial); }, &ms);
-    if (rc) return rc < 0 ? rc : -rc;
-    if (best_ms < 0.f || ms < best_ms) { best_ms = ms; best = cand[i]; }
+  int n = 1, best = 0, codes[3];
+  for (int i = 1; i < 3; ++i)
+    if (std::find(cand, cand + n, cand[i]) == cand + n) cand[n++] = cand[i];
+  if (n == 1) return c->split_cache[key] = s0;
+  float ms[3];
+  const int rc = time_variants(c, n, [&](int i) { Scratch trial(c); return run(cand[i], trial); }, ms, codes);
+  if (rc) return rc < 0 ? rc : -rc;
+  for (int i = 0; i < n; ++i) {
+    if (codes[i]) return codes[i] < 0 ? codes[i] : -codes[i];
+    if (ms[i] >= 0.f && (ms[best] < 0.f || ms[i] < ms[best])) best = i;
   }
-  c->split_cache[key] = best;
-  return best;
+  return c->split_cache[key] = cand[best];
 }
 
 GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
@@ -2027,15 +2068,26 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if (itc != c->algo_cache.end()) {
       try_group = itc->second;
     } else if (!c->capturing) {
-      float ms[2] = {0.f, 0.f};
       // own scratch, returned to the pool after each run: the next run then reuses the buffers and its timing
       // holds no allocation
-      rc = time_variant(c, [&] { Scratch trial(c); return wgrad_grouped(c, d, xin, gin, dw, flags, trial); }, &ms[1]);
-      const bool covered = rc != 2;
-      if (covered && rc) return rc;
-      if (covered && (rc = time_variant(c, [&] { return wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC); }, &ms[0])))
+      // Both kernels choose a slice count of their own: that is timed only where they are close with the models'.
+      float ms[2];                                            // 0: tap groups, 1: one tap per item
+      int codes[2];
+      bool covered = true;
+      auto kernel = [&](int v) -> int {
+        if (v) return covered ? wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC) : 2;
+        Scratch trial(c);
+        const int r = wgrad_grouped(c, d, xin, gin, dw, flags, trial);
+        covered = r != 2;
+        return r;
+      };
+      if ((rc = rough_times(c, 2, kernel, ms, codes))) return rc;
+      if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) &&
+          (rc = time_variants(c, 2, kernel, ms, codes)))
         return rc;
-      try_group = covered && ms[1] <= ms[0];
+      for (int code : codes)
+        if (code && code != 2) return code;
+      try_group = ms[0] >= 0.f && (ms[1] < 0.f || ms[0] <= ms[1]);
       c->algo_cache[key] = try_group;
     }
   }
