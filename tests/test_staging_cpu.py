@@ -1,4 +1,6 @@
 """The copy threads of the host-pointer calls (csrc/staging.h), compiled by itself and run on the CPU."""
+import os
+import re
 import subprocess
 
 from theano_b200 import build
@@ -50,3 +52,14 @@ def run(tmp_path, before=""):
 
 def test_copies_and_touches_over_sizes_and_offsets(tmp_path):
     assert run(tmp_path) == "ok"
+
+
+def test_other_processors_copy_with_memcpy(tmp_path):
+    """Without x86 (its macro taken away once the system's headers are in), no x86 header or instruction is needed."""
+    headers = ["stdint.h", "string.h", "sys/mman.h", "atomic", "chrono", "condition_variable", "mutex", "thread"]
+    before = "".join("#include <%s>\n" % h for h in headers) + "#undef __x86_64__\n"
+    assert run(tmp_path, before) == "ok"
+    staging = open(os.path.join(build.CSRC, "staging.h")).read()
+    guarded = staging[staging.index("#if defined(__x86_64__)\ninline"):staging.index("#else")]
+    rest = staging.replace(guarded, "").replace("#if defined(__x86_64__)\n#include <immintrin.h>\n#endif\n", "")
+    assert not re.search(r"_mm_|_mm256_|immintrin|cpuid|__asm__", rest)

@@ -10,8 +10,11 @@
 //  * Waking a sleeping thread costs tens of microseconds, as much as copying a megabyte.  The
 //    calling thread starts on the first piece at once, the workers spin for a moment after a job
 //    before they sleep, and pieces are handed out one by one so that nobody waits for a late one.
+// The streaming and evicting copies are x86 code, chosen by what the processor has; others copy with memcpy.
 #pragma once
+#if defined(__x86_64__)
 #include <immintrin.h>
+#endif
 #include <stdint.h>
 #include <string.h>
 #include <sys/mman.h>
@@ -25,6 +28,9 @@
 #include <vector>
 
 namespace b200 {
+
+#if defined(__x86_64__)
+inline void cpu_relax() { _mm_pause(); }
 
 // memcpy with streaming stores.
 __attribute__((target("avx2"))) inline void copy_streaming_avx2(char* d, const char* s, size_t n) {
@@ -64,15 +70,24 @@ inline bool cpu_has_clflushopt() {
   return (b >> 23) & 1;
 }
 
+inline bool cpu_has_avx2() { return __builtin_cpu_supports("avx2"); }
+#else
+inline void cpu_relax() {}
+inline void copy_streaming_avx2(char* d, const char* s, size_t n) { memcpy(d, s, n); }
+inline void copy_and_evict_clflushopt(char* d, const char* s, size_t n) { memcpy(d, s, n); }
+inline bool cpu_has_clflushopt() { return false; }
+inline bool cpu_has_avx2() { return false; }
+#endif
+
 inline void copy_to_pinned(char* d, const char* s, size_t n) {
-  static const bool avx2 = __builtin_cpu_supports("avx2");
+  static const bool avx2 = cpu_has_avx2();
   if (avx2) copy_streaming_avx2(d, s, n);
   else memcpy(d, s, n);
 }
 // Out of a pinned buffer; into an array beyond the caches with streaming stores, which do not read the lines they
 // overwrite (a call with 616 MB into an array that is used again: 25.7 -> 17.4 ms).
 inline void copy_from_pinned(char* d, const char* s, size_t n, bool large) {
-  static const bool flush = cpu_has_clflushopt(), avx2 = __builtin_cpu_supports("avx2");
+  static const bool flush = cpu_has_clflushopt(), avx2 = cpu_has_avx2();
   if (large && avx2) copy_streaming_avx2(d, s, n);
   else if (flush) copy_and_evict_clflushopt(d, s, n);
   else memcpy(d, s, n);
@@ -122,8 +137,10 @@ class CopyPool {
     const uint32_t pieces = static_cast<uint32_t>((bytes + lead + piece - 1) / piece);
     const uint64_t gen = (ticket_.load(std::memory_order_relaxed) >> 32) + 1;
     // nobody takes a piece while the job is being described: a worker takes one by exchanging the
-    // ticket it has read, so what it read in between belongs to that ticket's job
+    // ticket it has read, so what it read in between belongs to that ticket's job (the two fences: who
+    // has seen any of what follows also sees that the ticket is closed)
     ticket_.store(gen << 32 | 0xffffffffu, std::memory_order_seq_cst);
+    std::atomic_thread_fence(std::memory_order_release);
     dst_.store(static_cast<char*>(dst), std::memory_order_relaxed);
     src_.store(static_cast<const char*>(src), std::memory_order_relaxed);
     bytes_.store(bytes, std::memory_order_relaxed);
@@ -138,7 +155,7 @@ class CopyPool {
       cv_.notify_all();
     }
     work(gen);
-    while (done_.load(std::memory_order_acquire) != pieces) _mm_pause();
+    while (done_.load(std::memory_order_acquire) != pieces) cpu_relax();
   }
 
   void work(uint64_t gen) {
@@ -150,6 +167,7 @@ class CopyPool {
       const uint32_t pieces = pieces_.load(std::memory_order_relaxed);
       const size_t piece = piece_.load(std::memory_order_relaxed), lead = lead_.load(std::memory_order_relaxed);
       const Kind kind = kind_.load(std::memory_order_relaxed);
+      std::atomic_thread_fence(std::memory_order_acquire);
       const uint32_t i = static_cast<uint32_t>(t);
       if (t >> 32 != gen || i >= pieces) return;
       if (!ticket_.compare_exchange_strong(t, t + 1, std::memory_order_acq_rel)) continue;
@@ -169,7 +187,7 @@ class CopyPool {
       do {
         for (int k = 0; k < 32 && !fresh; ++k) {
           fresh = posted() != seen;
-          if (!fresh) _mm_pause();
+          if (!fresh) cpu_relax();
         }
       } while (!fresh && !stop_.load(std::memory_order_relaxed) && std::chrono::steady_clock::now() < until);
       if (!fresh) {
