@@ -24,6 +24,7 @@
 #include <chrono>
 #include <condition_variable>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -107,8 +108,13 @@ inline void touch_pages(char* d, size_t n) {
 // context's lock).
 class CopyPool {
  public:
+  // Fewer threads where the system gives no more: the caller alone copies everything, too.
   explicit CopyPool(int nthreads) {
-    for (int i = 1; i < nthreads; ++i) workers_.emplace_back([this] { loop(); });
+    workers_.reserve(nthreads);
+    try {
+      for (int i = 1; i < nthreads; ++i) workers_.emplace_back([this] { loop(); });
+    } catch (const std::system_error&) {
+    }
   }
   ~CopyPool() {
     {
