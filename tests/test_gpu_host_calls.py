@@ -89,6 +89,23 @@ def test_a_result_may_lie_over_the_input(start, c, page_locked):
 
 
 @pytest.mark.gpu
+def test_host_calls_without_a_staging_ring(monkeypatch):
+    """No copy threads, or no page-locked memory for the ring: small and large arrays travel the driver's way."""
+    monkeypatch.setenv("B200CONV_COPY_THREADS", "0")
+    ctx = shim.Context(0)
+    rs = np.random.RandomState(2)
+    kw = dict(border_mode="half", subsample=(1, 1))
+    for n, h in ((2, 9), (12, 96)):                          # 3 KB, and 14 MB in chunks
+        x = rs.standard_normal((n, 32, h, h)).astype(np.float32)
+        w = (rs.standard_normal((32, 32, 3, 3)) / 17).astype(np.float32)
+        out = np.full(x.shape, 7, np.float32)
+        assert O.rel_err(shim.conv2d_forward(x, w, out=out, ctx=ctx, **kw), O.conv2d(x, w, **kw)) < 5e-3
+        assert O.rel_err(shim.conv2d_grad_inputs(w, x, ctx=ctx, **kw), O.conv2d_grad_inputs(w, x, (h, h), **kw)) < 5e-3
+        assert O.rel_err(shim.conv2d_grad_weights(x, x, (3, 3), ctx=ctx, **kw), O.conv2d_grad_weights(x, x, (3, 3), **kw)) < 5e-3
+    ctx.close()
+
+
+@pytest.mark.gpu
 def test_a_capture_refuses_host_calls_and_leaves_the_staging_ring_alone():
     """An event of the ring recorded in a capture could not be waited for by the calls that come after it."""
     ctx = shim.Context(0)

@@ -152,6 +152,7 @@ struct b200conv_ctx {
   int comm_timeout_ms = 60000;              // host watchdog of streams that carry collectives
   // pinned ring of the host-pointer calls (made on first use); every such call ends with all slots free
   char* ring = nullptr;
+  bool no_ring = false;                     // there is no memory for it
   cudaEvent_t ring_ev[kRingSlots] = {};
   bool ring_busy[kRingSlots] = {};
   int ring_next = 0;
@@ -2179,24 +2180,26 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
 }
 
 // ---- host-pointer wrappers: copy in, run, copy out, synchronise ---------------------------
-int ring_setup(b200conv_ctx* c) {
-  if (c->copy_pool) return 0;
-  if (!c->ring) {
-    void* p = nullptr;
-    cudaError_t e = cudaHostAlloc(&p, kRingSlotBytes * kRingSlots, cudaHostAllocDefault);
-    c->ring = static_cast<char*>(p);
-    for (int i = 0; i < kRingSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&c->ring_ev[i], cudaEventDisableTiming);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(c, B200CONV_E_NOMEM, "pinned staging buffers: %s", cudaGetErrorString(e));
-    }
-  }
+// Makes the ring on first use.  False where the system gives no page-locked memory for it, or with no copy threads
+// asked for: pageable arrays then travel at the pace of the driver's own staging.
+bool ring_ready(b200conv_ctx* c) {
+  if (c->copy_pool || c->no_ring) return c->copy_pool != nullptr;
   const char* env = getenv("B200CONV_COPY_THREADS");
   const int cores = (int)std::thread::hardware_concurrency();
   // 16 MB into pinned memory: 1069 / 615 / 331 / 218 / 237 us with 1 / 2 / 4 / 8 / 12 threads (link: 310 us)
-  int n = env ? atoi(env) : std::min(8, std::max(2, cores / 2));
-  c->copy_pool = new CopyPool(std::max(1, std::min(n, 16)));
-  return 0;
+  const int n = env ? atoi(env) : std::min(8, std::max(2, cores / 2));
+  void* p = nullptr;
+  cudaError_t e = n <= 0 ? cudaErrorMemoryAllocation : cudaHostAlloc(&p, kRingSlotBytes * kRingSlots, cudaHostAllocDefault);
+  for (int i = 0; i < kRingSlots && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&c->ring_ev[i], cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    if (p) cudaFreeHost(p);
+    cudaGetLastError();
+    c->no_ring = true;
+    return false;
+  }
+  c->ring = static_cast<char*>(p);
+  c->copy_pool = new CopyPool(std::min(n, 16));
+  return true;
 }
 
 // A free slot of the ring (waits for the transfer that used it last).
@@ -2231,12 +2234,11 @@ bool is_pinned(const void* h, size_t bytes) {
 
 // Host array -> device memory on stream s.  The array may be reused when this returns unless it is pinned.
 int upload(b200conv_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s, bool pinned) {
-  if (pinned) {
+  if (pinned || !ring_ready(c)) {
     CU_OK(c, cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
     return 0;
   }
-  int rc = ring_setup(c);
-  if (rc) return rc;
+  int rc;
   for (size_t off = 0, n; off < bytes; off += n) {
     n = chunk_bytes(off, bytes);
     int k;
@@ -2253,12 +2255,11 @@ int upload(b200conv_ctx* c, void* d, const void* h, size_t bytes, cudaStream_t s
 // one when this returns: chunks travel into ring slots, up to half a ring ahead of the copy threads
 // that empty them.
 int download(b200conv_ctx* c, void* h, const void* d, size_t bytes, cudaStream_t s, bool pinned) {
-  if (pinned) {
+  if (pinned || !ring_ready(c)) {
     CU_OK(c, cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, s));
     return 0;
   }
-  int rc = ring_setup(c);
-  if (rc) return rc;
+  int rc;
   // Large arrays are likely to be fresh memory: while the transfers of a window fly, the threads make its pages present.
   constexpr size_t kTouchFrom = 4u << 20, kTouchWindow = 16u << 20, kLargeArray = 64u << 20;
   size_t touched = bytes >= kTouchFrom ? 0 : bytes;
@@ -2321,14 +2322,14 @@ struct HostIO {
   // A small input joins the group (start() sends it), a larger one is on its way when this returns.
   int in(const void* h, size_t bytes, void** d) {
     int rc;
-    if (bytes <= kSmallInput) {
+    if (bytes <= kSmallInput && ring_ready(c)) {
       if ((rc = small_space(bytes, d))) return rc;
       memcpy(group_host + (static_cast<char*>(*d) - group_dev), h, bytes);
       return 0;
     }
     // the ring turns under a large input, so the slot of a waiting group has to be on its way first
     if ((rc = start()) || (rc = tmp.get(bytes, d))) return rc;
-    return upload(c, *d, h, bytes, c->stream, is_pinned(h, bytes));
+    return bytes ? upload(c, *d, h, bytes, c->stream, is_pinned(h, bytes)) : 0;
   }
   int start() {
     if (!group_dev) return 0;
@@ -2348,7 +2349,7 @@ struct HostIO {
   int small_space(size_t bytes, void** d) {
     int rc;
     if (!group_dev) {
-      if ((rc = ring_setup(c)) || (rc = ring_slot(c, &group_slot))) return rc;
+      if ((rc = ring_slot(c, &group_slot))) return rc;
       void* p;
       if ((rc = tmp.get(4 * (kSmallInput + 256), &p))) return rc;      // at most four inputs per call
       group_dev = static_cast<char*>(p);
