@@ -206,3 +206,49 @@ def test_stems_off_the_boundary(ctx, dtype, xs, k, ks, s):
         DXs, owner2 = shifted(X, 7)
         assert np.array_equal(stored(shim.device_grad_inputs(W, DY, xs[2:], out=DXs, **kw)), stored(DX))
         assert not stored(DXs)[..., xs[1]:].any()
+
+
+def test_split_reductions_fall_back_to_whole_ones_without_memory_for_slices():
+    """A 1x1 forward call on channels-last tensors needs no scratch but the slices of a split reduction (4 MB and more
+    here); with the device's memory taken, it runs unsplit."""
+    rs = np.random.RandomState(9)
+    x = rs.standard_normal((1, 2048, 14, 14)).astype(np.float32)
+    w = (rs.standard_normal((512, 2048, 1, 1)) / 45).astype(np.float32)
+    c = shim.Context(0)
+    c.set_autotune(False)
+    c.set_pair_kernels(False)
+    # the kernels' code is on the device before its memory is taken: split and whole, with both kernels
+    many = T(c, (64, 2048, 14, 14), np.float32, "nhwc")
+    W = T.from_host(c, w)
+    for flags in (0, shim.NO_SLAB):
+        for X in (T.from_host(c, x, "nhwc"), many):
+            shim.device_conv2d(X, W, flags=flags)
+    c.sync()
+    c.close()
+    c = shim.Context(0)
+    c.set_autotune(False)
+    c.set_pair_kernels(False)
+    X, W, Y = T.from_host(c, x, "nhwc"), T.from_host(c, w), T(c, (1, 512, 14, 14), np.float32, "nhwc")
+    want = O.conv2d(x, w)
+    taken, size = [], 256 << 30
+    while size >= 2 << 20:
+        try:
+            taken.append(T(c, (1, 1, 1, size // 4), np.float32))
+        except (MemoryError, shim.B200Error):
+            size //= 2
+    try:
+        free = c.memory_info()[1]
+        assert free < 4 << 20, free
+        for flags in (0, shim.NO_SLAB):
+            before = c.launches
+            shim.device_conv2d(X, W, out=Y, flags=flags)
+            assert c.launches - before == 1                              # no second kernel that adds slices
+        c.sync()
+    finally:
+        for t in taken:
+            t.free()
+    assert O.rel_err(Y.to_host(), want) < 5e-3
+    before = c.launches
+    shim.device_conv2d(X, W, out=Y)
+    assert c.launches - before == 2                                      # with memory again: split
+    c.close()

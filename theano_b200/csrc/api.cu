@@ -1080,13 +1080,19 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                   long long sn, long long sc, long long sh, long long sw, long long off,
                   const void* bias, int relu, bool allow_slab = true) {
   if (view_parity.size() != 1) allow_slab = false;
-  auto run = [&](int variant) -> int {
+  auto run_one = [&](int variant) -> int {
     if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
       const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
                                    relu, slab_mode(variant));
       return rc == 2 ? fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool") : rc;
     }
     return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant);
+  };
+  auto run = [&](int variant) -> int {
+    const int rc = run_one(variant);
+    // no memory for the slices of a split reduction: whole reductions need none
+    if (rc != B200CONV_E_NOMEM || (variant != kConvSlabSpread && variant != kConvTapSpread)) return rc;
+    return run_one(variant == kConvSlabSpread ? kConvSlab : kConvTap);
   };
   int tsum = 0;
   for (const ConvTap& t : taps_in) tsum = tsum * 31 + t.dh * 7 + t.dw;
