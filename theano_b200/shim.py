@@ -598,15 +598,30 @@ def make_desc(xshape, wshape, yshape, pads, subsample, dilation, groups, flip, d
     return d
 
 
+def _same(a, b):
+    """Equal, and of the same types: 1.0 == 1 == True, but not all of them are accepted everywhere."""
+    if a is b:
+        return True
+    return type(a) is type(b) and (len(a) == len(b) and all(map(_same, a, b)) if type(a) is tuple else a == b)
+
+
 class _Plans(dict):
     """Results of the pure shape logic per call signature: (result shape, pads or kernel shape, descriptor
     reference).  A training loop repeats a few signatures for ever, and working them out again cost as
-    much host time as the launches.  Bounded: emptied when it holds LIMIT signatures."""
+    much host time as the launches.  Bounded: emptied when it holds LIMIT signatures.
+
+    A signature ends in border mode, strides, dilation, groups, flip and dtype.  A hit counts only if those are
+    of the types that the plan was made for (the very objects, as a rule), so that what the shape logic refuses
+    (a float border mode, float strides) is refused whatever equal integers were seen before."""
     LIMIT = 4096
 
     def find(self, make, *sig):
         try:
-            return self[sig]
+            made, plan = self[sig]
+            if made[-3] is sig[-3] and made[-4] is sig[-4] and made[-5] is sig[-5] and made[-6] is sig[-6]:
+                return plan
+            if _same(made[-6:-2], sig[-6:-2]):
+                return plan
         except KeyError:
             pass
         except TypeError:                # a list among the arguments: not remembered
@@ -614,7 +629,7 @@ class _Plans(dict):
         plan = make(*sig[1:])
         if len(self) >= self.LIMIT:
             self.clear()
-        self[sig] = plan
+        self[sig] = sig, plan
         return plan
 
 
