@@ -144,3 +144,44 @@ def test_large_host_arrays_travel_through_the_pinned_staging(ctx):
     xh = x.astype(np.float16)
     yh = shim.conv2d_forward(xh, w.astype(np.float16), ctx=ctx, **kw)
     assert O.rel_err(yh.astype(np.float32), O.conv2d(xh.astype(np.float32), w.astype(np.float16).astype(np.float32), **kw)) < 2e-2
+
+
+def test_range_checked_build_passes_the_later_kernels():
+    """The same for split reductions (their slabs and the kernel that adds them), pairs of CTAs, classes of strided
+    gradInputs, stacked taps, merged groups and the memory-bound kernels."""
+    import os
+    import subprocess
+    import sys
+    from theano_b200 import build as lib_build
+    lib = lib_build.DEBUG_LIB
+    if not os.path.exists(lib):
+        pytest.skip("libb200conv_debug.so is not built (python -m theano_b200.build --debug)")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    files = ["test_gpu_split_reductions.py", "test_gpu_slab_pairs.py", "test_gpu_strided_grad_inputs.py", "test_gpu_stacked_taps.py",
+             "test_group_merging.py", "test_gpu_memory_kernels.py", "test_gpu_in_place_residual.py"]
+    r = subprocess.run([sys.executable, "-m", "pytest", "-x", "-q", "-m", "gpu", "-p", "no:cacheprovider"] +
+                       [os.path.join(root, "tests", f) for f in files],
+                       cwd=root, env=dict(os.environ, B200CONV_LIB=lib), capture_output=True, text=True, timeout=900)
+    assert r.returncode == 0, r.stdout[-3000:] + r.stderr[-1000:]
+
+
+@pytest.mark.parametrize("layout", ["nhwc", "nchw"])
+def test_split_reductions_write_nothing_outside_the_output(ctx, layout):
+    """Few output tiles: an output framed by canary bytes, written by the kernel that adds the slices."""
+    rs = np.random.RandomState(12)
+    x = rs.standard_normal((1, 512, 9, 7)).astype(np.float32)
+    w = (rs.standard_normal((75, 512, 3, 3)) / 68).astype(np.float32)
+    own = shim.Context(0)
+    own.set_autotune(False)                       # the model's choice, split here
+    X, W = shim.DeviceTensor.from_host(own, x, "nhwc"), shim.DeviceTensor.from_host(own, w)
+    for flags in (0, shim.NO_SLAB):
+        probe = shim.DeviceTensor(own, (1, 75, 9, 7), np.float32, layout)
+        base, ptr = _framed(own, probe.nbytes)
+        out = shim.DeviceTensor(own, (1, 75, 9, 7), np.float32, layout, _ptr=ptr)
+        before = own.launches
+        shim.device_conv2d(X, W, border_mode="half", out=out, out_layout=layout, flags=flags)
+        assert own.launches - before == 3                       # packing, convolution, sum of the slices
+        assert _canaries_intact(own, base, probe.nbytes)
+        assert O.rel_err(out.to_host(), O.conv2d(x, w, border_mode="half")) < 5e-3
+        own.free(base)
+    own.close()

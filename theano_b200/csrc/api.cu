@@ -706,13 +706,19 @@ SlabTile tap_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int 
 
 // Slabs of a split launch and the parameters of its reduction that both kernels share.
 template <class P>
-int split_output(b200conv_ctx* c, Scratch& tmp, const P& p, int bn, int rows, ConvReduceParams* q) {
+int split_output(b200conv_ctx* c, Scratch& tmp, P& p, int bn, int rows, ConvReduceParams* q) {
   memset(q, 0, sizeof *q);
   const long long tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
   float* partial;
-  int rc = tmp.get(sizeof(float) * tiles * p.splits * rows * bn, reinterpret_cast<void**>(&partial));
+  const long long elems = tiles * p.splits * rows * bn;
+  int rc = tmp.get(sizeof(float) * elems, reinterpret_cast<void**>(&partial));
   if (rc) return rc;
-  q->partial = partial;
+  q->partial = p.partial = partial;
+  q->partial_elems = p.partial_elems = elems;
+  const int pl = p.epi.pool ? 2 : 1;
+  q->out_elems = p.out_off + (p.Nimg - 1) * p.out_sn + (p.Ht / pl - 1) * p.out_sh + (p.Wt / pl - 1) * p.out_sw +
+                 (1LL * p.n_out * p.groups - 1) * p.out_sc + 1;
+  q->status = p.status;
   q->splits = p.splits; q->rows = rows; q->bn_cols = bn;
   q->tiles_w = p.tiles_w; q->tiles_h = p.tiles_h; q->tiles_n = p.tiles_n; q->tiles_co = p.tiles_co; q->groups = p.groups;
   q->Wt = p.Wt; q->Ht = p.Ht; q->Nimg = p.Nimg; q->n_out = p.n_out; q->n_real = p.n_real;
@@ -927,7 +933,6 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   ConvReduceParams q;
   if ((rc = split_output(c, tmp, p, BN, p.n_acc * 128, &q))) return rc;
   q.Ws = p.Ws; q.Hs = p.Hs; q.wt = p.wt; q.th = p.th; q.nb = p.nb;
-  p.partial = const_cast<float*>(q.partial);
   KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
   KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
   return 0;
@@ -1000,7 +1005,6 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   ConvReduceParams q;
   if ((rc = split_output(c, tmp, p, BN, 128, &q))) return rc;
   q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
-  p.partial = const_cast<float*>(q.partial);
   KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
   KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
   return 0;

@@ -9,6 +9,7 @@
 // result does not depend on scheduling), applies the epilogue and writes the output.  It is bound by the
 // latency of its loads (all slices of a thread are in flight together) and runs on all SMs.
 #include "internal.h"
+#include "ptx.cuh"
 
 namespace b200 {
 namespace {
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const __grid_constant_
   float best[4];
   for (int k = 0; k < pl * pl; ++k) {
     const int row = (ni * p.Hs + hh * pl + (k >> 1)) * p.Ws + ww * pl + (k & 1);
+    if (!B200_IN_RANGE((reinterpret_cast<const float*>(base + row + (p.splits - 1) * slab) - p.partial) + 4 <= p.partial_elems, p.status)) return;
     const float4 a = sum_slices(base + row, p.splits, slab);
     const float v[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
@@ -64,6 +66,8 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const __grid_constant_
       best[e] = k == 0 ? f : fmaxf(best[e], f);
     }
   }
+  const long long at = out - static_cast<T*>(p.out), last = at + ((c0 + 4 < p.n_out ? 4 : p.n_out - c0) - 1) * p.out_sc;
+  if (!B200_IN_RANGE(at >= 0 && last < p.out_elems, p.status)) return;
   if (p.out_sc == 1 && ((p.n_out * sizeof(T) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0) { // four columns are all in
     if (sizeof(T) == 4) {
       *reinterpret_cast<float4*>(out) = make_float4(best[0], best[1], best[2], best[3]);

@@ -325,8 +325,9 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             if (!inbox) continue;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              dst[(ch * 8 + j) * rows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                                     __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+              if (B200_IN_RANGE((reinterpret_cast<float*>(dst + (ch * 8 + j) * rows) - p.partial) + 4 <= p.partial_elems, p.status))
+                dst[(ch * 8 + j) * rows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                       __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
           }
         }
       } else if (p.tma_out) {

@@ -223,8 +223,9 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
           if (!valid) continue;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            dst[(ch * 8 + j) * kRows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                                    __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+            if (B200_IN_RANGE((reinterpret_cast<float*>(dst + (ch * 8 + j) * kRows) - p.partial) + 4 <= p.partial_elems, p.status))
+              dst[(ch * 8 + j) * kRows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                                      __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
         }
       } else
 #pragma unroll 1

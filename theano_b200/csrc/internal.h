@@ -112,6 +112,7 @@ struct alignas(64) UmmaConvParams {
   int bn_cols;                   // accumulator columns of a tile (32, 64, 128 or 256)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
   float* partial;
+  long long partial_elems;       // elements of `partial` (checked in the range-checked build)
   int groups;
   int Wt, Ht, Nimg;              // extent of the output pixel grid this launch covers
   int bw, bh, bn;                // pixel tile (bw*bh*bn <= 128 rows of the accumulator)
@@ -160,6 +161,7 @@ struct alignas(64) SlabConvParams {
   int s_stages;                  // slab ring depth (2 .. 6)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
   float* partial;
+  long long partial_elems;       // elements of `partial` (checked in the range-checked build)
   int pair;                      // 1: CTA pairs (two pixel tiles side by side, M = 256); splits is 1
   int tap_boxes;                 // 1: one TMA box per tap; 0: the taps of a stage are neighbours in the packed filters
                                  // and arrive as one box (the map's box then is tps matrices deep)
@@ -204,6 +206,8 @@ struct ConvReduceParams {
   long long out_sn, out_sc, out_sh, out_sw, out_off;
   int relu;
   ConvEpilogue epi;
+  long long partial_elems, out_elems;      // of `partial` and of `out` that this launch may touch (range-checked build)
+  int* status;
 };
 cudaError_t launch_conv_reduce(const ConvReduceParams& p, int dtype, cudaStream_t s);
 
