@@ -308,6 +308,10 @@ int b200conv_set_wait_limit(b200conv_ctx* ctx, long long clocks);
 int b200conv_selftest_wait(b200conv_ctx* ctx);
 /* Name of the kernel family the last fwd/dgrad/wgrad call used: "umma" or "direct". */
 const char* b200conv_last_algo(b200conv_ctx* ctx);
+/* The kernel variant of the last tensor-core launch of a forward or gradInputs call: "tap", "tap split", "slab", "slab split",
+ * "slab pair", "slab classes", "slab classes pair" or "gemm pair" (split: the reduction in slices that a second kernel adds;
+ * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch). */
+const char* b200conv_last_variant(b200conv_ctx* ctx);
 /* Writes `bytes` of device scratch to evict the L2 cache between timed iterations. */
 int b200conv_flush_l2(b200conv_ctx* ctx);
 

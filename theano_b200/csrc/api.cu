@@ -108,6 +108,7 @@ struct b200conv_ctx {
   cudaEvent_t ev_tune0 = nullptr, ev_tune1 = nullptr;   // kernel selection timing
   long long launches = 0;
   const char* last_algo = "none";
+  const char* last_variant = "none";        // kernel variant of the last forward / gradInputs launch
   // optional per-kernel timing: an event pair around every launch of our own kernels
   bool prof = false;
   struct ProfRec { int kind; cudaEvent_t a, b; };
@@ -787,6 +788,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       q.bias = bias; q.relu = relu; q.epi = c->epi;
       q.status = c->d_status;
       q.wait_clocks = c->wait_clocks;
+      c->last_variant = "gemm pair";
       KLAUNCH(c, kKConvUmma, launch_gemm_pair(q, c->num_sms, c->stream));
       return 0;
     }
@@ -925,6 +927,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
             Wt, Ht, a.N, a.Cin_g, a.n_out, (int)taps.size(), BN, p.splits, p.wt, p.th, p.nb, p.n_acc, p.slab_bytes, p.s_stages, p.b_stages,
             p.tma_out, p.stage_nbuf);
 #endif
+  c->last_variant = p.ncls > 1 ? (pair ? "slab classes pair" : "slab classes") : pair ? "slab pair" : p.splits > 1 ? "slab split" : "slab";
   if (p.splits == 1) {
     KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
     return 0;
@@ -997,6 +1000,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.epi = c->epi;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
+  c->last_variant = p.splits > 1 ? "tap split" : "tap";
   if (p.splits == 1) {
     KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
     return 0;
@@ -3171,6 +3175,7 @@ int b200conv_kernel_time(b200conv_ctx* c, const char* name, float* total_ms, int
   return 0;
 }
 const char* b200conv_last_algo(b200conv_ctx* c) { return c ? c->last_algo : "none"; }
+const char* b200conv_last_variant(b200conv_ctx* c) { return c ? c->last_variant : "none"; }
 
 int b200conv_flush_l2(b200conv_ctx* c) {
   if (!c) return B200CONV_E_INVALID;

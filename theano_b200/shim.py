@@ -93,6 +93,7 @@ SIGNATURES = {
     "b200conv_set_wait_limit": (_I, [_P, ctypes.c_longlong]),
     "b200conv_selftest_wait": (_I, [_P]),
     "b200conv_last_algo": (ctypes.c_char_p, [_P]),
+    "b200conv_last_variant": (ctypes.c_char_p, [_P]),
     "b200conv_flush_l2": (_I, [_P]),
     "b200conv_nccl_unique_id": (_I, [_P, _P]),
     "b200conv_nccl_init": (_I, [_P, _I, _I, _P]),
@@ -298,6 +299,11 @@ class Context(object):
     @property
     def last_algo(self):
         return self.lib.b200conv_last_algo(self.h).decode()
+
+    @property
+    def last_variant(self):
+        """Kernel variant of the last forward or gradInputs launch ("tap", "slab pair", ...; see the header)."""
+        return self.lib.b200conv_last_variant(self.h).decode()
 
     def padded_channels(self, c, dtype):
         return int(self.lib.b200conv_padded_channels(int(c), _dtype_code(dtype)))
