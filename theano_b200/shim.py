@@ -489,7 +489,7 @@ class _ResultPool(object):
     def __init__(self):
         self.free = {}                   # size class -> addresses
         self.asked = {}                  # size class -> number of the last result of that class
-        self.count = {}                  # size class -> results of it before that, each within STALE of the next
+        self.count = {}                  # size class -> results of it that found no block, within STALE of the last
         self.lock = threading.RLock()
         self.total = self.kept = 0       # bytes out or kept / kept
         self.results = 0
@@ -517,6 +517,28 @@ class _ResultPool(object):
             self.kept -= s
         return [self.free[s].pop() for s, _ in gone]
 
+    def _lock_memory(self, ctx, size):
+        """New page-locked memory, or None: an ordinary array has to do."""
+        with self.lock:
+            before = self.count.get(size, 0) if self.asked.get(size, -self.STALE) > self.results - self.STALE else 0
+            self.asked[size], self.count[size] = self.results, before + 1
+            lock = size <= self.credit and (before >= 2 or size <= 1 << 20)
+            gone = self._make_room(size) if lock else None
+            if gone is None:
+                if before:
+                    self.credit = min(self.credit + size, self.LIMIT)
+                return None
+            self.credit -= size
+            self.total += size
+        for old in gone:
+            load_library().b200conv_host_free(None, _P(old))
+        p = _P()
+        if ctx.lib.b200conv_host_alloc(ctx.h, size, ctypes.byref(p)) != 0:
+            with self.lock:
+                self.total -= size
+            return None
+        return p.value
+
     def empty(self, ctx, shape, dtype, smallest=SMALLEST):
         n = dtype.itemsize
         for s in shape:
@@ -524,33 +546,17 @@ class _ResultPool(object):
         if n < smallest or n > self.LIMIT:
             return np.empty(shape, dtype)
         size = self.size_class(n)
-        ptr, gone = None, []
         with self.lock:
             self.results += 1
-            before = self.count.get(size, 0) if self.asked.get(size, -self.STALE) > self.results - self.STALE else 0
-            self.asked[size], self.count[size] = self.results, before + 1
-            blocks = self.free.setdefault(size, [])
-            if blocks:
-                ptr = blocks.pop()
+            blocks = self.free.get(size)
+            ptr = blocks.pop() if blocks else None
+            if ptr is not None:
                 self.kept -= size
-            else:
-                lock = size <= self.credit and (before >= 2 or size <= 1 << 20)
-                gone = self._make_room(size) if lock else None
-                if gone is None:
-                    if before:
-                        self.credit = min(self.credit + size, self.LIMIT)
-                    return np.empty(shape, dtype)
-                self.credit -= size
-                self.total += size
-        for old in gone:
-            load_library().b200conv_host_free(None, _P(old))
+                self.asked[size] = self.results
         if ptr is None:
-            p = _P()
-            if ctx.lib.b200conv_host_alloc(ctx.h, size, ctypes.byref(p)) != 0:
-                with self.lock:
-                    self.total -= size
+            ptr = self._lock_memory(ctx, size)
+            if ptr is None:
                 return np.empty(shape, dtype)
-            ptr = p.value
         block = _PinnedBlock(self, ptr, size)
         block.__array_interface__ = {"version": 3, "shape": shape, "typestr": dtype.str, "data": (ptr, False)}
         return np.asarray(block)
