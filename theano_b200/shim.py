@@ -610,8 +610,17 @@ def make_desc(xshape, wshape, yshape, pads, subsample, dilation, groups, flip, d
     return d
 
 
+def _plain(border_mode, strides, dilation, groups, *_):
+    """Whether these are what most calls pass: a name, an int or two as the border mode, and ints.  Of two equal
+    signatures (1.0 == 1 == True) that are both plain, neither holds anything the other does not."""
+    t = type(border_mode)
+    return ((t is str or t is int or t is tuple and type(border_mode[0]) is int and type(border_mode[1]) is int)
+            and type(strides[0]) is int and type(strides[1]) is int and type(dilation[0]) is int and type(dilation[1]) is int
+            and type(groups) is int)
+
+
 def _same(a, b):
-    """Equal, and of the same types: 1.0 == 1 == True, but not all of them are accepted everywhere."""
+    """Equal, and of the same types."""
     if a is b:
         return True
     return type(a) is type(b) and (len(a) == len(b) and all(map(_same, a, b)) if type(a) is tuple else a == b)
@@ -629,10 +638,10 @@ class _Plans(dict):
 
     def find(self, make, *sig):
         try:
-            made, plan = self[sig]
-            if made[-3] is sig[-3] and made[-4] is sig[-4] and made[-5] is sig[-5] and made[-6] is sig[-6]:
+            made, plain, plan = self[sig]
+            if made[-4] is sig[-4] and made[-5] is sig[-5] and made[-6] is sig[-6] and made[-3] is sig[-3]:
                 return plan
-            if _same(made[-6:-2], sig[-6:-2]):
+            if plain and _plain(*sig[-6:]) or _same(made[-6:-2], sig[-6:-2]):
                 return plan
         except KeyError:
             pass
@@ -641,7 +650,7 @@ class _Plans(dict):
         plan = make(*sig[1:])
         if len(self) >= self.LIMIT:
             self.clear()
-        self[sig] = sig, plan
+        self[sig] = sig, _plain(*sig[-6:]), plan
         return plan
 
 
