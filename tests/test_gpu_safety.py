@@ -128,9 +128,9 @@ def test_range_checked_build_passes_the_small_matrix():
 
 
 def test_large_host_arrays_travel_through_the_pinned_staging(ctx):
-    """Host-pointer calls with arrays beyond 4 MB are cut into 16 MB chunks that copy threads move
-    through pinned buffers while the DMA engine works on the previous chunk; sizes here are no
-    multiple of the chunk, and every direction must still equal the oracle."""
+    """Host-pointer calls with arrays beyond 64 KB travel in chunks of up to 2 MB through a ring of pinned slots that copy
+    threads fill and empty while the DMA engine works on other slots; sizes here are no multiple of a slot, and every
+    direction must still equal the oracle."""
     rs = np.random.RandomState(21)
     x = rs.standard_normal((37, 48, 50, 50)).astype(np.float32)            # 17.8 MB
     w = (rs.standard_normal((80, 48, 3, 3)) * 0.05).astype(np.float32)

@@ -63,3 +63,24 @@ def test_split_layers_run_split(ctx, dtype):
     for flags, variant in ((0, "slab split"), (shim.NO_SLAB, "tap split")):
         shim.device_conv2d(X, W, border_mode="half", flags=flags)
         assert ctx.last_variant == variant
+
+
+def test_choices_of_a_file_hold_for_the_switch_they_were_made_with(tmp_path):
+    """A file that names pairs for a geometry does not bring them to a context that has them switched off."""
+    path = str(tmp_path / "tuning")
+    xs, ws = (40, 512, 14, 14), (512, 512, 3, 3)
+    for step in ("make", "on", "off"):
+        c = shim.Context(0)
+        X, W = T(c, xs, np.float32, "nhwc"), T(c, ws, np.float32)
+        if step != "make":
+            c.set_pair_kernels(step == "on")
+            assert c.tuning_load(path) == 1
+        shim.device_conv2d(X, W, border_mode="half")
+        if step == "make":
+            c.tuning_save(path)
+            head, line = open(path).read().splitlines()
+            open(path, "w").write("\n".join([head, " ".join(line.split()[:2] + ["4"])]) + "\n")      # pairs, whatever was faster
+        else:
+            shim.device_conv2d(X, W, border_mode="half")
+            assert (c.last_variant == "slab pair") == (step == "on")
+        c.close()

@@ -599,7 +599,8 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
       const long long tiles = cdiv(Wt, wt) * cdiv(Ht, th) * cdiv(a.N, nb);
       const long long total = (pair ? cdiv(tiles, 2) : tiles) * tiles_co * a.groups;
       // Clocks of the busiest SM: per tile and (tap, channel block) 4 MMAs per accumulator plus
-      // about 120 clocks of stage hand-over in the issuing thread; then the accumulators are read
+      // 120 clocks of stage hand-over in the issuing thread (190 were measured, see slab_tps; with either
+      // number 24 layers of 64 to 512 channels get tiles of the same speed); then the accumulators are read
       // out, beside the next tile's MMAs when two accumulator sets fit the 512 TMEM columns.
       // Epilogue: through staged TMA stores when the output is channels-last and the staging
       // buffers fit beside two slabs and two filter stages (about 2500 clocks of latency per tile
@@ -615,6 +616,9 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
                            (total <= units ? ngr * stg <= 2 * slab_bytes + 2 * b_bytes
                                                 : 2 * slab_bytes + min_b * b_bytes + kSlabStageBytes <= kSlabSmemBudget);
       // plus about 1500 clocks per tile for the pipeline to fill again
+      // A pair's only accumulator of at most 128 columns is charged 96 clocks: its MMAs follow one another into the same
+      // columns, and the search then prefers two accumulators.  With the 64 of mma_clocks(): 512 -> 512 3x3 at 14x14,
+      // 128 images, 184.7 -> 234.6 us in float32 and 100 -> 122 in float16; 128 -> 128 at 28x28 float32 63 -> 79.
       const int mma_clk = pair && n_acc * ncls == 1 && BN <= 128 ? 96 : mma_clocks(BN);
       auto mma_part = [&](long long st) { return st * (1LL * std::min(tps, ntaps) * 4 * n_acc * mma_clk + 120) + 1500; };
       const long long whole = 1LL * kblocks_n * (ntaps * 4LL * n_acc * mma_clk + cdiv(ntaps, tps) * 120) + 1500;

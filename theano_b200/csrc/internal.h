@@ -66,6 +66,8 @@ template <class... Exp, class... Act>
 cudaError_t launch_chained(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
   return launch_linked(true, kernel, grid, block, smem, s, 1, args...);
 }
+// 148 (here and in the grids of the memory-bound kernels) are the SMs of a B200: these kernels fill the device whatever
+// b200conv_set_sm_count leaves to the persistent ones.
 constexpr unsigned kChainedBlocks = 148 * 8;      // of 256 threads
 template <class... Exp, class... Act>
 cudaError_t launch_streaming(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Act&&... args) {
