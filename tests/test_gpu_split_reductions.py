@@ -252,3 +252,26 @@ def test_split_reductions_fall_back_to_whole_ones_without_memory_for_slices():
     shim.device_conv2d(X, W, out=Y)
     assert c.launches - before == 2                                      # with memory again: split
     c.close()
+
+
+@DTYPES
+@pytest.mark.parametrize("flags", [0, shim.NO_SLAB], ids=["slab", "tap"])
+@pytest.mark.parametrize("xs,k,ks", [((1, 512, 8, 8), 75, 3), ((40, 16, 28, 28), 21, 3), ((16, 256, 40, 40), 255, 1)], ids=["split", "direct", "1x1"])
+def test_pad_channels_of_a_residual_stay_out_of_the_result(ctx, dtype, flags, xs, k, ks):
+    """Pad channels are written as zeros whatever the pad channels of the residual hold, also off the 16-byte boundaries."""
+    rs = np.random.RandomState(10)
+    x = rs.standard_normal(xs).astype(dtype)
+    w = (rs.standard_normal((k, xs[1], ks, ks)) / np.sqrt(xs[1] * ks * ks)).astype(dtype)
+    X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
+    conv = O.conv2d(x.astype(np.float32), w.astype(np.float32), border_mode="half", subsample=(1, 1))
+    r = rs.standard_normal(conv.shape).astype(dtype)
+    R = T.from_host(ctx, r, "nhwc")
+    a = stored(R)
+    a[..., k:] = np.nan
+    ctx.h2d(R.ptr, a)
+    out = T(ctx, conv.shape, dtype, "nhwc")
+    off, owner = shifted(out, 7)
+    for y in (out, off, R):                     # the last one accumulates in place
+        shim.device_conv2d(X, W, border_mode="half", residual=R, out=y, flags=flags)
+        assert not stored(y)[..., k:].any()
+        assert O.rel_err(y.to_host().astype(np.float32), conv + r.astype(np.float32)) < TOL[dtype]

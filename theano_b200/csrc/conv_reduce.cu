@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) conv_reduce_kernel(const __grid_constant_
       if (c0 + e >= p.n_out) continue;
       float f = p.epi.alpha * (c0 + e < p.n_real ? v[e] : 0.f);       // pad channels: 0 x infinity is NaN
       if (p.bias) f += to_f(static_cast<const T*>(p.bias)[g * p.n_out + c0 + e]);
-      if (p.epi.residual) f += p.epi.beta * to_f(static_cast<const T*>(p.epi.residual)[(out - static_cast<T*>(p.out)) + e * p.out_sc]);
+      if (p.epi.residual && c0 + e < p.n_real) f += p.epi.beta * to_f(static_cast<const T*>(p.epi.residual)[(out - static_cast<T*>(p.out)) + e * p.out_sc]);
       if (p.relu) f = p.epi.lin * f + p.epi.abs * fabsf(f);
       // pooling compares stored values, as the unsplit epilogue does
       f = to_f(static_cast<T>(f));

@@ -247,7 +247,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
             for (int q = 0; q < 16 / (int)sizeof(OutT); ++q) {
               f[q] = p.epi.alpha * __uint_as_float(r[j + q]);
               if (bias) f[q] += static_cast<float>(bias[j + q]);
-              if (res) f[q] += p.epi.beta * static_cast<float>(res[co0 + j + q]);
+              if (res && co0 + j + q < p.n_real) f[q] += p.epi.beta * static_cast<float>(res[co0 + j + q]);
               if (p.relu) f[q] = p.epi.lin * f[q] + p.epi.abs * fabsf(f[q]);
             }
             if (!B200_IN_RANGE((pix - out) + co0 + j >= 0 && (pix - out) + co0 + j + 16 / (long long)sizeof(OutT) <= p.out_elems, p.status))
@@ -271,7 +271,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
             if (co0 + j < p.n_out) {
               float v = p.epi.alpha * __uint_as_float(r[j]);
               if (bias) v += static_cast<float>(bias[j]);
-              if (res) v += p.epi.beta * static_cast<float>(res[(co0 + j) * p.out_sc]);
+              if (res && co0 + j < p.n_real) v += p.epi.beta * static_cast<float>(res[(co0 + j) * p.out_sc]);
               if (p.relu) v = p.epi.lin * v + p.epi.abs * fabsf(v);
               if (B200_IN_RANGE((pix - out) + (co0 + j) * p.out_sc >= 0 && (pix - out) + (co0 + j) * p.out_sc < p.out_elems, p.status))
                 OutPack<OutT>::store(pix + (co0 + j) * p.out_sc, v);
