@@ -556,17 +556,19 @@ long long split_clocks(long long items, int rows, int bn, int sms) {
   return 1LL * rows * bn * 4 / 32 + 4500 + items * rows * bn * 4 / (48LL * sms);
 }
 
-// Filter taps per stage of the slab kernel's filter ring.  A stage's hand-over in the issuing warp (about 190 clocks,
-// during which the tensor pipe runs dry) is paid once per stage, so a stage holds as many taps as leaves the ring two
-// or three stages: with one CTA 12 to 36 KB for narrow tiles and one tap for 128 and 256 filters, whose stages are 16
+// Filter taps per stage of the slab kernel's filter ring.  A stage's barriers cost the issuing warp some 50 to 90 clocks of
+// tensor time (about 190 when the times below were taken), so a stage holds as many taps as leaves the ring two
+// or three stages: with one CTA 12 to 40 KB for narrow tiles and one tap for 128 and 256 filters, whose stages are 16
 // and 32 KB already; a pair's CTAs hold half of the filters, so they take three taps of 128 and two of 256.
 // Measured (one tap -> several, 64 images, float32 3x3): pairs 256 -> 256 at 56x56 401 -> 340 us, 128 -> 128 at
 // 112x112 with pooling 406 -> 341, 64 -> 128 at 112x112 240 -> 201; float16 512 -> 512 at 7x7, 256 images 110 -> 89.
 // 32-filter tiles, a filter row -> five taps: 32 groups of 8 channels at 28x28 184 -> 172 us.
 int slab_tps(int bn, int ntaps, bool pair) {
-  if (bn >= 128) return pair ? std::min(bn >= 256 ? 2 : 3, ntaps) : 1;
-  if (bn == 32 && ntaps <= 9) return ntaps;
-  return ntaps % 3 == 0 ? 3 : std::min(4, ntaps);
+  const int most = bn >= 256 ? (pair ? 2 : 1) : bn == 128 ? (pair ? 3 : 1) : bn == 64 ? 5 : 9;
+  // a number that divides the taps and has straight-line code in the issuing warp
+  for (int t : {9, 5, 4, 3, 2, 1})
+    if (t <= most && ntaps % t == 0 && (t > 1 || ntaps == 1 || most == 1)) return t;
+  return std::min(most == 9 ? 7 : std::min(most, 4), ntaps);
 }
 // Filter stages that a tile with the staged epilogue has to keep.
 int slab_min_stages(bool pair, int tps) { return tps >= 9 || (pair && tps >= 3) ? 2 : 3; }
@@ -902,12 +904,10 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, b_rows, a.groups, p.tap_boxes ? 1 : tps);
   if (rc) return rc;
   for (const ConvTap& t : taps) {
-    p.tap_shift[p.ntaps] = (int16_t)((t.dh - dh_min) * p.Ws + (t.dw - dw_min));
     p.tap_wmat[p.ntaps] = t.wmat;
-    if (p.ncls > 1) {
-      p.tap_cls[p.ntaps] = a.tap_cls[p.ntaps];
-      p.tap_first[p.ntaps] = std::find(a.tap_cls.begin(), a.tap_cls.begin() + p.ntaps, a.tap_cls[p.ntaps]) == a.tap_cls.begin() + p.ntaps;
-    }
+    const int cls = p.ncls > 1 ? a.tap_cls[p.ntaps] : 0;
+    const bool adds = p.ncls > 1 && std::find(a.tap_cls.begin(), a.tap_cls.begin() + p.ntaps, cls) != a.tap_cls.begin() + p.ntaps;
+    p.tap_issue[p.ntaps] = slab_tap((t.dh - dh_min) * p.Ws + (t.dw - dw_min), cls * BN, adds);
     ++p.ntaps;
   }
   p.kblocks = (int)cdiv(a.Cin_g, kBK);
@@ -938,6 +938,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   }
   Scratch tmp(c);
   ConvReduceParams q;
+  CU_OK(c, load_conv_slab(a.dtype, conv_umma_bn(a.n_out)));
   if ((rc = split_output(c, tmp, p, BN, p.n_acc * 128, &q))) return rc;
   q.Ws = p.Ws; q.Hs = p.Hs; q.wt = p.wt; q.th = p.th; q.nb = p.nb;
   KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
@@ -1011,6 +1012,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   }
   Scratch tmp(c);
   ConvReduceParams q;
+  CU_OK(c, load_conv_umma(a.dtype, conv_umma_bn(a.n_out)));
   if ((rc = split_output(c, tmp, p, BN, 128, &q))) return rc;
   q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
   KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
@@ -1022,7 +1024,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
 // leaves ms[i] at -1.  Returns an error of the timing itself.
 // Every variant runs twice, the second time between two events (the first loads its code and makes the choices inside
 // it); with one exception this decides: variants within a fifth (and the 4 us by which short launches differ between
-// events) of the best are timed again in bursts of up to 8 back to back, the way a program issues them, once, and
+// events) of the best are timed again in bursts of up to 7 back to back, the way a program issues them, once, and
 // once more if they are still within 5 %.  Alone, a kernel of 5 us costs 5 us more and the chained launch hides nothing.
 // All variants in two bursts each made the first passes of 32 cases take 200 ms together, this and rough_times() 127.
 template <class Run>
@@ -1053,7 +1055,7 @@ int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool r
   }
   const float first = best();
   if (first < 0.f || first > 0.5f || rough) return 0;     // long enough for one measurement
-  const int reps = std::max(1, std::min(8, (int)(0.16f / std::max(first, 0.001f))));
+  const int reps = std::max(1, std::min(7, (int)(0.14f / std::max(first, 0.001f))));
   float limit = 1.2f * first + 0.004f;
   for (int round = 0; round < 2; ++round) {
     int close = 0;

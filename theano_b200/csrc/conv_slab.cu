@@ -47,12 +47,154 @@ template <typename T> __device__ __forceinline__ void store_out(T* p, float v);
 template <> __device__ __forceinline__ void store_out<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void store_out<__half>(__half* p, float v) { *p = __float2half_rn(v); }
 
+// Slice of a tile's reduction: channel blocks kb0..kb1, tap groups from tg0 in the first, up to tg1 in the last (inclusive).
+struct Range { int kb0, kb1, tg0, tg1; };
+__device__ __forceinline__ Range slice_range(const SlabConvParams& p, uint32_t slice) {
+  const uint32_t stages_kb = (p.ntaps + p.tps - 1) / p.tps, stages_all = stages_kb * p.kblocks;
+  if (p.splits == 1) return Range{0, p.kblocks - 1, 0, static_cast<int>(stages_kb) - 1};
+  const uint32_t a = stages_all * slice / p.splits, b = stages_all * (slice + 1) / p.splits - 1;
+  return Range{static_cast<int>(a / stages_kb), static_cast<int>(b / stages_kb), static_cast<int>(a % stages_kb), static_cast<int>(b % stages_kb)};
+}
+
+struct IssueLoop {
+  const SlabConvParams& p;
+  Bars* bars;
+  uint8_t *smem, *bring;
+  uint32_t tmem;
+  int a_begin, na;
+  uint32_t first, stride, total;
+  bool dbl, leader;
+  long long* trace;
+};
+
+// The MMAs of one issuing warp, all its tiles.  All 32 lanes follow the loop and wait on the barriers; one elected lane
+// issues the MMAs and their commits.  A lone lane (code under `if (lane == 0)`) computes every descriptor on the
+// per-thread datapath and moves it to uniform registers per MMA, which costs more clocks than a 128 x 64 or 128 x 128
+// MMA runs.
+// NT taps per filter stage, NA accumulators: a stage is straight-line code; 0: any number, in loops.  In loops the
+// branches and the look-ups of each tap's shift take the warp longer than narrow MMAs run, and the wait at the head of
+// each stage drains the tensor pipe.  The loop alone, operands always there, clocks per MMA in loops / straight-line
+// with mbar_look(): 128 x 64 float32, three taps per stage, one accumulator 83 / 66, one for each issuer 59.5 / 48.3 (what the
+// operands' reads take); one tap per stage and one accumulator: 128 x 32 133 / 71, 128 x 128 140 / 88, 128 x 256 147 / 132.
+// No branch may stand among the elected lane's instructions: with the release of the slab under an `if` there, one
+// tap per stage took 130 clocks again.
+template <MmaKind KIND, int BN, bool PAIR, int NT, int NA>
+__device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
+  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, false, false, PAIR ? 256 : 128, BN);
+  constexpr int kBBytes = (PAIR ? BN / 2 : BN) * 128;
+  constexpr bool kTogether = NT >= 4;      // many MMAs: issued by the whole warp (umma_words_if), under a branch their descriptors spill
+  const SlabConvParams& p = w.p;
+  Bars* bars = w.bars;
+  const bool leader = w.leader;
+  const int ncls = p.ncls, na = NA ? NA : w.na;
+  const uint64_t desc_bits = smem_desc(0, 16, 1024);
+  const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32), desc_lo = static_cast<uint32_t>(desc_bits);
+  const uint32_t slab0 = desc_lo + ((smem_u32(w.smem) + 16384u * w.a_begin) >> 4), ring0 = desc_lo + (smem_u32(w.bring) >> 4);
+  const uint32_t slab_units = static_cast<uint32_t>(p.slab_bytes) >> 4, stage_units = static_cast<uint32_t>(p.tps * kBBytes) >> 4;
+  const uint32_t acc_step = ncls * BN;             // columns from one accumulator to the next
+  auto commit = [&](uint64_t* bar) {
+    if (PAIR) umma_commit_pair(bar);
+    else umma_commit(bar);
+  };
+  int sb = 0, bs = 0, it = 0;
+  uint32_t sphase = 0, bphase = 0;
+  uint32_t slab_seen = 0, b_seen = 0, acc_seen = 0;  // the next slab / filter stage / accumulator already seen ready (mbar_look)
+  for (uint32_t item = w.first; item < w.total; item += w.stride, ++it) {
+    const Range r = slice_range(p, item % static_cast<uint32_t>(p.splits));
+    // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
+    // runs beside the MMAs of the next one
+    const int buf = w.dbl ? (it & 1) : 0;
+    const uint32_t aphase = w.dbl ? ((it >> 1) & 1) : (it & 1);
+    const uint32_t acc0 = w.tmem + buf * (p.n_acc * acc_step) + w.a_begin * acc_step;
+    if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) return false;
+    acc_seen = 0;
+    tc_fence_after();
+    for (int kb = r.kb0; kb <= r.kb1; ++kb) {
+      if (!wait_seen(slab_seen, &bars->slab_full[sb], sphase, bars, p.wait_clocks)) return false;
+      if (w.trace && it == 0 && kb == r.kb0) w.trace[2] = clock64();
+      const uint32_t slab_lo = slab0 + sb * slab_units;
+      const int tap_begin = kb == r.kb0 ? r.tg0 * p.tps : 0;
+      const int tap_end = kb == r.kb1 ? min(p.ntaps, (r.tg1 + 1) * p.tps) : p.ntaps;
+      for (int tap0 = tap_begin; tap0 < tap_end; tap0 += NT ? NT : p.tps) {
+        const int nt = NT ? NT : min(p.tps, p.ntaps - tap0);
+        uint32_t info[NT ? NT : 1];
+        if (NT) {
+#pragma unroll
+          for (int q = 0; q < NT; ++q) info[q] = p.tap_issue[tap0 + q];
+        }
+        if (!wait_seen(b_seen, &bars->b_full[bs], bphase, bars, p.wait_clocks)) return false;
+        tc_fence_after();
+        const uint32_t ring_lo = ring0 + bs * stage_units;
+        // 0 for the first products of the slice, or of the tap's class
+        const uint32_t more = kb != r.kb0 || (ncls == 1 && tap0 != tap_begin), rest = more | (ncls == 1);
+        auto mma = [&](int q, uint32_t tap, int a, int kk) {
+          const uint32_t a_lo = slab_lo + slab_tap_shift(tap) + a * (16384 >> 4);
+          const uint32_t acc = acc0 + slab_tap_column(tap) + a * acc_step, b_lo = ring_lo + ((q * kBBytes) >> 4), adds = kk ? 1u : (q ? rest : more) | slab_tap_adds(tap);
+          if (kTogether) umma_words_if<KIND, PAIR>(leader, acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, adds);
+          else umma_words<KIND, PAIR>(acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, adds);
+        };
+        // a stage's MMAs from u0 to u1, numbered (tap, accumulator, 32 bytes of the channels)
+        auto part = [&](int u0, int u1) {
+#pragma unroll
+          for (int q = 0; q < NT; ++q)
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                const int u = (q * NA + a) * 4 + kk;
+                if (u >= u0 && u < u1) mma(q, info[q], a, kk);
+              }
+        };
+        constexpr int kAll = NT * NA * 4, kBefore = kAll >= 16 ? kAll - 8 : kAll > 4 ? kAll - 4 : 2;
+        if (kTogether) part(0, kBefore);
+        if (!kTogether && leader) {
+          if (NT) {
+            part(0, kBefore);
+          } else {
+            for (int q = 0; q < nt; ++q) {
+              const uint32_t tap = p.tap_issue[tap0 + q];
+              for (int a = 0; a < (q + 1 == nt ? na - 1 : na); ++a) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) mma(q, tap, a, kk);
+              }
+            }
+          }
+        }
+        __syncwarp();
+        const int cur = bs;
+        if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
+        b_seen = mbar_look(&bars->b_full[bs], bphase);
+        if (tap0 + p.tps >= tap_end) {             // the channel block ends, perhaps the tile too
+          const int ns = sb + 1 == p.s_stages ? 0 : sb + 1;
+          slab_seen = mbar_look(&bars->slab_full[ns], ns ? sphase : sphase ^ 1);
+          if (w.dbl && kb == r.kb1) acc_seen = mbar_look(&bars->acc_empty[(it + 1) & 1], (((it + 1) >> 1) & 1) ^ 1);
+        }
+        if (kTogether) part(kBefore, kAll);
+        if (leader) {
+          if (NT) {
+            if (!kTogether) part(kBefore, kAll);
+          } else {
+            const uint32_t tap = p.tap_issue[tap0 + nt - 1];
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) mma(nt - 1, tap, na - 1, kk);
+          }
+          commit(&bars->b_empty[cur]);
+        }
+      }
+      if (leader) commit(&bars->slab_empty[sb]);
+      if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
+    }
+    if (leader) commit(&bars->acc_full[buf]);
+    if (w.trace && it == 0) w.trace[3] = clock64();
+  }
+  return true;
+}
+
 template <MmaKind KIND, int BN, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   using OutT = typename std::conditional<KIND == MmaKind::TF32, float, __half>::type;
   constexpr int kBK = KIND == MmaKind::TF32 ? 32 : 64;
-  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, false, false, PAIR ? 256 : 128, BN);
   constexpr int kBBytes = (PAIR ? BN / 2 : BN) * 128;   // filters this CTA loads per tap and channel block
 
   extern __shared__ uint8_t smem_raw[];
@@ -80,13 +222,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   // Work item = (tile, slice of the reduction), the slices of a tile side by side.  A slice is a range of
   // filter stages (channel block x group of tps taps), in the order the unsplit loop walks them.
   const uint32_t splits = p.splits;
-  const uint32_t stages_kb = (p.ntaps + p.tps - 1) / p.tps, stages_all = stages_kb * p.kblocks;
-  struct Range { int kb0, kb1, tg0, tg1; };        // channel blocks kb0..kb1, tap groups from tg0 in the first, up to tg1 in the last (inclusive)
-  auto slice_range = [&](uint32_t slice) {
-    if (splits == 1) return Range{0, p.kblocks - 1, 0, static_cast<int>(stages_kb) - 1};
-    const uint32_t a = stages_all * slice / splits, b = stages_all * (slice + 1) / splits - 1;
-    return Range{static_cast<int>(a / stages_kb), static_cast<int>(b / stages_kb), static_cast<int>(a % stages_kb), static_cast<int>(b % stages_kb)};
-  };
   const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
   const int ncls = p.ncls;                              // accumulator (a, class q): columns (a * ncls + q) * BN
   const bool dbl = 2 * p.n_acc * ncls * BN <= 512;
@@ -138,7 +273,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     bool ok = true;
     for (uint32_t item = first; item < total && ok; item += stride) {
       const uint32_t t = item / splits;
-      const Range r = slice_range(item - t * splits);
+      const Range r = slice_range(p, item - t * splits);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
       const uint32_t pt = PAIR ? t / co_groups * 2 + rank : t / co_groups;
       const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
@@ -164,7 +299,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     bool ok = true;
     for (uint32_t item = first; item < total && ok; item += stride) {
       const uint32_t t = item / splits;
-      const Range r = slice_range(item - t * splits);
+      const Range r = slice_range(p, item - t * splits);
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
       const int row0 = co_t * BN + static_cast<int>(rank) * (BN / 2);     // a pair's CTAs load one half each
@@ -195,86 +330,28 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     }
     if (!ok && leader) report_status(p.status, kStatusTimeout);
   } else if (warp == 1 || warp == kSecondIssuer) {
-    // this issuer's accumulators of every tile: [a_begin, a_end)
+    // this issuer's accumulators of every tile: [a_begin, a_begin + na)
     const int a_split = issuers == 2 ? (p.n_acc + 1) / 2 : p.n_acc;
-    const int a_begin = warp == 1 ? 0 : a_split, a_end = warp == 1 ? a_split : p.n_acc;
-    if (warp != 1) trace = nullptr;            // the stamps are the first issuer's
-    if (rank == 0 && a_begin < a_end) {        // a pair: the even CTA issues for both
-      // All 32 lanes follow the loop and wait on the barriers; one elected lane issues the MMAs
-      // and their commits.  A lone lane (code under `if (lane == 0)`) computes every descriptor
-      // on the per-thread datapath and moves it to uniform registers per MMA, which costs more
-      // clocks than a 128 x 64 or 128 x 128 MMA runs.
+    const int a_begin = warp == 1 ? 0 : a_split, na = warp == 1 ? a_split : p.n_acc - a_split;
+    if (rank == 0 && na > 0) {                 // a pair: the even CTA issues for both
       const bool leader = elect_one();
-      if (!leader) trace = nullptr;
-      int sb = 0, bs = 0;
-      uint32_t sphase = 0, bphase = 0;
-      bool ok = true;
-      int it = 0;
-      long long tw_acc = 0, tw_slab = 0, tw_b = 0;       // clocks spent waiting (only with trace)
-      const long long t_loop0 = trace ? clock64() : 0;
-      const uint64_t desc_bits = smem_desc(0, 16, 1024);
-      const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
-      const uint32_t desc_lo = static_cast<uint32_t>(desc_bits);
-      auto commit = [&](uint64_t* bar) {
-        if (PAIR) umma_commit_pair(bar);
-        else umma_commit(bar);
-      };
-      for (uint32_t item = first; item < total && ok; item += stride, ++it) {
-        const Range r = slice_range(item % splits);
-        // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
-        // runs beside the MMAs of the next one
-        const int buf = dbl ? (it & 1) : 0;
-        const uint32_t aphase = dbl ? ((it >> 1) & 1) : (it & 1);
-        const uint32_t acc_base = tmem + buf * (p.n_acc * ncls * BN);
-        long long tq = trace ? clock64() : 0;
-        if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
-        if (trace) tw_acc += clock64() - tq;
-        tc_fence_after();
-        for (int kb = r.kb0; kb <= r.kb1 && ok; ++kb) {
-          tq = trace ? clock64() : 0;
-          if (!uniform_wait(&bars->slab_full[sb], sphase, bars, p.wait_clocks)) { ok = false; break; }
-          if (trace) tw_slab += clock64() - tq;
-          if (trace && it == 0 && kb == r.kb0) trace[2] = clock64();
-          const uint32_t sbase = smem_u32(smem + sb * p.slab_bytes);
-          const int tap_begin = kb == r.kb0 ? r.tg0 * p.tps : 0;
-          const int tap_end = kb == r.kb1 ? min(p.ntaps, (r.tg1 + 1) * p.tps) : p.ntaps;
-          for (int tap0 = tap_begin; tap0 < tap_end; tap0 += p.tps) {
-            tq = trace ? clock64() : 0;
-            if (!uniform_wait(&bars->b_full[bs], bphase, bars, p.wait_clocks)) { ok = false; break; }
-            if (trace) tw_b += clock64() - tq;
-            tc_fence_after();
-            const int nt = min(p.tps, p.ntaps - tap0);
-            if (leader) {
-              for (int q = 0; q < nt; ++q) {
-                const int tap = tap0 + q;
-                // only the address field of the two descriptors changes from MMA to MMA
-                const uint32_t b_lo = desc_lo + (smem_u32(bring + bs * stage_b + q * kBBytes) >> 4);
-                // 0 for the first products of the slice, or of the tap's class
-                const uint32_t first = kb != r.kb0 || (ncls > 1 ? p.tap_first[tap] == 0 : tap != tap_begin);
-                const uint32_t acc_cls = acc_base + (ncls > 1 ? p.tap_cls[tap] * BN : 0);
-                uint32_t a_lo = desc_lo + ((sbase + static_cast<uint32_t>(p.tap_shift[tap] + 128 * a_begin) * 128u) >> 4);
-                for (int a = a_begin; a < a_end; ++a) {
-#pragma unroll
-                  for (int kk = 0; kk < 4; ++kk)
-                    umma_words<KIND, PAIR>(acc_cls + a * (ncls * BN), a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, first | (kk != 0));
-                  a_lo += (128 * 128) >> 4;      // next accumulator: 128 slab rows further
-                }
-              }
-              commit(&bars->b_empty[bs]);
-            }
-            if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
-          }
-          if (ok && leader) commit(&bars->slab_empty[sb]);
-          if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
-        }
-        if (ok && leader) commit(&bars->acc_full[buf]);
-        if (trace && it == 0) trace[3] = clock64();
-      }
+      IssueLoop w{p, bars, smem, bring, tmem, a_begin, na, first, stride, total, dbl, leader, warp == 1 && leader ? trace : nullptr};
+      const int nt = p.ntaps % p.tps == 0 ? p.tps : 0;       // 0: groups of taps of different sizes
+      bool ok;
+      if (nt == 1 && na == 1) ok = issue_tiles<KIND, BN, PAIR, 1, 1>(w);
+      else if (nt == 1 && na == 2) ok = issue_tiles<KIND, BN, PAIR, 1, 2>(w);
+      else if (nt == 2 && na == 1) ok = issue_tiles<KIND, BN, PAIR, 2, 1>(w);
+      else if (nt == 2 && na == 2) ok = issue_tiles<KIND, BN, PAIR, 2, 2>(w);
+      else if (nt == 3 && na == 1) ok = issue_tiles<KIND, BN, PAIR, 3, 1>(w);
+      else if (nt == 3 && na == 2) ok = issue_tiles<KIND, BN, PAIR, 3, 2>(w);
+      else if (BN <= 64 && nt == 4 && na == 1) ok = issue_tiles<KIND, BN, PAIR, BN <= 64 ? 4 : 0, 1>(w);
+      else if (BN <= 64 && nt == 4 && na == 2) ok = issue_tiles<KIND, BN, PAIR, BN <= 64 ? 4 : 0, 2>(w);
+      else if (BN <= 64 && nt == 5 && na == 1) ok = issue_tiles<KIND, BN, PAIR, BN <= 64 ? 5 : 0, 1>(w);
+      else if (BN <= 64 && nt == 5 && na == 2) ok = issue_tiles<KIND, BN, PAIR, BN <= 64 ? 5 : 0, 2>(w);
+      else if (BN <= 32 && nt == 9 && na == 1) ok = issue_tiles<KIND, BN, PAIR, BN <= 32 ? 9 : 0, 1>(w);
+      else if (BN <= 32 && nt == 9 && na == 2) ok = issue_tiles<KIND, BN, PAIR, BN <= 32 ? 9 : 0, 2>(w);
+      else ok = issue_tiles<KIND, BN, PAIR, 0, 0>(w);
       if (!ok && leader) report_status(p.status, kStatusTimeout);
-      if (trace) {
-        trace[9] = tw_acc; trace[10] = tw_slab; trace[11] = tw_b;
-        trace[12] = clock64() - t_loop0; trace[13] = it;
-      }
     }
   } else if (warp < kSecondIssuer) {
     // 16 epilogue warps: warp w reads TMEM lanes [32*(w%4), +32) (the hardware's rule) and, of
@@ -288,8 +365,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
     bool ok = true;
     int it = 0;
-    long long te_wait = 0, te_busy = 0;          // clocks of thread 64 (only with trace)
-    long long tp[5] = {0, 0, 0, 0, 0};           // its epilogue phases: buffer wait, TMEM read, convert + stage, fence + barrier, store issue
     int nstore = 0;                              // chunks this warp's group has staged so far
     for (uint32_t item = first; item < total && ok; item += stride, ++it) {
       const uint32_t t = item / splits;
@@ -301,10 +376,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const int n0 = (pt / tiles_wh) * p.nb;
       const int buf = dbl ? (it & 1) : 0;
       const uint32_t aphase = dbl ? ((it >> 1) & 1) : (it & 1);
-      const long long te0 = trace ? clock64() : 0;
       if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
-      const long long te1 = trace ? clock64() : 0;
       if (trace && it == 0 && threadIdx.x == 64) trace[4] = clock64();
       const int co_base = co_t * BN;
       const int nchunks = min(BN / 32, (p.n_out - co_base + 31) / 32);
@@ -355,7 +428,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           uint8_t* srow = stg + drow * 128;
           const int co0 = co_base + ch * kCh;
           const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
-          long long tq = trace ? clock64() : 0;
           if (nstore >= bufs) {                // the buffer's previous box must have been read
             if (issuer) {
               if (bufs == 2) bulk_wait_read<1>();
@@ -363,13 +435,11 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
             }
             named_barrier(1 + grp, gthreads);
           }
-          if (trace) { const long long t = clock64(); tp[0] += t - tq; tq = t; }
 #pragma unroll
           for (int part = 0; part < kCh / 32; ++part) {
             uint32_t r[32];
             tmem_ld32(lane_base + (a * ncls + cls) * BN + ch * kCh + part * 32, r);
             tmem_ld_wait();
-            if (trace) { const long long t = clock64(); tp[1] += t - tq; tq = t; }
             if (!inbox) continue;
             zero_pad_columns(r, co0 + part * 32, p.n_real);
             const OutT* bp = bias ? bias + part * 32 : nullptr;
@@ -424,7 +494,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
               }
             }
           }
-          if (trace) { const long long t = clock64(); tp[2] += t - tq; tq = t; }
           if (p.epi.pool) {
             // 2x2 max pooling of the staged chunk (Pool{ignore_border=True, mode='max'}, ws = stride = 2): the
             // tile's width and height are even, so every window lies inside it.  The group's threads read the
@@ -475,7 +544,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
           }
           fence_async_smem();
           named_barrier(1 + grp, gthreads);
-          if (trace) { const long long t = clock64(); tp[3] += t - tq; tq = t; }
           // a tiled store must not start at a negative coordinate, and its staging rows must lie
           // inside the reserved shared memory
           if (issuer && (!PAIR || n0 < p.Nimg) && (ncls == 1 || (w0 < p.cls_W[cls] && h0 < p.cls_H[cls])) &&
@@ -555,11 +623,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         mbar_arrive(&bars->acc_empty[buf]);
       }
       if (trace && it == 0 && threadIdx.x == 64) trace[5] = clock64();
-      if (trace) { te_wait += te1 - te0; te_busy += clock64() - te1; }
-    }
-    if (trace && threadIdx.x == 64) {
-      trace[14] = te_wait; trace[15] = te_busy;
-      for (int q = 0; q < 4; ++q) trace[16 + q] = tp[q];
     }
     if (p.tma_out && lane == 0) bulk_wait<0>();  // this thread's stores (if it issued any) have left shared memory
     if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
@@ -581,12 +644,17 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
 }
 
 template <MmaKind KIND, int BN, bool PAIR>
-cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cudaStream_t s) {
-  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.tps * (PAIR ? BN / 2 : BN) * 128 + p.stage_reserved + sizeof(Bars) + 1024;
+cudaError_t configure() {
   static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] {
+  return configured.ensure([] {
     return cudaFuncSetAttribute(conv_slab_kernel<KIND, BN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
   });
+}
+
+template <MmaKind KIND, int BN, bool PAIR>
+cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cudaStream_t s) {
+  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.tps * (PAIR ? BN / 2 : BN) * 128 + p.stage_reserved + sizeof(Bars) + 1024;
+  cudaError_t e = configure<KIND, BN, PAIR>();
   if (e != cudaSuccess) return e;
   const int units = PAIR ? num_sms / 2 : num_sms;
   const int grid = static_cast<int>(total < units ? total : units) * (PAIR ? 2 : 1);
@@ -595,6 +663,16 @@ cudaError_t launch_one(const SlabConvParams& p, long long total, int num_sms, cu
 }
 
 }  // namespace
+
+cudaError_t load_conv_slab(int dtype, int bn) {
+  const bool f16 = dtype == B200CONV_F16;
+  switch (bn) {
+    case 32: return f16 ? configure<MmaKind::F16, 32, false>() : configure<MmaKind::TF32, 32, false>();
+    case 64: return f16 ? configure<MmaKind::F16, 64, false>() : configure<MmaKind::TF32, 64, false>();
+    case 128: return f16 ? configure<MmaKind::F16, 128, false>() : configure<MmaKind::TF32, 128, false>();
+    default: return f16 ? configure<MmaKind::F16, 256, false>() : configure<MmaKind::TF32, 256, false>();
+  }
+}
 
 cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num_sms, cudaStream_t s) {
   const long long pix = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;

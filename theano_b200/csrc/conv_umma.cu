@@ -160,27 +160,35 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const uint64_t desc_bits = smem_desc(0, 16, 1024);
     const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
     const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
+    uint32_t seen = 0, acc_seen = 0;             // next stage / next accumulator already seen ready (mbar_look)
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
       const uint32_t slice = item % splits, k0 = kiters * slice / splits, k1 = kiters * (slice + 1) / splits;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
-      if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
+      if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem + buf * BN;
       for (uint32_t k = k0; k < k1; ++k) {
-        if (!uniform_wait(&bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
+        if (!wait_seen(seen, &bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
         // 8 tf32 / 16 f16 channels = 32 bytes along the swizzled row per MMA: only the address
         // field of the descriptors changes (by 2 units of 16 bytes)
         const uint32_t a_lo = lo_base + stage * (stage_bytes<BN>() >> 4);
         const uint32_t b_lo = a_lo + (kABytes >> 4);
         if (leader) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_words<KIND>(d_tmem, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, k != k0 || kk != 0);
-          umma_commit(&bars->empty[stage]);
+          umma_words<KIND>(d_tmem, a_lo, b_lo, desc_hi, kIdesc, k != k0);
+          umma_words<KIND>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, kIdesc, 1u);
         }
+        __syncwarp();
+        const int cur = stage;
         if (++stage == kStages) { stage = 0; phase ^= 1; }
+        seen = mbar_look(&bars->full[stage], phase);
+        if (k + 1 == k1) acc_seen = mbar_look(&bars->acc_empty[(it + 1) & 1], (((it + 1) >> 1) & 1) ^ 1);
+        if (leader) {
+          umma_words<KIND>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, kIdesc, 1u);
+          umma_words<KIND>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, kIdesc, 1u);
+          umma_commit(&bars->empty[cur]);
+        }
       }
       if (ok && leader) umma_commit(&bars->acc_full[buf]);
     }
@@ -294,11 +302,17 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   }
 }
 
+template <MmaKind KIND, int BN> constexpr int smem_bytes() { return num_stages<BN>() * stage_bytes<BN>() + sizeof(Bars) + 1024; }
+template <MmaKind KIND, int BN>
+cudaError_t configure() {
+  static PerDeviceOnce configured;
+  return configured.ensure([] { return cudaFuncSetAttribute(conv_umma_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<KIND, BN>()); });
+}
+
 template <MmaKind KIND, int BN>
 cudaError_t launch_one(const UmmaConvParams& p, long long total, int num_sms, cudaStream_t s) {
-  constexpr int smem = num_stages<BN>() * stage_bytes<BN>() + sizeof(Bars) + 1024;
-  static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(conv_umma_kernel<KIND, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+  constexpr int smem = smem_bytes<KIND, BN>();
+  cudaError_t e = configure<KIND, BN>();
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
   launch_chained(conv_umma_kernel<KIND, BN>, grid, kThreads, smem, s, p);
@@ -309,6 +323,16 @@ cudaError_t launch_one(const UmmaConvParams& p, long long total, int num_sms, cu
 
 // Accumulator width: the smallest of 32/64/128/256 columns that holds the group's outputs.
 int conv_umma_bn(int n_out) { return n_out <= 32 ? 32 : n_out <= 64 ? 64 : n_out <= 128 ? 128 : 256; }
+
+cudaError_t load_conv_umma(int dtype, int bn) {
+  const bool f16 = dtype == B200CONV_F16;
+  switch (bn) {
+    case 32: return f16 ? configure<MmaKind::F16, 32>() : configure<MmaKind::TF32, 32>();
+    case 64: return f16 ? configure<MmaKind::F16, 64>() : configure<MmaKind::TF32, 64>();
+    case 128: return f16 ? configure<MmaKind::F16, 128>() : configure<MmaKind::TF32, 128>();
+    default: return f16 ? configure<MmaKind::F16, 256>() : configure<MmaKind::TF32, 256>();
+  }
+}
 
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s) {
   const long long total = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;

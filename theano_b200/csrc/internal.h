@@ -133,21 +133,31 @@ struct alignas(64) UmmaConvParams {
 
 int conv_umma_bn(int n_out);      // accumulator columns that hold n_out outputs per group, at most 256
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s);
+// Puts the kernel's code on the device (it is otherwise loaded by its first launch, which needs memory): a launch that
+// runs split loads the code of the whole reduction with it, to fall back to when there is no memory for the slices.
+cudaError_t load_conv_umma(int dtype, int bn);
+cudaError_t load_conv_slab(int dtype, int bn);
 
 // ---- implicit GEMM with one activation slab per channel block (conv_slab.cu) ---------------
 // For launches whose taps all read the same view: the slab (output tile plus halo) is loaded
 // once per channel block and every tap is a row offset into it.
 constexpr int kMaxSlabClasses = 4;
+// A tap in one word: row offset of the tap inside the slab in 16-byte units, column of its class's accumulator, and
+// whether its products add to earlier ones of the class (set for all but the first tap of each class where there are several).
+inline uint32_t slab_tap(int row_shift, int column, bool adds) { return static_cast<uint32_t>(row_shift) * 8 | static_cast<uint32_t>(column) << 16 | (adds ? 1u << 31 : 0u); }
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t slab_tap_shift(uint32_t tap) { return tap & 0xFFFF; }
+__device__ __forceinline__ uint32_t slab_tap_column(uint32_t tap) { return (tap >> 16) & 0x7FFF; }
+__device__ __forceinline__ uint32_t slab_tap_adds(uint32_t tap) { return tap >> 31; }
+#endif
 struct alignas(64) SlabConvParams {
   CUtensorMap view;              // 5-D (c_in_group, group, w, h, n), box (kBK, 1, Ws, Hs, nb)
   CUtensorMap wmap;              // 4-D packed filters (k_red, n_out, group, tap), box (kBK, BN or half of it, 1, 1 or tps)
-  int16_t tap_shift[kMaxTaps];   // row offset of the tap inside the slab
+  uint32_t tap_issue[kMaxTaps];  // what the MMAs of the tap need (slab_tap)
   int16_t tap_wmat[kMaxTaps];
   // Output classes: the taps of class q add up in accumulators of their own, and the class has its own output tensor
   // (strided gradInputs: the stride's parity classes of dx, all from one slab of dy).  1: one output, no classes.
   int ncls;
-  uint8_t tap_cls[kMaxTaps];     // class of the tap
-  uint8_t tap_first[kMaxTaps];   // 1: first tap of its class
   int cls_W[kMaxSlabClasses], cls_H[kMaxSlabClasses];    // output grid of the class (at most Wt x Ht)
   int ntaps;
   int kblocks;
@@ -177,7 +187,7 @@ struct alignas(64) SlabConvParams {
   ConvEpilogue epi;
   int* status;
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
-  long long* trace;              // optional: 16 clock64 stamps per CTA (phase timing), or null
+  long long* trace;              // optional: 9 clock64 stamps per CTA (phase timing), 32 slots apart, or null
   // Channels-last outputs are written by TMA: the epilogue warps put 128-byte channel chunks (32
   // float32 / 64 float16) of the tile into shared memory (rows = the tile's pixels, dense) and one
   // thread per chunk stores the box (chunk, wt, th, nb) through out_map.

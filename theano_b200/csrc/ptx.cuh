@@ -128,6 +128,29 @@ __device__ __forceinline__ bool uniform_wait(uint64_t* bar, uint32_t parity, Bar
   return __all_sync(0xffffffffu, ok) != 0;
 }
 
+// A look ahead at a barrier that the warp will wait on next: one test that never blocks.  The issuing warps look at the
+// next stage's barrier in the middle of a stage's MMAs, when the tensor pipe still has work queued, and enter that stage
+// without a wait if the answer was yes (wait_seen).  A wait at the head of a stage, even on a barrier that completed
+// long ago, leaves the pipe without work for about 180 clocks when the MMAs are shorter than 128 (a B200, clocks per
+// stage without -> with the look ahead, operands always there): 24 MMAs of 128 x 128 1716 -> 1536 (their own time),
+// 8 of them 704 -> 512, 8 of 128 x 64 613 -> 437, 4 of them 411 -> 247; 128 x 256: 1024 for 8 either way.
+__device__ __forceinline__ uint32_t mbar_look(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok;
+}
+// uniform_wait() unless every lane has already seen the phase complete.
+template <class BarsT>
+__device__ __forceinline__ bool wait_seen(uint32_t seen, uint64_t* bar, uint32_t parity, BarsT* b, long long limit) {
+  return __all_sync(0xffffffffu, seen) ? true : uniform_wait(bar, parity, b, limit);
+}
+
 // Abort path of the tensor-core kernels.  A role that gives up (its wait of `limit` clocks ran
 // out) sets `abort`; every other role sees the flag at its next slow-path poll and stops issuing;
 // all threads then meet at the kernel's closing __syncthreads.  TMA boxes requested earlier may
@@ -408,6 +431,38 @@ __device__ __forceinline__ void umma_words(uint32_t d_tmem, uint32_t a_lo, uint3
         "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate)
         : "memory");
   }
+}
+// The MMA (and its commit) as instructions that a converged warp runs together and that take effect where `lane` is set,
+// in its elected lane: no branch, so addresses stay on the uniform datapath whatever their number.  A block of 24 MMAs
+// with run-time operand offsets under a branch has all of its descriptors worked out ahead of the branch, and spilled.
+// (8 steps x 3 taps of 128 x 128, clocks per MMA: 64.0, under a branch 64.8 without and about 85 with spills.)
+#define B200_UMMA_IF(GROUP, KIND)                                                                        \
+  asm volatile(                                                                                          \
+      "{\n\t.reg .pred p, l;\n\t.reg .b64 da, db;\n\t"                                                  \
+      "setp.ne.b32 p, %5, 0;\n\t"                                                                        \
+      "setp.ne.b32 l, %6, 0;\n\t"                                                                        \
+      "mov.b64 da, {%1, %3};\n\t"                                                                        \
+      "mov.b64 db, {%2, %3};\n\t"                                                                        \
+      "@l tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], da, db, %4, p;\n\t}" ::"r"(d_tmem),      \
+      "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate), "r"(lane)                         \
+      : "memory")
+template <MmaKind kind, bool PAIR = false>
+__device__ __forceinline__ void umma_words_if(uint32_t lane, uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi,
+                                              uint32_t idesc, uint32_t accumulate) {
+  if (kind == MmaKind::TF32) {
+    if (PAIR) B200_UMMA_IF("2", "tf32");
+    else B200_UMMA_IF("1", "tf32");
+  } else {
+    if (PAIR) B200_UMMA_IF("2", "f16");
+    else B200_UMMA_IF("1", "f16");
+  }
+}
+#undef B200_UMMA_IF
+__device__ __forceinline__ void umma_commit_if(uint32_t lane, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred l;\n\tsetp.ne.b32 l, %1, 0;\n\t"
+      "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane)
+      : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base+t).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {

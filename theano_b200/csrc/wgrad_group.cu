@@ -8,9 +8,9 @@
 // are widened by the column span of the taps (dy reads zeros there), so "shifted by dw" is a plain
 // row offset into one shared-memory x tile: per stage one dy tile and one x tile are fetched and
 // every tap of the group accumulates into its own 128 x 128 TMEM accumulator.  That divides the
-// number of TMA boxes per MMA.  (Measured: with MN-major operands the MMAs themselves run at about
-// 0.4 of their K-major rate and bound both gradWeights kernels; which of the two is faster
-// depends on the layer, so the first call of a geometry times both.)
+// number of TMA boxes per MMA.  (MN-major operands run at the same rate as K-major ones: 64 clocks per 128 x 128 MMA,
+// whatever the row offset.  Which of the two gradWeights kernels is faster depends on the layer, so the first call
+// of a geometry times both.)
 //
 // Operands are MN-major (the pixel is the slow index of a channels-last row): float16 with the
 // 16-byte swizzle, tf32 with the 32-byte-atom swizzle; row offsets that are not multiples of the
@@ -81,107 +81,113 @@ __device__ __forceinline__ Item decode(uint32_t it, const GroupWgradParams& p, u
   return r;
 }
 
-// The MMAs of one stage: `ksteps` reduction steps of kK rows, NT taps each (tap q accumulates into
-// TMEM columns [q * kBN, +kBN) and reads the x tile toff[q] address units further).  Straight-line
-// code in blocks of four steps: the issuing thread must spend fewer clocks per MMA than the MMA
-// takes (64 for 128 x 128 x 8 tf32).
-template <MmaKind KIND, int NT, int KS>
-__device__ __forceinline__ void issue_stage(uint32_t tmem, uint32_t a_lo, uint32_t b_lo, const uint32_t (&toff)[4],
-                                            uint32_t desc_hi, int ksteps, uint32_t acc, uint32_t stack_delta, uint32_t box2) {
-  constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;
-  constexpr uint32_t kStep = (kK * 128) >> 4;
-  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, kBN);
-  uint32_t bq[NT];
-#pragma unroll
-  for (int q = 0; q < NT; ++q) bq[q] = b_lo + toff[q];
-  if (stack_delta) {
-    // Layers with at most 64 channels: the NT taps become NT groups of columns of ONE MMA per swizzle atom of channels
-    // (64 in float16, 32 in tf32).  The x operand's leading-dimension offset (the distance between column groups)
-    // is set to the taps' row spacing, so that column group q reads the x tile q taps further: 128 x (64 NT)
-    // (tf32: at most two of 128 x (32 NT)) instead of NT half-empty 128 x 128 MMAs.
-    constexpr int kAtom = atom<KIND>();
-    constexpr bool kPlain = NT == 1;                 // a single tap: its atoms are the column groups, as ever
-    constexpr uint32_t kIdescStack = instr_desc(KIND == MmaKind::TF32, true, true, 128, kPlain ? 64 : kAtom * NT);
-    const uint32_t b0 = bq[0] + (kPlain ? 0u : stack_delta);
-    const bool second = KIND == MmaKind::TF32 && !kPlain && box2;   // box2: distance of the second atom of channels, or 0
-    for (int ks = 0; ks < ksteps; ++ks) {
-      umma_words<KIND>(tmem, a_lo + ks * kStep, b0 + ks * kStep, desc_hi, kIdescStack, acc);
-      if (second)
-        umma_words<KIND>(tmem + kAtom * NT, a_lo + ks * kStep, b0 + box2 + ks * kStep, desc_hi, kIdescStack, acc);
-      acc = 1u;
-    }
-    return;
-  }
-  if (KS > 0) {           // exactly KS steps: straight-line code
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-#pragma unroll
-      for (int q = 0; q < NT; ++q)
-        umma_words<KIND>(tmem + q * kBN, a_lo + ks * kStep, bq[q] + ks * kStep, desc_hi, kIdesc, ks == 0 ? acc : 1u);
-    }
-    return;
-  }
-  int ks = 0;
-  for (; ks + 4 <= ksteps; ks += 4) {
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-#pragma unroll
-      for (int q = 0; q < NT; ++q)
-        umma_words<KIND>(tmem + q * kBN, a_lo + (ks + u) * kStep, bq[q] + (ks + u) * kStep, desc_hi, kIdesc,
-                         u == 0 ? acc : 1u);
-    }
-    acc = 1u;
-  }
-  for (; ks < ksteps; ++ks) {
-#pragma unroll
-    for (int q = 0; q < NT; ++q)
-      umma_words<KIND>(tmem + q * kBN, a_lo + ks * kStep, bq[q] + ks * kStep, desc_hi, kIdesc, acc);
-    acc = 1u;
-  }
-}
+// Layers with at most 64 channels (STACK): the NT taps become NT groups of columns of ONE MMA per swizzle atom of channels
+// (64 in float16, 32 in tf32).  The x operand's leading-dimension offset (the distance between column groups)
+// is set to the taps' row spacing, so that column group q reads the x tile q taps further: 128 x (64 NT)
+// (tf32: at most two of 128 x (32 NT), kStackTwice) instead of NT half-empty 128 x 128 MMAs.
+enum Stack { kWide = 0, kStack, kStackTwice };
 
-// The MMA issuer's loop over the pixel tiles (pipeline stages) of one work item with NT taps.
-// Returns false when a wait ran out.  `stage`/`phase` carry the pipeline position across items.
-template <MmaKind KIND, int NT, int KS>
-__device__ __forceinline__ bool mma_item(Bars* bars, uint32_t tmem, uint32_t lo_base, uint32_t desc_hi,
-                                         const uint32_t (&toff)[4], int ksteps, int ntiles, int& stage,
-                                         uint32_t& phase, long long& t_wait, bool timed, bool leader,
-                                         long long limit, uint32_t stack_delta, uint32_t box2,
-                                         const GroupWgradParams& p) {
-  const uint32_t a_units = (p.a_boxes * p.box_bytes) >> 4, stage_units = ((p.a_boxes + p.b_boxes) * p.box_bytes) >> 4;
+struct IssueLoop {
+  Bars* bars;
+  uint32_t tmem, lo_base, desc_hi;
+  uint32_t toff[4];                  // row offset of every tap's x operand, in descriptor address units
+  int ksteps, ntiles, stages;
+  uint32_t a_units, stage_units;     // of the dy boxes of a stage / of a stage
+  uint32_t stack_delta, box2;        // added to the x descriptor of stacked taps / distance of their second atom of channels
+  bool leader, timed;
+  long long limit;
+  // the pipeline position, carried across items
+  int stage;
+  uint32_t phase, seen;
+  long long t_wait;
+};
+
+// The MMA issuer's loop over the pixel tiles (pipeline stages) of one work item with NT taps.  Returns false when a wait
+// ran out.  Exactly KS reduction steps per stage as straight-line code, or any number (0) in blocks of four: the issuing
+// thread must spend fewer clocks per MMA than the MMA takes (64 for 128 x 128 x 8 tf32), and a taken branch between
+// two of them alone costs 65 to 85.
+template <MmaKind KIND, int NT, int KS, Stack STACK>
+__device__ __forceinline__ bool mma_item(IssueLoop& w) {
+  constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16, kAtom = atom<KIND>();
+  constexpr uint32_t kStep = (kK * 128) >> 4;
+  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, STACK == kWide ? kBN : NT == 1 ? 64 : kAtom * NT);
+  Bars* bars = w.bars;
+  const uint32_t lane = w.leader, tmem = w.tmem, desc_hi = w.desc_hi;
+  const int ntiles = w.ntiles, stages = w.stages;
+  uint32_t toff[NT];                 // of the x operand of each tap (the column groups' start, when stacked)
+#pragma unroll
+  for (int q = 0; q < NT; ++q) toff[q] = w.a_units + w.toff[q] + (STACK != kWide && NT > 1 ? w.stack_delta : 0u);
+  int stage = w.stage;
+  uint32_t phase = w.phase, seen = w.seen;
+  const int ksteps = KS ? KS : w.ksteps, half = ksteps / 2;
   uint32_t acc = 0u;
   for (int t = 0; t < ntiles; ++t) {
-    if (timed) {
-      const long long tw = clock64();
-      if (!uniform_wait(&bars->full[stage], phase, bars, limit)) return false;
-      t_wait += clock64() - tw;
-    } else if (!uniform_wait(&bars->full[stage], phase, bars, limit)) {
-      return false;
-    }
+    const long long tw = w.timed ? clock64() : 0;
+    if (!wait_seen(seen, &bars->full[stage], phase, bars, w.limit)) return false;
+    if (w.timed) w.t_wait += clock64() - tw;
     tc_fence_after();
-    const uint32_t a_lo = lo_base + stage * stage_units;
-    const uint32_t b_lo = a_lo + a_units;
-    if (leader) {
-      issue_stage<KIND, NT, KS>(tmem, a_lo, b_lo, toff, desc_hi, ksteps, acc, stack_delta, box2);
-      umma_commit(&bars->empty[stage]);
-    }
-    acc = 1u;
-    const int next = stage + 1;
-    const bool wrap = next == p.stages;
-    stage = wrap ? 0 : next;
+    const uint32_t a_lo = w.lo_base + stage * w.stage_units;
+    auto step = [&](int ks, uint32_t accumulate) {
+      const uint32_t a = a_lo + ks * kStep;
+      if (STACK == kWide) {
+#pragma unroll
+        for (int q = 0; q < NT; ++q) umma_words_if<KIND>(lane, tmem + q * kBN, a, a + toff[q], desc_hi, kIdesc, accumulate);
+      } else {
+        // (a single tap is stacked with nothing: its atoms are the column groups, as ever)
+        umma_words_if<KIND>(lane, tmem, a, a + toff[0], desc_hi, kIdesc, accumulate);
+        if (STACK == kStackTwice && NT > 1) umma_words_if<KIND>(lane, tmem + kAtom * NT, a, a + toff[0] + w.box2, desc_hi, kIdesc, accumulate);
+      }
+    };
+    auto steps = [&](int k0, int k1) {
+      if (KS) {
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+          if (ks >= k0 && ks < k1) step(ks, ks ? 1u : acc);
+        return;
+      }
+      int ks = k0;
+      for (; ks + 4 <= k1; ks += 4) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) step(ks + u, ks + u ? 1u : acc);
+      }
+      for (; ks < k1; ++ks) step(ks, ks ? 1u : acc);
+    };
+    steps(0, half);
+    const int cur = stage;
+    const bool wrap = stage + 1 == stages;
+    stage = wrap ? 0 : stage + 1;
     phase ^= wrap ? 1u : 0u;
+    seen = mbar_look(&bars->full[stage], phase);
+    steps(half, ksteps);
+    umma_commit_if(lane, &bars->empty[cur]);
+    acc = 1u;
   }
+  w.stage = stage; w.phase = phase; w.seen = seen;
   return true;
 }
 
-template <MmaKind KIND>
+template <MmaKind KIND, int NT, Stack STACK>
+__device__ __forceinline__ bool mma_item_steps(IssueLoop& w) {
+  // the usual numbers of steps: images of 7, 14, 28 and 56 columns / segments of 56
+  if (w.ksteps == 8) return mma_item<KIND, NT, 8, STACK>(w);
+  if (w.ksteps == 7) return mma_item<KIND, NT, 7, STACK>(w);
+  return mma_item<KIND, NT, 0, STACK>(w);
+}
+template <MmaKind KIND, Stack STACK>
+__device__ __forceinline__ bool mma_item_taps(IssueLoop& w, int ntap) {
+  if (ntap == 1) return mma_item_steps<KIND, 1, STACK>(w);
+  if (ntap == 2) return mma_item_steps<KIND, 2, STACK>(w);
+  if (ntap == 3) return mma_item_steps<KIND, 3, STACK>(w);
+  return mma_item_steps<KIND, 4, STACK>(w);
+}
+
+template <MmaKind KIND, Stack STACK>
 __global__ void __launch_bounds__(kThreads, 1)
 wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   constexpr int kAtom = atom<KIND>();
   constexpr int kABoxes = 128 / kAtom, kBBoxes = kBN / kAtom;
   const int box_bytes = p.box_bytes, stage_bytes = (p.a_boxes + p.b_boxes) * box_bytes;
   constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;
-  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, kBN);
   constexpr uint32_t kSbo = KIND == MmaKind::TF32 ? 512 : 1024;
   constexpr uint64_t kLayout = KIND == MmaKind::TF32 ? kSwizzle128Base32 : kSwizzle128;
 
@@ -292,46 +298,35 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
     if (trace && leader && pw == 0) { trace[2] = t_wait; trace[3] = clock64() - t_begin; }
   } else if (warp == 1) {
     // all lanes follow the loop and wait; one elected lane issues the MMAs and their commits
-    const bool leader = elect_one();
-    int stage = 0;
-    uint32_t phase = 0;
+    const uint64_t desc_bits = smem_desc(0, box_bytes, kSbo, kLayout);
+    IssueLoop w;
+    w.bars = bars; w.tmem = tmem;
+    w.lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
+    w.desc_hi = static_cast<uint32_t>(desc_bits >> 32);
+    w.ksteps = ksteps; w.stages = p.stages;
+    w.a_units = (p.a_boxes * box_bytes) >> 4; w.stage_units = stage_bytes >> 4;
+    // stacked taps: the low descriptor word carries the leading-dimension offset in bits [16, 30)
+    w.stack_delta = ((static_cast<uint32_t>(p.stack_step * 128) >> 4) - (static_cast<uint32_t>(box_bytes) >> 4)) << 16;
+    w.box2 = static_cast<uint32_t>(box_bytes) >> 4;
+    w.leader = elect_one(); w.timed = trace != nullptr;
+    w.limit = p.wait_clocks;
+    w.stage = 0; w.phase = 0; w.seen = 0; w.t_wait = 0;
     bool ok = true;
     int n = 0;
-    long long t_wait = 0;
-    const uint64_t desc_bits = smem_desc(0, box_bytes, kSbo, kLayout);
-    const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
-    const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
-    const bool timed = trace != nullptr;
-    const long long lim = p.wait_clocks;
-    // stacked taps: the low descriptor word carries the leading-dimension offset in bits [16, 30)
-    const uint32_t stack_delta = p.stack_step > 0
-        ? ((static_cast<uint32_t>(p.stack_step * 128) >> 4) - (static_cast<uint32_t>(box_bytes) >> 4)) << 16 : 0u;
-    const uint32_t box2 = p.Cg > kAtom ? static_cast<uint32_t>(box_bytes) >> 4 : 0u;      // used with stacked taps
     for (uint32_t it = blockIdx.x; it < total && ok; it += gridDim.x, ++n) {
-      const Item w = decode(it, p, per_split, pix_tiles);
-      const int first_tap = p.grp_first[w.grp], ntap = p.grp_n[w.grp];
-      // row offset of every tap's x operand, in descriptor address units (16 bytes)
-      uint32_t toff[4];
+      const Item item = decode(it, p, per_split, pix_tiles);
+      const int first_tap = p.grp_first[item.grp], ntap = p.grp_n[item.grp];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        toff[q] = q < ntap ? static_cast<uint32_t>(p.tap_off[first_tap + q]) * (128u >> 4) : 0u;
-      if (!uniform_wait(&bars->acc_empty, (n & 1) ^ 1, bars, lim)) { ok = false; break; }
+        w.toff[q] = q < ntap ? static_cast<uint32_t>(p.tap_off[first_tap + q]) * (128u >> 4) : 0u;
+      if (!uniform_wait(&bars->acc_empty, (n & 1) ^ 1, bars, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
-      const int ntiles = static_cast<int>(w.t_end - w.t_begin);
-      switch (ntap) {
-        case 1: ok = (ksteps == 8 && !timed ? mma_item<KIND, 1, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
-                                             : mma_item<KIND, 1, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
-        case 2: ok = (ksteps == 8 && !timed ? mma_item<KIND, 2, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
-                                             : mma_item<KIND, 2, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
-        case 3: ok = (ksteps == 8 && !timed ? mma_item<KIND, 3, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
-                                             : mma_item<KIND, 3, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
-        default: ok = (ksteps == 8 && !timed ? mma_item<KIND, 4, 8>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, false, leader, lim, stack_delta, box2, p)
-                                             : mma_item<KIND, 4, 0>(bars, tmem, lo_base, desc_hi, toff, ksteps, ntiles, stage, phase, t_wait, timed, leader, lim, stack_delta, box2, p)); break;
-      }
-      if (ok && leader) umma_commit(&bars->acc_full);
+      w.ntiles = static_cast<int>(item.t_end - item.t_begin);
+      ok = mma_item_taps<KIND, STACK>(w, ntap);
+      if (ok && w.leader) umma_commit(&bars->acc_full);
     }
-    if (!ok && leader) report_status(p.status, kStatusTimeout);
-    if (trace && leader) { trace[0] = t_wait; trace[1] = clock64() - t_begin; }
+    if (!ok && w.leader) report_status(p.status, kStatusTimeout);
+    if (trace && w.leader) { trace[0] = w.t_wait; trace[1] = clock64() - t_begin; }
   } else {
     const int quad = warp & 3;
     const int sub = (warp - 2) >> 2;
@@ -356,7 +351,7 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
         if (c0 >= p.Cg) continue;
         uint32_t r[32];
         // columns of tap q, channels 32 ch: side by side per tap, or per atom of channels and then per tap
-        const int col = p.stack_step > 0 ? (ch * 32 / kAtom) * (kAtom * ntap) + q * kAtom + ch * 32 % kAtom : q * kBN + ch * 32;
+        const int col = STACK != kWide ? (ch * 32 / kAtom) * (kAtom * ntap) + q * kAtom + ch * 32 % kAtom : q * kBN + ch * 32;
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + col, r);
         tmem_ld_wait();
         if (!valid) continue;
@@ -399,14 +394,14 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
   }
 }
 
-template <MmaKind KIND>
+template <MmaKind KIND, Stack STACK>
 cudaError_t launch_one(const GroupWgradParams& p, long long total, int num_sms, cudaStream_t s) {
   const int smem = p.ring_bytes + static_cast<int>(sizeof(Bars)) + 1024;
   static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_group_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(wgrad_group_kernel<KIND, STACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
   if (e != cudaSuccess) return e;
   const int grid = static_cast<int>(total < num_sms ? total : num_sms);
-  launch_chained(wgrad_group_kernel<KIND>, grid, kThreads, smem, s, p);
+  launch_chained(wgrad_group_kernel<KIND, STACK>, grid, kThreads, smem, s, p);
   return cudaGetLastError();
 }
 
@@ -429,8 +424,10 @@ cudaError_t launch_wgrad_group(const GroupWgradParams& params, int dtype, int nu
   while (p.stages > 2 && ring_bytes(p.stages, at, p.a_boxes, p.b_boxes, p.box_bytes) > kSmemBudget) --p.stages;
   p.ring_bytes = ring_bytes(p.stages, at, p.a_boxes, p.b_boxes, p.box_bytes);
   if (p.ring_bytes > kSmemBudget) return cudaErrorInvalidValue;
-  return dtype == B200CONV_F16 ? launch_one<MmaKind::F16>(p, total, num_sms, s)
-                               : launch_one<MmaKind::TF32>(p, total, num_sms, s);
+  if (dtype == B200CONV_F16)
+    return p.stack_step > 0 ? launch_one<MmaKind::F16, kStack>(p, total, num_sms, s) : launch_one<MmaKind::F16, kWide>(p, total, num_sms, s);
+  if (p.stack_step <= 0) return launch_one<MmaKind::TF32, kWide>(p, total, num_sms, s);
+  return p.Cg > at ? launch_one<MmaKind::TF32, kStackTwice>(p, total, num_sms, s) : launch_one<MmaKind::TF32, kStack>(p, total, num_sms, s);
 }
 
 }  // namespace b200

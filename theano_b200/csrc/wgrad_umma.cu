@@ -83,7 +83,7 @@ __device__ __forceinline__ Item decode(uint32_t it, const UmmaWgradParams& p, ui
 // descriptors changes from one MMA to the next: kK rows further.  Returns false when a wait ran out.
 template <MmaKind KIND, int BN, int KS, bool TIMED>
 __device__ __forceinline__ bool mma_tiles(Bars* bars, uint32_t d_tmem, uint32_t lo_base, uint32_t desc_hi,
-                                          int ksteps, int ntiles, int& stage, uint32_t& phase,
+                                          int ksteps, int ntiles, int& stage, uint32_t& phase, uint32_t& seen,
                                           long long& t_wait, bool leader, long long limit) {
   constexpr int kAtom = atom<KIND>();
   constexpr int kABoxes = 128 / kAtom;
@@ -93,32 +93,36 @@ __device__ __forceinline__ bool mma_tiles(Bars* bars, uint32_t d_tmem, uint32_t 
   constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 128, BN);
   uint32_t acc = 0u;
   for (int t = 0; t < ntiles; ++t) {
-    if (TIMED) {
-      const long long tw = clock64();
-      if (!uniform_wait(&bars->full[stage], phase, bars, limit)) return false;
-      t_wait += clock64() - tw;
-    } else if (!uniform_wait(&bars->full[stage], phase, bars, limit)) {
-      return false;
-    }
+    const long long tw = TIMED ? clock64() : 0;
+    if (!wait_seen(seen, &bars->full[stage], phase, bars, limit)) return false;
+    if (TIMED) t_wait += clock64() - tw;
     tc_fence_after();
     const uint32_t a_lo = lo_base + stage * (stage_bytes<KIND, BN>() >> 4);
     const uint32_t b_lo = a_lo + ((kABoxes * box_bytes<KIND, BN>()) >> 4);
-    if (leader) {
+    const int half = (KS > 0 ? KS : ksteps) / 2;
+    auto steps = [&](int k0, int k1) {
       if (KS > 0) {
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks)
-          umma_words<KIND>(d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks == 0 ? acc : 1u);
+          if (ks >= k0 && ks < k1)
+            umma_words<KIND>(d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks == 0 ? acc : 1u);
       } else {
-        for (int ks = 0; ks < ksteps; ++ks)
+        for (int ks = k0; ks < k1; ++ks)
           umma_words<KIND>(d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks == 0 ? acc : 1u);
       }
-      umma_commit(&bars->empty[stage]);
+    };
+    if (leader) steps(0, half);
+    __syncwarp();
+    const int cur = stage;
+    const bool wrap = stage + 1 == kStages;
+    stage = wrap ? 0 : stage + 1;
+    phase ^= wrap ? 1u : 0u;
+    seen = mbar_look(&bars->full[stage], phase);
+    if (leader) {
+      steps(half, KS > 0 ? KS : ksteps);
+      umma_commit(&bars->empty[cur]);
     }
     acc = 1u;
-    const int next = stage + 1;
-    const bool wrap = next == kStages;
-    stage = wrap ? 0 : next;
-    phase ^= wrap ? 1u : 0u;
   }
   return true;
 }
@@ -253,6 +257,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
     const uint64_t desc_bits = smem_desc(0, kBoxBytes, kSbo, kLayout);
     const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
     const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
+    uint32_t seen = 0;                           // the next stage already seen full (mbar_look)
     for (uint32_t it = blockIdx.x; it < total && ok; it += gridDim.x, ++n) {
       const Item w = decode(it, p, per_split, pix_tiles);
       const int buf = kDouble ? (n & 1) : 0;
@@ -262,11 +267,11 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
       const uint32_t d_tmem = tmem + buf * BN;
       const int ntiles = static_cast<int>(w.t_end - w.t_begin);
       // the usual step counts get straight-line MMA blocks
-      if (trace) ok = mma_tiles<KIND, BN, 0, true>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
-      else if (ksteps == 8) ok = mma_tiles<KIND, BN, 8, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
-      else if (ksteps == 7) ok = mma_tiles<KIND, BN, 7, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
-      else if (ksteps == 4) ok = mma_tiles<KIND, BN, 4, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
-      else ok = mma_tiles<KIND, BN, 0, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, t_wait, leader, p.wait_clocks);
+      if (trace) ok = mma_tiles<KIND, BN, 0, true>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, t_wait, leader, p.wait_clocks);
+      else if (ksteps == 8) ok = mma_tiles<KIND, BN, 8, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, t_wait, leader, p.wait_clocks);
+      else if (ksteps == 7) ok = mma_tiles<KIND, BN, 7, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, t_wait, leader, p.wait_clocks);
+      else if (ksteps == 4) ok = mma_tiles<KIND, BN, 4, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, t_wait, leader, p.wait_clocks);
+      else ok = mma_tiles<KIND, BN, 0, false>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, t_wait, leader, p.wait_clocks);
       if (ok && leader) umma_commit(&bars->acc_full[buf]);
     }
     if (!ok && leader) report_status(p.status, kStatusTimeout);
