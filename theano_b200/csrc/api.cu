@@ -2162,8 +2162,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   p.groups = d.groups; p.Kg = Kg; p.Cg = Cg;
   p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
   p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
-  // 256+ filters and 256+ channels in float16: pairs of CTAs compute 256 x 256 tiles and share the x tile
-  const bool pair = c->use_pair && d.dtype == B200CONV_F16 && BN == 256 && Kg >= 256 && c->num_sms >= 2;
+  // 256+ filters and 256+ channels: pairs of CTAs compute 256 x 256 tiles and share the x tile
+  const bool pair = c->use_pair && BN == 256 && Kg >= 256 && c->num_sms >= 2;
   p.ktiles = (int)cdiv(Kg, pair ? 256 : 128); p.ctiles = (int)cdiv(Cg, BN);
   p.taps_total = d.kH * d.kW;
   const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
@@ -2184,7 +2184,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     p.partial = partial;
     p.partial_elems = (long long)slab_elems * slabs;
     if (p.ntaps > 0) {
-      if (pair) KLAUNCH(c, kKWgradUmma, launch_wgrad_pair(p, c->num_sms, c->stream));
+      if (pair) KLAUNCH(c, kKWgradUmma, launch_wgrad_pair(p, d.dtype, c->num_sms, c->stream));
       else KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, BN, c->num_sms, c->stream));
     }
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, odt, c->stream));

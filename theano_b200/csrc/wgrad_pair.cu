@@ -1,14 +1,17 @@
-// Filter gradient on pairs of CTAs (tcgen05.mma.cta_group::2), float16, layers with at least 256
+// Filter gradient on pairs of CTAs (tcgen05.mma.cta_group::2), layers with at least 256
 // filters and 256 channels per group.
 //
 //   dW[tap][k, c] = sum over output pixels q of  dy[q, k] * x_view_tap[q + offset_tap, c]
 //
-// One CTA with a 128 x 256 accumulator needs, per stage of 64 pixels, 16 KB of dy and 32 KB of x from
-// L2 for 512 clocks of MMAs: 94 B/clk where an SM gets 73.  Here two CTAs of a cluster compute a tile of
+// One CTA with a 128 x 256 accumulator needs, per stage of 64 float16 pixels, 16 KB of dy and 32 KB of x from
+// L2 for 512 clocks of MMAs (float32: twice both): 94 B/clk where an SM gets 73.  Here two CTAs of a cluster compute a tile of
 // 256 filters x 256 channels together: each loads the dy rows of ITS 128 filters and HALF of the x tile
 // (128 channels) into its own shared memory with plain TMA loads, one thread of the even CTA issues MMAs
 // of M = 256 over both CTAs' operands, and each CTA's TMEM receives its 128 filter rows x 256 channels.
 // Per CTA that is 32 KB per 512 clocks: 64 B/clk.  No load is shared between CTAs by the copy engine.
+// A thread gets a box accepted every 200 to 300 clocks: a stage's four (float32: eight) boxes of 8 KB are spread over
+// four producer warps.  256 -> 256 filters 3x3 at 14x14, 128 images, float32: 62.5 us with the tap groups of one CTA, whose
+// 128 x 128 MMAs read 128 B/clk of operands from shared memory beside the copies' writes, 51 us here (64 B/clk).
 //
 // Work items, split-K slices, slab layout and the reduction kernel are those of wgrad_umma.cu; an item is
 // (256-filter tile, 256-channel tile, group, tap, slice) and both CTAs of a pair walk the same items.
@@ -19,17 +22,23 @@ namespace b200 {
 namespace {
 
 constexpr int kEpilogueWarps = 16;
-constexpr int kThreads = 32 * (2 + kEpilogueWarps);
-constexpr int kPix = kWgradPixF16Wide;                 // reduction rows (pixels) per stage: 64
-constexpr int kBoxBytes = kPix * 128;                  // one TMA box: 64 pixels x 64 channels of float16
-constexpr int kBoxes = 4;                              // per CTA and stage: 2 of dy (128 filters), 2 of x (128 channels)
-constexpr int kStageBytes = kBoxes * kBoxBytes;        // 32 KB
-constexpr int kStages = 6;
+constexpr int kProducers = 4;                          // warp 0 and the last three warps; box j of a stage belongs to producer j % 4
+constexpr int kFirstExtraProducer = 2 + kEpilogueWarps;
+constexpr int kThreads = 32 * (kFirstExtraProducer + kProducers - 1);
+constexpr int kPix = 64;                               // reduction rows (pixels) per stage
+static_assert(kPix == kWgradPixF32 && kPix == kWgradPixF16Wide, "the pixel box of a stage");
+constexpr int kBoxBytes = kPix * 128;                  // one TMA box: 64 pixels x 128 bytes of channels
 constexpr int kBN = 256;
+constexpr int kMaxStages = 6;
+
+template <MmaKind KIND> constexpr int atom() { return KIND == MmaKind::TF32 ? 32 : 64; }
+template <MmaKind KIND> constexpr int half_boxes() { return 128 / atom<KIND>(); }               // of dy (128 filters), and of x (128 channels)
+template <MmaKind KIND> constexpr int stage_bytes() { return 2 * half_boxes<KIND>() * kBoxBytes; }   // 32 / 64 KB
+template <MmaKind KIND> constexpr int num_stages() { return 192 * 1024 / stage_bytes<KIND>(); }     // 6 / 3
 
 struct alignas(16) Bars {
-  uint64_t full[kStages];        // even CTA: both CTAs' boxes of a stage have landed
-  uint64_t empty[kStages];       // each CTA: the MMAs reading the stage are done
+  uint64_t full[kMaxStages];        // even CTA: both CTAs' boxes of a stage have landed
+  uint64_t empty[kMaxStages];       // each CTA: the MMAs reading the stage are done
   uint64_t acc_full[2];          // each CTA: the item's accumulator is complete
   uint64_t acc_empty[2];         // even CTA: both CTAs' epilogues have read the accumulator
   uint32_t tmem_base;
@@ -56,11 +65,49 @@ __device__ __forceinline__ Item decode(uint32_t it, const UmmaWgradParams& p, ui
   return r;
 }
 
+// The MMAs of an item's pixel tiles: KS steps of a stage as straight-line code, 0: any number.
+template <MmaKind KIND, int KS>
+__device__ __forceinline__ bool mma_tiles(Bars* bars, uint32_t d_tmem, uint32_t lo_base, uint32_t desc_hi, int ksteps, int ntiles, int& stage,
+                                          uint32_t& phase, uint32_t& seen, bool leader, long long limit) {
+  constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;               // reduction rows per MMA
+  constexpr uint32_t kStep = (kK * 128) >> 4;
+  constexpr uint32_t kIdesc = instr_desc(KIND == MmaKind::TF32, true, true, 256, kBN);
+  const uint32_t lane = leader;
+  uint32_t acc = 0u;
+  for (int t = 0; t < ntiles; ++t) {
+    if (!wait_seen(seen, &bars->full[stage], phase, bars, limit)) return false;
+    tc_fence_after();
+    const uint32_t a_lo = lo_base + stage * (stage_bytes<KIND>() >> 4);
+    const uint32_t b_lo = a_lo + ((half_boxes<KIND>() * kBoxBytes) >> 4);
+    const int half = (KS ? KS : ksteps) / 2;
+    auto steps = [&](int k0, int k1) {
+      if (KS) {
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+          if (ks >= k0 && ks < k1) umma_words_if<KIND, true>(lane, d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks ? 1u : acc);
+      } else {
+        for (int ks = k0; ks < k1; ++ks) umma_words_if<KIND, true>(lane, d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks ? 1u : acc);
+      }
+    };
+    steps(0, half);
+    const int cur = stage;
+    if (++stage == num_stages<KIND>()) { stage = 0; phase ^= 1; }
+    seen = mbar_look(&bars->full[stage], phase);
+    steps(half, KS ? KS : ksteps);
+    if (leader) umma_commit_pair(&bars->empty[cur]);
+    acc = 1u;
+  }
+  return true;
+}
+
+template <MmaKind KIND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
-  constexpr int kK = 16;                                           // reduction rows per MMA
-  constexpr uint32_t kStep = (kK * 128) >> 4;
-  constexpr uint32_t kIdesc = instr_desc(false, true, true, 256, kBN);
+  constexpr int kK = KIND == MmaKind::TF32 ? 8 : 16;               // reduction rows per MMA
+  constexpr int kHalf = half_boxes<KIND>(), kBoxes = 2 * kHalf, kStages = num_stages<KIND>(), kStageBytes = stage_bytes<KIND>();
+  // float16: 8-row groups 1024 bytes apart, 16-byte swizzle; float32: 4-row groups 512 bytes apart, 32-byte swizzle
+  constexpr uint32_t kSbo = KIND == MmaKind::TF32 ? 512 : 1024;
+  constexpr uint64_t kLayout = KIND == MmaKind::TF32 ? kSwizzle128Base32 : kSwizzle128;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -109,7 +156,8 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
   const uint32_t tmem = bars->tmem_base;
   pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
 
-  if (warp == 0) {
+  if (warp == 0 || warp >= kFirstExtraProducer) {
+    const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
     const bool leader = elect_one();
     if (leader) {
       for (int v = 0; v < kMaxViews; ++v) tma_prefetch_desc(&p.x_views[v]);
@@ -135,11 +183,12 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
         if (!uniform_wait(&bars->empty[stage], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         uint8_t* sa = smem + stage * kStageBytes;
         if (leader) {
-          if (rank == 0) mbar_expect_tx(&bars->full[stage], tx);
-          tma_load_5d_pair(sa, &p.dy_map, &bars->full[stage], k0, w.g, w0, h0, n0);
-          tma_load_5d_pair(sa + kBoxBytes, &p.dy_map, &bars->full[stage], k0 + 64, w.g, w0, h0, n0);
-          tma_load_5d_pair(sa + 2 * kBoxBytes, &p.x_views[tp.view], &bars->full[stage], c0, w.g, w0 + tp.dw, h0 + tp.dh, n0);
-          tma_load_5d_pair(sa + 3 * kBoxBytes, &p.x_views[tp.view], &bars->full[stage], c0 + 64, w.g, w0 + tp.dw, h0 + tp.dh, n0);
+          if (rank == 0 && pw == 0) mbar_expect_tx(&bars->full[stage], tx);
+#pragma unroll
+          for (int j = pw; j < kBoxes; j += kProducers) {
+            if (j < kHalf) tma_load_5d_pair(sa + j * kBoxBytes, &p.dy_map, &bars->full[stage], k0 + j * atom<KIND>(), w.g, w0, h0, n0);
+            else tma_load_5d_pair(sa + j * kBoxBytes, &p.x_views[tp.view], &bars->full[stage], c0 + (j - kHalf) * atom<KIND>(), w.g, w0 + tp.dw, h0 + tp.dh, n0);
+          }
         }
         if (++stage == kStages) { stage = 0; phase ^= 1; }
       }
@@ -151,30 +200,21 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
       int stage = 0, n = 0;
       uint32_t phase = 0;
       bool ok = true;
-      const uint64_t desc_bits = smem_desc(0, kBoxBytes, 1024, kSwizzle128);
+      uint32_t seen = 0;                                             // the next stage already seen full (mbar_look)
+      const uint64_t desc_bits = smem_desc(0, kBoxBytes, kSbo, kLayout);
       const uint32_t desc_hi = static_cast<uint32_t>(desc_bits >> 32);
       const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
       for (uint32_t it = pair; it < total && ok; it += npairs, ++n) {
         const Item w = decode(it, p, per_split, pix_tiles);
-        const int buf = n & 1;
+        const int buf = n & 1, ntiles = static_cast<int>(w.t_end - w.t_begin);
         const uint32_t aphase = (n >> 1) & 1;
         if (!uniform_wait(&bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem + buf * kBN;
-        uint32_t acc = 0u;
-        for (uint32_t t = w.t_begin; t < w.t_end; ++t) {
-          if (!uniform_wait(&bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t a_lo = lo_base + stage * (kStageBytes >> 4);
-          const uint32_t b_lo = a_lo + ((2 * kBoxBytes) >> 4);
-          if (leader) {
-            for (int ks = 0; ks < ksteps; ++ks)
-              umma_words_pair_f16(d_tmem, a_lo + ks * kStep, b_lo + ks * kStep, desc_hi, kIdesc, ks == 0 ? acc : 1u);
-            umma_commit_pair(&bars->empty[stage]);
-          }
-          acc = 1u;
-          if (++stage == kStages) { stage = 0; phase ^= 1; }
-        }
+        if (ksteps == 8) ok = mma_tiles<KIND, 8>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, leader, p.wait_clocks);
+        else if (ksteps == 7) ok = mma_tiles<KIND, 7>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, leader, p.wait_clocks);
+        else if (ksteps == 4) ok = mma_tiles<KIND, 4>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, leader, p.wait_clocks);
+        else ok = mma_tiles<KIND, 0>(bars, d_tmem, lo_base, desc_hi, ksteps, ntiles, stage, phase, seen, leader, p.wait_clocks);
         if (ok && leader) umma_commit_pair(&bars->acc_full[buf]);
       }
       if (!ok && leader) report_status(p.status, kStatusTimeout);
@@ -243,22 +283,27 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
   }
 }
 
+template <MmaKind KIND>
+cudaError_t launch_one(const UmmaWgradParams& p, long long total, int num_sms, cudaStream_t s) {
+  constexpr int smem = num_stages<KIND>() * stage_bytes<KIND>() + sizeof(Bars) + 1024;
+  static PerDeviceOnce configured;
+  cudaError_t e = configured.ensure([] {
+    return cudaFuncSetAttribute(wgrad_pair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
+  if (e != cudaSuccess) return e;
+  const long long pairs = std::min<long long>(total, num_sms / 2);
+  launch_chained(wgrad_pair_kernel<KIND>, static_cast<int>(2 * pairs), kThreads, smem, s, p);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
-cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int num_sms, cudaStream_t s) {
+cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int dtype, int num_sms, cudaStream_t s) {
   const long long total = 1LL * p.ktiles * p.ctiles * p.groups * p.ntaps * p.splits;
   if (total == 0) return cudaSuccess;
   if (total >= (1LL << 31) || 1LL * p.tiles_w * p.tiles_h * p.tiles_n >= (1LL << 31) || p.bw * p.bh * p.bn > kPix)
     return cudaErrorInvalidValue;
-  constexpr int smem = kStages * kStageBytes + sizeof(Bars) + 1024;
-  static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] {
-    return cudaFuncSetAttribute(wgrad_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  });
-  if (e != cudaSuccess) return e;
-  const long long pairs = std::min<long long>(total, num_sms / 2);
-  launch_chained(wgrad_pair_kernel, static_cast<int>(2 * pairs), kThreads, smem, s, p);
-  return cudaGetLastError();
+  return dtype == B200CONV_F16 ? launch_one<MmaKind::F16>(p, total, num_sms, s) : launch_one<MmaKind::TF32>(p, total, num_sms, s);
 }
 
 }  // namespace b200
