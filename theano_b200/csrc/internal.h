@@ -254,7 +254,8 @@ struct alignas(64) UmmaWgradParams {
   int tiles_w, tiles_h, tiles_n; // pixel tiles covering (Wo, Ho, N)
   int ktiles, ctiles;            // 128-filter tiles, BN-channel tiles
   int splits;                    // split-K slices
-  float* partial;                // [splits][taps_total][K][Cg] float32 (or the final buffer)
+  float* partial;                // one float32 slab per slice (wgrad_slab.cuh)
+  int diag_c, diag_k;            // merged groups of diag_k filters x diag_c channels: only their blocks are stored; 0: everything
   long long partial_elems;       // its extent (checked in the range-checked build)
   int taps_total;                // kH*kW
   int atomic;                    // 1: red.add into partial[0] instead of per-split slabs
@@ -279,9 +280,9 @@ cudaError_t launch_wgrad_umma(const UmmaWgradParams& p, int dtype, int bn_cols, 
 // The same work on pairs of CTAs (wgrad_pair.cu): 256-filter x 256-channel tiles, stages of 64 pixels;
 // `ktiles` / `ctiles` count 256-wide tiles.
 cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int dtype, int num_sms, cudaStream_t s);
-// Sums split-K slabs and writes the OIHW gradient: out[k][c][tap] = sum_s partial[s][tap][k][c].
-cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K,
-                                int Cg, int dtype, cudaStream_t s);
+// Sums split-K slabs and writes the OIHW gradient; diag_c / diag_k as above (Kg: filters per merged group).
+cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K, int Cg, int Kg, int diag_c, int diag_k,
+                                int dtype, cudaStream_t s);
 
 // ---- filter gradient with tap groups sharing their operands (wgrad_group.cu) -------------
 // Taps that read the same view with the same row offset differ only by a column offset.  With
@@ -309,7 +310,8 @@ struct alignas(64) GroupWgradParams {
   int tiles_w, tiles_h, tiles_n;
   int ktiles, ctiles;
   int splits;
-  float* partial;                  // [splits][taps_total][K][Cg]
+  float* partial;                  // one float32 slab per slice (wgrad_slab.cuh)
+  int diag_c, diag_k;              // merged groups of diag_k filters x diag_c channels: only their blocks are stored; 0: everything
   long long partial_elems;         // its extent (checked in the range-checked build)
   int taps_total;
   int atomic;

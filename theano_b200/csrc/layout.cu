@@ -1,6 +1,9 @@
 // Memory-bound helper kernels: NCHW <-> channels-last transposes, filter packing for the
 // implicit-GEMM kernels, bias conversion, 2x2 max pooling and the L2 flush.
+#include <algorithm>
+
 #include "internal.h"
+#include "wgrad_slab.cuh"
 
 namespace b200 {
 namespace {
@@ -260,51 +263,64 @@ __global__ void pack_filters_s2d_kernel(const T* __restrict__ w, T* __restrict__
   }
 }
 
-// Filter gradient of the space-to-depth form: dw[k][c][i'][j'] = sum_s partial[s][t][k][col] with
+// Adds the slabs (wgrad_slab.cuh, rows of ld columns) of a gradient whose columns are not the filters' own channels: place(c, i', j') gives
+// the slab tap and column of a filter element.  A block takes 32 filters of one element: neighbouring threads read neighbouring
+// filters (16 bytes apart), eight threads share a sum (slabs l, l + 8, ..., then in order of l), so that a chain of loads
+// is an eighth of the slices long.
+template <typename T, class Place>
+__device__ __forceinline__ void reduce_gathered(const float* __restrict__ partial, T* __restrict__ dw, int splits, int K, int C, int kH, int kW,
+                                                int ntaps, int ld, Place place) {
+  __shared__ float part[8][32];
+  const int kk = threadIdx.x & 31, lane = threadIdx.x >> 5, per_k = C * kH * kW, ktiles = (K + 31) / 32;
+  const long long slab = 1LL * ntaps * K * ld;
+  for (long long tl = blockIdx.x; tl < 1LL * per_k * ktiles; tl += gridDim.x) {
+    const int e = static_cast<int>(tl % per_k), k = static_cast<int>(tl / per_k) * 32 + kk;
+    const int wj = e % kW, wi = (e / kW) % kH, c = e / (kW * kH);
+    float acc = 0.f;
+    if (k < K) {
+      int t, col;
+      place(c, wi, wj, &t, &col);
+      const float* src = partial + slab_index(t, k, col, K, ld);
+#pragma unroll 8
+      for (int s = lane; s < splits; s += 8) acc += src[s * slab];
+    }
+    part[lane][kk] = acc;
+    __syncthreads();
+    if (lane == 0 && k < K) {
+      for (int l = 1; l < 8; ++l) acc += part[l][kk];
+      dw[1LL * k * per_k + e] = static_cast<T>(acc);
+    }
+    __syncthreads();
+  }
+}
+
+// Filter gradient of the space-to-depth form: dw[k][c][i'][j'] = sum_s slab s[t][k][col] with
 // (t, col) the place pack_filters_s2d_kernel gives tap (i, jj).
 template <typename T>
-__global__ void wgrad_reduce_s2d_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits,
+__global__ void __launch_bounds__(256) wgrad_reduce_s2d_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits,
                                         int K, int C, int kH, int kW, int ntaps, int t0, int q0, int padH,
                                         int padW, int ld, int flip) {
   pdl_enter();
-  const long long total = 1LL * K * C * kH * kW;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int wj = idx % kW;
-    const int wi = (idx / kW) % kH;
-    const int c = (idx / (1LL * kW * kH)) % C;
-    const int k = idx / (1LL * kW * kH * C);
+  reduce_gathered(partial, dw, splits, K, C, kH, kW, ntaps, ld, [=](int c, int wi, int wj, int* t, int* col) {
     const int i = flip ? kH - 1 - wi : wi, jj = flip ? kW - 1 - wj : wj;
     const int ah = i - padH, aw = jj - padW;                 // offsets from 2 * the output position
     const int th = ah >= 0 ? ah / 2 : -((1 - ah) / 2), tw = aw >= 0 ? aw / 2 : -((1 - aw) / 2);   // floor
     const int par = (ah - 2 * th) * 2 + (aw - 2 * tw);
-    const int t = th - t0, col = (tw - q0) * kS2dChannels + par * C + c;
-    float acc = 0.f;
-    for (int s = 0; s < splits; ++s)
-      acc += partial[((1LL * s * ntaps + t) * K + k) * ld + col];
-    dw[idx] = static_cast<T>(acc);
-  }
+    *t = th - t0;
+    *col = (tw - q0) * kS2dChannels + par * C + c;
+  });
 }
 
-// Folded filter gradient: dw[k][c][i'][j'] = sum_s partial[s][i][k][j*Cp + c].
+// Folded filter gradient: dw[k][c][i'][j'] = sum_s slab s[i][k][j*Cp + c].
 template <typename T>
-__global__ void wgrad_reduce_fold_kernel(const float* __restrict__ partial, T* __restrict__ dw,
+__global__ void __launch_bounds__(256) wgrad_reduce_fold_kernel(const float* __restrict__ partial, T* __restrict__ dw,
                                          int splits, int K, int C, int kH, int kW, int Cp, int ld,
                                          int flip) {
   pdl_enter();
-  const long long total = 1LL * K * C * kH * kW;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int wj = idx % kW;
-    const int wi = (idx / kW) % kH;
-    const int c = (idx / (1LL * kW * kH)) % C;
-    const int k = idx / (1LL * kW * kH * C);
-    const int i = flip ? kH - 1 - wi : wi, j = flip ? kW - 1 - wj : wj;
-    float acc = 0.f;
-    for (int s = 0; s < splits; ++s)
-      acc += partial[((1LL * s * kH + i) * K + k) * ld + j * Cp + c];
-    dw[idx] = static_cast<T>(acc);
-  }
+  reduce_gathered(partial, dw, splits, K, C, kH, kW, kH, ld, [=](int c, int wi, int wj, int* t, int* col) {
+    *t = flip ? kH - 1 - wi : wi;
+    *col = (flip ? kW - 1 - wj : wj) * Cp + c;
+  });
 }
 
 // Grouped convolutions with few channels per group: m neighbouring groups are merged into one
@@ -644,16 +660,19 @@ cudaError_t launch_pack_filters_fold(const void* w, void* dst, int K, int C, int
   return cudaGetLastError();
 }
 
+// Blocks of reduce_gathered: one per element and 32 filters, at most what fills the device a few times.
+static int gather_grid(int K, long long total) { return static_cast<int>(std::min<long long>(total / K * ((K + 31) / 32), 148 * 16)); }
+
 cudaError_t launch_wgrad_reduce_s2d(const float* partial, void* dw, int splits, int K, int C, int kH,
                                     int kW, int ntaps, int t0, int q0, int padH, int padW, int ld, int flip,
                                     int dtype, cudaStream_t s) {
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    launch_streaming(wgrad_reduce_s2d_kernel<__half>, grid_for(total, 256), 256, 0, s,
+    launch_streaming(wgrad_reduce_s2d_kernel<__half>, gather_grid(K, total), 256, 0, s,
         partial, static_cast<__half*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   else
-    launch_streaming(wgrad_reduce_s2d_kernel<float>, grid_for(total, 256), 256, 0, s,
+    launch_streaming(wgrad_reduce_s2d_kernel<float>, gather_grid(K, total), 256, 0, s,
         partial, static_cast<float*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   return cudaGetLastError();
 }
@@ -702,10 +721,10 @@ cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits,
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    launch_streaming(wgrad_reduce_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
+    launch_streaming(wgrad_reduce_fold_kernel<__half>, gather_grid(K, total), 256, 0, s,
         partial, static_cast<__half*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
   else
-    launch_streaming(wgrad_reduce_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
+    launch_streaming(wgrad_reduce_fold_kernel<float>, gather_grid(K, total), 256, 0, s,
         partial, static_cast<float*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
   return cudaGetLastError();
 }

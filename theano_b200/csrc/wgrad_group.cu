@@ -21,6 +21,7 @@
 
 #include "internal.h"
 #include "ptx.cuh"
+#include "wgrad_slab.cuh"
 
 namespace b200 {
 namespace {
@@ -341,8 +342,8 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
       tc_fence_after();
       const int kq = w.kt * 128 + row;
       const bool valid = kq < p.Kg;
-      const int slab = p.atomic ? 0 : w.sp;
-      const bool vec = (p.Cg & 3) == 0 && !p.atomic;
+      int c_lo, c_hi;
+      diagonal_range(p.diag_c, p.diag_k, kq, p.Cg, &c_lo, &c_hi);
       const int items = ntap * (kBN / 32);
 #pragma unroll 1
       for (int item = sub; item < items; item += kEpilogueWarps / 4) {
@@ -355,25 +356,8 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + col, r);
         tmem_ld_wait();
         if (!valid) continue;
-        float* dst = p.partial +
-                     ((1LL * slab * p.taps_total + p.tap_wmat[first_tap + q]) * K + w.g * p.Kg + kq) * p.Cg;
-        if (vec) {
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j + 4 <= p.partial_elems, p.status))
-              *reinterpret_cast<float4*>(dst + c0 + j) =
-                  make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]),
-                              __uint_as_float(r[j + 3]));
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j < p.partial_elems, p.status)) {
-              if (p.atomic) atomicAdd(dst + c0 + j, __uint_as_float(r[j]));
-              else dst[c0 + j] = __uint_as_float(r[j]);
-            }
-          }
-        }
+        float* slab = p.partial + (1LL * (p.atomic ? 0 : w.sp) * p.taps_total + p.tap_wmat[first_tap + q]) * K * p.Cg;
+        store_slab_chunk(r, slab, c0, c_lo, c_hi, p.Cg, K, w.g * p.Kg + kq, p.atomic, p.partial, p.partial_elems, p.status);
       }
       tc_fence_before();
       mbar_arrive(&bars->acc_empty);

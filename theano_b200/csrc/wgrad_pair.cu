@@ -17,6 +17,7 @@
 // (256-filter tile, 256-channel tile, group, tap, slice) and both CTAs of a pair walk the same items.
 #include "internal.h"
 #include "ptx.cuh"
+#include "wgrad_slab.cuh"
 
 namespace b200 {
 namespace {
@@ -221,7 +222,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
     }
   } else {
     // Epilogue, 16 warps: warp w reads TMEM lanes [32 * (w % 4), +32) = 32 of this CTA's 128 filter rows and,
-    // of those, every fourth 32-column chunk; rows go to the item's slab [slice][tap][K][C/g].
+    // of those, every fourth 32-column chunk; rows go to the item's slab.
     const int quad = warp & 3;
     const int sub = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
@@ -236,9 +237,9 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
       tc_fence_after();
       const int kq = w.kt * 256 + static_cast<int>(rank) * 128 + row;
       const bool valid = kq < p.Kg;
-      const int slab = p.atomic ? 0 : w.sp;
-      float* dst = p.partial + ((1LL * slab * p.taps_total + p.taps[w.tap].wmat) * K + w.g * p.Kg + kq) * p.Cg;
-      const bool vec = (p.Cg & 3) == 0 && !p.atomic;
+      float* slab = p.partial + (1LL * (p.atomic ? 0 : w.sp) * p.taps_total + p.taps[w.tap].wmat) * K * p.Cg;
+      int c_lo, c_hi;
+      diagonal_range(p.diag_c, p.diag_k, kq, p.Cg, &c_lo, &c_hi);
 #pragma unroll 1
       for (int ch = sub; ch < kBN / 32; ch += kEpilogueWarps / 4) {
         const int c0 = w.ct * kBN + ch * 32;
@@ -246,24 +247,7 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
         uint32_t r[32];
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * kBN + ch * 32, r);
         tmem_ld_wait();
-        if (valid) {
-          if (vec) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j + 4 <= p.partial_elems, p.status))
-                *reinterpret_cast<float4*>(dst + c0 + j) =
-                    make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j < p.partial_elems, p.status)) {
-                if (p.atomic) atomicAdd(dst + c0 + j, __uint_as_float(r[j]));
-                else dst[c0 + j] = __uint_as_float(r[j]);
-              }
-            }
-          }
-        }
+        if (valid) store_slab_chunk(r, slab, c0, c_lo, c_hi, p.Cg, K, w.g * p.Kg + kq, p.atomic, p.partial, p.partial_elems, p.status);
       }
       // every epilogue warp of this CTA has read its part: one arrival per CTA on the even CTA's barrier
       tc_fence_before();

@@ -13,11 +13,11 @@
 // 16 epilogue warps.
 // Work item = (filter tile, channel tile, group, tap, split-K slice).  Each item reduces its
 // slice of the pixel tiles into a TMEM accumulator (128 filters x BN channels, float32) and
-// writes it to its own slab of the partial buffer, laid out [slice][tap][K][C/groups] so the
-// stores are contiguous along c.  A second kernel adds the slabs in slice order (so the
-// result does not depend on scheduling) and writes OIHW.
+// writes it to its own slab of the partial buffer (wgrad_slab.cuh).  A second kernel adds the slabs in
+// slice order (so the result does not depend on scheduling) and writes OIHW.
 #include "internal.h"
 #include "ptx.cuh"
+#include "wgrad_slab.cuh"
 
 namespace b200 {
 namespace {
@@ -292,10 +292,9 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
       tc_fence_after();
       const int kq = w.kt * 128 + row;
       const bool valid = kq < p.Kg;
-      const int slab = p.atomic ? 0 : w.sp;
-      float* dst = p.partial +
-                   ((1LL * slab * p.taps_total + p.taps[w.tap].wmat) * K + w.g * p.Kg + kq) * p.Cg;
-      const bool vec = (p.Cg & 3) == 0 && !p.atomic;
+      float* slab = p.partial + (1LL * (p.atomic ? 0 : w.sp) * p.taps_total + p.taps[w.tap].wmat) * K * p.Cg;
+      int c_lo, c_hi;
+      diagonal_range(p.diag_c, p.diag_k, kq, p.Cg, &c_lo, &c_hi);
 #pragma unroll 1
       for (int ch = sub; ch < BN / 32; ch += kEpilogueWarps / 4) {
         const int c0 = w.ct * BN + ch * 32;
@@ -303,25 +302,7 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
         uint32_t r[32];
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
         tmem_ld_wait();
-        if (valid) {
-          if (vec) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j + 4 <= p.partial_elems, p.status))
-                *reinterpret_cast<float4*>(dst + c0 + j) =
-                    make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              if (c0 + j < p.Cg && B200_IN_RANGE((dst - p.partial) + c0 + j >= 0 && (dst - p.partial) + c0 + j < p.partial_elems, p.status)) {
-                if (p.atomic) atomicAdd(dst + c0 + j, __uint_as_float(r[j]));
-                else dst[c0 + j] = __uint_as_float(r[j]);
-              }
-            }
-          }
-        }
+        if (valid) store_slab_chunk(r, slab, c0, c_lo, c_hi, p.Cg, K, w.g * p.Kg + kq, p.atomic, p.partial, p.partial_elems, p.status);
       }
       tc_fence_before();
       mbar_arrive(&bars->acc_empty[buf]);
@@ -342,71 +323,70 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
   }
 }
 
-// out[k][c][tap] = sum_s partial[s][tap][k][c].  A block takes `elems` consecutive (k, c) elements and
-// all taps: (elems / 4) * taps groups of four, each added by `lanes` threads: lane q takes the slabs
-// q, q + lanes, ... in that order and the partial sums are then added in lane order, so the result
-// does not depend on scheduling (it is the same on every run).  The sums go to shared memory in
-// output order [element][tap] and leave as one contiguous run of elems * taps values.
+// out[k][c][tap] = sum over the slices of their slabs (wgrad_slab.cuh).  A block takes 2^log_k filters x 2^log_q groups
+// of four channels x all taps, one thread per four channels and share of the slices; neighbouring threads take neighbouring filters, 16 bytes
+// apart in a slab.  Each sum is split over 2^log_lanes threads: lane l takes the slabs l, l + lanes, ... in that order and the
+// partial sums are then added in lane order, so the result does not depend on scheduling (it is the same on every run).
+// The sums go to shared memory in output order [filter][channel][tap] (rows an odd number of words apart) and leave as
+// one contiguous run per filter.
 // The slabs are read once, from L2 or HBM; what bounds the kernel below a few megabytes is the length
-// of the chain of loads in a thread, so small gradients get small blocks (16 elements: two rounds of
-// 256 threads for a 3x3 filter; 64 x 64 x 3x3 float16: 7.5 -> 3 us) and only long sums are split over lanes.
+// of the chain of loads in a thread, so a block is one round of loads (up to 640 threads) and long sums are split over lanes.
+// diag_c / diag_k: only the diagonal blocks of merged groups are there and wanted (diag_c channels per filter, starting at the block of the
+// filter), 0: all.
 template <typename T>
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ dw,
-                                                            int splits, int taps, long long kc, int log_elems, int log_lanes) {
+__global__ void __launch_bounds__(640, 2) wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits, int taps, int K,
+                                                               int Cg, int Kg, int diag_c, int diag_k, int log_k, int log_q, int log_lanes) {
   pdl_enter();
-  extern __shared__ float tile[];
-  __shared__ float4 part[256];
-  const int elems = 1 << log_elems, lanes = 1 << log_lanes, slots = 256 >> log_lanes;
-  const int lane = threadIdx.x >> (8 - log_lanes), slot = threadIdx.x & (slots - 1);
-  const long long tiles = (kc + elems - 1) >> log_elems, slab = taps * kc;
-  const bool vec = (kc & 3) == 0;
-  const int units = (elems >> 2) * taps;
-  for (long long tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
-    const long long e0 = tl << log_elems;
-    const int ne = static_cast<int>(kc - e0 < elems ? kc - e0 : elems);
-    for (int base = 0; base < units; base += slots) {
-      const int u = base + slot, t = u >> (log_elems - 2), e = (u & ((elems >> 2) - 1)) << 2;
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (u < units && e < ne) {
-        const float* src = partial + 1LL * t * kc + e0 + e;
-        if (vec) {
-#pragma unroll 8
-          for (int s = lane; s < splits; s += lanes) {
-            const float4 v = *reinterpret_cast<const float4*>(src + s * slab);
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-          }
-        } else {
+  extern __shared__ float4 shared[];
+  const int kt = 1 << log_k, nq = 1 << log_q, lanes = 1 << log_lanes;
+  const int cols = diag_c ? diag_c : Cg;                      // channels per filter of the result
+  const int pitch = (4 * nq * taps) | 1, units = (kt << log_q) * taps;
+  float4* part = shared;                                      // [lane - 1][unit]
+  float* tile = reinterpret_cast<float*>(shared + (lanes - 1) * units);
+  const int lane = threadIdx.x / units, u = threadIdx.x - lane * units;
+  const int kk = u & (kt - 1), q = (u >> log_k) & (nq - 1), t = u >> (log_k + log_q);
+  const long long slab = 1LL * taps * K * Cg;
+  const int qtiles = (cols + 4 * nq - 1) / (4 * nq);
+  const bool whole = (((1LL * K * Cg) & 3) | (cols & 3) | (diag_c & 3)) == 0;
+  const int k0 = static_cast<int>(blockIdx.x) / qtiles << log_k, c0 = static_cast<int>(blockIdx.x) % qtiles * 4 * nq;
+  const int k = k0 + kk, co = c0 + 4 * q;                     // filter, first channel of the result
+  const bool on = lane < lanes && k < K && co < cols;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (on) {
+    const int c = co + (diag_c ? k % Kg / diag_k * diag_c : 0);
+    if (whole) {
+      const float4* src = reinterpret_cast<const float4*>(partial + slab_index(t, k, c, K, Cg)) + lane * (slab >> 2);
+      const long long step = lanes * (slab >> 2);
 #pragma unroll 4
-          for (int s = lane; s < splits; s += lanes) {
-            const float* ps = src + s * slab;
-            acc.x += ps[0];
-            if (e + 1 < ne) acc.y += ps[1];
-            if (e + 2 < ne) acc.z += ps[2];
-            if (e + 3 < ne) acc.w += ps[3];
-          }
-        }
+      for (int s = lane; s < splits; s += lanes, src += step) {
+        const float4 v = *src;
+        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
       }
-      if (lanes > 1) {
-        part[threadIdx.x] = acc;
-        __syncthreads();
-        if (lane == 0)
-          for (int l = 1; l < lanes; ++l) {
-            const float4 v = part[l * slots + slot];
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-          }
+    } else {
+      float* a = &acc.x;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (co + e >= cols) continue;
+        const float* src = partial + slab_index(t, k, c + e, K, Cg);
+        for (int s = lane; s < splits; s += lanes) a[e] += src[s * slab];
       }
-      if (lane == 0 && u < units && e < ne) {
-        tile[(e + 0) * taps + t] = acc.x;
-        tile[(e + 1) * taps + t] = acc.y;
-        tile[(e + 2) * taps + t] = acc.z;
-        tile[(e + 3) * taps + t] = acc.w;
-      }
-      if (lanes > 1) __syncthreads();
     }
-    __syncthreads();
-    T* dst = dw + e0 * taps;
-    for (int i = threadIdx.x; i < ne * taps; i += 256) dst[i] = static_cast<T>(tile[i]);
-    __syncthreads();
+    if (lane > 0) part[(lane - 1) * units + u] = acc;
+  }
+  if (lanes > 1) __syncthreads();
+  if (lane == 0 && on) {
+    for (int l = 0; l < lanes - 1; ++l) {
+      const float4 v = part[l * units + u];
+      acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+    }
+    float* dst = tile + kk * pitch + 4 * q * taps + t;
+    dst[0] = acc.x; dst[taps] = acc.y; dst[2 * taps] = acc.z; dst[3 * taps] = acc.w;
+  }
+  __syncthreads();
+  const int run = min(4 * nq, cols - c0) * taps;
+  for (int row = threadIdx.x >> 5; row < kt && k0 + row < K; row += blockDim.x >> 5) {
+    T* dst = dw + (1LL * (k0 + row) * cols + c0) * taps;
+    for (int i = threadIdx.x & 31; i < run; i += 32) dst[i] = static_cast<T>(tile[row * pitch + i]);
   }
 }
 
@@ -442,24 +422,26 @@ cudaError_t launch_wgrad_umma(const UmmaWgradParams& p, int dtype, int bn_cols, 
   return cudaErrorInvalidValue;
 }
 
-cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K,
-                                int Cg, int dtype, cudaStream_t s) {
-  const long long kc = 1LL * K * Cg;
-  if (kc == 0 || taps == 0) return cudaSuccess;
-  // 128 elements per block, fewer while that leaves SMs without two blocks; 2^log_lanes threads per
-  // sum: about four slabs each, at most 8 threads
-  int log_elems = 7, log_lanes = 0;
-  while (log_elems > 4 && (kc >> log_elems) < 2 * 148) --log_elems;
+cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K, int Cg, int Kg, int diag_c, int diag_k,
+                                int dtype, cudaStream_t s) {
+  if (1LL * K * Cg == 0 || taps == 0) return cudaSuccess;
+  const int cols = diag_c ? diag_c : Cg;
+  // About four slabs per thread, at most 8 threads per sum; as many channels as make a filter's run 128 bytes; up to 32 filters
+  // in a block of at most 640 threads, fewer while that leaves SMs without three blocks.
+  int log_k = 5, log_q = 0, log_lanes = 0;
   while (log_lanes < 3 && splits > (4 << log_lanes)) ++log_lanes;
-  long long g = (kc + (1 << log_elems) - 1) >> log_elems;
-  if (g > 148 * 16) g = 148 * 16;
-  const size_t smem = sizeof(float) * taps << log_elems;
+  while (log_q < 4 && (4 << log_q) < cols && (4 << log_q) * taps * static_cast<int>(elem_size(dtype)) < 128) ++log_q;
+  auto blocks = [&] { return ((cols + (4 << log_q) - 1) / (4 << log_q)) * static_cast<long long>((K + (1 << log_k) - 1) >> log_k); };
+  while (log_k > 2 && ((taps << (log_k + log_q + log_lanes)) > 640 || (1 << (log_k - 1)) >= K || blocks() < 3 * 148)) --log_k;
+  while (log_lanes > 0 && (taps << (log_k + log_q + log_lanes)) > 640) --log_lanes;
+  while (log_q > 0 && ((taps << (log_k + log_q + log_lanes)) > 640 || blocks() < 2 * 148)) --log_q;
+  if (blocks() >= (1LL << 31)) return cudaErrorInvalidValue;
+  const int units = taps << (log_k + log_q), threads = ((units << log_lanes) + 31) / 32 * 32, g = static_cast<int>(blocks());
+  const size_t smem = sizeof(float4) * ((1 << log_lanes) - 1) * units + (sizeof(float) * (((4 << log_q) * taps) | 1) << log_k);
   if (dtype == B200CONV_F16)
-    launch_streaming(wgrad_reduce_kernel<__half>, static_cast<int>(g), 256, smem, s,
-        partial, static_cast<__half*>(dw), splits, taps, kc, log_elems, log_lanes);
+    launch_streaming(wgrad_reduce_kernel<__half>, g, threads, smem, s, partial, static_cast<__half*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes);
   else
-    launch_streaming(wgrad_reduce_kernel<float>, static_cast<int>(g), 256, smem, s,
-        partial, static_cast<float*>(dw), splits, taps, kc, log_elems, log_lanes);
+    launch_streaming(wgrad_reduce_kernel<float>, g, threads, smem, s, partial, static_cast<float*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes);
   return cudaGetLastError();
 }
 
