@@ -64,11 +64,14 @@ enum {
   B200CONV_DW_F32 = 1 << 12,     /* gradWeights: store dw as float32 even for float16 tensors (the sum
                                     is float32 anyway); for gradient buckets that are all-reduced in
                                     float32 */
-  B200CONV_POOL2X2 = 1 << 13     /* forward, channels-last device tensors: y = maxpool2x2(act(conv + bias)) in one
+  B200CONV_POOL2X2 = 1 << 13,    /* forward, channels-last device tensors: y = maxpool2x2(act(conv + bias)) in one
                                     kernel (Pool{ignore_border=True, mode='max'} with ws = stride = (2, 2),
                                     theano/tensor/signal/pool.py:524-574, applied in the epilogue); y is
                                     [N][Ho/2][Wo/2][Kp]; Ho and Wo must be even; geometries whose epilogue cannot pool
                                     return B200CONV_E_UNSUPPORTED (run the two calls instead) */
+  B200CONV_ROWS = 1 << 14,       /* gradWeights: the kernel that stacks the filter's rows and columns inside one MMA
+                                    wherever it applies, timed or not */
+  B200CONV_NO_ROWS = 1 << 15     /* gradWeights: never that kernel */
 };
 
 /*
@@ -310,7 +313,8 @@ int b200conv_selftest_wait(b200conv_ctx* ctx);
 const char* b200conv_last_algo(b200conv_ctx* ctx);
 /* The kernel variant of the last tensor-core launch of a forward or gradInputs call: "tap", "tap split", "slab", "slab split",
  * "slab pair", "slab classes", "slab classes pair" or "gemm pair" (split: the reduction in slices that a second kernel adds;
- * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch). */
+ * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch); after gradWeights of a narrow
+ * layer by the kernel that stacks filter rows "wgrad rows". */
 const char* b200conv_last_variant(b200conv_ctx* ctx);
 /* Writes `bytes` of device scratch to evict the L2 cache between timed iterations. */
 int b200conv_flush_l2(b200conv_ctx* ctx);

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <initializer_list>
 #include <mutex>
@@ -84,7 +85,7 @@ struct GeoHash {
     return h ^ (h >> 29);
   }
 };
-enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance, kGeoClasses };      // kinds (first integer of a key)
+enum { kGeoSlab = 1, kGeoTile, kGeoConv, kGeoWgrad, kGeoSplits, kGeoBalance, kGeoClasses, kGeoRows };      // kinds (first integer of a key)
 
 // Tile of a convolution kernel for one geometry (the result of a search).
 struct SlabTile {
@@ -1889,6 +1890,145 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
   return 0;
 }
 
+// The taps of one stride parity class of x: filter rows x filter columns.
+struct RowsView {
+  std::vector<int> dh, dw;           // offsets of the filter rows / columns in the view's pixels, ascending
+  std::vector<int> tap;              // [row][column]
+  std::function<int(CUtensorMap*, int, int)> map;      // tensor map with a box of (columns, rows)
+};
+
+// The views of a plain layer for wgrad_rows (channels-last x of C channels); `dropped`: taps that read nothing.
+std::vector<RowsView> rows_views(b200conv_ctx* c, const b200conv_desc& d, const void* xin, bool* dropped) {
+  const int atom = d.dtype == B200CONV_F16 ? 64 : 32;
+  std::vector<RowsView> views;
+  *dropped = false;
+  for (int rh = 0; rh < d.sH; ++rh)
+    for (int rw = 0; rw < d.sW; ++rw) {
+      std::vector<int> is, js;
+      for (int i = 0; i < d.kH; ++i) if (pymod(i * d.dilH - d.padH_l, d.sH) == rh) is.push_back(i);
+      for (int j = 0; j < d.kW; ++j) if (pymod(j * d.dilW - d.padW_l, d.sW) == rw) js.push_back(j);
+      if (is.empty() || js.empty()) continue;
+      if (rh >= d.H || rw >= d.W) { *dropped = true; continue; }
+      RowsView v;
+      for (int i : is) v.dh.push_back(floordiv(i * d.dilH - d.padH_l, d.sH));
+      for (int j : js) v.dw.push_back(floordiv(j * d.dilW - d.padW_l, d.sW));
+      for (int i : is)
+        for (int j : js) v.tap.push_back((d.flip ? d.kH - 1 - i : i) * d.kW + (d.flip ? d.kW - 1 - j : j));
+      v.map = [=](CUtensorMap* m, int bw, int bh) {
+        return make_view(c, m, xin, d.dtype, d.C / d.groups, d.groups, pad_channels(d.C, d.dtype), d.W, d.H, d.N, rh, rw, d.sH, d.sW, atom, bw, bh, 1,
+                         d.dtype == B200CONV_F32);
+      };
+      views.push_back(v);
+    }
+  return views;
+}
+
+// gradWeights with the filter's rows and columns inside one MMA (wgrad_rows.cu).  Returns 0 when launched, 2 when the
+// layer is not one for it: more filters per group than a swizzle atom holds, uneven taps, rows too wide for a box.
+// `reduce(partial, slabs)` enqueues the kernel that adds the slabs.
+template <class Reduce>
+int wgrad_rows(b200conv_ctx* c, const b200conv_desc& d, const std::vector<RowsView>& views, int Cg, bool dropped, int taps_total, const void* gin,
+               int flags, Scratch& tmp, int diag_c, int diag_k, Reduce reduce) {
+  const bool f16 = d.dtype == B200CONV_F16;
+  const int atom = f16 ? 64 : 32, kk = f16 ? 16 : 8, copies = 128 / atom, Kg = d.K / d.groups;
+  if ((flags & (B200CONV_NO_ROWS | B200CONV_ATOMIC_SPLITK)) || Kg > atom || views.empty() || views.size() > (size_t)kMaxViews) return 2;
+  RowsWgradParams p;
+  memset(&p, 0, sizeof p);
+  p.nviews = (int)views.size();
+  p.stack_step = 1;
+  int row_step = 0, col_step = 0, taps = 0, span = 0, Ew = 0, n_max = 0, sets_max = 0;
+  for (int v = 0; v < p.nviews; ++v) {
+    const RowsView& w = views[v];
+    const int rows = (int)w.dh.size(), cols = (int)w.dw.size();
+    for (int i = 1; i < rows; ++i) { const int st = w.dh[i] - w.dh[i - 1]; if (st <= 0 || (row_step && st != row_step)) return 2; row_step = st; }
+    for (int j = 1; j < cols; ++j) { const int st = w.dw[j] - w.dw[j - 1]; if (st <= 0 || (col_step && st != col_step)) return 2; col_step = st; }
+    const int sets = (int)cdiv(rows, copies);
+    if (sets > kMaxRowSets || cols * atom > 256 || sets * cols * atom > 512 || taps + rows * cols > kMaxTaps) return 2;
+    p.view_nt[v] = (int16_t)cols; p.view_sets[v] = (int16_t)sets; p.view_tap0[v] = (int16_t)taps;
+    for (int t : w.tap) p.tap_id[taps++] = (int16_t)t;
+    for (int j = 0; j < sets; ++j) {
+      p.set_first[v][j] = (int16_t)(j * copies);
+      p.set_base[v][j] = (int16_t)std::min(rows - 1, j * copies + copies - 1);
+    }
+    p.view_dh[v] = (int16_t)w.dh[p.set_base[v][0]];
+    p.view_dw[v] = (int16_t)w.dw[0];
+    p.halo = std::max<int>(p.halo, p.set_base[v][0] * std::max(1, row_step));
+    span = std::max<int>(span, w.dh[p.set_base[v][sets - 1]] - w.dh[p.set_base[v][0]]);
+    Ew = std::max<int>(Ew, w.dw[cols - 1] - w.dw[0]);
+    n_max = std::max(n_max, cols * atom); sets_max = std::max(sets_max, sets);
+  }
+  if (row_step == 0 || p.halo == 0) return 2;                          // one filter row: nothing to stack
+  if (col_step) p.stack_step = col_step;
+  p.groups = d.groups; p.Kg = Kg; p.Cg = Cg; p.Nimg = d.N;
+  p.ctiles = (int)cdiv(Cg, atom);
+  p.taps_total = taps_total;
+  // Tile: grid pitch and rows with the least work per image, the larger of the MMAs' clocks and the boxes' bytes at
+  // 40 B/clk, and 200 clocks per stage.  Rows are whole (a segment's dy would have to end in zeros).
+  SlabTile& memo = c->pixel_tiles[GeoKey{kGeoRows, d.dtype, d.Wo, d.Ho, Ew, span, p.halo, row_step, p.stack_step, n_max, sets_max, p.nviews}];
+  auto plan = [&](int P, int th) -> bool {
+    p.pitch = P; p.th = th; p.a_step = row_step * P;
+    p.rows_a = (th + p.halo) * P; p.rows_b = (th + span) * P;
+    if (p.a_step > 2047 || p.rows_a > 1200 || p.rows_b > 1200) return false;
+    for (int v = 0; v < p.nviews; ++v)
+      for (int j = 0; j < p.view_sets[v]; ++j) p.set_rows[v][j] = (int16_t)((views[v].dh[p.set_base[v][j]] - p.view_dh[v]) * P);
+    p.tiles_h = (int)cdiv(d.Ho + p.halo, th);
+    return wgrad_rows_ring(&p, d.dtype);
+  };
+  if (!memo.found) {
+    long long best = -1;
+    for (int P = d.Wo + Ew; P < d.Wo + Ew + kk && P <= 256; ++P)
+      for (int th = 1; th <= d.Ho + p.halo && th + std::max(p.halo, span) <= 256; ++th) {
+        if (th * P % kk) continue;
+        if (!plan(P, th)) break;
+        const long long mma = 1LL * th * P / kk * sets_max * std::max(n_max / 2, 32 + n_max / 4), load = (p.rows_a + p.rows_b) * 128LL / 40;
+        const long long cost = p.tiles_h * (std::max(mma, load) + 200 + (p.stages < 3 ? mma / 8 : 0));
+        if (best < 0 || cost < best) { best = cost; memo.wt = P; memo.th = th; }
+      }
+    memo.found = true;
+  }
+  if (!memo.wt || !plan(memo.wt, memo.th)) return 2;
+  int rc = make_view(c, &p.dy_map, gin, d.dtype, Kg, d.groups, pad_channels(d.K, d.dtype), d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.pitch, p.th + p.halo, 1,
+                     d.dtype == B200CONV_F32);
+  if (rc) return rc;
+  for (int v = 0; v < p.nviews; ++v)
+    if ((rc = views[v].map(&p.x_views[v], p.pitch, p.th + span))) return rc;
+  p.diag_c = diag_c; p.diag_k = diag_k;
+  p.status = c->d_status;
+  p.wait_clocks = c->wait_clocks;
+  const size_t slab_elems = (size_t)taps_total * d.K * Cg;
+  auto run = [&](int splits, Scratch& sc) -> int {
+    p.splits = splits;
+    float* partial;
+    int r = sc.get(sizeof(float) * slab_elems * splits, reinterpret_cast<void**>(&partial));
+    if (r) return r;
+    if (dropped) CU_OK(c, cudaMemsetAsync(partial, 0, sizeof(float) * slab_elems * splits, c->stream));
+    p.partial = partial;
+    p.partial_elems = (long long)slab_elems * splits;
+    c->last_variant = "wgrad rows";
+    KLAUNCH(c, kKWgradUmma, launch_wgrad_rows(p, d.dtype, c->num_sms, c->stream));
+    return reduce(partial, splits);
+  };
+  GeoKey skey = wgrad_key(kGeoSplits, d, flags);
+  skey.add(3);
+  const long long tiles = 1LL * p.tiles_h * d.N;
+  const int splits = pick_splits(c, skey, tiles, tiles, 1LL * p.ctiles * d.groups * p.nviews, c->num_sms, 3, run);
+  if (splits < 0) return splits;
+  if ((rc = run(splits, tmp))) return rc;
+  c->last_algo = "umma";
+  return 0;
+}
+
+// The number of neighbouring groups that fill a swizzle atom of filters and channels (wgrad_rows), 1: none.
+int merge_factor_rows(const b200conv_desc& d) {
+  const int atom = d.dtype == B200CONV_F16 ? 64 : 32, Cg = d.C / d.groups, Kg = d.K / d.groups;
+  int best = 1;
+  for (int m = 2; m <= d.groups && Cg * m <= atom && Kg * m <= atom; ++m)
+    if (d.groups % m == 0 && umma_ok(merged_groups(d, m))) best = m;
+  return best;
+}
+
+enum { kWgradTaps = 0, kWgradGroups = 1, kWgradRows = 2 };      // the gradWeights kernels; the numbers appear in tuning files
+
 int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const void* dy, void* dw,
                  int flags) {
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;
@@ -1912,12 +2052,51 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     dm.groups = d.groups / mg;
     int t0, nt, q0;
     if (umma_ok(dm) && !fold_ok(dm) && !s2d_ok(dm, &t0, &nt, &q0)) {
-      // gradient of the block-diagonal filters, of which only the diagonal blocks are stored and added up (32 groups of 8 x 8
-      // channels 3x3 of 256 images of 28 x 28: 200 -> 180 us, with the layout of the slabs)
-      c->diag_c = Cg; c->diag_k = Kg;
-      const int rc = wgrad_device(c, dm, x, dy, dw, flags);
-      c->diag_c = c->diag_k = 0;
-      return rc;
+      // gradient of block-diagonal filters, of which only the diagonal blocks are stored and added up
+      Scratch tm(c);
+      const void *xin = x, *gin = dy;
+      int rc;
+      if (!x_nhwc && (rc = to_nhwc(c, tm, x, d.N, d.C, d.H, d.W, d.dtype, &xin))) return rc;
+      if (!dy_nhwc && (rc = to_nhwc(c, tm, dy, d.N, d.K, d.Ho, d.Wo, d.dtype, &gin))) return rc;
+      // groups merged to 128 filters x 128 channels, or to one swizzle atom with the filter's rows stacked (32 groups of 8 x 8 channels
+      // 3x3, 256 images of 28 x 28, float32: 180 -> 83 us)
+      const int mr = merge_factor_rows(d);
+      const b200conv_desc dr = merged_groups(d, mr);
+      auto kernel = [&](int v) -> int {
+        if (v == 0) {
+          c->diag_c = Cg; c->diag_k = Kg;
+          const int r = wgrad_device(c, dm, xin, gin, dw, flags | B200CONV_IN_NHWC | B200CONV_IN2_NHWC);
+          c->diag_c = c->diag_k = 0;
+          return r;
+        }
+        if (!umma_ok(dr)) return 2;
+        bool dropped;
+        const std::vector<RowsView> views = rows_views(c, dr, xin, &dropped);
+        Scratch trial(c);
+        const int dc = mr > 1 ? Cg : 0, dk = mr > 1 ? Kg : 0;
+        return wgrad_rows(c, dr, views, Cg * mr, dropped, d.kH * d.kW, gin, flags, trial, dc, dk, [&](float* partial, int slabs) {
+          KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg * mr, Kg * mr, dc, dk, odt, c->stream));
+          return 0;
+        });
+      };
+      const GeoKey key = wgrad_key(kGeoWgrad, d, flags);
+      int choice = 1;
+      if (c->autotune) {
+        auto it = c->algo_cache.find(key);
+        if (it != c->algo_cache.end()) choice = it->second == kWgradRows;
+        else if (!c->capturing && !c->model_only) {
+          float ms[2];
+          int codes[2];
+          if ((rc = rough_times(c, 2, kernel, ms, codes))) return rc;
+          if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) && (rc = time_variants(c, 2, kernel, ms, codes))) return rc;
+          for (int code : codes)
+            if (code && code != 2) return code;
+          choice = ms[1] >= 0.f && (ms[0] < 0.f || ms[1] < ms[0]);
+          c->algo_cache[key] = choice ? kWgradRows : kWgradTaps;
+        }
+      }
+      if (choice && (rc = kernel(1)) != 2) return rc;
+      return kernel(0);
     }
     if (umma_ok(dm)) {
       // few channels in all: the row-folded forms, then keep the diagonal blocks
@@ -1957,6 +2136,29 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * H2 * Wq * kS2dChannels, &xs))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_s2d(x, xs, d.N, d.C, d.H, d.W, Cp, H2, Wq, s2_q0, x_nhwc ? 1 : 0,
                                            d.dtype, c->stream));
+    {
+      // the filter's block rows stacked inside the MMAs where the filters leave room (7x7 stem 3 -> 64 of 256 images of
+      // 224 x 224, float16: 311 -> 183 us)
+      RowsView v;
+      for (int t = 0; t < s2_nt; ++t) { v.dh.push_back(t + s2_t0); v.tap.push_back(t); }
+      v.dw.push_back(0);
+      v.map = [&](CUtensorMap* m, int bw, int bh) -> int {
+        const size_t pix = (size_t)kS2dChannels * es, row = (size_t)Wq * pix;
+        cuuint64_t dims[5] = {(cuuint64_t)win, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
+        cuuint64_t strides[4] = {row, pix, row, (cuuint64_t)H2 * row};
+        cuuint32_t box[5] = {(cuuint32_t)kBK, 1, (cuuint32_t)bw, (cuuint32_t)bh, 1};
+        cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        CUresult r = c->encode(m, d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, xs, dims, strides, box, estr,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, d.dtype == B200CONV_F32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        return r == CUDA_SUCCESS ? 0 : fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
+      };
+      rc = wgrad_rows(c, d, {v}, win, false, s2_nt, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, slabs, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0, s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
+        return 0;
+      });
+      if (rc != 2) return rc;
+    }
     UmmaWgradParams p;
     memset(&p, 0, sizeof p);
     const int atom = kBK;
@@ -2017,6 +2219,38 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * d.H * Wp * Cp, &xp))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_fold(x, xp, d.N, d.C, d.H, d.W, Cp, Wp, d.padW_l, x_nhwc ? 1 : 0,
                                             d.dtype, c->stream));
+    {
+      // the filter rows stacked inside the MMAs where the filters leave room
+      std::vector<RowsView> views;
+      bool dropped = false;
+      for (int rh = 0; rh < d.sH; ++rh) {
+        RowsView v;
+        for (int i = 0; i < d.kH; ++i)
+          if (pymod(i * d.dilH - d.padH_l, d.sH) == rh) { v.dh.push_back(floordiv(i * d.dilH - d.padH_l, d.sH)); v.tap.push_back(i); }
+        if (v.dh.empty()) continue;
+        if (rh >= d.H) { dropped = true; continue; }
+        v.dw.push_back(0);
+        v.map = [=](CUtensorMap* m, int bw, int bh) -> int {
+          const size_t pix = (size_t)Cp * es, row = (size_t)Wp * pix;
+          const int H2 = (d.H - rh + d.sH - 1) / d.sH;
+          cuuint64_t dims[5] = {(cuuint64_t)kBK, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
+          cuuint64_t strides[4] = {row, (cuuint64_t)d.sW * pix, (cuuint64_t)d.sH * row, (cuuint64_t)d.H * row};
+          cuuint32_t box[5] = {(cuuint32_t)kBK, 1, (cuuint32_t)bw, (cuuint32_t)bh, 1};
+          cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+          CUresult r = c->encode(m, d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5,
+                                 static_cast<char*>(xp) + (size_t)rh * row, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                 d.dtype == B200CONV_F32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+          return r == CUDA_SUCCESS ? 0 : fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(folded x) failed: %d", (int)r);
+        };
+        views.push_back(v);
+      }
+      rc = wgrad_rows(c, d, views, kBK, dropped, d.kH, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, slabs, d.K, d.C, d.kH, d.kW, Cp, kBK, d.flip, odt, c->stream));
+        return 0;
+      });
+      if (rc != 2) return rc;
+    }
     FwdLikeArgs a;
     a.act = xp; a.Hs = d.H; a.Ws = d.Wo; a.Cin_g = kBK; a.Cp_in = Cp; a.N = d.N; a.dtype = d.dtype;
     a.groups = 1; a.view_sH = d.sH; a.view_sW = 1;
@@ -2088,42 +2322,63 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   if (!dy_nhwc && (rc = to_nhwc(c, tmp, dy, d.N, d.K, d.Ho, d.Wo, d.dtype, &gin))) return rc;
   const int Cp = pad_channels(d.C, d.dtype), Kp = pad_channels(d.K, d.dtype);
 
-  // Two tensor-core kernels: tap groups sharing operands, or one tap per work item.  As for the
-  // forward kernels the first call of a geometry times both and the context remembers the winner.
-  bool try_group = !(flags & B200CONV_NO_GROUP);
+  // Three tensor-core kernels: one tap per work item, tap groups sharing operands, or all taps of narrow layers in one MMA.  As for
+  // the forward kernels the first call of a geometry times those that apply and the context remembers the winner.
+  auto rows = [&](Scratch& sc) -> int {
+    bool dropped;
+    const std::vector<RowsView> views = rows_views(c, d, xin, &dropped);
+    return wgrad_rows(c, d, views, Cg, dropped, d.kH * d.kW, gin, flags, sc, c->diag_c, c->diag_k, [&](float* partial, int slabs) {
+      KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg, Kg, c->diag_c, c->diag_k, odt, c->stream));
+      return 0;
+    });
+  };
   const GeoKey key = wgrad_key(kGeoWgrad, d, flags);
   // without timings: the one-tap kernel where it runs 256-column MMAs (their issue and TMA
   // budgets are comfortable), tap groups for narrower layers (they read the operands 3x less)
-  if (try_group && !c->autotune && d.C / d.groups >= 256) try_group = false;
-  if (try_group && c->autotune) {
+  int choice = (flags & B200CONV_NO_GROUP) || (!c->autotune && Cg >= 256) ? kWgradTaps : kWgradGroups;
+  if (flags & B200CONV_ROWS) {
+    choice = kWgradRows;
+  } else if (choice == kWgradGroups && c->autotune) {
     auto itc = c->algo_cache.find(key);
     if (itc != c->algo_cache.end()) {
-      try_group = itc->second;
+      choice = itc->second;
     } else if (!c->capturing) {
       // own scratch, returned to the pool after each run: the next run then reuses the buffers and its timing
       // holds no allocation
-      // Both kernels choose a slice count of their own: that is timed only where they are close with the models'.
-      float ms[2];                                            // 0: tap groups, 1: one tap per item
-      int codes[2];
-      bool covered = true;
-      auto kernel = [&](int v) -> int {
-        if (v) return covered ? wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC) : 2;
+      // The kernels choose a slice count of their own: that is timed only where they are close with the models'.
+      const int order[3] = {kWgradRows, kWgradGroups, kWgradTaps};
+      float ms[3];
+      int codes[3];
+      bool others = false;                                    // another kernel than the one-tap form applies
+      auto kernel = [&](int i) -> int {
+        if (order[i] == kWgradTaps) return others ? wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC) : 2;
         Scratch trial(c);
-        const int r = wgrad_grouped(c, d, xin, gin, dw, flags, trial);
-        covered = r != 2;
+        const int r = order[i] == kWgradGroups ? wgrad_grouped(c, d, xin, gin, dw, flags, trial) : rows(trial);
+        others |= r != 2;
         return r;
       };
-      if ((rc = rough_times(c, 2, kernel, ms, codes))) return rc;
-      if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) &&
-          (rc = time_variants(c, 2, kernel, ms, codes)))
-        return rc;
+      if ((rc = rough_times(c, 3, kernel, ms, codes))) return rc;
+      float least = -1.f;
+      for (float m : ms) if (m >= 0.f && (least < 0.f || m < least)) least = m;
+      bool far[3];
+      int close = 0;
+      for (int i = 0; i < 3; ++i) { far[i] = ms[i] < 0.f || ms[i] > kFarBehind * least; close += !far[i]; }
       for (int code : codes)
         if (code && code != 2) return code;
-      try_group = ms[0] >= 0.f && (ms[1] < 0.f || ms[0] <= ms[1]);
-      c->algo_cache[key] = try_group;
+      if (close > 1) {
+        if ((rc = time_variants(c, 3, [&](int i) { return far[i] ? 2 : kernel(i); }, ms, codes))) return rc;
+        for (int code : codes)
+          if (code && code != 2) return code;
+      }
+      choice = kWgradTaps;
+      least = -1.f;
+      for (int i = 0; i < 3; ++i)
+        if (ms[i] >= 0.f && (least < 0.f || ms[i] < least)) { least = ms[i]; choice = order[i]; }
+      c->algo_cache[key] = choice;
     }
   }
-  if (try_group) {
+  if (choice == kWgradRows && (rc = rows(tmp)) != 2) return rc;
+  if (choice != kWgradTaps) {
     rc = wgrad_grouped(c, d, xin, gin, dw, flags, tmp);
     if (rc != 2) return rc;     // 2: geometry not covered, use the one-tap-per-item kernel
   }

@@ -321,6 +321,34 @@ struct alignas(64) GroupWgradParams {
 };
 cudaError_t launch_wgrad_group(const GroupWgradParams& p, int dtype, int num_sms, cudaStream_t s);
 
+// ---- filter gradient of narrow layers, filter rows and columns inside one MMA (wgrad_rows.cu) -----
+constexpr int kMaxRowSets = 4;       // sets of 128 / atom filter rows per view
+struct alignas(64) RowsWgradParams {
+  CUtensorMap dy_map;                // box (atom, 1, pitch, th + halo, 1)
+  CUtensorMap x_views[kMaxViews];    // box (atom, 1, pitch, x rows, 1), one per stride parity class
+  int nviews;
+  int16_t view_dh[kMaxViews], view_dw[kMaxViews];      // offset of the x box from the tile's origin
+  int16_t view_nt[kMaxViews], view_sets[kMaxViews];    // filter columns / sets of filter rows of the view
+  int16_t view_tap0[kMaxViews];                        // of its taps in tap_id, [filter row][filter column]
+  int16_t set_first[kMaxViews][kMaxRowSets], set_base[kMaxViews][kMaxRowSets];   // first / last filter row of the set
+  int16_t set_rows[kMaxViews][kMaxRowSets];            // x row offset of its last filter row
+  int16_t tap_id[kMaxTaps];          // filter tap index in OIHW order (after flip)
+  int stack_step, a_step;            // grid positions between the filter's columns / rows
+  int groups, Kg, Cg, Nimg, ctiles;
+  int pitch, th, halo, tiles_h;      // grid pitch, rows per tile, rows that the copies of dy reach back, tiles per image
+  int rows_a, rows_b;                // rows of the boxes in shared memory
+  int a_bytes, b_bytes, stages, ring_bytes;            // set by wgrad_rows_ring
+  int splits;
+  float* partial;                    // one float32 slab per slice (wgrad_slab.cuh)
+  long long partial_elems;           // its extent (checked in the range-checked build)
+  int diag_c, diag_k;                // merged groups of diag_k filters x diag_c channels: only their blocks are stored; 0: everything
+  int taps_total;
+  int* status;
+  long long wait_clocks;             // bound of every device-side wait, in SM clocks
+};
+bool wgrad_rows_ring(RowsWgradParams* p, int dtype);      // false: two stages do not fit
+cudaError_t launch_wgrad_rows(const RowsWgradParams& p, int dtype, int num_sms, cudaStream_t s);
+
 // ---- strided gradInputs with few channels: parity classes merged into channels ---------------
 // src[u][cls] = filter tap (i * kW + j, correlation coordinates) that class `cls` applies at the
 // merged offset u, or -1 when the class has no tap there.
