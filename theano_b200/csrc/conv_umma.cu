@@ -40,6 +40,9 @@ template <int BN> constexpr int num_stages() {
   return (kSmemBudget / stage_bytes<BN>()) > 8 ? 8 : (kSmemBudget / stage_bytes<BN>());
 }
 
+// Transpose buffers of the epilogue warps, 32 rows x 64 bytes each (float32; a float16 chunk is 64 bytes of a row already)
+template <MmaKind KIND> constexpr int transpose_bytes() { return KIND == MmaKind::TF32 ? 2048 : 0; }
+
 struct Bars {
   uint64_t full[8];
   uint64_t empty[8];
@@ -69,7 +72,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  Bars* bars = reinterpret_cast<Bars*>(smem + kStages * stage_bytes<BN>());
+  uint8_t* transposes = smem + kStages * stage_bytes<BN>();
+  Bars* bars = reinterpret_cast<Bars*>(transposes + kEpilogueWarps * transpose_bytes<KIND>());
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int rows_used = p.bw * p.bh * p.bn;
@@ -88,7 +92,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&bars->acc_full[b], 1);
-      mbar_init(&bars->acc_empty[b], 32 * kEpilogueWarps);
+      mbar_init(&bars->acc_empty[b], kEpilogueWarps);
     }
     bars->abort = 0;
     mbar_fence_init();
@@ -200,9 +204,11 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const int quad = warp & 3;
     const int sub = (warp - 2) >> 2;
     const int row = quad * 32 + lane;
+    uint8_t* mine = transposes + (warp - 2) * transpose_bytes<KIND>();
     const int rw = row % p.bw, rh = (row / p.bw) % p.bh, rn = row / (p.bw * p.bh);
     OutT* out = static_cast<OutT*>(p.out);
     const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
+    const bool transposed = KIND == MmaKind::TF32 && rowwise && total > gridDim.x;
     bool ok = true;
     int it = 0;
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
@@ -221,10 +227,16 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       OutT* pix = out + (p.out_off + n * p.out_sn + h * p.out_sh + w * p.out_sw) + 1LL * g * p.n_out * p.out_sc;
       const OutT* res = p.epi.residual ? static_cast<const OutT*>(p.epi.residual) + (pix - out) : nullptr;
       const int co_base = co_t * BN;
+      // element offsets of the four rows that this lane helps to write, -1: no pixel
+      long long rows[4] = {-1, -1, -1, -1};
+      if (transposed)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) rows[i] = __shfl_sync(0xffffffffu, valid ? static_cast<long long>(pix - out) : -1LL, i * 8 + (lane >> 2));
+      const int first_ch = (sub - it * min(BN / 32, (p.n_out - co_base + 31) / 32)) & 3;      // the warps take turns on narrow tiles
       if (splits > 1) {       // raw accumulators; conv_reduce.cu adds the slices and applies the epilogue
         float4* dst = reinterpret_cast<float4*>(p.partial) + static_cast<long long>(item) * (kRows * BN / 4) + row;
 #pragma unroll 1
-        for (int ch = sub; ch < BN / 32 && co_base + ch * 32 < p.n_out; ch += kEpilogueWarps / 4) {
+        for (int ch = first_ch; ch < BN / 32 && co_base + ch * 32 < p.n_out; ch += kEpilogueWarps / 4) {
           uint32_t r[32];
           tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
           tmem_ld_wait();
@@ -237,16 +249,47 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         }
       } else
 #pragma unroll 1
-      for (int ch = sub; ch < BN / 32; ch += kEpilogueWarps / 4) {
+      for (int ch = first_ch; ch < BN / 32; ch += kEpilogueWarps / 4) {
         const int co0 = co_base + ch * 32;          // first channel (within the group) of the chunk
         if (co0 >= p.n_out) break;
         uint32_t r[32];
         tmem_ld32(tmem + (static_cast<uint32_t>(quad * 32) << 16) + buf * BN + ch * 32, r);
         tmem_ld_wait();
-        if (!valid) continue;
+        if (!valid && !transposed) continue;
         zero_pad_columns(r, co0, p.n_real);
         const OutT* bias = p.bias ? static_cast<const OutT*>(p.bias) + g * p.n_out + co0 : nullptr;
-        if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
+        if (transposed) {
+          // Four lanes write 64 bytes of a row side by side.  With each lane writing its own row an instruction touched 32 lines and half of
+          // each sector, 2400 clocks per 128 x 32 block: more than the MMAs of a shallow reduction.  (64 -> 128 3x3 stride 2 at
+          // 56x56, 256 images: 106 -> 91 us.  Float16 gained nothing: half as many pieces; nor did a CTA's only tile.)
+#pragma unroll
+          for (int j0 = 0; j0 < 32; j0 += 16) {
+            if (co0 + j0 >= p.n_out) break;
+#pragma unroll
+            for (int piece = 0; piece < 4; ++piece) {
+              float f[4];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                const int j = j0 + 4 * piece + q;
+                f[q] = p.epi.alpha * __uint_as_float(r[j]);
+                if (bias && co0 + j < p.n_out) f[q] += static_cast<float>(bias[j]);
+                if (res && valid && co0 + j < p.n_real) f[q] += p.epi.beta * static_cast<float>(res[co0 + j]);
+                if (p.relu) f[q] = p.epi.lin * f[q] + p.epi.abs * fabsf(f[q]);
+              }
+              *reinterpret_cast<float4*>(mine + lane * 64 + ((piece ^ ((lane >> 1) & 3)) << 4)) = make_float4(f[0], f[1], f[2], f[3]);
+            }
+            __syncwarp();
+            const int cp = co0 + j0 + (lane & 3) * 4;                    // this lane's channels of the rows it writes
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int srow = i * 8 + (lane >> 2);
+              const float4 v = *reinterpret_cast<const float4*>(mine + srow * 64 + (((lane & 3) ^ ((srow >> 1) & 3)) << 4));
+              if (rows[i] >= 0 && cp < p.n_out && B200_IN_RANGE(rows[i] + cp + 4 <= p.out_elems, p.status))
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + rows[i] + cp) = v;
+            }
+            __syncwarp();
+          }
+        } else if (rowwise) {   // n_out is a whole number of 16-byte pieces: a piece is all in or all out
 #pragma unroll
           for (int j = 0; j < 32; j += 16 / sizeof(OutT)) {
             if (co0 + j >= p.n_out) break;
@@ -288,7 +331,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         }
       }
       tc_fence_before();
-      mbar_arrive(&bars->acc_empty[buf]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);
     }
     if (!ok && lane == 0) report_status(p.status, kStatusTimeout);
   }
@@ -302,7 +346,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   }
 }
 
-template <MmaKind KIND, int BN> constexpr int smem_bytes() { return num_stages<BN>() * stage_bytes<BN>() + sizeof(Bars) + 1024; }
+template <MmaKind KIND, int BN> constexpr int smem_bytes() { return num_stages<BN>() * stage_bytes<BN>() + kEpilogueWarps * transpose_bytes<KIND>() + sizeof(Bars) + 1024; }
 template <MmaKind KIND, int BN>
 cudaError_t configure() {
   static PerDeviceOnce configured;
