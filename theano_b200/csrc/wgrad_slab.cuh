@@ -31,6 +31,15 @@ __device__ __forceinline__ void diagonal_range(int diag_c, int diag_k, int kq, i
 __device__ __forceinline__ void store_slab_chunk(const uint32_t (&r)[32], float* slab, int c0, int c_lo, int c_hi, int Cg, int K, int k,
                                                  bool atomic, const float* partial, long long partial_elems, int* status) {
   const bool vec = ((1LL * K * Cg) & 3) == 0 && !atomic;
+  if (vec && c_lo <= c0 && c0 + 32 <= c_hi) {               // whole: one address, K pieces apart (c_hi <= Cg)
+    float* dst = slab + 1LL * c0 * K + 4LL * k;
+    if (!B200_IN_RANGE(dst - partial >= 0 && (dst - partial) + 28LL * K + 4 <= partial_elems, status)) return;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      reinterpret_cast<float4*>(dst)[static_cast<unsigned>(j) * static_cast<unsigned>(K)] =
+          make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+    return;
+  }
 #pragma unroll
   for (int j = 0; j < 32; j += 4) {
     const int c = c0 + j, w = min(4, Cg - c);
