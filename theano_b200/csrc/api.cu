@@ -1724,8 +1724,9 @@ int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long lo
   cap = std::max(1LL, std::min(cap, pix_tiles));
   if (c->force_splits > 0) return valid_splits(pix_tiles, std::min<long long>(c->force_splits, cap));
   if (c->autotune) {
+    // whatever call or file the count came from: a slice without a tile would add up what its accumulator held before
     auto it = c->split_cache.find(key);
-    if (it != c->split_cache.end()) return it->second;
+    if (it != c->split_cache.end()) return valid_splits(pix_tiles, std::min<long long>(it->second, cap));
   }
   const int s0 = (int)balanced_splits(c, pix_tiles, base_items, sms, cap, fixed);
   if (!c->autotune || c->capturing || c->model_only) return s0;
@@ -1749,6 +1750,9 @@ GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
   return GeoKey{kind, d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.Ho, d.Wo,
                 d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : 0))};
 }
+
+// Kernel and form of the layer in the key of a slice count: one layer's forms differ in their pixel tiles.
+enum { kSplitsGroups = 0, kSplitsTaps, kSplitsPair, kSplitsRows, kSplitsRowsS2d, kSplitsRowsFold };
 
 // gradWeights with tap groups (wgrad_group.cu).  Returns 0 when launched, 2 when the geometry is
 // left to the one-tap-per-item kernel (no two taps share a row offset, or the column span of the
@@ -1881,7 +1885,7 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
     return 0;
   };
   GeoKey skey = wgrad_key(kGeoSplits, d, flags);
-  skey.add(0);
+  skey.add(kSplitsGroups);
   // accumulators are not double buffered: aim at one item per SM
   const int splits = pick_splits(c, skey, pix_tiles, pix_tiles, base_items, c->num_sms, 6, run);
   if (splits < 0) return splits;
@@ -1925,9 +1929,9 @@ std::vector<RowsView> rows_views(b200conv_ctx* c, const b200conv_desc& d, const 
 
 // gradWeights with the filter's rows and columns inside one MMA (wgrad_rows.cu).  Returns 0 when launched, 2 when the
 // layer is not one for it: more filters per group than a swizzle atom holds, uneven taps, rows too wide for a box.
-// `reduce(partial, slabs)` enqueues the kernel that adds the slabs.
+// `form`: kSplitsRows, or the form of x that the views are of; `reduce(partial, slabs)` enqueues the kernel that adds the slabs.
 template <class Reduce>
-int wgrad_rows(b200conv_ctx* c, const b200conv_desc& d, const std::vector<RowsView>& views, int Cg, bool dropped, int taps_total, const void* gin,
+int wgrad_rows(b200conv_ctx* c, const b200conv_desc& d, int form, const std::vector<RowsView>& views, int Cg, bool dropped, int taps_total, const void* gin,
                int flags, Scratch& tmp, int diag_c, int diag_k, Reduce reduce) {
   const bool f16 = d.dtype == B200CONV_F16;
   const int atom = f16 ? 64 : 32, kk = f16 ? 16 : 8, copies = 128 / atom, Kg = d.K / d.groups;
@@ -2009,7 +2013,7 @@ int wgrad_rows(b200conv_ctx* c, const b200conv_desc& d, const std::vector<RowsVi
     return reduce(partial, splits);
   };
   GeoKey skey = wgrad_key(kGeoSplits, d, flags);
-  skey.add(3);
+  skey.add(form);
   const long long tiles = 1LL * p.tiles_h * d.N;
   const int splits = pick_splits(c, skey, tiles, tiles, 1LL * p.ctiles * d.groups * p.nviews, c->num_sms, 3, run);
   if (splits < 0) return splits;
@@ -2074,7 +2078,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         const std::vector<RowsView> views = rows_views(c, dr, xin, &dropped);
         Scratch trial(c);
         const int dc = mr > 1 ? Cg : 0, dk = mr > 1 ? Kg : 0;
-        return wgrad_rows(c, dr, views, Cg * mr, dropped, d.kH * d.kW, gin, flags, trial, dc, dk, [&](float* partial, int slabs) {
+        return wgrad_rows(c, dr, kSplitsRows, views, Cg * mr, dropped, d.kH * d.kW, gin, flags, trial, dc, dk, [&](float* partial, int slabs) {
           KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg * mr, Kg * mr, dc, dk, odt, c->stream));
           return 0;
         });
@@ -2153,7 +2157,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         return r == CUDA_SUCCESS ? 0 : fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
       };
-      rc = wgrad_rows(c, d, {v}, win, false, s2_nt, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+      rc = wgrad_rows(c, d, kSplitsRowsS2d, {v}, win, false, s2_nt, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
         KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, slabs, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0, s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
         return 0;
       });
@@ -2245,7 +2249,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         };
         views.push_back(v);
       }
-      rc = wgrad_rows(c, d, views, kBK, dropped, d.kH, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+      rc = wgrad_rows(c, d, kSplitsRowsFold, views, kBK, dropped, d.kH, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
         KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, slabs, d.K, d.C, d.kH, d.kW, Cp, kBK, d.flip, odt, c->stream));
         return 0;
       });
@@ -2327,7 +2331,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   auto rows = [&](Scratch& sc) -> int {
     bool dropped;
     const std::vector<RowsView> views = rows_views(c, d, xin, &dropped);
-    return wgrad_rows(c, d, views, Cg, dropped, d.kH * d.kW, gin, flags, sc, c->diag_c, c->diag_k, [&](float* partial, int slabs) {
+    return wgrad_rows(c, d, kSplitsRows, views, Cg, dropped, d.kH * d.kW, gin, flags, sc, c->diag_c, c->diag_k, [&](float* partial, int slabs) {
       KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg, Kg, c->diag_c, c->diag_k, odt, c->stream));
       return 0;
     });
@@ -2458,7 +2462,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     return 0;
   };
   GeoKey skey = wgrad_key(kGeoSplits, d, flags);
-  skey.add(pair ? 2 : 1);
+  skey.add(pair ? kSplitsPair : kSplitsTaps);
   const int splits = pick_splits(c, skey, pix_tiles, std::max(1LL, pix_tiles / 4), base_items, pair ? c->num_sms / 2 : c->num_sms, 2, run);
   if (splits < 0) return splits;
   if ((rc = run(splits, tmp))) return rc;
