@@ -1,0 +1,58 @@
+"""Which gradWeights kernel runs: what a context reports, and what the flags that ask for a kernel or bar one do on a context that
+other calls have used, with timing on."""
+import numpy as np
+import pytest
+
+from oracle import corr_oracle as O
+from theano_b200 import shim
+
+pytestmark = pytest.mark.gpu
+DTYPES = pytest.mark.parametrize("dtype", [np.float32, np.float16], ids=["f32", "f16"])
+ROWS, NO_ROWS, NO_GROUP = shim.ROWS, shim.NO_ROWS, shim.NO_GROUP
+KERNELS = ("wgrad tap", "wgrad groups", "wgrad rows")        # by the number in tuning files
+
+
+def _layer(ctx, dtype, xs, k, ks, s=1, g=1):
+    """run(flags) -> variant, on operands of values -1, 0, 1: sums are whole numbers that both types hold."""
+    kw = dict(border_mode="half", subsample=(s, s), num_groups=g)
+    rs = np.random.RandomState(k + ks)
+    x = rs.randint(-1, 2, xs).astype(dtype)
+    ho, wo = O.conv2d(np.zeros((1, g) + xs[2:], np.float32), np.zeros((g, 1, ks, ks), np.float32), **kw).shape[2:]
+    dy = rs.randint(-1, 2, (xs[0], k, ho, wo)).astype(dtype)
+    want = O.conv2d_grad_weights(x.astype(np.float32), dy.astype(np.float32), (ks, ks), **kw).astype(dtype)
+    X, DY = shim.DeviceTensor.from_host(ctx, x, "nhwc"), shim.DeviceTensor.from_host(ctx, dy, "nhwc")
+
+    def run(flags=0):
+        got = shim.device_grad_weights(X, DY, (ks, ks), flags=flags, **kw).to_host()
+        assert np.array_equal(got, want)
+        return ctx.last_variant
+    return run
+
+
+@DTYPES
+def test_reported_variant(dtype):
+    ctx = shim.Context(0)
+    narrow = _layer(ctx, dtype, (2, 32, 14, 14), 24, 3)
+    wide = _layer(ctx, dtype, (2, 256, 7, 7), 256, 3)
+    stem = _layer(ctx, dtype, (2, 3, 30, 30), 100, 3)
+    assert narrow(ROWS) == "wgrad rows"
+    assert wide(NO_GROUP) == "wgrad pair"
+    assert narrow(ROWS) == "wgrad rows"
+    assert stem() == "wgrad tap"
+    assert narrow(NO_GROUP) == "wgrad tap"
+    ctx.set_autotune(False)
+    assert narrow(NO_ROWS) == "wgrad groups"
+    ctx.close()
+
+
+@DTYPES
+@pytest.mark.parametrize("xs,k,ks", [((2, 32, 28, 28), 32, 3), ((16, 64, 14, 14), 30, 5), ((4, 100, 9, 30), 20, 2), ((8, 20, 40, 40), 128, 3)])
+def test_reported_variant_is_the_remembered_one(tmp_path, dtype, xs, k, ks):
+    ctx = shim.Context(0)
+    run = _layer(ctx, dtype, xs, k, ks)
+    first = run()
+    ctx.tuning_save(str(tmp_path / "tuning"))
+    choices = [l.split() for l in open(str(tmp_path / "tuning")).read().splitlines()]
+    (choice,) = [KERNELS[int(l[2])] for l in choices if l[0] == "a" and l[1].startswith("4.")]
+    assert first == choice and run() == choice
+    ctx.close()

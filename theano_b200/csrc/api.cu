@@ -109,7 +109,7 @@ struct b200conv_ctx {
   cudaEvent_t ev_tune0 = nullptr, ev_tune1 = nullptr;   // kernel selection timing
   long long launches = 0;
   const char* last_algo = "none";
-  const char* last_variant = "none";        // kernel variant of the last forward / gradInputs launch
+  const char* last_variant = "none";        // tensor-core kernel of the last result (timed trials come before it)
   // optional per-kernel timing: an event pair around every launch of our own kernels
   bool prof = false;
   struct ProfRec { int kind; cudaEvent_t a, b; };
@@ -1879,6 +1879,7 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
       CU_OK(c, cudaMemsetAsync(partial, 0, sizeof(float) * slab_elems * slabs, c->stream));
     p.partial = partial;
     p.partial_elems = (long long)slab_elems * slabs;
+    c->last_variant = "wgrad groups";
     KLAUNCH(c, kKWgradUmma, launch_wgrad_group(p, d.dtype, c->num_sms, c->stream));
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, Kg, p.diag_c, p.diag_k,
                                                   (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, c->stream));
@@ -2206,6 +2207,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     p.status = c->d_status;
     p.wait_clocks = c->wait_clocks;
     p.trace = c->trace;
+    c->last_variant = "wgrad tap";
     KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0,
                                                       s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
@@ -2316,6 +2318,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     p.status = c->d_status;
     p.wait_clocks = c->wait_clocks;
     p.trace = c->trace;
+    c->last_variant = "wgrad tap";
     if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, Cp, kBK,
                                                        d.flip, odt, c->stream));
@@ -2454,6 +2457,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       CU_OK(c, cudaMemsetAsync(partial, 0, sizeof(float) * slab_elems * slabs, c->stream));
     p.partial = partial;
     p.partial_elems = (long long)slab_elems * slabs;
+    c->last_variant = pair ? "wgrad pair" : "wgrad tap";
     if (p.ntaps > 0) {
       if (pair) KLAUNCH(c, kKWgradUmma, launch_wgrad_pair(p, d.dtype, c->num_sms, c->stream));
       else KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, BN, c->num_sms, c->stream));
@@ -3732,6 +3736,7 @@ extern "C" int b200conv_wgrad_static(b200conv_ctx* c, const b200conv_desc* dp, c
   p.partial_elems = (long long)(slab_bytes / sizeof(float)) * slabs;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
+  c->last_variant = "wgrad tap";
   if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, BN, c->num_sms, c->stream));
   KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(scratch, dw, slabs, p.taps_total, d.K, Cg, Kg, 0, 0,
                                                 (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, c->stream));

@@ -303,7 +303,7 @@ class Context(object):
 
     @property
     def last_variant(self):
-        """Kernel variant of the last forward or gradInputs launch ("tap", "slab pair", ...; see the header)."""
+        """Kernel variant of the last tensor-core launch ("tap", "slab pair", "wgrad rows", ...; see the header)."""
         return self.lib.b200conv_last_variant(self.h).decode()
 
     def padded_channels(self, c, dtype):
