@@ -56,7 +56,8 @@ enum {
   B200CONV_NO_SLAB = 1 << 8,     /* forward / gradInputs: fetch the activations once per filter tap
                                     (the general kernel) even where the slab kernel applies */
   B200CONV_NO_GROUP = 1 << 9,    /* gradWeights: one filter tap per work item (the general kernel)
-                                    even where taps can share their operands */
+                                    even where taps can share their operands, in merged groups and
+                                    folded stems too */
   B200CONV_NO_MERGE_PARITY = 1 << 10,/* strided gradInputs with few channels: one launch per stride
                                     parity class even where the classes can be merged into one */
   B200CONV_NO_S2D = 1 << 11,     /* forward, stride 2 with at most 4 channels: keep the pixels as they
@@ -70,8 +71,9 @@ enum {
                                     [N][Ho/2][Wo/2][Kp]; Ho and Wo must be even; geometries whose epilogue cannot pool
                                     return B200CONV_E_UNSUPPORTED (run the two calls instead) */
   B200CONV_ROWS = 1 << 14,       /* gradWeights: the kernel that stacks the filter's rows and columns inside one MMA
-                                    wherever it applies, timed or not */
-  B200CONV_NO_ROWS = 1 << 15     /* gradWeights: never that kernel */
+                                    wherever it applies, timed or not, whatever earlier calls chose and before
+                                    NO_GROUP; elsewhere as without the flag */
+  B200CONV_NO_ROWS = 1 << 15     /* gradWeights: never that kernel (before ROWS); calls without the flag choose for themselves */
 };
 
 /*

@@ -1746,9 +1746,11 @@ int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long lo
   return c->split_cache[key] = cand[best];
 }
 
+// NO_ROWS is part of a choice between kernels: what was chosen without one of them says nothing about calls that allow it.  (ROWS and
+// NO_GROUP decide before a choice is looked up.)
 GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
   return GeoKey{kind, d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.Ho, d.Wo,
-                d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : 0))};
+                d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : B200CONV_NO_ROWS))};
 }
 
 // Kernel and form of the layer in the key of a slice count: one layer's forms differ in their pixel tiles.
@@ -1929,14 +1931,15 @@ std::vector<RowsView> rows_views(b200conv_ctx* c, const b200conv_desc& d, const 
 }
 
 // gradWeights with the filter's rows and columns inside one MMA (wgrad_rows.cu).  Returns 0 when launched, 2 when the
-// layer is not one for it: more filters per group than a swizzle atom holds, uneven taps, rows too wide for a box.
+// layer is not one for it (more filters per group than a swizzle atom holds, uneven taps, rows too wide for a box) or the flags bar it.
 // `form`: kSplitsRows, or the form of x that the views are of; `reduce(partial, slabs)` enqueues the kernel that adds the slabs.
 template <class Reduce>
 int wgrad_rows(b200conv_ctx* c, const b200conv_desc& d, int form, const std::vector<RowsView>& views, int Cg, bool dropped, int taps_total, const void* gin,
                int flags, Scratch& tmp, int diag_c, int diag_k, Reduce reduce) {
   const bool f16 = d.dtype == B200CONV_F16;
   const int atom = f16 ? 64 : 32, kk = f16 ? 16 : 8, copies = 128 / atom, Kg = d.K / d.groups;
-  if ((flags & (B200CONV_NO_ROWS | B200CONV_ATOMIC_SPLITK)) || Kg > atom || views.empty() || views.size() > (size_t)kMaxViews) return 2;
+  const bool barred = (flags & (B200CONV_NO_ROWS | B200CONV_ATOMIC_SPLITK)) || (flags & (B200CONV_NO_GROUP | B200CONV_ROWS)) == B200CONV_NO_GROUP;
+  if (barred || Kg > atom || views.empty() || views.size() > (size_t)kMaxViews) return 2;
   RowsWgradParams p;
   memset(&p, 0, sizeof p);
   p.nviews = (int)views.size();
@@ -2085,8 +2088,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         });
       };
       const GeoKey key = wgrad_key(kGeoWgrad, d, flags);
-      int choice = 1;
-      if (c->autotune) {
+      int choice = 1;                                         // kernel(1) is 2 where the flags bar it
+      if (c->autotune && !(flags & (B200CONV_ROWS | B200CONV_NO_ROWS | B200CONV_NO_GROUP))) {
         auto it = c->algo_cache.find(key);
         if (it != c->algo_cache.end()) choice = it->second == kWgradRows;
         else if (!c->capturing && !c->model_only) {
@@ -2343,9 +2346,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   // without timings: the one-tap kernel where it runs 256-column MMAs (their issue and TMA
   // budgets are comfortable), tap groups for narrower layers (they read the operands 3x less)
   int choice = (flags & B200CONV_NO_GROUP) || (!c->autotune && Cg >= 256) ? kWgradTaps : kWgradGroups;
-  if (flags & B200CONV_ROWS) {
-    choice = kWgradRows;
-  } else if (choice == kWgradGroups && c->autotune) {
+  if ((flags & B200CONV_ROWS) && (rc = rows(tmp)) != 2) return rc;       // 2: not for this layer, then as without the flag
+  if (choice == kWgradGroups && c->autotune) {
     auto itc = c->algo_cache.find(key);
     if (itc != c->algo_cache.end()) {
       choice = itc->second;
