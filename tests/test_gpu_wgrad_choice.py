@@ -92,3 +92,26 @@ def test_rows_flag_where_the_kernel_does_not_apply(dtype):
     assert chosen in ("wgrad tap", "wgrad groups") and run(ROWS) == run() == chosen
     assert run(ROWS | NO_GROUP) == "wgrad tap"
     ctx.close()
+
+
+@pytest.mark.parametrize("tuned", [True, False])
+@pytest.mark.parametrize("dtype,n,kind", [(np.float32, 49, "wgrad tap"), (np.float32, 50, "wgrad rows"), (np.float16, 199, "wgrad tap"),
+                                          (np.float16, 200, None), (np.float16, 1000, "wgrad rows")])
+@pytest.mark.parametrize("xs,k,ks,s", [((3, 10, 10), 32, 3, 1), ((2, 20, 20), 16, 3, 2)], ids=["folded", "blocks"])
+def test_layers_with_few_channels(dtype, tuned, n, kind, xs, k, ks, s):
+    """100 output pixels per image: below and above the lines of the rule; None: between them, where a first call with timing on decides."""
+    ctx = shim.Context(0)
+    ctx.set_autotune(tuned)
+    run = _layer(ctx, dtype, (n,) + xs, k, ks, s)
+    first = run()
+    assert run() == first == (kind or (first if tuned else "wgrad rows"))
+    assert first in ("wgrad tap", "wgrad rows")
+    ctx.close()
+
+
+@pytest.mark.parametrize("dtype,n,kind", [(np.float32, 1, "wgrad rows"), (np.float16, 59, "wgrad groups"), (np.float16, 60, "wgrad rows")])
+def test_merged_groups_without_timing(dtype, n, kind):
+    ctx = shim.Context(0)
+    ctx.set_autotune(False)
+    assert _layer(ctx, dtype, (n, 64, 10, 10), 64, 3, g=8)() == kind
+    ctx.close()

@@ -1746,11 +1746,11 @@ int pick_splits(b200conv_ctx* c, const GeoKey& key, long long pix_tiles, long lo
   return c->split_cache[key] = cand[best];
 }
 
-// NO_ROWS is part of a choice between kernels: what was chosen without one of them says nothing about calls that allow it.  (ROWS and
-// NO_GROUP decide before a choice is looked up.)
+// NO_ROWS is part of a choice between kernels: what was chosen without one of them says nothing about calls that allow it.  So is NO_S2D,
+// which gives a layer another form.  (ROWS and NO_GROUP decide before a choice is looked up.)
 GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
   return GeoKey{kind, d.dtype, d.N, d.C, d.H, d.W, d.K, d.kH, d.kW, d.sH, d.sW, d.dilH, d.dilW, d.padH_l, d.padW_l, d.Ho, d.Wo,
-                d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : B200CONV_NO_ROWS))};
+                d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : B200CONV_NO_ROWS | B200CONV_NO_S2D))};
 }
 
 // Kernel and form of the layer in the key of a slice count: one layer's forms differ in their pixel tiles.
@@ -2037,6 +2037,47 @@ int merge_factor_rows(const b200conv_desc& d) {
 
 enum { kWgradTaps = 0, kWgradGroups = 1, kWgradRows = 2 };      // the gradWeights kernels; the numbers appear in tuning files
 
+// Stacked filter rows (true) or one tap per item for the forms of layers with few channels (pixel blocks, folded rows); *timed: too
+// close to tell, the first call of a geometry decides.  Replayed as graphs, one tap -> stacked: float32 up to 5000 output pixels
+// 7.8 to 10 us, 0.86 to 1.02 times as fast (one of 8 layers 1.25); from there on 9 to 323 us, 0.92 to 2.9 times (500 images 1 -> 20 filters 5x5
+// at 28x28 91 -> 32 us).  float16 up to 20000 pixels 7.5 to 11 us, 0.83 to 1.04 times; above 100000 1.13 to 2.1 times (7x7 stride 2, 256 images
+// of 224x224 306 -> 178 us); between them 0.88 (the same stem, 2 and 4 images: 12.4 -> 14.2, 14.9 -> 17.0 us) to 1.33.
+bool stem_rows(const b200conv_desc& d, bool* timed) {
+  const long long pixels = 1LL * d.N * d.Ho * d.Wo;
+  *timed = d.dtype == B200CONV_F16 && pixels >= 20000 && pixels < 100000;
+  return pixels >= (d.dtype == B200CONV_F16 ? 20000 : 5000);
+}
+
+// Stacked filter rows or another kernel, for the layers with two ways to run: timed on the first call of a geometry, or the former
+// if `prefer`.  rows() returns 2 where it does not apply; both leave the gradient and take scratch of their own.
+template <class Rows, class Other>
+int rows_or(b200conv_ctx* c, const GeoKey& key, int flags, bool timed, bool prefer, Rows rows, Other other) {
+  int rc, choice = prefer || (flags & B200CONV_ROWS) ? kWgradRows : kWgradTaps;
+  if (timed && c->autotune && !(flags & (B200CONV_ROWS | B200CONV_NO_ROWS | B200CONV_NO_GROUP))) {
+    auto it = c->algo_cache.find(key);
+    if (it != c->algo_cache.end()) choice = it->second;
+    else if (!c->capturing && !c->model_only) {
+      float ms[2];
+      int codes[2];
+      bool two = false;
+      auto run = [&](int v) -> int {
+        if (v) return two ? other() : 2;
+        const int r = rows();
+        two = r != 2;
+        return r;
+      };
+      if ((rc = rough_times(c, 2, run, ms, codes))) return rc;
+      if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) && (rc = time_variants(c, 2, run, ms, codes))) return rc;
+      for (int code : codes)
+        if (code && code != 2) return code;
+      choice = ms[0] >= 0.f && (ms[1] < 0.f || ms[0] < ms[1]) ? kWgradRows : kWgradTaps;
+      c->algo_cache[key] = choice;
+    }
+  }
+  if (choice == kWgradRows && (rc = rows()) != 2) return rc;
+  return other();
+}
+
 int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const void* dy, void* dw,
                  int flags) {
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;
@@ -2087,24 +2128,10 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
           return 0;
         });
       };
-      const GeoKey key = wgrad_key(kGeoWgrad, d, flags);
-      int choice = 1;                                         // kernel(1) is 2 where the flags bar it
-      if (c->autotune && !(flags & (B200CONV_ROWS | B200CONV_NO_ROWS | B200CONV_NO_GROUP))) {
-        auto it = c->algo_cache.find(key);
-        if (it != c->algo_cache.end()) choice = it->second == kWgradRows;
-        else if (!c->capturing && !c->model_only) {
-          float ms[2];
-          int codes[2];
-          if ((rc = rough_times(c, 2, kernel, ms, codes))) return rc;
-          if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) && (rc = time_variants(c, 2, kernel, ms, codes))) return rc;
-          for (int code : codes)
-            if (code && code != 2) return code;
-          choice = ms[1] >= 0.f && (ms[0] < 0.f || ms[1] < ms[0]);
-          c->algo_cache[key] = choice ? kWgradRows : kWgradTaps;
-        }
-      }
-      if (choice && (rc = kernel(1)) != 2) return rc;
-      return kernel(0);
+      // untimed: float32 gains at every size (2 to 256 images of 7x7 to 56x56, graphs: 0.99 to 2.1 times as fast), float16 not below 6000
+      // pixels (0.72 to 0.95, one of five layers 1.18; above 0.95 to 1.5, one of 11 layers 0.83)
+      const bool prefer = d.dtype == B200CONV_F32 || 1LL * d.N * d.Ho * d.Wo >= 6000;
+      return rows_or(c, wgrad_key(kGeoWgrad, d, flags), flags, true, prefer, [&] { return kernel(1); }, [&] { return kernel(0); });
     }
     if (umma_ok(dm)) {
       // few channels in all: the row-folded forms, then keep the diagonal blocks
@@ -2144,9 +2171,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * H2 * Wq * kS2dChannels, &xs))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_s2d(x, xs, d.N, d.C, d.H, d.W, Cp, H2, Wq, s2_q0, x_nhwc ? 1 : 0,
                                            d.dtype, c->stream));
-    {
-      // the filter's block rows stacked inside the MMAs where the filters leave room (7x7 stem 3 -> 64 of 256 images of
-      // 224 x 224, float16: 311 -> 183 us)
+    // the filter's block rows stacked inside the MMAs where the filters leave room
+    auto rows = [&]() -> int {
       RowsView v;
       for (int t = 0; t < s2_nt; ++t) { v.dh.push_back(t + s2_t0); v.tap.push_back(t); }
       v.dw.push_back(0);
@@ -2161,61 +2187,67 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         return r == CUDA_SUCCESS ? 0 : fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
       };
-      rc = wgrad_rows(c, d, kSplitsRowsS2d, {v}, win, false, s2_nt, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+      Scratch sc(c);
+      return wgrad_rows(c, d, kSplitsRowsS2d, {v}, win, false, s2_nt, gin, flags, sc, 0, 0, [&](float* partial, int slabs) {
         KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, slabs, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0, s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
         return 0;
       });
-      if (rc != 2) return rc;
-    }
-    UmmaWgradParams p;
-    memset(&p, 0, sizeof p);
-    const int atom = kBK;
-    choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
-    const bool swz32 = d.dtype == B200CONV_F32;
-    if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
-                        p.bn, swz32)))
-      return rc;
-    {
-      const size_t pix = (size_t)kS2dChannels * es, row = (size_t)Wq * pix;
-      cuuint64_t dims[5] = {(cuuint64_t)win, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
-      cuuint64_t strides[4] = {row, pix, row, (cuuint64_t)H2 * row};
-      cuuint32_t box[5] = {(cuuint32_t)atom, 1, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
-      cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-      CUresult r = c->encode(&p.x_views[0],
-                             d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                             5, xs, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             swz32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-      if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
-    }
-    for (int v = 1; v < kMaxViews; ++v) p.x_views[v] = p.x_views[0];
-    for (int t = 0; t < s2_nt; ++t) {
-      ConvTap tp;
-      tp.dh = (int16_t)(t + s2_t0); tp.dw = 0; tp.view = 0; tp.wmat = (int16_t)t;
-      p.taps[p.ntaps++] = tp;
-    }
-    p.groups = 1; p.Kg = d.K; p.Cg = win;
-    p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
-    p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
-    p.ktiles = (int)cdiv(d.K, 128); p.ctiles = 1;
-    p.taps_total = s2_nt;
-    const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
-    const long long base_items = 1LL * p.ktiles * p.ntaps;
-    p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
-    const size_t slab_elems = (size_t)s2_nt * d.K * win;
-    float* partial;
-    if ((rc = tmp.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
-    p.partial = partial;
-    p.partial_elems = (long long)slab_elems * p.splits;
-    p.status = c->d_status;
-    p.wait_clocks = c->wait_clocks;
-    p.trace = c->trace;
-    c->last_variant = "wgrad tap";
-    KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
-    KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0,
-                                                      s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
-    c->last_algo = "umma";
-    return 0;
+    };
+    auto single = [&]() -> int {
+      Scratch sc(c);
+      UmmaWgradParams p;
+      memset(&p, 0, sizeof p);
+      const int atom = kBK;
+      choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
+      const bool swz32 = d.dtype == B200CONV_F32;
+      if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
+                          p.bn, swz32)))
+        return rc;
+      {
+        const size_t pix = (size_t)kS2dChannels * es, row = (size_t)Wq * pix;
+        cuuint64_t dims[5] = {(cuuint64_t)win, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
+        cuuint64_t strides[4] = {row, pix, row, (cuuint64_t)H2 * row};
+        cuuint32_t box[5] = {(cuuint32_t)atom, 1, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
+        cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+        CUresult r = c->encode(&p.x_views[0],
+                               d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                               5, xs, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                               swz32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
+      }
+      for (int v = 1; v < kMaxViews; ++v) p.x_views[v] = p.x_views[0];
+      for (int t = 0; t < s2_nt; ++t) {
+        ConvTap tp;
+        tp.dh = (int16_t)(t + s2_t0); tp.dw = 0; tp.view = 0; tp.wmat = (int16_t)t;
+        p.taps[p.ntaps++] = tp;
+      }
+      p.groups = 1; p.Kg = d.K; p.Cg = win;
+      p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
+      p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
+      p.ktiles = (int)cdiv(d.K, 128); p.ctiles = 1;
+      p.taps_total = s2_nt;
+      const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
+      const long long base_items = 1LL * p.ktiles * p.ntaps;
+      p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
+      const size_t slab_elems = (size_t)s2_nt * d.K * win;
+      float* partial;
+      if ((rc = sc.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
+      p.partial = partial;
+      p.partial_elems = (long long)slab_elems * p.splits;
+      p.status = c->d_status;
+      p.wait_clocks = c->wait_clocks;
+      p.trace = c->trace;
+      c->last_variant = "wgrad tap";
+      KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
+      KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0,
+                                                        s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
+      c->last_algo = "umma";
+      return 0;
+    };
+    bool timed;
+    const bool stacked = stem_rows(d, &timed);
+    return rows_or(c, wgrad_key(kGeoWgrad, d, flags), flags, timed, stacked, rows, single);
   }
   if (fold_ok(d) && !(flags & B200CONV_ATOMIC_SPLITK)) {
     // few input channels: the x operand is the row-folded image (kW pixels x Cp channels per
@@ -2228,8 +2260,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * d.H * Wp * Cp, &xp))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_fold(x, xp, d.N, d.C, d.H, d.W, Cp, Wp, d.padW_l, x_nhwc ? 1 : 0,
                                             d.dtype, c->stream));
-    {
-      // the filter rows stacked inside the MMAs where the filters leave room
+    // the filter rows stacked inside the MMAs where the filters leave room
+    auto rows = [&]() -> int {
       std::vector<RowsView> views;
       bool dropped = false;
       for (int rh = 0; rh < d.sH; ++rh) {
@@ -2254,79 +2286,85 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         };
         views.push_back(v);
       }
-      rc = wgrad_rows(c, d, kSplitsRowsFold, views, kBK, dropped, d.kH, gin, flags, tmp, 0, 0, [&](float* partial, int slabs) {
+      Scratch sc(c);
+      return wgrad_rows(c, d, kSplitsRowsFold, views, kBK, dropped, d.kH, gin, flags, sc, 0, 0, [&](float* partial, int slabs) {
         KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, slabs, d.K, d.C, d.kH, d.kW, Cp, kBK, d.flip, odt, c->stream));
         return 0;
       });
-      if (rc != 2) return rc;
-    }
-    FwdLikeArgs a;
-    a.act = xp; a.Hs = d.H; a.Ws = d.Wo; a.Cin_g = kBK; a.Cp_in = Cp; a.N = d.N; a.dtype = d.dtype;
-    a.groups = 1; a.view_sH = d.sH; a.view_sW = 1;
-    a.fold = true; a.fold_Wp = Wp; a.fold_sW = d.sW;
-    UmmaWgradParams p;
-    memset(&p, 0, sizeof p);
-    const int atom = kBK;
-    choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
-    const bool swz32 = d.dtype == B200CONV_F32;
-    if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
-                        p.bn, swz32)))
-      return rc;
-    int nviews = 0, view_of_parity[kMaxViews];
-    for (int q = 0; q < kMaxViews; ++q) view_of_parity[q] = -2;
-    bool dropped = false;
-    for (int i = 0; i < d.kH; ++i) {
-      const int ah = i * d.dilH - d.padH_l, rh = pymod(ah, d.sH);
-      if (view_of_parity[rh] == -2) {
-        view_of_parity[rh] = -1;
-        if (rh < d.H) {
-          // the folded view with the 32-byte-atom swizzle gradWeights needs for tf32
-          const size_t pix = (size_t)Cp * es, row = (size_t)Wp * pix;
-          const int H2 = (d.H - rh + d.sH - 1) / d.sH;
-          cuuint64_t dims[5] = {(cuuint64_t)kBK, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
-          cuuint64_t strides[4] = {row, (cuuint64_t)d.sW * pix, (cuuint64_t)d.sH * row, (cuuint64_t)d.H * row};
-          cuuint32_t box[5] = {(cuuint32_t)atom, 1, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
-          cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-          char* base = static_cast<char*>(xp) + (size_t)rh * row;
-          CUresult r = c->encode(&p.x_views[nviews],
-                                 d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                                 5, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                 swz32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-          if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(folded x) failed: %d", (int)r);
-          view_of_parity[rh] = nviews++;
+    };
+    auto single = [&]() -> int {
+      Scratch sc(c);
+      FwdLikeArgs a;
+      a.act = xp; a.Hs = d.H; a.Ws = d.Wo; a.Cin_g = kBK; a.Cp_in = Cp; a.N = d.N; a.dtype = d.dtype;
+      a.groups = 1; a.view_sH = d.sH; a.view_sW = 1;
+      a.fold = true; a.fold_Wp = Wp; a.fold_sW = d.sW;
+      UmmaWgradParams p;
+      memset(&p, 0, sizeof p);
+      const int atom = kBK;
+      choose_tile(c, d.Wo, d.Ho, d.N, wgrad_pix(d.dtype), d.dtype == B200CONV_F16 ? 16 : 8, &p.bw, &p.bh, &p.bn);
+      const bool swz32 = d.dtype == B200CONV_F32;
+      if ((rc = make_view(c, &p.dy_map, gin, d.dtype, d.K, 1, Kp, d.Wo, d.Ho, d.N, 0, 0, 1, 1, atom, p.bw, p.bh,
+                          p.bn, swz32)))
+        return rc;
+      int nviews = 0, view_of_parity[kMaxViews];
+      for (int q = 0; q < kMaxViews; ++q) view_of_parity[q] = -2;
+      bool dropped = false;
+      for (int i = 0; i < d.kH; ++i) {
+        const int ah = i * d.dilH - d.padH_l, rh = pymod(ah, d.sH);
+        if (view_of_parity[rh] == -2) {
+          view_of_parity[rh] = -1;
+          if (rh < d.H) {
+            // the folded view with the 32-byte-atom swizzle gradWeights needs for tf32
+            const size_t pix = (size_t)Cp * es, row = (size_t)Wp * pix;
+            const int H2 = (d.H - rh + d.sH - 1) / d.sH;
+            cuuint64_t dims[5] = {(cuuint64_t)kBK, 1, (cuuint64_t)d.Wo, (cuuint64_t)H2, (cuuint64_t)d.N};
+            cuuint64_t strides[4] = {row, (cuuint64_t)d.sW * pix, (cuuint64_t)d.sH * row, (cuuint64_t)d.H * row};
+            cuuint32_t box[5] = {(cuuint32_t)atom, 1, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
+            cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+            char* base = static_cast<char*>(xp) + (size_t)rh * row;
+            CUresult r = c->encode(&p.x_views[nviews],
+                                   d.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                                   5, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   swz32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
+                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(folded x) failed: %d", (int)r);
+            view_of_parity[rh] = nviews++;
+          }
         }
+        if (view_of_parity[rh] < 0) { dropped = true; continue; }
+        ConvTap t;
+        t.dh = (int16_t)floordiv(ah, d.sH); t.dw = 0; t.view = (int16_t)view_of_parity[rh]; t.wmat = (int16_t)i;
+        p.taps[p.ntaps++] = t;
       }
-      if (view_of_parity[rh] < 0) { dropped = true; continue; }
-      ConvTap t;
-      t.dh = (int16_t)floordiv(ah, d.sH); t.dw = 0; t.view = (int16_t)view_of_parity[rh]; t.wmat = (int16_t)i;
-      p.taps[p.ntaps++] = t;
-    }
-    for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = nviews ? p.x_views[0] : p.dy_map;
-    p.groups = 1; p.Kg = d.K; p.Cg = kBK;
-    p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
-    p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
-    p.ktiles = (int)cdiv(d.K, 128); p.ctiles = 1;
-    p.taps_total = d.kH;
-    const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
-    const long long base_items = 1LL * p.ktiles * std::max(1, p.ntaps);
-    p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
-    const size_t slab_elems = (size_t)d.kH * d.K * kBK;
-    float* partial;
-    if ((rc = tmp.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
-    if (dropped || p.ntaps == 0)
-      CU_OK(c, cudaMemsetAsync(partial, 0, sizeof(float) * slab_elems * p.splits, c->stream));
-    p.partial = partial;
-    p.partial_elems = (long long)slab_elems * p.splits;
-    p.status = c->d_status;
-    p.wait_clocks = c->wait_clocks;
-    p.trace = c->trace;
-    c->last_variant = "wgrad tap";
-    if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
-    KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, Cp, kBK,
-                                                       d.flip, odt, c->stream));
-    c->last_algo = "umma";
-    return 0;
+      for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = nviews ? p.x_views[0] : p.dy_map;
+      p.groups = 1; p.Kg = d.K; p.Cg = kBK;
+      p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
+      p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
+      p.ktiles = (int)cdiv(d.K, 128); p.ctiles = 1;
+      p.taps_total = d.kH;
+      const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n;
+      const long long base_items = 1LL * p.ktiles * std::max(1, p.ntaps);
+      p.splits = (int)balanced_splits(c, pix_tiles, base_items, c->num_sms, pix_tiles / 4, 2);
+      const size_t slab_elems = (size_t)d.kH * d.K * kBK;
+      float* partial;
+      if ((rc = sc.get(sizeof(float) * slab_elems * p.splits, reinterpret_cast<void**>(&partial)))) return rc;
+      if (dropped || p.ntaps == 0)
+        CU_OK(c, cudaMemsetAsync(partial, 0, sizeof(float) * slab_elems * p.splits, c->stream));
+      p.partial = partial;
+      p.partial_elems = (long long)slab_elems * p.splits;
+      p.status = c->d_status;
+      p.wait_clocks = c->wait_clocks;
+      p.trace = c->trace;
+      c->last_variant = "wgrad tap";
+      if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
+      KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, Cp, kBK,
+                                                         d.flip, odt, c->stream));
+      c->last_algo = "umma";
+      return 0;
+    };
+    bool timed;
+    const bool stacked = stem_rows(d, &timed);
+    return rows_or(c, wgrad_key(kGeoWgrad, d, flags), flags, timed, stacked, rows, single);
   }
   if (!x_nhwc && (rc = to_nhwc(c, tmp, x, d.N, d.C, d.H, d.W, d.dtype, &xin))) return rc;
   if (!dy_nhwc && (rc = to_nhwc(c, tmp, dy, d.N, d.K, d.Ho, d.Wo, d.dtype, &gin))) return rc;
