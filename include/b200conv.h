@@ -290,8 +290,8 @@ int b200conv_set_splits(b200conv_ctx* ctx, int splits);
 /* The choices made by timing (kernel variant per geometry, slice counts) written to / read from a
  * text file, so that a later process starts with them instead of timing again: the persistent form
  * of the cache the reference's meta-optimizer keeps per process (theano/gpuarray/opt.py:2144-2222;
- * flags metaopt.*, theano/configdefaults.py:1545-1551).  A file written on another device model or
- * for another SM count is refused.  *loaded = number of choices read. */
+ * flags metaopt.*, theano/configdefaults.py:1545-1551).  A file written on another device model,
+ * for another SM count or by a version of the library whose kernels it does not fit is refused.  *loaded = number of choices read. */
 int b200conv_tuning_save(b200conv_ctx* ctx, const char* path);
 int b200conv_tuning_load(b200conv_ctx* ctx, const char* path, int* loaded);
 /* Development aid: while dbuf (device memory, 32 x int64 per SM) is set, the slab convolution

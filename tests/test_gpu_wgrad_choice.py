@@ -115,3 +115,19 @@ def test_merged_groups_without_timing(dtype, n, kind):
     ctx.set_autotune(False)
     assert _layer(ctx, dtype, (n, 64, 10, 10), 64, 3, g=8)() == kind
     ctx.close()
+
+
+def test_a_file_of_other_kernels_is_not_loaded(tmp_path):
+    """Choices timed on other kernels would keep this version's from being tried."""
+    path = str(tmp_path / "tuning")
+    ctx = shim.Context(0)
+    _layer(ctx, np.float32, (2, 32, 14, 14), 24, 3)()
+    ctx.tuning_save(path)
+    head, rest = open(path).read().split("\n", 1)
+    assert " kernels " in head and ctx.tuning_load(path) == len(rest.splitlines()) > 0
+    older = head[:head.index(" kernels ")]                       # as files before that number have it
+    for other in (older, older + " kernels 1", head + "1"):
+        open(path, "w").write(other + "\n" + rest)
+        with pytest.raises(ValueError, match="version of the kernels"):
+            ctx.tuning_load(path)
+    ctx.close()

@@ -3392,15 +3392,19 @@ int b200conv_set_splits(b200conv_ctx* c, int splits) {
   return 0;
 }
 
-// The tuning file: a header line naming the device the choices were timed on, then one line per
-// choice.  Choices made on another device model or SM count are not loaded.
+// The tuning file: a header line naming the device the choices were timed on and the kernels, then one line per
+// choice.  Choices made on another device model, SM count or set of kernels are not loaded.
+// kTuningKernels goes up with each change of the kernels after which earlier timings or the numbers of choices no longer hold.
+// 2: three gradWeights kernels to choose from where there were two, float32 pairs behind the one-tap choice.  (Files before it
+// have no such number.)
+constexpr int kTuningKernels = 2;
 static std::string tuning_header(b200conv_ctx* c) {
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, c->device);
   std::string name = prop.name;
   for (char& ch : name)
     if (ch == ' ') ch = '_';
-  return "b200conv-tuning 1 " + name + " " + std::to_string(c->num_sms);
+  return "b200conv-tuning 1 " + name + " " + std::to_string(c->num_sms) + " kernels " + std::to_string(kTuningKernels);
 }
 
 int b200conv_tuning_save(b200conv_ctx* c, const char* path) {
@@ -3433,7 +3437,7 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
   }
   if (!ok) {
     fclose(f);
-    return fail(c, B200CONV_E_INVALID, "%s was not written for this device and SM count", path);
+    return fail(c, B200CONV_E_INVALID, "%s was not written for this device, SM count and version of the kernels", path);
   }
   while (fgets(line, sizeof line, f)) {
     char kind = 0, text[400];
