@@ -2049,7 +2049,8 @@ bool stem_rows(const b200conv_desc& d, bool* timed) {
 }
 
 // Stacked filter rows or another kernel, for the layers with two ways to run: timed on the first call of a geometry, or the former
-// if `prefer`.  rows() returns 2 where it does not apply; both leave the gradient and take scratch of their own.
+// if `prefer`.  rows() returns 2 where it does not apply; both leave the gradient and take scratch of their own.  Stacked rows
+// have the most slices (an item is all taps of a channel tile), up to ten times the other kernels': without memory for them the other runs.
 template <class Rows, class Other>
 int rows_or(b200conv_ctx* c, const GeoKey& key, int flags, bool timed, bool prefer, Rows rows, Other other) {
   int rc, choice = prefer || (flags & B200CONV_ROWS) ? kWgradRows : kWgradTaps;
@@ -2059,22 +2060,23 @@ int rows_or(b200conv_ctx* c, const GeoKey& key, int flags, bool timed, bool pref
     else if (!c->capturing && !c->model_only) {
       float ms[2];
       int codes[2];
-      bool two = false;
+      bool two = false, no_memory = false;
       auto run = [&](int v) -> int {
         if (v) return two ? other() : 2;
         const int r = rows();
-        two = r != 2;
-        return r;
+        no_memory |= r == B200CONV_E_NOMEM;
+        two = r != 2 && r != B200CONV_E_NOMEM;
+        return two ? r : 2;
       };
       if ((rc = rough_times(c, 2, run, ms, codes))) return rc;
       if (!codes[0] && !codes[1] && std::max(ms[0], ms[1]) <= kFarBehind * std::min(ms[0], ms[1]) && (rc = time_variants(c, 2, run, ms, codes))) return rc;
       for (int code : codes)
         if (code && code != 2) return code;
       choice = ms[0] >= 0.f && (ms[1] < 0.f || ms[0] < ms[1]) ? kWgradRows : kWgradTaps;
-      c->algo_cache[key] = choice;
+      if (!no_memory) c->algo_cache[key] = choice;
     }
   }
-  if (choice == kWgradRows && (rc = rows()) != 2) return rc;
+  if (choice == kWgradRows && (rc = rows()) != 2 && rc != B200CONV_E_NOMEM) return rc;
   return other();
 }
 
@@ -2384,7 +2386,8 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
   // without timings: the one-tap kernel where it runs 256-column MMAs (their issue and TMA
   // budgets are comfortable), tap groups for narrower layers (they read the operands 3x less)
   int choice = (flags & B200CONV_NO_GROUP) || (!c->autotune && Cg >= 256) ? kWgradTaps : kWgradGroups;
-  if ((flags & B200CONV_ROWS) && (rc = rows(tmp)) != 2) return rc;       // 2: not for this layer, then as without the flag
+  // (2: not for this layer; without memory for its slices the others run, as in rows_or)
+  if ((flags & B200CONV_ROWS) && (rc = rows(tmp)) != 2 && rc != B200CONV_E_NOMEM) return rc;
   if (choice == kWgradGroups && c->autotune) {
     auto itc = c->algo_cache.find(key);
     if (itc != c->algo_cache.end()) {
@@ -2396,11 +2399,12 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       const int order[3] = {kWgradRows, kWgradGroups, kWgradTaps};
       float ms[3];
       int codes[3];
-      bool others = false;                                    // another kernel than the one-tap form applies
+      bool others = false, no_memory = false;                 // others: another kernel than the one-tap form applies
       auto kernel = [&](int i) -> int {
         if (order[i] == kWgradTaps) return others ? wgrad_device(c, d, xin, gin, dw, flags | B200CONV_NO_GROUP | B200CONV_IN_NHWC | B200CONV_IN2_NHWC) : 2;
         Scratch trial(c);
-        const int r = order[i] == kWgradGroups ? wgrad_grouped(c, d, xin, gin, dw, flags, trial) : rows(trial);
+        int r = order[i] == kWgradGroups ? wgrad_grouped(c, d, xin, gin, dw, flags, trial) : rows(trial);
+        if (order[i] == kWgradRows && r == B200CONV_E_NOMEM) { no_memory = true; r = 2; }
         others |= r != 2;
         return r;
       };
@@ -2421,10 +2425,10 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       least = -1.f;
       for (int i = 0; i < 3; ++i)
         if (ms[i] >= 0.f && (least < 0.f || ms[i] < least)) { least = ms[i]; choice = order[i]; }
-      c->algo_cache[key] = choice;
+      if (!no_memory) c->algo_cache[key] = choice;
     }
   }
-  if (choice == kWgradRows && (rc = rows(tmp)) != 2) return rc;
+  if (choice == kWgradRows && (rc = rows(tmp)) != 2 && rc != B200CONV_E_NOMEM) return rc;
   if (choice != kWgradTaps) {
     rc = wgrad_grouped(c, d, xin, gin, dw, flags, tmp);
     if (rc != 2) return rc;     // 2: geometry not covered, use the one-tap-per-item kernel
