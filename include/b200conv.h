@@ -128,7 +128,10 @@ int b200conv_fwd_epilogue(b200conv_ctx* ctx, const b200conv_desc* d, const void*
 /* Replaces corrMM(direction 2), corr_gemm.c:486-529: dx = gradient wrt the image. */
 int b200conv_dgrad(b200conv_ctx* ctx, const b200conv_desc* d, const void* w, const void* dy,
                    void* dx, int flags);
-/* Replaces corrMM(direction 1), corr_gemm.c:372-456: dw = gradient wrt the filters. */
+/* Replaces corrMM(direction 1), corr_gemm.c:372-456: dw = gradient wrt the filters.
+ * An infinity or NaN in x or dy reaches those elements of dw whose sums it belongs to, whichever kernel runs.  x outside of the
+ * image counts as zeros that take part, as in the reference's im2col form, so that an infinity in dy makes NaN of the taps that lie
+ * outside there (the direct kernels leave such products out). */
 int b200conv_wgrad(b200conv_ctx* ctx, const b200conv_desc* d, const void* x, const void* dy,
                    void* dw, int flags);
 

@@ -36,7 +36,7 @@ def test_forms_of_one_layer(dtype, order, n, h, k, ks):
 
 @DTYPES
 @pytest.mark.parametrize("factor", [1, 3, 1000])
-@pytest.mark.parametrize("xs,k,ks,flags", [((8, 3, 64, 64), 32, (4, 4), 0), ((3, 40, 20, 9), 24, (3, 3), shim.ROWS), ((3, 40, 20, 9), 24, (3, 3), 0),
+@pytest.mark.parametrize("xs,k,ks,flags", [((8, 3, 64, 64), 32, (4, 4), shim.ROWS), ((3, 40, 20, 9), 24, (3, 3), shim.ROWS), ((3, 40, 20, 9), 24, (3, 3), 0),
                                            ((3, 40, 20, 9), 24, (3, 3), shim.NO_GROUP), ((2, 260, 9, 9), 300, (2, 2), shim.NO_GROUP)])
 def test_counts_out_of_a_file(tmp_path, dtype, factor, xs, k, ks, flags):
     path, kw = str(tmp_path / "tuning"), dict(border_mode=(1, 1))

@@ -1753,6 +1753,27 @@ GeoKey wgrad_key(int kind, const b200conv_desc& d, int flags) {
                 d.groups, flags & (B200CONV_ATOMIC_SPLITK | (kind == kGeoSplits ? B200CONV_DW_F32 : B200CONV_NO_ROWS | B200CONV_NO_S2D))};
 }
 
+// The sums of a gradient (wgrad_exact.cuh); during a call on merged groups `d` is the merged layer, and its groups are the layer's own.
+WgradSum wgrad_sum(const b200conv_ctx* c, const b200conv_desc& d, const void* x, bool x_nhwc, const void* dy, bool dy_nhwc) {
+  WgradSum s;
+  s.x = x; s.dy = dy;
+  s.f16 = d.dtype == B200CONV_F16;
+  s.Cg = c->diag_c ? c->diag_c : d.C / d.groups;
+  s.Kg = c->diag_k ? c->diag_k : d.K / d.groups;
+  s.N = d.N; s.H = d.H; s.W = d.W; s.Ho = d.Ho; s.Wo = d.Wo; s.kH = d.kH; s.kW = d.kW;
+  s.sH = d.sH; s.sW = d.sW; s.dilH = d.dilH; s.dilW = d.dilW; s.padH = d.padH_l; s.padW = d.padW_l; s.flip = d.flip;
+  s.segments = 0;
+  s.x_c = x_nhwc ? 1 : 1LL * d.H * d.W;
+  s.x_w = x_nhwc ? pad_channels(d.C, d.dtype) : 1;
+  s.x_h = s.x_w * d.W;
+  s.x_n = x_nhwc ? s.x_h * d.H : s.x_c * d.C;
+  s.dy_c = dy_nhwc ? 1 : 1LL * d.Ho * d.Wo;
+  s.dy_w = dy_nhwc ? pad_channels(d.K, d.dtype) : 1;
+  s.dy_h = s.dy_w * d.Wo;
+  s.dy_n = dy_nhwc ? s.dy_h * d.Ho : s.dy_c * d.K;
+  return s;
+}
+
 // Kernel and form of the layer in the key of a slice count: one layer's forms differ in their pixel tiles.
 enum { kSplitsGroups = 0, kSplitsTaps, kSplitsPair, kSplitsRows, kSplitsRowsS2d, kSplitsRowsFold };
 
@@ -1883,8 +1904,10 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
     p.partial_elems = (long long)slab_elems * slabs;
     c->last_variant = "wgrad groups";
     KLAUNCH(c, kKWgradUmma, launch_wgrad_group(p, d.dtype, c->num_sms, c->stream));
+    WgradSum sum = wgrad_sum(c, d, xin, true, gin, true);
+    sum.segments = p.tiles_w > 1 && p.rows_a % (d.dtype == B200CONV_F16 ? 16 : 8);      // zeros fill the last MMA of every segment
     KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, Kg, p.diag_c, p.diag_k,
-                                                  (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, c->stream));
+                                                  (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, sum, c->stream));
     return 0;
   };
   GeoKey skey = wgrad_key(kGeoSplits, d, flags);
@@ -2126,7 +2149,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         Scratch trial(c);
         const int dc = mr > 1 ? Cg : 0, dk = mr > 1 ? Kg : 0;
         return wgrad_rows(c, dr, kSplitsRows, views, Cg * mr, dropped, d.kH * d.kW, gin, flags, trial, dc, dk, [&](float* partial, int slabs) {
-          KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg * mr, Kg * mr, dc, dk, odt, c->stream));
+          KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg * mr, Kg * mr, dc, dk, odt, wgrad_sum(c, d, xin, true, gin, true), c->stream));
           return 0;
         });
       };
@@ -2173,6 +2196,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * H2 * Wq * kS2dChannels, &xs))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_s2d(x, xs, d.N, d.C, d.H, d.W, Cp, H2, Wq, s2_q0, x_nhwc ? 1 : 0,
                                            d.dtype, c->stream));
+    const WgradSum sum = wgrad_sum(c, d, x, x_nhwc, gin, true);
     // the filter's block rows stacked inside the MMAs where the filters leave room
     auto rows = [&]() -> int {
       RowsView v;
@@ -2191,7 +2215,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       };
       Scratch sc(c);
       return wgrad_rows(c, d, kSplitsRowsS2d, {v}, win, false, s2_nt, gin, flags, sc, 0, 0, [&](float* partial, int slabs) {
-        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, slabs, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0, s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
+        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, slabs, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0, s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, sum, c->stream));
         return 0;
       });
     };
@@ -2243,7 +2267,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       c->last_variant = "wgrad tap";
       KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
       KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_s2d(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, s2_nt, s2_t0,
-                                                        s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, c->stream));
+                                                        s2_q0, d.padH_l, d.padW_l, win, d.flip, odt, sum, c->stream));
       c->last_algo = "umma";
       return 0;
     };
@@ -2262,6 +2286,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     if ((rc = tmp.get(es * (size_t)d.N * d.H * Wp * Cp, &xp))) return rc;
     KLAUNCH(c, kKTranspose, launch_pad_fold(x, xp, d.N, d.C, d.H, d.W, Cp, Wp, d.padW_l, x_nhwc ? 1 : 0,
                                             d.dtype, c->stream));
+    const WgradSum sum = wgrad_sum(c, d, x, x_nhwc, gin, true);
     // the filter rows stacked inside the MMAs where the filters leave room
     auto rows = [&]() -> int {
       std::vector<RowsView> views;
@@ -2290,7 +2315,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       }
       Scratch sc(c);
       return wgrad_rows(c, d, kSplitsRowsFold, views, kBK, dropped, d.kH, gin, flags, sc, 0, 0, [&](float* partial, int slabs) {
-        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, slabs, d.K, d.C, d.kH, d.kW, Cp, kBK, d.flip, odt, c->stream));
+        KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, slabs, d.K, d.C, d.kH, d.kW, Cp, kBK, d.flip, odt, sum, c->stream));
         return 0;
       });
     };
@@ -2360,7 +2385,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       c->last_variant = "wgrad tap";
       if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, 64, c->num_sms, c->stream));
       KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce_fold(partial, dw, p.splits, d.K, d.C, d.kH, d.kW, Cp, kBK,
-                                                         d.flip, odt, c->stream));
+                                                         d.flip, odt, sum, c->stream));
       c->last_algo = "umma";
       return 0;
     };
@@ -2378,7 +2403,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
     bool dropped;
     const std::vector<RowsView> views = rows_views(c, d, xin, &dropped);
     return wgrad_rows(c, d, kSplitsRows, views, Cg, dropped, d.kH * d.kW, gin, flags, sc, c->diag_c, c->diag_k, [&](float* partial, int slabs) {
-      KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg, Kg, c->diag_c, c->diag_k, odt, c->stream));
+      KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, d.kH * d.kW, d.K, Cg, Kg, c->diag_c, c->diag_k, odt, wgrad_sum(c, d, xin, true, gin, true), c->stream));
       return 0;
     });
   };
@@ -2506,7 +2531,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       if (pair) KLAUNCH(c, kKWgradUmma, launch_wgrad_pair(p, d.dtype, c->num_sms, c->stream));
       else KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, BN, c->num_sms, c->stream));
     }
-    KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, Kg, p.diag_c, p.diag_k, odt, c->stream));
+    KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(partial, dw, slabs, p.taps_total, d.K, Cg, Kg, p.diag_c, p.diag_k, odt, wgrad_sum(c, d, xin, true, gin, true), c->stream));
     return 0;
   };
   GeoKey skey = wgrad_key(kGeoSplits, d, flags);
@@ -3787,7 +3812,7 @@ extern "C" int b200conv_wgrad_static(b200conv_ctx* c, const b200conv_desc* dp, c
   c->last_variant = "wgrad tap";
   if (p.ntaps > 0) KLAUNCH(c, kKWgradUmma, launch_wgrad_umma(p, d.dtype, BN, c->num_sms, c->stream));
   KLAUNCH(c, kKWgradReduce, launch_wgrad_reduce(scratch, dw, slabs, p.taps_total, d.K, Cg, Kg, 0, 0,
-                                                (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, c->stream));
+                                                (flags & B200CONV_DW_F32) ? B200CONV_F32 : d.dtype, wgrad_sum(c, d, x, true, dy, true), c->stream));
   c->last_algo = "umma";
   return 0;
 }

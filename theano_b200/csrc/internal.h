@@ -280,9 +280,18 @@ cudaError_t launch_wgrad_umma(const UmmaWgradParams& p, int dtype, int bn_cols, 
 // The same work on pairs of CTAs (wgrad_pair.cu): 256-filter x 256-channel tiles, stages of 64 pixels;
 // `ktiles` / `ctiles` count 256-wide tiles.
 cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int dtype, int num_sms, cudaStream_t s);
+// What the elements of a gradient are sums of (wgrad_exact.cuh): the operands with their strides in elements, and the geometry.
+struct WgradSum {
+  const void *x, *dy;
+  long long x_n, x_c, x_h, x_w, dy_n, dy_c, dy_h, dy_w;
+  int f16;                               // type of x and dy
+  int Cg, Kg;                            // channels / filters per group (of a layer's own groups, not of merged ones)
+  int N, H, W, Ho, Wo, kH, kW, sH, sW, dilH, dilW, padH, padW, flip;
+  int segments;                          // 1: zeros for dy stand behind pieces of rows too, whose ends may lie anywhere in an image
+};
 // Sums split-K slabs and writes the OIHW gradient; diag_c / diag_k as above (Kg: filters per merged group).
 cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K, int Cg, int Kg, int diag_c, int diag_k,
-                                int dtype, cudaStream_t s);
+                                int dtype, const WgradSum& sum, cudaStream_t s);
 
 // ---- filter gradient with tap groups sharing their operands (wgrad_group.cu) -------------
 // Taps that read the same view with the same row offset differ only by a column offset.  With
@@ -405,9 +414,9 @@ cudaError_t launch_pack_filters_s2d(const void* w, void* dst, int K, int C, int 
                                     cudaStream_t s);
 cudaError_t launch_wgrad_reduce_s2d(const float* partial, void* dw, int splits, int K, int C, int kH,
                                     int kW, int ntaps, int t0, int q0, int padH, int padW, int ld, int flip,
-                                    int dtype, cudaStream_t s);
+                                    int dtype, const WgradSum& sum, cudaStream_t s);
 cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits, int K, int C, int kH,
-                                     int kW, int Cp, int ld, int flip, int dtype, cudaStream_t s);
+                                     int kW, int Cp, int ld, int flip, int dtype, const WgradSum& sum, cudaStream_t s);
 // Block-diagonal filters for merged groups (extract = 0) and the inverse for the gradient (1).
 cudaError_t launch_merge_groups(const void* src, void* dst, int K, int Cg, int Kg, int m, int taps,
                                 int extract, int dtype, cudaStream_t s);

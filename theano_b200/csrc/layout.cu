@@ -3,6 +3,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "wgrad_exact.cuh"
 #include "wgrad_slab.cuh"
 
 namespace b200 {
@@ -266,13 +267,14 @@ __global__ void pack_filters_s2d_kernel(const T* __restrict__ w, T* __restrict__
 // Adds the slabs (wgrad_slab.cuh, rows of ld columns) of a gradient whose columns are not the filters' own channels: place(c, i', j') gives
 // the slab tap and column of a filter element.  A block takes 32 filters of one element: neighbouring threads read neighbouring
 // filters (16 bytes apart), eight threads share a sum (slabs l, l + 8, ..., then in order of l), so that a chain of loads
-// is an eighth of the slices long.
+// is an eighth of the slices long.  `sum`: for sums that are NaN (wgrad_exact.cuh).
 template <typename T, class Place>
 __device__ __forceinline__ void reduce_gathered(const float* __restrict__ partial, T* __restrict__ dw, int splits, int K, int C, int kH, int kW,
-                                                int ntaps, int ld, Place place) {
+                                                int ntaps, int ld, const WgradSum& sum, Place place) {
   __shared__ float part[8][32];
   const int kk = threadIdx.x & 31, lane = threadIdx.x >> 5, per_k = C * kH * kW, ktiles = (K + 31) / 32;
   const long long slab = 1LL * ntaps * K * ld;
+  bool nan = false;
   for (long long tl = blockIdx.x; tl < 1LL * per_k * ktiles; tl += gridDim.x) {
     const int e = static_cast<int>(tl % per_k), k = static_cast<int>(tl / per_k) * 32 + kk;
     const int wj = e % kW, wi = (e / kW) % kH, c = e / (kW * kH);
@@ -289,8 +291,24 @@ __device__ __forceinline__ void reduce_gathered(const float* __restrict__ partia
     if (lane == 0 && k < K) {
       for (int l = 1; l < 8; ++l) acc += part[l][kk];
       dw[1LL * k * per_k + e] = static_cast<T>(acc);
+      nan |= isnan(acc);
     }
     __syncthreads();
+  }
+  if (!__syncthreads_or(nan)) return;
+#pragma unroll 1
+  for (long long tl = blockIdx.x; tl < 1LL * per_k * ktiles; tl += gridDim.x) {
+    const int e = static_cast<int>(tl % per_k), k0 = static_cast<int>(tl / per_k) * 32, wj = e % kW, wi = e / kW % kH, c = e / kW / kH;
+    bool looked = false, suspect = false;                   // the border of the channel
+#pragma unroll 1
+    for (int k = k0 + lane; k < min(K, k0 + 32); k += 8) {
+      if (!isnan(static_cast<float>(dw[1LL * k * per_k + e]))) continue;
+      if (!looked) suspect = border_not_finite(sum, c);
+      looked = true;
+      if (!suspect) break;
+      const float v = exact_sum(sum, k, c, sum.flip ? kH - 1 - wi : wi, sum.flip ? kW - 1 - wj : wj);
+      if (kk == 0) dw[1LL * k * per_k + e] = static_cast<T>(v);
+    }
   }
 }
 
@@ -299,9 +317,9 @@ __device__ __forceinline__ void reduce_gathered(const float* __restrict__ partia
 template <typename T>
 __global__ void __launch_bounds__(256) wgrad_reduce_s2d_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits,
                                         int K, int C, int kH, int kW, int ntaps, int t0, int q0, int padH,
-                                        int padW, int ld, int flip) {
+                                        int padW, int ld, int flip, const __grid_constant__ WgradSum sum) {
   pdl_enter();
-  reduce_gathered(partial, dw, splits, K, C, kH, kW, ntaps, ld, [=](int c, int wi, int wj, int* t, int* col) {
+  reduce_gathered(partial, dw, splits, K, C, kH, kW, ntaps, ld, sum, [=](int c, int wi, int wj, int* t, int* col) {
     const int i = flip ? kH - 1 - wi : wi, jj = flip ? kW - 1 - wj : wj;
     const int ah = i - padH, aw = jj - padW;                 // offsets from 2 * the output position
     const int th = ah >= 0 ? ah / 2 : -((1 - ah) / 2), tw = aw >= 0 ? aw / 2 : -((1 - aw) / 2);   // floor
@@ -315,9 +333,9 @@ __global__ void __launch_bounds__(256) wgrad_reduce_s2d_kernel(const float* __re
 template <typename T>
 __global__ void __launch_bounds__(256) wgrad_reduce_fold_kernel(const float* __restrict__ partial, T* __restrict__ dw,
                                          int splits, int K, int C, int kH, int kW, int Cp, int ld,
-                                         int flip) {
+                                         int flip, const __grid_constant__ WgradSum sum) {
   pdl_enter();
-  reduce_gathered(partial, dw, splits, K, C, kH, kW, kH, ld, [=](int c, int wi, int wj, int* t, int* col) {
+  reduce_gathered(partial, dw, splits, K, C, kH, kW, kH, ld, sum, [=](int c, int wi, int wj, int* t, int* col) {
     *t = flip ? kH - 1 - wi : wi;
     *col = (flip ? kW - 1 - wj : wj) * Cp + c;
   });
@@ -665,15 +683,15 @@ static int gather_grid(int K, long long total) { return static_cast<int>(std::mi
 
 cudaError_t launch_wgrad_reduce_s2d(const float* partial, void* dw, int splits, int K, int C, int kH,
                                     int kW, int ntaps, int t0, int q0, int padH, int padW, int ld, int flip,
-                                    int dtype, cudaStream_t s) {
+                                    int dtype, const WgradSum& sum, cudaStream_t s) {
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
     launch_streaming(wgrad_reduce_s2d_kernel<__half>, gather_grid(K, total), 256, 0, s,
-        partial, static_cast<__half*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
+        partial, static_cast<__half*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip, sum);
   else
     launch_streaming(wgrad_reduce_s2d_kernel<float>, gather_grid(K, total), 256, 0, s,
-        partial, static_cast<float*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
+        partial, static_cast<float*>(dw), splits, K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip, sum);
   return cudaGetLastError();
 }
 
@@ -717,15 +735,15 @@ cudaError_t launch_pack_filters_s2d(const void* w, void* dst, int K, int C, int 
 }
 
 cudaError_t launch_wgrad_reduce_fold(const float* partial, void* dw, int splits, int K, int C, int kH,
-                                     int kW, int Cp, int ld, int flip, int dtype, cudaStream_t s) {
+                                     int kW, int Cp, int ld, int flip, int dtype, const WgradSum& sum, cudaStream_t s) {
   const long long total = 1LL * K * C * kH * kW;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
     launch_streaming(wgrad_reduce_fold_kernel<__half>, gather_grid(K, total), 256, 0, s,
-        partial, static_cast<__half*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
+        partial, static_cast<__half*>(dw), splits, K, C, kH, kW, Cp, ld, flip, sum);
   else
     launch_streaming(wgrad_reduce_fold_kernel<float>, gather_grid(K, total), 256, 0, s,
-        partial, static_cast<float*>(dw), splits, K, C, kH, kW, Cp, ld, flip);
+        partial, static_cast<float*>(dw), splits, K, C, kH, kW, Cp, ld, flip, sum);
   return cudaGetLastError();
 }
 

@@ -17,6 +17,7 @@
 // slice order (so the result does not depend on scheduling) and writes OIHW.
 #include "internal.h"
 #include "ptx.cuh"
+#include "wgrad_exact.cuh"
 #include "wgrad_slab.cuh"
 
 namespace b200 {
@@ -332,10 +333,11 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
 // The slabs are read once, from L2 or HBM; what bounds the kernel below a few megabytes is the length
 // of the chain of loads in a thread, so a block is one round of loads (up to 640 threads) and long sums are split over lanes.
 // diag_c / diag_k: only the diagonal blocks of merged groups are there and wanted (diag_c channels per filter, starting at the block of the
-// filter), 0: all.
+// filter), 0: all.  `sum`: for sums that are NaN (wgrad_exact.cuh).
 template <typename T>
 __global__ void __launch_bounds__(640, 2) wgrad_reduce_kernel(const float* __restrict__ partial, T* __restrict__ dw, int splits, int taps, int K,
-                                                               int Cg, int Kg, int diag_c, int diag_k, int log_k, int log_q, int log_lanes) {
+                                                               int Cg, int Kg, int diag_c, int diag_k, int log_k, int log_q, int log_lanes,
+                                                               const __grid_constant__ WgradSum sum) {
   pdl_enter();
   extern __shared__ float4 shared[];
   const int kt = 1 << log_k, nq = 1 << log_q, lanes = 1 << log_lanes;
@@ -374,6 +376,7 @@ __global__ void __launch_bounds__(640, 2) wgrad_reduce_kernel(const float* __res
     if (lane > 0) part[(lane - 1) * units + u] = acc;
   }
   if (lanes > 1) __syncthreads();
+  bool nan = false;
   if (lane == 0 && on) {
     for (int l = 0; l < lanes - 1; ++l) {
       const float4 v = part[l * units + u];
@@ -381,13 +384,22 @@ __global__ void __launch_bounds__(640, 2) wgrad_reduce_kernel(const float* __res
     }
     float* dst = tile + kk * pitch + 4 * q * taps + t;
     dst[0] = acc.x; dst[taps] = acc.y; dst[2 * taps] = acc.z; dst[3 * taps] = acc.w;
+    nan = isnan(acc.x) || isnan(acc.y) || isnan(acc.z) || isnan(acc.w);
   }
-  __syncthreads();
   const int run = min(4 * nq, cols - c0) * taps;
-  for (int row = threadIdx.x >> 5; row < kt && k0 + row < K; row += blockDim.x >> 5) {
-    T* dst = dw + (1LL * (k0 + row) * cols + c0) * taps;
-    for (int i = threadIdx.x & 31; i < run; i += 32) dst[i] = static_cast<T>(tile[row * pitch + i]);
-  }
+  auto store = [&] {
+#pragma unroll 1
+    for (int row = threadIdx.x >> 5; row < kt && k0 + row < K; row += blockDim.x >> 5) {
+      T* dst = dw + (1LL * (k0 + row) * cols + c0) * taps;
+      for (int i = threadIdx.x & 31; i < run; i += 32) dst[i] = static_cast<T>(tile[row * pitch + i]);
+    }
+  };
+  const bool any_nan = __syncthreads_or(nan);
+  store();
+  if (!any_nan) return;
+  __syncthreads();
+  exact_tile(sum, tile, min(kt, K - k0), pitch, min(4 * nq, cols - c0), k0, c0);
+  store();
 }
 
 template <MmaKind KIND, int BN>
@@ -423,7 +435,7 @@ cudaError_t launch_wgrad_umma(const UmmaWgradParams& p, int dtype, int bn_cols, 
 }
 
 cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int taps, int K, int Cg, int Kg, int diag_c, int diag_k,
-                                int dtype, cudaStream_t s) {
+                                int dtype, const WgradSum& sum, cudaStream_t s) {
   if (1LL * K * Cg == 0 || taps == 0) return cudaSuccess;
   const int cols = diag_c ? diag_c : Cg;
   // About four slabs per thread, at most 8 threads per sum; as many channels as make a filter's run 128 bytes; up to 32 filters
@@ -439,9 +451,9 @@ cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int 
   const int units = taps << (log_k + log_q), threads = ((units << log_lanes) + 31) / 32 * 32, g = static_cast<int>(blocks());
   const size_t smem = sizeof(float4) * ((1 << log_lanes) - 1) * units + (sizeof(float) * (((4 << log_q) * taps) | 1) << log_k);
   if (dtype == B200CONV_F16)
-    launch_streaming(wgrad_reduce_kernel<__half>, g, threads, smem, s, partial, static_cast<__half*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes);
+    launch_streaming(wgrad_reduce_kernel<__half>, g, threads, smem, s, partial, static_cast<__half*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes, sum);
   else
-    launch_streaming(wgrad_reduce_kernel<float>, g, threads, smem, s, partial, static_cast<float*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes);
+    launch_streaming(wgrad_reduce_kernel<float>, g, threads, smem, s, partial, static_cast<float*>(dw), splits, taps, K, Cg, Kg, diag_c, diag_k, log_k, log_q, log_lanes, sum);
   return cudaGetLastError();
 }
 
