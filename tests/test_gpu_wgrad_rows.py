@@ -92,6 +92,9 @@ def test_it_may_be_the_timed_choice(dtype):
     x, dy = (rs.randint(-1, 2, (2, 32, 28, 28)).astype(dtype) for _ in range(2))
     X, DY = (shim.DeviceTensor.from_host(ctx, a, "nhwc") for a in (x, dy))
     want = O.conv2d_grad_weights(x.astype(np.float32), dy.astype(np.float32), (3, 3), border_mode="half")
+    kernels = []
     for _ in range(2):
         assert np.array_equal(shim.device_grad_weights(X, DY, (3, 3), border_mode="half").to_host(), want.astype(dtype))
+        kernels.append(ctx.last_variant)
+    assert kernels[0] == kernels[1] and kernels[0].startswith("wgrad ")
     ctx.close()
