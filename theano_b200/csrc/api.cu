@@ -603,8 +603,8 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
       const long long tiles = cdiv(Wt, wt) * cdiv(Ht, th) * cdiv(a.N, nb);
       const long long total = (pair ? cdiv(tiles, 2) : tiles) * tiles_co * a.groups;
       // Clocks of the busiest SM: per tile and (tap, channel block) 4 MMAs per accumulator plus
-      // 120 clocks of stage hand-over in the issuing thread (190 were measured, see slab_tps; with either
-      // number 24 layers of 64 to 512 channels get tiles of the same speed); then the accumulators are read
+      // 120 clocks of stage hand-over in the issuing thread (slab_tps: 190 once, 50 to 90 since the issue is straight-line
+      // code; with 120 or 190 24 layers of 64 to 512 channels get tiles of the same speed); then the accumulators are read
       // out, beside the next tile's MMAs when two accumulator sets fit the 512 TMEM columns.
       // Epilogue: through staged TMA stores when the output is channels-last and the staging
       // buffers fit beside two slabs and two filter stages (about 2500 clocks of latency per tile
@@ -1026,8 +1026,8 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
 // leaves ms[i] at -1.  Returns an error of the timing itself.
 // Every variant runs twice, the second time between two events (the first loads its code and makes the choices inside
 // it); with one exception this decides: variants within a fifth (and the 4 us by which short launches differ between
-// events) of the best are timed again in bursts of up to 7 back to back, the way a program issues them, once, and
-// once more if they are still within 5 %.  Alone, a kernel of 5 us costs 5 us more and the chained launch hides nothing.
+// events) of the best are timed again in bursts of up to 7 back to back (8 did as well), the way a program issues them, once,
+// and once more if they are still within 5 %.  Alone, a kernel of 5 us costs 5 us more and the chained launch hides nothing.
 // All variants in two bursts each made the first passes of 32 cases take 200 ms together, this and rough_times() 127.
 template <class Run>
 int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool rough = false) {

@@ -9,8 +9,8 @@
 // row offset into one shared-memory x tile: per stage one dy tile and one x tile are fetched and
 // every tap of the group accumulates into its own 128 x 128 TMEM accumulator.  That divides the
 // number of TMA boxes per MMA.  (MN-major operands run at the same rate as K-major ones: 64 clocks per 128 x 128 MMA,
-// whatever the row offset.  Which of the two gradWeights kernels is faster depends on the layer, so the first call
-// of a geometry times both.)
+// whatever the row offset.  Which of the three gradWeights kernels is fastest depends on the layer, so the first call
+// of a geometry times those that apply.)
 //
 // Operands are MN-major (the pixel is the slow index of a channels-last row): float16 with the
 // 16-byte swizzle, tf32 with the 32-byte-atom swizzle; row offsets that are not multiples of the

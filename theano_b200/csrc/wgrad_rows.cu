@@ -17,7 +17,8 @@
 // pixel blocks, 256 images of 224 x 224, 311 -> 183 us, 50 of them the pass that makes the blocks.
 //
 // The positions p of a tile are th grid rows from row h0 on, h0 >= -halo (the copies reach back halo rows); dy rows above and below the
-// image and columns behind it arrive as zeros, so every product of a tap is counted in exactly one tile; th * P is a multiple of an
+// image and columns behind it arrive as zeros, so every product of a tap is counted in exactly one tile (pixels of x that are not finite meet
+// those zeros: wgrad_exact.cuh); th * P is a multiple of an
 // MMA's reduction steps.
 //
 // Work item = (channel tile, group, stride parity view, slice).  Warp roles: warp 0 loads dy, the last warp loads x, warp 1 issues the
