@@ -1264,8 +1264,9 @@ bool plain_pack(const b200conv_desc& d, int mode, int* ldc) {
 // ======================================================================================
 // the three directions on device pointers
 // ======================================================================================
+// merge > 1: `d` is a layer whose groups were merged that many at a time, `w` still the bank of its own groups.
 int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const void* w,
-               const void* bias, void* y, int flags) {
+               const void* bias, void* y, int flags, int merge = 1) {
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;
   const size_t es = elem_size(d.dtype);
   const bool out_nhwc = flags & B200CONV_OUT_NHWC, in_nhwc = flags & B200CONV_IN_NHWC;
@@ -1279,7 +1280,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   }
   b200conv_desc flat;
   if (!(flags & B200CONV_FORCE_DIRECT) && !c->epi.pool && flatten_1x1(d, in_nhwc && out_nhwc, &flat))
-    return fwd_device(c, flat, x, w, bias, y, flags);
+    return fwd_device(c, flat, x, w, bias, y, flags, merge);
   Scratch tmp(c);
   // the direct kernels take the bias as float32; the tensor-core kernels read it in the data type
   const float* bias_f = d.dtype == B200CONV_F32 ? static_cast<const float*>(bias) : nullptr;
@@ -1299,10 +1300,13 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     KLAUNCH(c, kKPack, launch_pad_bias(bias, padded, d.K, Kp, d.dtype, c->stream));
     bias = padded;
   }
-  const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor(d);
+  const int mg = (flags & B200CONV_FORCE_DIRECT) || merge > 1 ? 1 : merge_factor(d);
   if (mg > 1) {
     b200conv_desc dm = d;
     dm.groups = d.groups / mg;
+    int a, b, e;
+    const bool stem = fold_ok(dm) || (!(flags & B200CONV_NO_S2D) && s2d_ok(dm, &a, &b, &e));     // those pack another form
+    if (umma_ok(dm) && !stem) return fwd_device(c, dm, x, w, bias, y, flags | kScratchFilters, mg);
     if (umma_ok(dm)) {
       void* wm;
       int rc = tmp.get(es * (size_t)d.K * Cg * mg * d.kH * d.kW, &wm);
@@ -1411,7 +1415,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
   const int ldw = pad_channels(Cg, d.dtype);
   void* wp;
   int rc = 0;
-  if (d.kH == 1 && d.kW == 1 && ldw == Cg && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
+  if (d.kH == 1 && d.kW == 1 && ldw == Cg && merge == 1 && reinterpret_cast<uintptr_t>(w) % 16 == 0) {
     // a 1x1 filter bank [K][C] already is its packed form (rows = filters, channels contiguous)
     wp = const_cast<void*>(w);
   } else {
@@ -1419,7 +1423,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
     if (!wp) {
       rc = tmp.get(es * (size_t)d.kH * d.kW * d.K * ldw, &wp);
       if (rc) return rc;
-      KLAUNCH(c, kKPack, launch_pack_filters(w, wp, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 0, ldw, d.dtype, c->stream));
+      KLAUNCH(c, kKPack, launch_pack_filters(pack_job(w, wp, d.K, Cg, d.kH * d.kW, d.groups, d.flip, 0, ldw, merge), d.dtype, c->stream));
     }
   }
 
@@ -1465,7 +1469,7 @@ int fwd_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const voi
 }
 
 int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const void* dy, void* dx,
-                 int flags) {
+                 int flags, int merge = 1) {
   const int Cg = d.C / d.groups, Kg = d.K / d.groups;
   const size_t es = elem_size(d.dtype);
   const bool out_nhwc = flags & B200CONV_OUT_NHWC, in_nhwc = flags & B200CONV_IN_NHWC;
@@ -1473,12 +1477,14 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
   if (d.N == 0 || d.C == 0) return 0;
   b200conv_desc flat;
   if (!(flags & B200CONV_FORCE_DIRECT) && flatten_1x1(d, in_nhwc && out_nhwc, &flat))
-    return dgrad_device(c, flat, w, dy, dx, flags);
+    return dgrad_device(c, flat, w, dy, dx, flags, merge);
   const size_t dx_bytes = es * (size_t)d.N * d.H * d.W * (out_nhwc ? Cp : d.C);
-  const int mg = (flags & B200CONV_FORCE_DIRECT) ? 1 : merge_factor(d);
+  const int mg = (flags & B200CONV_FORCE_DIRECT) || merge > 1 ? 1 : merge_factor(d);
   if (mg > 1) {
     b200conv_desc dm = d;
     dm.groups = d.groups / mg;
+    const bool classes = d.sH * d.sW > 1 && dm.groups == 1 && d.sH * d.sW * d.C <= 64;            // those pack another form
+    if (umma_ok(dm) && !classes) return dgrad_device(c, dm, w, dy, dx, flags | kScratchFilters, mg);
     if (umma_ok(dm)) {
       Scratch tm(c);
       void* wm;
@@ -1583,7 +1589,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
   void* wp = flags & kScratchFilters ? nullptr : packed_lookup(c, w, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 1, ldw, d.dtype);
   if (!wp) {
     if ((rc = tmp.get(es * (size_t)d.kH * d.kW * d.C * ldw, &wp))) return rc;
-    KLAUNCH(c, kKPack, launch_pack_filters(w, wp, d.K, Cg, d.kH, d.kW, d.groups, d.flip, 1, ldw, d.dtype, c->stream));
+    KLAUNCH(c, kKPack, launch_pack_filters(pack_job(w, wp, d.K, Cg, d.kH * d.kW, d.groups, d.flip, 1, ldw, merge), d.dtype, c->stream));
   }
   if (need_zero) CU_OK(c, cudaMemsetAsync(dx, 0, dx_bytes, c->stream));
   FwdLikeArgs a;
@@ -3322,7 +3328,7 @@ int b200conv_prepack(b200conv_ctx* c, int count, const b200conv_desc* descs, con
     if (!filters[i] || d.N == 0 || d.C == 0 || d.K == 0) continue;
     b200conv_desc flat;
     if (flatten_1x1(d, true, &flat)) d = flat;         // the geometry the channels-last calls will see
-    const int Cg = d.C / d.groups, Kg = d.K / d.groups;
+    const int Cg = d.C / d.groups;
     for (int mode = 0; mode < 2; ++mode) {
       int ldc = 0;
       if (!(directions & (1 << mode)) || !plain_pack(d, mode, &ldc)) continue;
@@ -3338,12 +3344,9 @@ int b200conv_prepack(b200conv_ctx* c, int count, const b200conv_desc* descs, con
       const int t = d.dtype == B200CONV_F16 ? 1 : 0;
       if (batch[t].njobs == kPackBatchJobs && (rc = flush(t))) return rc;
       PackJob& j = batch[t].jobs[batch[t].njobs++];
-      int gz = 1;
-      j.src = filters[i]; j.dst = it->second.ptr;
-      j.K = d.K; j.Cg = Cg; j.kH = d.kH; j.kW = d.kW; j.groups = d.groups; j.flip = d.flip; j.mode = mode; j.ldc = ldc;
-      pack_filters_grid(Kg, Cg, d.groups, mode, ldc, d.kH * d.kW, &j.gx, &j.gy, &gz);
+      j = pack_job(filters[i], it->second.ptr, d.K, Cg, d.kH * d.kW, d.groups, d.flip, mode, ldc);
       j.first_block = nblocks[t];
-      nblocks[t] += j.gx * j.gy * gz;
+      nblocks[t] += plan_pack(&j, d.dtype, kPackBlocks / std::max(1, count));
       it->second.valid = true;
     }
   }

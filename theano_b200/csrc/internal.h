@@ -379,25 +379,34 @@ cudaError_t launch_depth_to_space(const void* tmp, void* dx, int N, int C, int H
 // in[b][r][s] (row length ld_in) -> out[b][s][r] (row length ld_out, zero filled past R).
 cudaError_t launch_transpose(const void* in, void* out, int B, int R, int S, int ld_in,
                              int ld_out, int dtype, cudaStream_t s);
-// Filter packing; mode 0: forward (rows = filters, cols = channels),
-// mode 1: input gradient (rows = channels, cols = filters).  dst[(tap*groups+g)][rows][ldc].
-cudaError_t launch_pack_filters(const void* w, void* dst, int K, int Cg, int kH, int kW,
-                                int groups, int flip, int mode, int ldc, int dtype,
-                                cudaStream_t s);
-// Many filter banks packed by one launch (b200conv_prepack): the grid of job j is gx * gy * gz
-// blocks of launch_pack_filters' own grid, starting at block first_block.
+// Filter packing; mode 0: forward (rows = filters, cols = channels), mode 1: input gradient (rows = channels, cols = filters).
+// dst[(tap*groups+g)][rows][ldc].  Cg: channels per (merged) group; merge: how many of the bank's own groups make one.
 struct PackJob {
   const void* src;
   void* dst;
-  int K, Cg, kH, kW, groups, flip, mode, ldc;
-  int gx, gy, first_block;
+  int K, Cg, groups, ldc;
+  int gx, gy, first_block;             // blocks along channels and filters, first one in a batch
+  uint16_t taps, merge, pieces;        // pieces: 16 bytes each, of a filter's run in a patch
+  uint8_t flip, mode, log_k, log_c;    // filters and channels of a patch
 };
+inline PackJob pack_job(const void* w, void* dst, int K, int Cg, int taps, int groups, int flip, int mode, int ldc, int merge = 1) {
+  PackJob q = {};
+  q.src = w; q.dst = dst;
+  q.K = K; q.Cg = Cg; q.groups = groups; q.ldc = ldc;
+  q.taps = static_cast<uint16_t>(taps); q.merge = static_cast<uint16_t>(merge);
+  q.flip = flip != 0; q.mode = static_cast<uint8_t>(mode);
+  return q;
+}
+cudaError_t launch_pack_filters(PackJob q, int dtype, cudaStream_t s);
+// Many filter banks packed by one launch (b200conv_prepack): plan_pack() gives the blocks that a job takes.
 constexpr int kPackBatchJobs = 56;             // 56 x 64 bytes stay below the 4 KB kernel-parameter limit
 struct PackBatch {
   PackJob jobs[kPackBatchJobs];
   int njobs;
 };
-void pack_filters_grid(int Kg, int Cg, int groups, int mode, int ldc, int taps, int* gx, int* gy, int* gz);
+static_assert(sizeof(PackBatch) <= 4096, "kernel parameters");
+constexpr int kPackBlocks = 2 * 148;           // blocks of a launch that are worth smaller patches
+int plan_pack(PackJob* q, int dtype, int least);
 cudaError_t launch_pack_filters_batch(const PackBatch& b, int total_blocks, int dtype, cudaStream_t s);
 // Row folding for layers with very few input channels (see layout.cu).
 cudaError_t launch_pad_fold(const void* src, void* dst, int N, int C, int H, int W, int Cp, int Wp,

@@ -35,96 +35,119 @@ __global__ void transpose_kernel(const T* __restrict__ in, T* __restrict__ out, 
 //   mode 0 (forward):        rows = filters of the group, cols = channels,
 //                            tap t = i*kW + j multiplies the pixel at offset (i, j);
 //   mode 1 (input gradient): rows = channels, cols = filters of the group.
-// With flip the correlation tap t reads position taps - 1 - t of the filter.
-// A block moves a patch of filters x channels with all its taps through shared memory: the taps of
-// a filter's consecutive channels are one contiguous run of OIHW, the write runs along 32 columns
-// of the destination.  What bounds a small bank is the chain of loads in a block and the number of
-// blocks, so the patch is cut to about kPackPatch elements whatever the tap count (a warp loads a
-// filter's run without any division, all loads of a thread in flight), and rows of the patch go
-// to warps tap by tap.  Measured: 50 x 20 x 5x5 float32 25 -> 3 us, 64 x 64 x 3x3 float16 4.5 -> 3 us.
-constexpr int kPackPatch = 2560;
-constexpr int kPackSmem = kPackPatch + 64;
-// filters (mode 0) or channels (mode 1) of a patch beside the 32 along the destination's columns
-__host__ __device__ inline int pack_rows(int taps) {
-  const int r = kPackPatch / (32 * taps);
-  return r < 1 ? 1 : r > 8 ? 8 : r;
-}
+// With flip the correlation tap t reads position taps - 1 - t of the filter.  With `merge` neighbouring groups as one, the
+// bank is that of the layer's own groups and the packed form block-diagonal: a filter has channels of its own group only.
+// A block moves a patch of filters x channels with all its taps through shared memory: the taps of a filter's consecutive
+// channels are one run of OIHW, read in 16-byte pieces (elements at the ends of a run that lies off the 16-byte
+// boundaries), and leave as 16-byte pieces of the destination's rows.  Every call on its own filters waits for this kernel, and
+// what bounds it is latency: one round of loads (up to four pieces per thread) and one of stores.  Element by element it took
+// 10 rounds of each.  Forward / gradInputs calls with the packing (a B200, before -> now): 64 -> 64 3x3 at 28x28, 8 images, float16 9.6 -> 9.1 /
+// 11.9 -> 9.6 us; 100 -> 75 5x5, 37 images, float16 37.5 -> 28.5 / 35.4 -> 27.4; 256 -> 256 3x3 at 14x14, 128 images, float32 60.5 -> 56 / 66 -> 59.
+// All banks of ResNet-50 in one launch (float16, both forms, 47 MB) 138 -> 65 us, of the VGG-16 stack (float32, 49 MB) 102 -> 80.
+constexpr int kPackThreads = 256, kPackPieces = 4, kPackMaxK = 64;
 template <typename T>
-__device__ __forceinline__ void pack_filters_block(const T* __restrict__ w, T* __restrict__ dst, int K, int Cg,
-                                                   int taps, int groups, int flip, int mode, int ldc,
-                                                   int bx, int by, int g) {
-  __shared__ T tile[kPackSmem];
-  const int pr = pack_rows(taps);
-  const int PK = mode == 0 ? pr : 32, PC = mode == 0 ? 32 : pr;
-  const int Kg = K / groups, k0 = by * PK, c0 = bx * PC;
-  const int lane = threadIdx.x, wp = threadIdx.y;
-  const int nk = min(PK, Kg - k0), nc = min(PC, Cg - c0);      // <= 0 in patches that only pad
-  const int run = nc * taps, pitch = (PC * taps) | 1;
-  for (int kk = wp; kk < nk; kk += 8) {
-    const T* src = w + (1LL * (g * Kg + k0 + kk) * Cg + c0) * taps;
-#pragma unroll 8
-    for (int i = lane; i < run; i += 32) tile[kk * pitch + i] = src[i];
-  }
-  __syncthreads();
-  const int rows = mode == 0 ? Kg : Cg, nrow = mode == 0 ? nk : nc;
-  const int col = (mode == 0 ? c0 : k0) + lane, row0 = mode == 0 ? k0 : c0;
-  const bool real = lane < (mode == 0 ? nc : nk);
-  if (col >= ldc) return;
-  for (int rr = wp % pr, t = wp / pr; t < taps;) {             // warp unit u = t * pr + rr, u += 8
-    if (rr < nrow) {
-      const int tap = flip ? taps - 1 - t : t;
-      const T v = real ? (mode == 0 ? tile[rr * pitch + lane * taps + t] : tile[lane * pitch + rr * taps + t]) : T(0);
-      dst[(1LL * (tap * groups + g) * rows + row0 + rr) * ldc + col] = v;
+__device__ __forceinline__ void pack_filters_block(const PackJob& q, int bx, int by, int g) {
+  extern __shared__ uint4 pack_smem[];
+  __shared__ int4 row_of[kPackMaxK];            // per filter of the patch: shared-memory offset of (channel c0, tap 0), its channels [y, z)
+  uint8_t* tile = reinterpret_cast<uint8_t*>(pack_smem);
+  constexpr int V = 16 / static_cast<int>(sizeof(T));
+  const int taps = q.taps, Kg = q.K / q.groups, Cs = q.Cg / q.merge, Ks = Kg / q.merge;
+  const int k0 = by << q.log_k, c0 = bx << q.log_c, c_end = min(c0 + (1 << q.log_c), q.Cg), pitch = q.pieces * 16;
+  const int nk = min(1 << q.log_k, Kg - k0);                   // <= 0 in patches that only pad
+  const T* w = static_cast<const T*>(q.src);
+  // channels of filter k0 + kk in this patch, and where they start
+  auto run_of = [&](int kk, int* a, int* b) {
+    const int k = k0 + kk, lo = q.merge > 1 ? k / Ks * Cs : 0;
+    *a = max(c0, lo);
+    *b = max(*a, min(c_end, lo + Cs));
+    return w + ((1LL * g * Kg + k) * Cs + *a - lo) * taps;
+  };
+  if (threadIdx.x < (1 << q.log_k)) {
+    int a = 0, b = 0, at = 0;
+    if (static_cast<int>(threadIdx.x) < nk) {
+      const T* run = run_of(threadIdx.x, &a, &b);
+      at = threadIdx.x * pitch + threadIdx.x / V * 16 + static_cast<int>(reinterpret_cast<uintptr_t>(run) & 15) - (a - c0) * taps * static_cast<int>(sizeof(T));
     }
-    rr += 8;
-    while (rr >= pr) { rr -= pr; ++t; }
+    row_of[threadIdx.x] = make_int4(at, a, b, 0);
   }
-}
-
-// 1x1 banks for gradInputs are plain transposes [K][C] -> [C][ldc]: 64 x 64 tiles through shared memory, read
-// along c and written along k in 128-byte runs (the general patch kernel moves 16-byte runs here).
-template <typename T>
-__device__ __forceinline__ void transpose_1x1_block(const T* __restrict__ w, T* __restrict__ dst, int K, int Cg, int groups,
-                                                    int ldc, int bx, int by, int bz) {
-  __shared__ T tile[64][65];
-  const int Kg = K / groups;
-  const int k0 = bx * 64, c0 = by * 64, g = bz;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  for (int i = tid; i < 64 * 64; i += 256) {
-    const int kk = i >> 6, cc = i & 63;
-    T v = T(0);
-    if (k0 + kk < Kg && c0 + cc < Cg) v = w[(1LL * (g * Kg + k0 + kk)) * Cg + c0 + cc];
-    tile[kk][cc] = v;
+  for (int base = 0; base < nk * q.pieces; base += kPackThreads * kPackPieces) {
+    uint4 v[kPackPieces];
+    uintptr_t from[kPackPieces], lo[kPackPieces], hi[kPackPieces];    // of the piece, of its run
+    int to[kPackPieces];
+#pragma unroll
+    for (int u = 0; u < kPackPieces; ++u) {
+      const int i = base + u * kPackThreads + threadIdx.x, kk = i / q.pieces;
+      to[u] = (i + kk / V) * 16;
+      from[u] = lo[u] = hi[u] = 0;
+      if (kk >= nk) continue;
+      int a, b;
+      const T* run = run_of(kk, &a, &b);
+      lo[u] = reinterpret_cast<uintptr_t>(run);
+      hi[u] = reinterpret_cast<uintptr_t>(run + (b - a) * taps);
+      from[u] = (lo[u] & ~static_cast<uintptr_t>(15)) + (i - kk * q.pieces) * 16;
+      if (from[u] >= lo[u] && from[u] + 16 <= hi[u]) v[u] = *reinterpret_cast<const uint4*>(from[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kPackPieces; ++u) {
+      if (from[u] >= hi[u]) continue;
+      if (from[u] >= lo[u] && from[u] + 16 <= hi[u]) {
+        *reinterpret_cast<uint4*>(tile + to[u]) = v[u];
+        continue;
+      }
+      for (int e = 0; e < 16; e += sizeof(T))
+        if (from[u] + e >= lo[u] && from[u] + e < hi[u]) *reinterpret_cast<T*>(tile + to[u] + e) = *reinterpret_cast<const T*>(from[u] + e);
+    }
   }
   __syncthreads();
-  T* d = dst + 1LL * g * Cg * ldc;
-  for (int i = tid; i < 64 * 64; i += 256) {
-    const int cc = i >> 6, kk = i & 63;
-    if (c0 + cc < Cg && k0 + kk < ldc) d[1LL * (c0 + cc) * ldc + k0 + kk] = tile[kk][cc];
+  const int rows = q.mode == 0 ? Kg : q.Cg, log_rows = q.mode == 0 ? q.log_k : q.log_c;
+  const int log_v = (q.mode == 0 ? q.log_c : q.log_k) - (V == 8 ? 3 : 2), row0 = q.mode == 0 ? k0 : c0, col0 = q.mode == 0 ? c0 : k0;
+  T* dst = static_cast<T*>(q.dst) + 1LL * g * rows * q.ldc;
+  // whole patches of rows that start alike: no look-ups, neighbouring elements of a piece a constant apart
+  const bool whole = q.merge == 1 && nk == 1 << q.log_k && c0 + (1 << q.log_c) <= q.Cg && (Cs * taps * sizeof(T)) % 16 == 0;
+  const int first = row_of[0].x, apart = q.mode == 0 ? taps * static_cast<int>(sizeof(T)) : pitch;
+  for (int o = threadIdx.x; o < taps << (log_rows + log_v); o += kPackThreads) {
+    const int col = col0 + (o & ((1 << log_v) - 1)) * V, r = (o >> log_v) & ((1 << log_rows) - 1), t = o >> (log_rows + log_v);
+    if (col >= q.ldc || row0 + r >= rows) continue;
+    __align__(16) T v[V];
+    if (whole) {
+      const int k = q.mode == 0 ? r : col - k0, c = q.mode == 0 ? col - c0 : r;
+      const uint8_t* at = tile + first + k * pitch + k / V * 16 + (c * taps + t) * static_cast<int>(sizeof(T));
+#pragma unroll
+      for (int e = 0; e < V; ++e) v[e] = *reinterpret_cast<const T*>(at + e * apart);
+    } else
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const int c = q.mode == 0 ? col + e : c0 + r;
+      const int4 f = row_of[q.mode == 0 ? r : col + e - k0];
+      v[e] = c >= f.y && c < f.z ? *reinterpret_cast<const T*>(tile + f.x + ((c - c0) * taps + t) * static_cast<int>(sizeof(T))) : T(0);
+    }
+    const int tap = q.flip ? taps - 1 - t : t;
+    *reinterpret_cast<uint4*>(dst + (1LL * tap * q.groups * rows + row0 + r) * q.ldc + col) = *reinterpret_cast<const uint4*>(v);
   }
 }
 
 template <typename T>
 __device__ __forceinline__ void pack_job_block(const PackJob& q, int local) {
   const int bx = local % q.gx, by = local / q.gx % q.gy, bz = local / q.gx / q.gy;
-  const T* src = static_cast<const T*>(q.src);
-  T* dst = static_cast<T*>(q.dst);
-  if (q.kH * q.kW == 1 && q.mode == 1) transpose_1x1_block<T>(src, dst, q.K, q.Cg, q.groups, q.ldc, bx, by, bz);
-  else pack_filters_block<T>(src, dst, q.K, q.Cg, q.kH * q.kW, q.groups, q.flip, q.mode, q.ldc, bx, by, bz);
+  pack_filters_block<T>(q, bx, by, bz);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ PackJob q) {
+__global__ void __launch_bounds__(kPackThreads) pack_filters_kernel(const __grid_constant__ PackJob q) {
   pdl_enter();
   pack_job_block<T>(q, blockIdx.x);
 }
 
 // Many filter banks in one launch: block b belongs to the job j with first_block[j] <= b < first_block[j + 1].
 template <typename T>
-__global__ void __launch_bounds__(256) pack_filters_batch_kernel(const __grid_constant__ PackBatch b) {
+__global__ void __launch_bounds__(kPackThreads) pack_filters_batch_kernel(const __grid_constant__ PackBatch b) {
   pdl_enter();
-  int j = 0;
-  while (j + 1 < b.njobs && static_cast<int>(blockIdx.x) >= b.jobs[j + 1].first_block) ++j;
+  int j = 0, end = b.njobs;
+  while (j + 1 < end) {
+    const int mid = (j + end) >> 1;
+    if (static_cast<int>(blockIdx.x) >= b.jobs[mid].first_block) j = mid;
+    else end = mid;
+  }
   pack_job_block<T>(b.jobs[j], blockIdx.x - b.jobs[j].first_block);
 }
 
@@ -611,40 +634,43 @@ cudaError_t launch_transpose(const void* in, void* out, int B, int R, int S, int
   return cudaGetLastError();
 }
 
-void pack_filters_grid(int Kg, int Cg, int groups, int mode, int ldc, int taps, int* gx, int* gy, int* gz) {
-  if (taps == 1 && mode == 1) {            // the batched kernel's transposing path: 64 x 64 tiles
-    *gx = (ldc + 63) / 64;
-    *gy = (Cg + 63) / 64;
-    *gz = groups;
-    return;
-  }
-  // the patch grid covers the padded column range [0, ldc) of the destination as well
-  const int cols_c = mode == 0 ? ldc : Cg, cols_k = mode == 0 ? Kg : ldc;
-  const int PK = mode == 0 ? pack_rows(taps) : 32, PC = mode == 0 ? 32 : pack_rows(taps);
-  *gx = (cols_c + PC - 1) / PC;
-  *gy = (cols_k + PK - 1) / PK;
-  *gz = groups;
+// Patch of a block: 64 (float16, up to 16 taps) or 32 columns of the destination and as many of its rows as make four pieces per thread,
+// fewer while that makes fewer than `least` blocks: then rows down to runs of 64 bytes, at last columns down to 32 bytes.
+int plan_pack(PackJob* q, int dtype, int least) {
+  const int es = static_cast<int>(elem_size(dtype)), V = 16 / es, Kg = q->K / q->groups;
+  const int cols = q->ldc, rows = q->mode == 0 ? Kg : q->Cg;
+  int log_cols = es == 2 && q->taps <= 16 ? 6 : 5, log_rows = 0;
+  while ((1 << (log_cols - 1)) >= cols && (1 << (log_cols - 1)) >= V) --log_cols;
+  while (log_rows < 6 && (1 << log_rows) < rows && (q->taps * es << (log_cols + log_rows + 1)) <= kPackThreads * kPackPieces * 16) ++log_rows;
+  auto blocks = [&] { return cdiv(cols, 1 << log_cols) * cdiv(rows, 1 << log_rows) * q->groups; };
+  while (log_rows > 0 && blocks() < least && (q->mode == 0 || (q->taps * es << log_rows) > 64)) --log_rows;
+  while ((es << log_cols) > 32 && 2 * blocks() < least) --log_cols;
+  q->log_k = static_cast<uint8_t>(q->mode == 0 ? log_rows : log_cols);
+  q->log_c = static_cast<uint8_t>(q->mode == 0 ? log_cols : log_rows);
+  q->gx = static_cast<int>(cdiv(q->mode == 0 ? cols : rows, 1 << q->log_c));
+  q->gy = static_cast<int>(cdiv(q->mode == 0 ? rows : cols, 1 << q->log_k));
+  // a run that starts off a 16-byte boundary touches one piece more; an odd count, and a piece more every 16 bytes of filters: what a
+  // warp gathers for 16-byte pieces of several rows lies in different banks
+  q->pieces = static_cast<uint16_t>((((q->taps * es << q->log_c) + 15) / 16 + 1) | 1);
+  return q->gx * q->gy * q->groups;
 }
+static size_t pack_smem_bytes(const PackJob& q) { return (static_cast<size_t>(q.pieces * 16) << q.log_k) + (16 << q.log_k) / 4; }
 
 cudaError_t launch_pack_filters_batch(const PackBatch& b, int total_blocks, int dtype, cudaStream_t s) {
   if (b.njobs == 0 || total_blocks == 0) return cudaSuccess;
-  if (dtype == B200CONV_F16) launch_chained(pack_filters_batch_kernel<__half>, total_blocks, dim3(32, 8), 0, s, b);
-  else launch_chained(pack_filters_batch_kernel<float>, total_blocks, dim3(32, 8), 0, s, b);
+  size_t smem = 0;
+  for (int j = 0; j < b.njobs; ++j) smem = std::max(smem, pack_smem_bytes(b.jobs[j]));
+  if (dtype == B200CONV_F16) launch_chained(pack_filters_batch_kernel<__half>, total_blocks, kPackThreads, smem, s, b);
+  else launch_chained(pack_filters_batch_kernel<float>, total_blocks, kPackThreads, smem, s, b);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pack_filters(const void* w, void* dst, int K, int Cg, int kH, int kW,
-                                int groups, int flip, int mode, int ldc, int dtype,
-                                cudaStream_t s) {
-  if (1LL * kH * kW * K * Cg == 0) return cudaSuccess;
-  PackJob q;
-  int gz;
-  q.src = w; q.dst = dst;
-  q.K = K; q.Cg = Cg; q.kH = kH; q.kW = kW; q.groups = groups; q.flip = flip; q.mode = mode; q.ldc = ldc;
-  pack_filters_grid(K / groups, Cg, groups, mode, ldc, kH * kW, &q.gx, &q.gy, &gz);
+cudaError_t launch_pack_filters(PackJob q, int dtype, cudaStream_t s) {
+  if (1LL * q.taps * q.K * q.Cg == 0) return cudaSuccess;
+  const int blocks = plan_pack(&q, dtype, kPackBlocks);
   q.first_block = 0;
-  if (dtype == B200CONV_F16) launch_chained(pack_filters_kernel<__half>, q.gx * q.gy * gz, dim3(32, 8), 0, s, q);
-  else launch_chained(pack_filters_kernel<float>, q.gx * q.gy * gz, dim3(32, 8), 0, s, q);
+  if (dtype == B200CONV_F16) launch_chained(pack_filters_kernel<__half>, blocks, kPackThreads, pack_smem_bytes(q), s, q);
+  else launch_chained(pack_filters_kernel<float>, blocks, kPackThreads, pack_smem_bytes(q), s, q);
   return cudaGetLastError();
 }
 
