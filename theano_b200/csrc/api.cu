@@ -547,9 +547,10 @@ enum SlabMode { kSlabWide = 0, kSlabSpread, kSlabPair };      // of the slab ker
 
 SlabMode slab_mode(int variant) { return variant == kConvSlabSpread ? kSlabSpread : variant == kConvSlabPair ? kSlabPair : kSlabWide; }
 
-// Clocks of four MMAs over 128 rows x bn columns x 32 bytes of the reduction, one after the other: half the
-// columns up to 128 (N = 64 and 32 are bound by their operands' shared-memory reads).
-int mma_clocks(int bn) { return bn >= 256 ? 128 : bn == 128 ? 64 : bn == 64 ? 48 : 40; }
+// Clocks of an MMA over 128 rows x bn columns x 32 bytes of the reduction: half of the columns, and no less than its operands' reads of
+// shared memory, 128 bytes a clock, take.  (MMAs of a tile with fewer filters are narrower, mma_columns(); the searches compare
+// tiles as if they were full.)
+int mma_clocks(int bn) { return std::max(bn / 2, 32 + bn / 4); }
 
 // Clocks that splitting the reduction of `items` = tiles x slices work items of rows x bn accumulators adds:
 // raw accumulators leave at 32 B/clk per SM, and the reduction kernel costs about 4500 clocks of launch and

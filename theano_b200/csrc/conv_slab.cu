@@ -101,6 +101,13 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
   uint32_t slab_seen = 0, b_seen = 0, acc_seen = 0;  // the next slab / filter stage / accumulator already seen ready (mbar_look)
   for (uint32_t item = w.first; item < w.total; item += w.stride, ++it) {
     const Range r = slice_range(p, item % static_cast<uint32_t>(p.splits));
+    // a constant where the tiles are full, and for 32 columns, whose MMAs take 36 to 40 clocks whatever is left out of them: with a
+    // descriptor from a register these took 4 % longer
+    uint32_t idesc = kIdesc;
+    if (BN > 32 && p.n_out % BN) {
+      const int co_t = p.tiles_co == 1 ? 0 : item / static_cast<uint32_t>(p.splits) % static_cast<uint32_t>(p.tiles_co);
+      idesc = with_columns(kIdesc, mma_columns(p.n_out, co_t * BN, BN, PAIR));
+    }
     // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
     // runs beside the MMAs of the next one
     const int buf = w.dbl ? (it & 1) : 0;
@@ -130,8 +137,8 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
         auto mma = [&](int q, uint32_t tap, int a, int kk) {
           const uint32_t a_lo = slab_lo + slab_tap_shift(tap) + a * (16384 >> 4);
           const uint32_t acc = acc0 + slab_tap_column(tap) + a * acc_step, b_lo = ring_lo + ((q * kBBytes) >> 4), adds = kk ? 1u : (q ? rest : more) | slab_tap_adds(tap);
-          if (kTogether) umma_words_if<KIND, PAIR>(leader, acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, adds);
-          else umma_words<KIND, PAIR>(acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, kIdesc, adds);
+          if (kTogether) umma_words_if<KIND, PAIR>(leader, acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, idesc, adds);
+          else umma_words<KIND, PAIR>(acc, a_lo + 2 * kk, b_lo + 2 * kk, desc_hi, idesc, adds);
         };
         // a stage's MMAs from u0 to u1, numbered (tap, accumulator, 32 bytes of the channels)
         auto part = [&](int u0, int u1) {
@@ -302,7 +309,8 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const Range r = slice_range(p, item - t * splits);
       const int co_t = t % static_cast<uint32_t>(p.tiles_co);
       const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const int row0 = co_t * BN + static_cast<int>(rank) * (BN / 2);     // a pair's CTAs load one half each
+      // a pair's CTAs load one half each of what the tile's MMAs take (and rows that those leave out)
+      const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_out, co_t * BN, BN, true) / 2);
       auto load = [&](uint8_t* dst, int kb, int mat) {
         if (PAIR) tma_load_4d_pair(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);
         else tma_load_4d(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);

@@ -172,6 +172,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem + buf * BN;
+      uint32_t idesc = kIdesc;
+      if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, p.tiles_co == 1 ? 0 : item / splits % static_cast<uint32_t>(p.tiles_co) * BN, BN, false));
       for (uint32_t k = k0; k < k1; ++k) {
         if (!wait_seen(seen, &bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
@@ -180,8 +182,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         const uint32_t a_lo = lo_base + stage * (stage_bytes<BN>() >> 4);
         const uint32_t b_lo = a_lo + (kABytes >> 4);
         if (leader) {
-          umma_words<KIND>(d_tmem, a_lo, b_lo, desc_hi, kIdesc, k != k0);
-          umma_words<KIND>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, kIdesc, 1u);
+          umma_words<KIND>(d_tmem, a_lo, b_lo, desc_hi, idesc, k != k0);
+          umma_words<KIND>(d_tmem, a_lo + 2, b_lo + 2, desc_hi, idesc, 1u);
         }
         __syncwarp();
         const int cur = stage;
@@ -189,8 +191,8 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
         seen = mbar_look(&bars->full[stage], phase);
         if (k + 1 == k1) acc_seen = mbar_look(&bars->acc_empty[(it + 1) & 1], (((it + 1) >> 1) & 1) ^ 1);
         if (leader) {
-          umma_words<KIND>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, kIdesc, 1u);
-          umma_words<KIND>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, kIdesc, 1u);
+          umma_words<KIND>(d_tmem, a_lo + 4, b_lo + 4, desc_hi, idesc, 1u);
+          umma_words<KIND>(d_tmem, a_lo + 6, b_lo + 6, desc_hi, idesc, 1u);
           umma_commit(&bars->empty[cur]);
         }
       }

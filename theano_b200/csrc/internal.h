@@ -131,6 +131,16 @@ struct alignas(64) UmmaConvParams {
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
 };
 
+// Columns of the MMAs of a tile that starts at output channel `first` of n_out: an MMA takes clocks by its columns, and a layer of
+// 75 filters need not pay for the 128 that its accumulator has room for.  Multiples of 16, on pairs of CTAs of 32.  (37 images of 27 x 33,
+// 5x5, float16: 100 -> 75 filters on pairs 28.5 -> 26.0 us, 75 -> 100 on single CTAs 27.3 -> 26.6.)
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int mma_columns(int n_out, int first, int bn, bool pair) {
+  const int step = pair ? 32 : 16, n = (n_out - first + step - 1) / step * step;
+  return n < bn ? n : bn;
+}
 int conv_umma_bn(int n_out);      // accumulator columns that hold n_out outputs per group, at most 256
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s);
 // Puts the kernel's code on the device (it is otherwise loaded by its first launch, which needs memory): a launch that

@@ -523,4 +523,7 @@ __host__ __device__ constexpr uint32_t instr_desc(bool tf32, bool a_mn_major, bo
          ((m >> 4) << 24);
 }
 
+// The same descriptor with another N.
+__device__ __forceinline__ uint32_t with_columns(uint32_t idesc, int n) { return (idesc & ~(0x3Fu << 17)) | static_cast<uint32_t>(n >> 3) << 17; }
+
 }  // namespace b200
