@@ -540,9 +540,9 @@ bool overlap(const void* a, size_t na, const void* b, size_t nb) {
 
 // Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
 // the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
-// and / or a reduction cut into slices where that occupies more SMs; the slab kernel also on pairs of CTAs.  The
+// and / or a reduction cut into slices where that occupies more SMs; both also on pairs of CTAs.  The
 // numbers appear in tuning files.
-enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvVariants = 5 };
+enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvTapPair = 5, kConvVariants = 6 };
 enum SlabMode { kSlabWide = 0, kSlabSpread, kSlabPair };      // of the slab kernel's tile search
 
 SlabMode slab_mode(int variant) { return variant == kConvSlabSpread ? kSlabSpread : variant == kConvSlabPair ? kSlabPair : kSlabWide; }
@@ -714,13 +714,27 @@ SlabTile tap_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int 
   return best;
 }
 
+// How a launch of `tiles` pair tiles on `units` pairs is cut: the tiles beyond whole waves get `splits` pairs each, if that saves more than
+// their raw accumulators and the second kernel cost (split_clocks()).  256 -> 256 3x3 at 14x14, 128 images, float32: 98 tiles on
+// 74 pairs, 24 of them cut in three.
+struct PairCut { long long whole; int splits; };
+PairCut pair_cut(long long tiles, int units, long long kiters, int bn) {
+  const long long rest = tiles % units, step = bn >= 256 ? 512 : 340;       // clocks per stage: MMAs, or 24 KB at 73 B/clk
+  const long long most = rest ? std::min<long long>(units / rest, kiters) : 1;
+  if (most < 2) return PairCut{tiles, 1};
+  const long long saved = kiters * step - cdiv(kiters, most) * step, cost = split_clocks(2 * rest * most, 128, bn, 2 * units);
+  return saved > cost + cost / 4 ? PairCut{tiles - rest, (int)most} : PairCut{tiles, 1};
+}
+
 // Slabs of a split launch and the parameters of its reduction that both kernels share.
 template <class P>
-int split_output(b200conv_ctx* c, Scratch& tmp, P& p, int bn, int rows, ConvReduceParams* q) {
+int split_output(b200conv_ctx* c, Scratch& tmp, P& p, int bn, int rows, ConvReduceParams* q, long long pair_tiles = 0, int first_tile = 0) {
   memset(q, 0, sizeof *q);
-  const long long tiles = 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  const long long tiles = pair_tiles ? pair_tiles : 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
+  if (tiles > 65535 / 2) return fail(c, B200CONV_E_INVALID, "too many split tiles");
+  q->first_tile = first_tile; q->tiles = (int)tiles; q->pair = pair_tiles > 0;
   float* partial;
-  const long long elems = tiles * p.splits * rows * bn;
+  const long long elems = (pair_tiles ? 2 : 1) * tiles * p.splits * rows * bn;
   int rc = tmp.get(sizeof(float) * elems, reinterpret_cast<void**>(&partial));
   if (rc) return rc;
   q->partial = p.partial = partial;
@@ -949,6 +963,13 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   return 0;
 }
 
+// Can the per-tap kernel run on pairs of CTAs: staged TMA stores of whole 128-byte channel rows, tiles of at least 128 filters?
+bool tap_pair_ok(b200conv_ctx* c, const FwdLikeArgs& a, const void* out, long long sn, long long sc, long long sh, long long sw, long long off) {
+  const long long es = (long long)elem_size(a.dtype);
+  return c->use_pair && c->num_sms >= 2 && a.n_out > 64 && a.n_out % (int)(128 / es) == 0 && sc == 1 && !c->epi.residual && !c->epi.pool &&
+         ((sw | sh | sn) * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es) % 16 == 0;
+}
+
 int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps_in,
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
@@ -966,6 +987,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   UmmaConvParams p;
   memset(&p, 0, sizeof p);
   const int kBK = a.dtype == B200CONV_F16 ? 64 : 32;
+  const bool pair = variant == kConvTapPair && tap_pair_ok(c, a, out, sn, sc, sh, sw, off);     // (a tuning file may name it for any geometry)
   const SlabTile tile = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, variant == kConvTapSpread);
   p.bw = tile.wt; p.bh = tile.th; p.bn = tile.nb;
   p.splits = tile.splits;
@@ -989,7 +1011,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   if (p.ntaps == 0) return 1;  // caller zero-fills
   for (int v = nviews; v < kMaxViews; ++v) p.views[v] = p.views[0];
   const int BN = tile.bn;
-  int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, BN);
+  int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, pair ? BN / 2 : BN);
   if (rc) return rc;
   p.kblocks = static_cast<int>(cdiv(a.Cin_g, kBK));
   p.splits = std::min(p.splits, p.ntaps * p.kblocks);
@@ -1008,6 +1030,31 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.epi = c->epi;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
+  if (pair) {
+    const long long es = (long long)elem_size(a.dtype), tiles = cdiv(1LL * p.tiles_w * p.tiles_h * p.tiles_n, 2) * p.groups * p.tiles_co;
+    cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)Wt, (cuuint64_t)Ht, (cuuint64_t)a.N};
+    cuuint64_t strides[3] = {(cuuint64_t)(sw * es), (cuuint64_t)(sh * es), (cuuint64_t)(sn * es)};
+    cuuint32_t box[4] = {(cuuint32_t)kBK, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = c->encode(&p.out_map, a.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                           static_cast<char*>(out) + off * es, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, kConvTap);
+    const PairCut cut = pair_cut(tiles, c->num_sms / 2, 1LL * p.ntaps * p.kblocks, BN);
+    p.whole = (int)cut.whole; p.splits = cut.splits;
+    Scratch tmp(c);
+    ConvReduceParams q;
+    if (cut.splits > 1) {
+      rc = split_output(c, tmp, p, BN, 128, &q, tiles - cut.whole, p.whole);
+      if (rc && rc != B200CONV_E_NOMEM) return rc;
+      if (rc) { p.whole = (int)tiles; p.splits = 1; }             // no memory for the slices: whole reductions need none
+      q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
+    }
+    c->last_variant = p.splits > 1 ? "tap pair cut" : "tap pair";
+    KLAUNCH(c, kKConvUmma, launch_conv_pair(p, a.dtype, c->num_sms, c->stream));
+    if (p.splits > 1) KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
+    return 0;
+  }
   c->last_variant = p.splits > 1 ? "tap split" : "tap";
   if (p.splits == 1) {
     KLAUNCH(c, kKConvUmma, launch_conv_umma(p, a.dtype, c->num_sms, c->stream));
@@ -1122,6 +1169,9 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                    (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
   // what cannot pool does not depend on the choice that an earlier call left (a split reduction pools any output)
   if (c->epi.pool && !(allow_slab && tma)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
+#ifdef B200CONV_TUNE
+  if (getenv("B200_VARIANT")) return run(atoi(getenv("B200_VARIANT")));
+#endif
   if (c->autotune) {
     auto it = c->algo_cache.find(key);
     if (it != c->algo_cache.end()) return run(it->second);
@@ -1133,6 +1183,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   if (!c->epi.pool) {
     cand[ncand++] = kConvTap;
     if (tap_spread) cand[ncand++] = kConvTapSpread;
+    const int bn = conv_umma_bn(a.n_out);
+    const SlabTile t = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, false);
+    if (tap_pair_ok(c, a, out, sn, sc, sh, sw, off) &&
+        cdiv(cdiv(Wt, t.wt) * cdiv(Ht, t.th) * cdiv(a.N, t.nb), 2) * cdiv(a.n_out, bn) * a.groups >= c->num_sms / 4)
+      cand[ncand++] = kConvTapPair;
   }
   if (allow_slab) {
     int eh[2] = {0, 0}, ew[2] = {0, 0};
@@ -3430,7 +3485,8 @@ int b200conv_set_splits(b200conv_ctx* c, int splits) {
 // kTuningKernels goes up with each change of the kernels after which earlier timings or the numbers of choices no longer hold.
 // 2: three gradWeights kernels to choose from where there were two, float32 pairs behind the one-tap choice.  (Files before it
 // have no such number.)
-constexpr int kTuningKernels = 2;
+// 3: the per-tap kernel on pairs.
+constexpr int kTuningKernels = 3;
 static std::string tuning_header(b200conv_ctx* c) {
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, c->device);

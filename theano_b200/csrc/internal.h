@@ -113,6 +113,7 @@ struct alignas(64) UmmaConvParams {
   int kblocks;                   // ceil(reduction channels per group / channels per stage)
   int bn_cols;                   // accumulator columns of a tile (32, 64, 128 or 256)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
+  int whole;                     // conv_pair.cu: the first tiles (of pairs), which are not cut into `splits` slices
   float* partial;
   long long partial_elems;       // elements of `partial` (checked in the range-checked build)
   int groups;
@@ -129,6 +130,7 @@ struct alignas(64) UmmaConvParams {
   ConvEpilogue epi;
   int* status;
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
+  CUtensorMap out_map;            // conv_pair.cu: 4-D (channel, w, h, n) over the output, box (128 bytes, bw, bh, bn)
 };
 
 // Columns of the MMAs of a tile that starts at output channel `first` of n_out: an MMA takes clocks by its columns, and a layer of
@@ -143,6 +145,8 @@ inline int mma_columns(int n_out, int first, int bn, bool pair) {
 }
 int conv_umma_bn(int n_out);      // accumulator columns that hold n_out outputs per group, at most 256
 cudaError_t launch_conv_umma(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s);
+// The same on pairs of CTAs (conv_pair.cu): channels-last outputs of whole 128-byte channel rows, no residual, 128 or 256 accumulator columns.
+cudaError_t launch_conv_pair(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s);
 // Puts the kernel's code on the device (it is otherwise loaded by its first launch, which needs memory): a launch that
 // runs split loads the code of the whole reduction with it, to fall back to when there is no memory for the slices.
 cudaError_t load_conv_umma(int dtype, int bn);
@@ -219,6 +223,8 @@ cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num
 // which wt x th are the tile's); for the per-tap kernel Ws = wt and Hs = th.
 struct ConvReduceParams {
   const float* partial;          // [tile][slice][bn_cols / 4][rows][4]
+  int first_tile, tiles;         // the tiles that were split; pair: both pixel tiles of each pair tile, side by side
+  int pair;
   int splits, rows, bn_cols;
   int Ws, Hs, wt, th, nb;
   int tiles_w, tiles_h, tiles_n, tiles_co, groups;

@@ -359,10 +359,14 @@ __global__ void __launch_bounds__(640, 2) wgrad_reduce_kernel(const float* __res
     if (whole) {
       const float4* src = reinterpret_cast<const float4*>(partial + slab_index(t, k, c, K, Cg)) + lane * (slab >> 2);
       const long long step = lanes * (slab >> 2);
-#pragma unroll 4
-      for (int s = lane; s < splits; s += lanes, src += step) {
-        const float4 v = *src;
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+      for (int s0 = lane; s0 < splits; s0 += 4 * lanes, src += 4 * step) {      // four loads in flight, also where there are three
+        float4 v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (s0 + e * lanes < splits) v[e] = src[e * step];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (s0 + e * lanes < splits) { acc.x += v[e].x; acc.y += v[e].y; acc.z += v[e].z; acc.w += v[e].w; }
       }
     } else {
       float* a = &acc.x;
