@@ -1,0 +1,98 @@
+"""The columns kernel: filter widths that fill the pitches of 8, 16 and 32 positions, images that end inside tiles and rows, filter
+counts with rows of 32, 64 and 128 bytes, groups, dilation, both directions, pooling, and infinities in the input."""
+import numpy as np
+import pytest
+
+from oracle import corr_oracle as O
+from theano_b200 import shim
+
+pytestmark = pytest.mark.gpu
+DTYPES = pytest.mark.parametrize("dtype", [np.float32, np.float16], ids=["f32", "f16"])
+T = shim.DeviceTensor
+F = np.float32
+
+
+@pytest.fixture
+def ctx():
+    c = shim.Context(0)
+    yield c
+    c.close()
+
+
+def tol(dtype):
+    return 5e-3 if dtype == F else 2e-2            # the repository's bounds for TF32 factors and float16 tensors
+
+
+def columns_only(ctx, path, call):
+    """Makes the remembered choice of every geometry that `call` meets the columns kernel, then runs it."""
+    call()
+    ctx.tuning_save(path)
+    head, *rest = open(path).read().splitlines()
+    open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + ["6"]) if r.startswith("a 3.") else r for r in rest]) + "\n")
+    ctx.tuning_load(path)
+    y = call()
+    assert ctx.last_variant == "columns"
+    return y
+
+
+# images, height, width, channels, filters, kernel, dilation, groups
+LAYERS = [(2, 13, 30, 48, 32, (3, 3), 1, 1), (1, 9, 31, 24, 64, (3, 3), 1, 1), (3, 14, 14, 64, 16, (3, 3), 1, 1), (2, 7, 6, 40, 24, (3, 3), 1, 1),
+          (2, 28, 28, 128, 128, (3, 3), 1, 4), (1, 40, 45, 33, 12, (1, 5), 1, 1), (2, 19, 37, 70, 48, (5, 2), 2, 1), (1, 33, 17, 16, 8, (4, 8), 1, 1),
+          (1, 64, 50, 12, 30, (7, 7), 1, 1), (2, 20, 24, 96, 64, (2, 4), 3, 1), (150, 16, 16, 64, 64, (3, 3), 1, 2)]
+
+
+@DTYPES
+@pytest.mark.parametrize("n,h,w_,c,k,ks,d,g", LAYERS)
+def test_forward_against_the_oracle(ctx, tmp_path, dtype, n, h, w_, c, k, ks, d, g):
+    rs = np.random.RandomState(n + k)
+    kw = dict(border_mode="half", filter_dilation=(d, d), num_groups=g)
+    x = rs.standard_normal((n, c, h, w_)).astype(dtype)
+    w = (rs.standard_normal((k, c // g) + ks) / np.sqrt(c // g * ks[0] * ks[1])).astype(dtype)
+    b = rs.standard_normal((1, k, 1, 1)).astype(dtype)
+    X, W, B = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), T.from_host(ctx, b)
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, bias=B, relu=True, **kw))
+    ref = np.maximum(O.conv2d(x.astype(F), w.astype(F), **kw) + b.astype(F), 0)
+    assert O.rel_err(y.to_host().astype(F), ref) < tol(dtype)
+
+
+@DTYPES
+@pytest.mark.parametrize("n,h,w_,c,k,ks,d,g", [(2, 13, 30, 32, 40, (3, 3), 1, 1), (1, 24, 33, 60, 70, (5, 3), 2, 1), (2, 28, 28, 128, 128, (3, 3), 1, 4)])
+def test_grad_inputs_against_the_oracle(ctx, tmp_path, dtype, n, h, w_, c, k, ks, d, g):
+    rs = np.random.RandomState(n + k)
+    kw = dict(border_mode="half", filter_dilation=(d, d), num_groups=g)
+    w = (rs.standard_normal((k, c // g) + ks) / np.sqrt(k // g * ks[0] * ks[1])).astype(dtype)
+    dy = rs.standard_normal((n, k, h, w_)).astype(dtype)
+    W, DY = T.from_host(ctx, w), T.from_host(ctx, dy, "nhwc")
+    dx = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_grad_inputs(W, DY, (h, w_), **kw))
+    assert O.rel_err(dx.to_host().astype(F), O.conv2d_grad_inputs(w.astype(F), dy.astype(F), (h, w_), **kw)) < tol(dtype)
+
+
+@DTYPES
+@pytest.mark.parametrize("n,h,w_,c,k", [(2, 28, 30, 24, 64), (3, 10, 62, 40, 64)])
+def test_pooling(ctx, tmp_path, dtype, n, h, w_, c, k):
+    rs = np.random.RandomState(n)
+    x = rs.standard_normal((n, c, h, w_)).astype(dtype)
+    w = (rs.standard_normal((k, c, 3, 3)) / np.sqrt(c * 9)).astype(dtype)
+    X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, border_mode="half", relu=True, pool=True))
+    full = shim.device_conv2d(X, W, border_mode="half", relu=True).to_host().astype(F)
+    ref = full.reshape(n, k, h // 2, 2, w_ // 2, 2).max(axis=(3, 5))
+    assert O.rel_err(y.to_host().astype(F), ref) < (1e-5 if dtype == F else 1e-3)      # the same products, sums in another order
+
+
+@DTYPES
+def test_an_infinity_stays_with_the_outputs_that_it_belongs_to(ctx, tmp_path, dtype):
+    rs = np.random.RandomState(1)
+    x = rs.standard_normal((2, 20, 17, 29)).astype(dtype)
+    x[1, 3, 8, 28] = np.inf
+    w = (1 + rs.random_sample((30, 20, 3, 3))).astype(dtype)
+    X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, border_mode="half")).to_host()
+    touched = np.zeros(y.shape, bool)
+    touched[1, :, 7:10, 27:29] = True
+    assert np.array_equal(~np.isfinite(y), touched)
+    stored = np.empty((2, 17, 29, ctx.padded_channels(30, dtype)), dtype)
+    Y = shim.device_conv2d(X, W, border_mode="half")
+    ctx.d2h(stored, Y.ptr)
+    ctx.sync()
+    assert not stored[..., 30:].any()

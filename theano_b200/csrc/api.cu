@@ -540,9 +540,10 @@ bool overlap(const void* a, size_t na, const void* b, size_t nb) {
 
 // Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
 // the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
-// and / or a reduction cut into slices where that occupies more SMs; both also on pairs of CTAs.  The
+// and / or a reduction cut into slices where that occupies more SMs; both also on pairs of CTAs; the
+// columns kernel for layers of at most 64 filters.  The
 // numbers appear in tuning files.
-enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvTapPair = 5, kConvVariants = 6 };
+enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvTapPair = 5, kConvCols = 6, kConvVariants = 7 };
 enum SlabMode { kSlabWide = 0, kSlabSpread, kSlabPair };      // of the slab kernel's tile search
 
 SlabMode slab_mode(int variant) { return variant == kConvSlabSpread ? kSlabSpread : variant == kConvSlabPair ? kSlabPair : kSlabWide; }
@@ -963,6 +964,116 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   return 0;
 }
 
+// Columns kernel (conv_cols.cu) for layers of at most 64 filters per group whose taps are a whole grid of rows and columns over one view.
+// Returns 0 when it was launched (launch false: when it could be), 2 when the geometry does not fit, or an error code.  d2s_C > 0: the output
+// channels are the four classes of a stride-2 gradInputs with that many channels, `out` is the d2s_H x d2s_W gradient, channels-last, 16 bytes
+// per pixel.
+int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps, int rh, int rw, int Wt, int Ht, void* out, long long sn,
+                  long long sc, long long sh, long long sw, long long off, const void* bias, int relu, bool launch, int d2s_C = 0, int d2s_H = 0,
+                  int d2s_W = 0) {
+  const int es = (int)elem_size(a.dtype), kBK = a.dtype == B200CONV_F16 ? 64 : 32;
+  if (a.n_out > 64 || a.fold || !a.classes.empty() || c->epi.residual || sc != 1 || taps.size() < 2 || 1LL * Wt * Ht * a.N == 0) return 2;
+  if (!d2s_C && (((sw | sh | sn) * es) % 16 || reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es) % 16)) return 2;
+  ColsConvParams p;
+  memset(&p, 0, sizeof p);
+  // the grid: rows of the same dh, kW neighbouring matrices each, the same column offsets in every row
+  std::vector<ConvTap> t = taps;
+  std::sort(t.begin(), t.end(), [](const ConvTap& x, const ConvTap& y) { return x.wmat < y.wmat; });
+  int kW = 0;
+  while (kW < (int)t.size() && t[kW].dh == t[0].dh) ++kW;
+  if (kW < 2 || kW > kMaxColTaps || t.size() % kW || (int)t.size() / kW > kMaxColTaps) return 2;
+  p.kW = kW; p.kH = (int)t.size() / kW;
+  p.dh_min = t[0].dh; p.dw_min = t[0].dw;
+  int dh_max = t[0].dh, dw_max = t[0].dw;
+  for (size_t i = 0; i < t.size(); ++i) {
+    const ConvTap &first = t[i / kW * kW], &col = t[i % kW];
+    if (t[i].dh != first.dh || t[i].dw != col.dw || t[i].wmat != first.wmat + (int)(i % kW)) return 2;
+    p.dh_min = std::min<int>(p.dh_min, t[i].dh); dh_max = std::max<int>(dh_max, t[i].dh);
+    p.dw_min = std::min<int>(p.dw_min, t[i].dw); dw_max = std::max<int>(dw_max, t[i].dw);
+  }
+  const int Eh = dh_max - p.dh_min, Ew = dw_max - p.dw_min;
+  p.dil = std::abs(t[1].dw - t[0].dw);
+  for (int j = 1; j < kW; ++j)
+    if (t[j].dw - t[j - 1].dw != t[1].dw - t[0].dw || p.dil == 0) return 2;
+  p.bn = a.n_out <= 16 ? 16 : a.n_out <= 32 ? 32 : 64;
+  const int n_cols = kW * p.bn;
+  if (n_cols > 256 || (d2s_C && (d2s_C > 4 || a.n_out > 16))) return 2;
+  const bool rightwards = t[1].dw > t[0].dw;
+  p.col_first = rightwards ? 0 : n_cols - p.bn;
+  p.col_step = rightwards ? p.bn : -p.bn;
+  p.chunk_ch = std::min(32, p.bn);        // 32 at most: the groups of epilogue warps share a tile
+  if (!d2s_C && a.groups > 1 && a.n_out % p.chunk_ch) return 2;
+  // Tile: the pitch that leaves the fewest accumulator rows to compute; two accumulators where two sets of them fit 512 columns.
+  const int even = c->epi.pool ? 2 : 1, most_acc = 4 * n_cols <= 512 ? 2 : 1;
+  long long best = -1;
+  for (int pitch : {32, 16, 8})
+    for (int n_acc = most_acc; n_acc >= 1; --n_acc) {
+      const int widest = (pitch - Ew) / even * even, rows = 128 / pitch * n_acc / even * even;
+      if (widest < 1 || rows < 1) continue;
+      const int tw = (int)cdiv(Wt, widest), th_n = (int)cdiv(Ht, std::min(rows, 256 - Eh));
+      // clocks of the MMAs: with two accumulators each has an issuer of its own; one alone waits for itself (71 against 117 clocks per 128 x 96)
+      const long long work = 1LL * tw * th_n * n_acc * (n_cols > 128 ? 1 : n_acc == 2 ? 6 : 10);
+      if (256 - Eh < 1 || (best >= 0 && work >= best)) continue;
+      best = work;
+      p.pitch = pitch; p.n_acc = n_acc;
+      p.wt = round_up((int)cdiv(Wt, tw), even); p.th = round_up((int)cdiv(Ht, th_n), even);
+    }
+  if (best < 0) return 2;
+  p.Hs = p.th + Eh;
+  p.slab_bytes = std::max(p.Hs * p.pitch, 128 * p.n_acc + Eh * p.pitch) * 128;
+  p.slab_bytes = (p.slab_bytes + 1023) / 1024 * 1024;
+  // groups of epilogue warps: 4 / n_acc, one per chunk of channels, the rest on further tiles with accumulator sets of their own
+  const int nchunks = d2s_C ? 1 : (int)cdiv(a.n_out, p.chunk_ch);
+  p.step = 4 / p.n_acc / nchunks;
+  while (p.step > 2 && p.step * p.n_acc * n_cols > 512) --p.step;
+  p.sets = std::max(2, p.step);
+  const int ngrp = nchunks * p.step;
+  p.stage_bytes = d2s_C ? 0 : (p.wt * p.th * p.chunk_ch * es + 1023) / 1024 * 1024;
+  int bufs = 1;
+  p.s_stages = p.b_stages = 2;
+  auto fits = [&](int s, int b, int f) { return 1LL * s * p.slab_bytes + 1LL * b * p.rps * n_cols * 128 + 1LL * f * ngrp * p.stage_bytes <= kSlabSmemBudget; };
+  p.rps = p.kH <= 5 && t.back().wmat == t[0].wmat + (int)t.size() - 1 ? p.kH : 1;      // rows that are neighbours in the packed filters
+  if (!fits(2, 2, 1)) p.rps = 1;
+  if (!fits(2, 2, 1)) return 2;
+  if (!launch) return 0;
+  for (char step : {'s', 'b', 'f', 'b', 's', 'b', 'b'}) {
+    const int s = p.s_stages + (step == 's'), b = p.b_stages + (step == 'b'), f = step == 'f' ? 2 : bufs;
+    if (fits(s, b, f)) { p.s_stages = s; p.b_stages = b; bufs = f; }
+  }
+  p.stage_nbuf = bufs * ngrp;
+  for (int i = 0; i < p.kH; ++i) { p.row_mat[i] = t[i * kW].wmat; p.row_shift[i] = (int16_t)((t[i * kW].dh - p.dh_min) * p.pitch); }
+  int rc = make_act_view(c, &p.view, a, rh, rw, kBK, p.pitch, p.Hs, 1);
+  if (rc) return rc;
+  if ((rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, p.bn, a.groups, p.rps * kW))) return rc;
+  if (!d2s_C) {
+    const int pl = even;
+    cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)(Wt / pl), (cuuint64_t)(Ht / pl), (cuuint64_t)a.N};
+    cuuint64_t strides[3] = {(cuuint64_t)(sw * es), (cuuint64_t)(sh * es), (cuuint64_t)(sn * es)};
+    cuuint32_t box[4] = {(cuuint32_t)p.chunk_ch, (cuuint32_t)(p.wt / pl), (cuuint32_t)(p.th / pl), 1}, estr[4] = {1, 1, 1, 1};
+    const int row_bytes = p.chunk_ch * es;
+    CUresult r = c->encode(&p.out_map, a.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
+                           static_cast<char*>(out) + off * es, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return 2;
+  }
+  p.kblocks = (int)cdiv(a.Cin_g, kBK);
+  p.groups = a.groups;
+  p.Wt = Wt; p.Ht = Ht; p.Nimg = a.N;
+  p.tiles_w = (int)cdiv(Wt, p.wt); p.tiles_h = (int)cdiv(Ht, p.th);
+  p.by_groups = divisor(a.groups); p.by_tiles_w = divisor(p.tiles_w); p.by_tiles_h = divisor(p.tiles_h);
+  p.n_out = a.n_out; p.n_real = a.w_rows;
+  p.d2s = d2s_C > 0; p.d2s_C = d2s_C; p.d2s_H = d2s_H; p.d2s_W = d2s_W;
+  p.out = out;
+  p.out_elems = 1LL * a.N * d2s_H * d2s_W * (16 / es);
+  p.bias = bias; p.relu = relu; p.epi = c->epi;
+  p.status = c->d_status;
+  p.wait_clocks = c->wait_clocks;
+  c->last_variant = "columns";
+  KLAUNCH(c, kKConvUmma, launch_conv_cols(p, a.dtype, c->num_sms, c->stream));
+  return 0;
+}
+
 // Can the per-tap kernel run on pairs of CTAs: staged TMA stores of whole 128-byte channel rows, tiles of at least 128 filters?
 bool tap_pair_ok(b200conv_ctx* c, const FwdLikeArgs& a, const void* out, long long sn, long long sc, long long sh, long long sw, long long off) {
   const long long es = (long long)elem_size(a.dtype);
@@ -974,6 +1085,13 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
                       const void* bias, int relu, int variant) {
+  if (variant == kConvCols) {          // (a tuning file may name it for any geometry)
+    const int rh = view_parity[0].first, rw = view_parity[0].second;
+    const int rc = view_parity.size() == 1 && rh < a.Hs && rw < a.Ws
+                       ? try_conv_cols(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true) : 2;
+    if (rc != 2) return rc;
+    variant = kConvTap;
+  }
   if (variant == kConvSlab || variant == kConvSlabSpread || variant == kConvSlabPair) {
     // the slab kernel reads one view (a tuning file may name it for a geometry with several)
     const bool one_view = view_parity.size() == 1;
@@ -1145,6 +1263,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                   const void* bias, int relu, bool allow_slab = true) {
   if (view_parity.size() != 1) allow_slab = false;
   auto run_one = [&](int variant) -> int {
+    if (c->epi.pool && variant == kConvCols) {
+      const int rc = try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true);
+      if (rc != 2) return rc;
+      variant = kConvSlab;
+    }
     if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
       const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
                                    relu, slab_mode(variant));
@@ -1189,6 +1312,8 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
         cdiv(cdiv(Wt, t.wt) * cdiv(Ht, t.th) * cdiv(a.N, t.nb), 2) * cdiv(a.n_out, bn) * a.groups >= c->num_sms / 4)
       cand[ncand++] = kConvTapPair;
   }
+  if (allow_slab && try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, false) == 0)
+    cand[ncand++] = kConvCols;
   if (allow_slab) {
     int eh[2] = {0, 0}, ew[2] = {0, 0};
     for (size_t i = 0; i < taps_in.size(); ++i) {
@@ -1622,9 +1747,16 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       const int Ct = pad_channels(ncls * d.C, d.dtype);
       const int nu = (int)utaps.size(), n_out = Ct;      // padded with zero filters: whole 16-byte pieces
       const int Hq = (d.H + d.sH - 1) / d.sH, Wq = (d.W + d.sW - 1) / d.sW;
+      // row by row, so that a row's columns are neighbours in the packed filters
+      std::sort(utaps.begin(), utaps.end(), [](const ConvTap& x, const ConvTap& y) { return x.dh != y.dh ? x.dh < y.dh : x.dw < y.dw; });
+      MergedTapTable sorted;
+      for (int u = 0; u < nu; ++u) {
+        std::copy(std::begin(tb.src[utaps[u].wmat]), std::end(tb.src[utaps[u].wmat]), std::begin(sorted.src[u]));
+        utaps[u].wmat = (int16_t)u;
+      }
+      tb = sorted;
       void *wp, *merged;
       if ((rc = tmp.get(es * (size_t)nu * n_out * ldw, &wp))) return rc;
-      if ((rc = tmp.get(es * (size_t)d.N * Hq * Wq * Ct, &merged))) return rc;
       KLAUNCH(c, kKPack, launch_pack_filters_merged(w, wp, d.K, d.C, d.kH, d.kW, d.flip, tb, nu, ncls, n_out,
                                                     ldw, d.dtype, c->stream));
       FwdLikeArgs a;
@@ -1633,6 +1765,15 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       a.n_out = a.w_rows = n_out; a.groups = 1; a.N = d.N; a.dtype = d.dtype;
       a.view_sH = 1; a.view_sW = 1;
       std::vector<std::pair<int, int>> parity(1, {0, 0});
+      // The columns kernel writes the gradient's pixels itself; else the classes go through a tensor of their own and a depth-to-space pass.
+      // 64 -> 3 7x7 at 224x224, float16, 256 images 415 -> 143 us, one 13.3 -> 6.7; 32 -> 3 4x4 at 64x64, 2 images 10.1 -> 6.2; float32 688 -> 248,
+      // 17.1 -> 7.6 and 10.9 -> 6.0: of nine such layers in both types the columns kernel was slower on none.
+      if (d.sH == 2 && d.sW == 2 && out_nhwc && Cp * es == 16 && !(flags & B200CONV_NO_SLAB)) {
+        rc = try_conv_cols(c, a, utaps, 0, 0, Wq, Hq, dx, 0, 1, 0, 0, 0, nullptr, 0, true, d.C, d.H, d.W);
+        if (rc == 0) c->last_algo = "umma";
+        if (rc != 2) return rc;
+      }
+      if ((rc = tmp.get(es * (size_t)d.N * Hq * Wq * Ct, &merged))) return rc;
       rc = run_conv_umma(c, a, utaps, parity, Wq, Hq, merged, 1LL * Hq * Wq * Ct, 1, 1LL * Wq * Ct, Ct, 0,
                          nullptr, 0, !(flags & B200CONV_NO_SLAB));
       if (rc) return rc == 1 ? fail(c, B200CONV_E_CUDA, "internal: empty gradient view") : rc;

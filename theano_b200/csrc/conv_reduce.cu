@@ -24,15 +24,6 @@ template <typename T> __device__ __forceinline__ float to_f(T v) { return static
 
 constexpr int kReduceThreads = 128;
 
-// n / d for n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using multiplication")
-struct Divisor { uint32_t d, mul, shift; };
-Divisor divisor(uint32_t d) {
-  uint32_t shift = 0;
-  while ((1ull << shift) < d) ++shift;
-  return Divisor{d, static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - d)) / d + 1), shift};
-}
-__device__ __forceinline__ uint32_t quotient(uint32_t n, const Divisor& v) { return (__umulhi(n, v.mul) + n) >> v.shift; }
-
 // How a launch is walked: units of (pixel tile, 32 rows, columns of a block).
 struct ReduceWalk {
   Divisor row_chunks, col_blocks, per_w, per_h, tiles_w, tiles_h, tiles_co, groups;

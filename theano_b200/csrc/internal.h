@@ -81,6 +81,17 @@ inline bool aligned16(std::initializer_list<const void*> ptrs) {
   return true;
 }
 
+// n / d for n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using multiplication")
+struct Divisor { uint32_t d, mul, shift; };
+inline Divisor divisor(uint32_t d) {
+  uint32_t shift = 0;
+  while ((1ull << shift) < d) ++shift;
+  return Divisor{d, static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - d)) / d + 1), shift};
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t quotient(uint32_t n, const Divisor& v) { return (__umulhi(n, v.mul) + n) >> v.shift; }
+#endif
+
 // Codes a kernel writes to the device status word when it gives up.
 enum : int { kStatusOk = 0, kStatusTimeout = 1, kStatusBadIndex = 2 };
 
@@ -217,6 +228,42 @@ constexpr int kSlabStageBytes = 64 * 1024;    // staging buffers of the TMA-stor
 constexpr int kSlabSmemBudget = 220 * 1024;   // slab buffers + filter ring; the rest of the 227 KB
                                               // holds barriers and the epilogue's transpose tiles
 cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num_sms, cudaStream_t s);
+
+// ---- layers of at most 64 filters, the filter's columns inside one MMA (conv_cols.cu) ----------------
+constexpr int kMaxColTaps = 8;   // filter rows, filter columns
+struct alignas(64) ColsConvParams {
+  CUtensorMap view;              // 5-D (c_in_group, group, w, h, n), box (kBK, 1, pitch, Hs, 1)
+  CUtensorMap wmap;              // 4-D packed filters (k_red, n_out, group, tap), box (kBK, bn, 1, rps * kW)
+  CUtensorMap out_map;           // 4-D (channel, w, h, n) over the output, box (chunk_ch, wt, th, 1), pooled: half of wt and th
+  int kH, kW;
+  int16_t row_mat[kMaxColTaps];  // filter row: its first packed matrix
+  int16_t row_shift[kMaxColTaps];// and how many slab positions it lies behind the first
+  int col_first, col_step, dil;  // accumulator column of the leftmost filter column, from there to the next (to the right), positions between them
+  int bn;                        // accumulator columns per filter column (16, 32 or 64)
+  int kblocks, groups;
+  int Wt, Ht, Nimg;              // output grid
+  int wt, th, pitch, Hs;         // tile, positions from one slab row to the next (8, 16 or 32), slab rows
+  int dw_min, dh_min;            // view coordinate of slab column / row 0 relative to the tile origin
+  int tiles_w, tiles_h;
+  Divisor by_groups, by_tiles_w, by_tiles_h;
+  int n_acc;                     // 128-row accumulators of a tile: 1 or 2
+  int sets;                      // of accumulators: 2 to 4, and as many tiles apart are the ones of a group of epilogue warps (every tile, where it has no choice)
+  int step;                      // that distance
+  int slab_bytes, s_stages, b_stages;
+  int rps;                       // filter rows per filter stage (a divisor of kH)
+  int n_out, n_real;             // output channels per group as stored / with filters
+  int chunk_ch;                  // channels of a staged row: 16 or 32
+  int stage_bytes, stage_nbuf;   // staging buffers (one or two per group of epilogue warps)
+  int d2s, d2s_C, d2s_H, d2s_W;  // 1: the filters are the four classes of a stride-2 gradInputs with d2s_C channels, `out` the H x W gradient itself
+  void* out;
+  long long out_elems;           // of `out` (checked in the range-checked build)
+  const void* bias;
+  int relu;
+  ConvEpilogue epi;
+  int* status;
+  long long wait_clocks;         // bound of every device-side wait, in SM clocks
+};
+cudaError_t launch_conv_cols(const ColsConvParams& p, int dtype, int num_sms, cudaStream_t s);
 
 // ---- reductions split over CTAs (conv_reduce.cu) --------------------------------------------
 // The tile geometry is that of the slab kernel (rows of a tile on a grid of Ws x Hs positions per image, of
