@@ -317,8 +317,10 @@ int b200conv_selftest_wait(b200conv_ctx* ctx);
 /* Name of the kernel family the last fwd/dgrad/wgrad call used: "umma" or "direct". */
 const char* b200conv_last_algo(b200conv_ctx* ctx);
 /* The kernel variant of the last tensor-core launch: of a forward or gradInputs call "tap", "tap split", "slab", "slab split",
- * "slab pair", "slab classes", "slab classes pair", "tap pair", "tap pair cut" or "gemm pair" (split, cut: the reduction in slices that a second kernel adds;
- * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch); of gradWeights "wgrad tap" (one
+ * "slab pair", "slab classes", "slab classes pair", "tap pair", "tap pair cut",
+ * "columns", "columns pair" or "gemm pair" (split, cut: the reduction in slices that a second kernel adds;
+ * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch; columns: the filter's columns inside one
+ * MMA); of gradWeights "wgrad tap" (one
  * filter tap per work item), "wgrad pair" (the same on pairs of CTAs), "wgrad groups" (tap groups share operands) or "wgrad rows"
  * (the filter's rows and columns inside one MMA).  Of a call that times variants it is the one whose result is kept. */
 const char* b200conv_last_variant(b200conv_ctx* ctx);

@@ -23,15 +23,15 @@ def tol(dtype):
     return 5e-3 if dtype == F else 2e-2            # the repository's bounds for TF32 factors and float16 tensors
 
 
-def columns_only(ctx, path, call):
-    """Makes the remembered choice of every geometry that `call` meets the columns kernel, then runs it."""
+def columns_only(ctx, path, call, pair=False):
+    """Makes the remembered choice of every geometry that `call` meets the columns kernel (on pairs of CTAs), then runs it."""
     call()
     ctx.tuning_save(path)
     head, *rest = open(path).read().splitlines()
-    open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + ["6"]) if r.startswith("a 3.") else r for r in rest]) + "\n")
+    open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + ["7" if pair else "6"]) if r.startswith("a 3.") else r for r in rest]) + "\n")
     ctx.tuning_load(path)
     y = call()
-    assert ctx.last_variant == "columns"
+    assert ctx.last_variant == ("columns pair" if pair else "columns")
     return y
 
 
@@ -67,14 +67,36 @@ def test_grad_inputs_against_the_oracle(ctx, tmp_path, dtype, n, h, w_, c, k, ks
     assert O.rel_err(dx.to_host().astype(F), O.conv2d_grad_inputs(w.astype(F), dy.astype(F), (h, w_), **kw)) < tol(dtype)
 
 
+# odd numbers of tiles, more and fewer than pairs of SMs, filters between 33 and 64
+PAIRS = [(1, 9, 31, 24, 64, (3, 3), 1, 1), (3, 14, 14, 64, 40, (3, 3), 1, 1), (1, 200, 61, 33, 48, (1, 4), 1, 1), (5, 61, 61, 70, 64, (5, 2), 2, 1),
+         (150, 16, 16, 128, 128, (3, 3), 1, 2), (33, 56, 28, 130, 64, (3, 3), 1, 1)]
+
+
 @DTYPES
-@pytest.mark.parametrize("n,h,w_,c,k", [(2, 28, 30, 24, 64), (3, 10, 62, 40, 64)])
-def test_pooling(ctx, tmp_path, dtype, n, h, w_, c, k):
+@pytest.mark.parametrize("n,h,w_,c,k,ks,d,g", PAIRS)
+def test_pairs_against_the_oracle(ctx, tmp_path, dtype, n, h, w_, c, k, ks, d, g):
+    rs = np.random.RandomState(n + k)
+    kw = dict(border_mode="half", filter_dilation=(d, d), num_groups=g)
+    x = rs.standard_normal((n, c, h, w_)).astype(dtype)
+    w = (rs.standard_normal((k, c // g) + ks) / np.sqrt(c // g * ks[0] * ks[1])).astype(dtype)
+    b = rs.standard_normal((1, k, 1, 1)).astype(dtype)
+    X, W, B = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), T.from_host(ctx, b)
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, bias=B, relu=True, **kw), pair=True)
+    ref = np.maximum(O.conv2d(x.astype(F), w.astype(F), **kw) + b.astype(F), 0)
+    assert O.rel_err(y.to_host().astype(F), ref) < tol(dtype)
+    one = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, bias=B, relu=True, **kw))
+    assert np.array_equal(y.to_host(), one.to_host())      # the same sums
+
+
+@DTYPES
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("n,h,w_,c,k", [(2, 28, 30, 24, 64), (3, 10, 62, 40, 64), (40, 56, 56, 24, 64)])
+def test_pooling(ctx, tmp_path, dtype, n, h, w_, c, k, pair):
     rs = np.random.RandomState(n)
     x = rs.standard_normal((n, c, h, w_)).astype(dtype)
     w = (rs.standard_normal((k, c, 3, 3)) / np.sqrt(c * 9)).astype(dtype)
     X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
-    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, border_mode="half", relu=True, pool=True))
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, border_mode="half", relu=True, pool=True), pair)
     full = shim.device_conv2d(X, W, border_mode="half", relu=True).to_host().astype(F)
     ref = full.reshape(n, k, h // 2, 2, w_ // 2, 2).max(axis=(3, 5))
     assert O.rel_err(y.to_host().astype(F), ref) < (1e-5 if dtype == F else 1e-3)      # the same products, sums in another order

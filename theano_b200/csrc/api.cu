@@ -541,9 +541,9 @@ bool overlap(const void* a, size_t na, const void* b, size_t nb) {
 // Kernel variants of a forward / gradInputs launch: the slab kernel (one activation slab per channel block) or
 // the per-tap kernel, each with the widest tiles and a whole reduction per tile, or "spread": narrower tiles
 // and / or a reduction cut into slices where that occupies more SMs; both also on pairs of CTAs; the
-// columns kernel for layers of at most 64 filters.  The
+// columns kernel for layers of at most 64 filters, with more than 32 on pairs too.  The
 // numbers appear in tuning files.
-enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvTapPair = 5, kConvCols = 6, kConvVariants = 7 };
+enum { kConvTap = 0, kConvSlab = 1, kConvSlabSpread = 2, kConvTapSpread = 3, kConvSlabPair = 4, kConvTapPair = 5, kConvCols = 6, kConvColsPair = 7, kConvVariants = 8 };
 enum SlabMode { kSlabWide = 0, kSlabSpread, kSlabPair };      // of the slab kernel's tile search
 
 SlabMode slab_mode(int variant) { return variant == kConvSlabSpread ? kSlabSpread : variant == kConvSlabPair ? kSlabPair : kSlabWide; }
@@ -969,8 +969,8 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
 // channels are the four classes of a stride-2 gradInputs with that many channels, `out` is the d2s_H x d2s_W gradient, channels-last, 16 bytes
 // per pixel.
 int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvTap>& taps, int rh, int rw, int Wt, int Ht, void* out, long long sn,
-                  long long sc, long long sh, long long sw, long long off, const void* bias, int relu, bool launch, int d2s_C = 0, int d2s_H = 0,
-                  int d2s_W = 0) {
+                  long long sc, long long sh, long long sw, long long off, const void* bias, int relu, bool launch, bool pair, int d2s_C = 0,
+                  int d2s_H = 0, int d2s_W = 0) {
   const int es = (int)elem_size(a.dtype), kBK = a.dtype == B200CONV_F16 ? 64 : 32;
   if (a.n_out > 64 || a.fold || !a.classes.empty() || c->epi.residual || sc != 1 || taps.size() < 2 || 1LL * Wt * Ht * a.N == 0) return 2;
   if (!d2s_C && (((sw | sh | sn) * es) % 16 || reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es) % 16)) return 2;
@@ -997,14 +997,19 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     if (t[j].dw - t[j - 1].dw != t[1].dw - t[0].dw || p.dil == 0) return 2;
   p.bn = a.n_out <= 16 ? 16 : a.n_out <= 32 ? 32 : 64;
   const int n_cols = kW * p.bn;
+  if (pair && (p.bn != 64 || !c->use_pair || c->num_sms < 2)) return 2;
   if (n_cols > 256 || (d2s_C && (d2s_C > 4 || a.n_out > 16))) return 2;
   const bool rightwards = t[1].dw > t[0].dw;
-  p.col_first = rightwards ? 0 : n_cols - p.bn;
-  p.col_step = rightwards ? p.bn : -p.bn;
+  // a pair's MMAs take the columns of the even CTA's 32 filters first, then those of the other's
+  const int step = pair ? p.bn / 2 : p.bn;
+  p.pair = pair;
+  p.col_first = rightwards ? 0 : (kW - 1) * step;
+  p.col_step = rightwards ? step : -step;
+  p.chunk_step = pair ? kW * step : 32;
   p.chunk_ch = std::min(32, p.bn);        // 32 at most: the groups of epilogue warps share a tile
   if (!d2s_C && a.groups > 1 && a.n_out % p.chunk_ch) return 2;
   // Tile: the pitch that leaves the fewest accumulator rows to compute; two accumulators where two sets of them fit 512 columns.
-  const int even = c->epi.pool ? 2 : 1, most_acc = 4 * n_cols <= 512 ? 2 : 1;
+  const int even = c->epi.pool ? 2 : 1, most_acc = 4 * n_cols <= 512 && !pair ? 2 : 1;
   long long best = -1;
   for (int pitch : {32, 16, 8})
     for (int n_acc = most_acc; n_acc >= 1; --n_acc) {
@@ -1031,7 +1036,7 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.stage_bytes = d2s_C ? 0 : (p.wt * p.th * p.chunk_ch * es + 1023) / 1024 * 1024;
   int bufs = 1;
   p.s_stages = p.b_stages = 2;
-  auto fits = [&](int s, int b, int f) { return 1LL * s * p.slab_bytes + 1LL * b * p.rps * n_cols * 128 + 1LL * f * ngrp * p.stage_bytes <= kSlabSmemBudget; };
+  auto fits = [&](int s, int b, int f) { return 1LL * s * p.slab_bytes + 1LL * b * p.rps * (pair ? n_cols / 2 : n_cols) * 128 + 1LL * f * ngrp * p.stage_bytes <= kSlabSmemBudget; };
   p.rps = p.kH <= 5 && t.back().wmat == t[0].wmat + (int)t.size() - 1 ? p.kH : 1;      // rows that are neighbours in the packed filters
   if (!fits(2, 2, 1)) p.rps = 1;
   if (!fits(2, 2, 1)) return 2;
@@ -1044,7 +1049,7 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   for (int i = 0; i < p.kH; ++i) { p.row_mat[i] = t[i * kW].wmat; p.row_shift[i] = (int16_t)((t[i * kW].dh - p.dh_min) * p.pitch); }
   int rc = make_act_view(c, &p.view, a, rh, rw, kBK, p.pitch, p.Hs, 1);
   if (rc) return rc;
-  if ((rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, p.bn, a.groups, p.rps * kW))) return rc;
+  if ((rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, step, a.groups, p.rps * kW))) return rc;
   if (!d2s_C) {
     const int pl = even;
     cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)(Wt / pl), (cuuint64_t)(Ht / pl), (cuuint64_t)a.N};
@@ -1069,7 +1074,7 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.bias = bias; p.relu = relu; p.epi = c->epi;
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
-  c->last_variant = "columns";
+  c->last_variant = pair ? "columns pair" : "columns";
   KLAUNCH(c, kKConvUmma, launch_conv_cols(p, a.dtype, c->num_sms, c->stream));
   return 0;
 }
@@ -1085,10 +1090,10 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
                       const std::vector<std::pair<int, int>>& view_parity, int Wt, int Ht, void* out,
                       long long sn, long long sc, long long sh, long long sw, long long off,
                       const void* bias, int relu, int variant) {
-  if (variant == kConvCols) {          // (a tuning file may name it for any geometry)
+  if (variant == kConvCols || variant == kConvColsPair) {          // (a tuning file may name it for any geometry)
     const int rh = view_parity[0].first, rw = view_parity[0].second;
     const int rc = view_parity.size() == 1 && rh < a.Hs && rw < a.Ws
-                       ? try_conv_cols(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true) : 2;
+                       ? try_conv_cols(c, a, taps_in, rh, rw, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true, variant == kConvColsPair) : 2;
     if (rc != 2) return rc;
     variant = kConvTap;
   }
@@ -1263,8 +1268,9 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                   const void* bias, int relu, bool allow_slab = true) {
   if (view_parity.size() != 1) allow_slab = false;
   auto run_one = [&](int variant) -> int {
-    if (c->epi.pool && variant == kConvCols) {
-      const int rc = try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true);
+    if (c->epi.pool && (variant == kConvCols || variant == kConvColsPair)) {
+      const int rc = try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, true,
+                                   variant == kConvColsPair);
       if (rc != 2) return rc;
       variant = kConvSlab;
     }
@@ -1312,8 +1318,9 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
         cdiv(cdiv(Wt, t.wt) * cdiv(Ht, t.th) * cdiv(a.N, t.nb), 2) * cdiv(a.n_out, bn) * a.groups >= c->num_sms / 4)
       cand[ncand++] = kConvTapPair;
   }
-  if (allow_slab && try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, false) == 0)
-    cand[ncand++] = kConvCols;
+  for (int v = kConvCols; allow_slab && v <= kConvColsPair; ++v)
+    if (try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, false, v == kConvColsPair) == 0)
+      cand[ncand++] = v;
   if (allow_slab) {
     int eh[2] = {0, 0}, ew[2] = {0, 0};
     for (size_t i = 0; i < taps_in.size(); ++i) {
@@ -1769,7 +1776,7 @@ int dgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* w, const v
       // 64 -> 3 7x7 at 224x224, float16, 256 images 415 -> 143 us, one 13.3 -> 6.7; 32 -> 3 4x4 at 64x64, 2 images 10.1 -> 6.2; float32 688 -> 248,
       // 17.1 -> 7.6 and 10.9 -> 6.0: of nine such layers in both types the columns kernel was slower on none.
       if (d.sH == 2 && d.sW == 2 && out_nhwc && Cp * es == 16 && !(flags & B200CONV_NO_SLAB)) {
-        rc = try_conv_cols(c, a, utaps, 0, 0, Wq, Hq, dx, 0, 1, 0, 0, 0, nullptr, 0, true, d.C, d.H, d.W);
+        rc = try_conv_cols(c, a, utaps, 0, 0, Wq, Hq, dx, 0, 1, 0, 0, 0, nullptr, 0, true, false, d.C, d.H, d.W);
         if (rc == 0) c->last_algo = "umma";
         if (rc != 2) return rc;
       }

@@ -12,7 +12,9 @@
 // Measured (a B200, filters packed, slab kernel -> columns): 3x3 on 8 groups of 32 channels at 28x28, 256 images, float32 144 -> 97 us (67 without
 // the epilogue, HBM 63); 32 -> 32 at 112x112, 64 images 70 -> 49; float16 64 -> 32 at 112x112 100 -> 40; 5x5 64 -> 16 at 56x56, 256 images
 // 134 -> 46.  64 filters: float16 at 56x56, 256 images 73 -> 75, float32 at 224x224, 16 images 140 -> 133 (pairs of the slab kernel 136): an MMA
-// of 192 columns runs at its rate, but 72 KB of filters per 112 pixels come from L2.
+// of 192 columns runs at its rate, but 72 KB of filters per 112 pixels come from L2.  On pairs (PAIR: two pixel tiles, M = 256, each CTA
+// loading 32 of the 64 filters) 128 -> 64 at 112x112, 64 images, float32 247 -> 197 (columns on single CTAs 243, slab pairs 225 to 247; 149 if the
+// activations came for nothing: three slabs of 24 KB in flight beside two filter stages of 36 KB), 64 -> 64 at 224x224 127, float16 80.
 //
 // Warp roles (640 threads): warp 0 streams slabs (tile and halo, 128 bytes of channels per pixel), warp 19 filter rows, warps 1
 // and 18 issue the MMAs of one accumulator each, 16 epilogue warps (TMEM -> shuffles -> staged TMA stores, with 2x2 max pooling,
@@ -42,35 +44,41 @@ struct alignas(16) Bars {
   volatile int abort;
 };
 
-// Tile: one image's rows h0 .. h0 + th - 1, columns w0 .. w0 + wt - 1, of group g.
+// Tile: one image's rows h0 .. h0 + th - 1, columns w0 .. w0 + wt - 1, of group g.  A pair's CTAs take two neighbouring ones (the second of an
+// odd count's last pair lies behind the last image: its loads read zeros and its stores are left out).
 struct Tile { int g, w0, h0, n; };
-__device__ __forceinline__ Tile tile_of(const ColsConvParams& p, uint32_t t) {
-  const uint32_t pt = quotient(t, p.by_groups), row = quotient(pt, p.by_tiles_w), n = quotient(row, p.by_tiles_h);
-  return Tile{static_cast<int>(t - pt * p.groups), static_cast<int>(pt - row * p.tiles_w) * p.wt, static_cast<int>(row - n * p.tiles_h) * p.th, static_cast<int>(n)};
+template <bool PAIR>
+__device__ __forceinline__ Tile tile_of(const ColsConvParams& p, uint32_t t, uint32_t rank) {
+  const uint32_t gt = quotient(t, p.by_groups), pt = PAIR ? 2 * gt + rank : gt, row = quotient(pt, p.by_tiles_w), n = quotient(row, p.by_tiles_h);
+  return Tile{static_cast<int>(t - gt * p.groups), static_cast<int>(pt - row * p.tiles_w) * p.wt, static_cast<int>(row - n * p.tiles_h) * p.th, static_cast<int>(n)};
 }
 
 struct IssueLoop {
   const ColsConvParams& p;
   Bars* bars;
   uint32_t slab0, ring0, tmem;          // low descriptor words of the rings, accumulator a of set 0
-  uint32_t total;
+  uint32_t first, stride, total;
   bool leader;
 };
 
 // The MMAs of one issuing warp, all its tiles: RPS filter rows per filter stage as straight-line code, all 32 lanes in the loop, one
 // elected lane issues (conv_slab.cu, issue_tiles()).  With a stage per filter row its four MMAs of 128 x 96 took 470 clocks, twice their own time.
-template <MmaKind KIND, int RPS>
+template <MmaKind KIND, int RPS, bool PAIR>
 __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
   constexpr bool kTogether = RPS >= 4;
   const ColsConvParams& p = w.p;
   Bars* bars = w.bars;
   const bool leader = w.leader;
-  const uint32_t n_cols = p.kW * p.bn, idesc = with_columns(instr_desc(KIND == MmaKind::TF32, false, false, 128, 256), n_cols);
+  const uint32_t n_cols = p.kW * p.bn, idesc = with_columns(instr_desc(KIND == MmaKind::TF32, false, false, PAIR ? 256 : 128, 256), n_cols);
+  auto commit = [&](uint64_t* bar) {
+    if (PAIR) umma_commit_pair(bar);
+    else umma_commit(bar);
+  };
   const uint32_t desc_hi = static_cast<uint32_t>(smem_desc(0, 16, 1024) >> 32);
-  const uint32_t slab_units = static_cast<uint32_t>(p.slab_bytes) >> 4, row_units = n_cols * 8, stage_units = RPS * row_units;
+  const uint32_t slab_units = static_cast<uint32_t>(p.slab_bytes) >> 4, row_units = (PAIR ? n_cols / 2 : n_cols) * 8, stage_units = RPS * row_units;
   int sb = 0, bs = 0, buf = 0;
   uint32_t sphase = 0, bphase = 0, aphase = 0, slab_seen = 0, b_seen = 0, acc_seen = 0;
-  for (uint32_t t = blockIdx.x; t < w.total; t += gridDim.x) {
+  for (uint32_t t = w.first; t < w.total; t += w.stride) {
     if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) return false;
     acc_seen = 0;
     tc_fence_after();
@@ -91,8 +99,8 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
           for (int u = 0; u < RPS * 4; ++u) {
             if (u < u0 || u >= u1) continue;
             const uint32_t al = a_lo[u >> 2] + 2 * (u & 3), bl = b_lo + (u >> 2) * row_units + 2 * (u & 3), adds = u ? 1u : more;
-            if (kTogether) umma_words_if<KIND>(leader, acc, al, bl, desc_hi, idesc, adds);
-            else umma_words<KIND>(acc, al, bl, desc_hi, idesc, adds);
+            if (kTogether) umma_words_if<KIND, PAIR>(leader, acc, al, bl, desc_hi, idesc, adds);
+            else umma_words<KIND, PAIR>(acc, al, bl, desc_hi, idesc, adds);
           }
         };
         constexpr int kBefore = RPS > 1 ? RPS * 4 - 4 : 2;
@@ -113,13 +121,13 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
         if (kTogether) part(kBefore, RPS * 4);
         if (leader) {
           if (!kTogether) part(kBefore, RPS * 4);
-          umma_commit(&bars->b_empty[cur]);
+          commit(&bars->b_empty[cur]);
         }
       }
-      if (leader) umma_commit(&bars->slab_empty[sb]);
+      if (leader) commit(&bars->slab_empty[sb]);
       if (++sb == p.s_stages) { sb = 0; sphase ^= 1; }
     }
-    if (leader) umma_commit(&bars->acc_full[buf]);
+    if (leader) commit(&bars->acc_full[buf]);
     if (++buf == p.sets) { buf = 0; aphase ^= 1; }
   }
   return true;
@@ -155,7 +163,7 @@ __device__ __forceinline__ void column_sums(uint32_t col, int step, int dil, int
   for (int j = 2; j < kW; ++j) add_columns<1>(col, step, dil, j, f);
 }
 
-template <MmaKind KIND>
+template <MmaKind KIND, bool PAIR>
 __global__ void __launch_bounds__(kThreads, 1)
 conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
   using OutT = typename std::conditional<KIND == MmaKind::TF32, float, __half>::type;
@@ -164,12 +172,13 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* bring = smem + p.s_stages * p.slab_bytes;
-  const int n_cols = p.kW * p.bn, stage_b = p.rps * n_cols * 128;
+  const int n_cols = p.kW * p.bn, stage_b = p.rps * (PAIR ? n_cols / 2 : n_cols) * 128;      // a pair's CTAs load half of the filters each
   uint8_t* staging = bring + p.b_stages * stage_b;               // a multiple of 1024: bn is a multiple of 16
   Bars* bars = reinterpret_cast<Bars*>(staging + p.stage_nbuf * p.stage_bytes);
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
-  const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.Nimg * p.groups;      // fits 32 bits (the launcher checks)
+  const uint32_t pix_tiles = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.Nimg, total = (PAIR ? (pix_tiles + 1) / 2 : pix_tiles) * p.groups;      // fits 32 bits (the launcher checks)
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0, first = PAIR ? blockIdx.x >> 1 : blockIdx.x, stride = PAIR ? gridDim.x >> 1 : gridDim.x;
   const int issuers = p.n_acc;                                   // 1 or 2
   const int nchunks = p.d2s ? 1 : (p.n_out + p.chunk_ch - 1) / p.chunk_ch;
 
@@ -182,17 +191,23 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     }
     for (int b = 0; b < kMaxSets; ++b) {
       mbar_init(&bars->acc_full[b], issuers);
-      mbar_init(&bars->acc_empty[b], nchunks * 4 * p.n_acc);       // the warps that read a tile
+      mbar_init(&bars->acc_empty[b], PAIR ? 2 * nchunks : nchunks * 4 * p.n_acc);       // the warps that read a tile; a pair: one arrival per CTA and chunk
     }
     bars->abort = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(&bars->tmem_base, 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(&bars->tmem_base, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&bars->tmem_base, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();      // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
   pdl_enter();              // the next kernel may start once this CTA holds its TMEM; nothing global was touched before
@@ -204,13 +219,14 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     int sb = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
-      const Tile w = tile_of(p, t);
+    for (uint32_t t = first; t < total && ok; t += stride) {
+      const Tile w = tile_of<PAIR>(p, t, rank);
       for (int kb = 0; kb < p.kblocks; ++kb) {
         if (!uniform_wait(&bars->slab_empty[sb], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (leader) {
-          mbar_expect_tx(&bars->slab_full[sb], tx);
-          tma_load_5d(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, w.g, w.w0 + p.dw_min, w.h0 + p.dh_min, w.n);
+          if (rank == 0) mbar_expect_tx(&bars->slab_full[sb], PAIR ? 2 * tx : tx);      // both CTAs' bytes
+          if (PAIR) tma_load_5d_pair(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, w.g, w.w0 + p.dw_min, w.h0 + p.dh_min, w.n);
+          else tma_load_5d(smem + sb * p.slab_bytes, &p.view, &bars->slab_full[sb], kb * kBK, w.g, w.w0 + p.dw_min, w.h0 + p.dh_min, w.n);
         }
         if (++sb == p.s_stages) { sb = 0; phase ^= 1; }
       }
@@ -223,14 +239,15 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     int bs = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
+    for (uint32_t t = first; t < total && ok; t += stride) {
       const int g = t % static_cast<uint32_t>(p.groups);
       for (int kb = 0; kb < p.kblocks && ok; ++kb) {
         for (int i = 0; i < p.kH; i += p.rps) {
           if (!uniform_wait(&bars->b_empty[bs], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
           if (leader) {
-            mbar_expect_tx(&bars->b_full[bs], stage_b);
-            tma_load_4d(bring + bs * stage_b, &p.wmap, &bars->b_full[bs], kb * kBK, 0, g, p.row_mat[i]);
+            if (rank == 0) mbar_expect_tx(&bars->b_full[bs], (PAIR ? 2 : 1) * stage_b);
+            if (PAIR) tma_load_4d_pair(bring + bs * stage_b, &p.wmap, &bars->b_full[bs], kb * kBK, static_cast<int>(rank) * (p.bn / 2), g, p.row_mat[i]);
+            else tma_load_4d(bring + bs * stage_b, &p.wmap, &bars->b_full[bs], kb * kBK, 0, g, p.row_mat[i]);
           }
           if (++bs == p.b_stages) { bs = 0; phase ^= 1; }
         }
@@ -240,17 +257,17 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
   } else if (warp == 1 || warp == kSecondIssuer) {
     // Issuer a: accumulator a of every tile, all 32 lanes in the loop, one elected lane issues (conv_slab.cu).
     const int a = warp == 1 ? 0 : 1;
-    if (a < p.n_acc) {
+    if (rank == 0 && a < p.n_acc) {              // a pair: the even CTA issues for both
       const bool leader = elect_one();
       const uint32_t desc_lo = static_cast<uint32_t>(smem_desc(0, 16, 1024));
-      const IssueLoop w{p, bars, desc_lo + ((smem_u32(smem) + 16384u * a) >> 4), desc_lo + (smem_u32(bring) >> 4), tmem + a * n_cols, total, leader};
+      const IssueLoop w{p, bars, desc_lo + ((smem_u32(smem) + 16384u * a) >> 4), desc_lo + (smem_u32(bring) >> 4), tmem + a * n_cols, first, stride, total, leader};
       bool ok;
       switch (p.rps) {
-        case 2: ok = issue_tiles<KIND, 2>(w); break;
-        case 3: ok = issue_tiles<KIND, 3>(w); break;
-        case 4: ok = issue_tiles<KIND, 4>(w); break;
-        case 5: ok = issue_tiles<KIND, 5>(w); break;
-        default: ok = issue_tiles<KIND, 1>(w); break;
+        case 2: ok = issue_tiles<KIND, 2, PAIR>(w); break;
+        case 3: ok = issue_tiles<KIND, 3, PAIR>(w); break;
+        case 4: ok = issue_tiles<KIND, 4, PAIR>(w); break;
+        case 5: ok = issue_tiles<KIND, 5, PAIR>(w); break;
+        default: ok = issue_tiles<KIND, 1, PAIR>(w); break;
       }
       if (!ok && leader) report_status(p.status, kStatusTimeout);
     }
@@ -271,20 +288,25 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     auto piece_at = [&](int row, int piece) { return row * row_bytes + ((piece ^ ((row >> sw_shift) & sw_mask)) << 4); };
     const int my_row = drow * row_bytes, my_swizzle = (drow >> sw_shift) & sw_mask;
     constexpr int kPieces = 16 * static_cast<int>(sizeof(OutT)) / 16;                             // of 16 channels
-    const int bufs = p.stage_nbuf / (nchunks * p.step), ch = nchunks == 2 ? grp & 1 : 0, first = nchunks == 2 ? grp >> 1 : grp, co0 = ch * p.chunk_ch;
+    const int bufs = p.stage_nbuf / (nchunks * p.step), ch = nchunks == 2 ? grp & 1 : 0, mine = nchunks == 2 ? grp >> 1 : grp, co0 = ch * p.chunk_ch;
     bool ok = true;
-    int buf = first < p.sets ? first : 0, nstore = 0;
+    int buf = mine < p.sets ? mine : 0, nstore = 0;
     uint32_t phase = 0;
-    for (uint32_t t = first < p.step ? blockIdx.x + first * gridDim.x : total; t < total && ok; t += p.step * gridDim.x) {
-      const Tile w = tile_of(p, t);
+    for (uint32_t t = mine < p.step ? first + mine * stride : total; t < total && ok; t += p.step * stride) {
+      const Tile w = tile_of<PAIR>(p, t, rank);
       if (!warp_wait_or_abort(&bars->acc_full[buf], phase, bars, lane, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
       const uint32_t acc0 = tmem + (buf * p.n_acc + a) * n_cols + p.col_first + (static_cast<uint32_t>(quad * 32) << 16);
       // the accumulator goes back as soon as its last columns are in registers
       auto release = [&] {
         tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);
+        if (PAIR) {
+          named_barrier(5 + grp, gthreads);
+          if (issuer) mbar_arrive_leader(&bars->acc_empty[buf]);
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->acc_empty[buf]);
+        }
       };
       if (p.d2s) {
         // classes of a stride-2 gradInputs: filter cls * C + c is channel c of the pixel (2 h + cls / 2, 2 w + cls % 2), whose stored channels
@@ -332,7 +354,7 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
 #pragma unroll 1
           for (int c = 0; c < p.chunk_ch; c += 16) {
             float f[16];
-            column_sums(acc0 + co0 + c, p.col_step, p.dil, p.kW, f);
+            column_sums(acc0 + ch * p.chunk_step + c, p.col_step, p.dil, p.kW, f);
             if (c + 16 >= p.chunk_ch) release();
             if (p.n_real - co0 - c < 16) {
 #pragma unroll
@@ -410,7 +432,7 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
           }
           fence_async_smem();
           named_barrier(1 + grp, gthreads);
-          if (issuer && B200_IN_RANGE(w.w0 >= 0 && w.h0 >= 0 && w.w0 < p.Wt && w.h0 < p.Ht && w.n < p.Nimg && co0 < p.n_out, p.status)) {
+          if (issuer && (!PAIR || w.n < p.Nimg) && B200_IN_RANGE(w.w0 >= 0 && w.h0 >= 0 && w.w0 < p.Wt && w.h0 < p.Ht && w.n < p.Nimg && co0 < p.n_out, p.status)) {
             if (p.epi.pool) tma_store_4d(&p.out_map, stg, w.g * p.n_out + co0, w.w0 >> 1, w.h0 >> 1, w.n);
             else tma_store_4d(&p.out_map, stg, w.g * p.n_out + co0, w.w0, w.h0, w.n);
             bulk_commit();
@@ -427,30 +449,35 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
   tc_fence_before();
   __syncthreads();
   if (bars->abort) abort_grace(p.wait_clocks);
+  if (PAIR) cluster_sync_all();              // no CTA of the pair leaves (or frees TMEM) while the other may still signal it
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    if (PAIR) tmem_dealloc_pair(tmem, 512);
+    else tmem_dealloc(tmem, 512);
   }
 }
 
-template <MmaKind KIND>
+template <MmaKind KIND, bool PAIR>
 cudaError_t launch_one(const ColsConvParams& p, long long total, int num_sms, cudaStream_t s) {
   static PerDeviceOnce configured;
-  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(conv_cols_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
+  cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(conv_cols_kernel<KIND, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
   if (e != cudaSuccess) return e;
-  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.rps * p.kW * p.bn * 128 + p.stage_nbuf * p.stage_bytes + static_cast<int>(sizeof(Bars)) + 1024;
-  launch_chained(conv_cols_kernel<KIND>, static_cast<int>(total < num_sms ? total : num_sms), kThreads, smem, s, p);
+  const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.rps * p.kW * (PAIR ? p.bn / 2 : p.bn) * 128 + p.stage_nbuf * p.stage_bytes + static_cast<int>(sizeof(Bars)) + 1024;
+  const int units = PAIR ? num_sms / 2 : num_sms, grid = static_cast<int>(total < units ? total : units) * (PAIR ? 2 : 1);
+  launch_linked(true, conv_cols_kernel<KIND, PAIR>, grid, kThreads, smem, s, PAIR ? 2 : 1, p);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_conv_cols(const ColsConvParams& p, int dtype, int num_sms, cudaStream_t s) {
-  const long long total = 1LL * p.tiles_w * p.tiles_h * p.Nimg * p.groups;
+  const long long pix_tiles = 1LL * p.tiles_w * p.tiles_h * p.Nimg, total = (p.pair ? (pix_tiles + 1) / 2 : pix_tiles) * p.groups;
   if (total == 0) return cudaSuccess;
+  if (p.pair && (p.bn != 64 || p.d2s || p.n_acc != 1 || num_sms < 2)) return cudaErrorInvalidValue;
   if (total >= (1LL << 31) || p.n_acc < 1 || p.n_acc > 2 || p.sets < 2 || p.sets > kMaxSets || (p.step != p.sets && (p.step != 1 || p.sets != 2)) || p.sets * p.n_acc * p.kW * p.bn > 512 || p.kH > kMaxColTaps || p.rps < 1 || p.kH % p.rps || p.kW > kMaxColTaps ||
       p.s_stages < 2 || p.s_stages > kMaxStages || p.b_stages < 2 || p.b_stages > kMaxStages) return cudaErrorInvalidValue;
-  return dtype == B200CONV_F16 ? launch_one<MmaKind::F16>(p, total, num_sms, s) : launch_one<MmaKind::TF32>(p, total, num_sms, s);
+  if (p.pair) return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, true>(p, total, num_sms, s) : launch_one<MmaKind::TF32, true>(p, total, num_sms, s);
+  return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, false>(p, total, num_sms, s) : launch_one<MmaKind::TF32, false>(p, total, num_sms, s);
 }
 
 }  // namespace b200

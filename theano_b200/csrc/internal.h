@@ -252,6 +252,8 @@ struct alignas(64) ColsConvParams {
   int slab_bytes, s_stages, b_stages;
   int rps;                       // filter rows per filter stage (a divisor of kH)
   int n_out, n_real;             // output channels per group as stored / with filters
+  int pair;                      // 1: CTA pairs (two pixel tiles side by side, M = 256; 64 columns per filter column, 32 of them per CTA)
+  int chunk_step;                // accumulator columns from one chunk to the next
   int chunk_ch;                  // channels of a staged row: 16 or 32
   int stage_bytes, stage_nbuf;   // staging buffers (one or two per group of epilogue warps)
   int d2s, d2s_C, d2s_H, d2s_W;  // 1: the filters are the four classes of a stride-2 gradInputs with d2s_C channels, `out` the H x W gradient itself
