@@ -807,6 +807,7 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       q.kblocks = (int)kblocks_n;
       q.tiles_pix = (int)cdiv(Wt, 256);
       q.tiles_co = (int)cdiv(a.n_out, 256);
+      q.by_tiles_co = divisor(q.tiles_co);
       q.pixels = Wt; q.n_out = a.n_out; q.n_real = a.w_rows;
       q.stages = 5;
       q.bias = bias; q.relu = relu; q.epi = c->epi;
@@ -929,10 +930,12 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     ++p.ntaps;
   }
   p.kblocks = (int)cdiv(a.Cin_g, kBK);
+  p.tap_groups = (int)cdiv(p.ntaps, tps);
   p.groups = a.groups;
   p.Wt = Wt; p.Ht = Ht; p.Nimg = a.N;
   p.tiles_w = (int)cdiv(Wt, p.wt); p.tiles_h = (int)cdiv(Ht, p.th); p.tiles_n = (int)cdiv(a.N, p.nb);
   p.tiles_co = tiles_co;
+  p.walk = tile_walk(p.splits, p.tiles_co, p.groups, p.tiles_w, p.tiles_h);
   p.n_out = a.n_out;
   p.n_real = a.w_rows;
   p.out = out; p.bias = bias;
@@ -1144,6 +1147,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.tiles_h = static_cast<int>(cdiv(Ht, p.bh));
   p.tiles_n = static_cast<int>(cdiv(a.N, p.bn));
   p.tiles_co = static_cast<int>(cdiv(a.n_out, BN));
+  p.walk = tile_walk(p.splits, p.tiles_co, p.groups, p.tiles_w, p.tiles_h);
   p.n_out = a.n_out;
   p.n_real = a.w_rows;
   p.out = out; p.bias = bias;
@@ -1171,6 +1175,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
       rc = split_output(c, tmp, p, BN, 128, &q, tiles - cut.whole, p.whole);
       if (rc && rc != B200CONV_E_NOMEM) return rc;
       if (rc) { p.whole = (int)tiles; p.splits = 1; }             // no memory for the slices: whole reductions need none
+      p.walk.splits = divisor(p.splits);
       q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
     }
     c->last_variant = p.splits > 1 ? "tap pair cut" : "tap pair";

@@ -47,7 +47,7 @@ struct alignas(16) Bars {
 struct Item { uint32_t tile, k0, k1; int slice; };
 __device__ __forceinline__ Item item_of(const UmmaConvParams& p, uint32_t item, uint32_t kiters) {
   if (item < static_cast<uint32_t>(p.whole)) return Item{item, 0, kiters, -1};
-  const uint32_t r = item - p.whole, splits = p.splits, t = r / splits, s = r - t * splits;
+  const uint32_t r = item - p.whole, splits = p.splits, t = quotient(r, p.walk.splits), s = r - t * splits;
   return Item{p.whole + t, kiters * s / splits, kiters * (s + 1) / splits, static_cast<int>(s)};
 }
 
@@ -110,15 +110,12 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
     bool ok = true;
     for (uint32_t item = first; item < total && ok; item += stride) {
       const Item w = item_of(p, item, kiters);
-      const int co_t = w.tile % static_cast<uint32_t>(p.tiles_co);
-      const int g = (w.tile / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = w.tile / co_groups * 2 + rank;         // behind the last tile of an odd count: an image that is not there, zeros
-      const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.bw;
-      const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.bh;
-      const int n0 = (pt / tiles_wh) * p.bn;
+      const TileAt at = tile_at<true>(p.walk, w.tile, rank);     // behind the last tile of an odd count: an image that is not there, zeros
+      const int co_t = at.co_t, g = at.g, w0 = at.w * p.bw, h0 = at.h * p.bh, n0 = at.n * p.bn;
       const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_out, co_t * BN, BN, true) / 2);
       uint32_t k = w.k0;
-      for (int tap = k / p.kblocks, kb = k % p.kblocks; k < w.k1 && ok; ++tap, kb = 0) {
+      const int tap0 = k ? k / p.kblocks : 0;
+      for (int tap = tap0, kb = k - tap0 * p.kblocks; k < w.k1 && ok; ++tap, kb = 0) {
         const ConvTap tp = p.taps[tap];
         for (; kb < p.kblocks && k < w.k1; ++kb, ++k) {
           if (!uniform_wait(&bars->empty[stage], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
@@ -151,7 +148,7 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
         const int buf = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
         uint32_t idesc = kIdesc;
-        if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, w.tile % static_cast<uint32_t>(p.tiles_co) * BN, BN, true));
+        if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, (w.tile - quotient(w.tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, true));
         if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem + buf * BN;
@@ -191,12 +188,8 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
     int it = 0, turn = 0;
     for (uint32_t item = first; item < total && ok; item += stride, ++it) {
       const Item w = item_of(p, item, kiters);
-      const int co_t = w.tile % static_cast<uint32_t>(p.tiles_co);
-      const int g = (w.tile / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = w.tile / co_groups * 2 + rank;
-      const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.bw;
-      const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.bh;
-      const int n0 = (pt / tiles_wh) * p.bn;
+      const TileAt at = tile_at<true>(p.walk, w.tile, rank);
+      const int co_t = at.co_t, g = at.g, w0 = at.w * p.bw, h0 = at.h * p.bh, n0 = at.n * p.bn;
       const int buf = it & 1;
       if (!warp_wait_or_abort(&bars->acc_full[buf], (it >> 1) & 1, bars, lane, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();

@@ -50,7 +50,7 @@ template <> __device__ __forceinline__ void store_out<__half>(__half* p, float v
 // Slice of a tile's reduction: channel blocks kb0..kb1, tap groups from tg0 in the first, up to tg1 in the last (inclusive).
 struct Range { int kb0, kb1, tg0, tg1; };
 __device__ __forceinline__ Range slice_range(const SlabConvParams& p, uint32_t slice) {
-  const uint32_t stages_kb = (p.ntaps + p.tps - 1) / p.tps, stages_all = stages_kb * p.kblocks;
+  const uint32_t stages_kb = p.tap_groups, stages_all = stages_kb * p.kblocks;
   if (p.splits == 1) return Range{0, p.kblocks - 1, 0, static_cast<int>(stages_kb) - 1};
   const uint32_t a = stages_all * slice / p.splits, b = stages_all * (slice + 1) / p.splits - 1;
   return Range{static_cast<int>(a / stages_kb), static_cast<int>(b / stages_kb), static_cast<int>(a % stages_kb), static_cast<int>(b % stages_kb)};
@@ -100,12 +100,13 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
   uint32_t sphase = 0, bphase = 0;
   uint32_t slab_seen = 0, b_seen = 0, acc_seen = 0;  // the next slab / filter stage / accumulator already seen ready (mbar_look)
   for (uint32_t item = w.first; item < w.total; item += w.stride, ++it) {
-    const Range r = slice_range(p, item % static_cast<uint32_t>(p.splits));
+    const uint32_t tile = quotient(item, p.walk.splits);
+    const Range r = slice_range(p, item - tile * p.splits);
     // a constant where the tiles are full, and for 32 columns, whose MMAs take 36 to 40 clocks whatever is left out of them: with a
     // descriptor from a register these took 4 % longer
     uint32_t idesc = kIdesc;
     if (BN > 32 && p.n_out % BN) {
-      const int co_t = p.tiles_co == 1 ? 0 : item / static_cast<uint32_t>(p.splits) % static_cast<uint32_t>(p.tiles_co);
+      const int co_t = tile - quotient(tile, p.walk.tiles_co) * p.tiles_co;
       idesc = with_columns(kIdesc, mma_columns(p.n_out, co_t * BN, BN, PAIR));
     }
     // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
@@ -229,7 +230,6 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
   // Work item = (tile, slice of the reduction), the slices of a tile side by side.  A slice is a range of
   // filter stages (channel block x group of tps taps), in the order the unsplit loop walks them.
   const uint32_t splits = p.splits;
-  const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
   const int ncls = p.ncls;                              // accumulator (a, class q): columns (a * ncls + q) * BN
   const bool dbl = 2 * p.n_acc * ncls * BN <= 512;
   const int issuers = p.n_acc >= 2 ? 2 : 1;
@@ -279,13 +279,10 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     uint32_t sphase = 0;
     bool ok = true;
     for (uint32_t item = first; item < total && ok; item += stride) {
-      const uint32_t t = item / splits;
+      const uint32_t t = quotient(item, p.walk.splits);
       const Range r = slice_range(p, item - t * splits);
-      const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = PAIR ? t / co_groups * 2 + rank : t / co_groups;
-      const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
-      const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.th;
-      const int n0 = (pt / tiles_wh) * p.nb;
+      const TileAt at = tile_at<PAIR>(p.walk, t, rank);
+      const int g = at.g, w0 = at.w * p.wt, h0 = at.h * p.th, n0 = at.n * p.nb;
       for (int kb = r.kb0; kb <= r.kb1; ++kb) {
         if (!uniform_wait(&bars->slab_empty[sb], sphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         if (leader) {
@@ -305,10 +302,10 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     uint32_t bphase = 0;
     bool ok = true;
     for (uint32_t item = first; item < total && ok; item += stride) {
-      const uint32_t t = item / splits;
+      const uint32_t t = quotient(item, p.walk.splits);
       const Range r = slice_range(p, item - t * splits);
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
+      const TileAt at = tile_at<PAIR>(p.walk, t, rank);
+      const int co_t = at.co_t, g = at.g;
       // a pair's CTAs load one half each of what the tile's MMAs take (and rows that those leave out)
       const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_out, co_t * BN, BN, true) / 2);
       auto load = [&](uint8_t* dst, int kb, int mat) {
@@ -371,17 +368,17 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     const int per_img = p.Hs * p.Ws;
     // channels-last output whose 32-channel groups are 16-byte aligned: 16-byte stores
     const bool rowwise = p.out_sc == 1 && ((p.n_out * sizeof(OutT) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
+    // staged TMA stores: this lane's accumulator row, group and staged row (below)
+    const int s_a = p.tma_out ? sub % p.n_acc : 0, s_grp = p.tma_out ? sub / p.n_acc : 0, s_pos = s_a * 128 + quad * 32 + lane;
+    const int s_ni = s_pos / per_img, s_hh = s_pos % per_img / p.Ws, s_ww = s_pos % per_img % p.Ws;
+    const bool s_inbox = s_ni < p.nb && s_hh < p.th && s_ww < p.wt;
+    const int s_bufs = p.tma_out && p.stage_nbuf * p.n_acc / (kEpilogueWarps / 4) >= 2 ? 2 : 1;
     bool ok = true;
     int it = 0;
     int nstore = 0;                              // chunks this warp's group has staged so far
     for (uint32_t item = first; item < total && ok; item += stride, ++it) {
-      const uint32_t t = item / splits;
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = PAIR ? t / co_groups * 2 + rank : t / co_groups;
-      const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.wt;
-      const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.th;
-      const int n0 = (pt / tiles_wh) * p.nb;
+      const TileAt at = tile_at<PAIR>(p.walk, quotient(item, p.walk.splits), rank);
+      const int co_t = at.co_t, g = at.g, w0 = at.w * p.wt, h0 = at.h * p.th, n0 = at.n * p.nb;
       const int buf = dbl ? (it & 1) : 0;
       const uint32_t aphase = dbl ? ((it >> 1) & 1) : (it & 1);
       if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
@@ -418,16 +415,13 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
         // `bufs` staging buffers and fills them in turn; before a buffer is refilled only the
         // store that last read it must have finished reading, so a store runs beside the next
         // chunk's (or the next tile's) TMEM reads instead of being waited for.
-        const int a = sub % p.n_acc, grp = sub / p.n_acc, ngrp = (kEpilogueWarps / 4) / p.n_acc;
+        const int a = s_a, grp = s_grp, ngrp = (kEpilogueWarps / 4) >> (p.n_acc >> 1);       // n_acc is 1, 2 or 4
         const int gthreads = 128 * p.n_acc;
-        const int pos = a * 128 + quad * 32 + lane;
-        const int ni = pos / per_img, rem = pos % per_img;
-        const int hh = rem / p.Ws, ww = rem % p.Ws;
-        const bool inbox = ni < p.nb && hh < p.th && ww < p.wt;
-        const int drow = (ni * p.th + hh) * p.wt + ww;
+        const bool inbox = s_inbox;
+        const int drow = (s_ni * p.th + s_hh) * p.wt + s_ww;
         const bool issuer = a == 0 && quad == 0 && lane == 0;   // issues all of the group's stores
         const bool plain = p.epi.alpha == 1.f && !p.bias && !p.relu;
-        const int bufs = p.stage_nbuf / ngrp >= 2 ? 2 : 1;
+        const int bufs = s_bufs;
         constexpr int kCh = 128 / static_cast<int>(sizeof(OutT));   // channels of one 128-byte staged row
         const int nstaged = min(BN / kCh, (p.n_out - co_base + kCh - 1) / kCh);
         for (int cc = grp; cc < nstaged * ncls; cc += ngrp, ++nstore) {

@@ -83,7 +83,6 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
   // role about a thousand clocks, a fifth of a small tile
   const uint32_t total = static_cast<uint32_t>(p.tiles_w) * p.tiles_h * p.tiles_n * p.groups * p.tiles_co * p.splits;
   const uint32_t splits = p.splits;            // work item = (tile, slice of the reduction), slices of a tile side by side
-  const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -124,16 +123,13 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     uint32_t phase = 0, idx = 0;
     bool ok = true;
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x) {
-      const uint32_t t = item / splits, slice = item - t * splits;
-      const uint32_t k0 = kiters * slice / splits, k1 = kiters * (slice + 1) / splits;
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = t / co_groups;
-      const int w0 = (pt % static_cast<uint32_t>(p.tiles_w)) * p.bw;
-      const int h0 = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.bh;
-      const int n0 = (pt / tiles_wh) * p.bn;
+      const uint32_t t = quotient(item, p.walk.splits), slice = item - t * splits;
+      const uint32_t k0 = splits == 1 ? 0 : kiters * slice / splits, k1 = splits == 1 ? kiters : kiters * (slice + 1) / splits;
+      const TileAt at = tile_at(p.walk, t);
+      const int co_t = at.co_t, g = at.g, w0 = at.w * p.bw, h0 = at.h * p.bh, n0 = at.n * p.bn;
       uint32_t k = k0;
-      for (int tap = k0 / p.kblocks, kb = k0 % p.kblocks; k < k1 && ok; ++tap, kb = 0) {
+      const int tap0 = k0 ? k0 / p.kblocks : 0;
+      for (int tap = tap0, kb = k0 - tap0 * p.kblocks; k < k1 && ok; ++tap, kb = 0) {
         const ConvTap tp = p.taps[tap];
         for (; kb < p.kblocks && k < k1; ++kb, ++idx, ++k) {
           if ((idx & 1) == my_parity) {
@@ -166,14 +162,15 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const uint32_t lo_base = static_cast<uint32_t>(desc_bits) + (smem_u32(smem) >> 4);
     uint32_t seen = 0, acc_seen = 0;             // next stage / next accumulator already seen ready (mbar_look)
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
-      const uint32_t slice = item % splits, k0 = kiters * slice / splits, k1 = kiters * (slice + 1) / splits;
+      const uint32_t tile = quotient(item, p.walk.splits), slice = item - tile * splits;
+      const uint32_t k0 = splits == 1 ? 0 : kiters * slice / splits, k1 = splits == 1 ? kiters : kiters * (slice + 1) / splits;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem + buf * BN;
       uint32_t idesc = kIdesc;
-      if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, p.tiles_co == 1 ? 0 : item / splits % static_cast<uint32_t>(p.tiles_co) * BN, BN, false));
+      if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, (tile - quotient(tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, false));
       for (uint32_t k = k0; k < k1; ++k) {
         if (!wait_seen(seen, &bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
@@ -214,15 +211,10 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     bool ok = true;
     int it = 0;
     for (uint32_t item = blockIdx.x; item < total && ok; item += gridDim.x, ++it) {
-      const uint32_t t = item / splits;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int g = (t / static_cast<uint32_t>(p.tiles_co)) % static_cast<uint32_t>(p.groups);
-      const uint32_t pt = t / co_groups;
-      const int w = (pt % static_cast<uint32_t>(p.tiles_w)) * p.bw + rw;
-      const int h = ((pt / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h)) * p.bh + rh;
-      const int n = (pt / tiles_wh) * p.bn + rn;
+      const TileAt at = tile_at(p.walk, quotient(item, p.walk.splits));
+      const int co_t = at.co_t, g = at.g, w = at.w * p.bw + rw, h = at.h * p.bh + rh, n = at.n * p.bn + rn;
       const bool valid = row < rows_used && w < p.Wt && h < p.Ht && n < p.Nimg;
       if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
       tc_fence_after();

@@ -85,8 +85,8 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
     uint32_t phase = 0;
     bool ok = true;
     for (uint32_t t = pair; t < total && ok; t += npairs) {
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int pix0 = (t / static_cast<uint32_t>(p.tiles_co)) * 256 + rank * 128;
+      const uint32_t pt = quotient(t, p.by_tiles_co);
+      const int co_t = t - pt * p.tiles_co, pix0 = pt * 256 + rank * 128;
       for (int kb = 0; kb < p.kblocks; ++kb) {
         if (!uniform_wait(&bars->empty[stage], phase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         uint8_t* sa = smem + stage * kStageBytes;
@@ -144,8 +144,8 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
     bool ok = true;
     int it = 0, nstore = 0;
     for (uint32_t t = pair; t < total && ok; t += npairs, ++it) {
-      const int co_t = t % static_cast<uint32_t>(p.tiles_co);
-      const int pix0 = (t / static_cast<uint32_t>(p.tiles_co)) * 256 + rank * 128;
+      const uint32_t pt = quotient(t, p.by_tiles_co);
+      const int co_t = t - pt * p.tiles_co, pix0 = pt * 256 + rank * 128;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
       if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }

@@ -92,6 +92,24 @@ inline Divisor divisor(uint32_t d) {
 __device__ __forceinline__ uint32_t quotient(uint32_t n, const Divisor& v) { return (__umulhi(n, v.mul) + n) >> v.shift; }
 #endif
 
+// How the convolution kernels walk their work items: (pixel tile, group, filter tile, slice of the reduction), the slice fastest.  Every
+// role finds its place with these quotients once per tile; divided out, they cost a warp of the epilogue 2000 clocks, more than reading
+// the accumulators of a 256 x 64 tile out and storing them (a B200: 64 -> 256 1x1 at 56x56, float16, 256 images 107 -> 95 us, 64 -> 64 48 -> 37;
+// 3 -> 64 3x3 at 224x224, float32, 64 images 268 -> 202; 3 -> 64 7x7 stride 2 at 224x224, float16, 256 images 243 -> 194).
+struct TileWalk { Divisor splits, tiles_co, groups, tiles_w, tiles_h; };
+inline TileWalk tile_walk(int splits, int tiles_co, int groups, int tiles_w, int tiles_h) {
+  return TileWalk{divisor(splits), divisor(tiles_co), divisor(groups), divisor(tiles_w), divisor(tiles_h)};
+}
+#ifdef __CUDACC__
+struct TileAt { int co_t, g, w, h, n; };         // filter tile, group, pixel tile
+template <bool PAIR = false> __device__ __forceinline__ TileAt tile_at(const TileWalk& k, uint32_t tile, uint32_t rank = 0) {
+  const uint32_t tg = quotient(tile, k.tiles_co), tp = quotient(tg, k.groups), pt = PAIR ? 2 * tp + rank : tp;
+  const uint32_t row = quotient(pt, k.tiles_w), n = quotient(row, k.tiles_h);
+  return TileAt{static_cast<int>(tile - tg * k.tiles_co.d), static_cast<int>(tg - tp * k.groups.d), static_cast<int>(pt - row * k.tiles_w.d),
+                static_cast<int>(row - n * k.tiles_h.d), static_cast<int>(n)};
+}
+#endif
+
 // Codes a kernel writes to the device status word when it gives up.
 enum : int { kStatusOk = 0, kStatusTimeout = 1, kStatusBadIndex = 2 };
 
@@ -131,6 +149,7 @@ struct alignas(64) UmmaConvParams {
   int Wt, Ht, Nimg;              // extent of the output pixel grid this launch covers
   int bw, bh, bn;                // pixel tile (bw*bh*bn <= 128 rows of the accumulator)
   int tiles_w, tiles_h, tiles_n, tiles_co;
+  TileWalk walk;
   int n_out;                     // output channels per group as stored
   int n_real;                    // of these, the ones with filters: the pad channels behind them are stored as 0
   void* out;
@@ -192,6 +211,7 @@ struct alignas(64) SlabConvParams {
   int Ws, Hs;                    // slab columns / rows per image (tile + halo)
   int dw_min, dh_min;            // view coordinate of slab column / row 0 relative to the tile origin
   int tiles_w, tiles_h, tiles_n, tiles_co;
+  TileWalk walk;
   int n_acc;                     // 128-row accumulators in use (<= 512 / BN)
   int slab_bytes;                // bytes of one slab buffer (1024-byte multiple)
   int b_stages;                  // filter-tile ring depth
@@ -203,6 +223,7 @@ struct alignas(64) SlabConvParams {
   int tap_boxes;                 // 1: one TMA box per tap; 0: the taps of a stage are neighbours in the packed filters
                                  // and arrive as one box (the map's box then is tps matrices deep)
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
+  int tap_groups;                // stages of a channel block: ceil(ntaps / tps)
   int n_out, n_real;             // output channels per group as stored / with filters
   void* out;
   const void* bias;
@@ -295,6 +316,7 @@ struct alignas(64) PairGemmParams {
   CUtensorMap out_map;           // 4-D (channel, pixel, 1, 1) over the output, box (64, 128, 1, 1)
   int kblocks;                   // ceil(channels / 64)
   int tiles_pix, tiles_co;       // 256-pixel tiles, 256-filter tiles
+  Divisor by_tiles_co;
   int pixels, n_out, n_real;
   int stages;                    // ring depth (2 .. 5)
   const void* bias;
