@@ -151,21 +151,24 @@ __global__ void __launch_bounds__(kPackThreads) pack_filters_batch_kernel(const 
   pack_job_block<T>(b.jobs[j], blockIdx.x - b.jobs[j].first_block);
 }
 
+// idx / d: a multiplication for 32-bit indices; those of more than 2^31 elements are divided.
+__device__ __forceinline__ uint32_t over(uint32_t idx, const Divisor& d) { return quotient(idx, d); }
+__device__ __forceinline__ long long over(long long idx, const Divisor& d) { return idx / d.d; }
+constexpr long long kIndex32 = 1LL << 31;
+
 // Few-channel layers ("row folding"): the image is copied channels-last with explicit zero
 // columns left and right, [N][H][Wp][Cp], so that the kW * Cp values under one filter row are
 // contiguous and can serve as one reduction block of the implicit GEMM.  One thread per output
 // pixel; src is NCHW (nhwc_in = 0), channels-last [N][H][W][Cp] (1) or that off the 16-byte boundaries (2).
-template <typename T>
-__global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int C, int H,
-                                int W, int Cp, int Wp, int pad_l, int nhwc_in) {
+template <typename T, typename Index>
+__global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, Index total, Divisor by_H, Divisor by_Wp, int C,
+                                int W, int Cp, int pad_l, int nhwc_in) {
   pdl_enter();
-  const long long total = 1LL * N * H * Wp;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int wp = idx % Wp;
-    const int h = (idx / Wp) % H;
-    const int n = idx / (1LL * Wp * H);
-    const int w = wp - pad_l;
+  const int H = by_H.d;
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const Index row = over(idx, by_Wp);
+    const int n = static_cast<int>(over(row, by_H)), h = static_cast<int>(row - static_cast<Index>(n) * H);
+    const int w = static_cast<int>(idx - row * by_Wp.d) - pad_l;
     const bool inside = w >= 0 && w < W;
     if (Cp * sizeof(T) == 16) {
       // one pixel is 16 bytes: assemble it in registers, store it once
@@ -179,10 +182,10 @@ __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, 
             v[c] = nhwc_in ? src[((1LL * n * H + h) * W + w) * Cp + c] : src[((1LL * n * C + c) * H + h) * W + w];
         }
       }
-      *reinterpret_cast<uint4*>(dst + idx * Cp) = px;
+      *reinterpret_cast<uint4*>(dst + 1LL * idx * Cp) = px;
       continue;
     }
-    T* d = dst + idx * Cp;
+    T* d = dst + 1LL * idx * Cp;
     for (int c = 0; c < Cp; ++c) {
       T v = T(0);
       if (inside && c < C)
@@ -194,16 +197,14 @@ __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, 
 
 // Folded filters: dst[i][k][j*Cp + c] = w[k][c][i'][j'] (zero elsewhere up to ld columns), where
 // (i', j') = (i, j) or the flipped position.
-template <typename T>
+template <typename T, typename Index>
 __global__ void pack_filters_fold_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C,
                                          int kH, int kW, int Cp, int ld, int flip) {
   pdl_enter();
-  const long long total = 1LL * kH * K * ld;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int col = idx % ld;
-    const int k = (idx / ld) % K;
-    const int i = idx / (1LL * ld * K);
+  const Index total = static_cast<Index>(kH) * K * ld;
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const Index row = idx / ld;
+    const int col = static_cast<int>(idx - row * ld), i = static_cast<int>(row / K), k = static_cast<int>(row - static_cast<Index>(i) * K);
     const int j = col / Cp, c = col % Cp;
     T v = T(0);
     if (j < kW && c < C) {
@@ -221,16 +222,13 @@ __global__ void pack_filters_fold_kernel(const T* __restrict__ w, T* __restrict_
 // dst whose filter rows span a few consecutive pixels: one contiguous reduction block per row.
 // One thread per dst pixel; src is NCHW (nhwc_in = 0), channels-last [N][H][W][Cp_in] (1) or that off the 16-byte
 // boundaries (2).
-template <typename T, int C>
-__global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, int N, int H,
-                               int W, int Cp_in, int H2, int Wq, int q0, int nhwc_in) {
+template <typename T, int C, typename Index>
+__global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, Index total, Divisor by_H2, Divisor by_Wq, int H,
+                               int W, int Cp_in, int q0, int nhwc_in) {
   pdl_enter();
-  const long long total = 1LL * N * H2 * Wq;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int q = idx % Wq;
-    const int h2 = (idx / Wq) % H2;
-    const int n = idx / (1LL * Wq * H2);
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const Index row = over(idx, by_Wq);
+    const int n = static_cast<int>(over(row, by_H2)), h2 = static_cast<int>(row - static_cast<Index>(n) * by_H2.d), q = static_cast<int>(idx - row * by_Wq.d);
     __align__(16) T v[kS2dChannels];
 #pragma unroll
     for (int i = 0; i < kS2dChannels; ++i) v[i] = T(0);
@@ -251,7 +249,7 @@ __global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, i
         }
       }
     }
-    uint4* d = reinterpret_cast<uint4*>(dst + idx * kS2dChannels);
+    uint4* d = reinterpret_cast<uint4*>(dst + 1LL * idx * kS2dChannels);
     const uint4* sv = reinterpret_cast<const uint4*>(v);
 #pragma unroll
     for (int i = 0; i < (int)(kS2dChannels * sizeof(T) / 16); ++i) d[i] = sv[i];
@@ -262,17 +260,15 @@ __global__ void pad_s2d_kernel(const T* __restrict__ src, T* __restrict__ dst, i
 // element that multiplies input pixel (2*(t + t0) + dy, 2*(j + q0) + dx) relative to the output
 // position times the stride, i.e. tap (i, jj) = (2*(t + t0) + dy + padH, 2*(j + q0) + dx + padW);
 // zero where that tap does not exist.
-template <typename T>
+template <typename T, typename Index>
 __global__ void pack_filters_s2d_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C,
                                         int kH, int kW, int ntaps, int t0, int q0, int padH, int padW,
                                         int ld, int flip) {
   pdl_enter();
-  const long long total = 1LL * ntaps * K * ld;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int col = idx % ld;
-    const int k = (idx / ld) % K;
-    const int t = idx / (1LL * ld * K);
+  const Index total = static_cast<Index>(ntaps) * K * ld;
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const Index row = idx / ld;
+    const int col = static_cast<int>(idx - row * ld), t = static_cast<int>(row / K), k = static_cast<int>(row - static_cast<Index>(t) * K);
     const int j = col / kS2dChannels, r = col % kS2dChannels;
     T v = T(0);
     if (r < 4 * C) {
@@ -537,16 +533,14 @@ __global__ void __launch_bounds__(256) maxpool2x2_grad_nhwc_kernel(const T* __re
       *reinterpret_cast<P*>(gx + base + (k & 1) * Cp + (k >> 1) * W * Cp) = r[k];
 }
 
-template <typename T>
+template <typename T, typename Index>
 __global__ void pack_filters_merged_kernel(const T* __restrict__ w, T* __restrict__ dst, int K, int C, int kH,
                                            int kW, int flip, MergedTapTable tb, int nu, int ncls, int rows, int ldw) {
   pdl_enter();
-  const long long total = 1LL * nu * rows * ldw;
-  for (long long idx = blockIdx.x * 1LL * blockDim.x + threadIdx.x; idx < total;
-       idx += 1LL * gridDim.x * blockDim.x) {
-    const int kf = idx % ldw;
-    const int row = (idx / ldw) % rows;
-    const int u = idx / (1LL * ldw * rows);
+  const Index total = static_cast<Index>(nu) * rows * ldw;
+  for (Index idx = blockIdx.x * static_cast<Index>(blockDim.x) + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const Index ur = idx / ldw;
+    const int kf = static_cast<int>(idx - ur * ldw), u = static_cast<int>(ur / rows), row = static_cast<int>(ur - static_cast<Index>(u) * rows);
     const int cls = row / C, c = row % C;
     const int tap = cls < ncls ? tb.src[u][cls] : -1;     // rows past ncls * C are zero padding
     T v = T(0);
@@ -682,12 +676,17 @@ cudaError_t launch_pad_fold(const void* src, void* dst, int N, int C, int H, int
   const long long total = 1LL * N * H * Wp;
   if (total == 0) return cudaSuccess;
   nhwc_in = channels_last_form(nhwc_in, src);
-  if (dtype == B200CONV_F16)
-    launch_streaming(pad_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
-        static_cast<const __half*>(src), static_cast<__half*>(dst), N, C, H, W, Cp, Wp, pad_l, nhwc_in);
-  else
-    launch_streaming(pad_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
-        static_cast<const float*>(src), static_cast<float*>(dst), N, C, H, W, Cp, Wp, pad_l, nhwc_in);
+#define B200_FOLD(T, Index) \
+  launch_streaming(pad_fold_kernel<T, Index>, grid_for(total, 256), 256, 0, s, static_cast<const T*>(src), static_cast<T*>(dst), \
+                   static_cast<Index>(total), divisor(H), divisor(Wp), C, W, Cp, pad_l, nhwc_in)
+  if (total < kIndex32) {
+    if (dtype == B200CONV_F16) B200_FOLD(__half, uint32_t);
+    else B200_FOLD(float, uint32_t);
+  } else {
+    if (dtype == B200CONV_F16) B200_FOLD(__half, long long);
+    else B200_FOLD(float, long long);
+  }
+#undef B200_FOLD
   return cudaGetLastError();
 }
 
@@ -696,11 +695,11 @@ cudaError_t launch_pack_filters_fold(const void* w, void* dst, int K, int C, int
   const long long total = 1LL * kH * K * ld;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    launch_chained(pack_filters_fold_kernel<__half>, grid_for(total, 256), 256, 0, s,
-        static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, Cp, ld, flip);
+    total < kIndex32 ? launch_chained(pack_filters_fold_kernel<__half, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, Cp, ld, flip)
+                     : launch_chained(pack_filters_fold_kernel<__half, long long>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, Cp, ld, flip);
   else
-    launch_chained(pack_filters_fold_kernel<float>, grid_for(total, 256), 256, 0, s,
-        static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, Cp, ld, flip);
+    total < kIndex32 ? launch_chained(pack_filters_fold_kernel<float, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, Cp, ld, flip)
+                     : launch_chained(pack_filters_fold_kernel<float, long long>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, Cp, ld, flip);
   return cudaGetLastError();
 }
 
@@ -729,13 +728,21 @@ cudaError_t pad_s2d_typed(const void* src, void* dst, int N, int C, int H, int W
   T* out = static_cast<T*>(dst);
   nhwc_in = channels_last_form(nhwc_in, src);
   const int grid = grid_for(total, 256);
+#define B200_S2D(C)                                                                                                              \
+  case C:                                                                                                                        \
+    if (total < kIndex32)                                                                                                        \
+      launch_streaming(pad_s2d_kernel<T, C, uint32_t>, grid, 256, 0, s, in, out, static_cast<uint32_t>(total), divisor(H2), divisor(Wq), H, W, Cp_in, q0, nhwc_in); \
+    else                                                                                                                         \
+      launch_streaming(pad_s2d_kernel<T, C, long long>, grid, 256, 0, s, in, out, total, divisor(H2), divisor(Wq), H, W, Cp_in, q0, nhwc_in); \
+    break;
   switch (C) {   // the channel count as a constant keeps the assembled pixel in registers
-    case 1: launch_streaming(pad_s2d_kernel<T, 1>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 2: launch_streaming(pad_s2d_kernel<T, 2>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 3: launch_streaming(pad_s2d_kernel<T, 3>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
-    case 4: launch_streaming(pad_s2d_kernel<T, 4>, grid, 256, 0, s, in, out, N, H, W, Cp_in, H2, Wq, q0, nhwc_in); break;
+    B200_S2D(1)
+    B200_S2D(2)
+    B200_S2D(3)
+    B200_S2D(4)
     default: return cudaErrorInvalidValue;
   }
+#undef B200_S2D
   return cudaGetLastError();
 }
 
@@ -752,11 +759,11 @@ cudaError_t launch_pack_filters_s2d(const void* w, void* dst, int K, int C, int 
   const long long total = 1LL * ntaps * K * ld;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    launch_chained(pack_filters_s2d_kernel<__half>, grid_for(total, 256), 256, 0, s,
-        static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
+    total < kIndex32 ? launch_chained(pack_filters_s2d_kernel<__half, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip)
+                     : launch_chained(pack_filters_s2d_kernel<__half, long long>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   else
-    launch_chained(pack_filters_s2d_kernel<float>, grid_for(total, 256), 256, 0, s,
-        static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
+    total < kIndex32 ? launch_chained(pack_filters_s2d_kernel<float, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip)
+                     : launch_chained(pack_filters_s2d_kernel<float, long long>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, ntaps, t0, q0, padH, padW, ld, flip);
   return cudaGetLastError();
 }
 
@@ -885,11 +892,11 @@ cudaError_t launch_pack_filters_merged(const void* w, void* dst, int K, int C, i
   const long long total = 1LL * nu * rows * ldw;
   if (total == 0) return cudaSuccess;
   if (dtype == B200CONV_F16)
-    launch_chained(pack_filters_merged_kernel<__half>, grid_for(total, 256), 256, 0, s,
-        static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
+    total < kIndex32 ? launch_chained(pack_filters_merged_kernel<__half, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw)
+                     : launch_chained(pack_filters_merged_kernel<__half, long long>, grid_for(total, 256), 256, 0, s, static_cast<const __half*>(w), static_cast<__half*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
   else
-    launch_chained(pack_filters_merged_kernel<float>, grid_for(total, 256), 256, 0, s,
-        static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
+    total < kIndex32 ? launch_chained(pack_filters_merged_kernel<float, uint32_t>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw)
+                     : launch_chained(pack_filters_merged_kernel<float, long long>, grid_for(total, 256), 256, 0, s, static_cast<const float*>(w), static_cast<float*>(dst), K, C, kH, kW, flip, tb, nu, ncls, rows, ldw);
   return cudaGetLastError();
 }
 
