@@ -1,0 +1,55 @@
+"""Cut tiles whose slices are added by the CTA that leaves the last one: results repeat bit by bit over calls, graphs and contexts, and the
+counts of arrivals are back at zero after a wait that ran out."""
+import numpy as np
+import pytest
+
+from theano_b200 import shim
+
+pytestmark = pytest.mark.gpu
+T = shim.DeviceTensor
+
+
+def layer(ctx, dtype):
+    c = 256 if dtype == np.float32 else 512
+    rs = np.random.RandomState(11)
+    x = rs.standard_normal((100, c, 14, 14)).astype(dtype)
+    w = (rs.standard_normal((256, c, 3, 3)) / np.sqrt(c * 9)).astype(dtype)
+    X, W, Y = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), T(ctx, (100, 256, 14, 14), dtype, "nhwc")
+    return X, W, Y, lambda: shim.device_conv2d(X, W, border_mode="half", out=Y, flags=shim.NO_SLAB)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float16], ids=["f32", "f16"])
+def test_repeated_calls_graphs_and_contexts_agree(dtype):
+    first = None
+    for _ in range(2):
+        ctx = shim.Context(0)
+        ctx.set_autotune(False)
+        X, W, Y, call = layer(ctx, dtype)
+        call()
+        assert ctx.last_variant == "tap pair cut"
+        y = Y.to_host()
+        first = y if first is None else first
+        assert np.array_equal(first, y)
+        graph = ctx.capture(lambda: [call() for _ in range(5)])
+        for _ in range(4):
+            ctx.memset(Y.ptr, 255, Y.nbytes)
+            graph.launch()
+        ctx.sync()
+        assert np.array_equal(first, Y.to_host())
+        graph.destroy()
+        ctx.close()
+
+
+def test_counts_start_again_after_a_wait_ran_out():
+    ctx = shim.Context(0)
+    ctx.set_autotune(False)
+    X, W, Y, call = layer(ctx, np.float32)
+    call()
+    y = Y.to_host()
+    ctx.set_wait_limit(2000000)                      # about a millisecond
+    with pytest.raises(shim.B200Error):
+        ctx.selftest_wait()
+    ctx.set_wait_limit(4000000000)
+    call()
+    assert np.array_equal(y, Y.to_host())
+    ctx.close()

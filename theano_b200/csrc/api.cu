@@ -103,6 +103,7 @@ struct b200conv_ctx {
   std::mutex mu;
   std::string err;
   int* d_status = nullptr;  // status word of the kernels: h_status as the device sees it
+  unsigned int* d_arrivals = nullptr;   // counts of the slices of cut tiles (conv_pair.cu), zero between launches
   volatile int* h_status = nullptr;  // pinned and mapped: written by kernels only when they give up, so that
                                      // a synchronising call reads it without a transfer
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -295,11 +296,14 @@ struct Scratch {
   }
 };
 
+constexpr int kArrivals = 1024;
+
 int check_status(b200conv_ctx* c) {
   // called after a stream synchronisation
   const int st = *c->h_status;
   if (st != kStatusOk) {
     *c->h_status = 0;
+    cudaMemsetAsync(c->d_arrivals, 0, kArrivals * sizeof(unsigned int), c->stream);     // a launch that gave up leaves its counts behind
     if (st == kStatusBadIndex)
       return fail(c, B200CONV_E_CUDA, "a kernel of the range-checked build computed an index outside its buffer "
                   "(the access was skipped); results are invalid");
@@ -715,25 +719,28 @@ SlabTile tap_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int 
   return best;
 }
 
-// How a launch of `tiles` pair tiles on `units` pairs is cut: the tiles beyond whole waves get `splits` pairs each, if that saves more than
-// their raw accumulators and the second kernel cost (split_clocks()).  256 -> 256 3x3 at 14x14, 128 images, float32: 98 tiles on
-// 74 pairs, 24 of them cut in three.
-struct PairCut { long long whole; int splits; };
+// How a launch of `tiles` pair tiles on `units` pairs is cut: those beyond whole waves get `splits` pairs each.  Where whole tiles follow, the
+// slices are added beside their MMAs, at most 8 slices, whose sums take no longer; what remains is the way through memory, some 6000 clocks (512 -> 2048
+// 1x1 at 7x7, which would save 2700, took 32 us cut and 25 whole).  Else the raw
+// accumulators and the second kernel count in full (split_clocks()).  256 -> 256 3x3 at 14x14, 128 images, float32: 98 tiles on 74 pairs, 24 of
+// them cut in three.
+struct PairCut { long long tiles; int splits; };
 PairCut pair_cut(long long tiles, int units, long long kiters, int bn) {
   const long long rest = tiles % units, step = bn >= 256 ? 512 : 340;       // clocks per stage: MMAs, or 24 KB at 73 B/clk
-  const long long most = rest ? std::min<long long>(units / rest, kiters) : 1;
-  if (most < 2) return PairCut{tiles, 1};
-  const long long saved = kiters * step - cdiv(kiters, most) * step, cost = split_clocks(2 * rest * most, 128, bn, 2 * units);
-  return saved > cost + cost / 4 ? PairCut{tiles - rest, (int)most} : PairCut{tiles, 1};
+  const bool beside = tiles > units;
+  const long long most = rest ? std::min<long long>({units / rest, kiters, beside ? 8 : kiters}) : 1;
+  if (most < 2) return PairCut{0, 1};
+  const long long saved = kiters * step - cdiv(kiters, most) * step, cost = beside ? 6400 : split_clocks(2 * rest * most, 128, bn, 2 * units);
+  return saved > cost + cost / 4 ? PairCut{rest, (int)most} : PairCut{0, 1};
 }
 
 // Slabs of a split launch and the parameters of its reduction that both kernels share.
 template <class P>
-int split_output(b200conv_ctx* c, Scratch& tmp, P& p, int bn, int rows, ConvReduceParams* q, long long pair_tiles = 0, int first_tile = 0) {
+int split_output(b200conv_ctx* c, Scratch& tmp, P& p, int bn, int rows, ConvReduceParams* q, long long pair_tiles = 0) {
   memset(q, 0, sizeof *q);
   const long long tiles = pair_tiles ? pair_tiles : 1LL * p.tiles_w * p.tiles_h * p.tiles_n * p.groups * p.tiles_co;
   if (tiles > 65535 / 2) return fail(c, B200CONV_E_INVALID, "too many split tiles");
-  q->first_tile = first_tile; q->tiles = (int)tiles; q->pair = pair_tiles > 0;
+  q->tiles = (int)tiles; q->pair = pair_tiles > 0;
   float* partial;
   const long long elems = (pair_tiles ? 2 : 1) * tiles * p.splits * rows * bn;
   int rc = tmp.get(sizeof(float) * elems, reinterpret_cast<void**>(&partial));
@@ -1168,19 +1175,20 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, kConvTap);
     const PairCut cut = pair_cut(tiles, c->num_sms / 2, 1LL * p.ntaps * p.kblocks, BN);
-    p.whole = (int)cut.whole; p.splits = cut.splits;
+    p.cut = (int)cut.tiles; p.splits = cut.splits;
     Scratch tmp(c);
     ConvReduceParams q;
-    if (cut.splits > 1) {
-      rc = split_output(c, tmp, p, BN, 128, &q, tiles - cut.whole, p.whole);
+    if (p.cut) {
+      rc = split_output(c, tmp, p, BN, 128, &q, cut.tiles);
       if (rc && rc != B200CONV_E_NOMEM) return rc;
-      if (rc) { p.whole = (int)tiles; p.splits = 1; }             // no memory for the slices: whole reductions need none
+      if (rc) { p.cut = 0; p.splits = 1; }                        // no memory for the slices: whole reductions need none
+      if (p.cut < tiles && 2 * p.cut <= kArrivals) p.arrivals = c->d_arrivals;
       p.walk.splits = divisor(p.splits);
       q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
     }
     c->last_variant = p.splits > 1 ? "tap pair cut" : "tap pair";
     KLAUNCH(c, kKConvUmma, launch_conv_pair(p, a.dtype, c->num_sms, c->stream));
-    if (p.splits > 1) KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
+    if (p.cut && !p.arrivals) KLAUNCH(c, kKConvReduce, launch_conv_reduce(q, a.dtype, c->stream));
     return 0;
   }
   c->last_variant = p.splits > 1 ? "tap split" : "tap";
@@ -3057,6 +3065,8 @@ int b200conv_create(int device, b200conv_ctx** out) {
   bool ok = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) == cudaSuccess &&
             cudaHostAlloc(&hs, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
             cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->d_status), hs, 0) == cudaSuccess &&
+            cudaMalloc(reinterpret_cast<void**>(&c->d_arrivals), kArrivals * sizeof(unsigned int)) == cudaSuccess &&
+            cudaMemset(c->d_arrivals, 0, kArrivals * sizeof(unsigned int)) == cudaSuccess &&
             cudaEventCreate(&c->ev0) == cudaSuccess && cudaEventCreate(&c->ev1) == cudaSuccess;
   if (ok) {
     c->h_status = static_cast<volatile int*>(hs);
@@ -3102,6 +3112,7 @@ void b200conv_destroy(b200conv_ctx* c) {
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : c->chunk_ev) cudaEventDestroy(e);
   cudaFreeHost(const_cast<int*>(c->h_status));
+  cudaFree(c->d_arrivals);
   for (auto& r : c->prof_recs) { cudaEventDestroy(r.a); cudaEventDestroy(r.b); }
   for (auto& e : c->prof_pool) cudaEventDestroy(e);
   cudaEventDestroy(c->ev0);

@@ -5,17 +5,19 @@
 // operands, and each CTA's TMEM receives its own accumulator rows.  What bounds the one-CTA form with 256 filters is L2: 48 KB per
 // 512 clocks of MMAs are 96 B/clk, where an SM receives 73; in a pair it is 32 KB, 64 B/clk.
 //
-// Tiles beyond whole waves are cut: 98 pair tiles on 74 pairs of SMs take as long as 148.  The first `whole` tiles run as they are, one
-// more per pair and wave; the reduction of each remaining one goes to `splits` pairs, which leave float32 accumulators for
-// conv_reduce.cu.  (The model that decides, pair_cut() in api.cu, weighs a tile's MMAs against the second kernel.)
+// Tiles beyond whole waves are cut: 98 pair tiles on 74 pairs of SMs take as long as 148.  The reduction of the first `cut` tiles goes to
+// `splits` pairs each, which leave float32 accumulators in global memory; each pair then takes a whole tile.  Whoever leaves the last slice
+// of a CTA's half of a cut tile (an atomic count, nobody waits) adds the slices in order and writes the result, beside the MMAs of its
+// whole tile.  Where no whole tile follows, conv_reduce.cu does it, on all SMs.  (pair_cut() in api.cu decides.)
 //
 // Warp roles (608 threads): warps 0 and 18 TMA producers (pixels, filters: the issue of a box takes a thread about 300 clocks), warp 1
 // MMA issuer of the even CTA and TMEM owner, 16 epilogue warps.  Two accumulators, so that a tile's read-out runs beside the next tile's MMAs; the
 // results leave as staged TMA stores, 128 bytes of channels per group of four warps.  Nothing is multicast.
 //
 // Measured (a B200, filters packed, one-CTA kernel -> pairs): float16, 256 images, 3x3 256 -> 256 at 14x14 48 -> 43 us (37 without any
-// loads), 512 -> 512 at 7x7 (106 pair tiles, 32 of them cut in two) 52 -> 46, strided 1024 -> 2048 1x1 52 -> 45; float32 512 -> 512 at 14x14, 64 images
-// (98 tiles, 24 cut in three) 100 -> 80.  Flattened 1x1 layers stay with gemm_pair.cu (256 -> 1024 at 14x14 33 us here, 31 there).
+// loads), 512 -> 512 at 7x7 (106 pair tiles, 32 of them cut in two) 52 -> 42, strided 1024 -> 2048 1x1 52 -> 45; float32 256 -> 256 at 14x14, 128 images
+// (98 tiles, 24 cut in three) 58 -> 42, 512 -> 512, 64 images 100 -> 76.  With the slices added by a kernel of its own the cut ones took 46, 51 and 82.
+// Flattened 1x1 layers stay with gemm_pair.cu (256 -> 1024 at 14x14 33 us here, 31 there).
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -40,15 +42,16 @@ struct alignas(16) Bars {
   uint64_t acc_full[2];             // each CTA: the tile's accumulator is complete
   uint64_t acc_empty[2];            // even CTA: both CTAs' epilogues have read the accumulator
   uint32_t tmem_base;
-  volatile int abort;
+  volatile int abort, last;         // last: this CTA's slice of a cut tile was the last to arrive
 };
 
-// Work item: a tile (of a pair) and the stages [k0, k1) of its reduction; slice < 0: all of them.
+// Work item: a tile (of a pair) and the stages [k0, k1) of its reduction; slice < 0: all of them.  The slices of the cut tiles come first.
 struct Item { uint32_t tile, k0, k1; int slice; };
 __device__ __forceinline__ Item item_of(const UmmaConvParams& p, uint32_t item, uint32_t kiters) {
-  if (item < static_cast<uint32_t>(p.whole)) return Item{item, 0, kiters, -1};
-  const uint32_t r = item - p.whole, splits = p.splits, t = quotient(r, p.walk.splits), s = r - t * splits;
-  return Item{p.whole + t, kiters * s / splits, kiters * (s + 1) / splits, static_cast<int>(s)};
+  const uint32_t splits = p.splits, slices = p.cut * splits;
+  if (item >= slices) return Item{item - slices + p.cut, 0, kiters, -1};
+  const uint32_t t = quotient(item, p.walk.splits), s = item - t * splits;
+  return Item{t, kiters * s / splits, kiters * (s + 1) / splits, static_cast<int>(s)};
 }
 
 template <MmaKind KIND, int BN>
@@ -72,7 +75,7 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
   const uint32_t kiters = p.ntaps * p.kblocks;
   const uint32_t co_groups = static_cast<uint32_t>(p.tiles_co) * p.groups, tiles_wh = static_cast<uint32_t>(p.tiles_w) * p.tiles_h;
   const uint32_t tiles = (tiles_wh * p.tiles_n + 1) / 2 * co_groups;              // counts fit 32 bits (the launcher checks)
-  const uint32_t total = p.whole + (tiles - p.whole) * p.splits;
+  const uint32_t total = p.cut * p.splits + tiles - p.cut;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -195,23 +198,38 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
       tc_fence_after();
       const int co_base = co_t * BN;
       const uint32_t lane_base = tmem + buf * BN + (static_cast<uint32_t>(quad * 32) << 16);
+      // slices of this CTA's half of a cut tile, one after the other
+      float4* slabs = reinterpret_cast<float4*>(p.partial) + (static_cast<long long>(w.tile) * 2 + rank) * p.splits * (kRows * BN / 4) + row;
+      const bool present = row < rows_used && n0 < p.Nimg;
+      bool finish = true;
       if (w.slice >= 0) {
-        // raw accumulators; conv_reduce.cu adds the slices and applies the epilogue
-        const long long slab = (static_cast<long long>(w.tile - p.whole) * 2 + rank) * p.splits + w.slice;
-        float4* dst = reinterpret_cast<float4*>(p.partial) + slab * (kRows * BN / 4) + row;
+        // raw accumulators
+        float4* dst = slabs + w.slice * (kRows * BN / 4);
 #pragma unroll 1
         for (int ch = grp; ch < BN / 32 && co_base + ch * 32 < p.n_out; ch += 4) {
           uint32_t r[32];
           tmem_ld32(lane_base + ch * 32, r);
           tmem_ld_wait();
-          if (row >= rows_used || n0 >= p.Nimg) continue;
+          if (!present) continue;
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             if (B200_IN_RANGE((reinterpret_cast<float*>(dst + (ch * 8 + j) * kRows) - p.partial) + 4 <= p.partial_elems, p.status))
               dst[(ch * 8 + j) * kRows] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
                                                       __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
         }
-      } else {
+        tc_fence_before();
+        __threadfence();
+        named_barrier(5, 32 * kEpilogueWarps);
+        if (warp == 2 && lane == 0) {
+          mbar_arrive_leader(&bars->acc_empty[buf]);
+          // the count of the tile's slices that have arrived goes back to zero with the last one
+          bars->last = p.arrivals && atomicInc(p.arrivals + w.tile * 2 + rank, p.splits - 1) == static_cast<uint32_t>(p.splits) - 1;
+        }
+        named_barrier(5, 32 * kEpilogueWarps);
+        finish = bars->last;
+        if (finish) __threadfence();
+      }
+      if (finish) {
         const int nstaged = min(BN / kBK, (p.n_out - co_base + kBK - 1) / kBK);
         for (int ch = (grp - turn) & 3; ch < nstaged; ch += 4) {
           const int co0 = co_base + ch * kBK;
@@ -224,8 +242,27 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
 #pragma unroll
           for (int part = 0; part < kBK / 32; ++part) {
             uint32_t r[32];
-            tmem_ld32(lane_base + ch * kBK + part * 32, r);
-            tmem_ld_wait();
+            if (w.slice < 0) {
+              tmem_ld32(lane_base + ch * kBK + part * 32, r);
+              tmem_ld_wait();
+            } else {
+              // the slices in order, whichever arrived last; eight loads in flight
+              const float4* src = slabs + (ch * kBK + part * 32) / 4 * kRows;
+#pragma unroll
+              for (int j = 0; j < 32; ++j) r[j] = 0;
+#pragma unroll 1
+              for (int s = 0; s < (present ? p.splits : 0); ++s, src += kRows * BN / 4) {
+                float4 v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = __ldcg(src + j * kRows);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v[j].x); r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v[j].y);
+                  r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v[j].z); r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v[j].w);
+                }
+              }
+              __syncwarp();
+            }
             zero_pad_columns(r, co0 + part * 32, p.n_real);
             const OutT* bp = bias ? bias + part * 32 : nullptr;
             if (!plain) {
@@ -264,6 +301,7 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
         }
         turn += nstaged;
       }
+      if (w.slice >= 0) continue;
       tc_fence_before();
       // one arrival per CTA: sixteen releases at cluster scope, one per warp, cost 2000 clocks a tile (256 -> 1024 1x1 46 -> 33 us)
       named_barrier(5, 32 * kEpilogueWarps);
@@ -302,8 +340,8 @@ cudaError_t launch_one(const UmmaConvParams& p, long long items, int num_sms, cu
 cudaError_t launch_conv_pair(const UmmaConvParams& p, int dtype, int num_sms, cudaStream_t s) {
   const long long tiles = (1LL * p.tiles_w * p.tiles_h * p.tiles_n + 1) / 2 * p.groups * p.tiles_co;
   if (tiles == 0 || p.ntaps == 0) return cudaSuccess;
-  if (num_sms < 2 || p.whole < 0 || p.whole > tiles || p.splits < 1 || (p.whole < tiles && !p.partial)) return cudaErrorInvalidValue;
-  const long long items = p.whole + (tiles - p.whole) * p.splits;
+  if (num_sms < 2 || p.cut < 0 || p.cut > tiles || p.splits < 1 || (p.cut > 0 && !p.partial)) return cudaErrorInvalidValue;
+  const long long items = 1LL * p.cut * p.splits + tiles - p.cut;
   if (items >= (1LL << 30)) return cudaErrorInvalidValue;
   const bool f16 = dtype == B200CONV_F16;
   if (p.bn_cols == 256) return f16 ? launch_one<MmaKind::F16, 256>(p, items, num_sms, s) : launch_one<MmaKind::TF32, 256>(p, items, num_sms, s);

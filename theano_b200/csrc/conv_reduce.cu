@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kReduceThreads) conv_reduce_kernel(const __gri
   for (uint32_t unit = blockIdx.x; unit < static_cast<uint32_t>(walk.units); unit += gridDim.x) {
     const uint32_t u = quotient(unit, walk.col_blocks), cb = unit - u * walk.col_blocks.d;
     const uint32_t z = quotient(u, walk.row_chunks), idx = (u - z * walk.row_chunks.d) * 32 + (threadIdx.x & 31);
-    const uint32_t tile = p.first_tile + (p.pair ? z >> 1 : z);
+    const uint32_t tile = p.pair ? z >> 1 : z;
     const uint32_t tg = quotient(tile, walk.tiles_co), co_t = tile - tg * walk.tiles_co.d, tp = quotient(tg, walk.groups), g = tg - tp * walk.groups.d;
     const uint32_t pt = p.pair ? tp * 2 + (z & 1) : tp;
     const uint32_t th = quotient(pt, walk.tiles_w), tn = quotient(th, walk.tiles_h);

@@ -142,7 +142,8 @@ struct alignas(64) UmmaConvParams {
   int kblocks;                   // ceil(reduction channels per group / channels per stage)
   int bn_cols;                   // accumulator columns of a tile (32, 64, 128 or 256)
   int splits;                    // slices of the reduction; > 1: float32 accumulators go to `partial` (conv_reduce.cu)
-  int whole;                     // conv_pair.cu: the first tiles (of pairs), which are not cut into `splits` slices
+  int cut;                       // conv_pair.cu: that many tiles (of pairs), the first ones, are cut into `splits` slices
+  unsigned int* arrivals;        // counts of their slices, zero between launches; null: conv_reduce.cu adds the slices
   float* partial;
   long long partial_elems;       // elements of `partial` (checked in the range-checked build)
   int groups;
@@ -293,7 +294,7 @@ cudaError_t launch_conv_cols(const ColsConvParams& p, int dtype, int num_sms, cu
 // which wt x th are the tile's); for the per-tap kernel Ws = wt and Hs = th.
 struct ConvReduceParams {
   const float* partial;          // [tile][slice][bn_cols / 4][rows][4]
-  int first_tile, tiles;         // the tiles that were split; pair: both pixel tiles of each pair tile, side by side
+  int tiles;                     // the tiles that were split, from the first on; pair: both pixel tiles of each pair tile, side by side
   int pair;
   int splits, rows, bn_cols;
   int Ws, Hs, wt, th, nb;
