@@ -84,6 +84,7 @@ inline bool aligned16(std::initializer_list<const void*> ptrs) {
 // n / d for n < 2^31 by a multiplication (Granlund and Montgomery, "Division by invariant integers using multiplication")
 struct Divisor { uint32_t d, mul, shift; };
 inline Divisor divisor(uint32_t d) {
+  if (d == 0) d = 1;                     // of launches that have nothing to do
   uint32_t shift = 0;
   while ((1ull << shift) < d) ++shift;
   return Divisor{d, static_cast<uint32_t>(((1ull << 32) * ((1ull << shift) - d)) / d + 1), shift};
@@ -329,6 +330,14 @@ struct alignas(64) PairGemmParams {
 int gemm_pair_smem_bytes(int stages);
 cudaError_t launch_gemm_pair(const PairGemmParams& p, int num_sms, cudaStream_t s);
 
+// How the gradWeights kernels walk theirs: (filter tile, channel tile, group, tap or what the kernel puts in its place, slice), the slice fastest,
+// and pixel tiles within an image.  (Set by the launchers; a role looks once per item, but on small layers there is one item per CTA, and its first
+// load waited 1000 clocks for the quotients.)
+struct ItemWalk { Divisor splits, taps, groups, ctiles, tiles_w, tiles_h; };
+inline ItemWalk item_walk(int splits, int taps, int groups, int ctiles, int tiles_w, int tiles_h) {
+  return ItemWalk{divisor(splits), divisor(taps), divisor(groups), divisor(ctiles), divisor(tiles_w), divisor(tiles_h)};
+}
+
 // ---- implicit-GEMM filter gradient (wgrad_umma.cu) -------------------------------------
 struct alignas(64) UmmaWgradParams {
   CUtensorMap dy_map;            // 5-D (k_in_group, group, wo, ho, n) over dy, box 32/64 channels
@@ -347,6 +356,7 @@ struct alignas(64) UmmaWgradParams {
   long long partial_elems;       // its extent (checked in the range-checked build)
   int taps_total;                // kH*kW
   int atomic;                    // 1: red.add into partial[0] instead of per-split slabs
+  ItemWalk walk;                 // set by the launcher
   int* status;
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
   long long* trace;              // optional: 16 clock counters per CTA (phase timing), or null
@@ -412,6 +422,7 @@ struct alignas(64) GroupWgradParams {
   long long partial_elems;         // its extent (checked in the range-checked build)
   int taps_total;
   int atomic;
+  ItemWalk walk;                 // set by the launcher
   int* status;
   long long wait_clocks;          // bound of every device-side wait, in SM clocks
   long long* trace;                // optional: 16 clock counters per CTA (phase timing), or null
@@ -440,6 +451,7 @@ struct alignas(64) RowsWgradParams {
   long long partial_elems;           // its extent (checked in the range-checked build)
   int diag_c, diag_k;                // merged groups of diag_k filters x diag_c channels: only their blocks are stored; 0: everything
   int taps_total;
+  ItemWalk walk;                 // set by the launcher
   int* status;
   long long wait_clocks;             // bound of every device-side wait, in SM clocks
 };

@@ -64,19 +64,16 @@ struct Item {
   uint32_t t_begin, t_end;
 };
 
-// 32-bit arithmetic throughout (the launcher checks the counts): 64-bit divisions cost a role
-// about a hundred clocks each
+// 32-bit arithmetic throughout (the launcher checks the counts)
 __device__ __forceinline__ Item decode(uint32_t it, const GroupWgradParams& p, uint32_t per_split,
                                        uint32_t pix_tiles) {
   Item r;
-  r.sp = it % static_cast<uint32_t>(p.splits);
-  it /= static_cast<uint32_t>(p.splits);
-  r.grp = it % static_cast<uint32_t>(p.ngroups);
-  it /= static_cast<uint32_t>(p.ngroups);
-  r.g = it % static_cast<uint32_t>(p.groups);
-  it /= static_cast<uint32_t>(p.groups);
-  r.ct = it % static_cast<uint32_t>(p.ctiles);
-  r.kt = it / static_cast<uint32_t>(p.ctiles);
+  const uint32_t a = quotient(it, p.walk.splits), b = quotient(a, p.walk.taps), c = quotient(b, p.walk.groups);
+  r.sp = it - a * p.walk.splits.d;
+  r.grp = a - b * p.walk.taps.d;
+  r.g = b - c * p.walk.groups.d;
+  r.kt = quotient(c, p.walk.ctiles);
+  r.ct = c - r.kt * p.walk.ctiles.d;
   r.t_begin = r.sp * per_split;
   r.t_end = r.t_begin + per_split < pix_tiles ? r.t_begin + per_split : pix_tiles;
   return r;
@@ -267,9 +264,8 @@ wgrad_group_kernel(const __grid_constant__ GroupWgradParams p) {
       const uint32_t tx = (a_boxes * p.rows_a + b_boxes * p.rows_b) * 128;
       // tile coordinates advance by counting: 64-bit divisions per stage would cost the producers
       // more clocks than the stage's MMAs take
-      int tw = static_cast<int>(w.t_begin % static_cast<uint32_t>(p.tiles_w));
-      int th_ = static_cast<int>((w.t_begin / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h));
-      int tn = static_cast<int>(w.t_begin / (static_cast<uint32_t>(p.tiles_w) * p.tiles_h));
+      const uint32_t trow = quotient(w.t_begin, p.walk.tiles_w);
+      int tn = quotient(trow, p.walk.tiles_h), th_ = trow - tn * p.tiles_h, tw = w.t_begin - trow * p.tiles_w;
       for (uint32_t t = w.t_begin; t < w.t_end; ++t) {
         const int w0 = tw * p.wt, h0 = th_ * p.th, n0 = tn * p.nb;
         if (++tw == p.tiles_w) {
@@ -393,6 +389,7 @@ cudaError_t launch_one(const GroupWgradParams& p, long long total, int num_sms, 
 
 cudaError_t launch_wgrad_group(const GroupWgradParams& params, int dtype, int num_sms, cudaStream_t s) {
   GroupWgradParams p = params;
+  p.walk = item_walk(p.splits, p.ngroups, p.groups, p.ctiles, p.tiles_w, p.tiles_h);
   const long long total = 1LL * p.ktiles * p.ctiles * p.groups * p.ngroups * p.splits;
   if (total == 0) return cudaSuccess;
   if (total >= (1LL << 31) || 1LL * p.tiles_w * p.tiles_h * p.tiles_n >= (1LL << 31)) return cudaErrorInvalidValue;

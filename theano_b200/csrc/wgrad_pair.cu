@@ -53,14 +53,12 @@ struct Item {
 
 __device__ __forceinline__ Item decode(uint32_t it, const UmmaWgradParams& p, uint32_t per_split, uint32_t pix_tiles) {
   Item r;
-  r.sp = it % static_cast<uint32_t>(p.splits);
-  it /= static_cast<uint32_t>(p.splits);
-  r.tap = it % static_cast<uint32_t>(p.ntaps);
-  it /= static_cast<uint32_t>(p.ntaps);
-  r.g = it % static_cast<uint32_t>(p.groups);
-  it /= static_cast<uint32_t>(p.groups);
-  r.ct = it % static_cast<uint32_t>(p.ctiles);
-  r.kt = it / static_cast<uint32_t>(p.ctiles);
+  const uint32_t a = quotient(it, p.walk.splits), b = quotient(a, p.walk.taps), c = quotient(b, p.walk.groups);
+  r.sp = it - a * p.walk.splits.d;
+  r.tap = a - b * p.walk.taps.d;
+  r.g = b - c * p.walk.groups.d;
+  r.kt = quotient(c, p.walk.ctiles);
+  r.ct = c - r.kt * p.walk.ctiles.d;
   r.t_begin = r.sp * per_split;
   r.t_end = r.t_begin + per_split < pix_tiles ? r.t_begin + per_split : pix_tiles;
   return r;
@@ -172,9 +170,8 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
       const Item w = decode(it, p, per_split, pix_tiles);
       const ConvTap tp = p.taps[w.tap];
       const int k0 = w.kt * 256 + rank * 128, c0 = w.ct * kBN + rank * 128;
-      int tw = static_cast<int>(w.t_begin % static_cast<uint32_t>(p.tiles_w));
-      int th_ = static_cast<int>((w.t_begin / static_cast<uint32_t>(p.tiles_w)) % static_cast<uint32_t>(p.tiles_h));
-      int tn = static_cast<int>(w.t_begin / (static_cast<uint32_t>(p.tiles_w) * p.tiles_h));
+      const uint32_t trow = quotient(w.t_begin, p.walk.tiles_w);
+      int tn = quotient(trow, p.walk.tiles_h), th_ = trow - tn * p.tiles_h, tw = w.t_begin - trow * p.tiles_w;
       for (uint32_t t = w.t_begin; t < w.t_end; ++t) {
         const int w0 = tw * p.bw, h0 = th_ * p.bh, n0 = tn * p.bn;
         if (++tw == p.tiles_w) {
@@ -282,7 +279,9 @@ cudaError_t launch_one(const UmmaWgradParams& p, long long total, int num_sms, c
 
 }  // namespace
 
-cudaError_t launch_wgrad_pair(const UmmaWgradParams& p, int dtype, int num_sms, cudaStream_t s) {
+cudaError_t launch_wgrad_pair(const UmmaWgradParams& params, int dtype, int num_sms, cudaStream_t s) {
+  UmmaWgradParams p = params;
+  p.walk = item_walk(p.splits, p.ntaps, p.groups, p.ctiles, p.tiles_w, p.tiles_h);
   const long long total = 1LL * p.ktiles * p.ctiles * p.groups * p.ntaps * p.splits;
   if (total == 0) return cudaSuccess;
   if (total >= (1LL << 31) || 1LL * p.tiles_w * p.tiles_h * p.tiles_n >= (1LL << 31) || p.bw * p.bh * p.bn > kPix)

@@ -55,12 +55,11 @@ struct Item {
 };
 __device__ __forceinline__ Item decode(uint32_t it, const RowsWgradParams& p, uint32_t per_split, uint32_t tiles) {
   Item r;
-  r.sp = it % static_cast<uint32_t>(p.splits);
-  it /= static_cast<uint32_t>(p.splits);
-  r.v = it % static_cast<uint32_t>(p.nviews);
-  it /= static_cast<uint32_t>(p.nviews);
-  r.g = it % static_cast<uint32_t>(p.groups);
-  r.ct = it / static_cast<uint32_t>(p.groups);
+  const uint32_t a = quotient(it, p.walk.splits), b = quotient(a, p.walk.taps), c = quotient(b, p.walk.groups);
+  r.sp = it - a * p.walk.splits.d;
+  r.v = a - b * p.walk.taps.d;
+  r.g = b - c * p.walk.groups.d;
+  r.ct = c;
   r.t_begin = r.sp * per_split;
   r.t_end = min(r.t_begin + per_split, tiles);
   return r;
@@ -179,7 +178,7 @@ wgrad_rows_kernel(const __grid_constant__ RowsWgradParams p) {
     bool ok = true;
     for (uint32_t it = blockIdx.x; it < total && ok; it += gridDim.x) {
       const Item w = decode(it, p, per_split, tiles);
-      int th_ = static_cast<int>(w.t_begin % static_cast<uint32_t>(p.tiles_h)), n = static_cast<int>(w.t_begin / static_cast<uint32_t>(p.tiles_h));
+      int n = quotient(w.t_begin, p.walk.tiles_h), th_ = w.t_begin - n * p.tiles_h;
       for (uint32_t t = w.t_begin; t < w.t_end; ++t) {
         const int h0 = th_ * p.th - p.halo, n0 = n;
         if (++th_ == p.tiles_h) { th_ = 0; ++n; }
@@ -299,7 +298,9 @@ bool wgrad_rows_ring(RowsWgradParams* p, int dtype) {
   return p->stages >= 2;
 }
 
-cudaError_t launch_wgrad_rows(const RowsWgradParams& p, int dtype, int num_sms, cudaStream_t s) {
+cudaError_t launch_wgrad_rows(const RowsWgradParams& params, int dtype, int num_sms, cudaStream_t s) {
+  RowsWgradParams p = params;
+  p.walk = item_walk(p.splits, p.nviews, p.groups, p.ctiles, 1, p.tiles_h);
   const long long total = 1LL * p.ctiles * p.groups * p.nviews * p.splits;
   if (total == 0) return cudaSuccess;
   if (total >= (1LL << 31) || 1LL * p.tiles_h * p.Nimg >= (1LL << 31)) return cudaErrorInvalidValue;
