@@ -1143,6 +1143,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   }
   if (p.ntaps == 0) return 1;  // caller zero-fills
   for (int v = nviews; v < kMaxViews; ++v) p.views[v] = p.views[0];
+  p.nviews = nviews;
   const int BN = tile.bn;
   int rc = make_wmap(c, &p.wmap, a.wpacked, a.dtype, a.Cin_g, a.w_rows, a.nmats, a.ld_w, kBK, pair ? BN / 2 : BN);
   if (rc) return rc;
@@ -2103,6 +2104,7 @@ int wgrad_grouped(b200conv_ctx* c, const b200conv_desc& d, const void* xin, cons
     if (rc) return rc;
   }
   for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = p.x_views[0];
+  p.nviews = nviews;
   p.groups = d.groups; p.Kg = Kg; p.Cg = Cg;
   p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
   p.ktiles = (int)cdiv(Kg, 128); p.ctiles = (int)cdiv(Cg, 128);
@@ -2466,6 +2468,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         if (r != CUDA_SUCCESS) return fail(c, B200CONV_E_CUDA, "cuTensorMapEncodeTiled(space-to-depth x) failed: %d", (int)r);
       }
       for (int v = 1; v < kMaxViews; ++v) p.x_views[v] = p.x_views[0];
+      p.nviews = 1;
       for (int t = 0; t < s2_nt; ++t) {
         ConvTap tp;
         tp.dh = (int16_t)(t + s2_t0); tp.dw = 0; tp.view = 0; tp.wmat = (int16_t)t;
@@ -2587,6 +2590,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
         p.taps[p.ntaps++] = t;
       }
       for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = nviews ? p.x_views[0] : p.dy_map;
+      p.nviews = nviews;
       p.groups = 1; p.Kg = d.K; p.Cg = kBK;
       p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
       p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
@@ -2724,6 +2728,7 @@ int wgrad_device(b200conv_ctx* c, const b200conv_desc& d, const void* x, const v
       p.taps[p.ntaps++] = t;
     }
   for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = nviews ? p.x_views[0] : p.dy_map;
+  p.nviews = nviews;
   p.groups = d.groups; p.Kg = Kg; p.Cg = Cg;
   p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
   p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);
@@ -4015,6 +4020,7 @@ extern "C" int b200conv_wgrad_static(b200conv_ctx* c, const b200conv_desc* dp, c
       p.taps[p.ntaps++] = t;
     }
   for (int v = nviews; v < kMaxViews; ++v) p.x_views[v] = nviews ? p.x_views[0] : p.dy_map;
+  p.nviews = nviews;
   p.groups = d.groups; p.Kg = Kg; p.Cg = Cg;
   p.Wo = d.Wo; p.Ho = d.Ho; p.Nimg = d.N;
   p.tiles_w = (int)cdiv(d.Wo, p.bw); p.tiles_h = (int)cdiv(d.Ho, p.bh); p.tiles_n = (int)cdiv(d.N, p.bn);

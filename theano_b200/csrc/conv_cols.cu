@@ -196,6 +196,12 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    tma_prefetch_desc(&p.view);
+    tma_prefetch_desc(&p.wmap);
+    if (!p.d2s) tma_prefetch_desc(&p.out_map);
+  }
   if (warp == 1) {
     if (PAIR) {
       tmem_alloc_pair(&bars->tmem_base, 512);
@@ -214,7 +220,6 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
 
   if (warp == 0) {
     const bool leader = elect_one();
-    if (leader) tma_prefetch_desc(&p.view);
     const uint32_t tx = static_cast<uint32_t>(p.pitch * p.Hs) * 128u;
     int sb = 0;
     uint32_t phase = 0;
@@ -235,7 +240,6 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
   } else if (warp == kFilterProducer) {
     // a stage is rps filter rows of one channel block: neighbours in the packed filters, they arrive as one box
     const bool leader = elect_one();
-    if (leader) tma_prefetch_desc(&p.wmap);
     int bs = 0;
     uint32_t phase = 0;
     bool ok = true;

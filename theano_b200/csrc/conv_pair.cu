@@ -89,6 +89,12 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.views[v]);
+    tma_prefetch_desc(&p.wmap);
+    tma_prefetch_desc(&p.out_map);
+  }
   if (warp == 1) {                                               // the same warp in both CTAs
     tmem_alloc_pair(&bars->tmem_base, 2 * BN);
     tmem_relinquish_pair();
@@ -104,10 +110,6 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
     // all lanes follow the loop, one elected lane issues
     const bool leader = elect_one();
     const bool b_box = warp != 0;
-    if (leader) {
-      if (b_box) tma_prefetch_desc(&p.wmap);
-      else tma_prefetch_desc(&p.views[0]);
-    }
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;

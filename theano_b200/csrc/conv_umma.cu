@@ -96,6 +96,11 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.views[v]);
+    tma_prefetch_desc(&p.wmap);
+  }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
     tmem_relinquish();
@@ -115,10 +120,6 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
     const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
     const bool b_box = (pw & 1) != 0;
     const uint32_t my_parity = pw >> 1;
-    if (leader) {
-      for (int v = 0; v < kMaxViews; ++v) tma_prefetch_desc(&p.views[v]);
-      tma_prefetch_desc(&p.wmap);
-    }
     int stage = 0;
     uint32_t phase = 0, idx = 0;
     bool ok = true;

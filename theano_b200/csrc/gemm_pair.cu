@@ -64,6 +64,12 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    tma_prefetch_desc(&p.view);
+    tma_prefetch_desc(&p.wmap);
+    tma_prefetch_desc(&p.out_map);
+  }
   if (warp == 1) {                                               // the same warp in both CTAs
     tmem_alloc_pair(&bars->tmem_base, 512);
     tmem_relinquish_pair();
@@ -77,10 +83,6 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
 
   if (warp == 0) {
     const bool leader = elect_one();
-    if (leader) {
-      tma_prefetch_desc(&p.view);
-      tma_prefetch_desc(&p.wmap);
-    }
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;

@@ -137,6 +137,7 @@ inline ConvEpilogue default_epilogue() { return ConvEpilogue{nullptr, 1.f, 0.f, 
 
 struct alignas(64) UmmaConvParams {
   CUtensorMap views[kMaxViews];  // 5-D (c_in_group, group, w, h, n) channels-last views
+  int nviews;
   CUtensorMap wmap;              // 3-D (k_red, n_out, wmat*groups + g) packed filters
   ConvTap taps[kMaxTaps];
   int ntaps;
@@ -342,6 +343,7 @@ inline ItemWalk item_walk(int splits, int taps, int groups, int ctiles, int tile
 struct alignas(64) UmmaWgradParams {
   CUtensorMap dy_map;            // 5-D (k_in_group, group, wo, ho, n) over dy, box 32/64 channels
   CUtensorMap x_views[kMaxViews];// 5-D views over x (stride parity classes)
+  int nviews;
   ConvTap taps[kMaxTaps];        // wmat = flat filter tap index i*kW + j (after flip)
   int ntaps;
   int groups;
@@ -400,6 +402,7 @@ constexpr int kMaxTapGroups = 32;
 struct alignas(64) GroupWgradParams {
   CUtensorMap dy_map;              // box (atom, 1, Wa, th, nb)
   CUtensorMap x_views[kMaxViews];  // box (atom, 1, Wb, th, nb), one per stride parity class
+  int nviews;
   int16_t grp_view[kMaxTapGroups], grp_dh[kMaxTapGroups], grp_first[kMaxTapGroups], grp_n[kMaxTapGroups];
   int16_t view_dwmin[kMaxViews];
   int16_t tap_off[kMaxTaps];       // dw - dw_min of the tap's view: row offset into the x tile

@@ -133,6 +133,11 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.x_views[v]);
+    tma_prefetch_desc(&p.dy_map);
+  }
   if (warp == 1) {
     tmem_alloc_pair(&bars->tmem_base, 512);
     tmem_relinquish_pair();
@@ -158,10 +163,6 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
   if (warp == 0 || warp >= kFirstExtraProducer) {
     const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
     const bool leader = elect_one();
-    if (leader) {
-      for (int v = 0; v < kMaxViews; ++v) tma_prefetch_desc(&p.x_views[v]);
-      tma_prefetch_desc(&p.dy_map);
-    }
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;

@@ -150,6 +150,11 @@ wgrad_rows_kernel(const __grid_constant__ RowsWgradParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.x_views[v]);
+    tma_prefetch_desc(&p.dy_map);
+  }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
@@ -169,10 +174,6 @@ wgrad_rows_kernel(const __grid_constant__ RowsWgradParams p) {
 
   if (warp == 0 || warp == kXProducer) {
     const bool leader = elect_one(), is_x = warp != 0;
-    if (leader) {
-      if (!is_x) tma_prefetch_desc(&p.dy_map);
-      else for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.x_views[v]);
-    }
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;

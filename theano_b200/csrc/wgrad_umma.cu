@@ -169,6 +169,11 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
     bars->abort = 0;
     mbar_fence_init();
   }
+  // descriptors, beside the set-up and the wait for the kernel before (they are parameters, not global data)
+  if (warp == 2 && lane == 0) {
+    for (int v = 0; v < p.nviews; ++v) tma_prefetch_desc(&p.x_views[v]);
+    tma_prefetch_desc(&p.dy_map);
+  }
   if (warp == 1) {
     tmem_alloc(&bars->tmem_base, kTmemCols);
     tmem_relinquish();
@@ -193,10 +198,6 @@ wgrad_umma_kernel(const __grid_constant__ UmmaWgradParams p) {
 
   if (warp == 0 || warp >= kFirstExtraProducer) {
     const int pw = warp == 0 ? 0 : warp - kFirstExtraProducer + 1;
-    if (lane == 0) {
-      for (int v = 0; v < kMaxViews; ++v) tma_prefetch_desc(&p.x_views[v]);
-      tma_prefetch_desc(&p.dy_map);
-    }
     // every lane follows the loop (warp-uniform control flow and addresses); one elected lane issues
     // this warp's boxes of a stage: pw, pw + kProducers, ...
     const bool leader = elect_one();
