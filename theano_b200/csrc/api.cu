@@ -1051,7 +1051,12 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   if (!fits(2, 2, 1)) p.rps = 1;
   if (!fits(2, 2, 1)) return 2;
   if (!launch) return 0;
+  // A CTA whose tiles are all of one group loads the filters once where the ring holds them whole.
+  const int per_tile = (int)cdiv(a.Cin_g, kBK) * (p.kH / p.rps), units = pair ? c->num_sms / 2 : c->num_sms;
+  p.resident = units % a.groups == 0 && per_tile <= kMaxColStages && fits(2, per_tile, 1);
+  if (p.resident) p.b_stages = per_tile;
   for (char step : {'s', 'b', 'f', 'b', 's', 'b', 'b'}) {
+    if (step == 'b' && p.resident) continue;
     const int s = p.s_stages + (step == 's'), b = p.b_stages + (step == 'b'), f = step == 'f' ? 2 : bufs;
     if (fits(s, b, f)) { p.s_stages = s; p.b_stages = b; bufs = f; }
   }
@@ -3654,7 +3659,7 @@ int b200conv_set_splits(b200conv_ctx* c, int splits) {
 // kTuningKernels goes up with each change of the kernels after which earlier timings or the numbers of choices no longer hold.
 // 2: three gradWeights kernels to choose from where there were two, float32 pairs behind the one-tap choice.  (Files before it
 // have no such number.)
-// 3: the per-tap kernel on pairs.
+// 3: the per-tap kernel on pairs, with and without cut tiles; the columns kernel, on one CTA and on pairs.
 constexpr int kTuningKernels = 3;
 static std::string tuning_header(b200conv_ctx* c) {
   cudaDeviceProp prop;

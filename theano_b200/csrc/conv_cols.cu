@@ -31,7 +31,7 @@ constexpr int kEpilogueWarps = 16;
 constexpr int kSecondIssuer = 2 + kEpilogueWarps;     // warp index
 constexpr int kFilterProducer = kSecondIssuer + 1;    // warp index
 constexpr int kThreads = 32 * (kFilterProducer + 1);
-constexpr int kMaxStages = 8, kMaxSets = 4;
+constexpr int kMaxStages = kMaxColStages, kMaxSets = 4;
 
 struct alignas(16) Bars {
   uint64_t slab_full[kMaxStages];
@@ -59,6 +59,7 @@ struct IssueLoop {
   uint32_t slab0, ring0, tmem;          // low descriptor words of the rings, accumulator a of set 0
   uint32_t first, stride, total;
   bool leader;
+  uint32_t resident;                    // filters: the ring is one tile's, loaded once, its barriers stay in their first phase
 };
 
 // The MMAs of one issuing warp, all its tiles: RPS filter rows per filter stage as straight-line code, all 32 lanes in the loop, one
@@ -108,7 +109,7 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
         else if (leader) part(0, kBefore);
         __syncwarp();
         const int cur = bs;
-        if (++bs == p.b_stages) { bs = 0; bphase ^= 1; }
+        if (++bs == p.b_stages) { bs = 0; bphase ^= w.resident ^ 1; }
         b_seen = mbar_look(&bars->b_full[bs], bphase);
         if (i + RPS >= p.kH) {
           const int ns = sb + 1 == p.s_stages ? 0 : sb + 1;
@@ -121,7 +122,7 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
         if (kTogether) part(kBefore, RPS * 4);
         if (leader) {
           if (!kTogether) part(kBefore, RPS * 4);
-          commit(&bars->b_empty[cur]);
+          if (!w.resident) commit(&bars->b_empty[cur]);
         }
       }
       if (leader) commit(&bars->slab_empty[sb]);
@@ -243,7 +244,7 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     int bs = 0;
     uint32_t phase = 0;
     bool ok = true;
-    for (uint32_t t = first; t < total && ok; t += stride) {
+    for (uint32_t t = first; t < total && ok; t = p.resident ? total : t + stride) {
       const int g = t % static_cast<uint32_t>(p.groups);
       for (int kb = 0; kb < p.kblocks && ok; ++kb) {
         for (int i = 0; i < p.kH; i += p.rps) {
@@ -264,7 +265,7 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     if (rank == 0 && a < p.n_acc) {              // a pair: the even CTA issues for both
       const bool leader = elect_one();
       const uint32_t desc_lo = static_cast<uint32_t>(smem_desc(0, 16, 1024));
-      const IssueLoop w{p, bars, desc_lo + ((smem_u32(smem) + 16384u * a) >> 4), desc_lo + (smem_u32(bring) >> 4), tmem + a * n_cols, first, stride, total, leader};
+      const IssueLoop w{p, bars, desc_lo + ((smem_u32(smem) + 16384u * a) >> 4), desc_lo + (smem_u32(bring) >> 4), tmem + a * n_cols, first, stride, total, leader, p.resident ? 1u : 0u};
       bool ok;
       switch (p.rps) {
         case 2: ok = issue_tiles<KIND, 2, PAIR>(w); break;
@@ -479,7 +480,8 @@ cudaError_t launch_conv_cols(const ColsConvParams& p, int dtype, int num_sms, cu
   if (total == 0) return cudaSuccess;
   if (p.pair && (p.bn != 64 || p.d2s || p.n_acc != 1 || num_sms < 2)) return cudaErrorInvalidValue;
   if (total >= (1LL << 31) || p.n_acc < 1 || p.n_acc > 2 || p.sets < 2 || p.sets > kMaxSets || (p.step != p.sets && (p.step != 1 || p.sets != 2)) || p.sets * p.n_acc * p.kW * p.bn > 512 || p.kH > kMaxColTaps || p.rps < 1 || p.kH % p.rps || p.kW > kMaxColTaps ||
-      p.s_stages < 2 || p.s_stages > kMaxStages || p.b_stages < 2 || p.b_stages > kMaxStages) return cudaErrorInvalidValue;
+      p.s_stages < 2 || p.s_stages > kMaxStages || p.b_stages < (p.resident ? 1 : 2) || p.b_stages > kMaxStages ||
+      (p.resident && (p.b_stages != p.kblocks * (p.kH / p.rps) || (p.pair ? num_sms / 2 : num_sms) % p.groups))) return cudaErrorInvalidValue;
   if (p.pair) return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, true>(p, total, num_sms, s) : launch_one<MmaKind::TF32, true>(p, total, num_sms, s);
   return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, false>(p, total, num_sms, s) : launch_one<MmaKind::TF32, false>(p, total, num_sms, s);
 }

@@ -255,6 +255,7 @@ cudaError_t launch_conv_slab(const SlabConvParams& p, int dtype, int bn, int num
 
 // ---- layers of at most 64 filters, the filter's columns inside one MMA (conv_cols.cu) ----------------
 constexpr int kMaxColTaps = 8;   // filter rows, filter columns
+constexpr int kMaxColStages = 8; // of a ring
 struct alignas(64) ColsConvParams {
   CUtensorMap view;              // 5-D (c_in_group, group, w, h, n), box (kBK, 1, pitch, Hs, 1)
   CUtensorMap wmap;              // 4-D packed filters (k_red, n_out, group, tap), box (kBK, bn, 1, rps * kW)
@@ -275,6 +276,7 @@ struct alignas(64) ColsConvParams {
   int step;                      // that distance
   int slab_bytes, s_stages, b_stages;
   int rps;                       // filter rows per filter stage (a divisor of kH)
+  int resident;                  // 1: the filter ring is the filters of one tile, loaded once (a CTA's tiles are of one group)
   int n_out, n_real;             // output channels per group as stored / with filters
   int pair;                      // 1: CTA pairs (two pixel tiles side by side, M = 256; 64 columns per filter column, 32 of them per CTA)
   int chunk_step;                // accumulator columns from one chunk to the next
