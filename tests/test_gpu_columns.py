@@ -88,6 +88,26 @@ def test_pairs_against_the_oracle(ctx, tmp_path, dtype, n, h, w_, c, k, ks, d, g
     assert np.array_equal(y.to_host(), one.to_host())      # the same sums
 
 
+# filters that stay for all tiles of a CTA (several per CTA): one and more channel blocks, groups that divide the CTAs
+# and groups that leave some of them out, and numbers of blocks that do not fit
+STAY = [(40, 24, 64, 1), (40, 64, 64, 1), (40, 128, 64, 1), (40, 100, 36, 1), (40, 130, 64, 1), (20, 128, 128, 2), (6, 512, 512, 8), (6, 256, 256, 8),
+        (3, 96, 96, 3), (40, 256, 57, 1)]
+
+
+@DTYPES
+@pytest.mark.parametrize("n,c,k,g,pair", [a + (p,) for a in STAY for p in (False, True) if not p or a[2] // a[3] > 32])
+def test_filters_that_stay(ctx, tmp_path, dtype, n, c, k, g, pair):
+    rs = np.random.RandomState(k)
+    kw = dict(border_mode="half", num_groups=g)
+    x = rs.standard_normal((n, c, 56, 54)).astype(dtype)
+    w = (rs.standard_normal((k, c // g, 3, 3)) / np.sqrt(9 * c // g)).astype(dtype)
+    X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
+    y = columns_only(ctx, str(tmp_path / "t"), lambda: shim.device_conv2d(X, W, **kw), pair=pair)
+    some = [0, n // 2, n - 1]
+    ref = O.conv2d(x[some].astype(F), w.astype(F), **kw)
+    assert O.rel_err(y.to_host()[some].astype(F), ref) < tol(dtype)
+
+
 @DTYPES
 @pytest.mark.parametrize("pair", [False, True])
 @pytest.mark.parametrize("n,h,w_,c,k", [(2, 28, 30, 24, 64), (3, 10, 62, 40, 64), (40, 56, 56, 24, 64)])

@@ -1051,9 +1051,12 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   if (!fits(2, 2, 1)) p.rps = 1;
   if (!fits(2, 2, 1)) return 2;
   if (!launch) return 0;
-  // A CTA whose tiles are all of one group loads the filters once where the ring holds them whole.
-  const int per_tile = (int)cdiv(a.Cin_g, kBK) * (p.kH / p.rps), units = pair ? c->num_sms / 2 : c->num_sms;
-  p.resident = units % a.groups == 0 && per_tile <= kMaxColStages && fits(2, per_tile, 1);
+  // A CTA whose tiles are all of one group loads the filters once where the ring holds them whole.  For that the CTAs are a multiple of
+  // the groups.  Those left out may cost one tile in fourteen: 3x3 on 8 groups of 32 channels, 256 images, float32, 144 CTAs for 148:
+  // 15 tiles for 14 each (14x14) 30.6 -> 30.1 us, 57 for 56 (28x28) 100 -> 91.
+  const int per_tile = (int)cdiv(a.Cin_g, kBK) * (p.kH / p.rps), units = pair ? c->num_sms / 2 : c->num_sms, whole = units / a.groups * a.groups;
+  const long long pix_tiles = cdiv(Wt, p.wt) * cdiv(Ht, p.th) * a.N, tiles = (pair ? (pix_tiles + 1) / 2 : pix_tiles) * a.groups;
+  p.resident = whole > 0 && per_tile <= kMaxColStages && fits(2, per_tile, 1) && 14 * cdiv(tiles, whole) <= 15 * cdiv(tiles, units);
   if (p.resident) p.b_stages = per_tile;
   for (char step : {'s', 'b', 'f', 'b', 's', 'b', 'b'}) {
     if (step == 'b' && p.resident) continue;

@@ -14,7 +14,10 @@
 // 134 -> 46.  64 filters: float16 at 56x56, 256 images 73 -> 75, float32 at 224x224, 16 images 140 -> 133 (pairs of the slab kernel 136): an MMA
 // of 192 columns runs at its rate, but 72 KB of filters per 112 pixels come from L2.  On pairs (PAIR: two pixel tiles, M = 256, each CTA
 // loading 32 of the 64 filters) 128 -> 64 at 112x112, 64 images, float32 247 -> 197 (columns on single CTAs 243, slab pairs 225 to 247; 149 if the
-// activations came for nothing: three slabs of 24 KB in flight beside two filter stages of 36 KB), 64 -> 64 at 224x224 127, float16 80.
+// activations came for nothing: three slabs of 24 KB in flight beside two filter stages of 36 KB; a fourth slab changes nothing), 64 -> 64 at
+// 224x224 127, float16 80.
+// Filters that fit their ring whole stay in it (`resident`): 64 -> 64 at 224x224, 16 images, on pairs 128 -> 120, 64 images 511 -> 459, with
+// pooling 508 -> 495; the 8 groups 100 -> 91.  128 -> 64 fits beside two slabs and half of the staging only, and is slower so (205 -> 216).
 //
 // Warp roles (640 threads): warp 0 streams slabs (tile and halo, 128 bytes of channels per pixel), warp 19 filter rows, warps 1
 // and 18 issue the MMAs of one accumulator each, 16 epilogue warps (TMEM -> shuffles -> staged TMA stores, with 2x2 max pooling,
@@ -468,7 +471,7 @@ cudaError_t launch_one(const ColsConvParams& p, long long total, int num_sms, cu
   cudaError_t e = configured.ensure([] { return cudaFuncSetAttribute(conv_cols_kernel<KIND, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024); });
   if (e != cudaSuccess) return e;
   const int smem = p.s_stages * p.slab_bytes + p.b_stages * p.rps * p.kW * (PAIR ? p.bn / 2 : p.bn) * 128 + p.stage_nbuf * p.stage_bytes + static_cast<int>(sizeof(Bars)) + 1024;
-  const int units = PAIR ? num_sms / 2 : num_sms, grid = static_cast<int>(total < units ? total : units) * (PAIR ? 2 : 1);
+  const int all = PAIR ? num_sms / 2 : num_sms, units = p.resident ? all / p.groups * p.groups : all, grid = static_cast<int>(total < units ? total : units) * (PAIR ? 2 : 1);
   launch_linked(true, conv_cols_kernel<KIND, PAIR>, grid, kThreads, smem, s, PAIR ? 2 : 1, p);
   return cudaGetLastError();
 }
@@ -481,7 +484,7 @@ cudaError_t launch_conv_cols(const ColsConvParams& p, int dtype, int num_sms, cu
   if (p.pair && (p.bn != 64 || p.d2s || p.n_acc != 1 || num_sms < 2)) return cudaErrorInvalidValue;
   if (total >= (1LL << 31) || p.n_acc < 1 || p.n_acc > 2 || p.sets < 2 || p.sets > kMaxSets || (p.step != p.sets && (p.step != 1 || p.sets != 2)) || p.sets * p.n_acc * p.kW * p.bn > 512 || p.kH > kMaxColTaps || p.rps < 1 || p.kH % p.rps || p.kW > kMaxColTaps ||
       p.s_stages < 2 || p.s_stages > kMaxStages || p.b_stages < (p.resident ? 1 : 2) || p.b_stages > kMaxStages ||
-      (p.resident && (p.b_stages != p.kblocks * (p.kH / p.rps) || (p.pair ? num_sms / 2 : num_sms) % p.groups))) return cudaErrorInvalidValue;
+      (p.resident && (p.b_stages != p.kblocks * (p.kH / p.rps) || (p.pair ? num_sms / 2 : num_sms) < p.groups))) return cudaErrorInvalidValue;
   if (p.pair) return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, true>(p, total, num_sms, s) : launch_one<MmaKind::TF32, true>(p, total, num_sms, s);
   return dtype == B200CONV_F16 ? launch_one<MmaKind::F16, false>(p, total, num_sms, s) : launch_one<MmaKind::TF32, false>(p, total, num_sms, s);
 }
