@@ -81,3 +81,28 @@ def test_tiles_behind_the_last_whole_wave_are_cut(ctx, dtype, relu):
     assert O.rel_err(y[part].astype(F), np.maximum(ref, 0) if relu else ref) < tol(dtype)
     ctx.set_pair_kernels(False)
     assert O.rel_err(y.astype(F), call().astype(F)) < (1e-5 if dtype == F else 1e-3)
+
+
+# sides that tiles divide and that they do not, tiles of several images, filters off the tile width, a cut launch, more tiles than images
+@DTYPES
+@pytest.mark.parametrize("n,h,w_,c,k", [(61, 14, 14, 40, 128), (60, 16, 10, 64, 192), (25, 28, 28, 512, 128), (9, 34, 30, 33, 320), (90, 6, 70, 64, 256)])
+def test_pooling(ctx, tmp_path, dtype, n, h, w_, c, k):
+    rs = np.random.RandomState(n)
+    x = rs.standard_normal((n, c, h, w_)).astype(dtype)
+    w = (rs.standard_normal((k, c, 3, 3)) / np.sqrt(c * 9)).astype(dtype)
+    b = rs.standard_normal((1, k, 1, 1)).astype(dtype)
+    X, W, B = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), T.from_host(ctx, b)
+    call = lambda pool: shim.device_conv2d(X, W, border_mode="half", bias=B, relu=True, pool=pool)  # noqa: E731
+    ctx.set_autotune(True)
+    call(True)
+    path = str(tmp_path / "t")
+    ctx.tuning_save(path)
+    head, *rest = open(path).read().splitlines()
+    open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + ["5"]) if r.startswith("a 3.") else r for r in rest]) + "\n")
+    ctx.tuning_load(path)
+    y = call(True).to_host().astype(F)
+    assert ctx.last_variant == ("tap pair cut" if n == 25 else ctx.last_variant) and ctx.last_variant.startswith("tap pair")
+    ctx.set_autotune(False)
+    full = call(False).to_host().astype(F)[:, :, :h // 2 * 2, :w_ // 2 * 2]
+    ref = full.reshape(n, k, h // 2, 2, w_ // 2, 2).max(axis=(3, 5))
+    assert O.rel_err(y, ref) < (1e-5 if dtype == F else 1e-3)      # the same products, sums in another order

@@ -411,17 +411,17 @@ int validate(b200conv_ctx* c, const b200conv_desc* d) {
 }
 
 // Pixel tile for a grid of Wt x Ht x N positions holding at most `cap` rows: fewest tiles,
-// each tile weighted by the MMA steps it costs (`kk` rows per step); widest box on ties.
-void choose_tile(b200conv_ctx* c, int Wt, int Ht, int N, int cap, int kk, int* bw, int* bh, int* bn) {
-  SlabTile& memo = c->pixel_tiles[GeoKey{kGeoTile, Wt, Ht, N, cap, kk}];
+// each tile weighted by the MMA steps it costs (`kk` rows per step); widest box on ties.  even 2: sides that pooling windows do not straddle.
+void choose_tile(b200conv_ctx* c, int Wt, int Ht, int N, int cap, int kk, int* bw, int* bh, int* bn, int even = 1) {
+  SlabTile& memo = c->pixel_tiles[GeoKey{kGeoTile, Wt, Ht, N, cap, kk, even}];
   if (memo.found) {
     *bw = memo.wt; *bh = memo.th; *bn = memo.nb;
     return;
   }
   long long best = -1;
   *bw = *bh = *bn = 1;
-  for (int w = 1; w <= std::min(Wt, cap); ++w) {
-    for (int h = 1; h <= std::min(Ht, cap / w); ++h) {
+  for (int w = even; w <= std::min(round_up(Wt, even), cap); w += even) {
+    for (int h = even; h <= std::min(round_up(Ht, even), cap / w); h += even) {
       const int n = std::max(1, std::min(N, cap / (w * h)));
       const long long tiles = cdiv(Wt, w) * cdiv(Ht, h) * cdiv(N, n);
       const long long cost = tiles * (kk > 0 ? cdiv(w * h * n, kk) : 1);
@@ -696,7 +696,7 @@ SlabTile find_slab_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt
 // slices of the reduction where that occupies more SMs.
 SlabTile tap_tile(b200conv_ctx* c, const FwdLikeArgs& a, int ntaps, int Wt, int Ht, bool spread) {
   SlabTile best;
-  choose_tile(c, Wt, Ht, a.N, 128, 0, &best.wt, &best.th, &best.nb);
+  choose_tile(c, Wt, Ht, a.N, 128, 0, &best.wt, &best.th, &best.nb, c->epi.pool ? 2 : 1);
   best.bn = conv_umma_bn(a.n_out);
   best.found = true;
   if (!spread) return best;
@@ -1100,7 +1100,7 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
 // Can the per-tap kernel run on pairs of CTAs: staged TMA stores of whole 128-byte channel rows, tiles of at least 128 filters?
 bool tap_pair_ok(b200conv_ctx* c, const FwdLikeArgs& a, const void* out, long long sn, long long sc, long long sh, long long sw, long long off) {
   const long long es = (long long)elem_size(a.dtype);
-  return c->use_pair && c->num_sms >= 2 && a.n_out > 64 && a.n_out % (int)(128 / es) == 0 && sc == 1 && !c->epi.residual && !c->epi.pool &&
+  return c->use_pair && c->num_sms >= 2 && a.n_out > 64 && a.n_out % (int)(128 / es) == 0 && sc == 1 && !c->epi.residual &&
          ((sw | sh | sn) * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * es) % 16 == 0;
 }
 
@@ -1175,15 +1175,18 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
   p.wait_clocks = c->wait_clocks;
   if (pair) {
     const long long es = (long long)elem_size(a.dtype), tiles = cdiv(1LL * p.tiles_w * p.tiles_h * p.tiles_n, 2) * p.groups * p.tiles_co;
-    cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)Wt, (cuuint64_t)Ht, (cuuint64_t)a.N};
+    const int pl = c->epi.pool ? 2 : 1;
+    cuuint64_t dims[4] = {(cuuint64_t)a.n_out * a.groups, (cuuint64_t)(Wt / pl), (cuuint64_t)(Ht / pl), (cuuint64_t)a.N};
     cuuint64_t strides[3] = {(cuuint64_t)(sw * es), (cuuint64_t)(sh * es), (cuuint64_t)(sn * es)};
-    cuuint32_t box[4] = {(cuuint32_t)kBK, (cuuint32_t)p.bw, (cuuint32_t)p.bh, (cuuint32_t)p.bn};
+    cuuint32_t box[4] = {(cuuint32_t)kBK, (cuuint32_t)(p.bw / pl), (cuuint32_t)(p.bh / pl), (cuuint32_t)p.bn};
     cuuint32_t estr[4] = {1, 1, 1, 1};
     CUresult r = c->encode(&p.out_map, a.dtype == B200CONV_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4,
                            static_cast<char*>(out) + off * es, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS && c->epi.pool) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
     if (r != CUDA_SUCCESS) return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, kConvTap);
-    const PairCut cut = pair_cut(tiles, c->num_sms / 2, 1LL * p.ntaps * p.kblocks, BN);
+    PairCut cut = pair_cut(tiles, c->num_sms / 2, 1LL * p.ntaps * p.kblocks, BN);
+    if (c->epi.pool && (cut.tiles >= tiles || 2 * cut.tiles > kArrivals)) cut = PairCut{0, 1};      // the pair that adds the slices pools
     p.cut = (int)cut.tiles; p.splits = cut.splits;
     Scratch tmp(c);
     ConvReduceParams q;
@@ -1296,6 +1299,10 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       if (rc != 2) return rc;
       variant = kConvSlab;
     }
+    if (c->epi.pool && variant == kConvTapPair && tap_pair_ok(c, a, out, sn, sc, sh, sw, off)) {
+      const int rc = run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant);
+      if (rc != B200CONV_E_UNSUPPORTED) return rc;
+    }
     if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
       const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
                                    relu, slab_mode(variant));
@@ -1334,12 +1341,11 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   if (!c->epi.pool) {
     cand[ncand++] = kConvTap;
     if (tap_spread) cand[ncand++] = kConvTapSpread;
-    const int bn = conv_umma_bn(a.n_out);
-    const SlabTile t = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, false);
-    if (tap_pair_ok(c, a, out, sn, sc, sh, sw, off) &&
-        cdiv(cdiv(Wt, t.wt) * cdiv(Ht, t.th) * cdiv(a.N, t.nb), 2) * cdiv(a.n_out, bn) * a.groups >= c->num_sms / 4)
-      cand[ncand++] = kConvTapPair;
   }
+  const SlabTile t = tap_tile(c, a, (int)taps_in.size(), Wt, Ht, false);
+  if (tap_pair_ok(c, a, out, sn, sc, sh, sw, off) &&
+      cdiv(cdiv(Wt, t.wt) * cdiv(Ht, t.th) * cdiv(a.N, t.nb), 2) * cdiv(a.n_out, t.bn) * a.groups >= c->num_sms / 4)
+    cand[ncand++] = kConvTapPair;
   for (int v = kConvCols; allow_slab && v <= kConvColsPair; ++v)
     if (try_conv_cols(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, false, v == kConvColsPair) == 0)
       cand[ncand++] = v;

@@ -17,6 +17,8 @@
 // Measured (a B200, filters packed, one-CTA kernel -> pairs): float16, 256 images, 3x3 256 -> 256 at 14x14 48 -> 43 us (37 without any
 // loads), 512 -> 512 at 7x7 (106 pair tiles, 32 of them cut in two) 52 -> 42, strided 1024 -> 2048 1x1 52 -> 45; float32 256 -> 256 at 14x14, 128 images
 // (98 tiles, 24 cut in three) 58 -> 42, 512 -> 512, 64 images 100 -> 76.  With the slices added by a kernel of its own the cut ones took 46, 51 and 82.
+// With 2x2 max pooling in the epilogue (slab kernel on pairs -> here), float32, 64 images: 512 -> 512 at 28x28 365 -> 312, at 14x14 103 -> 85,
+// 256 -> 256 at 56x56 346 -> 329.
 // Flattened 1x1 layers stay with gemm_pair.cu (256 -> 1024 at 14x14 33 us here, 31 there).
 #include "internal.h"
 #include "ptx.cuh"
@@ -52,6 +54,19 @@ __device__ __forceinline__ Item item_of(const UmmaConvParams& p, uint32_t item, 
   if (item >= slices) return Item{item - slices + p.cut, 0, kiters, -1};
   const uint32_t t = quotient(item, p.walk.splits), s = item - t * splits;
   return Item{t, kiters * s / splits, kiters * (s + 1) / splits, static_cast<int>(s)};
+}
+
+// The larger of each of the float or half numbers in 16 bytes.
+template <class T>
+__device__ __forceinline__ uint4 larger(uint4 a, uint4 b) {
+  if (sizeof(T) == 4) {
+    auto most = [](uint32_t x, uint32_t y) { return __float_as_uint(fmaxf(__uint_as_float(x), __uint_as_float(y))); };
+    return make_uint4(most(a.x, b.x), most(a.y, b.y), most(a.z, b.z), most(a.w, b.w));
+  }
+  __half2 *ah = reinterpret_cast<__half2*>(&a), *bh = reinterpret_cast<__half2*>(&b);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) ah[e] = __hmax2(ah[e], bh[e]);
+  return a;
 }
 
 template <MmaKind KIND, int BN>
@@ -294,10 +309,38 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
               }
             }
           }
+          if (p.epi.pool) {
+            // 2x2 max pooling of the staged chunk, as in conv_slab.cu: the tile's sides are even, the maxima stay in registers until all rows
+            // are read, then go to the front of the buffer
+            named_barrier(1 + grp, 128);
+            const int pw = p.bw >> 1, ph = p.bh >> 1, prows = p.bn * ph * pw;
+            uint4 keep[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int i = row + u * 128, pr = i >> 3, piece = i & 7;
+              if (pr < prows) {
+                const int pl = pr / pw, w2 = pr - pl * pw, img = pl / ph, d00 = (img * p.bh + 2 * (pl - img * ph)) * p.bw + 2 * w2;
+                uint4 m = *reinterpret_cast<const uint4*>(stg + d00 * 128 + ((piece ^ (d00 & 7)) << 4));
+#pragma unroll
+                for (int k = 1; k < 4; ++k) {
+                  const int dk = d00 + (k & 1) + (k >> 1) * p.bw;
+                  m = larger<OutT>(m, *reinterpret_cast<const uint4*>(stg + dk * 128 + ((piece ^ (dk & 7)) << 4)));
+                }
+                keep[u] = m;
+              }
+            }
+            named_barrier(1 + grp, 128);
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int i = row + u * 128, pr = i >> 3, piece = i & 7;
+              if (pr < prows) *reinterpret_cast<uint4*>(stg + pr * 128 + ((piece ^ (pr & 7)) << 4)) = keep[u];
+            }
+          }
           fence_async_smem();
           named_barrier(1 + grp, 128);
           if (issuer && n0 < p.Nimg && B200_IN_RANGE(w0 >= 0 && w0 < p.Wt && h0 >= 0 && h0 < p.Ht && n0 >= 0 && co0 >= 0, p.status)) {
-            tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0, h0, n0);
+            if (p.epi.pool) tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0 >> 1, h0 >> 1, n0);
+            else tma_store_4d(&p.out_map, stg, g * p.n_out + co0, w0, h0, n0);
             bulk_commit();
           }
         }
