@@ -1303,7 +1303,7 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
       const int rc = run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, variant);
       if (rc != B200CONV_E_UNSUPPORTED) return rc;
     }
-    if (c->epi.pool) {                // the slab kernel pools, in its staged epilogue or in the reduction of its slices
+    if (c->epi.pool) {                // else the slab kernel pools, in its staged epilogue or in the reduction of its slices
       const int rc = try_conv_slab(c, a, taps_in, view_parity[0].first, view_parity[0].second, Wt, Ht, out, sn, sc, sh, sw, off, bias,
                                    relu, slab_mode(variant));
       return rc == 2 ? fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool") : rc;
