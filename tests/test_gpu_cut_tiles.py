@@ -1,5 +1,7 @@
 """Cut tiles whose slices are added by the CTA that leaves the last one: results repeat bit by bit over calls, graphs and contexts, and the
 counts of arrivals are back at zero after a wait that ran out."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -52,4 +54,40 @@ def test_counts_start_again_after_a_wait_ran_out():
     ctx.set_wait_limit(4000000000)
     call()
     assert np.array_equal(y, Y.to_host())
+    ctx.close()
+
+
+def test_a_context_made_while_the_default_stream_is_busy():
+    """The counts of a new context are zero before its first launch, whatever another library has queued on the default stream and
+    whatever their memory held before."""
+    torch = pytest.importorskip("torch")
+    ctx = shim.Context(0)
+    ctx.set_autotune(False)
+    X, W, Y, call = layer(ctx, np.float32)
+    call()
+    y = Y.to_host()
+    cudart = ctypes.CDLL("libcudart.so.12")
+    big = torch.empty(1 << 30, dtype=torch.float32, device="cuda")
+    blocks = [ctypes.c_void_p() for _ in range(512)]
+    for b in blocks:
+        assert cudart.cudaMalloc(ctypes.byref(b), ctypes.c_size_t(4096)) == 0
+        assert cudart.cudaMemset(b, 255, ctypes.c_size_t(4096)) == 0
+    torch.cuda.synchronize()
+    for b in blocks:
+        assert cudart.cudaFree(b) == 0
+    for _ in range(300):                             # some 180 ms of the default stream
+        big.fill_(1.0)
+    busy = torch.cuda.Event()
+    busy.record()
+    other = shim.Context(0)
+    other.set_autotune(False)
+    x, w, out = (T(other, t.shape, t.dtype, t.layout, _ptr=t.ptr) for t in (X, W, Y))
+    other.memset(out.ptr, 255, out.nbytes)
+    shim.device_conv2d(x, w, border_mode="half", out=out, flags=shim.NO_SLAB)
+    assert other.last_variant == "tap pair cut"
+    other.sync()
+    assert not busy.query()                          # the default stream was busy all the while
+    torch.cuda.synchronize()
+    assert np.array_equal(y, out.to_host())
+    other.close()
     ctx.close()

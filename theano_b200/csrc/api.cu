@@ -3085,7 +3085,7 @@ int b200conv_create(int device, b200conv_ctx** out) {
             cudaHostAlloc(&hs, sizeof(int), cudaHostAllocMapped) == cudaSuccess &&
             cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->d_status), hs, 0) == cudaSuccess &&
             cudaMalloc(reinterpret_cast<void**>(&c->d_arrivals), kArrivals * sizeof(unsigned int)) == cudaSuccess &&
-            cudaMemset(c->d_arrivals, 0, kArrivals * sizeof(unsigned int)) == cudaSuccess &&
+            cudaMemsetAsync(c->d_arrivals, 0, kArrivals * sizeof(unsigned int), c->stream) == cudaSuccess &&      // a non-blocking stream waits for no other
             cudaEventCreate(&c->ev0) == cudaSuccess && cudaEventCreate(&c->ev1) == cudaSuccess;
   if (ok) {
     c->h_status = static_cast<volatile int*>(hs);
