@@ -138,3 +138,22 @@ def test_an_infinity_stays_with_the_outputs_that_it_belongs_to(ctx, tmp_path, dt
     ctx.d2h(stored, Y.ptr)
     ctx.sync()
     assert not stored[..., 30:].any()
+
+
+@DTYPES
+@pytest.mark.parametrize("h,ks,d", [(150, (3, 3), (128, 1)), (260, (2, 4), (256, 2)), (40, (5, 3), (64, 1)), (150, (3, 2), (127, 1))])
+def test_filters_that_reach_over_256_rows(ctx, dtype, h, ks, d):
+    """Dilated filters of a box's 256 rows and about: no tile of the columns kernel holds them, the layer runs on another."""
+    rs = np.random.RandomState(h)
+    kw = dict(border_mode="half", filter_dilation=d)
+    x = rs.standard_normal((2, 20, h, 17)).astype(dtype)
+    w = (rs.standard_normal((24, 20) + ks) / np.sqrt(20 * ks[0] * ks[1])).astype(dtype)
+    X, W = T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w)
+    ref = O.conv2d(x.astype(F), w.astype(F), **kw)
+    y = shim.device_conv2d(X, W, **kw)
+    assert not ctx.last_variant.startswith("columns")
+    assert O.rel_err(y.to_host().astype(F), ref) < tol(dtype)
+    dy = rs.standard_normal(ref.shape).astype(dtype)
+    dx = shim.device_grad_inputs(W, T.from_host(ctx, dy, "nhwc"), (h, 17), **kw)
+    assert not ctx.last_variant.startswith("columns")
+    assert O.rel_err(dx.to_host().astype(F), O.conv2d_grad_inputs(w.astype(F), dy.astype(F), (h, 17), **kw)) < tol(dtype)

@@ -1018,22 +1018,11 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.chunk_step = pair ? kW * step : 32;
   p.chunk_ch = std::min(32, p.bn);        // 32 at most: the groups of epilogue warps share a tile
   if (!d2s_C && a.groups > 1 && a.n_out % p.chunk_ch) return 2;
-  // Tile: the pitch that leaves the fewest accumulator rows to compute; two accumulators where two sets of them fit 512 columns.
+  // two accumulators where two sets of them fit 512 columns
   const int even = c->epi.pool ? 2 : 1, most_acc = 4 * n_cols <= 512 && !pair ? 2 : 1;
-  long long best = -1;
-  for (int pitch : {32, 16, 8})
-    for (int n_acc = most_acc; n_acc >= 1; --n_acc) {
-      const int widest = (pitch - Ew) / even * even, rows = 128 / pitch * n_acc / even * even;
-      if (widest < 1 || rows < 1) continue;
-      const int tw = (int)cdiv(Wt, widest), th_n = (int)cdiv(Ht, std::min(rows, 256 - Eh));
-      // clocks of the MMAs: with two accumulators each has an issuer of its own; one alone waits for itself (71 against 117 clocks per 128 x 96)
-      const long long work = 1LL * tw * th_n * n_acc * (n_cols > 128 ? 1 : n_acc == 2 ? 6 : 10);
-      if (256 - Eh < 1 || (best >= 0 && work >= best)) continue;
-      best = work;
-      p.pitch = pitch; p.n_acc = n_acc;
-      p.wt = round_up((int)cdiv(Wt, tw), even); p.th = round_up((int)cdiv(Ht, th_n), even);
-    }
-  if (best < 0) return 2;
+  const ColsTile tile = cols_tile(Wt, Ht, Eh, Ew, n_cols, most_acc, even);
+  if (!tile.found) return 2;
+  p.wt = tile.wt; p.th = tile.th; p.pitch = tile.pitch; p.n_acc = tile.n_acc;
   p.Hs = p.th + Eh;
   p.slab_bytes = std::max(p.Hs * p.pitch, 128 * p.n_acc + Eh * p.pitch) * 128;
   p.slab_bytes = (p.slab_bytes + 1023) / 1024 * 1024;

@@ -4,6 +4,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "../../include/b200conv.h"
 
 namespace b200 {
@@ -69,6 +71,31 @@ inline int merge_factor_wgrad(const b200conv_desc& d) {
   for (int m = 2; m <= d.groups && Cg * m <= 128 && Kg * m <= 128; ++m)
     if (d.groups % m == 0 && umma_ok(merged_groups(d, m))) best = m;
   return best > 1 || umma_ok(d) ? best : merge_factor(d);
+}
+
+// Tile of the columns kernel (conv_cols.cu) for taps that reach Eh rows and Ew columns beyond their first: the pitch that leaves the fewest
+// accumulator rows to compute; at most `most_acc` accumulators of 128 rows, `n_cols` columns each; even 2: sides that pooling windows do not
+// straddle.  `found` is false where no row fits a pitch, or no tile a box of 256 rows.
+struct ColsTile {
+  int wt, th, pitch, n_acc;
+  bool found;
+};
+inline ColsTile cols_tile(int Wt, int Ht, int Eh, int Ew, int n_cols, int most_acc, int even) {
+  ColsTile best = {0, 0, 0, 0, false};
+  if (Eh > 256 - even) return best;
+  long long least = 0;
+  for (int pitch : {32, 16, 8})
+    for (int n_acc = most_acc; n_acc >= 1; --n_acc) {
+      const int widest = (pitch - Ew) / even * even, rows = 128 / pitch * n_acc, most = rows < 256 - Eh ? rows : 256 - Eh, tallest = most / even * even;
+      if (widest < 1 || tallest < 1) continue;
+      const int tw = static_cast<int>(cdiv(Wt, widest)), th_n = static_cast<int>(cdiv(Ht, tallest));
+      // clocks of the MMAs: with two accumulators each has an issuer of its own; one alone waits for itself (71 against 117 clocks per 128 x 96)
+      const long long work = 1LL * tw * th_n * n_acc * (n_cols > 128 ? 1 : n_acc == 2 ? 6 : 10);
+      if (best.found && work >= least) continue;
+      least = work;
+      best = ColsTile{round_up(static_cast<int>(cdiv(Wt, tw)), even), round_up(static_cast<int>(cdiv(Ht, th_n)), even), pitch, n_acc, true};
+    }
+  return best;
 }
 
 }  // namespace b200
