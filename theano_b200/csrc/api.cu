@@ -303,7 +303,8 @@ int check_status(b200conv_ctx* c) {
   const int st = *c->h_status;
   if (st != kStatusOk) {
     *c->h_status = 0;
-    cudaMemsetAsync(c->d_arrivals, 0, kArrivals * sizeof(unsigned int), c->stream);     // a launch that gave up leaves its counts behind
+    // a launch that gave up may leave its counts behind
+    CU_OK(c, cudaMemsetAsync(c->d_arrivals, 0, kArrivals * sizeof(unsigned int), c->stream));
     if (st == kStatusBadIndex)
       return fail(c, B200CONV_E_CUDA, "a kernel of the range-checked build computed an index outside its buffer "
                   "(the access was skipped); results are invalid");
@@ -3623,7 +3624,7 @@ int b200conv_selftest_wait(b200conv_ctx* c) {
   std::lock_guard<std::mutex> g(c->mu);
   DeviceGuard dg(c->device);
   if (c->capturing) return fail(c, B200CONV_E_INVALID, "not allowed while a graph is being captured");
-  CU_OK(c, launch_wait_selftest(c->d_status, c->wait_clocks, c->stream));
+  CU_OK(c, launch_wait_selftest(c->d_status, c->d_arrivals, kArrivals, c->wait_clocks, c->stream));
   return sync_and_check(c);
 }
 

@@ -554,7 +554,7 @@ cudaError_t launch_channel_sum(const void* x, float* partial, void* out, long lo
                                cudaStream_t st);
 
 // ---- bounded-wait self-test (selftest.cu): one CTA waits, with `limit`, on a barrier nobody arrives on
-cudaError_t launch_wait_selftest(int* status, long long limit, cudaStream_t s);
+cudaError_t launch_wait_selftest(int* status, unsigned int* arrivals, int narrivals, long long limit, cudaStream_t s);
 
 // ---- CUDA-core direct kernels (conv_direct.cu) ---------------------------------------------
 cudaError_t launch_direct_fwd(const b200conv_desc& d, const void* x, const void* w,

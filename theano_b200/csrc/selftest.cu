@@ -1,6 +1,7 @@
 // Self-test of the bounded device-side wait: a kernel that waits on a barrier nobody arrives on.
 // It exercises the path every tensor-core kernel takes when a wait runs out (status word written,
-// kernel returns, the context stays usable) without faulting or hanging anything.
+// kernel returns, the context stays usable) without faulting or hanging anything.  It also leaves counts of arrived slices behind
+// that are not zero, as a launch that gave up may; with these no slice would ever be found the last of its tile.
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -12,13 +13,14 @@ struct Bars {
   volatile int abort;
 };
 
-__global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int* status, long long limit) {
+__global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int* status, unsigned int* arrivals, int narrivals, long long limit) {
   __shared__ Bars bars;
   if (threadIdx.x == 0) {
     mbar_init(&bars.never, 1);
     bars.abort = 0;
     mbar_fence_init();
   }
+  for (int i = threadIdx.x; i < narrivals; i += blockDim.x) arrivals[i] = 0xFFFFFFFFu;
   __syncthreads();
   const int warp = uniform_warp_index();
   bool ok;
@@ -35,8 +37,8 @@ __global__ void __launch_bounds__(64, 1) wait_selftest_kernel(int* status, long 
 
 }  // namespace
 
-cudaError_t launch_wait_selftest(int* status, long long limit, cudaStream_t s) {
-  wait_selftest_kernel<<<1, 64, 0, s>>>(status, limit);
+cudaError_t launch_wait_selftest(int* status, unsigned int* arrivals, int narrivals, long long limit, cudaStream_t s) {
+  wait_selftest_kernel<<<1, 64, 0, s>>>(status, arrivals, narrivals, limit);
   return cudaGetLastError();
 }
 
