@@ -464,8 +464,10 @@ __device__ __forceinline__ void umma_commit_if(uint32_t lane, uint64_t* bar) {
       "@l tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lane)
       : "memory");
 }
-// 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base+t).
+// 32 lanes x 32 consecutive 32-bit columns: thread t of the warp gets lane (base+t).  A whole warp: the instruction wants its lanes
+// converged, and the callers' loops send lanes without a pixel past the stores, straight to the next load.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
@@ -478,7 +480,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr)
       : "memory");
 }
-// The same for 16 columns.
+// The same for 16 columns; the caller brings the warp together.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
