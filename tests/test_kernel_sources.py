@@ -32,3 +32,20 @@ def test_accumulators_are_read_by_converged_warps():
     assert users == ["conv_cols.cu"]                  # there the caller brings the warp together
     sums = body(source("conv_cols.cu"), "void column_sums")
     assert sums.index("__syncwarp()") < sums.index("add_columns<") and source("conv_cols.cu").count("tmem_ld16(") == 1
+
+
+def test_no_warp_leaves_others_at_a_named_barrier():
+    """A named barrier waits without a bound.  Warps whose items end at one may not leave their loop when a wait runs out: the warps beside
+    them may have seen that phase complete."""
+    seen = []
+    for f in KERNELS:
+        text = source(f)
+        if "named_barrier(" not in text:
+            continue
+        seen.append(f)
+        assert "warp_wait_or_abort(" not in text, f
+        for m in re.finditer(r"wait_or_walk_on\(", text):
+            head = text.rindex("for (", 0, m.start())
+            assert "ok" not in text[head:text.index("{", head)], (f, text[head:head + 120])
+            assert "break" not in text[head:text.index("named_barrier(", m.start())].split("wait_or_walk_on", 1)[0], f
+    assert seen == ["conv_slab.cu", "gemm_pair.cu", "conv_pair.cu", "conv_cols.cu", "wgrad_pair.cu"]

@@ -300,9 +300,9 @@ conv_cols_kernel(const __grid_constant__ ColsConvParams p) {
     bool ok = true;
     int buf = mine < p.sets ? mine : 0, nstore = 0;
     uint32_t phase = 0;
-    for (uint32_t t = mine < p.step ? first + mine * stride : total; t < total && ok; t += p.step * stride) {
+    for (uint32_t t = mine < p.step ? first + mine * stride : total; t < total; t += p.step * stride) {
       const Tile w = tile_of<PAIR>(p, t, rank);
-      if (!warp_wait_or_abort(&bars->acc_full[buf], phase, bars, lane, p.wait_clocks)) { ok = false; break; }
+      wait_or_walk_on(ok, &bars->acc_full[buf], phase, bars, lane, p.wait_clocks);
       tc_fence_after();
       const uint32_t acc0 = tmem + (buf * p.n_acc + a) * n_cols + p.col_first + (static_cast<uint32_t>(quad * 32) << 16);
       // the accumulator goes back as soon as its last columns are in registers

@@ -206,12 +206,12 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
     uint8_t* srow = stg + row * 128;
     bool ok = true, stored = false;
     int it = 0, turn = 0;
-    for (uint32_t item = first; item < total && ok; item += stride, ++it) {
+    for (uint32_t item = first; item < total; item += stride, ++it) {
       const Item w = item_of(p, item, kiters);
       const TileAt at = tile_at<true>(p.walk, w.tile, rank);
       const int co_t = at.co_t, g = at.g, w0 = at.w * p.bw, h0 = at.h * p.bh, n0 = at.n * p.bn;
       const int buf = it & 1;
-      if (!warp_wait_or_abort(&bars->acc_full[buf], (it >> 1) & 1, bars, lane, p.wait_clocks)) { ok = false; break; }
+      wait_or_walk_on(ok, &bars->acc_full[buf], (it >> 1) & 1, bars, lane, p.wait_clocks);
       tc_fence_after();
       const int co_base = co_t * BN;
       const uint32_t lane_base = tmem + buf * BN + (static_cast<uint32_t>(quad * 32) << 16);

@@ -376,12 +376,12 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
     bool ok = true;
     int it = 0;
     int nstore = 0;                              // chunks this warp's group has staged so far
-    for (uint32_t item = first; item < total && ok; item += stride, ++it) {
+    for (uint32_t item = first; item < total; item += stride, ++it) {
       const TileAt at = tile_at<PAIR>(p.walk, quotient(item, p.walk.splits), rank);
       const int co_t = at.co_t, g = at.g, w0 = at.w * p.wt, h0 = at.h * p.th, n0 = at.n * p.nb;
       const int buf = dbl ? (it & 1) : 0;
       const uint32_t aphase = dbl ? ((it >> 1) & 1) : (it & 1);
-      if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
+      wait_or_walk_on(ok, &bars->acc_full[buf], aphase, bars, lane, p.wait_clocks);
       tc_fence_after();
       if (trace && it == 0 && threadIdx.x == 64) trace[4] = clock64();
       const int co_base = co_t * BN;

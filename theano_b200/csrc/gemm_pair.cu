@@ -145,12 +145,12 @@ gemm_pair_kernel(const __grid_constant__ PairGemmParams p) {
     uint8_t* srow = stg + drow * 128;
     bool ok = true;
     int it = 0, nstore = 0;
-    for (uint32_t t = pair; t < total && ok; t += npairs, ++it) {
+    for (uint32_t t = pair; t < total; t += npairs, ++it) {
       const uint32_t pt = quotient(t, p.by_tiles_co);
       const int co_t = t - pt * p.tiles_co, pix0 = pt * 256 + rank * 128;
       const int buf = it & 1;
       const uint32_t aphase = (it >> 1) & 1;
-      if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
+      wait_or_walk_on(ok, &bars->acc_full[buf], aphase, bars, lane, p.wait_clocks);
       tc_fence_after();
       const int co_base = co_t * kBN;
       const int nstaged = min(kBN / 64, (p.n_out - co_base + 63) / 64);

@@ -195,6 +195,15 @@ __device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parit
   return ok != 0;
 }
 
+// The same for the epilogue warps that meet others at named barriers.  A warp that gave up waits for nothing more, but walks on through its
+// remaining items (what it reads and stores is void, and the call fails): the phase may have completed for the warps
+// beside it a moment later, and these would wait at the next named barrier, which has no bound, for ever.  So the loop
+// around it ends with its items and not with `ok`.
+template <class BarsT>
+__device__ __forceinline__ void wait_or_walk_on(bool& ok, uint64_t* bar, uint32_t parity, BarsT* b, int lane, long long limit) {
+  if (ok) ok = warp_wait_or_abort(bar, parity, b, lane, limit);
+}
+
 // ---- TMA ----------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");

@@ -227,11 +227,11 @@ wgrad_pair_kernel(const __grid_constant__ UmmaWgradParams p) {
     bool ok = true;
     int n = 0;
     const int K = p.Kg * p.groups;
-    for (uint32_t it = pair; it < total && ok; it += npairs, ++n) {
+    for (uint32_t it = pair; it < total; it += npairs, ++n) {
       const Item w = decode(it, p, per_split, pix_tiles);
       const int buf = n & 1;
       const uint32_t aphase = (n >> 1) & 1;
-      if (!warp_wait_or_abort(&bars->acc_full[buf], aphase, bars, lane, p.wait_clocks)) { ok = false; break; }
+      wait_or_walk_on(ok, &bars->acc_full[buf], aphase, bars, lane, p.wait_clocks);
       tc_fence_after();
       const int kq = w.kt * 256 + static_cast<int>(rank) * 128 + row;
       const bool valid = kq < p.Kg;
