@@ -1215,8 +1215,9 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
 // events) of the best are timed again in bursts of up to 7 back to back (8 did as well), the way a program issues them, once,
 // and once more if they are still within 5 %.  Alone, a kernel of 5 us costs 5 us more and the chained launch hides nothing.
 // All variants in two bursts each made the first passes of 32 cases take 200 ms together, this and rough_times() 127.
+// `alone` takes the times of the single runs, those of variants that are then out of the running among them.
 template <class Run>
-int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool rough = false) {
+int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool rough = false, float* alone = nullptr) {
   if (!c->ev_tune0) {
     CU_OK(c, cudaEventCreate(&c->ev_tune0));
     CU_OK(c, cudaEventCreate(&c->ev_tune1));
@@ -1241,6 +1242,7 @@ int time_variants(b200conv_ctx* c, int n, Run run, float* ms, int* codes, bool r
     if ((codes[i] = run(i))) continue;
     if (int rc = timed(i, 1, &ms[i])) return rc;
   }
+  if (alone) std::copy(ms, ms + n, alone);
   const float first = best();
   if (first < 0.f || first > 0.5f || rough) return 0;     // long enough for one measurement
   const int reps = std::max(1, std::min(7, (int)(0.14f / std::max(first, 0.001f))));
@@ -1311,8 +1313,17 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   GeoKey key{kGeoConv, a.dtype, a.N, a.Hs, a.Ws, a.Cin_g, a.n_out, a.groups, Wt, Ht, a.view_sH, a.view_sW, (int)taps_in.size(), tsum};
   key.add(sc);
   key.add(sw);
-  key.add(c->epi.pool * 4 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
   const size_t es = elem_size(a.dtype);
+  // Channels-last outputs that the kernels with staged stores only (per-tap pairs, columns) cannot write, with a residual or off the 16-byte
+  // boundaries, have a choice of their own, timed on their first call: the layer's may be one of those, and the lanes' own stores are bound by
+  // other things (64 -> 32 3x3 at 112x112, 64 images, float32, with a residual: per-tap 205 us, slab 279; without, slab 117 of 150).  Where such a call may
+  // not be timed, the layer's choice serves, or the best of the others when the layer was timed, which its choice then carries along
+  // (choice + kConvVariants * (other + 1)).
+  const bool lane_stores = sc == 1 && (c->epi.residual || ((sw | sh | sn) * (long long)es) % 16 ||
+                                       reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16);
+  GeoKey lane_key = key;
+  key.add(c->epi.pool * 4 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
+  lane_key.add(8 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
   const bool tma = sc == 1 && a.n_out % (int)(128 / es) == 0 && !c->epi.residual && (sw * es) % 16 == 0 && (sh * es) % 16 == 0 &&
                    (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
   // what cannot pool does not depend on the choice that an earlier call left (a split reduction pools any output)
@@ -1320,9 +1331,19 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
 #ifdef B200CONV_TUNE
   if (getenv("B200_VARIANT")) return run(atoi(getenv("B200_VARIANT")));
 #endif
+  // A launch that adds to its own output (residual == y) must run once: it is not timed, and the choice is left to a
+  // later call that may repeat it.
+  const size_t out_bytes = es * out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
+  const bool in_place = c->epi.residual && overlap(c->epi.residual, out_bytes, out, out_bytes);
+  const bool timed = c->autotune && !c->capturing && !c->model_only && !in_place;
   if (c->autotune) {
-    auto it = c->algo_cache.find(key);
-    if (it != c->algo_cache.end()) return run(it->second);
+    auto it = c->algo_cache.find(lane_stores ? lane_key : key);
+    if (it != c->algo_cache.end()) return run(it->second % kConvVariants);
+    if (lane_stores && !timed && (it = c->algo_cache.find(key)) != c->algo_cache.end()) {
+      const int layers = it->second % kConvVariants, lanes = it->second / kConvVariants - 1;
+      if (layers <= kConvSlabPair) return run(layers);
+      if (lanes >= 0) return run(lanes);
+    }
   }
   // the variants that apply, the static preference last
   int cand[kConvVariants], ncand = 0;
@@ -1358,20 +1379,20 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     if (pair) cand[ncand++] = kConvSlabPair;
   }
   if (ncand == 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
-  // A launch that adds to its own output (residual == y) must run once: it is not timed, and the choice is left to a
-  // later call that may repeat it.
-  const size_t out_bytes = elem_size(a.dtype) * out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
-  const bool in_place = c->epi.residual && overlap(c->epi.residual, out_bytes, out, out_bytes);
-  if (!c->autotune || c->capturing || c->model_only || ncand == 1 || in_place) return run(cand[ncand - 1]);
-  int best = -1, codes[kConvVariants];
-  float ms[kConvVariants], best_ms = 0.f;
-  if (const int rc = time_variants(c, ncand, [&](int i) { return run(cand[i]); }, ms, codes)) return rc;
+  if (!timed || ncand == 1) return run(cand[ncand - 1]);
+  int best = -1, lane_best = -1, codes[kConvVariants];
+  float ms[kConvVariants], alone[kConvVariants], best_ms = 0.f, lane_ms = 0.f;
+  if (const int rc = time_variants(c, ncand, [&](int i) { return run(cand[i]); }, ms, codes, false, alone)) return rc;
   for (int i = 0; i < ncand; ++i) {
     if (codes[i] && !(codes[i] == B200CONV_E_UNSUPPORTED && c->epi.pool)) return codes[i];
     if (ms[i] >= 0.f && (best < 0 || ms[i] < best_ms)) { best = cand[i]; best_ms = ms[i]; }
+    // the best of those that write any output; a single run's time counts where it did not come to bursts
+    const float m = ms[i] >= 0.f ? ms[i] : alone[i];
+    if (cand[i] <= kConvSlabPair && m >= 0.f && (lane_best < 0 || m < lane_ms)) { lane_best = cand[i]; lane_ms = m; }
   }
   if (best < 0) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
-  c->algo_cache[key] = best;
+  if (lane_stores) c->algo_cache[lane_key] = best;
+  else c->algo_cache[key] = best > kConvSlabPair && lane_best >= 0 ? best + kConvVariants * (lane_best + 1) : best;
   return run(best);     // the last run may have been another variant: leave the output of the chosen one
 }
 
@@ -3710,7 +3731,7 @@ int b200conv_tuning_load(b200conv_ctx* c, const char* path, int* loaded) {
     const bool known = kind == 'a' ? (key.v[0] == kGeoConv && key.n == 17) || ((key.v[0] == kGeoWgrad || key.v[0] == kGeoClasses) && key.n == 19)
                                    : key.v[0] == kGeoSplits && key.n == 20;
     if (!known) continue;
-    if (kind == 'a' && val >= 0 && val < kConvVariants) { c->algo_cache[key] = val; ++n; }
+    if (kind == 'a' && val >= 0 && val < (key.v[0] == kGeoConv ? kConvVariants * (kConvSlabPair + 2) : kConvVariants)) { c->algo_cache[key] = val; ++n; }
     else if (kind == 's' && val >= 1) { c->split_cache[key] = val; ++n; }
   }
   fclose(f);
