@@ -74,3 +74,23 @@ def test_a_layers_choice_is_not_taken_for_outputs_it_cannot_write(tmp_path, dtyp
     assert choice(ctx, path) == (layers, others if layers > 4 else -1)
     ctx.free(room)
     ctx.close()
+
+
+def test_a_residual_has_a_choice_of_its_own_in_every_layout(tmp_path):
+    """A plain call's choice is not taken over: the call with a residual is timed (and counted) itself, once."""
+    for layout in ("nhwc", "nchw"):
+        ctx = shim.Context(0)
+        rs = np.random.RandomState(3)
+        x, w = rs.standard_normal((4, 32, 30, 30)).astype(F), rs.standard_normal((32, 32, 3, 3)).astype(F) / F(17)
+        X, W = T.from_host(ctx, x, layout), T.from_host(ctx, w)
+        Y = shim.device_conv2d(X, W, border_mode="half")
+        assert Y.layout == layout
+        out, counts = T(ctx, Y.shape, F, layout), []
+        for _ in range(3):
+            before = ctx.launches
+            shim.device_conv2d(X, W, border_mode="half", residual=Y, out=out)
+            counts.append(ctx.launches - before)
+        assert counts[0] >= 8 and counts[1] == counts[2] <= 4, counts       # two runs of each of the kernels; transposition, packing, convolution, sums
+        ref = O.conv2d(x, w, border_mode="half")
+        assert O.rel_err(out.to_host(), 2 * ref) < 5e-3
+        ctx.close()

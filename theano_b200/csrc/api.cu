@@ -1314,13 +1314,13 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   key.add(sc);
   key.add(sw);
   const size_t es = elem_size(a.dtype);
-  // Channels-last outputs that the kernels with staged stores only (per-tap pairs, columns) cannot write, with a residual or off the 16-byte
-  // boundaries, have a choice of their own, timed on their first call: the layer's may be one of those, and the lanes' own stores are bound by
-  // other things (64 -> 32 3x3 at 112x112, 64 images, float32, with a residual: per-tap 205 us, slab 279; without, slab 117 of 150).  Where such a call may
-  // not be timed, the layer's choice serves, or the best of the others when the layer was timed, which its choice then carries along
+  // Outputs that staged stores cannot write, with a residual or, channels-last, off the 16-byte boundaries, have a choice of their own, timed on
+  // their first call: the layer's may be a kernel that has no other stores (per-tap pairs, columns), and the lanes' own stores are bound by
+  // other things (64 -> 32 3x3 at 112x112, 64 images, float32, with a residual: per-tap 205 us, slab 279; NCHW without: 175, 150).  Where such a call
+  // may not be timed, the layer's choice serves, or the best of the others when the layer was timed, which its choice then carries along
   // (choice + kConvVariants * (other + 1)).
-  const bool lane_stores = sc == 1 && (c->epi.residual || ((sw | sh | sn) * (long long)es) % 16 ||
-                                       reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16);
+  const bool lane_stores = c->epi.residual || (sc == 1 && (((sw | sh | sn) * (long long)es) % 16 ||
+                                                           reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16));
   GeoKey lane_key = key;
   key.add(c->epi.pool * 4 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
   lane_key.add(8 + (c->use_pair ? 2 : 0) + (allow_slab ? 1 : 0));
