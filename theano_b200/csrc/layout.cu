@@ -39,7 +39,7 @@ __global__ void transpose_kernel(const T* __restrict__ in, T* __restrict__ out, 
 // bank is that of the layer's own groups and the packed form block-diagonal: a filter has channels of its own group only.
 // A block moves a patch of filters x channels with all its taps through shared memory: the taps of a filter's consecutive
 // channels are one run of OIHW, read in 16-byte pieces (elements at the ends of a run that lies off the 16-byte
-// boundaries), and leave as 16-byte pieces of the destination's rows.  Every call on its own filters waits for this kernel, and
+// boundaries, all on their way together: one after the other they took eight latencies), and leave as 16-byte pieces of the destination's rows.  Every call on its own filters waits for this kernel, and
 // what bounds it is latency: one round of loads (up to four pieces per thread) and one of stores.  Element by element it took
 // 10 rounds of each.  Forward / gradInputs calls with the packing (a B200, before -> now): 64 -> 64 3x3 at 28x28, 8 images, float16 9.6 -> 9.1 /
 // 11.9 -> 9.6 us; 100 -> 75 5x5, 37 images, float16 37.5 -> 28.5 / 35.4 -> 27.4; 256 -> 256 3x3 at 14x14, 128 images, float32 60.5 -> 56 / 66 -> 59.
@@ -72,31 +72,34 @@ __device__ __forceinline__ void pack_filters_block(const PackJob& q, int bx, int
   }
   for (int base = 0; base < nk * q.pieces; base += kPackThreads * kPackPieces) {
     uint4 v[kPackPieces];
-    uintptr_t from[kPackPieces], lo[kPackPieces], hi[kPackPieces];    // of the piece, of its run
     int to[kPackPieces];
 #pragma unroll
     for (int u = 0; u < kPackPieces; ++u) {
       const int i = base + u * kPackThreads + threadIdx.x, kk = i / q.pieces;
-      to[u] = (i + kk / V) * 16;
-      from[u] = lo[u] = hi[u] = 0;
+      to[u] = -1;
       if (kk >= nk) continue;
       int a, b;
       const T* run = run_of(kk, &a, &b);
-      lo[u] = reinterpret_cast<uintptr_t>(run);
-      hi[u] = reinterpret_cast<uintptr_t>(run + (b - a) * taps);
-      from[u] = (lo[u] & ~static_cast<uintptr_t>(15)) + (i - kk * q.pieces) * 16;
-      if (from[u] >= lo[u] && from[u] + 16 <= hi[u]) v[u] = *reinterpret_cast<const uint4*>(from[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < kPackPieces; ++u) {
-      if (from[u] >= hi[u]) continue;
-      if (from[u] >= lo[u] && from[u] + 16 <= hi[u]) {
-        *reinterpret_cast<uint4*>(tile + to[u]) = v[u];
+      const uintptr_t lo = reinterpret_cast<uintptr_t>(run), hi = reinterpret_cast<uintptr_t>(run + (b - a) * taps);
+      const uintptr_t from = (lo & ~static_cast<uintptr_t>(15)) + (i - kk * q.pieces) * 16;
+      if (from >= hi) continue;
+      to[u] = (i + kk / V) * 16;
+      if (from >= lo && from + 16 <= hi) {
+        v[u] = *reinterpret_cast<const uint4*>(from);
         continue;
       }
-      for (int e = 0; e < 16; e += sizeof(T))
-        if (from[u] + e >= lo[u] && from[u] + e < hi[u]) *reinterpret_cast<T*>(tile + to[u] + e) = *reinterpret_cast<const T*>(from[u] + e);
+      // an end of the run: its elements, all on their way together
+      __align__(16) T part[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const uintptr_t at = from + e * sizeof(T);
+        part[e] = at >= lo && at < hi ? *reinterpret_cast<const T*>(at) : T(0);
+      }
+      v[u] = *reinterpret_cast<const uint4*>(part);
     }
+#pragma unroll
+    for (int u = 0; u < kPackPieces; ++u)
+      if (to[u] >= 0) *reinterpret_cast<uint4*>(tile + to[u]) = v[u];
   }
   __syncthreads();
   const int rows = q.mode == 0 ? Kg : q.Cg, log_rows = q.mode == 0 ? q.log_k : q.log_c;
@@ -629,7 +632,9 @@ cudaError_t launch_transpose(const void* in, void* out, int B, int R, int S, int
 }
 
 // Patch of a block: 64 (float16, up to 16 taps) or 32 columns of the destination and as many of its rows as make four pieces per thread,
-// fewer while that makes fewer than `least` blocks: then rows down to runs of 64 bytes, at last columns down to 32 bytes.
+// fewer while that makes fewer than `least` blocks: then rows down to runs of 64 bytes and blocks of 1.5 KB, at last columns down to 32 bytes.
+// (With a row of 128 bytes to a block, 37 -> 418 1x1 took 418 blocks: forward at 8x8, 8 images, float16 8.6 us, 7.6 from 1 KB and 6.2 from 1.5 KB on; 2 -> 440
+// 7.5, 6.2; 64 -> 64 3x3 7.7, 7.1.  From 2 KB on 100 -> 75 5x5, 37 images, goes from 33.9 to 34.5.)
 int plan_pack(PackJob* q, int dtype, int least) {
   const int es = static_cast<int>(elem_size(dtype)), V = 16 / es, Kg = q->K / q->groups;
   const int cols = q->ldc, rows = q->mode == 0 ? Kg : q->Cg;
@@ -637,7 +642,7 @@ int plan_pack(PackJob* q, int dtype, int least) {
   while ((1 << (log_cols - 1)) >= cols && (1 << (log_cols - 1)) >= V) --log_cols;
   while (log_rows < 6 && (1 << log_rows) < rows && (q->taps * es << (log_cols + log_rows + 1)) <= kPackThreads * kPackPieces * 16) ++log_rows;
   auto blocks = [&] { return cdiv(cols, 1 << log_cols) * cdiv(rows, 1 << log_rows) * q->groups; };
-  while (log_rows > 0 && blocks() < least && (q->mode == 0 || (q->taps * es << log_rows) > 64)) --log_rows;
+  while (log_rows > 0 && blocks() < least && (q->taps * es << (log_cols + log_rows - 1)) >= 1536 && (q->mode == 0 || (q->taps * es << log_rows) > 64)) --log_rows;
   while ((es << log_cols) > 32 && 2 * blocks() < least) --log_cols;
   q->log_k = static_cast<uint8_t>(q->mode == 0 ? log_rows : log_cols);
   q->log_c = static_cast<uint8_t>(q->mode == 0 ? log_cols : log_rows);
