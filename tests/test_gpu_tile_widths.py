@@ -34,3 +34,28 @@ def test_filter_counts_off_the_tile_widths(dtype, n, k):
     assert any(v.startswith("tap") for v in seen) and any(v.startswith("slab") for v in seen)
     assert n == 1 or "slab pair" in seen
     ctx.close()
+
+
+# channels whose filter rows are whole 128-byte blocks (narrow MMAs on pairs) and others, with and without staged stores; shallow and deep
+@DTYPES
+@pytest.mark.parametrize("c,k,kernel", [(128, 75, 3), (64, 178, 3), (24, 75, 3), (24, 75, 5), (40, 96, 3), (24, 192, 3), (136, 192, 3), (72, 320, 3), (200, 330, 1)])
+def test_pairs_with_whole_and_narrow_tiles(tmp_path, dtype, c, k, kernel):
+    rs = np.random.RandomState(c + k)
+    f = np.float32
+    x = rs.standard_normal((14, c, 28, 28)).astype(dtype)
+    w = (rs.standard_normal((k, c, kernel, kernel)) / np.sqrt(c * kernel * kernel)).astype(dtype)
+    ref = O.conv2d(x.astype(f), w.astype(f), border_mode="half")
+    path = str(tmp_path / "t")
+    first = shim.Context(0)
+    shim.device_conv2d(T.from_host(first, x, "nhwc"), T.from_host(first, w), border_mode="half")
+    first.tuning_save(path)
+    first.close()
+    head, *rest = open(path).read().splitlines()
+    for choice in (4, 5):                                # the slab and the per-tap kernel on pairs, where they take the layer
+        open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + [str(choice)]) for r in rest if r.startswith("a 3.")]) + "\n")
+        ctx = shim.Context(0)
+        assert ctx.tuning_load(path) == 1
+        y = shim.device_conv2d(T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), border_mode="half")
+        assert choice == 5 or "pair" in ctx.last_variant
+        assert O.rel_err(y.to_host().astype(f), ref) < (5e-3 if dtype == f else 2e-2), ctx.last_variant
+        ctx.close()

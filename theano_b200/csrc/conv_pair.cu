@@ -132,7 +132,7 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
       const Item w = item_of(p, item, kiters);
       const TileAt at = tile_at<true>(p.walk, w.tile, rank);     // behind the last tile of an odd count: an image that is not there, zeros
       const int co_t = at.co_t, g = at.g, w0 = at.w * p.bw, h0 = at.h * p.bh, n0 = at.n * p.bn;
-      const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_out, co_t * BN, BN, true) / 2);
+      const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_mma, co_t * BN, BN, true) / 2);
       uint32_t k = w.k0;
       const int tap0 = k ? k / p.kblocks : 0;
       for (int tap = tap0, kb = k - tap0 * p.kblocks; k < w.k1 && ok; ++tap, kb = 0) {
@@ -168,7 +168,7 @@ conv_pair_kernel(const __grid_constant__ UmmaConvParams p) {
         const int buf = it & 1;
         const uint32_t aphase = (it >> 1) & 1;
         uint32_t idesc = kIdesc;
-        if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, (w.tile - quotient(w.tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, true));
+        if (p.n_mma % BN) idesc = with_columns(kIdesc, mma_columns(p.n_mma, (w.tile - quotient(w.tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, true));
         if (!wait_seen(acc_seen, &bars->acc_empty[buf], aphase ^ 1, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem + buf * BN;

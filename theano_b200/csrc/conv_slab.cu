@@ -105,9 +105,9 @@ __device__ __forceinline__ bool issue_tiles(const IssueLoop& w) {
     // a constant where the tiles are full, and for 32 columns, whose MMAs take 36 to 40 clocks whatever is left out of them: with a
     // descriptor from a register these took 4 % longer
     uint32_t idesc = kIdesc;
-    if (BN > 32 && p.n_out % BN) {
+    if (BN > 32 && p.n_mma % BN) {
       const int co_t = tile - quotient(tile, p.walk.tiles_co) * p.tiles_co;
-      idesc = with_columns(kIdesc, mma_columns(p.n_out, co_t * BN, BN, PAIR));
+      idesc = with_columns(kIdesc, mma_columns(p.n_mma, co_t * BN, BN, PAIR));
     }
     // two accumulator sets when they fit the 512 TMEM columns: the epilogue of a tile then
     // runs beside the MMAs of the next one
@@ -307,7 +307,7 @@ conv_slab_kernel(const __grid_constant__ SlabConvParams p) {
       const TileAt at = tile_at<PAIR>(p.walk, t, rank);
       const int co_t = at.co_t, g = at.g;
       // a pair's CTAs load one half each of what the tile's MMAs take (and rows that those leave out)
-      const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_out, co_t * BN, BN, true) / 2);
+      const int row0 = co_t * BN + static_cast<int>(rank) * (mma_columns(p.n_mma, co_t * BN, BN, true) / 2);
       auto load = [&](uint8_t* dst, int kb, int mat) {
         if (PAIR) tma_load_4d_pair(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);
         else tma_load_4d(dst, &p.wmap, &bars->b_full[bs], kb * kBK, row0, g, mat);

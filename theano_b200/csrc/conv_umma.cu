@@ -171,7 +171,7 @@ conv_umma_kernel(const __grid_constant__ UmmaConvParams p) {
       tc_fence_after();
       const uint32_t d_tmem = tmem + buf * BN;
       uint32_t idesc = kIdesc;
-      if (p.n_out % BN) idesc = with_columns(kIdesc, mma_columns(p.n_out, (tile - quotient(tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, false));
+      if (p.n_mma % BN) idesc = with_columns(kIdesc, mma_columns(p.n_mma, (tile - quotient(tile, p.walk.tiles_co) * p.tiles_co) * BN, BN, false));
       for (uint32_t k = k0; k < k1; ++k) {
         if (!wait_seen(seen, &bars->full[stage], phase, bars, p.wait_clocks)) { ok = false; break; }
         tc_fence_after();

@@ -154,6 +154,7 @@ struct alignas(64) UmmaConvParams {
   int tiles_w, tiles_h, tiles_n, tiles_co;
   TileWalk walk;
   int n_out;                     // output channels per group as stored
+  int n_mma;                     // those that the widths of the MMAs follow: n_out, or whole tiles
   int n_real;                    // of these, the ones with filters: the pad channels behind them are stored as 0
   void* out;
   const void* bias;              // per output channel (groups*n_out), in the data type, or null
@@ -228,6 +229,7 @@ struct alignas(64) SlabConvParams {
   int tps;                       // filter taps per stage of the filter ring (narrow tiles: several taps share a barrier round)
   int tap_groups;                // stages of a channel block: ceil(ntaps / tps)
   int n_out, n_real;             // output channels per group as stored / with filters
+  int n_mma;                     // those that the widths of the MMAs follow: n_out, or whole tiles
   void* out;
   const void* bias;
   long long out_sn, out_sc, out_sh, out_sw, out_off;
