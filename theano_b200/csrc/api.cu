@@ -867,12 +867,6 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
     s_ = std::min(s_, 2 + (int)cdiv(4, cdiv((long long)taps.size(), tps)));
     b = (int)std::min<long long>(8, (avail - 1LL * s_ * b_slab) / b_bytes);
     *ss = s_; *bs = b;
-#ifdef B200CONV_TUNE
-    if (getenv("B200_SS") && getenv("B200_BS")) {
-      const int es_ = atoi(getenv("B200_SS")), eb_ = atoi(getenv("B200_BS"));
-      if (es_ >= 2 && es_ <= 6 && eb_ >= 2 && eb_ <= 8 && 1LL * es_ * b_slab + 1LL * eb_ * b_bytes <= avail) { *ss = es_; *bs = eb_; }
-    }
-#endif
     return true;
   };
   if (!plan_rings(kSlabSmemBudget, &p.s_stages, &p.b_stages)) return 2;
@@ -969,12 +963,6 @@ int try_conv_slab(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   p.status = c->d_status;
   p.wait_clocks = c->wait_clocks;
   p.trace = c->trace;
-#ifdef B200CONV_TUNE
-  if (getenv("B200_VERBOSE"))
-    fprintf(stderr, "slab: Wt %d Ht %d N %d Cin %d n_out %d taps %d | BN %d splits %d wt %d th %d nb %d n_acc %d slab %d s %d b %d tma %d nbuf %d\n",
-            Wt, Ht, a.N, a.Cin_g, a.n_out, (int)taps.size(), BN, p.splits, p.wt, p.th, p.nb, p.n_acc, p.slab_bytes, p.s_stages, p.b_stages,
-            p.tma_out, p.stage_nbuf);
-#endif
   c->last_variant = p.ncls > 1 ? (pair ? "slab classes pair" : "slab classes") : pair ? "slab pair" : p.splits > 1 ? "slab split" : "slab";
   if (p.splits == 1) {
     KLAUNCH(c, kKConvUmma, launch_conv_slab(p, a.dtype, BN, c->num_sms, c->stream));
@@ -1344,9 +1332,6 @@ int run_conv_umma(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
                    (sn * es) % 16 == 0 && reinterpret_cast<uintptr_t>(static_cast<const char*>(out) + off * (long long)es) % 16 == 0;
   // what cannot pool does not depend on the choice that an earlier call left (a split reduction pools any output)
   if (c->epi.pool && !(allow_slab && tma)) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
-#ifdef B200CONV_TUNE
-  if (getenv("B200_VARIANT")) return run(atoi(getenv("B200_VARIANT")));
-#endif
   // A launch that adds to its own output (residual == y) must run once: it is not timed, and the choice is left to a
   // later call that may repeat it.
   const size_t out_bytes = es * out_extent(a, Wt, Ht, sn, sc, sh, sw, off);
