@@ -54,3 +54,33 @@ def test_a_stack_of_layers_against_float64(tuned, n):
         exact = np.maximum(O.conv2d(exact, w.astype(np.float64), border_mode="half", subsample=(1, 1), real="double") + b.astype(np.float64)[None, :, None, None], 0)
         assert exact.dtype == np.float64 and rel(X.to_host(), exact) < layer * BOUND
     ctx.close()
+
+
+# the kernel's number in a tuning file, its names, a layer: sums of 576, 1600 and 2304 products
+@pytest.mark.parametrize("choice,variants,n,c,k,h,ks", [(6, {"columns"}, 6, 64, 32, 40, 3), (7, {"columns pair"}, 6, 64, 64, 40, 3), (6, {"columns"}, 4, 64, 16, 30, 5),
+                                                        (5, {"tap pair", "tap pair cut"}, 128, 256, 256, 14, 3), (5, {"tap pair"}, 20, 64, 128, 28, 5)])
+def test_columns_and_pairs_against_float64(tmp_path, choice, variants, n, c, k, h, ks):
+    """The columns kernel and the per-tap kernel on pairs are no further from float64 than the one-CTA per-tap kernel: the same products, added in
+    float32.  What the order of the sums adds is below one rounding per product, 2^-24, times the square root of their number."""
+    rs = np.random.RandomState(k + ks)
+    x = rs.standard_normal((n, c, h, h)).astype(np.float32)
+    w = (rs.standard_normal((k, c, ks, ks)) / np.sqrt(c * ks * ks)).astype(np.float32)
+    want = O.conv2d(x[:3].astype(np.float64), w.astype(np.float64), border_mode="half", subsample=(1, 1), real="double")
+    assert want.dtype == np.float64
+    path, errors, results = str(tmp_path / "t"), {}, {}
+    first = shim.Context(0)
+    shim.device_conv2d(T.from_host(first, x, "nhwc"), T.from_host(first, w), border_mode="half")
+    first.tuning_save(path)
+    first.close()
+    head, *rest = open(path).read().splitlines()
+    for value in (0, choice):
+        open(path, "w").write("\n".join([head] + [" ".join(r.split()[:2] + [str(value)]) for r in rest if r.startswith("a 3.")]) + "\n")
+        ctx = shim.Context(0)
+        assert ctx.tuning_load(path) == 1
+        y = shim.device_conv2d(T.from_host(ctx, x, "nhwc"), T.from_host(ctx, w), border_mode="half").to_host()
+        assert ctx.last_variant in (variants if value else {"tap"})
+        results[value], errors[value] = y, rel(y[:3], want)
+        ctx.close()
+    order = 2.0 ** -24 * np.sqrt(c * ks * ks)
+    assert errors[choice] < BOUND and errors[choice] <= errors[0] + order, errors
+    assert rel(results[choice], results[0].astype(np.float64)) <= 2 * order

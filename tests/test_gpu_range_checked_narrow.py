@@ -1,5 +1,5 @@
-"""The range-checked build runs the tests of the columns kernel, the per-tap kernel on pairs, tile widths and filter packing: every store
-of theirs, slab index and tiled store lies inside of its buffer."""
+"""The range-checked build runs the tests of the columns kernel, the per-tap kernel on pairs with its cut tiles, tile widths and filter packing:
+every store of theirs, slab index and tiled store lies inside of its buffer."""
 import os
 import subprocess
 import sys
@@ -9,7 +9,7 @@ import pytest
 from theano_b200 import build as lib_build
 
 pytestmark = pytest.mark.gpu
-FILES = ["test_gpu_columns.py", "test_gpu_stem_gradient.py", "test_gpu_tap_pairs.py", "test_gpu_tile_widths.py", "test_gpu_filter_packing.py"]
+FILES = ["test_gpu_columns.py", "test_gpu_stem_gradient.py", "test_gpu_tap_pairs.py", "test_gpu_cut_tiles.py", "test_gpu_tile_widths.py", "test_gpu_filter_packing.py"]
 
 
 @pytest.mark.parametrize("name", FILES)
