@@ -318,7 +318,8 @@ int b200conv_selftest_wait(b200conv_ctx* ctx);
 const char* b200conv_last_algo(b200conv_ctx* ctx);
 /* The kernel variant of the last tensor-core launch: of a forward or gradInputs call "tap", "tap split", "slab", "slab split",
  * "slab pair", "slab classes", "slab classes pair", "tap pair", "tap pair cut",
- * "columns", "columns pair" or "gemm pair" (split, cut: the reduction in slices that a second kernel adds;
+ * "columns", "columns pair" or "gemm pair" (split: the reduction in slices that a second kernel adds; cut: the reduction of the last
+ * tiles in slices, added by the CTA that leaves a tile's last one, or, where no whole tile follows, by a second kernel;
  * pair: on pairs of CTAs; classes: all parity classes of strided gradInputs in one launch; columns: the filter's columns inside one
  * MMA); of gradWeights "wgrad tap" (one
  * filter tap per work item), "wgrad pair" (the same on pairs of CTAs), "wgrad groups" (tap groups share operands) or "wgrad rows"
