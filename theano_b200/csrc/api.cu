@@ -1045,11 +1045,12 @@ int try_conv_cols(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<ConvT
   if (!fits(2, 2, 1)) return 2;
   if (!launch) return 0;
   // A CTA whose tiles are all of one group loads the filters once where the ring holds them whole.  For that the CTAs are a multiple of
-  // the groups.  Those left out may cost one tile in fourteen: 3x3 on 8 groups of 32 channels, 256 images, float32, 144 CTAs for 148:
-  // 15 tiles for 14 each (14x14) 30.6 -> 30.1 us, 57 for 56 (28x28) 100 -> 91.
+  // the groups; those left out cost the rest some tiles more.  Groups of 32 channels, 3x3 at 28x28, 64 images, most tiles of a CTA with whole
+  // multiples over those without -> time with over without: float32 1.06 0.91 (20 groups), 1.07 0.93 (23), 1.10 0.96 (15), 1.18 1.01 (25), 1.23 1.03 (30);
+  // float16, whose filters are half the bytes, 1.02 0.96 (5), 1.06 0.95 (20, merged to 10), 1.07 1.06 (23), 1.10 1.09 (15), 1.18 1.16 (25).
   const int per_tile = (int)cdiv(a.Cin_g, kBK) * (p.kH / p.rps), units = pair ? c->num_sms / 2 : c->num_sms, whole = units / a.groups * a.groups;
   const long long pix_tiles = cdiv(Wt, p.wt) * cdiv(Ht, p.th) * a.N, tiles = (pair ? (pix_tiles + 1) / 2 : pix_tiles) * a.groups;
-  p.resident = whole > 0 && per_tile <= kMaxColStages && fits(2, per_tile, 1) && 14 * cdiv(tiles, whole) <= 15 * cdiv(tiles, units);
+  p.resident = whole > 0 && per_tile <= kMaxColStages && fits(2, per_tile, 1) && (es == 4 ? 10 * cdiv(tiles, whole) <= 11 * cdiv(tiles, units) : 16 * cdiv(tiles, whole) <= 17 * cdiv(tiles, units));
   if (p.resident) p.b_stages = per_tile;
   for (char step : {'s', 'b', 'f', 'b', 's', 'b', 'b'}) {
     if (step == 'b' && p.resident) continue;

@@ -9,19 +9,21 @@
 // slab's pitch is 32, 16 or 8 positions, of which the filter's width less one are halo.  The A operand of every filter row then
 // starts on a whole swizzle atom (8 rows), too; where each tap is a shift of its own, it starts anywhere.
 //
-// Measured (a B200, filters packed, slab kernel -> columns): 3x3 on 8 groups of 32 channels at 28x28, 256 images, float32 144 -> 97 us (67 without
-// the epilogue, HBM 63); 32 -> 32 at 112x112, 64 images 70 -> 49; float16 64 -> 32 at 112x112 100 -> 40; 5x5 64 -> 16 at 56x56, 256 images
-// 134 -> 46.  64 filters: float16 at 56x56, 256 images 73 -> 75, float32 at 224x224, 16 images 140 -> 133 (pairs of the slab kernel 136): an MMA
-// of 192 columns runs at its rate, but 72 KB of filters per 112 pixels come from L2.  On pairs (PAIR: two pixel tiles, M = 256, each CTA
-// loading 32 of the 64 filters) 128 -> 64 at 112x112, 64 images, float32 247 -> 197 (columns on single CTAs 243, slab pairs 225 to 247; 149 if the
-// activations came for nothing: three slabs of 24 KB in flight beside two filter stages of 36 KB; a fourth slab changes nothing), 64 -> 64 at
-// 224x224 127, float16 80.
-// Filters that fit their ring whole stay in it (`resident`): 64 -> 64 at 224x224, 16 images, on pairs 128 -> 120, 64 images 511 -> 459, with
-// pooling 508 -> 495; the 8 groups 100 -> 91.  128 -> 64 fits beside two slabs and half of the staging only, and is slower so (205 -> 216).
+// Measured (a B200, filters packed ahead, replayed as a graph, all in one build; slab kernel or its pairs, whichever is faster -> columns on single
+// CTAs): 3x3 on 8 groups of 32 channels at 28x28, 256 images, float32 121 -> 88 us (the pixels alone take HBM 63); 32 -> 32 at 112x112, 64 images 58 -> 41;
+// float16 64 -> 32 at 112x112 79 -> 40; 5x5 64 -> 16 at 56x56, 256 images 124 -> 45, float32 235 -> 91.  64 filters on single CTAs: float16 at 56x56, 256
+// images 65 -> 68, float32 at 224x224, 16 images 132 -> 138: an MMA of 192 columns runs at its rate, but 72 KB of filters per 112 pixels
+// come from L2.  On pairs (PAIR: two pixel tiles, M = 256, each CTA loading 32 of the 64 filters) the latter take 122, 64 images 507 -> 472, with pooling
+// 456 -> 449, 128 -> 64 at 112x112, 64 images 235 -> 211; float16 at 56x56 80.
+// What the steps gave, each in the build that brought it: filters that fit their ring whole and stay in it (`resident`) 64 -> 64 at 224x224, 64 images, on
+// pairs 511 -> 459, the 8 groups 100 -> 91.  Tried there: 128 -> 64 with its filters whole beside two slabs and half of the staging 205 -> 216; a fourth slab
+// for it, no change; its pixels for nothing, 197 -> 149; the 8 groups without their epilogue 97 -> 67.
 //
 // Warp roles (640 threads): warp 0 streams slabs (tile and halo, 128 bytes of channels per pixel), warp 19 filter rows, warps 1
 // and 18 issue the MMAs of one accumulator each, 16 epilogue warps (TMEM -> shuffles -> staged TMA stores, with 2x2 max pooling,
-// or, for the merged classes of a strided gradInputs, straight to the gradient's pixels).  Two accumulator sets.
+// or, for the merged classes of a strided gradInputs, straight to the gradient's pixels).  Accumulator sets: `sets`, two to four of n_acc
+// accumulators, sets * n_acc * kW * bn <= 512 columns.  The groups of epilogue warps that share no tile are `step`: with two or more each has a set of
+// its own (sets = step), a single one takes two in turn.
 #include "internal.h"
 #include "ptx.cuh"
 

@@ -125,7 +125,7 @@ cudaError_t launch_conv_reduce(const ConvReduceParams& p, int dtype, cudaStream_
   const int pl = p.epi.pool ? 2 : 1, cols = p.n_out < p.bn_cols ? p.n_out : p.bn_cols;
   const long long tiles = p.pair ? 2LL * p.tiles : p.tiles, rows = cdiv((p.wt / pl) * (p.th / pl) * p.nb, 32);
   if (tiles == 0 || rows == 0) return cudaSuccess;
-  const bool many = !p.epi.pool && tiles * rows * cdiv(cols, 16) >= 8 * 148;
+  const bool many = !p.epi.pool && tiles * rows * cdiv(cols, 16) >= 8 * kB200Sms;
   const long long col_blocks = cdiv(cols, many ? 64 : 16), units = tiles * rows * col_blocks;
   if (units >= (1LL << 30)) return cudaErrorInvalidValue;
   ReduceWalk walk;

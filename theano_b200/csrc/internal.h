@@ -512,7 +512,8 @@ struct PackBatch {
   int njobs;
 };
 static_assert(sizeof(PackBatch) <= 4096, "kernel parameters");
-constexpr int kPackBlocks = 2 * 148;           // blocks of a launch that are worth smaller patches
+constexpr int kB200Sms = 148;                 // for how finely work is cut that the hardware deals out
+constexpr int kPackBlocks = 2 * kB200Sms;      // blocks of a launch that are worth smaller patches
 int plan_pack(PackJob* q, int dtype, int least);
 cudaError_t launch_pack_filters_batch(const PackBatch& b, int total_blocks, int dtype, cudaStream_t s);
 // Row folding for layers with very few input channels (see layout.cu).

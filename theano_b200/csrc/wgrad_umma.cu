@@ -444,7 +444,9 @@ cudaError_t launch_wgrad_reduce(const float* partial, void* dw, int splits, int 
   // About four slabs per thread, at most 8 threads per sum; as many channels as make a filter's run 128 bytes; up to 32 filters
   // in a block of at most 640 threads, fewer while that leaves SMs without three blocks.  1x1 layers of few slices keep their filters, 512 bytes
   // of a slab in a row, and give up threads per sum instead: 256 -> 1024 at 14x14, 18 slices, float16, all of gradWeights 37.5 -> 33.3 us
-  // (64 -> 64 at 56x56, 148 slices, that way 39.8 -> 45.5; 128 -> 512 at 28x28, 37 slices 47.6 -> 50.1).
+  // (64 -> 64 at 56x56, 148 slices, that way 39.8 -> 45.5).  Where the line lies, by pinned slice counts, float16, 256 images: 128 -> 512 at 28x28 18 slices 58.0 -> 57.6, 24
+  // 50.2 -> 50.0, 28 47.6 -> 49.4, 37 47.5 -> 50.1; 64 -> 64 24 96.4 -> 97.2, 28 83.8 -> 85.1; wide layers gain with any count (256 -> 1024 28 44.7 -> 40.4, but 14 to
+  // 18 are faster).  The one seen to lose below it: 512 -> 2048 at 7x7, 64 images, float32, 6 slices 28.6 -> 29.7.
   const bool flat = taps == 1 && splits <= 24;
   int log_k = 5, log_q = 0, log_lanes = 0;
   while (log_lanes < 3 && splits > (4 << log_lanes)) ++log_lanes;
