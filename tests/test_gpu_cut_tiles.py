@@ -94,3 +94,35 @@ def test_a_context_made_while_the_default_stream_is_busy():
     assert np.array_equal(y, out.to_host())
     other.close()
     ctx.close()
+
+
+def test_a_replay_beside_other_launches():
+    """A graph replayed on another context's stream counts the slices of its cut tiles for itself: beside launches of the context that captured it
+    (and beside another graph's) every result is what it is alone."""
+    a, b = shim.Context(0), shim.Context(0)
+    for ctx in (a, b):
+        ctx.set_autotune(False)
+    X, W, Y, call = layer(a, np.float32)
+    call()
+    y = Y.to_host()
+    outs = [T(a, Y.shape, np.float32, "nhwc") for _ in range(2)]
+    graphs = []
+    for out in outs:
+        graphs.append(a.capture(lambda: [shim.device_conv2d(X, W, border_mode="half", out=out, flags=shim.NO_SLAB) for _ in range(3)]))
+        assert a.last_variant == "tap pair cut"
+    for _ in range(10):
+        for t in outs + [Y]:
+            a.memset(t.ptr, 255, t.nbytes)
+        a.sync()
+        for _ in range(5):
+            b.check(b.lib.b200conv_graph_launch(b.h, graphs[0].h))
+            graphs[1].launch()
+            call()
+        b.sync()
+        a.sync()
+        for t in outs + [Y]:
+            assert np.array_equal(y, t.to_host())
+    for g in graphs:
+        g.destroy()
+    b.close()
+    a.close()

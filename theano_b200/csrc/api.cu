@@ -43,6 +43,7 @@ struct b200conv_graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<void*> retained;
+  unsigned int* arrivals = nullptr;   // its own counts of slices of cut tiles: a replay may run beside other launches, on another context's stream
   long long launches = 0;   // kernels in the graph
 };
 
@@ -1181,7 +1182,9 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
     if (r != CUDA_SUCCESS && c->epi.pool) return fail(c, B200CONV_E_UNSUPPORTED, "this geometry's epilogue cannot pool");
     if (r != CUDA_SUCCESS) return run_conv_umma_one(c, a, taps_in, view_parity, Wt, Ht, out, sn, sc, sh, sw, off, bias, relu, kConvTap);
     PairCut cut = pair_cut(tiles, c->num_sms / 2, 1LL * p.ntaps * p.kblocks, BN);
-    if (c->epi.pool && (cut.tiles >= tiles || 2 * cut.tiles > kArrivals)) cut = PairCut{0, 1};      // the pair that adds the slices pools
+    unsigned int* counts = c->capturing ? c->capturing->arrivals : c->d_arrivals;
+    if (cut.tiles >= tiles || 2 * cut.tiles > kArrivals) counts = nullptr;
+    if (c->epi.pool && !counts) cut = PairCut{0, 1};                // the pair that adds the slices pools
     p.cut = (int)cut.tiles; p.splits = cut.splits;
     Scratch tmp(c);
     ConvReduceParams q;
@@ -1189,7 +1192,7 @@ int run_conv_umma_one(b200conv_ctx* c, const FwdLikeArgs& a, const std::vector<C
       rc = split_output(c, tmp, p, BN, 128, &q, cut.tiles);
       if (rc && rc != B200CONV_E_NOMEM) return rc;
       if (rc) { p.cut = 0; p.splits = 1; }                        // no memory for the slices: whole reductions need none
-      if (p.cut < tiles && 2 * p.cut <= kArrivals) p.arrivals = c->d_arrivals;
+      if (p.cut) p.arrivals = counts;
       p.walk.splits = divisor(p.splits);
       q.Ws = q.wt = p.bw; q.Hs = q.th = p.bh; q.nb = p.bn;
     }
@@ -3511,8 +3514,20 @@ int b200conv_graph_begin(b200conv_ctx* c) {
   if (c->capturing) return fail(c, B200CONV_E_INVALID, "a graph is already being captured");
   int rc = join_comm(c);
   if (rc) return rc;
+  // without memory for the counts of its own the graph's cut tiles are summed by a second kernel
+  void* counts = nullptr;
+  if (pool_alloc(c, kArrivals * sizeof(unsigned int), &counts) == 0) {
+    const cudaError_t e = cudaMemsetAsync(counts, 0, kArrivals * sizeof(unsigned int), c->stream);
+    rc = e == cudaSuccess ? wait_stream(c) : fail(c, B200CONV_E_CUDA, "clearing a graph's counts failed: %s", cudaGetErrorString(e));
+    if (rc) {                                            // they are zero for a replay on any stream, or there is no graph
+      pool_free(c, counts);
+      return rc;
+    }
+  }
   CU_OK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed));
   c->capturing = new b200conv_graph();
+  c->capturing->arrivals = static_cast<unsigned int*>(counts);
+  if (counts) c->capturing->retained.push_back(counts);
   return 0;
 }
 
