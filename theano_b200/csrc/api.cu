@@ -563,14 +563,14 @@ int mma_clocks(int bn) { return std::max(bn / 2, 32 + bn / 4); }
 // by a box of half a tile: with fewer columns the odd CTA's box starts earlier and brings rows that the even CTA has too.  Rows of whole 128-byte
 // blocks cost little (a B200, whole tiles -> narrower, 56x56, float32: 128 -> 75 3x3 73 -> 61 us; float16 178 filters 47.0 -> 45.9).  Others reach into a
 // line more each, and pay where the MMAs bound the tile: staged stores and not the very shallowest reductions (float32 40 -> 96 at 28x28 30.8 -> 27.2; float16
-// 24 -> 192 32.8 -> 35.2), the lanes' stores with 128 columns from 25 stages on (float16 200 -> 75 51 -> 44, 100 -> 75 5x5 27.6 -> 25.7, 24 -> 75 5x5
-// 69.9 -> 69.0; 72 -> 75 3x3, 18 stages, 65 -> 74; 178 filters, 25 stages, 118 -> 130).  The per-tap kernel, bound by L2, gains on whole blocks only (float32
+// 24 -> 192 32.8 -> 35.2), the lanes' stores with 128 columns, or with two rows to a line, from 25 stages on (float16 200 -> 75 51 -> 44, 100 -> 75 5x5 27.6 -> 25.7, 24 -> 75
+// 5x5 69.9 -> 69.0, 32 -> 144 5x5 162 -> 151; 72 -> 75 3x3, 18 stages, 65 -> 74; 24 -> 140 5x5 104 -> 119).  The per-tap kernel, bound by L2, gains on whole blocks only (float32
 // 128 -> 160 61.8 -> 57.3; 40 -> 160 49.7 -> 52.6, float16 200 -> 192 49.7 -> 53.4).
 bool narrow_pair_mmas(const FwdLikeArgs& a, int bn, long long stages, bool per_tap, bool staged) {
   const long long row_bytes = a.ld_w * (long long)elem_size(a.dtype);
   if (row_bytes % 128 == 0) return true;
   if (per_tap) return false;
-  return staged ? stages >= 18 || row_bytes >= 96 : bn <= 128 && stages >= 25;
+  return staged ? stages >= 18 || row_bytes >= 96 : stages >= 25 && (bn <= 128 || row_bytes % 64 == 0);
 }
 
 // Clocks that splitting the reduction of `items` = tiles x slices work items of rows x bn accumulators adds:
