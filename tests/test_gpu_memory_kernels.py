@@ -98,3 +98,34 @@ def test_elementwise_and_channel_sum(dtype, shape):
     n = shape[0] * shape[2] * shape[3]
     eps = 2.0 ** -24 if dtype == np.float32 else 2.0 ** -11
     assert got.dtype == dtype and np.all(np.abs(got - ref) <= n * 2.0 ** -24 * size + eps * np.abs(ref) + 1e-7)
+
+
+@DTYPES
+@pytest.mark.parametrize("layout", ["nhwc", "nchw", "off"])
+@pytest.mark.parametrize("c,kw,d,border", [(1, 3, 1, "half"), (4, 3, 1, "valid"), (5, 3, 1, (1, 2)), (8, 4, 2, "half"), (9, 3, 1, "half"), (12, 2, 1, (2, 3)), (16, 3, 1, "half")])
+def test_folded_images_of_one_and_two_pieces_per_pixel(dtype, layout, c, kw, d, border):
+    """Few channels: a filter row is one reduction block over a copy of the image; from both layouts, and from channels-last tensors off the 16-byte
+    boundaries.  What the pad channels of a channels-last tensor hold does not matter."""
+    ctx = shim.get_context(0)
+    rs = np.random.RandomState(c * 10 + kw)
+    f = np.float32
+    c = c if dtype == np.float16 else (c + 1) // 2           # a block is 64 float16 or 32 float32 numbers
+    x = rs.standard_normal((3, c, 12, 9)).astype(dtype)
+    w = (rs.standard_normal((20, c, 3, kw)) / np.sqrt(c * 3 * kw)).astype(dtype)
+    kw_ = dict(border_mode=border, subsample=(1, 1), filter_dilation=(d, 1))
+    if layout == "nchw":
+        X = shim.DeviceTensor.from_host(ctx, x)
+    else:
+        cp = ctx.padded_channels(c, dtype)
+        stored = np.full((3, 12, 9, cp), np.inf if cp * x.itemsize > 16 else 0, dtype)
+        stored[..., :c] = x.transpose(0, 2, 3, 1)
+        room = shim.DeviceTensor(ctx, (1, 1, 1, stored.size + 8), dtype)
+        X = shim.DeviceTensor(ctx, x.shape, dtype, "nhwc", _ptr=room.ptr + (4 if layout == "off" else 0))
+        ctx.h2d(X.ptr, stored)
+    ref = O.conv2d(x.astype(f), w.astype(f), **kw_)
+    tol = 5e-3 if dtype == f else 2e-2                       # the repository's bounds, as above
+    y = shim.device_conv2d(X, shim.DeviceTensor.from_host(ctx, w), out_layout="nhwc", **kw_)
+    assert O.rel_err(y.to_host().astype(f), ref) < tol
+    dy = rs.standard_normal(ref.shape).astype(dtype)
+    dw = shim.device_grad_weights(X, shim.DeviceTensor.from_host(ctx, dy, X.layout), (3, kw), **kw_).to_host()
+    assert O.rel_err(dw.astype(f), O.conv2d_grad_weights(x.astype(f), dy.astype(f), (3, kw), **kw_)) < tol

@@ -173,27 +173,29 @@ __global__ void pad_fold_kernel(const T* __restrict__ src, T* __restrict__ dst, 
     const int n = static_cast<int>(over(row, by_H)), h = static_cast<int>(row - static_cast<Index>(n) * H);
     const int w = static_cast<int>(idx - row * by_Wp.d) - pad_l;
     const bool inside = w >= 0 && w < W;
-    if (Cp * sizeof(T) == 16) {
-      // one pixel is 16 bytes: assemble it in registers, store it once
+    // A pixel is one to a few 16-byte pieces, each assembled in registers and stored once.  (Channel by channel, pixels of two pieces: 9 -> 80 3x3 at 14x46, 22 images,
+    // float16, forward 19.3 -> 11.0 us from NCHW, 16.0 -> 8.8 from channels-last; 12 -> 40 at 56x56, 64 images, 52 -> 34.)
+    constexpr int V = 16 / static_cast<int>(sizeof(T));
+    const T* s = src + (nhwc_in ? ((1LL * n * H + h) * W + w) * Cp : (1LL * n * C * H + h) * W + w);
+    for (int c0 = 0; c0 < Cp; c0 += V) {
       uint4 px = make_uint4(0, 0, 0, 0);
       if (inside) {
         if (nhwc_in == 1) {
-          px = *reinterpret_cast<const uint4*>(src + ((1LL * n * H + h) * W + w) * Cp);
+          px = *reinterpret_cast<const uint4*>(s + c0);
+          if (c0 + V > C) {
+            T* v = reinterpret_cast<T*>(&px);
+#pragma unroll
+            for (int e = 0; e < V; ++e)
+              if (c0 + e >= C) v[e] = T(0);
+          }
         } else {
           T* v = reinterpret_cast<T*>(&px);
-          for (int c = 0; c < C; ++c)
-            v[c] = nhwc_in ? src[((1LL * n * H + h) * W + w) * Cp + c] : src[((1LL * n * C + c) * H + h) * W + w];
+#pragma unroll
+          for (int e = 0; e < V; ++e)
+            if (c0 + e < C) v[e] = nhwc_in ? s[c0 + e] : s[1LL * (c0 + e) * H * W];
         }
       }
-      *reinterpret_cast<uint4*>(dst + 1LL * idx * Cp) = px;
-      continue;
-    }
-    T* d = dst + 1LL * idx * Cp;
-    for (int c = 0; c < Cp; ++c) {
-      T v = T(0);
-      if (inside && c < C)
-        v = nhwc_in ? src[((1LL * n * H + h) * W + w) * Cp + c] : src[((1LL * n * C + c) * H + h) * W + w];
-      d[c] = v;
+      *reinterpret_cast<uint4*>(dst + 1LL * idx * Cp + c0) = px;
     }
   }
 }
